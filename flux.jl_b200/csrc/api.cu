@@ -51,6 +51,8 @@ FB_API int32_t fb_ctx_create(int32_t device, fb_ctx** out) {
   c->smem_optin = prop.sharedMemPerBlockOptin;
   c->scratch = nullptr;
   c->scratch_bytes = 0;
+  c->pack = nullptr;
+  c->pack_bytes = 0;
   c->retired_count = 0;
   c->dev_error = nullptr;
   c->gemm_ws = nullptr;
@@ -85,6 +87,7 @@ FB_API int32_t fb_ctx_destroy(fb_ctx* ctx) {
   cudaSetDevice(ctx->device);
   cudaDeviceSynchronize();
   if (ctx->scratch) cudaFree(ctx->scratch);
+  if (ctx->pack) cudaFree(ctx->pack);
   for (int i = 0; i < ctx->retired_count; ++i) cudaFree(ctx->retired[i]);
   if (ctx->dev_error) cudaFree(ctx->dev_error);
   fb_gemm_workspace_destroy(ctx);
@@ -92,13 +95,12 @@ FB_API int32_t fb_ctx_destroy(fb_ctx* ctx) {
   return FB_OK;
 }
 
-void* fb_scratch(fb_ctx* ctx, cudaStream_t stream, size_t bytes) {
-  (void)stream;
-  if (bytes <= ctx->scratch_bytes && ctx->scratch != nullptr) return ctx->scratch;
+static void* arena_get(fb_ctx* ctx, void** block, size_t* have, size_t bytes) {
+  if (bytes <= *have && *block != nullptr) return *block;
   // grow geometrically; the outgrown block stays allocated until the context is destroyed, because work already
   // enqueued - or captured in a CUDA graph - may still name it
   size_t want = bytes < (size_t(1) << 22) ? (size_t(1) << 22) : bytes;
-  if (want < 2 * ctx->scratch_bytes) want = 2 * ctx->scratch_bytes;
+  if (want < 2 * *have) want = 2 * *have;
   want = (want + 255) & ~size_t(255);
   void* p = nullptr;
   if (cudaMalloc(&p, want) != cudaSuccess) {
@@ -106,10 +108,24 @@ void* fb_scratch(fb_ctx* ctx, cudaStream_t stream, size_t bytes) {
     fb_set_error("scratch arena: cudaMalloc of %zu bytes failed", want);
     return nullptr;
   }
-  if (ctx->scratch != nullptr && ctx->retired_count < FB_MAX_RETIRED) ctx->retired[ctx->retired_count++] = ctx->scratch;
-  ctx->scratch = p;
-  ctx->scratch_bytes = want;
+  if (*block != nullptr && ctx->retired_count < FB_MAX_RETIRED) ctx->retired[ctx->retired_count++] = *block;
+  *block = p;
+  *have = want;
   return p;
+}
+
+void* fb_scratch(fb_ctx* ctx, cudaStream_t stream, size_t bytes) {
+  (void)stream;
+  return arena_get(ctx, &ctx->scratch, &ctx->scratch_bytes, bytes);
+}
+
+void* fb_pack_scratch(fb_ctx* ctx, cudaStream_t stream, size_t bytes) {
+  if (bytes > ctx->pack_bytes) {
+    cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(stream, &cs) != cudaSuccess) cudaGetLastError();
+    if (cs != cudaStreamCaptureStatusNone) return nullptr;
+  }
+  return arena_get(ctx, &ctx->pack, &ctx->pack_bytes, bytes);
 }
 
 FB_API int32_t fb_malloc(fb_ctx* ctx, int64_t bytes, void** out) {

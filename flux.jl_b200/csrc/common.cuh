@@ -20,6 +20,8 @@ struct fb_ctx {
   size_t smem_optin;
   void* scratch;         // device arena, grown on demand, reused by every call on this context
   size_t scratch_bytes;
+  void* pack;            // second arena: 16-byte-aligned copies of GEMM operands (a caller's scratch stays untouched)
+  size_t pack_bytes;
   void* retired[FB_MAX_RETIRED];   // outgrown arena blocks, released with the context
   int retired_count;
   int32_t* dev_error;    // device error word written by kernels whose bounded waits ran out
@@ -33,6 +35,8 @@ int32_t fb_fail(int32_t code, const char* fmt, ...);
 // Returns a pointer into the context arena of at least `bytes` (256-byte aligned); grows the arena when it is
 // too small (outgrown blocks are kept until fb_ctx_destroy).  NULL on allocation failure.
 void* fb_scratch(fb_ctx* ctx, cudaStream_t stream, size_t bytes);
+// The same from the operand-copy arena; NULL (without an error) also when it would have to grow inside a stream capture.
+void* fb_pack_scratch(fb_ctx* ctx, cudaStream_t stream, size_t bytes);
 
 #define FB_CHECK_CTX(ctx)                                                   \
   do {                                                                      \
@@ -226,6 +230,8 @@ int32_t fb_gemm_tc_launch(fb_ctx* ctx, cudaStream_t stream, const fb_gemm_args& 
 bool fb_gemm_tc_supported(const fb_gemm_args& a);
 int32_t fb_gemm_dispatch(fb_ctx* ctx, cudaStream_t stream, const fb_gemm_args& a, int precision);
 void fb_gemm_workspace_destroy(fb_ctx* ctx);
+// clusters of `size` (2, 4, 8) CTAs that hold an SM each and are resident at once
+int fb_gemm_resident_clusters(fb_ctx* ctx, int size);
 // attention_tc.cu: tensor-core attention forward; FB_ERR_UNSUPPORTED when the shape is not taken
 int32_t fb_attn_fwd_tc(fb_ctx* ctx, cudaStream_t stream, const float* q, const float* k, const float* v, const uint8_t* mask,
                        float* o, float* lse, int64_t e_dim, int64_t ev_dim, int64_t lq, int64_t lk, int64_t batch, int nheads,

@@ -56,6 +56,8 @@ struct Sched {
   int num_tiles, tiles_n, dp_tiles;
   int nu;            // units per tile
   int U;             // units in the tail: (num_tiles - dp_tiles) * nu
+  int ksplit;        // CTAs of one cluster that share a tile, each with a part of its K range (1: no split)
+  int vec;           // rows of C (and Z, bias) start on 16-byte boundaries
   float* ws;         // [2 * G * ranks] slots of BM x 256 floats
   int* tickets;      // [G * ranks * 4], zero between launches
 };
@@ -68,10 +70,20 @@ struct Portion {
 struct WorkIter {
   int w, ta, tb, t0;
   __device__ WorkIter(const Sched& s, int cid, int G) : w(0) {
+    if (s.ksplit > 1) return;
     ta = t0 = (int)((long long)cid * s.U / G);
     tb = (int)((long long)(cid + 1) * s.U / G);
   }
   __device__ bool next(const Sched& s, int cid, int G, int num_kb, Portion& p) {
+    if (s.ksplit > 1) {   // one portion per CTA: part cid % ksplit of tile cid / ksplit
+      if (w++ != 0) return false;
+      const int part = cid % s.ksplit;
+      p.tile = cid / s.ksplit;
+      p.kb0 = (int)((long long)num_kb * part / s.ksplit);
+      p.kb1 = (int)((long long)num_kb * (part + 1) / s.ksplit);
+      p.partial = 0; p.tail_tile = 0; p.trail = 0;
+      return true;
+    }
     if (w * G + cid < s.dp_tiles) {
       p.tile = w * G + cid; p.kb0 = 0; p.kb1 = num_kb; p.partial = 0; p.tail_tile = 0; p.trail = 0;
       ++w;
@@ -136,7 +148,9 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
   volatile int* s_skip = (volatile int*)(bars + 3 * STAGES + 6);   // [0] mine, [1] written by the peer CTA
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const uint32_t rank = PAIR ? cluster_ctarank() : 0u;
+  const bool ksplit = !PAIR && sch.ksplit > 1;   // (pairs take whole tiles: the spare registers of their 22 warps are few)
+  const uint32_t crank = (PAIR || ksplit) ? cluster_ctarank() : 0u;
+  const uint32_t rank = PAIR ? crank : 0u;   // half of the pair's tile
   const bool leader = (rank == 0);
   const int cid = PAIR ? (int)(blockIdx.x >> 1) : (int)blockIdx.x;
   const int G = PAIR ? (int)(gridDim.x >> 1) : (int)gridDim.x;
@@ -163,21 +177,22 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     fence_proxy_async();
   }
-  if (PAIR) {
+  if (PAIR || ksplit) {
     __syncwarp();
-    cluster_sync_all();   // both CTAs run and their barriers exist: remote accesses may start
-    if (threadIdx.x == 0) {
-      // both CTAs of a pair must take the same decision
-      asm volatile("st.shared::cluster.u32 [%0], %1;" ::"r"(map_to_cta(smem_u32((const void*)(s_skip + 1)), rank ^ 1u)),
-                   "r"((int)s_skip[0])
-                   : "memory");
+    cluster_sync_all();   // all CTAs of the cluster run and their barriers exist: remote accesses may start
+    if (threadIdx.x == 0 && crank == 0) {
+      // the whole cluster must take the same decision: its first CTA's
+      for (uint32_t r = 0; r < (PAIR ? 2u : (uint32_t)sch.ksplit); ++r)
+        asm volatile("st.shared::cluster.u32 [%0], %1;" ::"r"(map_to_cta(smem_u32((const void*)(s_skip + 1)), r)), "r"((int)s_skip[0])
+                     : "memory");
     }
     __syncwarp();
     cluster_sync_all();
+    if (s_skip[1] != 0) return;
   } else {
     __syncthreads();
+    if (s_skip[0] != 0) return;
   }
-  if (s_skip[0] != 0 || s_skip[1] != 0) return;   // uniform over the CTA (pair)
 
   if (warp == 1) {
     if (PAIR) {
@@ -196,6 +211,45 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = *s_tmem;
+
+  // u: 4 consecutive columns starting at n of one row.  add_c: add what C holds; fin: this is the tile's final value,
+  // so bias, pre-activation store and activation apply.
+  auto emit4 = [&](int row, float* u, int n, bool add_c, bool fin) {
+    if (row >= M) return;
+    float* crow = C + (int64_t)row * ldc;
+    float* zrow = Z ? Z + (int64_t)row * ldc : nullptr;
+    if (n + 3 < N && (PAIR || sch.vec)) {
+      if (add_c) {
+        const float4 c4 = *(const float4*)(crow + n);
+        u[0] += c4.x; u[1] += c4.y; u[2] += c4.z; u[3] += c4.w;
+      }
+      if (fin) {
+        if (bias_n) {
+          const float4 b4 = __ldg((const float4*)(bias_n + n));
+          u[0] += b4.x; u[1] += b4.y; u[2] += b4.z; u[3] += b4.w;
+        }
+        if (zrow) *(float4*)(zrow + n) = make_float4(u[0], u[1], u[2], u[3]);
+        if (act != FB_ACT_IDENTITY) {
+#pragma unroll
+          for (int e = 0; e < 4; ++e) u[e] = fb_act_apply(act, u[e]);
+        }
+      }
+      *(float4*)(crow + n) = make_float4(u[0], u[1], u[2], u[3]);
+    } else {
+#pragma unroll
+      for (int e = 0; e < 4; ++e) {
+        if (n + e >= N) break;
+        float x = u[e];
+        if (add_c) x += crow[n + e];
+        if (fin) {
+          if (bias_n) x += __ldg(bias_n + n + e);
+          if (zrow) zrow[n + e] = x;
+          x = fb_act_apply(act, x);
+        }
+        crow[n + e] = x;
+      }
+    }
+  };
 
   if (warp == 0) {
     // ------------------------------------------------------------------ TMA producer ---
@@ -319,42 +373,6 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
     while (ok && wi.next(sch, cid, G, num_kb, p)) {
       const int n0 = tile_n0(p.tile);
       const int row = tile_m0(p.tile) + 32 * q + lane;
-      float* crow = C + (int64_t)row * ldc;
-      float* zrow = Z ? Z + (int64_t)row * ldc : nullptr;
-      // u: 4 consecutive columns starting at n of this lane's row.  add_c: add what C holds; fin: this is the
-      // tile's final value, so bias, pre-activation store and activation apply.
-      auto emit4 = [&](float* u, int n, bool add_c, bool fin) {
-        if (row >= M) return;
-        if (n + 3 < N) {
-          if (add_c) {
-            const float4 c4 = *(const float4*)(crow + n);
-            u[0] += c4.x; u[1] += c4.y; u[2] += c4.z; u[3] += c4.w;
-          }
-          if (fin) {
-            if (bias_n) {
-              const float4 b4 = __ldg((const float4*)(bias_n + n));
-              u[0] += b4.x; u[1] += b4.y; u[2] += b4.z; u[3] += b4.w;
-            }
-            if (zrow) *(float4*)(zrow + n) = make_float4(u[0], u[1], u[2], u[3]);
-            if (act != FB_ACT_IDENTITY) {
-#pragma unroll
-              for (int e = 0; e < 4; ++e) u[e] = fb_act_apply(act, u[e]);
-            }
-          }
-          *(float4*)(crow + n) = make_float4(u[0], u[1], u[2], u[3]);
-        } else {
-          for (int e = 0; e < 4 && n + e < N; ++e) {
-            float x = u[e];
-            if (add_c) x += crow[n + e];
-            if (fin) {
-              if (bias_n) x += __ldg(bias_n + n + e);
-              if (zrow) zrow[n + e] = x;
-              x = fb_act_apply(act, x);
-            }
-            crow[n + e] = x;
-          }
-        }
-      };
       // A part of a split tile collects its sums in a workspace slot (always 256 floats per row).  The parts of
       // a tile are the CTAs c_first .. c_last whose unit ranges meet it (those with an empty range excepted).
       float* srow = nullptr;
@@ -362,6 +380,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
       int* ticket = nullptr;
       const int row_off = (32 * q + lane) * 256;
       const int step_q = sch.U / G, step_r = sch.U % G;
+      if (ksplit) srow = sch.ws + (size_t)blockIdx.x * BM * 256 + row_off;   // only used beyond one segment
       if (p.partial) {
         srow = sch.ws + (size_t)((2 * cid + p.trail) * RANKS + (int)rank) * BM * 256 + row_off;
         u_lo = p.tail_tile * sch.nu;
@@ -434,10 +453,24 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
           tc_ld_32x32b_x32(tmem_base + ((uint32_t)(32 * q) << 16) + (uint32_t)(buf * BN + cc * 32), r);
           tc_wait_ld();
           float* v = reinterpret_cast<float*>(r);
-          if (!p.partial) {
+          if (ksplit) {
+            // earlier segments collect in this CTA's slot; the last one leaves the sums in shared memory (all MMAs have
+            // read their stages by now), from where the cluster adds them up
+            if (seg > 0) {
+              const float4* s4 = (const float4*)(srow + cc * 32);
+#pragma unroll
+              for (int j = 0; j < 8; ++j) {
+                const float4 o = s4[j];
+                v[4 * j] += o.x; v[4 * j + 1] += o.y; v[4 * j + 2] += o.z; v[4 * j + 3] += o.w;
+              }
+            }
+            float4* d4 = last ? (float4*)((float*)smem + (32 * q + lane) * (BN + 4) + cc * 32) : (float4*)(srow + cc * 32);
+#pragma unroll
+            for (int j = 0; j < 8; ++j) d4[j] = make_float4(v[4 * j], v[4 * j + 1], v[4 * j + 2], v[4 * j + 3]);
+          } else if (!p.partial) {
             const bool add_c = (seg > 0) || (accumulate != 0);
 #pragma unroll
-            for (int j = 0; j < 8; ++j) emit4(v + 4 * j, nb + 4 * j, add_c, last);
+            for (int j = 0; j < 8; ++j) emit4(row, v + 4 * j, nb + 4 * j, add_c, last);
           } else {
             float4* s4 = (float4*)(srow + cc * 32);
             if (seg > 0) {
@@ -451,7 +484,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
               add_parts(v, cc * 32, c_first + 1);
               add_parts(v + 16, cc * 32 + 16, c_first + 1);
 #pragma unroll
-              for (int j = 0; j < 8; ++j) emit4(v + 4 * j, nb + 4 * j, accumulate != 0, true);
+              for (int j = 0; j < 8; ++j) emit4(row, v + 4 * j, nb + 4 * j, accumulate != 0, true);
             } else {
 #pragma unroll
               for (int j = 0; j < 8; ++j) s4[j] = make_float4(v[4 * j], v[4 * j + 1], v[4 * j + 2], v[4 * j + 3]);
@@ -488,7 +521,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
               for (int j = 0; j < 16; ++j) v[j] = 0.0f;
               add_parts(v, hc * 16, c_first);
 #pragma unroll
-              for (int j = 0; j < 4; ++j) emit4(v + 4 * j, nb + 4 * j, accumulate != 0, true);
+              for (int j = 0; j < 4; ++j) emit4(row, v + 4 * j, nb + 4 * j, accumulate != 0, true);
             }
             __syncwarp();
             if (lane == 0) *ticket = 0;   // ready for the next launch
@@ -539,10 +572,35 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
     }
   }
 
+  // ---------------------------------------------- split K: the cluster adds up its parts ---
+  if (ksplit) {
+    __syncwarp();
+    cluster_sync_all();
+    const int S = sch.ksplit, part = (int)crank, rows = BM / S;
+    const int m0 = tile_m0(cid / S), n0 = tile_n0(cid / S);
+    for (int e = threadIdx.x; e < rows * (BN / 4); e += cfg::NUM_THREADS) {
+      const int r = part * rows + e / (BN / 4), c = 4 * (e % (BN / 4));
+      if (m0 + r >= M || n0 + c >= N) continue;
+      const uint32_t src = smem_base + (uint32_t)((r * (BN + 4) + c) * 4);
+      float4 x[8];
+#pragma unroll
+      for (int i = 0; i < 8; ++i)
+        if (i < S) {
+          const uint32_t a = map_to_cta(src, (uint32_t)i);
+          asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(x[i].x), "=f"(x[i].y), "=f"(x[i].z), "=f"(x[i].w) : "r"(a) : "memory");
+        }
+      float v[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+#pragma unroll
+      for (int i = 0; i < 8; ++i)
+        if (i < S) { v[0] += x[i].x; v[1] += x[i].y; v[2] += x[i].z; v[3] += x[i].w; }
+      emit4(m0 + r, v, n0 + c, accumulate != 0, true);
+    }
+  }
+
   // ---------------------------------------------------------------------- teardown ---
   tc_fence_before();
   __syncthreads();
-  if (PAIR) cluster_sync_all();   // neither CTA may release tensor memory while its peer can still touch it
+  if (PAIR || ksplit) cluster_sync_all();   // no CTA may release its tensor or shared memory while a peer can still touch it
   if (warp == 1) {
     __syncwarp();
     if (PAIR)
@@ -558,6 +616,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
 struct GemmWorkspace {
   float* ws;
   int* tickets;
+  int clusters[4];   // clusters of 1, 2, 4, 8 CTAs that are resident at once
 };
 
 // 3-d view {32, K, MN / 32} of an MN-major matrix (row k holds MN contiguous floats): box {32, BK, chunks}.
@@ -575,7 +634,7 @@ bool encode_map_mn3d(CUtensorMap* map, const float* base, int64_t K, int64_t MN,
 }
 
 template <bool A_MN, bool B_MN, int BN, int PASSES, bool PAIR, int SG>
-int32_t launch_variant(fb_ctx* ctx, cudaStream_t stream, const fb_gemm_args& a) {
+int32_t launch_variant(fb_ctx* ctx, cudaStream_t stream, const fb_gemm_args& a, int ksplit) {
   using cfg = Cfg<BN, PASSES, PAIR, SG>;
   CUtensorMap tmA, tmB;
   bool ok;
@@ -617,6 +676,8 @@ int32_t launch_variant(fb_ctx* ctx, cudaStream_t stream, const fb_gemm_args& a) 
   sch.dp_tiles = (int)num_tiles;
   sch.nu = (num_kb + UNIT_KB - 1) / UNIT_KB;
   sch.U = 0;
+  sch.ksplit = ksplit;
+  sch.vec = (a.ldc % 4 == 0 && fb_aligned16(a.C) && (!a.Z || fb_aligned16(a.Z)) && (!a.bias_n || fb_aligned16(a.bias_n))) ? 1 : 0;
   sch.ws = nullptr;
   sch.tickets = nullptr;
   int64_t G = Gmax < num_tiles ? Gmax : num_tiles;
@@ -624,7 +685,10 @@ int32_t launch_variant(fb_ctx* ctx, cudaStream_t stream, const fb_gemm_args& a) 
   // gain nothing: the kernel runs at the power limit, where idle SMs let the busy ones clock higher.)
   const int64_t rest = num_tiles % Gmax;
   const GemmWorkspace* gw = (const GemmWorkspace*)ctx->gemm_ws;
-  if (rest != 0 && 4 * rest < 3 * Gmax && sch.nu > 1 && rest * sch.nu < 0x40000000 && gw != nullptr) {
+  if (ksplit > 1) {
+    G = num_tiles * ksplit;
+    sch.ws = gw->ws;
+  } else if (num_tiles > Gmax && rest != 0 && 4 * rest < 3 * Gmax && sch.nu > 1 && rest * sch.nu < 0x40000000 && gw != nullptr) {
     sch.dp_tiles = (int)(num_tiles - rest);
     sch.U = (int)(rest * sch.nu);
     sch.ws = gw->ws;
@@ -639,7 +703,7 @@ int32_t launch_variant(fb_ctx* ctx, cudaStream_t stream, const fb_gemm_args& a) 
   lc.stream = stream;
   cudaLaunchAttribute attr[1];
   attr[0].id = cudaLaunchAttributeClusterDimension;
-  attr[0].val.clusterDim.x = PAIR ? 2 : 1;
+  attr[0].val.clusterDim.x = (PAIR ? 2 : 1) * ksplit;
   attr[0].val.clusterDim.y = 1;
   attr[0].val.clusterDim.z = 1;
   lc.attrs = attr;
@@ -651,37 +715,101 @@ int32_t launch_variant(fb_ctx* ctx, cudaStream_t stream, const fb_gemm_args& a) 
 }
 
 template <int BN, int PASSES, bool PAIR, int SG>
-int32_t launch_layout_sg(fb_ctx* ctx, cudaStream_t stream, const fb_gemm_args& a) {
+int32_t launch_layout_sg(fb_ctx* ctx, cudaStream_t stream, const fb_gemm_args& a, int ksplit) {
   if (a.a_mn_major) {
-    if (a.b_mn_major) return launch_variant<true, true, BN, PASSES, PAIR, SG>(ctx, stream, a);
-    return launch_variant<true, false, BN, PASSES, PAIR, SG>(ctx, stream, a);
+    if (a.b_mn_major) return launch_variant<true, true, BN, PASSES, PAIR, SG>(ctx, stream, a, ksplit);
+    return launch_variant<true, false, BN, PASSES, PAIR, SG>(ctx, stream, a, ksplit);
   }
-  if (a.b_mn_major) return launch_variant<false, true, BN, PASSES, PAIR, SG>(ctx, stream, a);
-  return launch_variant<false, false, BN, PASSES, PAIR, SG>(ctx, stream, a);
+  if (a.b_mn_major) return launch_variant<false, true, BN, PASSES, PAIR, SG>(ctx, stream, a, ksplit);
+  return launch_variant<false, false, BN, PASSES, PAIR, SG>(ctx, stream, a, ksplit);
 }
 
 // Split-warp groups: the one-CTA tile is bound by shared-memory bandwidth and gains nothing beyond two groups; the
 // two-CTA tile is bound by the latency of one split (wait, load, store, proxy fence, remote arrive) and keeps
 // gaining up to four (measured 157 -> 175 -> 182 TFLOP/s for 2 -> 3 -> 4 groups at 4096^3).
 template <int BN, int PASSES, bool PAIR>
-int32_t launch_layout(fb_ctx* ctx, cudaStream_t stream, const fb_gemm_args& a) {
-  return launch_layout_sg<BN, PASSES, PAIR, (PAIR ? 4 : 2)>(ctx, stream, a);
+int32_t launch_layout(fb_ctx* ctx, cudaStream_t stream, const fb_gemm_args& a, int ksplit) {
+  return launch_layout_sg<BN, PASSES, PAIR, (PAIR ? 4 : 2)>(ctx, stream, a, ksplit);
 }
 
 // Measured on B200 (4096^3, 3xTF32, persistent kernels): one-CTA 128 x 256 tiles 200-213 TFLOP/s (every MMA re-reads
 // all 256 B columns from shared memory), two-CTA 256 x 256 tiles 215-232 TFLOP/s (each CTA reads only its 128 B
 // columns).  At 1024 x 4096 x 4096 (one wave of 64 two-CTA tiles on 74 SM pairs) both, and cutting every tile along
 // K over all pairs, take 0.204-0.207 ms: what is left there is the unoverlapped prologue and epilogue of a single tile.
+// How a 3xTF32 product is cut.  Shapes: 128 x 128 (0) and 128 x 256 (1) tiles of one CTA, 256 x 256 tiles of a CTA pair
+// (2); ksplit CTAs of one cluster share a tile's K range where whole tiles would leave SMs idle.  The choice is
+// the smallest of the modelled times; its constants (us) are fitted to measurements on B200: a k-block of 16 costs
+// 0.53 / 0.62 / 0.62, a tile's prologue and epilogue that the next one does not hide 0.5 / 2.5 / 2.5, a launch 5, the
+// cluster's reduction 3.5.  A split runs in one wave (its clusters must all fit) so that a slot of the workspace belongs
+// to one CTA.  1024 x 1024 x 16384: 259 -> 158 us; 784 x 512 x 1024: 41 -> 17 us; 231 x 512 x 512: 27 -> 12 us.
+struct Plan { int shape, ksplit; };
+Plan plan_3xtf32(fb_ctx* ctx, const fb_gemm_args& a, bool force_pair) {
+  const GemmWorkspace* gw = (const GemmWorkspace*)ctx->gemm_ws;
+  const int sms = ctx->sm_count - ctx->reserved_sms;
+  const int num_kb = (int)((a.K + BK - 1) / BK);
+  static const int bm[3] = {128, 128, 256}, bn[3] = {128, 256, 256};
+  static const double t_kb[3] = {0.53, 0.62, 0.62}, t_tile[3] = {0.5, 2.5, 2.5};
+  Plan best = {0, 1};
+  double best_t = 1e30;
+  for (int sh = 2; sh >= 0; --sh) {
+    if (sh == 2 && (a.M < 256 || a.N < 256 || a.ldc % 4 || !fb_aligned16(a.C) || !fb_aligned16(a.Z) || !fb_aligned16(a.bias_n))) continue;
+    if (force_pair && sh != 2 && best_t < 1e30) continue;
+    if (sh == 1 && a.N <= 128) continue;
+    const int ranks = sh == 2 ? 2 : 1;
+    const int64_t tiles = ((a.M + bm[sh] - 1) / bm[sh]) * ((a.N + bn[sh] - 1) / bn[sh]);
+    for (int lg = 0; lg < 4; ++lg) {
+      const int s = 1 << lg;
+      double t;
+      if (s == 1) {
+        const int64_t slots = sms / ranks > 0 ? sms / ranks : 1;
+        double waves = (double)((tiles + slots - 1) / slots);
+        const int64_t rest = tiles % slots;
+        if (tiles > slots && rest != 0 && 4 * rest < 3 * slots && num_kb > UNIT_KB) waves = (double)tiles / (double)slots + 0.15;   // the tail is split
+        t = 5.0 + waves * (num_kb * t_kb[sh] + t_tile[sh]);
+      } else {
+        if (sh == 2 || gw == nullptr || ctx->reserved_sms != 0 || num_kb < 2 * s || tiles > gw->clusters[lg]) break;
+        t = 8.5 + ((num_kb + s - 1) / s) * t_kb[sh] + t_tile[sh];
+      }
+      if (t < best_t) { best_t = t; best.shape = sh; best.ksplit = s; }
+    }
+  }
+  return best;
+}
+
+// How many clusters of 2, 4 and 8 CTAs with the GEMM's shared memory are resident at once.
+void query_clusters(fb_ctx* ctx, int* clusters) {
+  auto kern = gemm_tc_kernel<false, true, 256, 3, false, 2>;
+  using cfg = Cfg<256, 3, false, 2>;
+  clusters[0] = ctx->sm_count;
+  for (int lg = 1; lg < 4; ++lg) {
+    clusters[lg] = 0;
+    cudaLaunchConfig_t lc;
+    memset(&lc, 0, sizeof(lc));
+    lc.gridDim = dim3((unsigned)(ctx->sm_count / (1 << lg) * (1 << lg)), 1, 1);
+    lc.blockDim = dim3(cfg::NUM_THREADS, 1, 1);
+    lc.dynamicSmemBytes = cfg::SMEM_BYTES;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = 1u << lg;
+    attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+    lc.attrs = attr;
+    lc.numAttrs = 1;
+    int n = 0;
+    if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, cfg::SMEM_BYTES) == cudaSuccess &&
+        cudaOccupancyMaxActiveClusters(&n, kern, &lc) == cudaSuccess)
+      clusters[lg] = n;
+    else
+      cudaGetLastError();
+  }
+}
+
 }  // namespace
 
 bool fb_gemm_tc_supported(const fb_gemm_args& a) {
   if (a.M < 1 || a.N < 1 || a.K < 1) return false;
   if (a.M > 0x7fffff00 || a.N > 0x7fffff00 || a.K > 0x7fffff00) return false;
   if (a.bias_m != nullptr) return false;
-  if (!fb_aligned16(a.A) || !fb_aligned16(a.B) || !fb_aligned16(a.C)) return false;
-  if (a.Z && !fb_aligned16(a.Z)) return false;
-  if (a.bias_n && !fb_aligned16(a.bias_n)) return false;
-  if (a.lda % 4 || a.ldb % 4 || a.ldc % 4) return false;
+  if (!fb_aligned16(a.A) || !fb_aligned16(a.B) || a.lda % 4 || a.ldb % 4) return false;   // TMA; C may be unaligned
   // the leading dimension must cover the contiguous extent
   if (a.lda < (a.a_mn_major ? a.M : a.K) || a.ldb < (a.b_mn_major ? a.N : a.K) || a.ldc < a.N) return false;
   return true;
@@ -690,22 +818,14 @@ bool fb_gemm_tc_supported(const fb_gemm_args& a) {
 // passes: 3 = 3xTF32, 1 = one TF32 pass, 32 = 3xTF32 on two-CTA tiles where the shape allows
 int32_t fb_gemm_tc_launch(fb_ctx* ctx, cudaStream_t stream, const fb_gemm_args& a, int passes) {
   if (!fb_gemm_tc_supported(a)) return FB_ERR_UNSUPPORTED;
-  const bool passes_flag_pair = (passes == 32);
-  if (passes_flag_pair) passes = 3;
-  // 128 x 256 tiles unless they would leave most of the machine idle: the wider tile does twice the MMA work per
-  // split / barrier round trip, so one 86 %-full wave of them beats two waves of 128 x 128 tiles
-  const int64_t tiles256 = ((a.M + BM - 1) / BM) * ((a.N + 255) / 256);
-  const bool narrow = (a.N <= 128) || (2 * tiles256 <= ctx->sm_count);
-  if (passes == 3) {
-    // two-CTA 256 x 256 tiles once there are enough of them to occupy a good part of the SM pairs
-    const int64_t pair_tiles = ((a.M + 255) / 256) * ((a.N + 255) / 256);
-    if (a.M >= 256 && a.N >= 256 && (passes_flag_pair || 4 * pair_tiles >= ctx->sm_count))
-      return launch_layout<256, 3, true>(ctx, stream, a);
-    if (narrow) return launch_layout<128, 3, false>(ctx, stream, a);
-    return launch_layout<256, 3, false>(ctx, stream, a);
+  if (passes == 1) {
+    const bool narrow1 = (a.N <= 128) || (2 * ((a.M + BM - 1) / BM) * ((a.N + 255) / 256) <= ctx->sm_count);
+    return narrow1 ? launch_layout<128, 1, false>(ctx, stream, a, 1) : launch_layout<256, 1, false>(ctx, stream, a, 1);
   }
-  if (narrow) return launch_layout<128, 1, false>(ctx, stream, a);
-  return launch_layout<256, 1, false>(ctx, stream, a);
+  const Plan p = plan_3xtf32(ctx, a, passes == 32);
+  if (p.shape == 0) return launch_layout<128, 3, false>(ctx, stream, a, p.ksplit);
+  if (p.shape == 1) return launch_layout<256, 3, false>(ctx, stream, a, p.ksplit);
+  return launch_layout<256, 3, true>(ctx, stream, a, p.ksplit);
 }
 
 // Called by fb_ctx_create / fb_ctx_destroy.  The workspace is allocated up front (2 slots of 128 x 256 floats per
@@ -724,6 +844,7 @@ int32_t fb_gemm_workspace_create(fb_ctx* ctx) {
     return fb_fail(FB_ERR_ALLOC, "fb_ctx_create: GEMM workspace allocation failed");
   }
   cudaMemset(gw->tickets, 0, tickets * sizeof(int));
+  query_clusters(ctx, gw->clusters);
   ctx->gemm_ws = gw;
   return FB_OK;
 }
@@ -731,6 +852,11 @@ int32_t fb_gemm_workspace_create(fb_ctx* ctx) {
 void fb_gemm_workspace_reset(fb_ctx* ctx, cudaStream_t stream) {
   GemmWorkspace* gw = (GemmWorkspace*)ctx->gemm_ws;
   if (gw != nullptr && gw->tickets != nullptr) cudaMemsetAsync(gw->tickets, 0, (size_t)ctx->sm_count * 4 * sizeof(int), stream);
+}
+
+int fb_gemm_resident_clusters(fb_ctx* ctx, int size) {
+  const GemmWorkspace* gw = (const GemmWorkspace*)ctx->gemm_ws;
+  return gw == nullptr ? 0 : gw->clusters[size == 8 ? 3 : size == 4 ? 2 : size == 2 ? 1 : 0];
 }
 
 void fb_gemm_workspace_destroy(fb_ctx* ctx) {

@@ -1,0 +1,84 @@
+"""GPU tests of the matmul kernels where their cuts fall: K ranges shared by a cluster, 16-wide tiles, remainders of the
+64 x 64 and 128 x 256 tiles, rows that do not start on 16-byte boundaries.  Reference: the product in float64.
+
+Tolerance: an FMA chain of K terms of N(0, 1) products is off by at most K * 2^-24 * sum|a b| / 2 and in practice by
+sqrt(K) of it; the tensor-core path drops terms of 2^-22 and truncates while it accumulates (at most 2048 terms at a time).
+3e-5 of the result's norm covers both; bf16 storage rounds the result to 2^-9."""
+import ctypes as C
+
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module")
+def ctx():
+    import fluxb200 as F
+    return F.context(0)
+
+
+def _operands(ta, tb, m, n, k, pad, dtype):
+    """Column-major op(A)[m, k] op(B)[k, n] as row-major torch views with `pad` extra values per row."""
+    g = torch.Generator(device="cuda").manual_seed(m * 31 + n * 7 + k)
+    ra, ca = (m, k) if ta else (k, m)
+    rb, cb = (k, n) if tb else (n, k)
+    A = torch.randn(ra, ca + pad, generator=g, device="cuda").to(dtype)
+    B = torch.randn(rb, cb + pad, generator=g, device="cuda").to(dtype)
+    a64, b64 = A[:, :ca].double(), B[:, :cb].double()
+    ref = (b64.T if tb else b64) @ (a64.T if ta else a64)      # [n][m]
+    return A, B, ref
+
+
+# the FMA kernel: one row, 16-row and 16-column tiles and one past them, K of less than a stage, of several clusters, odd
+# leading dimensions; the tensor-core kernel: K split over 2, 4 and 8 CTAs (with a ragged last part and two accumulation
+# segments per part), pairs, packed operands
+@pytest.mark.parametrize("ta,tb", [(0, 0), (1, 0), (0, 1), (1, 1)])
+@pytest.mark.parametrize("m,n,k,pad", [(512, 1, 784, 0), (10, 16, 33, 1), (65, 17, 1, 0), (16, 300, 1000, 3), (33, 129, 260, 2),
+                                       (520, 300, 1000, 0), (264, 140, 2100, 0), (516, 1030, 4100, 0), (1000, 1000, 9000, 0),
+                                       (601, 515, 701, 0), (1003, 259, 2049, 1)])
+@pytest.mark.parametrize("accumulate", [0, 1])
+def test_gemm_f32_cuts(ctx, ta, tb, m, n, k, pad, accumulate):
+    from fluxb200 import lib
+    A, B, ref = _operands(ta, tb, m, n, k, pad, torch.float32)
+    out = torch.ones(n, m + pad, device="cuda")
+    lib.call("fb_gemm_f32", ctx.handle, ctx.stream, ta, tb, m, n, k, C.c_void_p(A.data_ptr()), A.shape[1], C.c_void_p(B.data_ptr()),
+             B.shape[1], C.c_void_p(out.data_ptr()), m + pad, accumulate, 0)
+    assert ctx.device_error() == 0
+    err = (out[:, :m].double() - (1.0 if accumulate else 0.0) - ref).norm() / ref.norm()
+    assert err < 3e-5, float(err)
+    assert bool((out[:, m:] == 1.0).all())     # nothing is written between the rows
+
+
+@pytest.mark.parametrize("ta,tb", [(0, 0), (1, 0), (0, 1), (1, 1)])
+@pytest.mark.parametrize("m,n,k", [(512, 104, 784), (264, 200, 1000), (1000, 2048, 4096), (1024, 1024, 8200), (136, 8, 64), (520, 264, 64)])
+@pytest.mark.parametrize("f32", [0, 1])
+def test_gemm_bf16_cuts(ctx, ta, tb, m, n, k, f32):
+    from fluxb200 import lib
+    A, B, ref = _operands(ta, tb, m, n, k, 0, torch.bfloat16)
+    for accumulate in (0, 1):
+        out = torch.ones(n, m, device="cuda", dtype=torch.float32 if f32 else torch.bfloat16)
+        lib.call("fb_gemm_bf16", ctx.handle, ctx.stream, ta, tb, m, n, k, C.c_void_p(A.data_ptr()), A.shape[1], C.c_void_p(B.data_ptr()),
+                 B.shape[1], C.c_void_p(out.data_ptr()), m, accumulate, f32)
+        err = (out.double() - (1.0 if accumulate else 0.0) - ref).norm() / ref.norm()
+        assert err < (3e-5 if f32 else 2.0 ** -9), float(err)
+    assert ctx.device_error() == 0
+
+
+@pytest.mark.parametrize("act", ["identity", "relu", "gelu_tanh"])
+@pytest.mark.parametrize("out_dim,in_dim,n", [(512, 784, 1), (10, 512, 100), (513, 300, 70), (512, 784, 1024), (1001, 520, 500)])
+def test_dense_forward_epilogues_of_cut_tiles(ctx, act, out_dim, in_dim, n):
+    """bias, activation and pre-activation store behind every way a tile is finished"""
+    from fluxb200 import lib
+    g = torch.Generator(device="cuda").manual_seed(out_dim + n)
+    W = torch.randn(in_dim, out_dim, generator=g, device="cuda") / in_dim ** 0.5
+    b = torch.randn(out_dim, generator=g, device="cuda")
+    x = torch.randn(n, in_dim, generator=g, device="cuda")
+    y, z = torch.empty(n, out_dim, device="cuda"), torch.empty(n, out_dim, device="cuda")
+    p = lambda t: C.c_void_p(t.data_ptr())
+    lib.call("fb_dense_fwd", ctx.handle, ctx.stream, lib.ACT[act], 0, p(W), p(b), p(x), p(y), p(z), out_dim, in_dim, n)
+    zr = x.double() @ W.double() + b.double()
+    yr = {"identity": lambda v: v, "relu": torch.relu, "gelu_tanh": lambda v: torch.nn.functional.gelu(v, approximate="tanh")}[act](zr)
+    assert ((z.double() - zr).norm() / zr.norm()) < 3e-5
+    assert ((y.double() - yr).norm() / yr.norm()) < 3e-5
+    assert ctx.device_error() == 0
