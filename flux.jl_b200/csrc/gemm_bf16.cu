@@ -75,7 +75,7 @@ template <bool A_MN, bool B_MN, int BN, bool PAIR>
 __global__ void __launch_bounds__(HCfg<BN, PAIR>::NUM_THREADS, 1)
 gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB, void* __restrict__ Cv,
                  int64_t ldc, uint16_t* __restrict__ Z, const uint16_t* __restrict__ bias_n, int M, int N, int K, int act,
-                 int accumulate, int out_f32, int32_t* __restrict__ dev_err, int a3d, int b3d, int num_tiles, int tiles_n) {
+                 int accumulate, int out_f32, int32_t* __restrict__ dev_err, int a3d, int b3d, int num_tiles, int tiles_n, int ksplit) {
   using cfg = HCfg<BN, PAIR>;
   constexpr int STAGES = cfg::STAGES;
   extern __shared__ uint8_t smem_raw[];
@@ -93,11 +93,16 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
   volatile int* s_skip = (volatile int*)(bars + 3 * STAGES + 6);   // [0] mine, [1] written by the peer CTA
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const uint32_t rank = PAIR ? cluster_ctarank() : 0u;
+  // ksplit > 1: the CTAs (pairs) of a cluster share one tile, each with a part of its K range
+  const uint32_t crank = (PAIR || ksplit > 1) ? cluster_ctarank() : 0u;
+  const uint32_t rank = PAIR ? (crank & 1u) : 0u;
+  const uint32_t lead_rank = crank - rank;
   const bool leader = (rank == 0);
   const int cid = PAIR ? (int)(blockIdx.x >> 1) : (int)blockIdx.x;
   const int G = PAIR ? (int)(gridDim.x >> 1) : (int)gridDim.x;
-  const int num_kb = (K + HBK - 1) / HBK;
+  const int all_kb = (K + HBK - 1) / HBK, part = cid % ksplit;
+  const int kb0 = (int)((long long)all_kb * part / ksplit), num_kb = (int)((long long)all_kb * (part + 1) / ksplit) - kb0;
+  const int tile_beg = cid / ksplit, tile_step = ksplit > 1 ? num_tiles : G;
   auto tile_m0 = [&](int t) { return PAIR ? (t / tiles_n) * 256 + 128 * (int)rank : (t / tiles_n) * HBM_; };
   auto tile_n0 = [&](int t) { return (t % tiles_n) * BN; };
 
@@ -116,20 +121,22 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     fence_proxy_async();
   }
-  if (PAIR) {
+  if (PAIR || ksplit > 1) {
     __syncwarp();
-    cluster_sync_all();   // both CTAs run and their barriers exist: remote accesses may start
-    if (threadIdx.x == 0) {
-      asm volatile("st.shared::cluster.u32 [%0], %1;" ::"r"(map_to_cta(smem_u32((const void*)(s_skip + 1)), rank ^ 1u)),
-                   "r"((int)s_skip[0])
-                   : "memory");
+    cluster_sync_all();   // all CTAs of the cluster run and their barriers exist: remote accesses may start
+    if (threadIdx.x == 0 && crank == 0) {
+      // the whole cluster must take the same decision: its first CTA's
+      for (uint32_t r = 0; r < (uint32_t)ksplit * (PAIR ? 2u : 1u); ++r)
+        asm volatile("st.shared::cluster.u32 [%0], %1;" ::"r"(map_to_cta(smem_u32((const void*)(s_skip + 1)), r)), "r"((int)s_skip[0])
+                     : "memory");
     }
     __syncwarp();
     cluster_sync_all();
+    if (s_skip[1] != 0) return;
   } else {
     __syncthreads();
+    if (s_skip[0] != 0) return;
   }
-  if (s_skip[0] != 0 || s_skip[1] != 0) return;   // uniform over the CTA (pair)
 
   if (warp == 1) {
     if (PAIR) {
@@ -149,12 +156,64 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
   tc_fence_after();
   const uint32_t tmem_base = *s_tmem;
 
+  // 8 consecutive columns of one row: accumulate, bias, pre-activation, activation, store
+  auto emit8 = [&](int row, float* u, int n) {
+    if (row >= M || n >= N) return;
+    if (n + 7 < N) {
+      const int64_t o = (int64_t)row * ldc + n;
+      uint16_t* crow = (uint16_t*)Cv + o;
+      float* frow = (float*)Cv + o;
+      if (accumulate) {
+        if (out_f32) {
+#pragma unroll
+          for (int h = 0; h < 2; ++h) {
+            const float4 c4 = *(const float4*)(frow + 4 * h);
+            u[4 * h] += c4.x; u[4 * h + 1] += c4.y; u[4 * h + 2] += c4.z; u[4 * h + 3] += c4.w;
+          }
+        } else {
+          const uint4 c4 = *(const uint4*)crow;
+          u[0] += bf16_lo(c4.x); u[1] += bf16_hi(c4.x); u[2] += bf16_lo(c4.y); u[3] += bf16_hi(c4.y);
+          u[4] += bf16_lo(c4.z); u[5] += bf16_hi(c4.z); u[6] += bf16_lo(c4.w); u[7] += bf16_hi(c4.w);
+        }
+      }
+      if (bias_n) {
+        const uint4 b4 = __ldg((const uint4*)(bias_n + n));
+        u[0] += bf16_lo(b4.x); u[1] += bf16_hi(b4.x); u[2] += bf16_lo(b4.y); u[3] += bf16_hi(b4.y);
+        u[4] += bf16_lo(b4.z); u[5] += bf16_hi(b4.z); u[6] += bf16_lo(b4.w); u[7] += bf16_hi(b4.w);
+      }
+      if (Z) *(uint4*)(Z + o) = make_uint4(pack_bf16(u[0], u[1]), pack_bf16(u[2], u[3]), pack_bf16(u[4], u[5]), pack_bf16(u[6], u[7]));
+      if (act != FB_ACT_IDENTITY) {
+#pragma unroll
+        for (int e = 0; e < 8; ++e) u[e] = fb_act_apply(act, u[e]);
+      }
+      if (out_f32) {
+        *(float4*)frow = make_float4(u[0], u[1], u[2], u[3]);
+        *(float4*)(frow + 4) = make_float4(u[4], u[5], u[6], u[7]);
+      } else {
+        *(uint4*)crow = make_uint4(pack_bf16(u[0], u[1]), pack_bf16(u[2], u[3]), pack_bf16(u[4], u[5]), pack_bf16(u[6], u[7]));
+      }
+    } else {
+#pragma unroll
+      for (int e = 0; e < 8; ++e) {
+        if (n + e >= N) break;
+        const int64_t o = (int64_t)row * ldc + n + e;
+        float x = u[e];
+        if (accumulate) x += out_f32 ? ((float*)Cv)[o] : bf16_lo((uint32_t)((uint16_t*)Cv)[o]);
+        if (bias_n) x += bf16_lo((uint32_t)bias_n[n + e]);
+        if (Z) Z[o] = (uint16_t)(pack_bf16(x, 0.0f) & 0xffffu);
+        x = fb_act_apply(act, x);
+        if (out_f32) ((float*)Cv)[o] = x;
+        else ((uint16_t*)Cv)[o] = (uint16_t)(pack_bf16(x, 0.0f) & 0xffffu);
+      }
+    }
+  };
+
   if (warp == 0) {
     // ------------------------------------------------------------------ TMA producer ---
     if (lane == 0) {
       int it = 0;   // k-blocks issued so far over all tiles: names the stage and its phase
       bool ok = true;
-      for (int t = cid; t < num_tiles && ok; t += G) {
+      for (int t = tile_beg; t < num_tiles && ok; t += tile_step) {
         const int m0 = tile_m0(t);
         const int nb0 = tile_n0(t) + (PAIR ? cfg::BNC * (int)rank : 0);
         for (int kb = 0; kb < num_kb; ++kb, ++it) {
@@ -163,11 +222,11 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
           ok = mbar_wait_cluster(empty_bar(s), ph ^ 1u, s_abort);
           if (!ok) break;
           // pairs: the leader's barrier counts the bytes of both CTAs' halves; the peer only issues its loads
-          const uint32_t fb = PAIR ? map_to_cta(full_bar(s), 0u) : full_bar(s);
+          const uint32_t fb = PAIR ? map_to_cta(full_bar(s), lead_rank) : full_bar(s);
           if (!PAIR || leader) mbar_arrive_expect_tx(full_bar(s), (uint32_t)((PAIR ? 2 : 1) * (cfg::A_BYTES + cfg::B_BYTES)));
           const uint32_t a_dst = smem_base + (uint32_t)(s * cfg::STAGE_BYTES);
           const uint32_t b_dst = a_dst + (uint32_t)cfg::A_BYTES;
-          const int k0 = kb * HBK;
+          const int k0 = (kb0 + kb) * HBK;
           auto load2 = [&](uint32_t dst, const CUtensorMap* map, int x, int y) {
             if (PAIR) tma_load_2d_pair(dst, map, x, y, fb);
             else tma_load_2d(dst, map, x, y, fb);
@@ -207,7 +266,7 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
                              ((uint32_t)(BN >> 3) << 17) | ((uint32_t)((PAIR ? 256 : HBM_) >> 4) << 24);
       bool ok = true;
       int it = 0, tc = 0;   // k-blocks and tiles issued so far
-      for (int t = cid; t < num_tiles && ok; t += G, ++tc) {
+      for (int t = tile_beg; t < num_tiles && ok; t += tile_step, ++tc) {
         const int buf = tc & 1, use = tc >> 1;
         if (use > 0) {
           // the epilogue warps must have drained this accumulator buffer's previous tile
@@ -238,8 +297,8 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
           }
           const bool last = (kb == num_kb - 1);
           if (PAIR) {
-            tc_commit2_mc(empty_bar(s), (uint16_t)3);                 // frees the stage in both CTAs
-            if (last) tc_commit2_mc(tmem_full_bar(buf), (uint16_t)3);
+            tc_commit2_mc(empty_bar(s), (uint16_t)(3u << lead_rank));                 // frees the stage in both CTAs
+            if (last) tc_commit2_mc(tmem_full_bar(buf), (uint16_t)(3u << lead_rank));
           } else {
             tc_commit(empty_bar(s));
             if (last) tc_commit(tmem_full_bar(buf));
@@ -252,7 +311,7 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
     const int q = warp & 3;                 // TMEM lane quadrant this warp may read
     bool ok = true;
     int tc = 0;
-    for (int t = cid; t < num_tiles && ok; t += G, ++tc) {
+    for (int t = tile_beg; t < num_tiles && ok; t += tile_step, ++tc) {
       const int buf = tc & 1, use = tc >> 1;
       const int n0 = tile_n0(t);
       const int row = tile_m0(t) + 32 * q + lane;
@@ -267,68 +326,60 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
         tc_ld_32x32b_x32(tmem_base + ((uint32_t)(32 * q) << 16) + (uint32_t)(buf * BN + cc * 32), r);
         tc_wait_ld();
         float* v = reinterpret_cast<float*>(r);
-        if (row < M) {
-          const bool full = (nb + 31 < N);
-          if (out_f32) {
-            float* crow = (float*)Cv + (int64_t)row * ldc + nb;
-            for (int e = 0; e < 32 && nb + e < N; ++e) {
-              float x = v[e];
-              if (accumulate) x += crow[e];
-              if (bias_n) x += bf16_lo((uint32_t)bias_n[nb + e]);
-              if (Z) Z[(int64_t)row * ldc + nb + e] = (uint16_t)(pack_bf16(x, 0.0f) & 0xffffu);
-              crow[e] = fb_act_apply(act, x);
-            }
-          } else if (full) {
-            uint16_t* crow = (uint16_t*)Cv + (int64_t)row * ldc + nb;
-            uint16_t* zrow = Z ? Z + (int64_t)row * ldc + nb : nullptr;
+        if (ksplit > 1) {   // all MMAs have read their stages: the sums go where the cluster can add them up
+          float4* d4 = (float4*)((float*)smem + (32 * q + lane) * (BN + 4) + cc * 32);
 #pragma unroll
-            for (int j = 0; j < 4; ++j) {       // 8 columns = one 16-byte store
-              float u[8];
+          for (int j = 0; j < 8; ++j) d4[j] = make_float4(v[4 * j], v[4 * j + 1], v[4 * j + 2], v[4 * j + 3]);
+        } else {
 #pragma unroll
-              for (int e = 0; e < 8; ++e) u[e] = v[8 * j + e];
-              if (accumulate) {
-                const uint4 c4 = *(const uint4*)(crow + 8 * j);
-                u[0] += bf16_lo(c4.x); u[1] += bf16_hi(c4.x); u[2] += bf16_lo(c4.y); u[3] += bf16_hi(c4.y);
-                u[4] += bf16_lo(c4.z); u[5] += bf16_hi(c4.z); u[6] += bf16_lo(c4.w); u[7] += bf16_hi(c4.w);
-              }
-              if (bias_n) {
-                const uint4 b4 = __ldg((const uint4*)(bias_n + nb + 8 * j));
-                u[0] += bf16_lo(b4.x); u[1] += bf16_hi(b4.x); u[2] += bf16_lo(b4.y); u[3] += bf16_hi(b4.y);
-                u[4] += bf16_lo(b4.z); u[5] += bf16_hi(b4.z); u[6] += bf16_lo(b4.w); u[7] += bf16_hi(b4.w);
-              }
-              if (zrow) *(uint4*)(zrow + 8 * j) = make_uint4(pack_bf16(u[0], u[1]), pack_bf16(u[2], u[3]), pack_bf16(u[4], u[5]), pack_bf16(u[6], u[7]));
-              if (act != FB_ACT_IDENTITY) {
-#pragma unroll
-                for (int e = 0; e < 8; ++e) u[e] = fb_act_apply(act, u[e]);
-              }
-              *(uint4*)(crow + 8 * j) = make_uint4(pack_bf16(u[0], u[1]), pack_bf16(u[2], u[3]), pack_bf16(u[4], u[5]), pack_bf16(u[6], u[7]));
-            }
-          } else {
-            uint16_t* crow = (uint16_t*)Cv + (int64_t)row * ldc + nb;
-            for (int e = 0; e < 32 && nb + e < N; ++e) {
-              float x = v[e];
-              if (accumulate) x += bf16_lo((uint32_t)crow[e]);
-              if (bias_n) x += bf16_lo((uint32_t)bias_n[nb + e]);
-              if (Z) Z[(int64_t)row * ldc + nb + e] = (uint16_t)(pack_bf16(x, 0.0f) & 0xffffu);
-              crow[e] = (uint16_t)(pack_bf16(fb_act_apply(act, x), 0.0f) & 0xffffu);
-            }
-          }
+          for (int j = 0; j < 4; ++j) emit8(row, v + 8 * j, nb + 8 * j);
         }
       }
       // this buffer may be overwritten once every epilogue warp (of both CTAs) has read its quadrant
       tc_fence_before();
       __syncwarp();
       if (lane == 0) {
-        if (PAIR) mbar_arrive_cluster(map_to_cta(tmem_empty_bar(buf), 0u));
+        if (PAIR) mbar_arrive_cluster(map_to_cta(tmem_empty_bar(buf), lead_rank));
         else mbar_arrive(tmem_empty_bar(buf));
       }
+    }
+  }
+
+  // ---------------------------------------------- split K: the cluster adds up its parts ---
+  if (ksplit > 1) {
+    __syncwarp();
+    cluster_sync_all();
+    const int rows = HBM_ / ksplit, m0 = tile_m0(tile_beg), n0 = tile_n0(tile_beg);
+    for (int e = threadIdx.x; e < rows * (BN / 8); e += cfg::NUM_THREADS) {
+      const int r = part * rows + e / (BN / 8), c = 8 * (e % (BN / 8));
+      if (m0 + r >= M || n0 + c >= N) continue;
+      const uint32_t src = smem_base + (uint32_t)((r * (BN + 4) + c) * 4);
+      float4 x[8][2];
+#pragma unroll
+      for (int i = 0; i < 8; ++i)
+        if (i < ksplit) {
+          const uint32_t a = map_to_cta(src, (uint32_t)i * (PAIR ? 2u : 1u) + rank);
+#pragma unroll
+          for (int h = 0; h < 2; ++h)
+            asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];"
+                         : "=f"(x[i][h].x), "=f"(x[i][h].y), "=f"(x[i][h].z), "=f"(x[i][h].w) : "r"(a + 16u * (uint32_t)h) : "memory");
+        }
+      float v[8];
+#pragma unroll
+      for (int h = 0; h < 2; ++h) { v[4 * h] = x[0][h].x; v[4 * h + 1] = x[0][h].y; v[4 * h + 2] = x[0][h].z; v[4 * h + 3] = x[0][h].w; }
+#pragma unroll
+      for (int i = 1; i < 8; ++i)
+        if (i < ksplit)
+#pragma unroll
+          for (int h = 0; h < 2; ++h) { v[4 * h] += x[i][h].x; v[4 * h + 1] += x[i][h].y; v[4 * h + 2] += x[i][h].z; v[4 * h + 3] += x[i][h].w; }
+      emit8(m0 + r, v, n0 + c);
     }
   }
 
   // ---------------------------------------------------------------------- teardown ---
   tc_fence_before();
   __syncthreads();
-  if (PAIR) cluster_sync_all();   // neither CTA may release tensor memory while its peer can still touch it
+  if (PAIR || ksplit > 1) cluster_sync_all();   // no CTA may release its tensor or shared memory while a peer can still touch it
   if (warp == 1) {
     __syncwarp();
     if (PAIR)
@@ -366,7 +417,7 @@ bool encode_map_bf16_mn3d(CUtensorMap* map, const uint16_t* base, int64_t K, int
 }
 
 template <bool A_MN, bool B_MN, int BN, bool PAIR>
-int32_t launch_bf16(fb_ctx* ctx, cudaStream_t stream, const fb_gemm_bf16_args& a) {
+int32_t launch_bf16(fb_ctx* ctx, cudaStream_t stream, const fb_gemm_bf16_args& a, int ksplit) {
   using cfg = HCfg<BN, PAIR>;
   CUtensorMap tmA, tmB;
   bool ok;
@@ -398,7 +449,7 @@ int32_t launch_bf16(fb_ctx* ctx, cudaStream_t stream, const fb_gemm_bf16_args& a
   if (num_tiles > 0x7fffffff) return fb_fail(FB_ERR_UNSUPPORTED, "bf16 gemm: too many tiles");
   const int sms = ctx->sm_count - ctx->reserved_sms;
   const int64_t Gmax = PAIR ? (sms / 2 > 0 ? sms / 2 : 1) : sms;
-  const int64_t G = Gmax < num_tiles ? Gmax : num_tiles;
+  const int64_t G = ksplit > 1 ? num_tiles * ksplit : Gmax < num_tiles ? Gmax : num_tiles;
   cudaLaunchConfig_t lc;
   memset(&lc, 0, sizeof(lc));
   lc.gridDim = dim3((unsigned)(PAIR ? 2 * G : G), 1, 1);
@@ -407,25 +458,25 @@ int32_t launch_bf16(fb_ctx* ctx, cudaStream_t stream, const fb_gemm_bf16_args& a
   lc.stream = stream;
   cudaLaunchAttribute attr[1];
   attr[0].id = cudaLaunchAttributeClusterDimension;
-  attr[0].val.clusterDim.x = PAIR ? 2 : 1;
+  attr[0].val.clusterDim.x = (PAIR ? 2 : 1) * ksplit;
   attr[0].val.clusterDim.y = 1;
   attr[0].val.clusterDim.z = 1;
   lc.attrs = attr;
   lc.numAttrs = 1;
   FB_CUDA(cudaLaunchKernelEx(&lc, kern, tmA, tmB, a.C, a.ldc, a.Z, a.bias_n, (int)a.M, (int)a.N, (int)a.K, a.act, a.accumulate,
-                             a.out_f32, ctx->dev_error, a3d, b3d, (int)num_tiles, tiles_n));
+                             a.out_f32, ctx->dev_error, a3d, b3d, (int)num_tiles, tiles_n, ksplit));
   FB_LAUNCH_CHECK();
   return FB_OK;
 }
 
 template <int BN, bool PAIR>
-int32_t launch_bf16_layout(fb_ctx* ctx, cudaStream_t stream, const fb_gemm_bf16_args& a) {
+int32_t launch_bf16_layout(fb_ctx* ctx, cudaStream_t stream, const fb_gemm_bf16_args& a, int ksplit) {
   if (a.a_mn_major) {
-    if (a.b_mn_major) return launch_bf16<true, true, BN, PAIR>(ctx, stream, a);
-    return launch_bf16<true, false, BN, PAIR>(ctx, stream, a);
+    if (a.b_mn_major) return launch_bf16<true, true, BN, PAIR>(ctx, stream, a, ksplit);
+    return launch_bf16<true, false, BN, PAIR>(ctx, stream, a, ksplit);
   }
-  if (a.b_mn_major) return launch_bf16<false, true, BN, PAIR>(ctx, stream, a);
-  return launch_bf16<false, false, BN, PAIR>(ctx, stream, a);
+  if (a.b_mn_major) return launch_bf16<false, true, BN, PAIR>(ctx, stream, a, ksplit);
+  return launch_bf16<false, false, BN, PAIR>(ctx, stream, a, ksplit);
 }
 
 }  // namespace
@@ -448,8 +499,35 @@ int32_t fb_gemm_bf16_launch(fb_ctx* ctx, cudaStream_t stream, const fb_gemm_bf16
                    "bf16 gemm: needs 16-byte aligned pointers and leading dimensions that are multiples of 8 "
                    "(M=%lld N=%lld K=%lld lda=%lld ldb=%lld ldc=%lld)",
                    (long long)a.M, (long long)a.N, (long long)a.K, (long long)a.lda, (long long)a.ldb, (long long)a.ldc);
-  // two-CTA 256 x 256 tiles once there are enough of them to occupy a good part of the SM pairs
-  const int64_t pair_tiles = ((a.M + 255) / 256) * ((a.N + 255) / 256);
-  if (a.M >= 256 && a.N >= 256 && 4 * pair_tiles >= ctx->sm_count) return launch_bf16_layout<256, true>(ctx, stream, a);
-  return launch_bf16_layout<128, false>(ctx, stream, a);
+  // Tile and K split by the smallest modelled time (us, fitted to measurements on B200): 128 x 128 and 128 x 256 tiles of
+  // one CTA, 256 x 256 tiles of a pair; a k-block of 64 costs 0.33 / 0.38 / 0.36, a tile 0.7 / 2.5 / 3 besides, a launch 5,
+  // a cluster's reduction 3.  Splits run in one wave.  1024 x 1024 x 16384: 95 -> 39 us; 16384 x 1024 x 1024: 42 -> 38 us;
+  // 2048 x 1000 x 4096: 34 -> 25 us; 784 x 512 x 1024: 12.4 -> 11.1 us.
+  static const int bm[3] = {128, 128, 256}, bn[3] = {128, 256, 256};
+  static const double t_kb[3] = {0.33, 0.38, 0.36}, t_tile[3] = {0.7, 2.5, 3.0};
+  const int sms = ctx->sm_count - ctx->reserved_sms;
+  const int num_kb = (int)((a.K + HBK - 1) / HBK);
+  int best_sh = 0, best_s = 1;
+  double best_t = 1e30;
+  for (int sh = 2; sh >= 0; --sh) {
+    if (sh == 2 && (a.M < 256 || a.N < 256)) continue;
+    if (sh == 1 && a.N <= 128) continue;
+    const int ranks = sh == 2 ? 2 : 1;
+    const int64_t tiles = ((a.M + bm[sh] - 1) / bm[sh]) * ((a.N + bn[sh] - 1) / bn[sh]);
+    for (int lg = 0; lg < 4; ++lg) {
+      const int s = 1 << lg;
+      double t;
+      if (s == 1) {
+        const int64_t slots = sms / ranks > 0 ? sms / ranks : 1;
+        t = 5.0 + (double)((tiles + slots - 1) / slots) * (num_kb * t_kb[sh] + t_tile[sh]);
+      } else {
+        if (ctx->reserved_sms != 0 || num_kb < 2 * s || s * ranks > 8 || tiles > fb_gemm_resident_clusters(ctx, s * ranks)) break;
+        t = 8.0 + ((num_kb + s - 1) / s) * t_kb[sh] + t_tile[sh];
+      }
+      if (t < best_t) { best_t = t; best_sh = sh; best_s = s; }
+    }
+  }
+  if (best_sh == 2) return launch_bf16_layout<256, true>(ctx, stream, a, best_s);
+  if (best_sh == 1) return launch_bf16_layout<256, false>(ctx, stream, a, best_s);
+  return launch_bf16_layout<128, false>(ctx, stream, a, best_s);
 }
