@@ -3,7 +3,8 @@
     python flux.jl_b200/build.py [--force] [--verbose]
 
 Each csrc/*.cu is compiled to an object file (in parallel) and linked into
-fluxb200/libfluxb200.so.  The CUDA runtime is linked statically and the driver API is reached
+fluxb200/libfluxb200.so; native Python wrappers of its entry points are generated from the header
+(fluxb200/_fastcall*.so).  The CUDA runtime is linked statically and the driver API is reached
 through cudaGetDriverEntryPoint, so the library also loads on a machine without a GPU driver
 (where every compute entry point reports FB_ERR_CUDA).
 """
@@ -11,9 +12,11 @@ from __future__ import annotations
 
 import concurrent.futures
 import os
+import re
 import shutil
 import subprocess
 import sys
+import sysconfig
 
 HERE = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(HERE, "csrc")
@@ -38,6 +41,65 @@ def _newer(src_paths, target) -> bool:
         return True
     t = os.path.getmtime(target)
     return any(os.path.getmtime(s) > t for s in src_paths)
+
+
+def _fastcall_source(header: str) -> str:
+    """C source of the `_fastcall` extension module: one METH_FASTCALL wrapper per entry point of the header that returns
+    int32 and takes numbers and single pointers only."""
+    text = re.sub(r"/\*.*?\*/", "", open(header).read(), flags=re.S)
+    funcs = []
+    for m in re.finditer(r"\bint32_t\s+(fb_[a-z0-9_]+)\s*\(([^;]*?)\)\s*;", text, flags=re.S):
+        kinds = []
+        for a in m.group(2).split(","):
+            a = " ".join(a.split())
+            stars = a.count("*")
+            base = a.replace("const", "").replace("*", "").split()[0]
+            if a == "void":
+                continue
+            kinds.append("?" if stars > 1 else "p" if stars else {"int32_t": "i", "int64_t": "l", "uint64_t": "u", "float": "f"}.get(base, "?"))
+        if kinds and "?" not in kinds:
+            funcs.append((m.group(1), kinds))
+    ctype = {"p": "void*", "i": "int32_t", "l": "int64_t", "u": "uint64_t", "f": "float"}
+    out = [open(os.path.join(HERE, "csrc", "fastcall_head.h")).read()]
+    for i, (name, kinds) in enumerate(funcs):
+        decl = " ".join(f"{ctype[k]} a{j};" for j, k in enumerate(kinds))
+        test = " || ".join(f"!get_{k}(a[{j}], &a{j})" for j, k in enumerate(kinds))
+        out.append(f"""
+static void* fp_{name};
+static PyObject* w_{name}(PyObject* self, PyObject* const* a, Py_ssize_t n) {{
+  (void)self;
+  {decl}
+  if (fp_{name} == NULL || n != {len(kinds)} || {test}) Py_RETURN_NONE;
+  int32_t r;
+  Py_BEGIN_ALLOW_THREADS
+  r = ((int32_t (*)({", ".join(ctype[k] for k in kinds)}))fp_{name})({", ".join(f"a{j}" for j in range(len(kinds)))});
+  Py_END_ALLOW_THREADS
+  return PyLong_FromLong(r);
+}}
+""")
+    out.append("static const struct { const char* name; void** slot; } slots[] = {\n")
+    out += [f'  {{"{n}", &fp_{n}}},\n' for n, _ in funcs]
+    out.append("  {NULL, NULL}};\nFASTCALL_BIND_AND_NAMES\nstatic PyMethodDef methods[] = {\n")
+    out += [f'  {{"{n}", (PyCFunction)(void (*)(void))w_{n}, METH_FASTCALL, NULL}},\n' for n, _ in funcs]
+    out.append('  {"bind", do_bind, METH_VARARGS, NULL},\n  {"names", do_names, METH_NOARGS, NULL},\n  {NULL, NULL, 0, NULL}};\nFASTCALL_MODULE\n')
+    return "".join(out)
+
+
+def build_fastcall(force: bool = False) -> str:
+    """The native call wrappers, generated from the header and compiled with the host compiler."""
+    header = os.path.join(HERE, "..", "include", "fluxb200.h")
+    head = os.path.join(HERE, "csrc", "fastcall_head.h")
+    out = os.path.join(HERE, "fluxb200", "_fastcall" + sysconfig.get_config_var("EXT_SUFFIX"))
+    if force or _newer([header, head, os.path.abspath(__file__)], out):
+        src = os.path.join(OBJ, "fastcall.c")
+        with open(src, "w") as f:
+            f.write(_fastcall_source(header))
+        cmd = [os.environ.get("CC") or "gcc", "-O2", "-shared", "-fPIC", "-I", sysconfig.get_paths()["include"], src, "-o", out]
+        r = subprocess.run(cmd, capture_output=True, text=True)
+        if r.returncode != 0:
+            print(r.stdout + r.stderr)
+            raise RuntimeError("building the native call wrappers failed")
+    return out
 
 
 def build(force: bool = False, verbose: bool = False) -> str:
@@ -76,6 +138,7 @@ def build(force: bool = False, verbose: bool = False) -> str:
         if r.returncode != 0:
             print(r.stdout + r.stderr)
             raise RuntimeError("link failed")
+    build_fastcall(force)
     return OUT
 
 

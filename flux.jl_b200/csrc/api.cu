@@ -62,11 +62,20 @@ FB_API int32_t fb_ctx_create(int32_t device, fb_ctx** out) {
     return fb_fail(FB_ERR_ALLOC, "fb_ctx_create: cudaMalloc failed: %s", cudaGetErrorString(e));
   }
   cudaMemset(c->dev_error, 0, 256);
+  c->host_seq = 0;
+  if (cudaHostAlloc((void**)&c->host_page, 64, cudaHostAllocMapped | cudaHostAllocPortable) != cudaSuccess) {
+    cudaGetLastError();
+    cudaFree(c->dev_error);
+    delete c;
+    return fb_fail(FB_ERR_ALLOC, "fb_ctx_create: cudaHostAlloc failed");
+  }
+  memset((void*)c->host_page, 0, 64);
   int32_t ws_status = fb_side_kernels_prepare_elementwise();
   if (ws_status == FB_OK) ws_status = fb_side_kernels_prepare_peer();
   if (ws_status == FB_OK) ws_status = fb_gemm_workspace_create(c);
   if (ws_status != FB_OK) {
     cudaFree(c->dev_error);
+    cudaFreeHost((void*)c->host_page);
     delete c;
     return ws_status;
   }
@@ -90,6 +99,7 @@ FB_API int32_t fb_ctx_destroy(fb_ctx* ctx) {
   if (ctx->pack) cudaFree(ctx->pack);
   for (int i = 0; i < ctx->retired_count; ++i) cudaFree(ctx->retired[i]);
   if (ctx->dev_error) cudaFree(ctx->dev_error);
+  cudaFreeHost((void*)ctx->host_page);
   fb_gemm_workspace_destroy(ctx);
   delete ctx;
   return FB_OK;
@@ -201,6 +211,38 @@ FB_API int32_t fb_device_error(fb_ctx* ctx, void* stream, int32_t* out_host) {
     fb_gemm_workspace_reset(ctx, (cudaStream_t)stream);
     FB_CUDA(cudaMemsetAsync(ctx->dev_error, 0, sizeof(int32_t), (cudaStream_t)stream));
   }
+  return FB_OK;
+}
+
+// host page: [0] value bits, [1] error word, [2] sequence number
+__global__ void read_scalar_kernel(const float* x, const int32_t* dev_err, volatile uint32_t* page, uint32_t seq) {
+  page[0] = __float_as_uint(*x);
+  page[1] = (uint32_t)*(const volatile int32_t*)dev_err;
+  __threadfence_system();
+  page[2] = seq;
+}
+
+FB_API int32_t fb_read_scalar(fb_ctx* ctx, void* stream_, const float* x, float* value_host, int32_t* error_host) {
+  FB_CHECK_CTX(ctx);
+  FB_REQUIRE(x && value_host && error_host, FB_ERR_INVALID_ARG, "fb_read_scalar: NULL pointer");
+  cudaStream_t stream = (cudaStream_t)stream_;
+  volatile uint32_t* page = ctx->host_page;
+  const uint32_t seq = ++ctx->host_seq;
+  read_scalar_kernel<<<1, 1, 0, stream>>>(x, ctx->dev_error, page, seq);
+  FB_LAUNCH_CHECK();
+  for (uint32_t spin = 0; page[2] != seq; ++spin) {
+    if ((spin & 4095u) != 4095u) continue;
+    // the stream's state is looked at now and then: it has either not come this far, or failed, or the page is current
+    const cudaError_t e = cudaStreamQuery(stream);
+    if (e == cudaErrorNotReady) continue;
+    if (e != cudaSuccess) return fb_fail(FB_ERR_CUDA, "fb_read_scalar: %s", cudaGetErrorString(e));
+    if (page[2] != seq) FB_CUDA(cudaStreamSynchronize(stream));
+    break;
+  }
+  __sync_synchronize();
+  const uint32_t bits = page[0];
+  memcpy(value_host, &bits, 4);
+  *error_host = (int32_t)page[1];
   return FB_OK;
 }
 

@@ -25,6 +25,8 @@ struct fb_ctx {
   void* retired[FB_MAX_RETIRED];   // outgrown arena blocks, released with the context
   int retired_count;
   int32_t* dev_error;    // device error word written by kernels whose bounded waits ran out
+  uint32_t* host_page;   // pinned page that fb_read_scalar's kernel writes
+  uint32_t host_seq;
   void* gemm_ws;      // opaque (gemm_tc.cu): workspace of the split-tile GEMM schedule
 };
 

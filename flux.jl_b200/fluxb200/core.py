@@ -11,6 +11,7 @@ the data is in libfluxb200.so.
 from __future__ import annotations
 
 import ctypes as C
+import math
 import threading
 
 import numpy as np
@@ -19,6 +20,8 @@ import torch
 from . import lib
 
 _state = threading.local()
+_raw_stream = torch._C._cuda_getCurrentRawStream if hasattr(torch._C, "_cuda_getCurrentRawStream") else (
+    lambda device: torch.cuda.current_stream(device).cuda_stream)
 
 
 class Context:
@@ -31,11 +34,20 @@ class Context:
         torch.cuda.set_device(device)
         h = C.c_void_p()
         lib.call("fb_ctx_create", device, C.byref(h))
-        self.handle = h
+        self.handle = h.value
+        self.torch_device = torch.device("cuda", device)
+        self._out, self._err = C.c_float(0.0), C.c_int32(0)
+        self._out_ptr, self._err_ptr = C.addressof(self._out), C.addressof(self._err)
 
     @property
     def stream(self):
-        return C.c_void_p(torch.cuda.current_stream(self.device).cuda_stream)
+        return _raw_stream(self.device)
+
+    def read_scalar(self, a: "B200Array"):
+        """(value of a one-element Float32 array, device error word) once the current stream has reached this point.
+        The error word is not cleared."""
+        lib.call("fb_read_scalar", self.handle, _raw_stream(self.device), a.t.data_ptr(), self._out_ptr, self._err_ptr)
+        return self._out.value, self._err.value
 
     def set_reserved_sms(self, n: int):
         """SMs the persistent GEMM leaves free for communication kernels that run beside it (0 = none)."""
@@ -74,7 +86,7 @@ class B200Array:
 
     @property
     def ptr(self):
-        return C.c_void_p(self.t.data_ptr())
+        return self.t.data_ptr()
 
     @property
     def ndim(self):
@@ -102,14 +114,23 @@ class B200Array:
         return f"B200Array{self.size}"
 
 
+def _wrap(t: torch.Tensor, size: tuple) -> B200Array:
+    """B200Array over a tensor that is known to fit (no checks: this runs several times per layer call)."""
+    a = B200Array.__new__(B200Array)
+    a.t = t
+    a.size = size
+    a._node = None
+    return a
+
+
 def empty(size, dtype=torch.float32) -> B200Array:
-    n = int(np.prod(size, dtype=np.int64)) if len(size) else 1
-    return B200Array(torch.empty(n, dtype=dtype, device=f"cuda:{context().device}"), size)
+    size = tuple(map(int, size))
+    return _wrap(torch.empty(math.prod(size), dtype=dtype, device=context().torch_device), size)
 
 
 def zeros(size, dtype=torch.float32) -> B200Array:
-    n = int(np.prod(size, dtype=np.int64)) if len(size) else 1
-    return B200Array(torch.zeros(n, dtype=dtype, device=f"cuda:{context().device}"), size)
+    size = tuple(map(int, size))
+    return _wrap(torch.zeros(math.prod(size), dtype=dtype, device=context().torch_device), size)
 
 
 def gpu(x):
@@ -222,6 +243,8 @@ def accumulate(grads: dict, keep: dict, arr: B200Array, g: B200Array):
     if k in grads:
         if grads[k].t.data_ptr() != g.t.data_ptr():
             ctx = context()
+            if getattr(grads[k], "_is_one", False):   # the shared constant 1 is never written
+                grads[k] = _wrap(grads[k].t.clone(), grads[k].size)
             if grads[k].t.dtype == torch.bfloat16:
                 g = to_bf16(g)
                 lib.call("fb_axpy_bf16", ctx.handle, ctx.stream, 1.0, g.ptr, grads[k].ptr, g.numel())

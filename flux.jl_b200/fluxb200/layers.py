@@ -8,6 +8,8 @@ LSTMCell :383-419, GRUCell :586-628, LSTM :491-524, GRU :685-718), attention.jl 
 """
 from __future__ import annotations
 
+import math
+
 import numpy as np
 import torch
 
@@ -310,7 +312,7 @@ class LayerNorm(Layer):
             _wait_params(self.diag.scale, self.diag.bias)
             for d, s in enumerate(self.size):
                 _size_check(self, x, d + 1, s)
-        d = int(np.prod(self.size))
+        d = math.prod(self.size)
         if x.numel() % d != 0 or x.size[:len(self.size)] != self.size:
             raise DimensionMismatch(f"layer {self} expects leading dims {self.size}, got {x}")
         n = x.numel() // d
@@ -371,7 +373,7 @@ class BatchNorm(Layer):
             raise DimensionMismatch(f"layer {self} expects ndims(input) >= 2, but got {x}")
         _size_check(self, x, N - 1, self.chs)
         training = self._isactive()
-        s = int(np.prod(x.size[:N - 2], dtype=np.int64)) if N > 2 else 1
+        s = math.prod(x.size[:N - 2])
         c, n = self.chs, x.size[-1]
         if training and s * n == 1:
             raise ArgumentError(
@@ -764,7 +766,7 @@ class GroupNorm(Layer):
         if N < 2:
             raise DimensionMismatch(f"layer {self} expects ndims(input) >= 2, but got {x}")
         _size_check(self, x, N - 1, self.chs)
-        s = int(np.prod(x.size[:N - 2], dtype=np.int64)) if N > 2 else 1
+        s = math.prod(x.size[:N - 2])
         c, n, G = self.chs, x.size[-1], self._groups()
         ctx = context()
         act = lib.ACT[self.λ]
@@ -815,7 +817,7 @@ class InstanceNorm(GroupNorm):
         if self.track_stats and not self._isactive():
             N = x.ndim
             _size_check(self, x, N - 1, self.chs)
-            s = int(np.prod(x.size[:N - 2], dtype=np.int64)) if N > 2 else 1
+            s = math.prod(x.size[:N - 2])
             ctx = context()
             y = empty(x.size)
             lib.call("fb_batchnorm_fwd_infer", ctx.handle, ctx.stream, x.ptr, _ptr(self.γ), _ptr(self.β), self.μ.ptr, self.σ2.ptr,

@@ -54,6 +54,7 @@ PROTOTYPES = {
     "fb_memset": (_i32, [_p, _p, _p, _i32, _i64]),
     "fb_sync": (_i32, [_p, _p]),
     "fb_device_error": (_i32, [_p, _p, C.POINTER(_i32)]),
+    "fb_read_scalar": (_i32, [_p, _p, _p, _p, _p]),
     "fb_selftest_bounded_wait": (_i32, [_p, _p, _i32]),
     "fb_gemm_f32": (_i32, [_p, _p, _i32, _i32, _i64, _i64, _i64, _p, _i64, _p, _i64, _p, _i64, _i32, _i32]),
     "fb_dense_fwd": (_i32, [_p, _p, _i32, _i32, _p, _p, _p, _p, _p, _i64, _i64, _i64]),
@@ -142,6 +143,21 @@ for _name, (_res, _args) in PROTOTYPES.items():
     _fn.argtypes = _args
 
 
+# Entry points whose arguments are plain numbers and pointers also have a native wrapper (built beside the library from
+# its header): a call through ctypes converts every argument through a Python-level type object, about 3 us at 15
+# arguments against 0.3.  A wrapper answers None for arguments it does not take (ctypes arrays, byref objects).
+_fast = {}
+try:
+    from . import _fastcall
+except ImportError:
+    _fastcall = None
+if _fastcall is not None:
+    for _name in _fastcall.names():
+        if _name in PROTOTYPES:
+            _fast[_name] = getattr(_fastcall, _name)
+            _fastcall.bind(_name, C.cast(getattr(_lib, _name), C.c_void_p).value)
+
+
 def raw():
     """The ctypes handle (tests call entry points directly through it)."""
     return _lib
@@ -162,7 +178,15 @@ PROFILE = None   # optional {"names": set, "events": list}: CUDA events recorded
 def call(name: str, *args):
     """Calls an int32-status entry point and raises FluxB200Error on failure."""
     prof = PROFILE
-    if prof is not None and name in prof["names"]:
+    if prof is None:
+        f = _fast.get(name)
+        if f is not None:
+            status = f(*args)
+            if status == 0:
+                return
+            if status is not None:
+                check(status)
+    elif name in prof["names"]:
         import torch
         e0, e1 = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
         e0.record()

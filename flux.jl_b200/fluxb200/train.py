@@ -184,7 +184,7 @@ def _withgradient_device(f, model, grad_sink=None):
             grad_sink.expect_uses(counts)
         grads: dict = {}
         keep: dict = {}
-        grads[id(loss)] = _One(B200Array(torch.ones(1, device=loss.t.device), ()))
+        grads[id(loss)] = _one(loss.t.device)
         keep[id(loss)] = loss
         # gradient averaging runs beside the reverse sweep: leave it the SMs it needs
         reserve = int(getattr(grad_sink, "reserved_sms", 0) or 0)
@@ -217,11 +217,17 @@ def withgradient(f, model, grad_sink=None):
     auxiliary-output form).  The loss value comes back as a Python float (one device -> host read,
     the same sync `_eager_step!` pays at src/train.jl:377).
     """
+    return _withgradient(f, model, grad_sink)[0]
+
+
+def _withgradient(f, model, grad_sink=None):
+    """withgradient's result and the device error word, which is read together with the loss."""
     loss, aux, tree = _withgradient_device(f, model, grad_sink)
-    val = float(loss.t.item())
+    loss = to_f32(loss)
+    val, err = context().read_scalar(loss)
     if aux is not None:
-        return (val,) + tuple(aux), (tree,)
-    return val, (tree,)
+        return ((val,) + tuple(aux), (tree,)), err
+    return (val, (tree,)), err
 
 
 class _One(B200Array):
@@ -232,6 +238,20 @@ class _One(B200Array):
     def __init__(self, a: B200Array):
         super().__init__(a.t, a.size)
         self._is_one = True
+
+
+_ones: dict = {}
+
+
+def _one(device) -> _One:
+    """The constant 1 of a device (nothing writes into it)."""
+    o = _ones.get(device)
+    if o is None:
+        if torch.cuda.is_current_stream_capturing():   # memory of a graph's pool is the graph's
+            return _One(B200Array(torch.ones(1, device=device), ()))
+        o = _ones[device] = _One(B200Array(torch.ones(1, device=device), ()))
+        torch.cuda.current_stream(device).synchronize()   # other streams may use it at once
+    return o
 
 
 def gradient(f, model):
@@ -348,12 +368,17 @@ def update(opt_state: OptState, model, grad_tree):
         cnt = (C.c_int64 * k)(*[p.numel() for p in plist])
         lib.call("fb_adam_step", ctx.handle, ctx.stream, k, w, g, m, v, cnt, rule.eta, rule.beta[0], rule.beta[1],
                  rule.epsilon, b1t, b2t, 1.0)
-        f32 = np.float32
-        nb = (float(f32(b1t) * f32(rule.beta[0])), float(f32(b2t) * f32(rule.beta[1])))
+        nb = _advance_powers((b1t, b2t), rule.beta)
         for p in plist:
             opt_state.leaves[id(p)].state[2] = nb
     _write_back(low, wmap)
     return opt_state, model
+
+
+def _advance_powers(bt, beta):
+    """(β1ᵗ, β2ᵗ) of the next step, in Float32 as the rule's state keeps them."""
+    f32 = np.float32
+    return (float(f32(bt[0]) * f32(beta[0])), float(f32(bt[1]) * f32(beta[1])))
 
 
 def _write_back(low, wmap):
@@ -373,14 +398,15 @@ def trainstep(loss, model, batch, opt_state):
         outer.check_async_error()
     if sink is not None:
         sink.begin_step()
-    l, gs = withgradient(lambda m: loss(m, *batch), model, grad_sink=sink)
+    (l, gs), err = _withgradient(lambda m: loss(m, *batch), model, grad_sink=sink)
     lv = l[0] if isinstance(l, tuple) else l
     finite = outer.all_finite(lv) if isinstance(outer, DistributedOptimizerBase) else math.isfinite(lv)
     if finite:
         update(opt_state, model, gs[0])
     elif sink is not None:
         sink.finish()   # the collectives already started must be matched on every worker
-    _raise_on_device_error()
+    if err != 0 or isinstance(outer, DistributedOptimizerBase):   # the update alone contains no bounded wait
+        _raise_on_device_error()
     return l
 
 
@@ -458,8 +484,6 @@ class GraphedTrainStep:
     `step(*batch)` accepts B200 arrays / OneHotLabels, or pinned host tensors of the same sizes (copied into the
     step's static input buffers on the current stream).
     """
-
-    error_poll_every = 16   # the device error word is read back every this many steps (one 4-byte copy)
 
     def __init__(self, loss, model, opt_state, example_batch, grad_sink=None, shard_optimizer=False, defer_gather=False):
         from .layers import BatchNorm, _walk
@@ -593,15 +617,17 @@ class GraphedTrainStep:
         self.graph.replay()
         if prefetch is not None:
             self.prefetch(*prefetch)
-        lv = float(self.loss_arr.t.item())
-        gv = lv if self.guard_arr is self.loss_arr else float(self.guard_arr.t.item())
-        self._calls = getattr(self, "_calls", 0) + 1
-        if self._calls % self.error_poll_every == 0:
+        ctx = context()
+        lv, err = ctx.read_scalar(self.loss_arr)
+        gv = lv if self.guard_arr is self.loss_arr else ctx.read_scalar(self.guard_arr)[0]
+        if err != 0:
             _raise_on_device_error()
         if math.isfinite(gv):
-            rule = self.opt_state.rule
-            f32 = np.float32
+            beta, last, nxt = self.opt_state.rule.beta, None, None
             for p in self._updated:
                 st = self.opt_state.leaves[id(p)].state
-                st[2] = (float(f32(st[2][0]) * f32(rule.beta[0])), float(f32(st[2][1]) * f32(rule.beta[1])))
+                if st[2] != last:     # the leaves share their step count
+                    last = st[2]
+                    nxt = _advance_powers(last, beta)
+                st[2] = nxt
         return lv

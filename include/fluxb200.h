@@ -99,6 +99,12 @@ int32_t fb_sync(fb_ctx* ctx, void* stream);
  * tensor-core kernels return without computing.  Reading it synchronises the stream and clears it. */
 int32_t fb_device_error(fb_ctx* ctx, void* stream, int32_t* out_host);
 
+/* Reads one device Float32 (a loss) together with the device error word: a one-thread kernel on `stream` stores both in
+ * a host page that this call watches, which is several us quicker than a copy and a stream synchronisation each.
+ * Returns when the stream has reached this point.  The error word is left as it is (fb_device_error clears it).  Not
+ * for a stream that is being captured.  Replaces the implicit device-to-host read of a loss (src/train.jl:377). */
+int32_t fb_read_scalar(fb_ctx* ctx, void* stream, const float* x, float* value_host, int32_t* error_host);
+
 /* Launches a one-block kernel whose only act is a bounded wait (at most `polls` <= 4096 polls) on a barrier
  * that nothing signals: the wait runs out, code 9001 lands in the device error word, the kernel returns.  It lets
  * a caller exercise its handling of that word (report, clear, carry on) without any real kernel misbehaving.

@@ -504,3 +504,28 @@ def test_multiheadattention_bias_dropout_and_loss_on_the_weights(F):
     assert np.abs(y1 - y0).max() > 1e-3 and np.abs(y1 - y2).max() > 1e-3
     _, al = md(xg)
     assert 0.3 < (F.cpu(al.materialize()) == 0).mean() < 0.7
+
+
+def test_read_scalar_sees_the_stream_and_the_error_word():
+    """fb_read_scalar returns the value the stream has at that point, call after call, and leaves the error word set."""
+    import ctypes as C
+    import fluxb200 as F
+    from fluxb200 import lib
+    ctx = F.context()
+    x = F.zeros((1,))
+    for i in range(50):
+        lib.call("fb_fill", ctx.handle, ctx.stream, x.ptr, float(i), 1)
+        assert ctx.read_scalar(x) == (float(i), 0)
+    lib.call("fb_selftest_bounded_wait", ctx.handle, ctx.stream, 16)
+    assert ctx.read_scalar(x)[1] == 9001 and ctx.read_scalar(x)[1] == 9001
+    assert ctx.device_error() == 9001 and ctx.read_scalar(x)[1] == 0
+    # the constant cotangent of the loss is shared and must not change when a loss receives a second contribution
+    d = F.Dense(np.ones((1, 1), np.float32), False)
+    xg = F.gpu(np.full((1, 1), 3.0, np.float32))
+
+    def f(m):
+        a = F.sum_all(m(xg))
+        return F.add(a, F.scale(2.0, a))
+    for _ in range(2):
+        v, (g,) = F.withgradient(f, d)
+        assert v == 9.0 and float(F.cpu(g["weight"])[0, 0]) == 9.0
