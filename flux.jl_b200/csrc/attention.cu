@@ -504,7 +504,7 @@ FB_API int32_t fb_attn_fwd_ex(fb_ctx* ctx, void* stream_, const float* q, const 
   if (st != FB_OK) return st;
   if (lq == 0 || batch == 0) return FB_OK;
   FB_REQUIRE(q && k && v && o && lse, FB_ERR_INVALID_ARG, "fb_attn_fwd: NULL pointer");
-  // head size 64 without an explicit mask, bias or dropout runs on the tensor cores
+  // head sizes up to 64 without an explicit mask, bias or dropout run on the tensor cores
   st = attn_has_extras(D) ? FB_ERR_UNSUPPORTED
                           : fb_attn_fwd_tc(ctx, stream, q, k, v, mask, o, lse, e_dim, ev_dim, lq, lk, batch, nheads, causal);
   if (st != FB_ERR_UNSUPPORTED) return st;
@@ -546,6 +546,13 @@ FB_API int32_t fb_attn_bwd_ex(fb_ctx* ctx, void* stream_, const float* q, const 
   if (batch == 0) return FB_OK;
   FB_REQUIRE(lq >= 1 && lk >= 1, FB_ERR_SHAPE, "fb_attn_bwd: empty sequence");
   FB_REQUIRE(q && k && v && o && lse && dout && dq && dk && dv, FB_ERR_INVALID_ARG, "fb_attn_bwd: NULL pointer");
+  // without extras, head size 64 and at most 2048 queries (dK, dV) and keys (dQ): the tensor cores
+  bool did_kv = false, did_q = false;
+  if (!attn_has_extras(D)) {
+    st = fb_attn_bwd_tc(ctx, stream, q, k, v, mask, o, lse, dout, dq, dk, dv, e_dim, ev_dim, lq, lk, batch, nheads, causal, &did_kv, &did_q);
+    if (st != FB_OK && st != FB_ERR_UNSUPPORTED) return st;
+    if (did_kv && did_q) return FB_OK;
+  }
   float* dlt = (float*)fb_scratch(ctx, stream, (size_t)(batch * nheads * lq) * sizeof(float));
   if (!dlt) return FB_ERR_ALLOC;
   const int64_t warps = batch * lq * nheads;
@@ -568,7 +575,6 @@ FB_API int32_t fb_attn_bwd_ex(fb_ctx* ctx, void* stream_, const float* q, const 
     }
     FB_LAUNCH_CHECK();
   }
-  const bool extras = attn_has_extras(D);
   const size_t smem_kv = (size_t)(4 * TS * ld + 2 * TS * PLD) * sizeof(float);
   const size_t smem_q = (size_t)(4 * TS * ld + TS * PLD) * sizeof(float);
   dim3 grid_kv((unsigned)((lk + TS - 1) / TS), (unsigned)nheads, (unsigned)batch);
@@ -576,19 +582,11 @@ FB_API int32_t fb_attn_bwd_ex(fb_ctx* ctx, void* stream_, const float* q, const 
   if (nc == 1) {
     FB_CUDA(cudaFuncSetAttribute(attn_bwd_dkdv_kernel<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_kv));
     FB_CUDA(cudaFuncSetAttribute(attn_bwd_dq_kernel<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_q));
-    // dK / dV on the tensor cores where the shape allows (head size 64, no explicit mask, at most 2048 queries)
-    st = extras ? FB_ERR_UNSUPPORTED
-                : fb_attn_bwd_dkdv_tc(ctx, stream, q, k, v, mask, lse, dlt, dout, dk, dv, e_dim, ev_dim, lq, lk, batch, nheads, causal);
-    if (st == FB_ERR_UNSUPPORTED) {
+    if (!did_kv) {
       attn_bwd_dkdv_kernel<1><<<grid_kv, AT, smem_kv, stream>>>(q, k, v, mask, lse, dlt, dout, dk, dv, D);
       FB_LAUNCH_CHECK();
-    } else if (st != FB_OK) {
-      return st;
     }
-    // dQ on the tensor cores where the shape allows (head size 64, no explicit mask, at most 2048 keys)
-    st = extras ? FB_ERR_UNSUPPORTED
-                : fb_attn_bwd_dq_tc(ctx, stream, q, k, v, mask, lse, dlt, dout, dq, e_dim, ev_dim, lq, lk, batch, nheads, causal);
-    if (st != FB_ERR_UNSUPPORTED) return st;
+    if (did_q) return FB_OK;
     attn_bwd_dq_kernel<1><<<grid_q, AT, smem_q, stream>>>(q, k, v, mask, lse, dlt, dout, dq, D);
   } else {
     FB_CUDA(cudaFuncSetAttribute(attn_bwd_dkdv_kernel<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_kv));

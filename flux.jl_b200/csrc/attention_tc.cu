@@ -1,22 +1,27 @@
-// Flash-style attention forward on the tensor cores for Float32 data (head size 64): S = Q K' and O += P V are
-// tcgen05 TF32 MMAs with the error-compensated 3-pass split (hi / lo operands), the online softmax runs on the
-// accumulator read back from tensor memory, and no L x L array ever exists in HBM.
+// Flash-style attention on the tensor cores (tcgen05), forward and backward, for head sizes up to 64.
 //
-// One CTA owns 128 queries of one (batch, head) and walks the keys in blocks of 64:
-//   warp 0      TMA producer: the Q tile once, then a K and a V tile per block (single-buffered; a tile is reloaded
-//               as soon as the MMAs that read it have completed)
-//   warp 1      owns tensor memory (128 columns: S in 0..63, P V in 64..127) and issues the MMAs
-//   warps 2-5   softmax: thread = one query row (its TMEM lane).  Reads S, keeps the running maximum and sum,
-//               writes P (raw value = hi operand, and lo = p - tf32(p)) to shared memory in the K-major 64-byte
-//               swizzled layout the MMA descriptor names, then adds P V (read back from tensor memory) to its
-//               64 output accumulators with round-to-nearest adds
-//   warps 6-9   split warps: write the lo = x - tf32(x) twin of every Q / K / V tile beside the raw tile
+// Float32 operands are cut into three bf16 planes by truncation (8 + 8 + 8 mantissa bits: the split is exact) and a
+// product is the sum of the six plane products that lie above 2^-24 of it, the smallest ones first, accumulated in
+// Float32 in tensor memory.  Compared with a two-plane TF32 split this takes the same tensor time (six bf16 MMAs of
+// K = 16 against three TF32 passes of K = 8), but
+//   - a bf16 tile in the 128-byte swizzle serves as K-major AND as MN-major operand, where TF32 needs the tile twice in
+//     two layouts: a 64 x 64 tile costs 24 KB instead of 64 KB, so that two or three blocks are in flight;
+//   - a small kernel cuts K, V, Q and dO once per call (`attn_split_kernel`) and lays the planes out as the images the
+//     MMAs read from shared memory: tiles arrive by plain bulk copies, and no warp rewrites them there;
+//   - head sizes below 64 are padded with zeros in those images; their zero 16-feature steps are skipped.
+// bf16 operands are one plane, exactly; the probabilities and dS keep three.
 //
-// Shared-memory tiles use the layouts already proven by the GEMM: K-major chunks of 16 floats with the 64-byte
-// swizzle for Q, K and P; the 128-byte swizzle with 32-byte atoms for the MN-major V tile (keys are its K rows).
-// Every mbarrier wait is bounded; when one runs out the kernel records 4001 in the context's device error word,
-// all roles leave their loops, tensor memory is released and the kernel returns.
+// Measured against the TF32 kernels that rewrote their tiles in shared memory (batch 8, 16 heads of 64, 2048 x 2048, causal,
+// Float32): forward 0.65 -> 0.57 ms (of that 0.04 the images), backward 2.45 -> 2.12 ms (0.08).  Errors against float64 at
+// that size: output 1.3e-6 -> 2.3e-7, dQ 5.9e-6 -> 4.8e-6, dK / dV 2.2e-5 -> 1.9e-5.  What bounds them: the tensor core's
+// queue is 61 - 72 % busy (ncu); an MMA with N = 64 takes 44 clocks where its multiplications need 32.
+//
+// A block is 64 keys (64 queries in the dK / dV kernel) against the 128 rows of a CTA; a thread of a compute warp owns
+// one row (one TMEM lane).  Every mbarrier wait is bounded; when one runs out the kernel records 4002 (forward), 4003
+// (dQ) or 4004 (dK / dV) in the context's device error word, all roles leave their loops, tensor memory is released and
+// the kernel returns.
 #include <cuda.h>
+#include <cuda_bf16.h>
 #include <stdlib.h>
 
 #include "common.cuh"
@@ -24,32 +29,59 @@
 
 namespace {
 
-constexpr int QT = 128;   // queries per CTA
-constexpr int KT = 64;    // keys per block
-constexpr int HD = 64;    // head size (q/k features and v features per head)
-constexpr int ATC_THREADS = 320;
+constexpr int QT = 128;        // rows (queries, or keys in the dK / dV kernel) per CTA
+constexpr int KT = 64;         // keys (queries) per block
+constexpr int HD = 64;         // padded head size
+constexpr int TILE = 8192;     // one plane of a 64 x 64 tile: 64 rows of 128 bytes, 128-byte swizzle
+constexpr uint32_t LAYOUT_SW128 = 2;
+constexpr float LOG2E = 1.4426950408889634f;
 
-__device__ __forceinline__ void tc_st_32x32b_x32(uint32_t taddr, const uint32_t* r) {
+struct AtcDims {
+  int64_t E, Ev, Lq, Lk;
+  int H, causal, d, dv;
+  int qtiles, ktiles;   // 64-row tiles per (batch, head) in the plane images (even)
+  int vec;              // rows can be read and written 16 bytes at a time
+  float scale_log2;     // log2(e) / sqrt(d)
+  float scale;          // 1 / sqrt(d)
+};
+
+// --------------------------------------------------------------------------------------------------- wrappers ---
+__device__ __forceinline__ void tc_st_32x32b_x16(uint32_t taddr, const uint32_t* r) {
   asm volatile(
-      "tcgen05.st.sync.aligned.32x32b.x32.b32 [%0], "
-      "{%1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16, "
-      "%17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31, %32};"
+      "tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], "
+      "{%1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16};"
       ::"r"(taddr), "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]), "r"(r[8]), "r"(r[9]),
-      "r"(r[10]), "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15]), "r"(r[16]), "r"(r[17]), "r"(r[18]), "r"(r[19]),
-      "r"(r[20]), "r"(r[21]), "r"(r[22]), "r"(r[23]), "r"(r[24]), "r"(r[25]), "r"(r[26]), "r"(r[27]), "r"(r[28]), "r"(r[29]),
-      "r"(r[30]), "r"(r[31])
+      "r"(r[10]), "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15])
       : "memory");
 }
 __device__ __forceinline__ void tc_wait_st() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
 
-// D[tmem] (+)= A[tmem] * B[smem]: the A tile (128 rows x 8 TF32 values) sits in 8 consecutive TMEM columns
-__device__ __forceinline__ void tc_mma_tf32_ta(uint32_t d_tmem, uint32_t a_tmem, uint64_t b_desc, uint32_t idesc, uint32_t accumulate) {
+// D[tmem] (+)= A[tmem] * B[smem]: the A tile (128 rows x 16 bf16 values) sits in 8 consecutive TMEM columns, two values each
+__device__ __forceinline__ void tc_mma_bf16_ta(uint32_t d_tmem, uint32_t a_tmem, uint64_t b_desc, uint32_t idesc, uint32_t accumulate) {
   asm volatile(
       "{\n\t.reg .pred p;\n\t"
       "setp.ne.b32 p, %4, 0;\n\t"
-      "tcgen05.mma.cta_group::1.kind::tf32 [%0], [%1], %2, %3, {%5, %6, %7, %8}, p;\n\t}"
+      "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, {%5, %6, %7, %8}, p;\n\t}"
       ::"r"(d_tmem), "r"(a_tmem), "l"(b_desc), "r"(idesc), "r"(accumulate), "r"(0u), "r"(0u), "r"(0u), "r"(0u)
       : "memory");
+}
+// the same with A from shared memory; both descriptors by their low words (address, leading offset), `hi` above both
+__device__ __forceinline__ void tc_mma_bf16_sa(uint32_t d_tmem, uint32_t a_lo, uint32_t b_lo, uint32_t hi, uint32_t idesc, uint32_t accumulate) {
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t.reg .b64 da, db;\n\t"
+      "setp.ne.b32 p, %4, 0;\n\t"
+      "mov.b64 da, {%1, %9};\n\t"
+      "mov.b64 db, {%2, %9};\n\t"
+      "tcgen05.mma.cta_group::1.kind::f16 [%0], da, db, %3, {%5, %6, %7, %8}, p;\n\t}"
+      ::"r"(d_tmem), "r"(a_lo), "r"(b_lo), "r"(idesc), "r"(accumulate), "r"(0u), "r"(0u), "r"(0u), "r"(0u), "r"(hi)
+      : "memory");
+}
+
+// plain bulk copy of a piece of a plane image (both addresses and the size are multiples of 16 bytes)
+__device__ __forceinline__ void bulk_load(uint32_t dst, const void* src, uint32_t bytes, uint32_t bar) {
+  asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
+               ::"r"(dst), "l"(src), "r"(bytes), "r"(bar)
+               : "memory");
 }
 
 // 2^x by the special-function unit (relative error ~2^-22, far inside the tolerance of a softmax weight)
@@ -59,64 +91,307 @@ __device__ __forceinline__ float fast_exp2(float x) {
   return y;
 }
 
-struct AtcDims {
-  int64_t E, Ev, Lq, Lk;
-  int H, causal;
-  float scale_log2;   // log2(e) / sqrt(d)
-  float scale;        // 1 / sqrt(d)
+// Two values as three bf16 planes (x in the low half of each word): truncation to the upper 16 bits leaves a remainder of
+// at most 16 significant bits, the same again one of at most 8, which is a bf16 value.
+__device__ __forceinline__ void split3(float x, float y, uint32_t& p0, uint32_t& p1, uint32_t& p2) {
+  const uint32_t xb = __float_as_uint(x), yb = __float_as_uint(y);
+  p0 = __byte_perm(xb, yb, 0x7632);
+  const float rx = x - __uint_as_float(xb & 0xffff0000u), ry = y - __uint_as_float(yb & 0xffff0000u);
+  const uint32_t rxb = __float_as_uint(rx), ryb = __float_as_uint(ry);
+  p1 = __byte_perm(rxb, ryb, 0x7632);
+  p2 = __byte_perm(__float_as_uint(rx - __uint_as_float(rxb & 0xffff0000u)), __float_as_uint(ry - __uint_as_float(ryb & 0xffff0000u)), 0x7632);
+}
+__device__ __forceinline__ uint32_t pack2(float lo, float hi) {
+  const __nv_bfloat162 v = __floats2bfloat162_rn(lo, hi);
+  return *reinterpret_cast<const uint32_t*>(&v);
+}
+
+// 32 values of a thread's row into the three planes of an A operand: 16 columns each at t0, t1 and t2
+__device__ __forceinline__ void store_planes32(uint32_t t0, uint32_t t1, uint32_t t2, const uint32_t* v) {
+  uint32_t a[16], b[16], c[16];
+#pragma unroll
+  for (int e = 0; e < 16; ++e) split3(__uint_as_float(v[2 * e]), __uint_as_float(v[2 * e + 1]), a[e], b[e], c[e]);
+  tc_st_32x32b_x16(t0, a);
+  tc_st_32x32b_x16(t1, b);
+  tc_st_32x32b_x16(t2, c);
+}
+
+// 32 consecutive features (from c0) of one row as Float32 values; zero beyond the head size or for a dead row
+__device__ __forceinline__ void row_f32(const float* src, int c0, int width, bool live, bool vec, uint32_t* v) {
+  if (vec) {
+#pragma unroll
+    for (int c = 0; c < 32; c += 4) {
+      float4 x = make_float4(0.f, 0.f, 0.f, 0.f);
+      if (live && c0 + c < width) x = __ldg((const float4*)(src + c0 + c));
+      v[c] = __float_as_uint(x.x); v[c + 1] = __float_as_uint(x.y); v[c + 2] = __float_as_uint(x.z); v[c + 3] = __float_as_uint(x.w);
+    }
+  } else {
+#pragma unroll
+    for (int c = 0; c < 32; ++c) v[c] = (live && c0 + c < width) ? __float_as_uint(__ldg(src + c0 + c)) : 0u;
+  }
+}
+
+// One row of a CTA's own operand into tensor memory: NP planes of 32 columns each (Float32 source: 3, bf16 source: 1)
+template <int NP>
+__device__ __forceinline__ void row_to_tmem(const void* src, int width, bool live, bool vec, uint32_t t_addr) {
+#pragma unroll
+  for (int hf = 0; hf < 2; ++hf) {
+    if (NP == 3) {
+      uint32_t v[32];
+      row_f32((const float*)src, 32 * hf, width, live, vec, v);
+      store_planes32(t_addr + 16u * hf, t_addr + 32u + 16u * hf, t_addr + 64u + 16u * hf, v);
+    } else {
+      uint32_t v[16];
+#pragma unroll
+      for (int c = 0; c < 16; c += 4) {   // bf16 head sizes are multiples of 8
+        uint4 x = make_uint4(0u, 0u, 0u, 0u);
+        if (live && 32 * hf + 2 * c < width) x = __ldg((const uint4*)((const uint16_t*)src + 32 * hf + 2 * c));
+        v[c] = x.x; v[c + 1] = x.y; v[c + 2] = x.z; v[c + 3] = x.w;
+      }
+      tc_st_32x32b_x16(t_addr + 16u * hf, v);
+    }
+  }
+}
+
+// 32 columns (from c0) of an output row, scaled; Float32, or bf16 rounded to nearest
+template <bool BF16>
+__device__ __forceinline__ void store_row32(void* dst, int c0, int width, bool vec, const float* v, float sc) {
+  if (BF16) {
+#pragma unroll
+    for (int c = 0; c < 32; c += 8)
+      if (c0 + c < width)
+        *(uint4*)((uint16_t*)dst + c0 + c) = make_uint4(pack2(v[c] * sc, v[c + 1] * sc), pack2(v[c + 2] * sc, v[c + 3] * sc),
+                                                        pack2(v[c + 4] * sc, v[c + 5] * sc), pack2(v[c + 6] * sc, v[c + 7] * sc));
+  } else if (vec) {
+#pragma unroll
+    for (int c = 0; c < 32; c += 4)
+      if (c0 + c < width) *(float4*)((float*)dst + c0 + c) = make_float4(v[c] * sc, v[c + 1] * sc, v[c + 2] * sc, v[c + 3] * sc);
+  } else {
+#pragma unroll
+    for (int c = 0; c < 32; ++c)
+      if (c0 + c < width) ((float*)dst)[c0 + c] = v[c] * sc;
+  }
+}
+
+// The plane products of A (NA planes) and B (NB planes) from the smallest to the largest: 3 x 3 leaves out the three below
+// 2^-24 of the whole.
+template <int NA, int NB>
+struct Prod {
+  static constexpr int N = NA == 3 && NB == 3 ? 6 : NA == 3 ? 3 : 1;
+  static __device__ __forceinline__ constexpr int a(int i) { return N == 6 ? (i == 0 ? 2 : i == 2 || i == 3 ? 1 : 0) : N == 3 ? 2 - i : 0; }
+  static __device__ __forceinline__ constexpr int b(int i) { return N == 6 ? (i == 1 ? 2 : i == 2 || i == 4 ? 1 : 0) : 0; }
 };
 
-// Pipelined variant: three K / V stages in shared memory (a K tile is reloaded three blocks ahead, which covers the
-// latency of its TMA load); Q lives in tensor memory as the A operand of Q K' (hi and lo parts, stored once by the
-// softmax warps), next to two S buffers (P hi overwrites S in place), two P lo buffers and two P V buffers.  The MMA
-// warp issues Q K' of block j + 1 before P V of block j, so the tensor pipe works on the next scores while the softmax
-// warps are busy with the current ones; the softmax warps add P V of block j - 1 after they have handed P of block j
-// to the tensor core.
-//   TMEM columns: Q hi 0..63, Q lo 64..127; S/P_hi 128.., 192..; P_lo 256.., 320..; P V 384.., 448..
-constexpr int P2_NSTAGE = 3;
-constexpr int P2_STAGE0 = 0, P2_STAGE_BYTES = 65536;          // per stage: K hi, K lo, V hi, V lo (16 KB each)
-constexpr int P2_BAR = P2_STAGE0 + P2_NSTAGE * P2_STAGE_BYTES;   // 196608
-constexpr int ATC2_SMEM = P2_BAR + 512 + 1024;
-enum { C_QREADY = 0, C_KFULL, C_KREADY = C_KFULL + 3, C_KFREE = C_KREADY + 3, C_VFULL = C_KFREE + 3, C_VREADY = C_VFULL + 3,
-       C_VFREE = C_VREADY + 3, C_SFULL = C_VFREE + 3, C_PREADY = C_SFULL + 2, C_OFULL = C_PREADY + 2, C_COUNT = C_OFULL + 2 };
+// instruction descriptors: D = F32, A = B = BF16, M = 128; B K-major (n columns = rows of the tile) or MN-major
+__device__ __forceinline__ uint32_t idesc_bf16(int n, bool b_mn) {
+  return (1u << 4) | (1u << 7) | (1u << 10) | ((b_mn ? 1u : 0u) << 16) | ((uint32_t)(n >> 3) << 17) | ((uint32_t)(QT >> 4) << 24);
+}
+// operand tiles at 1024-byte boundaries: K-major (one k-step of 16 values = 32 bytes) and MN-major (16 rows of 128 bytes)
+__device__ __forceinline__ uint64_t desc_k(uint32_t saddr) { return make_smem_desc(saddr, 16, 1024, LAYOUT_SW128); }
+__device__ __forceinline__ uint64_t desc_mn(uint32_t saddr) { return make_smem_desc(saddr, KT * 128, 1024, LAYOUT_SW128); }
 
-__global__ void __launch_bounds__(ATC_THREADS, 1)
-attn_fwd_tc2_kernel(const float* __restrict__ qmat, const __grid_constant__ CUtensorMap tmK,
-                    const __grid_constant__ CUtensorMap tmV, float* __restrict__ o, float* __restrict__ lse, AtcDims D,
-                    int32_t* __restrict__ dev_err) {
+// D = A B', A = NP planes in tensor memory (32 columns each), B = NP K-major planes; nks steps of 16 features
+template <int NP>
+__device__ __forceinline__ void mma_rows_t(uint32_t d, uint32_t a_tmem, uint32_t b_smem, int nks) {
+  const uint64_t b0 = desc_k(b_smem);
+  const uint32_t idesc = idesc_bf16(KT, false);
+  using P = Prod<NP, NP>;
+#pragma unroll
+  for (int i = 0; i < P::N; ++i)
+#pragma unroll
+    for (int ks = 0; ks < 4; ++ks)
+      if (ks < nks)
+        tc_mma_bf16_ta(d, a_tmem + (uint32_t)(32 * P::a(i) + 8 * ks), b0 + (uint64_t)((P::b(i) * TILE + ks * 32) >> 4), idesc,
+                       (i > 0 || ks > 0) ? 1u : 0u);
+}
+// the same with A in shared memory: planes of 128 rows, 2 * TILE apart, all four steps (head sizes are zero-padded)
+template <int NP>
+__device__ __forceinline__ void mma_rows_s(uint32_t d, uint32_t a_smem, uint32_t b_smem) {
+  const uint64_t a0 = desc_k(a_smem), b0 = desc_k(b_smem);
+  const uint32_t idesc = idesc_bf16(KT, false), hi = (uint32_t)(a0 >> 32);
+  using P = Prod<NP, NP>;
+#pragma unroll
+  for (int i = 0; i < P::N; ++i)
+#pragma unroll
+    for (int ks = 0; ks < 4; ++ks)
+      tc_mma_bf16_sa(d, (uint32_t)a0 + (uint32_t)((P::a(i) * 2 * TILE + ks * 32) >> 4), (uint32_t)b0 + (uint32_t)((P::b(i) * TILE + ks * 32) >> 4),
+                     hi, idesc, (i > 0 || ks > 0) ? 1u : 0u);
+}
+// D (+)= A B with A = three planes of 64 values in tensor memory that the compute warps stored in halves of 32 values:
+// plane 0 at t01 + 32 half, plane 1 sixteen columns behind it, plane 2 at t2 + hstep2 half; B = NP MN-major planes whose K
+// rows are the tile's rows; n columns (features, a multiple of 16)
+template <int NP>
+__device__ __forceinline__ void mma_planes(uint32_t d, uint32_t t01, uint32_t t2, uint32_t hstep2, uint32_t b_smem, int n, bool accumulate) {
+  const uint64_t b0 = desc_mn(b_smem);
+  const uint32_t idesc = idesc_bf16(n, true);
+  using P = Prod<3, NP>;
+#pragma unroll
+  for (int i = 0; i < P::N; ++i)
+#pragma unroll
+    for (int ks = 0; ks < 4; ++ks) {
+      const uint32_t hf = (uint32_t)(ks >> 1), in = (uint32_t)(8 * (ks & 1));
+      const uint32_t a = P::a(i) == 2 ? t2 + hstep2 * hf + in : t01 + 32u * hf + 16u * (uint32_t)P::a(i) + in;
+      tc_mma_bf16_ta(d, a, b0 + (uint64_t)((P::b(i) * TILE + ks * 2048) >> 4), idesc, (accumulate || i > 0 || ks > 0) ? 1u : 0u);
+    }
+}
+
+// -------------------------------------------------------------------------------------------- plane images ---
+// One 64 x 64 tile of one (batch, head): rows of Float32 or bf16 values -> NP bf16 planes, each the shared-memory image of
+// the tile (row r at 128 r, its 16-byte chunks permuted by r & 7); rows past the end and features past the head size are 0.
+// For dO the same pass forms what the softmax backward needs per query: {log2(e) lse, delta = sum_c dO_c O_c}; queries past
+// the end get {inf, 0}, which makes their weights 0.
+// Bound by memory: 4 bytes in, 6 out per value (Float32).
+struct SplitJob {
+  const void* src;
+  uint8_t* dst;
+  int64_t L, E;
+  int width, tiles;
+};
+struct SplitArgs {
+  SplitJob job[4];
+  const float* o;       // for the job of index 3 (dO)
+  const float* lse;
+  float2* rv;
+  int H, vec;
+};
+
+template <int NP>
+__global__ void __launch_bounds__(256) attn_split_kernel(SplitArgs A) {
+  const SplitJob J = A.job[blockIdx.z];
+  if ((int)blockIdx.x >= J.tiles) return;
+  const int64_t bh = blockIdx.y;
+  const int64_t b = bh / A.H;
+  const int h = (int)(bh - b * A.H);
+  uint8_t* dst = J.dst + (bh * J.tiles + blockIdx.x) * (int64_t)(NP * TILE);
+  const int ch = threadIdx.x & 7;
+  const bool is_do = blockIdx.z == 3;
+#pragma unroll
+  for (int it = 0; it < 2; ++it) {
+    const int r = (threadIdx.x >> 3) + 32 * it;
+    const int64_t row = (int64_t)blockIdx.x * KT + r;
+    const bool live = row < J.L;
+    const int64_t off = (b * J.L + row) * J.E + (int64_t)h * J.width;
+    uint8_t* out = dst + r * 128 + ((ch ^ (r & 7)) << 4);
+    float x[8];
+    if (NP == 3) {
+      const float* s = (const float*)J.src + off;
+      if (A.vec) {
+#pragma unroll
+        for (int e = 0; e < 8; e += 4) {
+          float4 t = make_float4(0.f, 0.f, 0.f, 0.f);
+          if (live && 8 * ch + e < J.width) t = __ldg((const float4*)(s + 8 * ch + e));
+          x[e] = t.x; x[e + 1] = t.y; x[e + 2] = t.z; x[e + 3] = t.w;
+        }
+      } else {
+#pragma unroll
+        for (int e = 0; e < 8; ++e) x[e] = (live && 8 * ch + e < J.width) ? __ldg(s + 8 * ch + e) : 0.0f;
+      }
+      uint32_t p0[4], p1[4], p2[4];
+#pragma unroll
+      for (int e = 0; e < 4; ++e) split3(x[2 * e], x[2 * e + 1], p0[e], p1[e], p2[e]);
+      *(uint4*)out = make_uint4(p0[0], p0[1], p0[2], p0[3]);
+      *(uint4*)(out + TILE) = make_uint4(p1[0], p1[1], p1[2], p1[3]);
+      *(uint4*)(out + 2 * TILE) = make_uint4(p2[0], p2[1], p2[2], p2[3]);
+    } else {
+      uint4 t = make_uint4(0u, 0u, 0u, 0u);
+      if (live && 8 * ch < J.width) t = __ldg((const uint4*)((const uint16_t*)J.src + off + 8 * ch));
+      *(uint4*)out = t;
+      const uint32_t w[4] = {t.x, t.y, t.z, t.w};
+#pragma unroll
+      for (int e = 0; e < 4; ++e) {
+        x[2 * e] = __uint_as_float(w[e] << 16);
+        x[2 * e + 1] = __uint_as_float(w[e] & 0xffff0000u);
+      }
+    }
+    if (is_do) {
+      float s = 0.0f;
+#pragma unroll
+      for (int e = 0; e < 8; e += 4) {
+        if (!live || 8 * ch + e >= J.width) break;
+        const float* po = A.o + off + 8 * ch + e;
+        if (A.vec) {
+          const float4 t = __ldg((const float4*)po);
+          s = fmaf(x[e], t.x, s); s = fmaf(x[e + 1], t.y, s); s = fmaf(x[e + 2], t.z, s); s = fmaf(x[e + 3], t.w, s);
+        } else {
+          for (int u = 0; u < 4 && 8 * ch + e + u < J.width; ++u) s = fmaf(x[e + u], __ldg(po + u), s);
+        }
+      }
+      s += __shfl_xor_sync(0xffffffffu, s, 1);
+      s += __shfl_xor_sync(0xffffffffu, s, 2);
+      s += __shfl_xor_sync(0xffffffffu, s, 4);
+      if (ch == 0) A.rv[bh * ((int64_t)J.tiles * KT) + row] = live ? make_float2(A.lse[bh * J.L + row] * LOG2E, s) : make_float2(INFINITY, 0.0f);
+    }
+  }
+}
+
+// ---------------------------------------------------------------------------------- what the kernels share ---
+struct Shared {
+  uint8_t* smem;
+  uint32_t sb;       // its shared-space address (1024-byte aligned)
+};
+__device__ __forceinline__ Shared aligned_smem(uint8_t* raw) {
+  Shared s;
+  s.smem = (uint8_t*)(((uintptr_t)raw + 1023) & ~(uintptr_t)1023);
+  s.sb = smem_u32(s.smem);
+  return s;
+}
+__device__ __forceinline__ void tmem_alloc(volatile uint32_t* slot, uint32_t cols) {
+  asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32((const void*)slot)), "r"(cols) : "memory");
+  asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+}
+__device__ __forceinline__ void tmem_free(uint32_t base, uint32_t cols) {
+  asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(base), "r"(cols) : "memory");
+}
+
+// ------------------------------------------------------------------------------------------------------ forward ---
+// One CTA owns 128 queries of one (batch, head); warp 0 copies K and V tiles into a ring of slots (K0 V0 K1 V1 ...),
+// warp 1 issues the MMAs, warps 2-5 are the softmax (thread = query).  S = Q K' lands in 64 columns, the weights replace it
+// as three planes (96 columns), P V lands in 64 more and is added to the thread's registers with round-to-nearest adds.
+// Within a CTA these steps follow one another; what keeps the tensor pipe busy is the SECOND CTA on the SM: 256 of the 512
+// TMEM columns, half of the registers and of shared memory each.
+//   TMEM columns: Q planes 0..95, S -> P planes 96..191, P V 192..255
+constexpr int FWD_THREADS = 192;
+template <int NP>
+struct FwdCfg {
+  static constexpr int SLOTS = NP == 3 ? 4 : 8;
+  static constexpr int SLOT_BYTES = NP * TILE;
+  static constexpr int BAR = SLOTS * SLOT_BYTES;
+  static constexpr int SMEM = BAR + 256 + 1024;
+};
+
+template <int NP>
+__global__ void __launch_bounds__(FWD_THREADS, 2)
+attn_fwd_tc_kernel(const void* __restrict__ qmat, const uint8_t* __restrict__ kimg, const uint8_t* __restrict__ vimg,
+                   float* __restrict__ o, uint16_t* __restrict__ o16, float* __restrict__ lse, AtcDims D, int32_t* __restrict__ dev_err) {
+  using cfg = FwdCfg<NP>;
+  constexpr int S = cfg::SLOTS;
+  enum { B_FULL = 0, B_FREE = S, B_QREADY = 2 * S, B_SFULL, B_PREADY, B_OFULL, B_COUNT };
   extern __shared__ uint8_t smem_raw[];
-  uint8_t* smem = (uint8_t*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
-  const uint32_t sb = smem_u32(smem);
-  const uint32_t bar0 = sb + P2_BAR;
+  const Shared sh = aligned_smem(smem_raw);
+  const uint32_t sb = sh.sb, bar0 = sb + cfg::BAR;
   auto bar = [&](int i) { return bar0 + 8u * (uint32_t)i; };
-  volatile uint32_t* s_tmem = (volatile uint32_t*)(smem + P2_BAR + 8 * C_COUNT);
-  volatile int* s_abort = (volatile int*)(smem + P2_BAR + 8 * C_COUNT + 8);
-  volatile int* s_skip = (volatile int*)(smem + P2_BAR + 8 * C_COUNT + 16);
+  volatile uint32_t* s_tmem = (volatile uint32_t*)(sh.smem + cfg::BAR + 8 * B_COUNT);
+  volatile int* s_abort = (volatile int*)(s_tmem + 1);
+  volatile int* s_skip = (volatile int*)(s_tmem + 2);
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   // causal: the last query tiles have the most key blocks, so they are scheduled first
   const int64_t i0 = (int64_t)(D.causal ? gridDim.x - 1 - blockIdx.x : blockIdx.x) * QT;
   const int h = blockIdx.y;
-  const int64_t b = blockIdx.z;
+  const int64_t b = blockIdx.z, bh = b * D.H + h;
   int64_t kv_end = D.Lk;
   if (D.causal && i0 + QT < kv_end) kv_end = i0 + QT;
   const int nkb = (int)((kv_end + KT - 1) / KT);
 
   if (threadIdx.x == 0) {
-    mbar_init(bar(C_QREADY), 4);
-    for (int st = 0; st < P2_NSTAGE; ++st) {
-      mbar_init(bar(C_KFULL + st), 1);
-      mbar_init(bar(C_KREADY + st), 4);
-      mbar_init(bar(C_KFREE + st), 1);
-      mbar_init(bar(C_VFULL + st), 1);
-      mbar_init(bar(C_VREADY + st), 4);
-      mbar_init(bar(C_VFREE + st), 1);
+    for (int s = 0; s < S; ++s) {
+      mbar_init(bar(B_FULL + s), 1);
+      mbar_init(bar(B_FREE + s), 1);
     }
-    for (int st = 0; st < 2; ++st) {
-      mbar_init(bar(C_SFULL + st), 1);
-      mbar_init(bar(C_PREADY + st), 4);
-      mbar_init(bar(C_OFULL + st), 1);
-    }
+    mbar_init(bar(B_QREADY), 4);
+    mbar_init(bar(B_SFULL), 1);
+    mbar_init(bar(B_PREADY), 4);
+    mbar_init(bar(B_OFULL), 1);
     *s_abort = 0;
     *s_skip = (*(volatile int32_t*)dev_err != 0) ? 1 : 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -124,148 +399,91 @@ attn_fwd_tc2_kernel(const float* __restrict__ qmat, const __grid_constant__ CUte
   }
   __syncthreads();
   if (*s_skip != 0) return;
-  if (warp == 1) {
-    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32((const void*)s_tmem)), "r"(512u)
-                 : "memory");
-    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
-  }
+  if (warp == 1) tmem_alloc(s_tmem, 256u);
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
-  const uint32_t tmem_base = *s_tmem;
-  // block j uses TMEM buffer j & 1 for the (j >> 1)-th time and shared-memory stage j % 3 for the (j / 3)-th time
-  auto par = [](int j) { return (uint32_t)(j >> 1) & 1u; };
-  auto par3 = [](int j) { return (uint32_t)(j / P2_NSTAGE) & 1u; };
+  const uint32_t tmem = *s_tmem;
+  constexpr uint32_t T_R = 96, T_O = 192;
 
   if (warp == 0) {
-    // ---------------------------------------------------------------- TMA producer ---
+    // ---------------------------------------------------------------- producer ---
     if (lane == 0) {
-      const int krow0 = (int)(b * D.Lk);
-      for (int j = 0; j < nkb; ++j) {
-        const int st = j % P2_NSTAGE;
-        const uint32_t base = sb + P2_STAGE0 + (uint32_t)(st * P2_STAGE_BYTES);
-        if (j >= P2_NSTAGE && !mbar_wait(bar(C_KFREE + st), par3(j - P2_NSTAGE), s_abort)) break;
-        mbar_arrive_expect_tx(bar(C_KFULL + st), 16384u);
-#pragma unroll
-        for (int c = 0; c < 4; ++c) tma_load_2d(base + c * 4096, &tmK, h * HD + 16 * c, krow0 + j * KT, bar(C_KFULL + st));
-        if (j >= P2_NSTAGE && !mbar_wait(bar(C_VFREE + st), par3(j - P2_NSTAGE), s_abort)) break;
-        mbar_arrive_expect_tx(bar(C_VFULL + st), 16384u);
-        tma_load_3d(base + 32768, &tmV, 0, krow0 + j * KT, 2 * h, bar(C_VFULL + st));
+      const int64_t base = bh * D.ktiles * (int64_t)cfg::SLOT_BYTES;
+      for (int n = 0; n < 2 * nkb; ++n) {
+        const int s = n % S;
+        if (n >= S && !mbar_wait(bar(B_FREE + s), (uint32_t)(n / S - 1) & 1u, s_abort)) break;
+        mbar_arrive_expect_tx(bar(B_FULL + s), (uint32_t)cfg::SLOT_BYTES);
+        bulk_load(sb + (uint32_t)(s * cfg::SLOT_BYTES), ((n & 1) ? vimg : kimg) + base + (int64_t)(n >> 1) * cfg::SLOT_BYTES,
+                  (uint32_t)cfg::SLOT_BYTES, bar(B_FULL + s));
       }
     }
   } else if (warp == 1) {
-    // ------------------------------------------------------------------ MMA issuer ---
+    // -------------------------------------------------------------- MMA issuer ---
     if (lane == 0) {
-      const uint32_t idesc_qk = (1u << 4) | (2u << 7) | (2u << 10) | ((uint32_t)(KT >> 3) << 17) | ((uint32_t)(QT >> 4) << 24);
-      const uint32_t idesc_pv = idesc_qk | (1u << 16);
-      // descriptors differ only in their 14-bit start-address field (units of 16 bytes): build one per tile and add
-      // the per-k-step offsets, so that issuing an MMA costs a couple of integer adds
-      auto issue_qk = [&](int j) -> bool {
-        const int st = j % P2_NSTAGE, buf = j & 1;
-        if (!mbar_wait(bar(C_KREADY + st), par3(j), s_abort)) return false;
+      const int nks = (D.d + 15) >> 4, nv = (D.dv + 15) & ~15;
+      auto issue_s = [&](int j) -> bool {
+        const int n = 2 * j, s = n % S;
+        if (!mbar_wait(bar(B_FULL + s), (uint32_t)(n / S) & 1u, s_abort)) return false;
         tc_fence_after();
-        const uint32_t kb = sb + P2_STAGE0 + (uint32_t)(st * P2_STAGE_BYTES);
-        const uint64_t dk_hi = make_smem_desc(kb, 16, 512, LAYOUT_SW64), dk_lo = make_smem_desc(kb + 16384, 16, 512, LAYOUT_SW64);
-        const uint32_t d = tmem_base + 128u + (uint32_t)(64 * buf);
-#pragma unroll
-        for (int ks = 0; ks < 8; ++ks) {
-          const uint64_t ko = (uint64_t)(((ks >> 1) * 4096 + (ks & 1) * 32) >> 4);
-          const uint32_t ao = (uint32_t)(8 * ks);
-          tc_mma_tf32_ta(d, tmem_base + 64u + ao, dk_hi + ko, idesc_qk, ks > 0 ? 1u : 0u);
-          tc_mma_tf32_ta(d, tmem_base + ao, dk_lo + ko, idesc_qk, 1u);
-          tc_mma_tf32_ta(d, tmem_base + ao, dk_hi + ko, idesc_qk, 1u);
-        }
-        tc_commit(bar(C_SFULL + buf));
-        tc_commit(bar(C_KFREE + st));
+        mma_rows_t<NP>(tmem + T_R, tmem, sb + (uint32_t)(s * cfg::SLOT_BYTES), nks);
+        tc_commit(bar(B_SFULL));
+        tc_commit(bar(B_FREE + s));
         return true;
       };
-      bool ok = mbar_wait(bar(C_QREADY), 0u, s_abort);
-      ok = ok && issue_qk(0);
+      bool ok = mbar_wait(bar(B_QREADY), 0u, s_abort) && issue_s(0);
       for (int j = 0; j < nkb && ok; ++j) {
-        const int st = j % P2_NSTAGE, buf = j & 1;
-        if (j + 1 < nkb) {
-          ok = issue_qk(j + 1);
-          if (!ok) break;
-        }
-        ok = mbar_wait(bar(C_PREADY + buf), par(j), s_abort) && mbar_wait(bar(C_VREADY + st), par3(j), s_abort);
+        const int n = 2 * j + 1, s = n % S;
+        ok = mbar_wait(bar(B_FULL + s), (uint32_t)(n / S) & 1u, s_abort) && mbar_wait(bar(B_PREADY), (uint32_t)j & 1u, s_abort);
         if (!ok) break;
         tc_fence_after();
-        const uint32_t vb = sb + P2_STAGE0 + (uint32_t)(st * P2_STAGE_BYTES) + 32768;
-        const uint32_t d = tmem_base + 384u + (uint32_t)(64 * buf);
-        const uint64_t dv_hi = make_smem_desc(vb, KT * 128, 512, LAYOUT_SW128_32B);
-        const uint64_t dv_lo = make_smem_desc(vb + 16384, KT * 128, 512, LAYOUT_SW128_32B);
-        const uint32_t a_hi0 = tmem_base + 128u + (uint32_t)(64 * buf), a_lo0 = a_hi0 + 128u;
-#pragma unroll
-        for (int ks = 0; ks < 8; ++ks) {
-          const uint64_t vo = (uint64_t)((ks * 1024) >> 4);
-          tc_mma_tf32_ta(d, a_lo0 + (uint32_t)(8 * ks), dv_hi + vo, idesc_pv, ks > 0 ? 1u : 0u);
-          tc_mma_tf32_ta(d, a_hi0 + (uint32_t)(8 * ks), dv_lo + vo, idesc_pv, 1u);
-          tc_mma_tf32_ta(d, a_hi0 + (uint32_t)(8 * ks), dv_hi + vo, idesc_pv, 1u);
-        }
-        tc_commit(bar(C_OFULL + buf));
-        tc_commit(bar(C_VFREE + st));
+        mma_planes<NP>(tmem + T_O, tmem + T_R, tmem + T_R + 64u, 16u, sb + (uint32_t)(s * cfg::SLOT_BYTES), nv, false);
+        tc_commit(bar(B_OFULL));
+        tc_commit(bar(B_FREE + s));
+        // the next scores go where the weights are: the tensor pipe runs in order
+        if (j + 1 < nkb) ok = issue_s(j + 1);
       }
     }
-  } else if (warp < 6) {
-    // ------------------------------------------------------------------ softmax warps ---
+  } else {
+    // ------------------------------------------------------------ softmax warps ---
     const int q = warp & 3;
-    const int row = 32 * q + lane;
-    const int64_t gi = i0 + row;
-    const uint32_t t_row = tmem_base + ((uint32_t)(32 * q) << 16);
+    const int64_t gi = i0 + 32 * q + lane;
+    const bool live = gi < D.Lq;
+    const uint32_t t_row = tmem + ((uint32_t)(32 * q) << 16);
+    const int64_t el = NP == 3 ? 4 : 2;
+    row_to_tmem<NP>((const uint8_t*)qmat + el * ((b * D.Lq + gi) * D.E + (int64_t)h * D.d), D.d, live, D.vec != 0, t_row);
+    tc_wait_st();
+    tc_fence_before();
+    __syncwarp();
+    if (lane == 0) mbar_arrive(bar(B_QREADY));
     float m = -INFINITY, l = 0.0f;
     float acc[HD];
 #pragma unroll
     for (int c = 0; c < HD; ++c) acc[c] = 0.0f;
-    bool ok = true;
-    {
-      // Q row of this thread into tensor memory: the raw value is the hi operand, lo = x - tf32(x)
-      const float* src = qmat + (b * D.Lq + gi) * D.E + (int64_t)h * HD;
+    // adds P V of block j to the accumulators (waits for its MMAs)
+    auto add_pv = [&](int j) -> bool {
+      if (!mbar_wait(bar(B_OFULL), (uint32_t)j & 1u, s_abort)) return false;
+      tc_fence_after();
 #pragma unroll
       for (int hf = 0; hf < 2; ++hf) {
-        uint32_t hi[32], lo[32];
+        uint32_t v[32];
+        tc_ld_32x32b_x32(t_row + T_O + 32u * hf, v);
+        tc_wait_ld();
 #pragma unroll
-        for (int c4 = 0; c4 < 8; ++c4) {
-          float4 x = make_float4(0.f, 0.f, 0.f, 0.f);
-          if (gi < D.Lq) x = __ldg((const float4*)(src + 32 * hf + 4 * c4));
-          hi[4 * c4] = __float_as_uint(x.x); hi[4 * c4 + 1] = __float_as_uint(x.y);
-          hi[4 * c4 + 2] = __float_as_uint(x.z); hi[4 * c4 + 3] = __float_as_uint(x.w);
-          lo[4 * c4] = __float_as_uint(tf32_lo(x.x)); lo[4 * c4 + 1] = __float_as_uint(tf32_lo(x.y));
-          lo[4 * c4 + 2] = __float_as_uint(tf32_lo(x.z)); lo[4 * c4 + 3] = __float_as_uint(tf32_lo(x.w));
-        }
-        tc_st_32x32b_x32(t_row + (uint32_t)(32 * hf), hi);
-        tc_st_32x32b_x32(t_row + (uint32_t)(64 + 32 * hf), lo);
-      }
-      tc_wait_st();
-      tc_fence_before();
-      __syncwarp();
-      if (lane == 0) mbar_arrive(bar(C_QREADY));
-    }
-    // adds P V of block jj to the accumulators (waits for its MMAs)
-    auto add_pv = [&](int jj) -> bool {
-      const int st = jj & 1;
-      if (!mbar_wait(bar(C_OFULL + st), par(jj), s_abort)) return false;
-      tc_fence_after();
-      uint32_t v0[32], v1[32];
-      tc_ld_32x32b_x32(t_row + 384u + (uint32_t)(64 * st), v0);
-      tc_ld_32x32b_x32(t_row + 416u + (uint32_t)(64 * st), v1);
-      tc_wait_ld();
-#pragma unroll
-      for (int c = 0; c < 32; ++c) {
-        acc[c] += __uint_as_float(v0[c]);
-        acc[c + 32] += __uint_as_float(v1[c]);
+        for (int c = 0; c < 32; ++c) acc[32 * hf + c] += __uint_as_float(v[c]);
       }
       return true;
     };
+    bool ok = true;
     for (int j = 0; j < nkb && ok; ++j) {
-      const int st = j & 1;
-      const int64_t j0 = (int64_t)j * KT;
-      ok = mbar_wait(bar(C_SFULL + st), par(j), s_abort);
+      // P V of the block before joins the accumulators while the tensor cores compute these scores
+      ok = (j == 0 || add_pv(j - 1)) && mbar_wait(bar(B_SFULL), (uint32_t)j & 1u, s_abort);
       if (!ok) break;
       tc_fence_after();
+      const int64_t j0 = (int64_t)j * KT;
       uint32_t s0[32], s1[32];
-      const uint32_t t_s = t_row + 128u + (uint32_t)(64 * st);
-      tc_ld_32x32b_x32(t_s, s0);
-      tc_ld_32x32b_x32(t_s + 32u, s1);
+      tc_ld_32x32b_x32(t_row + T_R, s0);
+      tc_ld_32x32b_x32(t_row + T_R + 32u, s1);
       tc_wait_ld();
       int64_t lim = D.Lk - j0;
       if (D.causal && gi - j0 + 1 < lim) lim = gi - j0 + 1;
@@ -289,39 +507,25 @@ attn_fwd_tc2_kernel(const float* __restrict__ qmat, const __grid_constant__ CUte
       const float alpha = fast_exp2((m - m_use) * D.scale_log2);   // m = -inf gives 0
       const float mc = m_use * D.scale_log2;
       float rs0 = 0.0f, rs1 = 0.0f;
-      {
-        // P = 2^(s c - m c) over S in place (the raw value is the hi operand) and its lo part, 32 columns at a time
-        uint32_t lo[32];
 #pragma unroll
-        for (int c = 0; c < 32; ++c) {
-          const float p0 = fast_exp2(fmaf(__uint_as_float(s0[c]), D.scale_log2, -mc));
-          rs0 += p0;
-          s0[c] = __float_as_uint(p0);
-          lo[c] = __float_as_uint(tf32_lo(p0));
-        }
-        tc_st_32x32b_x32(t_s, s0);
-        tc_st_32x32b_x32(t_s + 128u, lo);
-#pragma unroll
-        for (int c = 0; c < 32; ++c) {
-          const float p1 = fast_exp2(fmaf(__uint_as_float(s1[c]), D.scale_log2, -mc));
-          rs1 += p1;
-          s1[c] = __float_as_uint(p1);
-          lo[c] = __float_as_uint(tf32_lo(p1));
-        }
-        tc_st_32x32b_x32(t_s + 32u, s1);
-        tc_st_32x32b_x32(t_s + 160u, lo);
-        tc_wait_st();
+      for (int c = 0; c < 32; ++c) {
+        const float p = fast_exp2(fmaf(__uint_as_float(s0[c]), D.scale_log2, -mc));
+        rs0 += p;
+        s0[c] = __float_as_uint(p);
       }
-      const float rs = rs0 + rs1;
+      store_planes32(t_row + T_R, t_row + T_R + 16u, t_row + T_R + 64u, s0);
+#pragma unroll
+      for (int c = 0; c < 32; ++c) {
+        const float p = fast_exp2(fmaf(__uint_as_float(s1[c]), D.scale_log2, -mc));
+        rs1 += p;
+        s1[c] = __float_as_uint(p);
+      }
+      store_planes32(t_row + T_R + 32u, t_row + T_R + 48u, t_row + T_R + 80u, s1);
+      tc_wait_st();
       tc_fence_before();
       __syncwarp();
-      if (lane == 0) mbar_arrive(bar(C_PREADY + st));
-      // the previous block's P V joins the accumulators before they are rescaled for this block
-      if (j > 0) {
-        ok = add_pv(j - 1);
-        if (!ok) break;
-      }
-      l = l * alpha + rs;
+      if (lane == 0) mbar_arrive(bar(B_PREADY));
+      l = l * alpha + (rs0 + rs1);
       m = m_new;
       if (alpha != 1.0f) {   // the running maximum moved (rare after the first blocks)
 #pragma unroll
@@ -329,40 +533,15 @@ attn_fwd_tc2_kernel(const float* __restrict__ qmat, const __grid_constant__ CUte
       }
     }
     if (ok) ok = add_pv(nkb - 1);
-    if (ok && gi < D.Lq) {
+    if (ok && live) {
       const float inv = l > 0.0f ? 1.0f / l : 0.0f;
-      float* orow = o + (b * D.Lq + gi) * D.Ev + (int64_t)h * HD;
+      const int64_t off = (b * D.Lq + gi) * D.Ev + (int64_t)h * D.dv;
 #pragma unroll
-      for (int c = 0; c < HD; c += 4)
-        *(float4*)(orow + c) = make_float4(acc[c] * inv, acc[c + 1] * inv, acc[c + 2] * inv, acc[c + 3] * inv);
-      lse[(b * D.H + h) * D.Lq + gi] = (l > 0.0f) ? m * D.scale + logf(l) : -INFINITY;
-    }
-  } else {
-    // --------------------------------------------- split warps: lo = x - tf32(x) twins ---
-    const int tt = (warp - 6) * 32 + lane;
-    auto split = [&](int off_hi, int off_lo, int n16) {
-      const float4* hi = (const float4*)(smem + off_hi);
-      float4* lo = (float4*)(smem + off_lo);
-      for (int i = 0; i < n16; ++i) {
-        float4 v = hi[tt + i * 128];
-        v.x = tf32_lo(v.x); v.y = tf32_lo(v.y); v.z = tf32_lo(v.z); v.w = tf32_lo(v.w);
-        lo[tt + i * 128] = v;
+      for (int hf = 0; hf < 2; ++hf) {
+        if (o != nullptr) store_row32<false>(o + off, 32 * hf, D.dv, D.vec != 0, acc + 32 * hf, inv);
+        if (NP == 1) store_row32<true>(o16 + off, 32 * hf, D.dv, true, acc + 32 * hf, inv);
       }
-      fence_proxy_async();
-      __syncwarp();
-    };
-    bool ok = true;
-    for (int j = 0; j < nkb && ok; ++j) {
-      const int st = j % P2_NSTAGE;
-      const int base = P2_STAGE0 + st * P2_STAGE_BYTES;
-      ok = mbar_wait(bar(C_KFULL + st), par3(j), s_abort);
-      if (!ok) break;
-      split(base, base + 16384, 8);
-      if (lane == 0) mbar_arrive(bar(C_KREADY + st));
-      ok = mbar_wait(bar(C_VFULL + st), par3(j), s_abort);
-      if (!ok) break;
-      split(base + 32768, base + 49152, 8);
-      if (lane == 0) mbar_arrive(bar(C_VREADY + st));
+      lse[bh * D.Lq + gi] = (l > 0.0f) ? m * D.scale + logf(l) : -INFINITY;
     }
   }
 
@@ -370,57 +549,64 @@ attn_fwd_tc2_kernel(const float* __restrict__ qmat, const __grid_constant__ CUte
   __syncthreads();
   if (warp == 1) {
     __syncwarp();
-    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(512u) : "memory");
+    tmem_free(tmem, 256u);
   }
   if (threadIdx.x == 0 && *s_abort != 0) atomicExch(dev_err, 4002);
 }
 
-// ------------------------------------------------------------------------------------------------------------------
-// dQ of the attention backward pass on the tensor cores.  One CTA owns 128 queries of one (batch, head); Q and dO of
-// those queries live in tensor memory for the whole kernel (hi and lo parts, A operands of the MMAs).  For every
-// block of 64 keys: S = Q K' and dP = dO V' (B operands: K and V tiles, K-major), the compute warps turn them into
-// dS = P (dP - delta) with P = exp(S / sqrt(d) - lse) and hand dS back through tensor memory, and dQ += dS K (B
-// operand: the same K tile loaded a second time in the MN-major layout, keys being its K rows).  dQ accumulates in
-// tensor memory over at most 32 blocks (2048 keys, the accumulation length the GEMM also uses).
-//   TMEM columns: Q hi 0, Q lo 64, dO hi 128, dO lo 192, S -> dS hi 256, dS lo 320, dP 384, dQ 448
-constexpr int DQ_STAGE_BYTES = 98304;   // K k-major hi/lo (32 KB), K mn-major hi/lo (32 KB), V k-major hi/lo (32 KB)
-constexpr int DQ_BAR = 2 * DQ_STAGE_BYTES;
-constexpr int DQ_SMEM = DQ_BAR + 256 + 1024;
-constexpr int DQ_MAX_BLOCKS = 32;
-enum { E_QREADY = 0, E_FULL, E_READY = E_FULL + 2, E_FREE = E_READY + 2, E_SFULL = E_FREE + 2, E_DSREADY, E_DQFULL, E_COUNT };
+// ----------------------------------------------------------------------------------------------------------- dQ ---
+// One CTA owns 128 queries of one (batch, head).  Q and dO of those queries live in tensor memory for the whole kernel.
+// For every block of 64 keys: S = Q K' and dP = dO V', the compute warps turn them into dS = P (dP - delta) with
+// P = exp(S / sqrt(d) - lse) and put its planes over them, and dQ += dS K with the same K tile read MN-major.  Two S / dP
+// regions and two sets of four compute warps take the blocks in turn: the tensor cores work on block j + 1 and on dQ of
+// block j - 1 while a set is busy with block j.  dQ accumulates in tensor memory over at most 32 blocks (2048 keys: the
+// adds truncate).
+//   TMEM columns: Q planes 0..95, dO planes 96..191, two regions of 128 (S, dP -> dS planes) 192..447, dQ 448..511
+constexpr int BWD_THREADS = 320;
+constexpr int BWD_MAX_BLOCKS = 32;
+template <int NP>
+struct DqCfg {
+  static constexpr int SLOTS = NP == 3 ? 4 : 6;
+  static constexpr int SLOT_BYTES = 2 * NP * TILE;   // K tile, V tile
+  static constexpr int BAR = SLOTS * SLOT_BYTES;
+  static constexpr int SMEM = BAR + 256 + 1024;
+};
 
-__global__ void __launch_bounds__(ATC_THREADS, 1)
-attn_bwd_dq_tc_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant__ CUtensorMap tmKmn,
-                      const __grid_constant__ CUtensorMap tmV, const float* __restrict__ q, const float* __restrict__ dout,
-                      const float* __restrict__ lse, const float* __restrict__ dlt, float* __restrict__ dq, AtcDims D,
+template <int NP>
+__global__ void __launch_bounds__(BWD_THREADS, 1)
+attn_bwd_dq_tc_kernel(const void* __restrict__ q, const void* __restrict__ dout, const uint8_t* __restrict__ kimg,
+                      const uint8_t* __restrict__ vimg, const float2* __restrict__ rv, void* __restrict__ dq, AtcDims D,
                       int32_t* __restrict__ dev_err) {
+  using cfg = DqCfg<NP>;
+  constexpr int S = cfg::SLOTS;
+  enum { B_FULL = 0, B_FREE = S, B_QREADY = 2 * S, B_SFULL, B_DSREADY = B_SFULL + 2, B_DONE = B_DSREADY + 2, B_COUNT };
   extern __shared__ uint8_t smem_raw[];
-  uint8_t* smem = (uint8_t*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
-  const uint32_t sb = smem_u32(smem);
-  const uint32_t bar0 = sb + DQ_BAR;
+  const Shared sh = aligned_smem(smem_raw);
+  const uint32_t sb = sh.sb, bar0 = sb + cfg::BAR;
   auto bar = [&](int i) { return bar0 + 8u * (uint32_t)i; };
-  volatile uint32_t* s_tmem = (volatile uint32_t*)(smem + DQ_BAR + 8 * E_COUNT);
-  volatile int* s_abort = (volatile int*)(smem + DQ_BAR + 8 * E_COUNT + 8);
-  volatile int* s_skip = (volatile int*)(smem + DQ_BAR + 8 * E_COUNT + 16);
+  volatile uint32_t* s_tmem = (volatile uint32_t*)(sh.smem + cfg::BAR + 8 * B_COUNT);
+  volatile int* s_abort = (volatile int*)(s_tmem + 1);
+  volatile int* s_skip = (volatile int*)(s_tmem + 2);
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int64_t i0 = (int64_t)(D.causal ? gridDim.x - 1 - blockIdx.x : blockIdx.x) * QT;
   const int h = blockIdx.y;
-  const int64_t b = blockIdx.z;
+  const int64_t b = blockIdx.z, bh = b * D.H + h;
   int64_t kv_end = D.Lk;
   if (D.causal && i0 + QT < kv_end) kv_end = i0 + QT;
   const int nkb = (int)((kv_end + KT - 1) / KT);
 
   if (threadIdx.x == 0) {
-    mbar_init(bar(E_QREADY), 4);
-    for (int st = 0; st < 2; ++st) {
-      mbar_init(bar(E_FULL + st), 1);
-      mbar_init(bar(E_READY + st), 4);
-      mbar_init(bar(E_FREE + st), 1);
+    for (int s = 0; s < S; ++s) {
+      mbar_init(bar(B_FULL + s), 1);
+      mbar_init(bar(B_FREE + s), 1);
     }
-    mbar_init(bar(E_SFULL), 1);
-    mbar_init(bar(E_DSREADY), 4);
-    mbar_init(bar(E_DQFULL), 1);
+    mbar_init(bar(B_QREADY), 8);
+    for (int r = 0; r < 2; ++r) {
+      mbar_init(bar(B_SFULL + r), 1);
+      mbar_init(bar(B_DSREADY + r), 4);
+    }
+    mbar_init(bar(B_DONE), 1);
     *s_abort = 0;
     *s_skip = (*(volatile int32_t*)dev_err != 0) ? 1 : 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -428,183 +614,116 @@ attn_bwd_dq_tc_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_cons
   }
   __syncthreads();
   if (*s_skip != 0) return;
-  if (warp == 1) {
-    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32((const void*)s_tmem)), "r"(512u)
-                 : "memory");
-    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
-  }
+  if (warp == 1) tmem_alloc(s_tmem, 512u);
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
-  const uint32_t tmem_base = *s_tmem;
-  auto par = [](int j) { return (uint32_t)(j >> 1) & 1u; };
+  const uint32_t tmem = *s_tmem;
+  constexpr uint32_t T_DO = 96, T_R = 192, T_DQ = 448;
 
   if (warp == 0) {
-    // ---------------------------------------------------------------- TMA producer ---
+    // ---------------------------------------------------------------- producer ---
     if (lane == 0) {
-      const int krow0 = (int)(b * D.Lk);
+      const int64_t base = bh * D.ktiles * (int64_t)(NP * TILE);
       for (int j = 0; j < nkb; ++j) {
-        const int st = j & 1;
-        const uint32_t base = sb + (uint32_t)(st * DQ_STAGE_BYTES);
-        if (j >= 2 && !mbar_wait(bar(E_FREE + st), par(j - 2), s_abort)) break;
-        mbar_arrive_expect_tx(bar(E_FULL + st), 49152u);
-#pragma unroll
-        for (int c = 0; c < 4; ++c) tma_load_2d(base + c * 4096, &tmK, h * HD + 16 * c, krow0 + j * KT, bar(E_FULL + st));
-        tma_load_3d(base + 32768, &tmKmn, 0, krow0 + j * KT, 2 * h, bar(E_FULL + st));
-#pragma unroll
-        for (int c = 0; c < 4; ++c) tma_load_2d(base + 65536 + c * 4096, &tmV, h * HD + 16 * c, krow0 + j * KT, bar(E_FULL + st));
+        const int s = j % S;
+        if (j >= S && !mbar_wait(bar(B_FREE + s), (uint32_t)(j / S - 1) & 1u, s_abort)) break;
+        mbar_arrive_expect_tx(bar(B_FULL + s), (uint32_t)cfg::SLOT_BYTES);
+        const uint32_t dst = sb + (uint32_t)(s * cfg::SLOT_BYTES);
+        const int64_t off = base + (int64_t)j * (NP * TILE);
+        bulk_load(dst, kimg + off, NP * TILE, bar(B_FULL + s));
+        bulk_load(dst + NP * TILE, vimg + off, NP * TILE, bar(B_FULL + s));
       }
     }
   } else if (warp == 1) {
-    // ------------------------------------------------------------------ MMA issuer ---
+    // -------------------------------------------------------------- MMA issuer ---
     if (lane == 0) {
-      const uint32_t idesc_kk = (1u << 4) | (2u << 7) | (2u << 10) | ((uint32_t)(KT >> 3) << 17) | ((uint32_t)(QT >> 4) << 24);
-      const uint32_t idesc_mn = idesc_kk | (1u << 16);   // N = 64 either way (keys, or features of dQ)
-      const uint32_t t_q = tmem_base, t_do = tmem_base + 128u, t_s = tmem_base + 256u, t_dp = tmem_base + 384u, t_dq = tmem_base + 448u;
-      bool ok = mbar_wait(bar(E_QREADY), 0u, s_abort);
-      for (int j = 0; j < nkb && ok; ++j) {
-        const int st = j & 1;
-        ok = mbar_wait(bar(E_READY + st), par(j), s_abort);
-        if (!ok) break;
-        tc_fence_after();
-        const uint32_t base = sb + (uint32_t)(st * DQ_STAGE_BYTES);
-        const uint64_t dk_hi = make_smem_desc(base, 16, 512, LAYOUT_SW64), dk_lo = make_smem_desc(base + 16384, 16, 512, LAYOUT_SW64);
-        const uint64_t dv_hi = make_smem_desc(base + 65536, 16, 512, LAYOUT_SW64), dv_lo = make_smem_desc(base + 81920, 16, 512, LAYOUT_SW64);
-#pragma unroll
-        for (int ks = 0; ks < 8; ++ks) {   // S = Q K' and dP = dO V' over the 64 features
-          const uint64_t bo = (uint64_t)(((ks >> 1) * 4096 + (ks & 1) * 32) >> 4);
-          const uint32_t ao = (uint32_t)(8 * ks);
-          tc_mma_tf32_ta(t_s, t_q + 64u + ao, dk_hi + bo, idesc_kk, ks > 0 ? 1u : 0u);
-          tc_mma_tf32_ta(t_s, t_q + ao, dk_lo + bo, idesc_kk, 1u);
-          tc_mma_tf32_ta(t_s, t_q + ao, dk_hi + bo, idesc_kk, 1u);
-          tc_mma_tf32_ta(t_dp, t_do + 64u + ao, dv_hi + bo, idesc_kk, ks > 0 ? 1u : 0u);
-          tc_mma_tf32_ta(t_dp, t_do + ao, dv_lo + bo, idesc_kk, 1u);
-          tc_mma_tf32_ta(t_dp, t_do + ao, dv_hi + bo, idesc_kk, 1u);
+      const int nks = (D.d + 15) >> 4, nvs = (D.dv + 15) >> 4, nd = (D.d + 15) & ~15;
+      bool ok = mbar_wait(bar(B_QREADY), 0u, s_abort);
+      // step j: S and dP of block j + 2 (j >= -2) behind dQ of block j, whose planes they overwrite: the tensor pipe runs
+      // in order
+      for (int j = -2; j < nkb && ok; ++j) {
+        if (j >= 0) {
+          ok = mbar_wait(bar(B_DSREADY + (j & 1)), (uint32_t)(j >> 1) & 1u, s_abort);
+          if (!ok) break;
+          tc_fence_after();
+          const uint32_t r = tmem + T_R + (uint32_t)(128 * (j & 1));
+          mma_planes<NP>(tmem + T_DQ, r, r + 64u, 32u, sb + (uint32_t)((j % S) * cfg::SLOT_BYTES), nd, j > 0);
+          tc_commit(bar(B_FREE + j % S));
+          if (j == nkb - 1) tc_commit(bar(B_DONE));
         }
-        tc_commit(bar(E_SFULL));
-        ok = mbar_wait(bar(E_DSREADY), (uint32_t)j & 1u, s_abort);
-        if (!ok) break;
-        tc_fence_after();
-        const uint64_t dm_hi = make_smem_desc(base + 32768, KT * 128, 512, LAYOUT_SW128_32B);
-        const uint64_t dm_lo = make_smem_desc(base + 49152, KT * 128, 512, LAYOUT_SW128_32B);
-#pragma unroll
-        for (int ks = 0; ks < 8; ++ks) {   // dQ += dS K over the 64 keys
-          const uint64_t bo = (uint64_t)((ks * 1024) >> 4);
-          const uint32_t ao = (uint32_t)(8 * ks);
-          tc_mma_tf32_ta(t_dq, t_s + 64u + ao, dm_hi + bo, idesc_mn, (j > 0 || ks > 0) ? 1u : 0u);
-          tc_mma_tf32_ta(t_dq, t_s + ao, dm_lo + bo, idesc_mn, 1u);
-          tc_mma_tf32_ta(t_dq, t_s + ao, dm_hi + bo, idesc_mn, 1u);
-        }
-        tc_commit(bar(E_FREE + st));
-        if (j == nkb - 1) tc_commit(bar(E_DQFULL));
-      }
-    }
-  } else if (warp < 6) {
-    // ------------------------------------------------------------------ compute warps ---
-    const int qd = warp & 3;
-    const int row = 32 * qd + lane;
-    const int64_t gi = i0 + row;
-    const bool live = gi < D.Lq;
-    const uint32_t t_row = tmem_base + ((uint32_t)(32 * qd) << 16);
-    // Q and dO rows of this thread into tensor memory: the raw value is the hi operand, lo = x - tf32(x)
-    {
-      const float* src[2] = {q + (b * D.Lq + gi) * D.E + (int64_t)h * HD, dout + (b * D.Lq + gi) * D.Ev + (int64_t)h * HD};
-#pragma unroll
-      for (int w = 0; w < 2; ++w) {
-#pragma unroll
-        for (int half = 0; half < 2; ++half) {
-          uint32_t hi[32], lo[32];
-#pragma unroll
-          for (int c4 = 0; c4 < 8; ++c4) {
-            float4 x = make_float4(0.f, 0.f, 0.f, 0.f);
-            if (live) x = __ldg((const float4*)(src[w] + 32 * half + 4 * c4));
-            hi[4 * c4] = __float_as_uint(x.x); hi[4 * c4 + 1] = __float_as_uint(x.y);
-            hi[4 * c4 + 2] = __float_as_uint(x.z); hi[4 * c4 + 3] = __float_as_uint(x.w);
-            lo[4 * c4] = __float_as_uint(tf32_lo(x.x)); lo[4 * c4 + 1] = __float_as_uint(tf32_lo(x.y));
-            lo[4 * c4 + 2] = __float_as_uint(tf32_lo(x.z)); lo[4 * c4 + 3] = __float_as_uint(tf32_lo(x.w));
-          }
-          tc_st_32x32b_x32(t_row + (uint32_t)(128 * w + 32 * half), hi);
-          tc_st_32x32b_x32(t_row + (uint32_t)(128 * w + 64 + 32 * half), lo);
-        }
-      }
-      tc_wait_st();
-      tc_fence_before();
-      __syncwarp();
-      if (lane == 0) mbar_arrive(bar(E_QREADY));
-    }
-    const float l2 = live ? lse[(b * D.H + h) * D.Lq + gi] * 1.4426950408889634f : INFINITY;   // a dead row gets P = 0
-    const float dl = live ? dlt[(b * D.H + h) * D.Lq + gi] : 0.0f;
-    bool ok = true;
-    for (int j = 0; j < nkb && ok; ++j) {
-      const int64_t j0 = (int64_t)j * KT;
-      ok = mbar_wait(bar(E_SFULL), (uint32_t)j & 1u, s_abort);
-      if (!ok) break;
-      tc_fence_after();
-      int64_t lim = D.Lk - j0;
-      if (D.causal && gi - j0 + 1 < lim) lim = gi - j0 + 1;
-      const int nvalid = lim < 0 ? 0 : (lim > KT ? KT : (int)lim);
-#pragma unroll
-      for (int half = 0; half < 2; ++half) {
-        uint32_t sv[32], dp[32];
-        tc_ld_32x32b_x32(t_row + 256u + (uint32_t)(32 * half), sv);
-        tc_ld_32x32b_x32(t_row + 384u + (uint32_t)(32 * half), dp);
-        tc_wait_ld();
-#pragma unroll
-        for (int c = 0; c < 32; ++c) {
-          float p = fast_exp2(fmaf(__uint_as_float(sv[c]), D.scale_log2, -l2));
-          if (c + 32 * half >= nvalid) p = 0.0f;
-          const float ds = p * (__uint_as_float(dp[c]) - dl);
-          sv[c] = __float_as_uint(ds);
-          dp[c] = __float_as_uint(tf32_lo(ds));
-        }
-        tc_st_32x32b_x32(t_row + 256u + (uint32_t)(32 * half), sv);
-        tc_st_32x32b_x32(t_row + 320u + (uint32_t)(32 * half), dp);
-      }
-      tc_wait_st();
-      tc_fence_before();
-      __syncwarp();
-      if (lane == 0) mbar_arrive(bar(E_DSREADY));
-    }
-    if (ok) ok = mbar_wait(bar(E_DQFULL), 0u, s_abort);
-    if (ok) {
-      tc_fence_after();
-      uint32_t r0[32], r1[32];
-      tc_ld_32x32b_x32(t_row + 448u, r0);
-      tc_ld_32x32b_x32(t_row + 480u, r1);
-      tc_wait_ld();
-      if (live) {
-        float* drow = dq + (b * D.Lq + gi) * D.E + (int64_t)h * HD;
-#pragma unroll
-        for (int c = 0; c < 32; c += 4) {
-          *(float4*)(drow + c) = make_float4(__uint_as_float(r0[c]) * D.scale, __uint_as_float(r0[c + 1]) * D.scale,
-                                             __uint_as_float(r0[c + 2]) * D.scale, __uint_as_float(r0[c + 3]) * D.scale);
-          *(float4*)(drow + 32 + c) = make_float4(__uint_as_float(r1[c]) * D.scale, __uint_as_float(r1[c + 1]) * D.scale,
-                                                  __uint_as_float(r1[c + 2]) * D.scale, __uint_as_float(r1[c + 3]) * D.scale);
+        const int t = j + 2, s = t % S;
+        if (t < nkb) {
+          ok = mbar_wait(bar(B_FULL + s), (uint32_t)(t / S) & 1u, s_abort);
+          if (!ok) break;
+          tc_fence_after();
+          const uint32_t base = sb + (uint32_t)(s * cfg::SLOT_BYTES), r = tmem + T_R + (uint32_t)(128 * (t & 1));
+          mma_rows_t<NP>(r, tmem, base, nks);
+          mma_rows_t<NP>(r + 64u, tmem + T_DO, base + NP * TILE, nvs);
+          tc_commit(bar(B_SFULL + (t & 1)));
         }
       }
     }
   } else {
-    // --------------------------------------------- split warps: lo = x - tf32(x) twins ---
-    const int tt = (warp - 6) * 32 + lane;
+    // ------------------------------------------------------------ compute warps ---
+    const int set = (warp - 2) >> 2, qd = warp & 3;
+    const int64_t gi = i0 + 32 * qd + lane;
+    const bool live = gi < D.Lq;
+    const uint32_t t_row = tmem + ((uint32_t)(32 * qd) << 16);
+    const int64_t el = NP == 3 ? 4 : 2;
+    // the first set brings Q into tensor memory, the second dO
+    if (set == 0) row_to_tmem<NP>((const uint8_t*)q + el * ((b * D.Lq + gi) * D.E + (int64_t)h * D.d), D.d, live, D.vec != 0, t_row);
+    else row_to_tmem<NP>((const uint8_t*)dout + el * ((b * D.Lq + gi) * D.Ev + (int64_t)h * D.dv), D.dv, live, D.vec != 0, t_row + T_DO);
+    tc_wait_st();
+    tc_fence_before();
+    __syncwarp();
+    if (lane == 0) mbar_arrive(bar(B_QREADY));
+    const float2 ld = rv[bh * ((int64_t)D.qtiles * KT) + gi];   // {inf, 0} past the end: the weights become 0
     bool ok = true;
-    for (int j = 0; j < nkb && ok; ++j) {
-      const int st = j & 1;
-      ok = mbar_wait(bar(E_FULL + st), par(j), s_abort);
+    for (int j = set; j < nkb && ok; j += 2) {
+      ok = mbar_wait(bar(B_SFULL + set), (uint32_t)(j >> 1) & 1u, s_abort);
       if (!ok) break;
+      tc_fence_after();
+      const int64_t j0 = (int64_t)j * KT;
+      int64_t lim = D.Lk - j0;
+      if (D.causal && gi - j0 + 1 < lim) lim = gi - j0 + 1;
+      const int nvalid = lim < 0 ? 0 : (lim > KT ? KT : (int)lim);
+      const uint32_t r = t_row + T_R + (uint32_t)(128 * set);
 #pragma unroll
-      for (int tile = 0; tile < 3; ++tile) {
-        const float4* hi = (const float4*)(smem + st * DQ_STAGE_BYTES + tile * 32768);
-        float4* lo = (float4*)(smem + st * DQ_STAGE_BYTES + tile * 32768 + 16384);
+      for (int hf = 0; hf < 2; ++hf) {
+        uint32_t sv[32], dp[32];
+        tc_ld_32x32b_x32(r + 32u * hf, sv);
+        tc_ld_32x32b_x32(r + 64u + 32u * hf, dp);
+        tc_wait_ld();
+        if (nvalid >= KT) {
 #pragma unroll
-        for (int i = 0; i < 8; ++i) {
-          float4 v = hi[tt + i * 128];
-          v.x = tf32_lo(v.x); v.y = tf32_lo(v.y); v.z = tf32_lo(v.z); v.w = tf32_lo(v.w);
-          lo[tt + i * 128] = v;
+          for (int c = 0; c < 32; ++c)
+            sv[c] = __float_as_uint(fast_exp2(fmaf(__uint_as_float(sv[c]), D.scale_log2, -ld.x)) * (__uint_as_float(dp[c]) - ld.y));
+        } else {
+#pragma unroll
+          for (int c = 0; c < 32; ++c) {
+            float p = fast_exp2(fmaf(__uint_as_float(sv[c]), D.scale_log2, -ld.x));
+            if (c + 32 * hf >= nvalid) p = 0.0f;
+            sv[c] = __float_as_uint(p * (__uint_as_float(dp[c]) - ld.y));
+          }
         }
+        // columns this thread has read already: 32 hf .. and 64 + 32 hf ..
+        store_planes32(r + 32u * hf, r + 32u * hf + 16u, r + 64u + 32u * hf, sv);
       }
-      fence_proxy_async();
+      tc_wait_st();
+      tc_fence_before();
       __syncwarp();
-      if (lane == 0) mbar_arrive(bar(E_READY + st));
+      if (lane == 0) mbar_arrive(bar(B_DSREADY + set));
+    }
+    // each set writes 32 columns
+    if (ok) ok = mbar_wait(bar(B_DONE), 0u, s_abort);
+    if (ok) {
+      tc_fence_after();
+      uint32_t v[32];
+      tc_ld_32x32b_x32(t_row + T_DQ + 32u * set, v);
+      tc_wait_ld();
+      if (live)
+        store_row32<NP == 1>((uint8_t*)dq + el * ((b * D.Lq + gi) * D.E + (int64_t)h * D.d), 32 * set, D.d, D.vec != 0, (const float*)v, D.scale);
     }
   }
 
@@ -612,66 +731,66 @@ attn_bwd_dq_tc_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_cons
   __syncthreads();
   if (warp == 1) {
     __syncwarp();
-    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(512u) : "memory");
+    tmem_free(tmem, 512u);
   }
   if (threadIdx.x == 0 && *s_abort != 0) atomicExch(dev_err, 4003);
 }
 
-// ------------------------------------------------------------------------------------------------------------------
-// dK and dV of the attention backward pass on the tensor cores, in transposed form so that keys are the rows
-// (TMEM lanes) of every accumulator.  One CTA owns 128 keys of one (batch, head): K lives in tensor memory (A operand),
-// V in shared memory (A operand, K-major).  For every block of 64 queries:
+// ------------------------------------------------------------------------------------------------------ dK, dV ---
+// Transposed, so that keys are the rows (TMEM lanes) of every accumulator.  One CTA owns 128 keys of one (batch, head); K
+// and V stay in shared memory as A operands.  For every block of 64 queries:
 //   S' = K Q'  and  dP' = V dO'    (B operands: the Q and dO tiles, K-major)
-//   P' = exp(S' / sqrt(d) - lse_q),  dS' = P' (dP' - delta_q)     (compute warps; back through tensor memory)
-//   dV += P' dO  and  dK += dS' Q   (B operands: the same Q and dO tiles loaded a second time MN-major, queries
-//                                    being their K rows)
-// A tile's shared memory is reloaded as soon as the MMAs that read it have completed, so the loads of the next block
-// overlap the rest of the current one.  dK and dV accumulate in tensor memory over at most 32 query blocks.
-//   TMEM columns: K hi 0, K lo 64, S' -> P' hi 128, P' lo 192, dP' -> dS' hi 256, dS' lo 320, dV 384, dK 448
-constexpr int KV_VHI = 0, KV_VLO = 32768;                       // 4 chunks x [128 keys][16 floats]
-constexpr int KV_QK = 65536, KV_DOK = 98304, KV_DOM = 131072, KV_QM = 163840;   // 64-query tiles: hi 16 KB + lo 16 KB each
-constexpr int KV_ROWV = 196608;                                 // lse * log2(e) and delta of the block's 64 queries, two sets
-constexpr int KV_BAR = KV_ROWV + 1024;
-constexpr int KV_SMEM = KV_BAR + 256 + 1024;
-constexpr int KV_MAX_BLOCKS = 32;
-enum { F_KREADY = 0, F_VFULL, F_VREADY, F_FULL, F_READY = F_FULL + 4, F_FREE = F_READY + 4, F_SFULL = F_FREE + 4, F_PREADY, F_DONE, F_COUNT };
+//   P' = exp(S' / sqrt(d) - lse_q),  dS' = P' (dP' - delta_q)     (compute warps; planes back into tensor memory)
+//   dV += P' dO  and  dK += dS' Q   (B operands: the same Q and dO tiles, MN-major)
+// As in the dQ kernel two regions and two sets of compute warps take the blocks in turn.  The ring of five tile slots
+// holds dO0 Q0 dO1 Q1 dO2 ...; dV is issued before dK and dP' before S', so that a slot freed by dV of block i is
+// reloaded (with Q of block i + 2) under dK of block i and dP' of block i + 2.  K and V in tensor memory would leave room
+// for one region only; from shared memory an MMA of 128 x 64 x 16 takes 48 clocks, from tensor memory 44.
+//   TMEM columns: two regions of 192 (S', dP', 64 more -> P' and dS' planes) 0..383, dV 384..447, dK 448..511
+template <int NP>
+struct KvCfg {
+  static constexpr int SLOTS = NP == 3 ? 5 : 8;
+  static constexpr int SLOT_BYTES = NP * TILE + 1024;   // a tile and, behind dO, {lse, delta} of its 64 queries
+  static constexpr int K_OFF = SLOTS * SLOT_BYTES, V_OFF = K_OFF + NP * 2 * TILE;
+  static constexpr int BAR = V_OFF + NP * 2 * TILE;
+  static constexpr int SMEM = BAR + 256 + 1024;
+};
 
-__global__ void __launch_bounds__(ATC_THREADS, 1)
-attn_bwd_dkdv_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmQmn,
-                        const __grid_constant__ CUtensorMap tmDO, const __grid_constant__ CUtensorMap tmDOmn,
-                        const __grid_constant__ CUtensorMap tmV, const float* __restrict__ k, const float* __restrict__ lse,
-                        const float* __restrict__ dlt, float* __restrict__ dk, float* __restrict__ dv, AtcDims D,
-                        int32_t* __restrict__ dev_err) {
+template <int NP>
+__global__ void __launch_bounds__(BWD_THREADS, 1)
+attn_bwd_dkdv_tc_kernel(const uint8_t* __restrict__ qimg, const uint8_t* __restrict__ doimg, const uint8_t* __restrict__ kimg,
+                        const uint8_t* __restrict__ vimg, const float2* __restrict__ rv, void* __restrict__ dk, void* __restrict__ dv,
+                        AtcDims D, int32_t* __restrict__ dev_err) {
+  using cfg = KvCfg<NP>;
+  constexpr int S = cfg::SLOTS;
+  enum { B_FULL = 0, B_FREE = S, B_KV = 2 * S, B_SFULL, B_PREADY = B_SFULL + 2, B_DONE = B_PREADY + 2, B_COUNT };
   extern __shared__ uint8_t smem_raw[];
-  uint8_t* smem = (uint8_t*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
-  const uint32_t sb = smem_u32(smem);
-  const uint32_t bar0 = sb + KV_BAR;
+  const Shared sh = aligned_smem(smem_raw);
+  const uint32_t sb = sh.sb, bar0 = sb + cfg::BAR;
   auto bar = [&](int i) { return bar0 + 8u * (uint32_t)i; };
-  volatile uint32_t* s_tmem = (volatile uint32_t*)(smem + KV_BAR + 8 * F_COUNT);
-  volatile int* s_abort = (volatile int*)(smem + KV_BAR + 8 * F_COUNT + 8);
-  volatile int* s_skip = (volatile int*)(smem + KV_BAR + 8 * F_COUNT + 16);
-  float* rowv = (float*)(smem + KV_ROWV);   // [set][0: lse * log2e, 1: delta][64]
+  volatile uint32_t* s_tmem = (volatile uint32_t*)(sh.smem + cfg::BAR + 8 * B_COUNT);
+  volatile int* s_abort = (volatile int*)(s_tmem + 1);
+  volatile int* s_skip = (volatile int*)(s_tmem + 2);
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int64_t j0 = (int64_t)blockIdx.x * QT;   // first key of this CTA
   const int h = blockIdx.y;
-  const int64_t b = blockIdx.z;
+  const int64_t b = blockIdx.z, bh = b * D.H + h;
   // query blocks that see these keys: all of them, or under a causal mask those from the diagonal on
   const int ib0 = D.causal ? (int)(j0 / KT) : 0;
   const int nqb = (int)((D.Lq + KT - 1) / KT) - ib0;   // may be <= 0: nothing attends to these keys
 
   if (threadIdx.x == 0) {
-    mbar_init(bar(F_KREADY), 4);
-    mbar_init(bar(F_VFULL), 1);
-    mbar_init(bar(F_VREADY), 4);
-    for (int t = 0; t < 4; ++t) {
-      mbar_init(bar(F_FULL + t), 1);
-      mbar_init(bar(F_READY + t), 4);
-      mbar_init(bar(F_FREE + t), 1);
+    for (int s = 0; s < S; ++s) {
+      mbar_init(bar(B_FULL + s), 1);
+      mbar_init(bar(B_FREE + s), 1);
     }
-    mbar_init(bar(F_SFULL), 1);
-    mbar_init(bar(F_PREADY), 4);
-    mbar_init(bar(F_DONE), 1);
+    mbar_init(bar(B_KV), 1);
+    for (int r = 0; r < 2; ++r) {
+      mbar_init(bar(B_SFULL + r), 1);
+      mbar_init(bar(B_PREADY + r), 4);
+    }
+    mbar_init(bar(B_DONE), 1);
     *s_abort = 0;
     *s_skip = (*(volatile int32_t*)dev_err != 0) ? 1 : 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -679,243 +798,136 @@ attn_bwd_dkdv_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_co
   }
   __syncthreads();
   if (*s_skip != 0) return;
-  if (warp == 1) {
-    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32((const void*)s_tmem)), "r"(512u)
-                 : "memory");
-    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
-  }
+  if (warp == 1) tmem_alloc(s_tmem, 512u);
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
-  const uint32_t tmem_base = *s_tmem;
-  // tile order: 0 = Q k-major, 1 = dO k-major, 2 = dO mn-major, 3 = Q mn-major
-  const int tile_off[4] = {KV_QK, KV_DOK, KV_DOM, KV_QM};
+  const uint32_t tmem = *s_tmem;
+  constexpr uint32_t T_DV = 384, T_DK = 448;
 
   if (warp == 0) {
-    // ---------------------------------------------------------------- TMA producer ---
+    // ---------------------------------------------------------------- producer ---
     if (lane == 0 && nqb > 0) {
-      mbar_arrive_expect_tx(bar(F_VFULL), 32768u);
+      mbar_arrive_expect_tx(bar(B_KV), (uint32_t)(4 * NP * TILE));
 #pragma unroll
-      for (int c = 0; c < 4; ++c) tma_load_2d(sb + KV_VHI + c * 8192, &tmV, h * HD + 16 * c, (int)(b * D.Lk + j0), bar(F_VFULL));
-      bool ok = true;
-      for (int i = 0; i < nqb && ok; ++i) {
-        const int qrow = (int)(b * D.Lq + (int64_t)(ib0 + i) * KT);
-        const uint32_t ph = (uint32_t)(i - 1) & 1u;
+      for (int p = 0; p < NP; ++p)
 #pragma unroll
-        for (int t = 0; t < 4; ++t) {
-          if (i > 0 && !mbar_wait(bar(F_FREE + t), ph, s_abort)) { ok = false; break; }
-          mbar_arrive_expect_tx(bar(F_FULL + t), 16384u);
-          const uint32_t dst = sb + (uint32_t)tile_off[t];
-          if (t == 0) {
-            for (int c = 0; c < 4; ++c) tma_load_2d(dst + c * 4096, &tmQ, h * HD + 16 * c, qrow, bar(F_FULL + t));
-          } else if (t == 1) {
-            for (int c = 0; c < 4; ++c) tma_load_2d(dst + c * 4096, &tmDO, h * HD + 16 * c, qrow, bar(F_FULL + t));
-          } else if (t == 2) {
-            tma_load_3d(dst, &tmDOmn, 0, qrow, 2 * h, bar(F_FULL + t));
-          } else {
-            tma_load_3d(dst, &tmQmn, 0, qrow, 2 * h, bar(F_FULL + t));
-          }
+        for (int t = 0; t < 2; ++t) {   // plane p of the CTA's two 64-key tiles, one after the other
+          const int64_t off = ((bh * D.ktiles + 2 * (int64_t)blockIdx.x + t) * NP + p) * (int64_t)TILE;
+          bulk_load(sb + (uint32_t)(cfg::K_OFF + (2 * p + t) * TILE), kimg + off, TILE, bar(B_KV));
+          bulk_load(sb + (uint32_t)(cfg::V_OFF + (2 * p + t) * TILE), vimg + off, TILE, bar(B_KV));
         }
+      for (int n = 0; n < 2 * nqb; ++n) {
+        const int s = n % S;
+        if (n >= S && !mbar_wait(bar(B_FREE + s), (uint32_t)(n / S - 1) & 1u, s_abort)) break;
+        const bool is_do = (n & 1) == 0;
+        const int64_t tile = bh * D.qtiles + ib0 + (n >> 1);
+        const uint32_t dst = sb + (uint32_t)(s * cfg::SLOT_BYTES);
+        mbar_arrive_expect_tx(bar(B_FULL + s), (uint32_t)(NP * TILE + (is_do ? 512 : 0)));
+        bulk_load(dst, (is_do ? doimg : qimg) + tile * (int64_t)(NP * TILE), NP * TILE, bar(B_FULL + s));
+        if (is_do) bulk_load(dst + NP * TILE, rv + tile * KT, 512u, bar(B_FULL + s));
       }
     }
   } else if (warp == 1) {
-    // ------------------------------------------------------------------ MMA issuer ---
+    // -------------------------------------------------------------- MMA issuer ---
     if (lane == 0 && nqb > 0) {
-      const uint32_t idesc_kk = (1u << 4) | (2u << 7) | (2u << 10) | ((uint32_t)(KT >> 3) << 17) | ((uint32_t)(QT >> 4) << 24);
-      const uint32_t idesc_mn = idesc_kk | (1u << 16);
-      const uint32_t t_k = tmem_base, t_p = tmem_base + 128u, t_ds = tmem_base + 256u, t_dv = tmem_base + 384u, t_dk = tmem_base + 448u;
-      const uint64_t dv_hi = make_smem_desc(sb + KV_VHI, 16, 512, LAYOUT_SW64), dv_lo = make_smem_desc(sb + KV_VLO, 16, 512, LAYOUT_SW64);
-      const uint64_t dqk_hi = make_smem_desc(sb + KV_QK, 16, 512, LAYOUT_SW64), dqk_lo = make_smem_desc(sb + KV_QK + 16384, 16, 512, LAYOUT_SW64);
-      const uint64_t dok_hi = make_smem_desc(sb + KV_DOK, 16, 512, LAYOUT_SW64), dok_lo = make_smem_desc(sb + KV_DOK + 16384, 16, 512, LAYOUT_SW64);
-      const uint64_t dom_hi = make_smem_desc(sb + KV_DOM, KT * 128, 512, LAYOUT_SW128_32B), dom_lo = make_smem_desc(sb + KV_DOM + 16384, KT * 128, 512, LAYOUT_SW128_32B);
-      const uint64_t dqm_hi = make_smem_desc(sb + KV_QM, KT * 128, 512, LAYOUT_SW128_32B), dqm_lo = make_smem_desc(sb + KV_QM + 16384, KT * 128, 512, LAYOUT_SW128_32B);
-      bool ok = mbar_wait(bar(F_KREADY), 0u, s_abort) && mbar_wait(bar(F_VREADY), 0u, s_abort);
-      for (int i = 0; i < nqb && ok; ++i) {
-        const uint32_t ph = (uint32_t)i & 1u;
-        ok = mbar_wait(bar(F_READY + 0), ph, s_abort) && mbar_wait(bar(F_READY + 1), ph, s_abort);
-        if (!ok) break;
-        tc_fence_after();
-#pragma unroll
-        for (int ks = 0; ks < 8; ++ks) {   // S' = K Q' over the 64 features
-          const uint64_t bo = (uint64_t)(((ks >> 1) * 4096 + (ks & 1) * 32) >> 4);
-          const uint32_t ao = (uint32_t)(8 * ks);
-          tc_mma_tf32_ta(t_p, t_k + 64u + ao, dqk_hi + bo, idesc_kk, ks > 0 ? 1u : 0u);
-          tc_mma_tf32_ta(t_p, t_k + ao, dqk_lo + bo, idesc_kk, 1u);
-          tc_mma_tf32_ta(t_p, t_k + ao, dqk_hi + bo, idesc_kk, 1u);
+      const int nd = (D.d + 15) & ~15, nv = (D.dv + 15) & ~15;
+      auto slot = [&](int n) { return sb + (uint32_t)((n % S) * cfg::SLOT_BYTES); };
+      auto full = [&](int n) { return mbar_wait(bar(B_FULL + n % S), (uint32_t)(n / S) & 1u, s_abort); };
+      bool ok = mbar_wait(bar(B_KV), 0u, s_abort);
+      // step i: S' and dP' of block i + 2 (i >= -2) behind dV and dK of block i, whose planes they overwrite
+#pragma unroll 1
+      for (int i = -2; i < nqb && ok; ++i) {
+        if (i >= 0) {
+          ok = mbar_wait(bar(B_PREADY + (i & 1)), (uint32_t)(i >> 1) & 1u, s_abort);
+          if (!ok) break;
+          tc_fence_after();
+          const uint32_t r = tmem + (uint32_t)(192 * (i & 1));
+          mma_planes<NP>(tmem + T_DV, r, r + 128u, 32u, slot(2 * i), nv, i > 0);
+          tc_commit(bar(B_FREE + (2 * i) % S));
+          mma_planes<NP>(tmem + T_DK, r + 64u, r + 144u, 32u, slot(2 * i + 1), nd, i > 0);
+          tc_commit(bar(B_FREE + (2 * i + 1) % S));
+          if (i == nqb - 1) tc_commit(bar(B_DONE));
         }
-        tc_commit(bar(F_FREE + 0));
-#pragma unroll
-        for (int ks = 0; ks < 8; ++ks) {   // dP' = V dO' over the 64 value features (A = V from shared memory)
-          const uint64_t ao = (uint64_t)(((ks >> 1) * 8192 + (ks & 1) * 32) >> 4), bo = (uint64_t)(((ks >> 1) * 4096 + (ks & 1) * 32) >> 4);
-          tc_mma_tf32(t_ds, dv_lo + ao, dok_hi + bo, idesc_kk, ks > 0 ? 1u : 0u);
-          tc_mma_tf32(t_ds, dv_hi + ao, dok_lo + bo, idesc_kk, 1u);
-          tc_mma_tf32(t_ds, dv_hi + ao, dok_hi + bo, idesc_kk, 1u);
+        const int t = i + 2;
+        if (t < nqb) {
+          const uint32_t r = tmem + (uint32_t)(192 * (t & 1));
+          ok = full(2 * t);
+          if (!ok) break;
+          tc_fence_after();
+          mma_rows_s<NP>(r + 64u, sb + cfg::V_OFF, slot(2 * t));
+          ok = full(2 * t + 1);
+          if (!ok) break;
+          tc_fence_after();
+          mma_rows_s<NP>(r, sb + cfg::K_OFF, slot(2 * t + 1));
+          tc_commit(bar(B_SFULL + (t & 1)));
         }
-        tc_commit(bar(F_FREE + 1));
-        tc_commit(bar(F_SFULL));
-        ok = mbar_wait(bar(F_PREADY), ph, s_abort) && mbar_wait(bar(F_READY + 2), ph, s_abort) && mbar_wait(bar(F_READY + 3), ph, s_abort);
-        if (!ok) break;
-        tc_fence_after();
-#pragma unroll
-        for (int ks = 0; ks < 8; ++ks) {   // dV += P' dO over the 64 queries
-          const uint64_t bo = (uint64_t)((ks * 1024) >> 4);
-          const uint32_t ao = (uint32_t)(8 * ks);
-          tc_mma_tf32_ta(t_dv, t_p + 64u + ao, dom_hi + bo, idesc_mn, (i > 0 || ks > 0) ? 1u : 0u);
-          tc_mma_tf32_ta(t_dv, t_p + ao, dom_lo + bo, idesc_mn, 1u);
-          tc_mma_tf32_ta(t_dv, t_p + ao, dom_hi + bo, idesc_mn, 1u);
-        }
-        tc_commit(bar(F_FREE + 2));
-#pragma unroll
-        for (int ks = 0; ks < 8; ++ks) {   // dK += dS' Q over the 64 queries
-          const uint64_t bo = (uint64_t)((ks * 1024) >> 4);
-          const uint32_t ao = (uint32_t)(8 * ks);
-          tc_mma_tf32_ta(t_dk, t_ds + 64u + ao, dqm_hi + bo, idesc_mn, (i > 0 || ks > 0) ? 1u : 0u);
-          tc_mma_tf32_ta(t_dk, t_ds + ao, dqm_lo + bo, idesc_mn, 1u);
-          tc_mma_tf32_ta(t_dk, t_ds + ao, dqm_hi + bo, idesc_mn, 1u);
-        }
-        tc_commit(bar(F_FREE + 3));
-        if (i == nqb - 1) tc_commit(bar(F_DONE));
-      }
-    }
-  } else if (warp < 6) {
-    // ------------------------------------------------------------------ compute warps ---
-    const int qd = warp & 3;
-    const int row = 32 * qd + lane;
-    const int64_t kj = j0 + row;             // this thread's key
-    const bool live = kj < D.Lk;
-    const uint32_t t_row = tmem_base + ((uint32_t)(32 * qd) << 16);
-    if (nqb > 0) {
-      // K row of this thread into tensor memory: the raw value is the hi operand, lo = x - tf32(x)
-      const float* src = k + (b * D.Lk + kj) * D.E + (int64_t)h * HD;
-#pragma unroll
-      for (int half = 0; half < 2; ++half) {
-        uint32_t hi[32], lo[32];
-#pragma unroll
-        for (int c4 = 0; c4 < 8; ++c4) {
-          float4 x = make_float4(0.f, 0.f, 0.f, 0.f);
-          if (live) x = __ldg((const float4*)(src + 32 * half + 4 * c4));
-          hi[4 * c4] = __float_as_uint(x.x); hi[4 * c4 + 1] = __float_as_uint(x.y);
-          hi[4 * c4 + 2] = __float_as_uint(x.z); hi[4 * c4 + 3] = __float_as_uint(x.w);
-          lo[4 * c4] = __float_as_uint(tf32_lo(x.x)); lo[4 * c4 + 1] = __float_as_uint(tf32_lo(x.y));
-          lo[4 * c4 + 2] = __float_as_uint(tf32_lo(x.z)); lo[4 * c4 + 3] = __float_as_uint(tf32_lo(x.w));
-        }
-        tc_st_32x32b_x32(t_row + (uint32_t)(32 * half), hi);
-        tc_st_32x32b_x32(t_row + (uint32_t)(64 + 32 * half), lo);
-      }
-      tc_wait_st();
-      tc_fence_before();
-      __syncwarp();
-      if (lane == 0) mbar_arrive(bar(F_KREADY));
-    }
-    bool ok = true;
-    for (int i = 0; i < nqb && ok; ++i) {
-      const int64_t i0b = (int64_t)(ib0 + i) * KT;   // first query of the block
-      const float* rv = rowv + (i & 1) * 128;
-      ok = mbar_wait(bar(F_SFULL), (uint32_t)i & 1u, s_abort);
-      if (!ok) break;
-      tc_fence_after();
-      // queries of the block this key is seen by: query < Lq (dead ones carry lse = +inf), and query >= key when causal
-      int clo = 0;
-      if (D.causal && kj - i0b > 0) clo = (kj - i0b) > KT ? KT : (int)(kj - i0b);
-      if (!live) clo = KT;
-#pragma unroll
-      for (int half = 0; half < 2; ++half) {
-        uint32_t sv[32], dp[32], lo[32];
-        tc_ld_32x32b_x32(t_row + 128u + (uint32_t)(32 * half), sv);
-        tc_ld_32x32b_x32(t_row + 256u + (uint32_t)(32 * half), dp);
-        tc_wait_ld();
-#pragma unroll
-        for (int c = 0; c < 32; ++c) {
-          const int cq = c + 32 * half;
-          float p = fast_exp2(fmaf(__uint_as_float(sv[c]), D.scale_log2, -rv[cq]));
-          if (cq < clo) p = 0.0f;
-          const float ds = p * (__uint_as_float(dp[c]) - rv[64 + cq]);
-          sv[c] = __float_as_uint(p);
-          lo[c] = __float_as_uint(tf32_lo(p));
-          dp[c] = __float_as_uint(ds);
-        }
-        tc_st_32x32b_x32(t_row + 128u + (uint32_t)(32 * half), sv);
-        tc_st_32x32b_x32(t_row + 192u + (uint32_t)(32 * half), lo);
-#pragma unroll
-        for (int c = 0; c < 32; ++c) lo[c] = __float_as_uint(tf32_lo(__uint_as_float(dp[c])));
-        tc_st_32x32b_x32(t_row + 256u + (uint32_t)(32 * half), dp);
-        tc_st_32x32b_x32(t_row + 320u + (uint32_t)(32 * half), lo);
-      }
-      tc_wait_st();
-      tc_fence_before();
-      __syncwarp();
-      if (lane == 0) mbar_arrive(bar(F_PREADY));
-    }
-    if (nqb > 0) {
-      if (ok) ok = mbar_wait(bar(F_DONE), 0u, s_abort);
-      if (ok) {
-        tc_fence_after();
-#pragma unroll
-        for (int w = 0; w < 2; ++w) {   // 0: dV, 1: dK (scaled by 1 / sqrt(d))
-          uint32_t r0[32], r1[32];
-          tc_ld_32x32b_x32(t_row + 384u + (uint32_t)(64 * w), r0);
-          tc_ld_32x32b_x32(t_row + 416u + (uint32_t)(64 * w), r1);
-          tc_wait_ld();
-          if (live) {
-            const float sc = w == 0 ? 1.0f : D.scale;
-            float* drow = (w == 0 ? dv + (b * D.Lk + kj) * D.Ev : dk + (b * D.Lk + kj) * D.E) + (int64_t)h * HD;
-#pragma unroll
-            for (int c = 0; c < 32; c += 4) {
-              *(float4*)(drow + c) = make_float4(__uint_as_float(r0[c]) * sc, __uint_as_float(r0[c + 1]) * sc,
-                                                 __uint_as_float(r0[c + 2]) * sc, __uint_as_float(r0[c + 3]) * sc);
-              *(float4*)(drow + 32 + c) = make_float4(__uint_as_float(r1[c]) * sc, __uint_as_float(r1[c + 1]) * sc,
-                                                      __uint_as_float(r1[c + 2]) * sc, __uint_as_float(r1[c + 3]) * sc);
-            }
-          }
-        }
-      }
-    } else if (live) {
-      // no query sees these keys: their gradients are zero
-      float* r1 = dv + (b * D.Lk + kj) * D.Ev + (int64_t)h * HD;
-      float* r2 = dk + (b * D.Lk + kj) * D.E + (int64_t)h * HD;
-#pragma unroll
-      for (int c = 0; c < HD; c += 4) {
-        *(float4*)(r1 + c) = make_float4(0.f, 0.f, 0.f, 0.f);
-        *(float4*)(r2 + c) = make_float4(0.f, 0.f, 0.f, 0.f);
       }
     }
   } else {
-    // --------------------------------- split warps: lo twins, and the per-query lse / delta of each block ---
-    const int tt = (warp - 6) * 32 + lane;
-    auto split = [&](int off, int n16) {
-      const float4* hi = (const float4*)(smem + off);
-      float4* lo = (float4*)(smem + off + (n16 == 16 ? 32768 : 16384));
-      for (int i = 0; i < n16; ++i) {
-        float4 v = hi[tt + i * 128];
-        v.x = tf32_lo(v.x); v.y = tf32_lo(v.y); v.z = tf32_lo(v.z); v.w = tf32_lo(v.w);
-        lo[tt + i * 128] = v;
+    // ------------------------------------------------------------ compute warps ---
+    const int set = (warp - 2) >> 2, qd = warp & 3;
+    const int64_t kj = j0 + 32 * qd + lane;   // this thread's key
+    const bool live = kj < D.Lk;
+    const uint32_t t_row = tmem + ((uint32_t)(32 * qd) << 16);
+    const int64_t el = NP == 3 ? 4 : 2;
+    bool ok = true;
+    for (int i = set; i < nqb && ok; i += 2) {
+      const int n = 2 * i;
+      ok = mbar_wait(bar(B_FULL + n % S), (uint32_t)(n / S) & 1u, s_abort) && mbar_wait(bar(B_SFULL + set), (uint32_t)(i >> 1) & 1u, s_abort);
+      if (!ok) break;
+      tc_fence_after();
+      const float4* row = (const float4*)(sh.smem + (n % S) * cfg::SLOT_BYTES + NP * TILE);   // {lse, delta} of two queries
+      // queries of the block this key is seen by: query < Lq (dead ones carry lse = inf), and query >= key when causal
+      const int64_t i0b = (int64_t)(ib0 + i) * KT;
+      int clo = 0;
+      if (D.causal && kj - i0b > 0) clo = (kj - i0b) > KT ? KT : (int)(kj - i0b);
+      if (!live) clo = KT;
+      const uint32_t r = t_row + (uint32_t)(192 * set);
+#pragma unroll
+      for (int hf = 0; hf < 2; ++hf) {
+        uint32_t sv[32], dp[32];
+        tc_ld_32x32b_x32(r + 32u * hf, sv);
+        tc_ld_32x32b_x32(r + 64u + 32u * hf, dp);
+        tc_wait_ld();
+#pragma unroll
+        for (int c = 0; c < 32; c += 2) {
+          const float4 w = row[16 * hf + (c >> 1)];
+          float p0 = fast_exp2(fmaf(__uint_as_float(sv[c]), D.scale_log2, -w.x));
+          float p1 = fast_exp2(fmaf(__uint_as_float(sv[c + 1]), D.scale_log2, -w.z));
+          if (c + 32 * hf < clo) p0 = 0.0f;
+          if (c + 1 + 32 * hf < clo) p1 = 0.0f;
+          sv[c] = __float_as_uint(p0);
+          sv[c + 1] = __float_as_uint(p1);
+          dp[c] = __float_as_uint(p0 * (__uint_as_float(dp[c]) - w.y));
+          dp[c + 1] = __float_as_uint(p1 * (__uint_as_float(dp[c + 1]) - w.w));
+        }
+        // over columns this thread has read already; the third planes lie behind both
+        store_planes32(r + 32u * hf, r + 32u * hf + 16u, r + 128u + 32u * hf, sv);
+        store_planes32(r + 64u + 32u * hf, r + 80u + 32u * hf, r + 144u + 32u * hf, dp);
       }
-    };
-    bool ok = nqb > 0;
-    if (ok) ok = mbar_wait(bar(F_VFULL), 0u, s_abort);
-    if (ok) {
-      split(KV_VHI, 16);
-      fence_proxy_async();
+      tc_wait_st();
+      tc_fence_before();
       __syncwarp();
-      if (lane == 0) mbar_arrive(bar(F_VREADY));
+      if (lane == 0) mbar_arrive(bar(B_PREADY + set));
     }
-    for (int i = 0; i < nqb && ok; ++i) {
-      const uint32_t ph = (uint32_t)i & 1u;
-      // lse * log2(e) and delta of the block's queries (set i & 1: the compute warps may still read the other set)
-      if (tt < KT) {
-        const int64_t gq = (int64_t)(ib0 + i) * KT + tt;
-        float* rv = rowv + (i & 1) * 128;
-        rv[tt] = gq < D.Lq ? lse[(b * D.H + h) * D.Lq + gq] * 1.4426950408889634f : INFINITY;
-        rv[64 + tt] = gq < D.Lq ? dlt[(b * D.H + h) * D.Lq + gq] : 0.0f;
-      }
-#pragma unroll 1
-      for (int t = 0; t < 4 && ok; ++t) {
-        ok = mbar_wait(bar(F_FULL + t), ph, s_abort);
-        if (!ok) break;
-        split(tile_off[t], 8);
-        fence_proxy_async();
-        __syncwarp();
-        if (lane == 0) mbar_arrive(bar(F_READY + t));
+    // the first set writes dV, the second dK (scaled by 1 / sqrt(d)); zero where no query sees the keys
+    if (ok && nqb > 0) ok = mbar_wait(bar(B_DONE), 0u, s_abort);
+    if (ok) {
+      tc_fence_after();
+      uint8_t* drow = set == 0 ? (uint8_t*)dv + el * ((b * D.Lk + kj) * D.Ev + (int64_t)h * D.dv)
+                               : (uint8_t*)dk + el * ((b * D.Lk + kj) * D.E + (int64_t)h * D.d);
+#pragma unroll
+      for (int hf = 0; hf < 2; ++hf) {
+        uint32_t v[32];
+        if (nqb > 0) {
+          tc_ld_32x32b_x32(t_row + (set == 0 ? T_DV : T_DK) + 32u * hf, v);
+          tc_wait_ld();
+        } else {
+#pragma unroll
+          for (int c = 0; c < 32; ++c) v[c] = 0u;
+        }
+        if (live) store_row32<NP == 1>(drow, 32 * hf, set == 0 ? D.dv : D.d, D.vec != 0, (const float*)v, set == 0 ? 1.0f : D.scale);
       }
     }
   }
@@ -924,123 +936,150 @@ attn_bwd_dkdv_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_co
   __syncthreads();
   if (warp == 1) {
     __syncwarp();
-    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(512u) : "memory");
+    tmem_free(tmem, 512u);
   }
   if (threadIdx.x == 0 && *s_abort != 0) atomicExch(dev_err, 4004);
 }
 
-// FLUXB200_ATTN_TC = 0 keeps attention on the Float32 FMA kernels.
+// ------------------------------------------------------------------------------------------------------- host side ---
+// FLUXB200_ATTN_TC = 0 keeps attention on the Float32 FMA kernels, FLUXB200_ATTN_BWD_TC = 0 its backward pass.
+bool env_on(const char* name) {
+  const char* e = getenv(name);
+  return !(e != nullptr && e[0] == '0');
+}
 bool attn_tc_enabled() {
-  static int on = -1;
-  if (on < 0) {
-    const char* e = getenv("FLUXB200_ATTN_TC");
-    on = (e != nullptr && e[0] == '0') ? 0 : 1;
-  }
-  return on != 0;
+  static const bool on = env_on("FLUXB200_ATTN_TC");
+  return on;
 }
-
-// FLUXB200_ATTN_BWD_TC = 0 keeps the backward pass on the Float32 FMA kernels.
 bool attn_bwd_tc_enabled() {
-  static int on = -1;
-  if (on < 0) {
-    const char* e = getenv("FLUXB200_ATTN_BWD_TC");
-    on = (e != nullptr && e[0] == '0') ? 0 : 1;
-  }
-  return on != 0;
+  static const bool on = env_on("FLUXB200_ATTN_BWD_TC");
+  return on;
 }
 
-// 3-d view {32, rows, cols / 32} of a row-major [rows][cols] matrix whose rows are the K dimension of an MN-major
-// operand: box {32, box_rows, chunks}.
-bool encode_rows3d(CUtensorMap* map, const float* base, int64_t rows, int64_t cols, uint32_t box_rows, uint32_t chunks) {
-  EncodeTiledFn fn = get_encode_fn();
-  if (!fn || cols % 32 != 0) return false;
-  cuuint64_t gdim[3] = {32, (cuuint64_t)rows, (cuuint64_t)(cols / 32)};
-  cuuint64_t gstride[2] = {(cuuint64_t)cols * sizeof(float), 128};
-  cuuint32_t box[3] = {32, box_rows, chunks};
-  cuuint32_t estr[3] = {1, 1, 1};
-  CUresult r = fn(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 3, (void*)base, gdim, gstride, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
-                  CU_TENSOR_MAP_SWIZZLE_128B_ATOM_32B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-  return r == CUDA_SUCCESS;
+// plane images of one call take at most this much scratch memory unless one batch entry needs more: a call is cut along
+// the batch otherwise
+constexpr int64_t IMAGE_BYTES = (int64_t)512 << 20;
+
+struct AtcPlan {
+  AtcDims D;
+  int64_t qbytes, kbytes;   // image of one batch entry's Q (dO), K (V)
+  int64_t rvbytes;
+};
+
+bool make_plan(AtcPlan* P, int np, int64_t e_dim, int64_t ev_dim, int64_t lq, int64_t lk, int64_t batch, int nheads, int causal) {
+  if (nheads < 1 || lq < 1 || lk < 1 || batch < 1 || batch > 65535 || nheads > 65535) return false;
+  const int64_t d = e_dim / nheads, dv = ev_dim / nheads;
+  if (d < 1 || dv < 1 || d > HD || dv > HD) return false;
+  if (np == 1 && (d % 8 != 0 || dv % 8 != 0)) return false;
+  if (lq > 0x3fffff00 || lk > 0x3fffff00) return false;
+  AtcDims& D = P->D;
+  D.E = e_dim; D.Ev = ev_dim; D.Lq = lq; D.Lk = lk; D.H = nheads; D.causal = causal ? 1 : 0;
+  D.d = (int)d; D.dv = (int)dv;
+  D.qtiles = (int)((lq + QT - 1) / QT) * 2;
+  D.ktiles = (int)((lk + QT - 1) / QT) * 2;
+  D.vec = (d % 4 == 0 && dv % 4 == 0) ? 1 : 0;   // with 16-byte aligned arrays every row of a head is 16-byte aligned
+  D.scale = 1.0f / sqrtf((float)d);
+  D.scale_log2 = D.scale * LOG2E;
+  P->qbytes = (int64_t)nheads * D.qtiles * np * TILE;
+  P->kbytes = (int64_t)nheads * D.ktiles * np * TILE;
+  P->rvbytes = (int64_t)nheads * D.qtiles * KT * (int64_t)sizeof(float2);
+  return true;
+}
+
+template <int NP>
+int32_t fwd_impl(fb_ctx* ctx, cudaStream_t stream, const uint8_t* q, const uint8_t* k, const uint8_t* v, float* o, uint16_t* o16, float* lse,
+                 const AtcPlan& P, int64_t batch) {
+  const AtcDims& D = P.D;
+  const int64_t el = NP == 3 ? 4 : 2, per = 2 * P.kbytes;
+  int64_t chunk = IMAGE_BYTES / per;
+  chunk = chunk < 1 ? 1 : (chunk > batch ? batch : chunk);
+  uint8_t* img = (uint8_t*)fb_pack_scratch(ctx, stream, (size_t)(chunk * per));
+  if (!img) return FB_ERR_UNSUPPORTED;
+  FB_CUDA(cudaFuncSetAttribute(attn_fwd_tc_kernel<NP>, cudaFuncAttributeMaxDynamicSharedMemorySize, FwdCfg<NP>::SMEM));
+  for (int64_t b0 = 0; b0 < batch; b0 += chunk) {
+    const int64_t nb = b0 + chunk > batch ? batch - b0 : chunk;
+    SplitArgs A = {};
+    A.H = D.H; A.vec = D.vec;
+    A.job[0] = {k + el * b0 * D.Lk * D.E, img, D.Lk, D.E, D.d, D.ktiles};
+    A.job[1] = {v + el * b0 * D.Lk * D.Ev, img + nb * P.kbytes, D.Lk, D.Ev, D.dv, D.ktiles};
+    attn_split_kernel<NP><<<dim3((unsigned)D.ktiles, (unsigned)(nb * D.H), 2), 256, 0, stream>>>(A);
+    FB_LAUNCH_CHECK();
+    attn_fwd_tc_kernel<NP><<<dim3((unsigned)(D.qtiles / 2), (unsigned)D.H, (unsigned)nb), FWD_THREADS, FwdCfg<NP>::SMEM, stream>>>(
+        q + el * b0 * D.Lq * D.E, img, img + nb * P.kbytes, o ? o + b0 * D.Lq * D.Ev : nullptr, o16 ? o16 + b0 * D.Lq * D.Ev : nullptr,
+        lse + b0 * D.H * D.Lq, D, ctx->dev_error);
+    FB_LAUNCH_CHECK();
+  }
+  return FB_OK;
+}
+
+template <int NP>
+int32_t bwd_impl(fb_ctx* ctx, cudaStream_t stream, const uint8_t* q, const uint8_t* k, const uint8_t* v, const float* o, const float* lse,
+                 const uint8_t* dout, uint8_t* dq, uint8_t* dk, uint8_t* dv, const AtcPlan& P, int64_t batch, bool do_kv, bool do_q) {
+  const AtcDims& D = P.D;
+  const int64_t el = NP == 3 ? 4 : 2, per = 2 * P.kbytes + 2 * P.qbytes + P.rvbytes;
+  int64_t chunk = IMAGE_BYTES / per;
+  chunk = chunk < 1 ? 1 : (chunk > batch ? batch : chunk);
+  uint8_t* img = (uint8_t*)fb_pack_scratch(ctx, stream, (size_t)(chunk * per));
+  if (!img) return FB_ERR_UNSUPPORTED;
+  FB_CUDA(cudaFuncSetAttribute(attn_bwd_dkdv_tc_kernel<NP>, cudaFuncAttributeMaxDynamicSharedMemorySize, KvCfg<NP>::SMEM));
+  FB_CUDA(cudaFuncSetAttribute(attn_bwd_dq_tc_kernel<NP>, cudaFuncAttributeMaxDynamicSharedMemorySize, DqCfg<NP>::SMEM));
+  for (int64_t b0 = 0; b0 < batch; b0 += chunk) {
+    const int64_t nb = b0 + chunk > batch ? batch - b0 : chunk;
+    uint8_t *ki = img, *vi = ki + nb * P.kbytes, *qi = vi + nb * P.kbytes, *doi = qi + nb * P.qbytes;
+    float2* rv = (float2*)(doi + nb * P.qbytes);
+    const int64_t qoff = b0 * D.Lq * D.E, qvoff = b0 * D.Lq * D.Ev, koff = b0 * D.Lk * D.E, kvoff = b0 * D.Lk * D.Ev;
+    SplitArgs A = {};
+    A.H = D.H; A.vec = D.vec;
+    A.job[0] = {k + el * koff, ki, D.Lk, D.E, D.d, D.ktiles};
+    A.job[1] = {v + el * kvoff, vi, D.Lk, D.Ev, D.dv, D.ktiles};
+    A.job[2] = {q + el * qoff, qi, D.Lq, D.E, D.d, D.qtiles};
+    A.job[3] = {dout + el * qvoff, doi, D.Lq, D.Ev, D.dv, D.qtiles};
+    A.o = o + qvoff; A.lse = lse + b0 * D.H * D.Lq; A.rv = rv;
+    const int tiles = D.ktiles > D.qtiles ? D.ktiles : D.qtiles;
+    attn_split_kernel<NP><<<dim3((unsigned)tiles, (unsigned)(nb * D.H), 4), 256, 0, stream>>>(A);
+    FB_LAUNCH_CHECK();
+    if (do_kv) attn_bwd_dkdv_tc_kernel<NP><<<dim3((unsigned)(D.ktiles / 2), (unsigned)D.H, (unsigned)nb), BWD_THREADS, KvCfg<NP>::SMEM, stream>>>(
+        qi, doi, ki, vi, rv, dk + el * koff, dv + el * kvoff, D, ctx->dev_error);
+    FB_LAUNCH_CHECK();
+    if (do_q) attn_bwd_dq_tc_kernel<NP><<<dim3((unsigned)(D.qtiles / 2), (unsigned)D.H, (unsigned)nb), BWD_THREADS, DqCfg<NP>::SMEM, stream>>>(
+        q + el * qoff, dout + el * qvoff, ki, vi, rv, dq + el * qoff, D, ctx->dev_error);
+    FB_LAUNCH_CHECK();
+  }
+  return FB_OK;
 }
 
 }  // namespace
 
-// Returns FB_ERR_UNSUPPORTED when the shape is not one this kernel takes (the caller then uses the FMA kernels).
+// Both return FB_ERR_UNSUPPORTED when the call is not one these kernels take (the caller then uses the FMA kernels).
 int32_t fb_attn_fwd_tc(fb_ctx* ctx, cudaStream_t stream, const float* q, const float* k, const float* v, const uint8_t* mask,
                        float* o, float* lse, int64_t e_dim, int64_t ev_dim, int64_t lq, int64_t lk, int64_t batch, int nheads,
                        int causal) {
-  if (!attn_tc_enabled() || mask != nullptr || nheads < 1) return FB_ERR_UNSUPPORTED;
-  if (e_dim != (int64_t)nheads * HD || ev_dim != (int64_t)nheads * HD) return FB_ERR_UNSUPPORTED;
-  if (lq < 1 || lk < 1 || batch < 1 || batch * lq > 0x7fffff00 || batch * lk > 0x7fffff00 || batch > 65535 || nheads > 65535)
-    return FB_ERR_UNSUPPORTED;
-  if (!fb_aligned16(q) || !fb_aligned16(k) || !fb_aligned16(v) || !fb_aligned16(o)) return FB_ERR_UNSUPPORTED;
-  CUtensorMap tmK, tmV;
-  if (!encode_map(&tmK, k, batch * lk, e_dim, e_dim, 16, KT, CU_TENSOR_MAP_SWIZZLE_64B) ||
-      !encode_rows3d(&tmV, v, batch * lk, ev_dim, KT, HD / 32))
-    return FB_ERR_UNSUPPORTED;
-  AtcDims D;
-  D.E = e_dim; D.Ev = ev_dim; D.Lq = lq; D.Lk = lk; D.H = nheads; D.causal = causal ? 1 : 0;
-  D.scale = 1.0f / sqrtf((float)HD);
-  D.scale_log2 = D.scale * 1.4426950408889634f;
-  dim3 grid((unsigned)((lq + QT - 1) / QT), (unsigned)nheads, (unsigned)batch);
-  FB_CUDA(cudaFuncSetAttribute(attn_fwd_tc2_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, ATC2_SMEM));
-  attn_fwd_tc2_kernel<<<grid, ATC_THREADS, ATC2_SMEM, stream>>>(q, tmK, tmV, o, lse, D, ctx->dev_error);
-  FB_LAUNCH_CHECK();
-  return FB_OK;
+  AtcPlan P;
+  if (!attn_tc_enabled() || mask != nullptr || !make_plan(&P, 3, e_dim, ev_dim, lq, lk, batch, nheads, causal)) return FB_ERR_UNSUPPORTED;
+  if (!fb_aligned16(q) || !fb_aligned16(k) || !fb_aligned16(v) || !fb_aligned16(o)) P.D.vec = 0;
+  return fwd_impl<3>(ctx, stream, (const uint8_t*)q, (const uint8_t*)k, (const uint8_t*)v, o, nullptr, lse, P, batch);
 }
 
-// dQ of the backward pass; FB_ERR_UNSUPPORTED when the shape is not one this kernel takes.
-int32_t fb_attn_bwd_dq_tc(fb_ctx* ctx, cudaStream_t stream, const float* q, const float* k, const float* v, const uint8_t* mask,
-                          const float* lse, const float* dlt, const float* dout, float* dq, int64_t e_dim, int64_t ev_dim,
-                          int64_t lq, int64_t lk, int64_t batch, int nheads, int causal) {
-  if (!attn_tc_enabled() || !attn_bwd_tc_enabled() || mask != nullptr || nheads < 1) return FB_ERR_UNSUPPORTED;
-  if (e_dim != (int64_t)nheads * HD || ev_dim != (int64_t)nheads * HD) return FB_ERR_UNSUPPORTED;
-  if (lq < 1 || lk < 1 || batch < 1 || batch * lq > 0x7fffff00 || batch * lk > 0x7fffff00 || batch > 65535 || nheads > 65535)
+// *did_kv, *did_q: which part was done.  dQ, dK and dV accumulate in tensor memory with truncating adds; beyond 2048 keys
+// (queries), and for the other head sizes, the FMA kernels are the more accurate ones.
+int32_t fb_attn_bwd_tc(fb_ctx* ctx, cudaStream_t stream, const float* q, const float* k, const float* v, const uint8_t* mask, const float* o,
+                       const float* lse, const float* dout, float* dq, float* dk, float* dv, int64_t e_dim, int64_t ev_dim, int64_t lq,
+                       int64_t lk, int64_t batch, int nheads, int causal, bool* did_kv, bool* did_q) {
+  AtcPlan P;
+  *did_kv = *did_q = false;
+  if (!attn_tc_enabled() || !attn_bwd_tc_enabled() || mask != nullptr || !make_plan(&P, 3, e_dim, ev_dim, lq, lk, batch, nheads, causal) ||
+      P.D.d != HD || P.D.dv != HD)
     return FB_ERR_UNSUPPORTED;
-  if ((lk + KT - 1) / KT > DQ_MAX_BLOCKS) return FB_ERR_UNSUPPORTED;   // dQ accumulates in tensor memory over <= 2048 keys
-  if (!fb_aligned16(q) || !fb_aligned16(k) || !fb_aligned16(v) || !fb_aligned16(dout) || !fb_aligned16(dq)) return FB_ERR_UNSUPPORTED;
-  CUtensorMap tmK, tmKmn, tmV;
-  if (!encode_map(&tmK, k, batch * lk, e_dim, e_dim, 16, KT, CU_TENSOR_MAP_SWIZZLE_64B) ||
-      !encode_rows3d(&tmKmn, k, batch * lk, e_dim, KT, HD / 32) ||
-      !encode_map(&tmV, v, batch * lk, ev_dim, ev_dim, 16, KT, CU_TENSOR_MAP_SWIZZLE_64B))
-    return FB_ERR_UNSUPPORTED;
-  AtcDims D;
-  D.E = e_dim; D.Ev = ev_dim; D.Lq = lq; D.Lk = lk; D.H = nheads; D.causal = causal ? 1 : 0;
-  D.scale = 1.0f / sqrtf((float)HD);
-  D.scale_log2 = D.scale * 1.4426950408889634f;
-  FB_CUDA(cudaFuncSetAttribute(attn_bwd_dq_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, DQ_SMEM));
-  dim3 grid((unsigned)((lq + QT - 1) / QT), (unsigned)nheads, (unsigned)batch);
-  attn_bwd_dq_tc_kernel<<<grid, ATC_THREADS, DQ_SMEM, stream>>>(tmK, tmKmn, tmV, q, dout, lse, dlt, dq, D, ctx->dev_error);
-  FB_LAUNCH_CHECK();
-  return FB_OK;
-}
-
-// dK and dV of the backward pass; FB_ERR_UNSUPPORTED when the shape is not one this kernel takes.
-int32_t fb_attn_bwd_dkdv_tc(fb_ctx* ctx, cudaStream_t stream, const float* q, const float* k, const float* v, const uint8_t* mask,
-                            const float* lse, const float* dlt, const float* dout, float* dk, float* dv, int64_t e_dim,
-                            int64_t ev_dim, int64_t lq, int64_t lk, int64_t batch, int nheads, int causal) {
-  if (!attn_tc_enabled() || !attn_bwd_tc_enabled() || mask != nullptr || nheads < 1) return FB_ERR_UNSUPPORTED;
-  if (e_dim != (int64_t)nheads * HD || ev_dim != (int64_t)nheads * HD) return FB_ERR_UNSUPPORTED;
-  if (lq < 1 || lk < 1 || batch < 1 || batch * lq > 0x7fffff00 || batch * lk > 0x7fffff00 || batch > 65535 || nheads > 65535)
-    return FB_ERR_UNSUPPORTED;
-  if ((lq + KT - 1) / KT > KV_MAX_BLOCKS) return FB_ERR_UNSUPPORTED;   // accumulation in tensor memory over <= 2048 queries
-  if (!fb_aligned16(q) || !fb_aligned16(k) || !fb_aligned16(v) || !fb_aligned16(dout) || !fb_aligned16(dk) || !fb_aligned16(dv))
-    return FB_ERR_UNSUPPORTED;
-  CUtensorMap tmQ, tmQmn, tmDO, tmDOmn, tmV;
-  if (!encode_map(&tmQ, q, batch * lq, e_dim, e_dim, 16, KT, CU_TENSOR_MAP_SWIZZLE_64B) ||
-      !encode_rows3d(&tmQmn, q, batch * lq, e_dim, KT, HD / 32) ||
-      !encode_map(&tmDO, dout, batch * lq, ev_dim, ev_dim, 16, KT, CU_TENSOR_MAP_SWIZZLE_64B) ||
-      !encode_rows3d(&tmDOmn, dout, batch * lq, ev_dim, KT, HD / 32) ||
-      !encode_map(&tmV, v, batch * lk, ev_dim, ev_dim, 16, QT, CU_TENSOR_MAP_SWIZZLE_64B))
-    return FB_ERR_UNSUPPORTED;
-  AtcDims D;
-  D.E = e_dim; D.Ev = ev_dim; D.Lq = lq; D.Lk = lk; D.H = nheads; D.causal = causal ? 1 : 0;
-  D.scale = 1.0f / sqrtf((float)HD);
-  D.scale_log2 = D.scale * 1.4426950408889634f;
-  FB_CUDA(cudaFuncSetAttribute(attn_bwd_dkdv_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, KV_SMEM));
-  dim3 grid((unsigned)((lk + QT - 1) / QT), (unsigned)nheads, (unsigned)batch);
-  attn_bwd_dkdv_tc_kernel<<<grid, ATC_THREADS, KV_SMEM, stream>>>(tmQ, tmQmn, tmDO, tmDOmn, tmV, k, lse, dlt, dk, dv, D,
-                                                                   ctx->dev_error);
-  FB_LAUNCH_CHECK();
-  return FB_OK;
+  const bool kv = lq <= BWD_MAX_BLOCKS * KT, qq = lk <= BWD_MAX_BLOCKS * KT;
+  if (!kv && !qq) return FB_ERR_UNSUPPORTED;
+  if (!fb_aligned16(q) || !fb_aligned16(k) || !fb_aligned16(v) || !fb_aligned16(o) || !fb_aligned16(dout) || !fb_aligned16(dq) ||
+      !fb_aligned16(dk) || !fb_aligned16(dv))
+    P.D.vec = 0;
+  const int32_t st = bwd_impl<3>(ctx, stream, (const uint8_t*)q, (const uint8_t*)k, (const uint8_t*)v, o, lse, (const uint8_t*)dout,
+                                 (uint8_t*)dq, (uint8_t*)dk, (uint8_t*)dv, P, batch, kv, qq);
+  if (st == FB_OK) {
+    *did_kv = kv;
+    *did_q = qq;
+  }
+  return st;
 }

@@ -234,16 +234,13 @@ int32_t fb_gemm_dispatch(fb_ctx* ctx, cudaStream_t stream, const fb_gemm_args& a
 void fb_gemm_workspace_destroy(fb_ctx* ctx);
 // clusters of `size` (2, 4, 8) CTAs that hold an SM each and are resident at once
 int fb_gemm_resident_clusters(fb_ctx* ctx, int size);
-// attention_tc.cu: tensor-core attention forward; FB_ERR_UNSUPPORTED when the shape is not taken
+// attention_tc.cu: tensor-core attention; FB_ERR_UNSUPPORTED when the call is not taken
 int32_t fb_attn_fwd_tc(fb_ctx* ctx, cudaStream_t stream, const float* q, const float* k, const float* v, const uint8_t* mask,
                        float* o, float* lse, int64_t e_dim, int64_t ev_dim, int64_t lq, int64_t lk, int64_t batch, int nheads,
                        int causal);
-int32_t fb_attn_bwd_dq_tc(fb_ctx* ctx, cudaStream_t stream, const float* q, const float* k, const float* v, const uint8_t* mask,
-                          const float* lse, const float* dlt, const float* dout, float* dq, int64_t e_dim, int64_t ev_dim,
-                          int64_t lq, int64_t lk, int64_t batch, int nheads, int causal);
-int32_t fb_attn_bwd_dkdv_tc(fb_ctx* ctx, cudaStream_t stream, const float* q, const float* k, const float* v, const uint8_t* mask,
-                            const float* lse, const float* dlt, const float* dout, float* dk, float* dv, int64_t e_dim,
-                            int64_t ev_dim, int64_t lq, int64_t lk, int64_t batch, int nheads, int causal);
+int32_t fb_attn_bwd_tc(fb_ctx* ctx, cudaStream_t stream, const float* q, const float* k, const float* v, const uint8_t* mask, const float* o,
+                       const float* lse, const float* dout, float* dq, float* dk, float* dv, int64_t e_dim, int64_t ev_dim, int64_t lq,
+                       int64_t lk, int64_t batch, int nheads, int causal, bool* did_kv, bool* did_q);
 int32_t fb_gemm_workspace_create(fb_ctx* ctx);
 // Kernels that run on a communication stream beside a resident GEMM CTA (update, peer exchange, time marks) ask for
 // the same shared-memory carve-out as the GEMM: an SM runs CTAs of different kernels together only when they agree

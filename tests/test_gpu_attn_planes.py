@@ -1,0 +1,60 @@
+"""Tensor-core attention (bf16 planes): head sizes, ragged tiles, unseen keys and slot / region reuse against float64."""
+import numpy as np
+import pytest
+
+torch = pytest.importorskip("torch")
+pytestmark = pytest.mark.gpu
+
+# (head size of q / k, of v, heads, Lq, Lk, batch, causal)
+CASES = [
+    (64, 64, 2, 128, 64, 2, 0), (64, 64, 1, 129, 65, 1, 1), (64, 64, 3, 1, 9, 2, 0), (64, 64, 1, 63, 300, 2, 0), (64, 64, 1, 700, 65, 1, 0),
+    (32, 32, 2, 200, 200, 2, 1), (20, 12, 2, 77, 130, 1, 0), (7, 5, 3, 70, 131, 2, 1), (1, 64, 1, 64, 64, 1, 0), (64, 16, 2, 127, 191, 1, 1),
+    (64, 64, 1, 100, 400, 1, 1),                                   # keys that no query sees
+    (64, 64, 1, 2048, 2112, 1, 0), (64, 64, 1, 2113, 2048, 1, 0),  # the longest accumulations, and one block more
+]
+
+
+def _reference(q, k, v, do, d, dv, heads, causal):
+    """out, dq, dk, dv in float64; arrays are [batch][len][heads * size]."""
+    q, k, v = (t.double().requires_grad_(True) for t in (q, k, v))
+    B, Lq, Lk = q.shape[0], q.shape[1], k.shape[1]
+    qh, kh, vh = q.view(B, Lq, heads, d).transpose(1, 2), k.view(B, Lk, heads, d).transpose(1, 2), v.view(B, Lk, heads, dv).transpose(1, 2)
+    s = qh @ kh.transpose(2, 3) / np.sqrt(d)
+    if causal:
+        s = s.masked_fill(torch.arange(Lk, device=s.device)[None, :] > torch.arange(Lq, device=s.device)[:, None], -np.inf)
+    out = (torch.softmax(s, -1) @ vh).transpose(1, 2).reshape(B, Lq, heads * dv)
+    out.backward(do.double())
+    return [t.detach() for t in (out, q.grad, k.grad, v.grad)]
+
+
+def _err(a, b):
+    return float((a.double() - b).norm() / b.norm().clamp_min(1e-30))
+
+
+@pytest.mark.parametrize("d,dv,heads,lq,lk,batch,causal", CASES)
+@pytest.mark.parametrize("shift", [0, 1])
+def test_attention_planes(d, dv, heads, lq, lk, batch, causal, shift):
+    """shift = 1: arrays that start 4 bytes past a 16-byte boundary."""
+    import fluxb200 as F
+    from fluxb200 import lib
+    g = torch.Generator(device="cuda")
+    g.manual_seed(lq * 7 + lk + d)
+
+    def arr(length, size, fill=True):
+        flat = torch.empty(batch * length * size + 4, device="cuda")
+        t = flat[shift:shift + batch * length * size].view(batch, length, size)
+        return t.normal_(generator=g) if fill else t.fill_(float("nan"))
+
+    q, k, v, do = arr(lq, heads * d), arr(lk, heads * d), arr(lk, heads * dv), arr(lq, heads * dv)
+    o, dq, dk, dvv = arr(lq, heads * dv, False), arr(lq, heads * d, False), arr(lk, heads * d, False), arr(lk, heads * dv, False)
+    lse = torch.empty(batch * heads * lq, device="cuda")
+    ctx = F.context()
+    p = [t.data_ptr() for t in (q, k, v)]
+    dims = (heads * d, heads * dv, lq, lk, batch, heads, causal)
+    lib.call("fb_attn_fwd", ctx.handle, ctx.stream, *p, None, o.data_ptr(), lse.data_ptr(), *dims)
+    lib.call("fb_attn_bwd", ctx.handle, ctx.stream, *p, None, o.data_ptr(), lse.data_ptr(), do.data_ptr(), dq.data_ptr(), dk.data_ptr(),
+             dvv.data_ptr(), *dims)
+    assert ctx.device_error() == 0
+    # at most 6 products x 4 steps x 32 blocks truncating adds of 2^-24 into an accumulator, and the scores' own 24: 5e-5
+    for name, got, ref in zip(("o", "dq", "dk", "dv"), (o, dq, dk, dvv), _reference(q, k, v, do, d, dv, heads, causal)):
+        assert _err(got, ref) < 5e-5, (name, _err(got, ref))
