@@ -1083,3 +1083,34 @@ int32_t fb_attn_bwd_tc(fb_ctx* ctx, cudaStream_t stream, const float* q, const f
   }
   return st;
 }
+
+// The same for bf16 q, k, v (and dO): one plane each, outputs rounded to bf16 once.  o32 (optional in the forward call) keeps
+// the Float32 output for the backward pass.  FB_ERR_UNSUPPORTED, without a message, for every call these kernels do not
+// take: the caller then casts and takes the Float32 entry points, which also report what is wrong with a bad one.
+FB_API int32_t fb_attn_fwd_bf16(fb_ctx* ctx, void* stream, const uint16_t* q, const uint16_t* k, const uint16_t* v, float* o32, uint16_t* o,
+                                float* lse, int64_t e_dim, int64_t ev_dim, int64_t lq, int64_t lk, int64_t batch, int32_t nheads,
+                                int32_t causal) {
+  FB_CHECK_CTX(ctx);
+  AtcPlan P;
+  if (!attn_tc_enabled() || !q || !k || !v || !o || !lse || nheads < 1 || e_dim % nheads != 0 || ev_dim % nheads != 0 || batch * nheads > 65535 ||
+      !make_plan(&P, 1, e_dim, ev_dim, lq, lk, batch, nheads, causal))
+    return FB_ERR_UNSUPPORTED;
+  if (!fb_aligned16(q) || !fb_aligned16(k) || !fb_aligned16(v) || !fb_aligned16(o) || !fb_aligned16(o32)) return FB_ERR_UNSUPPORTED;
+  return fwd_impl<1>(ctx, (cudaStream_t)stream, (const uint8_t*)q, (const uint8_t*)k, (const uint8_t*)v, o32, o, lse, P, batch);
+}
+
+FB_API int32_t fb_attn_bwd_bf16(fb_ctx* ctx, void* stream, const uint16_t* q, const uint16_t* k, const uint16_t* v, const float* o32,
+                                const float* lse, const uint16_t* dout, uint16_t* dq, uint16_t* dk, uint16_t* dv, int64_t e_dim, int64_t ev_dim,
+                                int64_t lq, int64_t lk, int64_t batch, int32_t nheads, int32_t causal) {
+  FB_CHECK_CTX(ctx);
+  AtcPlan P;
+  if (!attn_tc_enabled() || !attn_bwd_tc_enabled() || !q || !k || !v || !o32 || !lse || !dout || !dq || !dk || !dv || nheads < 1 ||
+      e_dim % nheads != 0 || ev_dim % nheads != 0 || batch * nheads > 65535 || lq > BWD_MAX_BLOCKS * KT || lk > BWD_MAX_BLOCKS * KT ||
+      !make_plan(&P, 1, e_dim, ev_dim, lq, lk, batch, nheads, causal))
+    return FB_ERR_UNSUPPORTED;
+  if (!fb_aligned16(q) || !fb_aligned16(k) || !fb_aligned16(v) || !fb_aligned16(o32) || !fb_aligned16(dout) || !fb_aligned16(dq) ||
+      !fb_aligned16(dk) || !fb_aligned16(dv))
+    return FB_ERR_UNSUPPORTED;
+  return bwd_impl<1>(ctx, (cudaStream_t)stream, (const uint8_t*)q, (const uint8_t*)k, (const uint8_t*)v, o32, lse, (const uint8_t*)dout,
+                     (uint8_t*)dq, (uint8_t*)dk, (uint8_t*)dv, P, batch, true, true);
+}

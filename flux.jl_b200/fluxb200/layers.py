@@ -618,6 +618,7 @@ class AttnScores:
             bias, sh, sb, p, seed, off = self._extras
             ctx = context()
             a = empty((Lk, Lq, H, B))
+            q, k = _float_copy(q), _float_copy(k)
             lib.call("fb_attn_scores_ex", ctx.handle, ctx.stream, q.ptr, k.ptr, _ptr(mask), _ptr(bias), sh, sb, p, seed, off, lse.ptr,
                      a.ptr, q.size[0], Lq, Lk, B, nheads, 1 if causal else 0)
             self._val = a
@@ -642,11 +643,57 @@ def _attention_bias(bias, Lk, Lq, H, B):
     return bias, sh, sb
 
 
+def _float_copy(a: B200Array) -> B200Array:
+    """The values of a bf16 array as Float32, off the tape (a Float32 array is returned as it is)."""
+    if not is_bf16(a):
+        return a
+    ctx, out = context(), empty(a.size)
+    lib.call("fb_cast_bf16_f32", ctx.handle, ctx.stream, a.ptr, out.ptr, a.numel())
+    return out
+
+
+def _attention_bf16(q, k, v, nheads, causal, Lq, Lk, B):
+    """(x, alpha) on the bf16 tensor-core kernels, or None for a call they do not take."""
+    E, Ev = q.size[0], v.size[0]
+    ctx = context()
+    dims = (E, Ev, Lq, Lk, B, nheads, 1 if causal else 0)
+    o, lse = empty((Ev, Lq, B), torch.bfloat16), empty((Lq, nheads, B))
+    o32 = empty((Ev, Lq, B)) if Tape.active else None
+    try:
+        lib.call("fb_attn_fwd_bf16", ctx.handle, ctx.stream, q.ptr, k.ptr, v.ptr, _ptr(o32), o.ptr, lse.ptr, *dims)
+    except lib.FluxB200Error as err:
+        if err.code != lib.ERR_UNSUPPORTED:
+            raise
+        return None
+    entry = None
+    if Tape.active:
+        def pullback(gs):
+            do = gs[0] if gs[0] is not None else zeros(o.size, torch.bfloat16)
+            dalpha = gs[1] if len(gs) > 1 else None
+            if dalpha is None and is_bf16(do):
+                dq, dk, dv = (empty(a.size, torch.bfloat16) for a in (q, k, v))
+                try:
+                    lib.call("fb_attn_bwd_bf16", ctx.handle, ctx.stream, q.ptr, k.ptr, v.ptr, o32.ptr, lse.ptr, do.ptr, dq.ptr, dk.ptr, dv.ptr,
+                             *dims)
+                    return [(q, dq), (k, dk), (v, dv)]
+                except lib.FluxB200Error as err:
+                    if err.code != lib.ERR_UNSUPPORTED:
+                        raise
+            qf, kf, vf, do = (_float_copy(a) for a in (q, k, v, do))
+            dq, dk, dv = empty(q.size), empty(k.size), empty(v.size)
+            lib.call("fb_attn_bwd_ex", ctx.handle, ctx.stream, qf.ptr, kf.ptr, vf.ptr, None, None, 0, 0, 0.0, 0, 0, o32.ptr, lse.ptr, do.ptr,
+                     _ptr(dalpha), dq.ptr, dk.ptr, dv.ptr, *dims)
+            return [(a, to_bf16(g)) for a, g in ((q, dq), (k, dk), (v, dv))]
+
+        Tape.record(o, [q, k, v], pullback)
+        entry = Tape.entries[-1]
+    return o, AttnScores(q, k, lse, None, causal, nheads, (Lk, Lq, nheads, B), (None, 0, 0, 0.0, 0, 0), entry)
+
+
 def dot_product_attention(q: B200Array, k: B200Array, v: B200Array, bias=None, nheads=1, mask=None, fdrop=None):
     """NNlib.dot_product_attention(q, k, v, bias; nheads, mask, fdrop) -> (x, alpha) for 3-d B200 arrays.  `fdrop` is a
     Dropout layer acting on the attention weights (MultiHeadAttention's `attn_drop`)."""
     low = is_bf16(q)
-    q, k, v = to_f32(q), to_f32(k), to_f32(v)
     E, Lq, B = q.size
     Ev, Lk, _ = v.size
     if k.size != (E, Lk, B):
@@ -654,6 +701,12 @@ def dot_product_attention(q: B200Array, k: B200Array, v: B200Array, bias=None, n
     if E % nheads or Ev % nheads:
         raise ArgumentError(f"qk_dim = {E} and v_dim = {Ev} should be divisible by nheads = {nheads}")
     causal = isinstance(mask, CausalMask)
+    if low and is_bf16(k) and is_bf16(v) and bias is None and (mask is None or causal) and \
+            not (fdrop is not None and fdrop.p > 0 and fdrop._isactive()):
+        res = _attention_bf16(q, k, v, nheads, causal, Lq, Lk, B)
+        if res is not None:
+            return res
+    q, k, v = to_f32(q), to_f32(k), to_f32(v)
     m = None
     if mask is not None and not causal:
         m = gpu(np.asarray(mask, dtype=np.uint8)) if isinstance(mask, np.ndarray) else mask

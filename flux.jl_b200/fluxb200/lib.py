@@ -15,6 +15,7 @@ LIB_PATH = os.path.join(_HERE, "libfluxb200.so")
 FB_OK = 0
 ERR_NAMES = {-1: "FB_ERR_INVALID_ARG", -2: "FB_ERR_SHAPE", -3: "FB_ERR_ALLOC", -4: "FB_ERR_CUDA",
              -5: "FB_ERR_NCCL", -6: "FB_ERR_TIMEOUT", -7: "FB_ERR_UNSUPPORTED"}
+ERR_UNSUPPORTED = -7
 
 ACT = {"identity": 0, "relu": 1, "tanh": 2, "sigmoid": 3, "gelu_tanh": 4, "gelu": 4, "gelu_erf": 5}
 # "bf16": operands hold bf16 values (see fluxb200.bf16); the GEMM is the single TF32 pass, exact for such operands
@@ -111,6 +112,8 @@ PROTOTYPES = {
     "fb_attn_bwd_ex": (_i32, [_p, _p, _p, _p, _p, _p, _p, _i64, _i64, _f, C.c_uint64, C.c_uint64, _p, _p, _p, _p, _p, _p, _p,
                               _i64, _i64, _i64, _i64, _i64, _i32, _i32]),
     "fb_attn_scores_ex": (_i32, [_p, _p, _p, _p, _p, _p, _i64, _i64, _f, C.c_uint64, C.c_uint64, _p, _p, _i64, _i64, _i64, _i64, _i32, _i32]),
+    "fb_attn_fwd_bf16": (_i32, [_p] * 8 + [_i64] * 5 + [_i32] * 2),
+    "fb_attn_bwd_bf16": (_i32, [_p] * 11 + [_i64] * 5 + [_i32] * 2),
     "fb_comm_get_unique_id": (_i32, [_p]),
     "fb_comm_init_rank": (_i32, [_p, _p, _i32, _i32, C.POINTER(_p)]),
     "fb_comm_destroy": (_i32, [_p]),

@@ -58,3 +58,32 @@ def test_attention_planes(d, dv, heads, lq, lk, batch, causal, shift):
     # at most 6 products x 4 steps x 32 blocks truncating adds of 2^-24 into an accumulator, and the scores' own 24: 5e-5
     for name, got, ref in zip(("o", "dq", "dk", "dv"), (o, dq, dk, dvv), _reference(q, k, v, do, d, dv, heads, causal)):
         assert _err(got, ref) < 5e-5, (name, _err(got, ref))
+
+
+@pytest.mark.parametrize("d,heads,lq,lk,causal", [(64, 2, 129, 65, 1), (64, 1, 1, 9, 0), (32, 3, 300, 300, 1), (8, 2, 700, 131, 0),
+                                                  (64, 1, 100, 400, 1), (64, 1, 2048, 2048, 0), (64, 1, 2049, 70, 0)])
+def test_attention_bf16(d, heads, lq, lk, causal):
+    """bf16 operands through the public call (2049 queries: the backward pass takes the Float32 kernels).  Every output is
+    rounded to bf16 once (2^-9 of each value at most): 3e-3 with room for the Float32 sums and the scaled rounding of dO."""
+    import fluxb200 as F
+    g = torch.Generator(device="cuda")
+    g.manual_seed(lq + lk + d)
+    batch, E = 2, heads * d
+    q, k, v = (torch.randn(batch, n, E, device="cuda", generator=g).bfloat16() for n in (lq, lk, lk))
+    arrays = tuple(F.B200Array(t.flatten(), (E, t.shape[1], batch)) for t in (q, k, v))
+    mask = F.make_causal_mask() if causal else None
+
+    def f(a):
+        y, _ = F.dot_product_attention(*a, nheads=heads, mask=mask)
+        return F.sum_abs2(y), y
+
+    (_, y), (grads,) = F.withgradient(f, arrays)
+    assert y.t.dtype == torch.bfloat16 and grads[0].t.dtype == torch.bfloat16
+    yt = y.t.view(batch, lq, E)
+    out, dq, dk, dv = _reference(q, k, v, 2 * yt.double(), d, d, heads, causal)
+    for name, got, ref in (("y", yt, out), ("dq", grads[0].t, dq), ("dk", grads[1].t, dk), ("dv", grads[2].t, dv)):
+        assert _err(got.view(ref.shape), ref) < 3e-3, (name, _err(got.view(ref.shape), ref))
+    plain, alpha = F.dot_product_attention(*arrays, nheads=heads, mask=mask)
+    assert torch.equal(plain.t, y.t)
+    a = alpha.materialize().t.view(batch, heads, lq, lk)
+    assert float((a.sum(-1) - 1).abs().max()) < 1e-4
