@@ -1,4 +1,6 @@
 // Element-wise helpers, the loss kernels and the multi-tensor Adam step (all memory-bound).
+#include <cuda_bf16.h>
+
 #include "common.cuh"
 
 namespace {
@@ -216,6 +218,69 @@ adam_kernel(const __grid_constant__ AdamTable tab, float eta, float beta1, float
       m[i] = mk; v[i] = vk;
       w[i] -= mk * inv_c1 / (sqrtf(vk * inv_c2) + eps) * eta;
     }
+  }
+}
+
+// The update of bf16 parameters: the rule runs on the Float32 master copy with the bf16 gradient widened in registers, and
+// the rounded parameter is written in the same pass.  Bound by memory: 28 bytes a parameter; as three passes (gradient to
+// Float32, update, rounding) it moved 40.  54.5 M parameters in 14 leaves: 400 us in 15 launches -> 235 us in one (6490 GB/s).
+struct AdamLowTable {
+  AdamTable t;                          // g unused
+  const uint16_t* g[ADAM_MAX_TENSORS];
+  uint16_t* p[ADAM_MAX_TENSORS];
+};
+
+__device__ __forceinline__ uint16_t adam_round(float w) {
+  const __nv_bfloat16 b = __float2bfloat16_rn(w);
+  return *reinterpret_cast<const uint16_t*>(&b);
+}
+
+__global__ void __launch_bounds__(256)
+adam_bf16_kernel(const __grid_constant__ AdamLowTable tab, float eta, float beta1, float beta2, float eps, float inv_c1, float inv_c2,
+                 float grad_scale) {
+  int t = 0;
+  while (t + 1 < tab.t.ntensors && (int)blockIdx.x >= tab.t.block_start[t + 1]) ++t;
+  const int64_t begin = (int64_t)(blockIdx.x - tab.t.block_start[t]) * ADAM_CHUNK;
+  const int64_t count = tab.t.count[t];
+  const int64_t end = begin + ADAM_CHUNK > count ? count : begin + ADAM_CHUNK;
+  float *w = tab.t.w[t], *m = tab.t.m[t], *v = tab.t.v[t];
+  const uint16_t* g = tab.g[t];
+  uint16_t* p = tab.p[t];
+  const float omb1 = 1.0f - beta1, omb2 = 1.0f - beta2;
+  auto rule = [&](float gk, float& mk, float& vk, float& wk) {
+    gk *= grad_scale;
+    mk = beta1 * mk + omb1 * gk;
+    vk = beta2 * vk + omb2 * gk * gk;
+    wk -= mk * inv_c1 / (sqrtf(vk * inv_c2) + eps) * eta;
+  };
+  const bool vec = ((reinterpret_cast<uintptr_t>(w) | reinterpret_cast<uintptr_t>(m) | reinterpret_cast<uintptr_t>(v)) & 15u) == 0 &&
+                   ((reinterpret_cast<uintptr_t>(g) | reinterpret_cast<uintptr_t>(p)) & 7u) == 0;
+  int64_t i0 = begin;
+  if (vec) {
+    i0 = begin + ((end - begin) & ~int64_t(3));
+    for (int64_t i = begin + 4 * threadIdx.x; i < i0; i += 4 * 256) {
+      const uint2 gw = __ldcs((const uint2*)(g + i));
+      const float gv[4] = {__uint_as_float(gw.x << 16), __uint_as_float(gw.x & 0xffff0000u), __uint_as_float(gw.y << 16),
+                           __uint_as_float(gw.y & 0xffff0000u)};
+      float4 mv = *(const float4*)(m + i), vv = *(const float4*)(v + i), wv = *(const float4*)(w + i);
+      float *mp = &mv.x, *vp = &vv.x, *wp = &wv.x;
+      uint32_t r[4];
+#pragma unroll
+      for (int k = 0; k < 4; ++k) {
+        rule(gv[k], mp[k], vp[k], wp[k]);
+        r[k] = adam_round(wp[k]);
+      }
+      *(float4*)(m + i) = mv;
+      *(float4*)(v + i) = vv;
+      *(float4*)(w + i) = wv;
+      *(uint2*)(p + i) = make_uint2(r[0] | (r[1] << 16), r[2] | (r[3] << 16));
+    }
+  }
+  for (int64_t i = i0 + threadIdx.x; i < end; i += 256) {
+    float mk = m[i], vk = v[i], wk = w[i];
+    rule(__uint_as_float((uint32_t)g[i] << 16), mk, vk, wk);
+    m[i] = mk; v[i] = vk; w[i] = wk;
+    p[i] = adam_round(wk);
   }
 }
 
@@ -490,6 +555,42 @@ FB_API int32_t fb_adam_step(fb_ctx* ctx, void* stream_, int32_t ntensors, float*
   FB_CHECK_CTX(ctx);
   return adam_common(ctx, (cudaStream_t)stream_, ntensors, w_host, g_host, m_host, v_host, counts_host, eta, beta1, beta2, eps,
                      b1t, b2t, grad_scale, nullptr, nullptr);
+}
+
+FB_API int32_t fb_adam_step_bf16(fb_ctx* ctx, void* stream_, int32_t ntensors, uint16_t* const* p_host, float* const* w_host,
+                                 const uint16_t* const* g_host, float* const* m_host, float* const* v_host, const int64_t* counts_host,
+                                 float eta, float beta1, float beta2, float eps, float b1t, float b2t, float grad_scale) {
+  FB_CHECK_CTX(ctx);
+  FB_REQUIRE(ntensors >= 0, FB_ERR_INVALID_ARG, "fb_adam_step_bf16: negative tensor count");
+  if (ntensors == 0) return FB_OK;
+  FB_REQUIRE(p_host && w_host && g_host && m_host && v_host && counts_host, FB_ERR_INVALID_ARG, "fb_adam_step_bf16: NULL table");
+  for (int i = 0; i < ntensors; ++i) {
+    FB_REQUIRE(counts_host[i] >= 0 && counts_host[i] < (int64_t)ADAM_CHUNK << 24, FB_ERR_INVALID_ARG,
+               "fb_adam_step_bf16: bad element count for leaf %d", i);
+    FB_REQUIRE(counts_host[i] == 0 || (p_host[i] && w_host[i] && g_host[i] && m_host[i] && v_host[i]), FB_ERR_INVALID_ARG,
+               "fb_adam_step_bf16: NULL pointer for leaf %d", i);
+  }
+  const float inv_c1 = 1.0f / (1.0f - b1t), inv_c2 = 1.0f / (1.0f - b2t);
+  int done = 0;
+  while (done < ntensors) {
+    AdamLowTable tab;
+    memset(&tab, 0, sizeof(tab));
+    int k = 0, blocks = 0;
+    for (; done < ntensors && k < ADAM_MAX_TENSORS; ++done) {
+      if (counts_host[done] == 0) continue;
+      tab.t.w[k] = w_host[done]; tab.t.m[k] = m_host[done]; tab.t.v[k] = v_host[done];
+      tab.g[k] = g_host[done]; tab.p[k] = p_host[done];
+      tab.t.count[k] = counts_host[done];
+      tab.t.block_start[k++] = blocks;
+      blocks += (int)((counts_host[done] + ADAM_CHUNK - 1) / ADAM_CHUNK);   // 32 leaves of < 2^24 blocks
+    }
+    if (k == 0) continue;
+    tab.t.block_start[k] = blocks;
+    tab.t.ntensors = k;
+    adam_bf16_kernel<<<(unsigned)blocks, 256, 0, (cudaStream_t)stream_>>>(tab, eta, beta1, beta2, eps, inv_c1, inv_c2, grad_scale);
+    FB_LAUNCH_CHECK();
+  }
+  return FB_OK;
 }
 
 FB_API int32_t fb_adam_step_dev(fb_ctx* ctx, void* stream_, int32_t ntensors, float* const* w_host,

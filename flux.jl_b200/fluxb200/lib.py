@@ -89,6 +89,8 @@ PROTOTYPES = {
     "fb_round_bf16": (_i32, [_p, _p, _p, _p, _i64]),
     "fb_adam_step": (_i32, [_p, _p, _i32, C.POINTER(_p), C.POINTER(_p), C.POINTER(_p), C.POINTER(_p),
                             C.POINTER(_i64), _f, _f, _f, _f, _f, _f, _f]),
+    "fb_adam_step_bf16": (_i32, [_p, _p, _i32, C.POINTER(_p), C.POINTER(_p), C.POINTER(_p), C.POINTER(_p), C.POINTER(_p),
+                            C.POINTER(_i64), _f, _f, _f, _f, _f, _f, _f]),
     "fb_adam_step_dev": (_i32, [_p, _p, _i32, C.POINTER(_p), C.POINTER(_p), C.POINTER(_p), C.POINTER(_p),
                                 C.POINTER(_i64), _f, _f, _f, _f, _p, _p, _f]),
     "fb_adam_block_dev": (_i32, [_p, _p, _p, _p, _p, _p, _i64, _f, _f, _f, _f, _p, _p, _f]),

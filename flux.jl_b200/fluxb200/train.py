@@ -348,7 +348,10 @@ def update(opt_state: OptState, model, grad_tree):
     # parameter is the master rounded back
     low = [p for p in ps if opt_state.leaves[id(p)].master is not None]
     wmap = {id(p): (opt_state.leaves[id(p)].master if opt_state.leaves[id(p)].master is not None else p) for p in ps}
-    gmap = {k: to_f32(g) for k, g in gmap.items()}
+    # (in one pass where the gradient is bf16 and the rule Adam)
+    fused = {id(p) for p in low if isinstance(rule, Adam) and gmap[id(p)].t.dtype == torch.bfloat16}
+    low = [p for p in low if id(p) not in fused]
+    gmap = {k: g if k in fused else to_f32(g) for k, g in gmap.items()}
     if isinstance(rule, Descent):
         for p in ps:
             lib.call("fb_axpy", ctx.handle, ctx.stream, -rule.eta, gmap[id(p)].ptr, wmap[id(p)].ptr, p.numel())
@@ -357,8 +360,8 @@ def update(opt_state: OptState, model, grad_tree):
     # leaves share (β1ᵗ, β2ᵗ) when they have seen the same number of steps: group by that pair
     groups: dict = {}
     for p in ps:
-        groups.setdefault(opt_state.leaves[id(p)].state[2], []).append(p)
-    for (b1t, b2t), plist in groups.items():
+        groups.setdefault((opt_state.leaves[id(p)].state[2], id(p) in fused), []).append(p)
+    for ((b1t, b2t), one_pass), plist in groups.items():
         k = len(plist)
         arr_t = C.c_void_p * k
         w = arr_t(*[wmap[id(p)].t.data_ptr() for p in plist])
@@ -366,8 +369,11 @@ def update(opt_state: OptState, model, grad_tree):
         m = arr_t(*[opt_state.leaves[id(p)].state[0].t.data_ptr() for p in plist])
         v = arr_t(*[opt_state.leaves[id(p)].state[1].t.data_ptr() for p in plist])
         cnt = (C.c_int64 * k)(*[p.numel() for p in plist])
-        lib.call("fb_adam_step", ctx.handle, ctx.stream, k, w, g, m, v, cnt, rule.eta, rule.beta[0], rule.beta[1],
-                 rule.epsilon, b1t, b2t, 1.0)
+        rest = (w, g, m, v, cnt, rule.eta, rule.beta[0], rule.beta[1], rule.epsilon, b1t, b2t, 1.0)
+        if one_pass:
+            lib.call("fb_adam_step_bf16", ctx.handle, ctx.stream, k, arr_t(*[p.t.data_ptr() for p in plist]), *rest)
+        else:
+            lib.call("fb_adam_step", ctx.handle, ctx.stream, k, *rest)
         nb = _advance_powers((b1t, b2t), rule.beta)
         for p in plist:
             opt_state.leaves[id(p)].state[2] = nb

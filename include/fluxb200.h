@@ -303,6 +303,13 @@ int32_t fb_adam_step(fb_ctx* ctx, void* stream, int32_t ntensors, float* const* 
                      const int64_t* counts_host, float eta, float beta1, float beta2, float eps,
                      float b1t, float b2t, float grad_scale);
 
+/* The update of bf16 parameters p in one pass: w is the Float32 master copy, g the bf16 gradient (widened exactly), p
+ * receives w rounded to nearest even. */
+int32_t fb_adam_step_bf16(fb_ctx* ctx, void* stream, int32_t ntensors, uint16_t* const* p_host, float* const* w_host,
+                          const uint16_t* const* g_host, float* const* m_host, float* const* v_host,
+                          const int64_t* counts_host, float eta, float beta1, float beta2, float eps,
+                          float b1t, float b2t, float grad_scale);
+
 /* The same update with its step state on the device, for a train step replayed from a CUDA graph (the
  * device-specific one-launch `trainstep!` hook, src/train.jl:335-339): bt_dev[2] holds the running powers
  * (beta1^t, beta2^t); guard_dev (optional) is a device scalar - the loss - whose non-finite value skips the update,
