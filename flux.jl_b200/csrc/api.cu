@@ -53,6 +53,8 @@ FB_API int32_t fb_ctx_create(int32_t device, fb_ctx** out) {
   c->scratch_bytes = 0;
   c->pack = nullptr;
   c->pack_bytes = 0;
+  c->pack_stream = nullptr;
+  c->pack_used = false;
   c->retired_count = 0;
   c->dev_error = nullptr;
   c->gemm_ws = nullptr;
@@ -70,10 +72,18 @@ FB_API int32_t fb_ctx_create(int32_t device, fb_ctx** out) {
     return fb_fail(FB_ERR_ALLOC, "fb_ctx_create: cudaHostAlloc failed");
   }
   memset((void*)c->host_page, 0, 64);
+  if (cudaEventCreateWithFlags(&c->pack_event, cudaEventDisableTiming) != cudaSuccess) {
+    cudaGetLastError();
+    cudaFree(c->dev_error);
+    cudaFreeHost((void*)c->host_page);
+    delete c;
+    return fb_fail(FB_ERR_CUDA, "fb_ctx_create: cudaEventCreate failed");
+  }
   int32_t ws_status = fb_side_kernels_prepare_elementwise();
   if (ws_status == FB_OK) ws_status = fb_side_kernels_prepare_peer();
   if (ws_status == FB_OK) ws_status = fb_gemm_workspace_create(c);
   if (ws_status != FB_OK) {
+    cudaEventDestroy(c->pack_event);
     cudaFree(c->dev_error);
     cudaFreeHost((void*)c->host_page);
     delete c;
@@ -97,6 +107,7 @@ FB_API int32_t fb_ctx_destroy(fb_ctx* ctx) {
   cudaDeviceSynchronize();
   if (ctx->scratch) cudaFree(ctx->scratch);
   if (ctx->pack) cudaFree(ctx->pack);
+  cudaEventDestroy(ctx->pack_event);
   for (int i = 0; i < ctx->retired_count; ++i) cudaFree(ctx->retired[i]);
   if (ctx->dev_error) cudaFree(ctx->dev_error);
   cudaFreeHost((void*)ctx->host_page);
@@ -129,13 +140,33 @@ void* fb_scratch(fb_ctx* ctx, cudaStream_t stream, size_t bytes) {
   return arena_get(ctx, &ctx->scratch, &ctx->scratch_bytes, bytes);
 }
 
+static bool stream_capturing(cudaStream_t stream) {
+  cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+  if (cudaStreamIsCapturing(stream, &cs) != cudaSuccess) {
+    cudaGetLastError();
+    return true;
+  }
+  return cs != cudaStreamCaptureStatusNone;
+}
+
 void* fb_pack_scratch(fb_ctx* ctx, cudaStream_t stream, size_t bytes) {
-  if (bytes > ctx->pack_bytes) {
-    cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
-    if (cudaStreamIsCapturing(stream, &cs) != cudaSuccess) cudaGetLastError();
-    if (cs != cudaStreamCaptureStatusNone) return nullptr;
+  const bool capturing = stream_capturing(stream);
+  if (bytes > ctx->pack_bytes && capturing) return nullptr;
+  if (ctx->pack_used && ctx->pack_stream != stream && !capturing && cudaStreamWaitEvent(stream, ctx->pack_event, 0) != cudaSuccess) {
+    cudaGetLastError();
+    return nullptr;
   }
   return arena_get(ctx, &ctx->pack, &ctx->pack_bytes, bytes);
+}
+
+void fb_pack_done(fb_ctx* ctx, cudaStream_t stream) {
+  if (stream_capturing(stream)) return;
+  if (cudaEventRecord(ctx->pack_event, stream) != cudaSuccess) {
+    cudaGetLastError();
+    return;
+  }
+  ctx->pack_stream = stream;
+  ctx->pack_used = true;
 }
 
 FB_API int32_t fb_malloc(fb_ctx* ctx, int64_t bytes, void** out) {

@@ -1009,6 +1009,7 @@ int32_t fwd_impl(fb_ctx* ctx, cudaStream_t stream, const uint8_t* q, const uint8
         lse + b0 * D.H * D.Lq, D, ctx->dev_error);
     FB_LAUNCH_CHECK();
   }
+  fb_pack_done(ctx, stream);
   return FB_OK;
 }
 
@@ -1045,6 +1046,7 @@ int32_t bwd_impl(fb_ctx* ctx, cudaStream_t stream, const uint8_t* q, const uint8
         q + el * qoff, dout + el * qvoff, ki, vi, rv, dq + el * qoff, D, ctx->dev_error);
     FB_LAUNCH_CHECK();
   }
+  fb_pack_done(ctx, stream);
   return FB_OK;
 }
 

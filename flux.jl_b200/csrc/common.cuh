@@ -20,8 +20,11 @@ struct fb_ctx {
   size_t smem_optin;
   void* scratch;         // device arena, grown on demand, reused by every call on this context
   size_t scratch_bytes;
-  void* pack;            // second arena: 16-byte-aligned copies of GEMM operands (a caller's scratch stays untouched)
+  void* pack;            // second arena: copies of GEMM and attention operands (a caller's scratch stays untouched)
   size_t pack_bytes;
+  cudaEvent_t pack_event;     // behind the last work that reads the arena, enqueued on pack_stream
+  cudaStream_t pack_stream;
+  bool pack_used;
   void* retired[FB_MAX_RETIRED];   // outgrown arena blocks, released with the context
   int retired_count;
   int32_t* dev_error;    // device error word written by kernels whose bounded waits ran out
@@ -38,7 +41,10 @@ int32_t fb_fail(int32_t code, const char* fmt, ...);
 // too small (outgrown blocks are kept until fb_ctx_destroy).  NULL on allocation failure.
 void* fb_scratch(fb_ctx* ctx, cudaStream_t stream, size_t bytes);
 // The same from the operand-copy arena; NULL (without an error) also when it would have to grow inside a stream capture.
+// Work enqueued on another stream waits for the last use of the arena (not inside a capture, whose replays the caller
+// orders): call fb_pack_done behind the last kernel that reads the copies.
 void* fb_pack_scratch(fb_ctx* ctx, cudaStream_t stream, size_t bytes);
+void fb_pack_done(fb_ctx* ctx, cudaStream_t stream);
 
 #define FB_CHECK_CTX(ctx)                                                   \
   do {                                                                      \

@@ -84,8 +84,11 @@ int32_t fb_gemm_dispatch(fb_ctx* ctx, cudaStream_t stream, const fb_gemm_args& a
       if (macs >= 1.0e8 && a.K >= 32 && a.N >= 32 && a.M >= 32) {
         if (fb_gemm_tc_supported(a)) return fb_gemm_tc_launch(ctx, stream, a, 3);
         fb_gemm_args p = a;
-        if (macs >= 2.0e8 && a.bias_m == nullptr && pack_operands(ctx, stream, p) && fb_gemm_tc_supported(p))
-          return fb_gemm_tc_launch(ctx, stream, p, 3);
+        if (macs >= 2.0e8 && a.bias_m == nullptr && pack_operands(ctx, stream, p) && fb_gemm_tc_supported(p)) {
+          const int32_t st = fb_gemm_tc_launch(ctx, stream, p, 3);
+          fb_pack_done(ctx, stream);
+          return st;
+        }
       }
       return fb_gemm_simt_launch(ctx, stream, a);
     }

@@ -87,3 +87,32 @@ def test_attention_bf16(d, heads, lq, lk, causal):
     assert torch.equal(plain.t, y.t)
     a = alpha.materialize().t.view(batch, heads, lq, lk)
     assert float((a.sum(-1) - 1).abs().max()) < 1e-4
+
+
+def test_attention_two_streams():
+    """Calls of one thread on two streams share the context's operand arena: neither may read the other's copies."""
+    import fluxb200 as F
+    from fluxb200 import lib
+    heads, d, n, batch = 8, 64, 512, 4
+    g = torch.Generator(device="cuda")
+    g.manual_seed(5)
+    dims = (heads * d, heads * d, n, n, batch, heads, 0)
+    ctx = F.context()
+    sets = []
+    for _ in range(2):
+        q, k, v = (torch.randn(batch, n, heads * d, device="cuda", generator=g) for _ in range(3))
+        sets.append((q, k, v, torch.empty_like(q), torch.empty(batch * heads * n, device="cuda"), torch.empty_like(q)))
+
+    def forward(s, out, stream):
+        lib.call("fb_attn_fwd", ctx.handle, stream, *[t.data_ptr() for t in s[:3]], None, out.data_ptr(), s[4].data_ptr(), *dims)
+
+    for s in sets:
+        forward(s, s[5], ctx.stream)
+    torch.cuda.synchronize()
+    streams = [torch.cuda.Stream(), torch.cuda.Stream()]
+    for _ in range(20):
+        for s, st in zip(sets, streams):
+            forward(s, s[3], st.cuda_stream)
+    torch.cuda.synchronize()
+    for s in sets:
+        assert torch.equal(s[3], s[5])
