@@ -236,19 +236,29 @@ class Tape:
         cls.tracked = set()
 
 
-def accumulate(grads: dict, keep: dict, arr: B200Array, g: B200Array):
-    """grads[id(arr)] += g (tangent accumulation, Zygote's `accum`)."""
+def accumulate(grads: dict, owned: set, arr: B200Array, g: B200Array, fresh: bool):
+    """grads[id(arr)] += g (tangent accumulation, Zygote's `accum`).
+
+    Only memory that belongs to this one gradient is added to in place: `owned` holds the keys for which that is so.
+    `fresh` says that g's memory was handed over to `arr` alone; a pullback may also pass its cotangent's memory on
+    (reshape, add), which other gradients then share, so that the sum needs memory of its own."""
     k = id(arr)
-    keep[k] = arr
-    if k in grads:
-        if grads[k].t.data_ptr() != g.t.data_ptr():
-            ctx = context()
-            if getattr(grads[k], "_is_one", False):   # the shared constant 1 is never written
-                grads[k] = _wrap(grads[k].t.clone(), grads[k].size)
-            if grads[k].t.dtype == torch.bfloat16:
-                g = to_bf16(g)
-                lib.call("fb_axpy_bf16", ctx.handle, ctx.stream, 1.0, g.ptr, grads[k].ptr, g.numel())
-            else:
-                lib.call("fb_axpy", ctx.handle, ctx.stream, 1.0, to_f32(g).ptr, grads[k].ptr, g.numel())
-    else:
+    if k not in grads:
         grads[k] = g
+        if fresh:
+            owned.add(k)
+    else:
+        own_gradient(grads, owned, k)
+        ctx, acc = context(), grads[k]
+        if acc.t.dtype == torch.bfloat16:
+            g = to_bf16(g)
+            lib.call("fb_axpy_bf16", ctx.handle, ctx.stream, 1.0, g.ptr, acc.ptr, g.numel())
+        else:
+            lib.call("fb_axpy", ctx.handle, ctx.stream, 1.0, to_f32(g).ptr, acc.ptr, g.numel())
+
+
+def own_gradient(grads: dict, owned: set, k: int):
+    """Gives grads[k] memory that no other gradient shares."""
+    if k not in owned:
+        grads[k] = _wrap(grads[k].t.clone(), grads[k].size)
+        owned.add(k)

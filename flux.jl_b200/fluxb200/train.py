@@ -14,7 +14,7 @@ import numpy as np
 import torch
 
 from . import lib
-from .core import B200Array, Tape, accumulate, context, empty, gpu, to_bf16, to_f32, zeros
+from .core import B200Array, Tape, accumulate, context, empty, gpu, own_gradient, to_bf16, to_f32, zeros
 from .layers import DimensionMismatch, Layer, trainables
 
 
@@ -182,10 +182,9 @@ def _withgradient_device(f, model, grad_sink=None):
                     if a is not None and id(a) in pid:
                         counts[id(a)] = counts.get(id(a), 0) + 1
             grad_sink.expect_uses(counts)
-        grads: dict = {}
-        keep: dict = {}
-        grads[id(loss)] = _one(loss.t.device)
-        keep[id(loss)] = loss
+        one = _One(loss.t.device)
+        grads: dict = {id(loss): one}
+        owned: set = set()
         # gradient averaging runs beside the reverse sweep: leave it the SMs it needs
         reserve = int(getattr(grad_sink, "reserved_sms", 0) or 0)
         if reserve:
@@ -194,12 +193,17 @@ def _withgradient_device(f, model, grad_sink=None):
             gs = [grads.get(id(o)) for o in outs]
             if all(g is None for g in gs):
                 continue
-            for arr, g in pullback(gs):
-                if arr is None or g is None:
-                    continue
-                accumulate(grads, keep, arr, g)
+            res = [(arr, g) for arr, g in pullback(gs) if arr is not None and g is not None]
+            # memory that the pullback passed on from its cotangents, or gave to two inputs, is shared
+            given = [g.t.data_ptr() for g in gs if g is not None and not (g is one and one.untouched)]
+            ptrs = [None if g is one else g.t.data_ptr() for _, g in res]
+            for (arr, g), ptr in zip(res, ptrs):
+                accumulate(grads, owned, arr, g, ptr is not None and ptr not in given and ptrs.count(ptr) == 1)
                 if grad_sink is not None:
                     grad_sink.ready(arr)
+        for p in params:   # a gradient that is handed out is its receiver's alone
+            if id(p) in grads:
+                own_gradient(grads, owned, id(p))
         tree = _grad_tree(model, grads)
     finally:
         if int(getattr(grad_sink, "reserved_sms", 0) or 0):
@@ -231,27 +235,24 @@ def _withgradient(f, model, grad_sink=None):
 
 
 class _One(B200Array):
-    """Cotangent 1 of the top-level loss."""
+    """Cotangent 1 of the top-level loss of one reverse sweep; its memory exists from the first reader on (the pullbacks of
+    the losses know the value)."""
 
-    __slots__ = ("_is_one",)
+    __slots__ = ("_is_one", "_device", "_value")
 
-    def __init__(self, a: B200Array):
-        super().__init__(a.t, a.size)
-        self._is_one = True
+    def __init__(self, device):
+        self.size, self._node = (), None
+        self._is_one, self._device, self._value = True, device, None
 
+    @property
+    def untouched(self) -> bool:
+        return self._value is None
 
-_ones: dict = {}
-
-
-def _one(device) -> _One:
-    """The constant 1 of a device (nothing writes into it)."""
-    o = _ones.get(device)
-    if o is None:
-        if torch.cuda.is_current_stream_capturing():   # memory of a graph's pool is the graph's
-            return _One(B200Array(torch.ones(1, device=device), ()))
-        o = _ones[device] = _One(B200Array(torch.ones(1, device=device), ()))
-        torch.cuda.current_stream(device).synchronize()   # other streams may use it at once
-    return o
+    @property
+    def t(self):
+        if self._value is None:
+            self._value = torch.ones(1, device=self._device)
+        return self._value
 
 
 def gradient(f, model):

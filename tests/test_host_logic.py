@@ -162,3 +162,123 @@ def test_nccl_fallback_keeps_its_order_and_ignores_early_reports(monkeypatch):
             assert log == ["fb_reduce_scatter", "fb_adam_step_dev", "fb_allgather"] * 4
         else:
             assert log == ["fb_allreduce"] * 4
+
+
+# --------------------------------------------------- the reverse sweep with the entry points replaced by their arithmetic ---
+class _HostEntryPoints:
+    """Element-wise entry points on host memory; `log` holds the names of all that were called, `error` is the device error
+    word that the read-back of the loss reports."""
+
+    def __init__(self):
+        self.log, self.error = [], 0
+
+    def read_scalar(self, a):
+        return float(a.t[0]), self.error
+
+    def device_error(self):
+        e, self.error = self.error, 0
+        return e
+
+    def call(self, name, ctx, stream, *a):
+        import ctypes as C
+        self.log.append(name)
+        arr = lambda ptr, n: np.ctypeslib.as_array(C.cast(ptr, C.POINTER(C.c_float)), (n,))
+        if name == "fb_sum":
+            arr(a[2], 1)[0] = arr(a[0], a[1]).sum()
+        elif name == "fb_sumsq":
+            arr(a[2], 1)[0] = (arr(a[0], a[1]) ** 2).sum()
+        elif name == "fb_scale":
+            arr(a[2], a[3])[:] = np.float32(a[1]) * arr(a[0], a[3])
+        elif name == "fb_fill":
+            arr(a[0], a[2])[:] = a[1]
+        elif name == "fb_axpy":
+            arr(a[2], a[3])[:] += np.float32(a[0]) * arr(a[1], a[3])
+        elif name == "fb_adam_step":
+            k, w = a[0], a[1]
+            for i in range(k):
+                arr(w[i], a[5][i])[:] -= 1.0
+        else:
+            raise AssertionError(f"{name} has no host arithmetic here")
+
+
+@pytest.fixture
+def host(monkeypatch):
+    import sys
+    import types
+
+    import torch
+
+    import fluxb200 as F
+    core, train = sys.modules["fluxb200.core"], sys.modules["fluxb200.train"]
+    h = _HostEntryPoints()
+
+    def init(self, t, size):
+        self.t, self.size, self._node = t, tuple(int(v) for v in size), None
+        assert t.numel() == int(np.prod(self.size, dtype=np.int64))
+    ctx = types.SimpleNamespace(handle=None, stream=None, torch_device=torch.device("cpu"), read_scalar=h.read_scalar,
+                                device_error=h.device_error)
+    monkeypatch.setattr(core.B200Array, "__init__", init)
+    for module in (core, train):
+        monkeypatch.setattr(module, "context", lambda: ctx)
+    monkeypatch.setattr(core.lib, "call", h.call)
+    monkeypatch.setattr(torch.cuda, "is_current_stream_capturing", lambda: False)
+    monkeypatch.setattr(torch.cuda, "current_stream", lambda *a: _FakeStream())
+    h.array = lambda *v, size=None: F.B200Array(torch.tensor(v, dtype=torch.float32), (len(v),) if size is None else size)
+    return h
+
+
+def _grad(F, f, *arrays):
+    value, (g,) = F.withgradient(f, tuple(arrays))
+    return value, [None if a is None else a.t.tolist() for a in g]
+
+
+def test_the_cotangent_one_survives_a_reshaped_loss(host):
+    """reshape hands its cotangent's memory on: a second contribution must not be added into it, in either order, and the
+    constant of one sweep must not reach the next."""
+    import fluxb200 as F
+    w = host.array(3.0)
+
+    def reshape_last(m):
+        s = F.sum_all(m[0])
+        z = F.scale(2.0, s)
+        return F.add(s.reshape(()), z)
+
+    def reshape_first(m):
+        s = F.sum_all(m[0])
+        r = s.reshape(())
+        return F.add(r, F.scale(2.0, s))
+    for f in (reshape_last, reshape_first):
+        for _ in range(3):
+            assert _grad(F, f, w) == (9.0, [[3.0]])
+    assert _grad(F, lambda m: F.sum_all(m[0]).reshape(()), w) == (3.0, [[1.0]])
+
+
+def test_shared_cotangents_inside_one_sweep(host):
+    """One cotangent that several arrays receive is read after one of them has been added to."""
+    import fluxb200 as F
+
+    def f(m):
+        s = F.sum_all(m[0])
+        c = F.scale(3.0, F.sum_all(m[1]))
+        b = F.scale(2.0, s)
+        return F.add(F.add(s.reshape(()), b), c)
+    assert _grad(F, f, host.array(1.0, 2.0), host.array(5.0)) == (24.0, [[3.0, 3.0], [3.0]])
+    # both operands of one add
+    assert _grad(F, lambda m: F.sum_all(F.add(m[0], m[0])), host.array(1.0, 2.0)) == (6.0, [[2.0, 2.0]])
+
+
+def test_a_handed_out_gradient_belongs_to_its_receiver(host):
+    """Parameters that receive the loss's own cotangent, or one cotangent between them, get memory of their own."""
+    import fluxb200 as F
+    a, b = host.array(2.0, size=()), host.array(5.0, size=())
+    for _ in range(2):
+        _, (g,) = F.withgradient(lambda m: F.add(m[0], m[1]), (a, b))
+        assert g[0].t.tolist() == [1.0] and g[1].t.tolist() == [1.0]
+        g[0].t += 7.0                                       # what the owner does with it is nobody else's business
+        assert g[1].t.tolist() == [1.0]
+    _, (g,) = F.withgradient(lambda m: m[0], (a,))
+    g[0].t += 7.0
+    assert _grad(F, lambda m: m[0], a) == (2.0, [[1.0]])
+    x, y = host.array(1.0, 2.0), host.array(3.0, 4.0)
+    _, (g,) = F.withgradient(lambda m: F.sum_all(F.add(m[0], m[1])), (x, y))
+    assert g[0].t.data_ptr() != g[1].t.data_ptr()
