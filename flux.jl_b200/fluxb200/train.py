@@ -407,12 +407,15 @@ def trainstep(loss, model, batch, opt_state):
         sink.begin_step()
     (l, gs), err = _withgradient(lambda m: loss(m, *batch), model, grad_sink=sink)
     lv = l[0] if isinstance(l, tuple) else l
-    finite = outer.all_finite(lv) if isinstance(outer, DistributedOptimizerBase) else math.isfinite(lv)
+    shared = isinstance(outer, DistributedOptimizerBase)
+    if err != 0 and not shared:   # a kernel left its gradients unwritten: they must not reach the parameters
+        _raise_on_device_error()
+    finite = outer.all_finite(lv) if shared else math.isfinite(lv)
     if finite:
         update(opt_state, model, gs[0])
     elif sink is not None:
         sink.finish()   # the collectives already started must be matched on every worker
-    if err != 0 or isinstance(outer, DistributedOptimizerBase):   # the update alone contains no bounded wait
+    if shared:   # (the other workers' collectives had to be matched first; an update alone contains no bounded wait)
         _raise_on_device_error()
     return l
 

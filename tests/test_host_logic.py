@@ -282,3 +282,22 @@ def test_a_handed_out_gradient_belongs_to_its_receiver(host):
     x, y = host.array(1.0, 2.0), host.array(3.0, 4.0)
     _, (g,) = F.withgradient(lambda m: F.sum_all(F.add(m[0], m[1])), (x, y))
     assert g[0].t.data_ptr() != g[1].t.data_ptr()
+
+
+def test_a_step_whose_kernel_gave_up_leaves_the_parameters_alone(host):
+    """The device error word is read with the loss: it raises before the optimiser sees the gradients."""
+    import fluxb200 as F
+    w = host.array(1.0, 2.0)
+    model = (w,)
+    opt = F.setup(F.Adam(), model)
+    state = opt.leaves[id(w)].state
+    loss = lambda m, x: F.sum_abs2(F.add(m[0], x))
+    x = host.array(1.0, 1.0)
+    F.trainstep(loss, model, (x,), opt)
+    assert w.t.tolist() == [0.0, 1.0] and host.log.count("fb_adam_step") == 1      # (the stand-in subtracts 1)
+    powers, host.error = state[2], 3002
+    with pytest.raises(F.lib.FluxB200Error, match="3002"):
+        F.trainstep(loss, model, (x,), opt)
+    assert w.t.tolist() == [0.0, 1.0] and host.log.count("fb_adam_step") == 1 and state[2] == powers
+    F.trainstep(loss, model, (x,), opt)                                            # the word has been cleared
+    assert host.log.count("fb_adam_step") == 2
