@@ -20,7 +20,7 @@ struct fb_ctx {
   size_t smem_optin;
   void* scratch;         // device arena, grown on demand, reused by every call on this context
   size_t scratch_bytes;
-  void* pack;            // second arena: copies of GEMM and attention operands (a caller's scratch stays untouched)
+  void* pack;            // second arena: images of attention operands (a caller's scratch stays untouched)
   size_t pack_bytes;
   cudaEvent_t pack_event;     // behind the last work that reads the arena, enqueued on pack_stream
   cudaStream_t pack_stream;

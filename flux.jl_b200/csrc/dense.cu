@@ -24,36 +24,6 @@ static int default_precision_override() {
   return cached;
 }
 
-// dst[r][0 .. ld) = src[r][0 .. cols) (the padding of a row is never read)
-__global__ void __launch_bounds__(256)
-pack_rows_kernel(const float* __restrict__ src, int64_t lds, float* __restrict__ dst, int64_t ld, int64_t rows, int64_t cols) {
-  const int lane = threadIdx.x & 31;
-  for (int64_t r = (int64_t)blockIdx.x * 8 + (threadIdx.x >> 5); r < rows; r += (int64_t)gridDim.x * 8)
-    for (int64_t c = lane; c < cols; c += 32) dst[r * ld + c] = __ldg(src + r * lds + c);
-}
-
-// Operands whose rows do not start on 16-byte boundaries cannot be read by TMA.  A product of more than 2e8 multiply-adds
-// is worth a copy of them with padded rows into the context's operand arena: the copy is one pass over memory (a few us),
-// the tensor-core kernel several times faster than the FMA one (1001 x 1003 x 1005: 90 us FMA, 24 us packed).
-static bool pack_operands(fb_ctx* ctx, cudaStream_t stream, fb_gemm_args& a) {
-  const bool pa = a.lda % 4 != 0 || !fb_aligned16(a.A), pb = a.ldb % 4 != 0 || !fb_aligned16(a.B);
-  const int64_t ar = a.a_mn_major ? a.K : a.M, ac = a.a_mn_major ? a.M : a.K, ald = (ac + 3) / 4 * 4;
-  const int64_t br = a.b_mn_major ? a.K : a.N, bc = a.b_mn_major ? a.N : a.K, bld = (bc + 3) / 4 * 4;
-  const size_t abytes = pa ? ((size_t)(ar * ald) * 4 + 255) & ~size_t(255) : 0, bbytes = pb ? (size_t)(br * bld) * 4 : 0;
-  if (abytes + bbytes == 0) return true;
-  char* ws = (char*)fb_pack_scratch(ctx, stream, abytes + bbytes);
-  if (ws == nullptr) return false;
-  auto copy = [&](const float* src, int64_t lds, float* dst, int64_t ld, int64_t rows, int64_t cols) {
-    int64_t blocks = (rows + 7) / 8;
-    if (blocks > (int64_t)ctx->sm_count * 8) blocks = (int64_t)ctx->sm_count * 8;
-    pack_rows_kernel<<<(unsigned)blocks, 256, 0, stream>>>(src, lds, dst, ld, rows, cols);
-    ++g_fb_kernel_launches;
-  };
-  if (pa) { copy(a.A, a.lda, (float*)ws, ald, ar, ac); a.A = (const float*)ws; a.lda = ald; }
-  if (pb) { copy(a.B, a.ldb, (float*)(ws + abytes), bld, br, bc); a.B = (const float*)(ws + abytes); a.ldb = bld; }
-  return cudaPeekAtLastError() == cudaSuccess;
-}
-
 int32_t fb_gemm_dispatch(fb_ctx* ctx, cudaStream_t stream, const fb_gemm_args& a, int precision) {
   if (a.M == 0 || a.N == 0) return FB_OK;
   if (precision == FB_PREC_DEFAULT) {
@@ -80,16 +50,11 @@ int32_t fb_gemm_dispatch(fb_ctx* ctx, cudaStream_t stream, const fb_gemm_args& a
       // memory, operand split, read-back: ~9 us with a split K range) is paid: 231 x 512 x 512 9 us against 12, 512 x 512
       // x 512 14.6 against 12.7, 1024 x 512 x 784 32 against 16.  With fewer than 32 rows, columns or k-values most of a
       // 128-wide tile is padding.
+      // Operands or results whose rows are not 16-byte aligned stay on the FMA kernel: copies with padded rows would let the
+      // tensor cores take them faster (1001 x 1003 x 1005 in 48 us against 87, 4095^3 in 1.06 ms against 3.9), but with
+      // 3xTF32's errors (2.1e-6 against 5.7e-7, 1.5e-5 against 1.1e-6) and a NaN for every product with an infinite factor.
       const double macs = (double)a.M * (double)a.N * (double)a.K;
-      if (macs >= 1.0e8 && a.K >= 32 && a.N >= 32 && a.M >= 32) {
-        if (fb_gemm_tc_supported(a)) return fb_gemm_tc_launch(ctx, stream, a, 3);
-        fb_gemm_args p = a;
-        if (macs >= 2.0e8 && a.bias_m == nullptr && pack_operands(ctx, stream, p) && fb_gemm_tc_supported(p)) {
-          const int32_t st = fb_gemm_tc_launch(ctx, stream, p, 3);
-          fb_pack_done(ctx, stream);
-          return st;
-        }
-      }
+      if (macs >= 1.0e8 && a.K >= 32 && a.N >= 32 && a.M >= 32 && fb_gemm_tc_supported(a)) return fb_gemm_tc_launch(ctx, stream, a, 3);
       return fb_gemm_simt_launch(ctx, stream, a);
     }
     default:

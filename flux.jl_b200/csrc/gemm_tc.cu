@@ -57,7 +57,6 @@ struct Sched {
   int nu;            // units per tile
   int U;             // units in the tail: (num_tiles - dp_tiles) * nu
   int ksplit;        // CTAs of one cluster that share a tile, each with a part of its K range (1: no split)
-  int vec;           // rows of C (and Z, bias) start on 16-byte boundaries
   float* ws;         // [2 * G * ranks] slots of BM x 256 floats
   int* tickets;      // [G * ranks * 4], zero between launches
 };
@@ -218,7 +217,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
     if (row >= M) return;
     float* crow = C + (int64_t)row * ldc;
     float* zrow = Z ? Z + (int64_t)row * ldc : nullptr;
-    if (n + 3 < N && (PAIR || sch.vec)) {
+    if (n + 3 < N) {
       if (add_c) {
         const float4 c4 = *(const float4*)(crow + n);
         u[0] += c4.x; u[1] += c4.y; u[2] += c4.z; u[3] += c4.w;
@@ -677,7 +676,6 @@ int32_t launch_variant(fb_ctx* ctx, cudaStream_t stream, const fb_gemm_args& a, 
   sch.nu = (num_kb + UNIT_KB - 1) / UNIT_KB;
   sch.U = 0;
   sch.ksplit = ksplit;
-  sch.vec = (a.ldc % 4 == 0 && fb_aligned16(a.C) && (!a.Z || fb_aligned16(a.Z)) && (!a.bias_n || fb_aligned16(a.bias_n))) ? 1 : 0;
   sch.ws = nullptr;
   sch.tickets = nullptr;
   int64_t G = Gmax < num_tiles ? Gmax : num_tiles;
@@ -752,7 +750,7 @@ Plan plan_3xtf32(fb_ctx* ctx, const fb_gemm_args& a, bool force_pair) {
   Plan best = {0, 1};
   double best_t = 1e30;
   for (int sh = 2; sh >= 0; --sh) {
-    if (sh == 2 && (a.M < 256 || a.N < 256 || a.ldc % 4 || !fb_aligned16(a.C) || !fb_aligned16(a.Z) || !fb_aligned16(a.bias_n))) continue;
+    if (sh == 2 && (a.M < 256 || a.N < 256)) continue;
     if (force_pair && sh != 2 && best_t < 1e30) continue;
     if (sh == 1 && a.N <= 128) continue;
     const int ranks = sh == 2 ? 2 : 1;
@@ -809,7 +807,10 @@ bool fb_gemm_tc_supported(const fb_gemm_args& a) {
   if (a.M < 1 || a.N < 1 || a.K < 1) return false;
   if (a.M > 0x7fffff00 || a.N > 0x7fffff00 || a.K > 0x7fffff00) return false;
   if (a.bias_m != nullptr) return false;
-  if (!fb_aligned16(a.A) || !fb_aligned16(a.B) || a.lda % 4 || a.ldb % 4) return false;   // TMA; C may be unaligned
+  if (!fb_aligned16(a.A) || !fb_aligned16(a.B) || !fb_aligned16(a.C)) return false;
+  if (a.Z && !fb_aligned16(a.Z)) return false;
+  if (a.bias_n && !fb_aligned16(a.bias_n)) return false;
+  if (a.lda % 4 || a.ldb % 4 || a.ldc % 4) return false;
   // the leading dimension must cover the contiguous extent
   if (a.lda < (a.a_mn_major ? a.M : a.K) || a.ldb < (a.b_mn_major ? a.N : a.K) || a.ldc < a.N) return false;
   return true;

@@ -32,7 +32,7 @@ def _operands(ta, tb, m, n, k, pad, dtype):
 
 # the FMA kernel: one row, 16-row and 16-column tiles and one past them, K of less than a stage, of several clusters, odd
 # leading dimensions; the tensor-core kernel: K split over 2, 4 and 8 CTAs (with a ragged last part and two accumulation
-# segments per part), pairs, packed operands
+# segments per part), pairs
 @pytest.mark.parametrize("ta,tb", [(0, 0), (1, 0), (0, 1), (1, 1)])
 @pytest.mark.parametrize("m,n,k,pad", [(512, 1, 784, 0), (10, 16, 33, 1), (65, 17, 1, 0), (16, 300, 1000, 3), (33, 129, 260, 2),
                                        (520, 300, 1000, 0), (264, 140, 2100, 0), (516, 1030, 4100, 0), (1000, 1000, 9000, 0),
@@ -48,6 +48,36 @@ def test_gemm_f32_cuts(ctx, ta, tb, m, n, k, pad, accumulate):
     err = (out[:, :m].double() - (1.0 if accumulate else 0.0) - ref).norm() / ref.norm()
     assert err < 3e-5, float(err)
     assert bool((out[:, m:] == 1.0).all())     # nothing is written between the rows
+
+
+# an odd leading dimension of one operand, of the result alone, and a start off the 16-byte boundary
+@pytest.mark.parametrize("ta,tb", [(0, 0), (1, 0), (0, 1), (1, 1)])
+@pytest.mark.parametrize("m,n,k,lda,ldb,ldc,shift", [(1001, 1003, 1005, 0, 0, 0, 0), (512, 1024, 2048, 1, 0, 0, 0), (512, 1024, 2048, 0, 3, 0, 0),
+                                                     (512, 1024, 2048, 0, 0, 2, 0), (1024, 512, 512, 0, 0, 0, 1), (4095, 33, 2049, 0, 0, 0, 0)])
+def test_unaligned_products_keep_float32_sums(ctx, ta, tb, m, n, k, lda, ldb, ldc, shift):
+    """The default precision computes them with Float32 FMAs: rounding to nearest, the errors of a sum of K terms add up as a
+    random walk, sqrt(K) * 2^-24 of the result's norm with room to spare (3xTF32: truncated sums, 2^-22 terms left out);
+    an infinite operand gives an infinite result."""
+    from fluxb200 import lib
+    g = torch.Generator(device="cuda").manual_seed(m + n + k)
+
+    def mat(rows, cols, pad):
+        flat = torch.randn(rows * (cols + pad) + 1, generator=g, device="cuda")
+        return flat[shift:shift + rows * (cols + pad)].view(rows, cols + pad)
+    (ra, ca), (rb, cb) = ((m, k) if ta else (k, m)), ((k, n) if tb else (n, k))
+    A, B, out = mat(ra, ca, lda), mat(rb, cb, ldb), mat(n, m, ldc)
+
+    def run():
+        lib.call("fb_gemm_f32", ctx.handle, ctx.stream, ta, tb, m, n, k, A.data_ptr(), ca + lda, B.data_ptr(), cb + ldb, out.data_ptr(),
+                 m + ldc, 0, 0)
+        a, b = A[:, :ca].double(), B[:, :cb].double()
+        return out[:, :m].double(), (b.T if tb else b) @ (a.T if ta else a)
+    got, ref = run()
+    err = float((got - ref).norm() / ref.norm())
+    assert err < k ** 0.5 * 2.0 ** -24, err
+    A[1, 2] = float("inf")
+    got, ref = run()
+    assert torch.equal(torch.isnan(got), torch.isnan(ref)) and torch.equal(torch.isinf(got), torch.isinf(ref))
 
 
 @pytest.mark.parametrize("ta,tb", [(0, 0), (1, 0), (0, 1), (1, 1)])
