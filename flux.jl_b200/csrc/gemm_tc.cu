@@ -26,10 +26,13 @@
 // atoms) and, for MN-major tiles, the 128-byte swizzle with 32-byte atoms (128 B x 4 k-rows per atom), which
 // is the only MN-major layout the tensor core accepts for 32-bit operands.
 //
-// The tensor core adds into its fp32 accumulator with truncation, so a long K chain drifts (about 3e-5 of
-// max|C| at K = 4096).  K is therefore cut into segments of 2048 that alternate between two accumulator
-// buffers in tensor memory: while the MMAs fill one, the epilogue warps drain the other into C with
-// round-to-nearest adds.
+// The tensor core adds into its fp32 accumulator with truncation, so a long K chain drifts: the error of a sum of
+// L k-values is 7.3e-9 L of the result's norm (N(0, 1) operands), whatever K is.  K is therefore cut into segments
+// that alternate between two accumulator buffers in tensor memory: while the MMAs fill one, the epilogue warps
+// drain the other and add it to the segments before with round-to-nearest adds (in C; a launch of one wave: in
+// the CTA's slot of the workspace, where a lane's 16 bytes lie beside the next lane's: a drain of 128 x 256 then
+// costs about 2.5 us, through rows of C or of the slot four to eight times that).  segment_kblocks() says how long
+// a segment is.
 //
 // Every mbarrier wait is bounded; when a wait runs out the kernel records a code in the context's
 // device error word, every role leaves its loop, tensor memory is released and the kernel returns.
@@ -43,7 +46,7 @@ namespace {
 
 constexpr int BM = 128;
 constexpr int BK = 16;               // floats per k-block (64 bytes)
-constexpr int SEG_KB = 128;          // k-blocks per accumulation segment (2048 k-values)
+constexpr int SEG_KB = 128;          // the longest accumulation segment in k-blocks (2048 k-values)
 
 // Work schedule of one launch.  Tiles [0, dp_tiles) are taken whole: CTA (pair) cid of G takes cid, cid + G, ...
 // (n fastest, so the tiles in flight are neighbours and share operand panels in L2).  The remaining tiles - a
@@ -57,6 +60,7 @@ struct Sched {
   int nu;            // units per tile
   int U;             // units in the tail: (num_tiles - dp_tiles) * nu
   int ksplit;        // CTAs of one cluster that share a tile, each with a part of its K range (1: no split)
+  int seg;           // k-blocks per accumulation segment
   float* ws;         // [2 * G * ranks] slots of BM x 256 floats
   int* tickets;      // [G * ranks * 4], zero between launches
 };
@@ -66,15 +70,16 @@ struct Portion {
   int tail_tile;     // index of the tile inside the tail (partial only)
   int trail;         // 1 when this CTA's range began before the tile's first unit (names the slot)
 };
+template <bool SPLIT>
 struct WorkIter {
   int w, ta, tb, t0;
   __device__ WorkIter(const Sched& s, int cid, int G) : w(0) {
-    if (s.ksplit > 1) return;
+    if (SPLIT) return;
     ta = t0 = (int)((long long)cid * s.U / G);
     tb = (int)((long long)(cid + 1) * s.U / G);
   }
   __device__ bool next(const Sched& s, int cid, int G, int num_kb, Portion& p) {
-    if (s.ksplit > 1) {   // one portion per CTA: part cid % ksplit of tile cid / ksplit
+    if (SPLIT) {   // one portion per CTA (pair): part cid % ksplit of tile cid / ksplit
       if (w++ != 0) return false;
       const int part = cid % s.ksplit;
       p.tile = cid / s.ksplit;
@@ -122,7 +127,10 @@ struct Cfg {
   static constexpr uint32_t ARRIVALS = PAIR ? 8 : 4;        // four warps per CTA arrive on ready / tmem_empty
 };
 
-template <bool A_MN, bool B_MN, int BN, int PASSES, bool PAIR, int SG>
+// SPLIT: a launch of one wave whose tiles are shared by the CTAs of a cluster (sch.ksplit > 1) or take several accumulation
+// segments.  A kernel of its own: with both kinds in one the plain launches of small K lose 10 % (336 x 3136 x 120: 16.5
+// -> 18.6 us), tiles of a pair up to 12 %.
+template <bool A_MN, bool B_MN, int BN, int PASSES, bool PAIR, int SG, bool SPLIT>
 __global__ void __launch_bounds__(Cfg<BN, PASSES, PAIR, SG>::NUM_THREADS, 1)
 gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
                float* __restrict__ C, int64_t ldc, float* __restrict__ Z, const float* __restrict__ bias_n, int M,
@@ -147,7 +155,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
   volatile int* s_skip = (volatile int*)(bars + 3 * STAGES + 6);   // [0] mine, [1] written by the peer CTA
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const bool ksplit = !PAIR && sch.ksplit > 1;   // (pairs take whole tiles: the spare registers of their 22 warps are few)
+  const bool ksplit = SPLIT && !PAIR && sch.ksplit > 1;   // (pairs take whole tiles: the spare registers of their 22 warps are few)
   const uint32_t crank = (PAIR || ksplit) ? cluster_ctarank() : 0u;
   const uint32_t rank = PAIR ? crank : 0u;   // half of the pair's tile
   const bool leader = (rank == 0);
@@ -256,7 +264,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
       int m0 = 0, nb0 = 0;
       int it = 0;   // k-blocks issued so far over all tiles: names the stage and its phase
       bool ok = true;
-      WorkIter wi(sch, cid, G);
+      WorkIter<SPLIT> wi(sch, cid, G);
       Portion p;
       while (ok && wi.next(sch, cid, G, num_kb, p)) {
         m0 = tile_m0(p.tile);
@@ -301,13 +309,12 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
                              ((uint32_t)(BN >> 3) << 17) | ((uint32_t)((PAIR ? 256 : BM) >> 4) << 24);
       bool ok = true;
       int it = 0, sc = 0;   // k-blocks and accumulation segments issued so far over all tiles
-      WorkIter wi(sch, cid, G);
+      WorkIter<SPLIT> wi(sch, cid, G);
       Portion p;
       while (ok && wi.next(sch, cid, G, num_kb, p))
-      for (int kb = p.kb0; kb < p.kb1 && ok; ++kb, ++it) {
+      for (int kb = p.kb0, kb_in_seg = 0; kb < p.kb1 && ok; ++kb, ++it) {
         const int s = it % STAGES;
         const uint32_t ph = (uint32_t)(it / STAGES) & 1u;
-        const int kb_in_seg = (kb - p.kb0) % SEG_KB;
         const int buf = sc & 1, use = sc >> 1;
         if (kb_in_seg == 0 && use > 0) {
           // the epilogue warps must have drained this accumulator buffer's previous segment
@@ -350,7 +357,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
             tc_mma_tf32(d_tmem, da_hi, db_hi, idesc, first);
           }
         }
-        const bool seg_end = (kb_in_seg == SEG_KB - 1 || kb == p.kb1 - 1);
+        const bool seg_end = (kb_in_seg == sch.seg - 1 || kb == p.kb1 - 1);
         if (PAIR) {
           tc_commit2_mc(empty_bar(s), (uint16_t)3);                 // frees the stage in both CTAs
           if (seg_end) tc_commit2_mc(tmem_full_bar(buf), (uint16_t)3);
@@ -358,6 +365,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
           tc_commit(empty_bar(s));
           if (seg_end) tc_commit(tmem_full_bar(buf));
         }
+        kb_in_seg = seg_end ? 0 : kb_in_seg + 1;
         if (seg_end) ++sc;
       }
     }
@@ -367,7 +375,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
     constexpr int RANKS = PAIR ? 2 : 1;
     bool ok = true;
     int sc = 0;                             // segments drained so far over all tiles
-    WorkIter wi(sch, cid, G);
+    WorkIter<SPLIT> wi(sch, cid, G);
     Portion p;
     while (ok && wi.next(sch, cid, G, num_kb, p)) {
       const int n0 = tile_n0(p.tile);
@@ -379,8 +387,9 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
       int* ticket = nullptr;
       const int row_off = (32 * q + lane) * 256;
       const int step_q = sch.U / G, step_r = sch.U % G;
-      if (ksplit) srow = sch.ws + (size_t)blockIdx.x * BM * 256 + row_off;   // only used beyond one segment
-      if (p.partial) {
+      // where earlier segments wait: the warp's 16-byte pieces of one column quad lie side by side
+      float4* park = SPLIT ? (float4*)(sch.ws + (size_t)blockIdx.x * BM * 256) + 32 * q + lane : nullptr;
+      if (!SPLIT && p.partial) {
         srow = sch.ws + (size_t)((2 * cid + p.trail) * RANKS + (int)rank) * BM * 256 + row_off;
         u_lo = p.tail_tile * sch.nu;
         const int u_hi = u_lo + sch.nu - 1;
@@ -425,7 +434,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
           rem = rem1;
         }
       };
-      const int nseg = (p.kb1 - p.kb0 + SEG_KB - 1) / SEG_KB;
+      const int nseg = (p.kb1 - p.kb0 + sch.seg - 1) / sch.seg;
       bool fused = false;
       for (int seg = 0; seg < nseg && ok; ++seg, ++sc) {
         const int buf = sc & 1, use = sc >> 1;
@@ -434,7 +443,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
         tc_fence_after();
         // later segments add into what the earlier ones left (round-to-nearest fp32 adds)
         const bool last = (seg == nseg - 1);
-        if (p.partial && last && cid == c_first) {
+        if (!SPLIT && p.partial && last && cid == c_first) {
           // The first part of a tile usually finishes last (it is the end of its CTA's range, the other parts are
           // the beginning of theirs).  When every other part has already drawn its ticket, their slots are
           // complete: add them to this last segment on its way out and write C directly.
@@ -452,24 +461,27 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
           tc_ld_32x32b_x32(tmem_base + ((uint32_t)(32 * q) << 16) + (uint32_t)(buf * BN + cc * 32), r);
           tc_wait_ld();
           float* v = reinterpret_cast<float*>(r);
-          if (ksplit) {
-            // earlier segments collect in this CTA's slot; the last one leaves the sums in shared memory (all MMAs have
-            // read their stages by now), from where the cluster adds them up
-            if (seg > 0) {
-              const float4* s4 = (const float4*)(srow + cc * 32);
+          if (SPLIT || !p.partial) {
+            if (SPLIT && seg > 0) {
 #pragma unroll
               for (int j = 0; j < 8; ++j) {
-                const float4 o = s4[j];
+                const float4 o = park[(8 * cc + j) * BM];
                 v[4 * j] += o.x; v[4 * j + 1] += o.y; v[4 * j + 2] += o.z; v[4 * j + 3] += o.w;
               }
             }
-            float4* d4 = last ? (float4*)((float*)smem + (32 * q + lane) * (BN + 4) + cc * 32) : (float4*)(srow + cc * 32);
+            if (SPLIT && !last) {
 #pragma unroll
-            for (int j = 0; j < 8; ++j) d4[j] = make_float4(v[4 * j], v[4 * j + 1], v[4 * j + 2], v[4 * j + 3]);
-          } else if (!p.partial) {
-            const bool add_c = (seg > 0) || (accumulate != 0);
+              for (int j = 0; j < 8; ++j) park[(8 * cc + j) * BM] = make_float4(v[4 * j], v[4 * j + 1], v[4 * j + 2], v[4 * j + 3]);
+            } else if (ksplit) {
+              // the sums go to shared memory (all MMAs have read their stages by now), from where the cluster adds them up
+              float4* d4 = (float4*)((float*)smem + (32 * q + lane) * (BN + 4) + cc * 32);
 #pragma unroll
-            for (int j = 0; j < 8; ++j) emit4(row, v + 4 * j, nb + 4 * j, add_c, last);
+              for (int j = 0; j < 8; ++j) d4[j] = make_float4(v[4 * j], v[4 * j + 1], v[4 * j + 2], v[4 * j + 3]);
+            } else {
+              const bool add_c = (!SPLIT && seg > 0) || (accumulate != 0);
+#pragma unroll
+              for (int j = 0; j < 8; ++j) emit4(row, v + 4 * j, nb + 4 * j, add_c, last);
+            }
           } else {
             float4* s4 = (float4*)(srow + cc * 32);
             if (seg > 0) {
@@ -498,7 +510,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
           else mbar_arrive(tmem_empty_bar(buf));
         }
       }
-      if (p.partial && ok) {
+      if (!SPLIT && p.partial && ok) {
         if (fused) {
           __syncwarp();
           if (lane == 0) *ticket = 0;   // every part is accounted for: ready for the next launch
@@ -535,7 +547,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
     bool ok = true;
     int total_kb = 0;   // the stage ring runs on across tiles
     {
-      WorkIter wi(sch, cid, G);
+      WorkIter<SPLIT> wi(sch, cid, G);
       Portion p;
       while (wi.next(sch, cid, G, num_kb, p)) total_kb += p.kb1 - p.kb0;
     }
@@ -612,11 +624,36 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
 
 // --------------------------------------------------------------------------- host side ---
 // Workspace of the split-tile schedule, owned by the context: slots for partial sums and the tickets.
+struct Plan {
+  int shape, ksplit, seg;   // tile shape (0, 1, 2: see plan_3xtf32), CTAs that share a tile, k-blocks per accumulation segment
+  bool split;               // the SPLIT kernel: one wave of shared tiles, or of tiles of several segments
+};
+
 struct GemmWorkspace {
   float* ws;
   int* tickets;
   int clusters[4];   // clusters of 1, 2, 4, 8 CTAs that are resident at once
 };
+
+// Accumulation segment of a launch of one wave.  An even cut of all k-blocks over the SMs gives each of them num_kb * tiles / SMs
+// (tiles: 256 x 256 by two SMs, 128 x 256 or 128 x 128, the largest that occupy half of the GPU); no truncating sum is longer
+// than that, nor than 1664 k-values, and where the tiles fill 3/4 of the SMs by themselves 2048: a shared tile is then at
+// least as exact as the tail split below would make it (104 x 1032 x 12256: 6.4e-6 of the result's norm).  Against one
+// segment for every CTA's range, up to 2048: 104 x 1032 x 12256 1.1e-5 in 62 us -> 4.0e-6 in 63, 1296 x 2216 x 1528 1.1e-5
+// -> 5.8e-6, both 76 us, 1024 x 1024 x 16384 1.5e-5 in 170 us -> 1.0e-5 in 163.
+int segment_kblocks(const fb_gemm_args& a, int num_kb, int part_kb, int sms, int* drains) {
+  const int64_t pairs = ((a.M + 255) / 256) * ((a.N + 255) / 256);
+  const int64_t t256 = ((a.M + BM - 1) / BM) * ((a.N + 255) / 256), t128 = ((a.M + BM - 1) / BM) * ((a.N + 127) / 128);
+  const int64_t tiles = a.M >= 256 && a.N >= 256 && 4 * pairs >= sms ? 2 * pairs : a.N <= 128 || 2 * t256 <= sms ? t128 : t256;
+  int64_t most = SEG_KB;
+  if (4 * tiles < 3 * (int64_t)sms) {
+    most = (int64_t)num_kb * tiles / sms;
+    most = most < UNIT_KB ? UNIT_KB : most > 104 ? 104 : most;
+  }
+  const int n = (int)((part_kb + most - 1) / most);
+  *drains = n - 1;
+  return (part_kb + n - 1) / n;
+}
 
 // 3-d view {32, K, MN / 32} of an MN-major matrix (row k holds MN contiguous floats): box {32, BK, chunks}.
 // Only for MN a multiple of 32, so that no chunk straddles the end of a row.
@@ -632,8 +669,8 @@ bool encode_map_mn3d(CUtensorMap* map, const float* base, int64_t K, int64_t MN,
   return r == CUDA_SUCCESS;
 }
 
-template <bool A_MN, bool B_MN, int BN, int PASSES, bool PAIR, int SG>
-int32_t launch_variant(fb_ctx* ctx, cudaStream_t stream, const fb_gemm_args& a, int ksplit) {
+template <bool A_MN, bool B_MN, int BN, int PASSES, bool PAIR, int SG, bool SPLIT>
+int32_t launch_variant(fb_ctx* ctx, cudaStream_t stream, const fb_gemm_args& a, const Plan& plan) {
   using cfg = Cfg<BN, PASSES, PAIR, SG>;
   CUtensorMap tmA, tmB;
   bool ok;
@@ -654,7 +691,7 @@ int32_t launch_variant(fb_ctx* ctx, cudaStream_t stream, const fb_gemm_args& a, 
   }
   if (!ok) return fb_fail(FB_ERR_CUDA, "gemm: cuTensorMapEncodeTiled failed (M=%lld N=%lld K=%lld lda=%lld ldb=%lld)",
                           (long long)a.M, (long long)a.N, (long long)a.K, (long long)a.lda, (long long)a.ldb);
-  auto kern = gemm_tc_kernel<A_MN, B_MN, BN, PASSES, PAIR, SG>;
+  auto kern = gemm_tc_kernel<A_MN, B_MN, BN, PASSES, PAIR, SG, SPLIT>;
   FB_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, cfg::SMEM_BYTES));
   // the whole L1 / shared array as shared memory: the communication-stream kernels ask for the same split, and an SM
   // takes CTAs of two kernels together only when their splits agree
@@ -675,7 +712,8 @@ int32_t launch_variant(fb_ctx* ctx, cudaStream_t stream, const fb_gemm_args& a, 
   sch.dp_tiles = (int)num_tiles;
   sch.nu = (num_kb + UNIT_KB - 1) / UNIT_KB;
   sch.U = 0;
-  sch.ksplit = ksplit;
+  sch.ksplit = plan.ksplit;
+  sch.seg = plan.seg;
   sch.ws = nullptr;
   sch.tickets = nullptr;
   int64_t G = Gmax < num_tiles ? Gmax : num_tiles;
@@ -683,8 +721,8 @@ int32_t launch_variant(fb_ctx* ctx, cudaStream_t stream, const fb_gemm_args& a, 
   // gain nothing: the kernel runs at the power limit, where idle SMs let the busy ones clock higher.)
   const int64_t rest = num_tiles % Gmax;
   const GemmWorkspace* gw = (const GemmWorkspace*)ctx->gemm_ws;
-  if (ksplit > 1) {
-    G = num_tiles * ksplit;
+  if (SPLIT) {
+    G = num_tiles * plan.ksplit;
     sch.ws = gw->ws;
   } else if (num_tiles > Gmax && rest != 0 && 4 * rest < 3 * Gmax && sch.nu > 1 && rest * sch.nu < 0x40000000 && gw != nullptr) {
     sch.dp_tiles = (int)(num_tiles - rest);
@@ -701,7 +739,7 @@ int32_t launch_variant(fb_ctx* ctx, cudaStream_t stream, const fb_gemm_args& a, 
   lc.stream = stream;
   cudaLaunchAttribute attr[1];
   attr[0].id = cudaLaunchAttributeClusterDimension;
-  attr[0].val.clusterDim.x = (PAIR ? 2 : 1) * ksplit;
+  attr[0].val.clusterDim.x = (PAIR ? 2 : 1) * plan.ksplit;
   attr[0].val.clusterDim.y = 1;
   attr[0].val.clusterDim.z = 1;
   lc.attrs = attr;
@@ -712,22 +750,23 @@ int32_t launch_variant(fb_ctx* ctx, cudaStream_t stream, const fb_gemm_args& a, 
   return FB_OK;
 }
 
-template <int BN, int PASSES, bool PAIR, int SG>
-int32_t launch_layout_sg(fb_ctx* ctx, cudaStream_t stream, const fb_gemm_args& a, int ksplit) {
+template <int BN, int PASSES, bool PAIR, int SG, bool SPLIT>
+int32_t launch_layout_sg(fb_ctx* ctx, cudaStream_t stream, const fb_gemm_args& a, const Plan& plan) {
   if (a.a_mn_major) {
-    if (a.b_mn_major) return launch_variant<true, true, BN, PASSES, PAIR, SG>(ctx, stream, a, ksplit);
-    return launch_variant<true, false, BN, PASSES, PAIR, SG>(ctx, stream, a, ksplit);
+    if (a.b_mn_major) return launch_variant<true, true, BN, PASSES, PAIR, SG, SPLIT>(ctx, stream, a, plan);
+    return launch_variant<true, false, BN, PASSES, PAIR, SG, SPLIT>(ctx, stream, a, plan);
   }
-  if (a.b_mn_major) return launch_variant<false, true, BN, PASSES, PAIR, SG>(ctx, stream, a, ksplit);
-  return launch_variant<false, false, BN, PASSES, PAIR, SG>(ctx, stream, a, ksplit);
+  if (a.b_mn_major) return launch_variant<false, true, BN, PASSES, PAIR, SG, SPLIT>(ctx, stream, a, plan);
+  return launch_variant<false, false, BN, PASSES, PAIR, SG, SPLIT>(ctx, stream, a, plan);
 }
 
 // Split-warp groups: the one-CTA tile is bound by shared-memory bandwidth and gains nothing beyond two groups; the
 // two-CTA tile is bound by the latency of one split (wait, load, store, proxy fence, remote arrive) and keeps
 // gaining up to four (measured 157 -> 175 -> 182 TFLOP/s for 2 -> 3 -> 4 groups at 4096^3).
-template <int BN, int PASSES, bool PAIR>
-int32_t launch_layout(fb_ctx* ctx, cudaStream_t stream, const fb_gemm_args& a, int ksplit) {
-  return launch_layout_sg<BN, PASSES, PAIR, (PAIR ? 4 : 2)>(ctx, stream, a, ksplit);
+template <int BN, bool PAIR>
+int32_t launch_layout(fb_ctx* ctx, cudaStream_t stream, const fb_gemm_args& a, const Plan& plan) {
+  constexpr int SG = PAIR ? 4 : 2;
+  return plan.split ? launch_layout_sg<BN, 3, PAIR, SG, true>(ctx, stream, a, plan) : launch_layout_sg<BN, 3, PAIR, SG, false>(ctx, stream, a, plan);
 }
 
 // Measured on B200 (4096^3, 3xTF32, persistent kernels): one-CTA 128 x 256 tiles 200-213 TFLOP/s (every MMA re-reads
@@ -738,16 +777,15 @@ int32_t launch_layout(fb_ctx* ctx, cudaStream_t stream, const fb_gemm_args& a, i
 // (2); ksplit CTAs of one cluster share a tile's K range where whole tiles would leave SMs idle.  The choice is
 // the smallest of the modelled times; its constants (us) are fitted to measurements on B200: a k-block of 16 costs
 // 0.53 / 0.62 / 0.62, a tile's prologue and epilogue that the next one does not hide 0.5 / 2.5 / 2.5, a launch 5, the
-// cluster's reduction 3.5.  A split runs in one wave (its clusters must all fit) so that a slot of the workspace belongs
-// to one CTA.  1024 x 1024 x 16384: 259 -> 158 us; 784 x 512 x 1024: 41 -> 17 us; 231 x 512 x 512: 27 -> 12 us.
-struct Plan { int shape, ksplit; };
+// cluster's reduction 3.5, an accumulation segment that waits for the next one 2.5.  A split runs in one wave (its clusters
+// must all fit) so that a slot of the workspace belongs to one CTA.  1024 x 1024 x 16384: 259 -> 158 us; 784 x 512 x 1024: 41 -> 17 us; 231 x 512 x 512: 27 -> 12 us.
 Plan plan_3xtf32(fb_ctx* ctx, const fb_gemm_args& a, bool force_pair) {
   const GemmWorkspace* gw = (const GemmWorkspace*)ctx->gemm_ws;
   const int sms = ctx->sm_count - ctx->reserved_sms;
   const int num_kb = (int)((a.K + BK - 1) / BK);
   static const int bm[3] = {128, 128, 256}, bn[3] = {128, 256, 256};
   static const double t_kb[3] = {0.53, 0.62, 0.62}, t_tile[3] = {0.5, 2.5, 2.5};
-  Plan best = {0, 1};
+  Plan best = {0, 1, SEG_KB, false};
   double best_t = 1e30;
   for (int sh = 2; sh >= 0; --sh) {
     if (sh == 2 && (a.M < 256 || a.N < 256)) continue;
@@ -758,17 +796,22 @@ Plan plan_3xtf32(fb_ctx* ctx, const fb_gemm_args& a, bool force_pair) {
     for (int lg = 0; lg < 4; ++lg) {
       const int s = 1 << lg;
       double t;
+      int seg = SEG_KB, drains = 0;   // of a launch of one wave: accumulation segment, segments before the last
       if (s == 1) {
         const int64_t slots = sms / ranks > 0 ? sms / ranks : 1;
         double waves = (double)((tiles + slots - 1) / slots);
         const int64_t rest = tiles % slots;
         if (tiles > slots && rest != 0 && 4 * rest < 3 * slots && num_kb > UNIT_KB) waves = (double)tiles / (double)slots + 0.15;   // the tail is split
         t = 5.0 + waves * (num_kb * t_kb[sh] + t_tile[sh]);
+        if (tiles <= slots && gw != nullptr) seg = segment_kblocks(a, num_kb, num_kb, sms, &drains);
       } else {
         if (sh == 2 || gw == nullptr || ctx->reserved_sms != 0 || num_kb < 2 * s || tiles > gw->clusters[lg]) break;
-        t = 8.5 + ((num_kb + s - 1) / s) * t_kb[sh] + t_tile[sh];
+        const int part_kb = (num_kb + s - 1) / s;
+        t = 8.5 + part_kb * t_kb[sh] + t_tile[sh];
+        seg = segment_kblocks(a, num_kb, part_kb, sms, &drains);
       }
-      if (t < best_t) { best_t = t; best.shape = sh; best.ksplit = s; }
+      t += 2.5 * drains;
+      if (t < best_t) { best_t = t; best = {sh, s, seg, s > 1 || drains > 0}; }
     }
   }
   return best;
@@ -776,7 +819,7 @@ Plan plan_3xtf32(fb_ctx* ctx, const fb_gemm_args& a, bool force_pair) {
 
 // How many clusters of 2, 4 and 8 CTAs with the GEMM's shared memory are resident at once.
 void query_clusters(fb_ctx* ctx, int* clusters) {
-  auto kern = gemm_tc_kernel<false, true, 256, 3, false, 2>;
+  auto kern = gemm_tc_kernel<false, true, 256, 3, false, 2, true>;
   using cfg = Cfg<256, 3, false, 2>;
   clusters[0] = ctx->sm_count;
   for (int lg = 1; lg < 4; ++lg) {
@@ -821,12 +864,13 @@ int32_t fb_gemm_tc_launch(fb_ctx* ctx, cudaStream_t stream, const fb_gemm_args& 
   if (!fb_gemm_tc_supported(a)) return FB_ERR_UNSUPPORTED;
   if (passes == 1) {
     const bool narrow1 = (a.N <= 128) || (2 * ((a.M + BM - 1) / BM) * ((a.N + 255) / 256) <= ctx->sm_count);
-    return narrow1 ? launch_layout<128, 1, false>(ctx, stream, a, 1) : launch_layout<256, 1, false>(ctx, stream, a, 1);
+    const Plan whole = {0, 1, SEG_KB, false};
+    return narrow1 ? launch_layout_sg<128, 1, false, 2, false>(ctx, stream, a, whole) : launch_layout_sg<256, 1, false, 2, false>(ctx, stream, a, whole);
   }
   const Plan p = plan_3xtf32(ctx, a, passes == 32);
-  if (p.shape == 0) return launch_layout<128, 3, false>(ctx, stream, a, p.ksplit);
-  if (p.shape == 1) return launch_layout<256, 3, false>(ctx, stream, a, p.ksplit);
-  return launch_layout<256, 3, true>(ctx, stream, a, p.ksplit);
+  if (p.shape == 0) return launch_layout<128, false>(ctx, stream, a, p);
+  if (p.shape == 1) return launch_layout<256, false>(ctx, stream, a, p);
+  return launch_layout<256, true>(ctx, stream, a, p);
 }
 
 // Called by fb_ctx_create / fb_ctx_destroy.  The workspace is allocated up front (2 slots of 128 x 256 floats per
