@@ -627,6 +627,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
 struct Plan {
   int shape, ksplit, seg;   // tile shape (0, 1, 2: see plan_3xtf32), CTAs that share a tile, k-blocks per accumulation segment
   bool split;               // the SPLIT kernel: one wave of shared tiles, or of tiles of several segments
+  bool tail;                // the last wave is cut along K and dealt out over all CTAs
 };
 
 struct GemmWorkspace {
@@ -717,14 +718,12 @@ int32_t launch_variant(fb_ctx* ctx, cudaStream_t stream, const fb_gemm_args& a, 
   sch.ws = nullptr;
   sch.tickets = nullptr;
   int64_t G = Gmax < num_tiles ? Gmax : num_tiles;
-  // A last wave that fills less than 3/4 of the machine is cut along K and spread over all CTAs.  (Fuller waves
-  // gain nothing: the kernel runs at the power limit, where idle SMs let the busy ones clock higher.)
   const int64_t rest = num_tiles % Gmax;
   const GemmWorkspace* gw = (const GemmWorkspace*)ctx->gemm_ws;
   if (SPLIT) {
     G = num_tiles * plan.ksplit;
     sch.ws = gw->ws;
-  } else if (num_tiles > Gmax && rest != 0 && 4 * rest < 3 * Gmax && sch.nu > 1 && rest * sch.nu < 0x40000000 && gw != nullptr) {
+  } else if (plan.tail && rest * sch.nu < 0x40000000) {
     sch.dp_tiles = (int)(num_tiles - rest);
     sch.U = (int)(rest * sch.nu);
     sch.ws = gw->ws;
@@ -778,14 +777,28 @@ int32_t launch_layout(fb_ctx* ctx, cudaStream_t stream, const fb_gemm_args& a, c
 // the smallest of the modelled times; its constants (us) are fitted to measurements on B200: a k-block of 16 costs
 // 0.53 / 0.62 / 0.62, a tile's prologue and epilogue that the next one does not hide 0.5 / 2.5 / 2.5, a launch 5, the
 // cluster's reduction 3.5, an accumulation segment that waits for the next one 2.5.  A split runs in one wave (its clusters
-// must all fit) so that a slot of the workspace belongs to one CTA.  1024 x 1024 x 16384: 259 -> 158 us; 784 x 512 x 1024: 41 -> 17 us; 231 x 512 x 512: 27 -> 12 us.
+// must all fit) so that a slot of the workspace belongs to one CTA.  1024 x 1024 x 16384: 259 -> 158 us; 784 x 512 x 1024:
+// 41 -> 17 us; 231 x 512 x 512: 27 -> 12 us.
+//
+// tail_time: `rest` tiles cut into units of UNIT_KB k-blocks, dealt out over all slots: the units of the longest range, and
+// the sums of a tile's parts, which its last CTA adds up by itself (12 us and 5 for each part).  Without the units' rounding
+// 7000 x 280 x 592 looked best as 128 x 128 tiles with 17 of 165 in the tail (57 us; 43 as pairs), 1240 x 4960 x 4896 as
+// 128 x 256 tiles (350 us; 325 as pairs).
+double tail_time(int64_t rest, int64_t slots, int num_kb, double t_kb, double t_tile) {
+  const int64_t nu = (num_kb + UNIT_KB - 1) / UNIT_KB;
+  if (nu < 2) return 1e30;
+  const int64_t units = (rest * nu + slots - 1) / slots;
+  const double kb = (double)(units * UNIT_KB < num_kb ? units * UNIT_KB : num_kb);
+  return kb * t_kb + t_tile + 12.0 + 5.0 * (double)(nu / units + 1);
+}
+
 Plan plan_3xtf32(fb_ctx* ctx, const fb_gemm_args& a, bool force_pair) {
   const GemmWorkspace* gw = (const GemmWorkspace*)ctx->gemm_ws;
   const int sms = ctx->sm_count - ctx->reserved_sms;
   const int num_kb = (int)((a.K + BK - 1) / BK);
   static const int bm[3] = {128, 128, 256}, bn[3] = {128, 256, 256};
   static const double t_kb[3] = {0.53, 0.62, 0.62}, t_tile[3] = {0.5, 2.5, 2.5};
-  Plan best = {0, 1, SEG_KB, false};
+  Plan best = {0, 1, SEG_KB, false, false};
   double best_t = 1e30;
   for (int sh = 2; sh >= 0; --sh) {
     if (sh == 2 && (a.M < 256 || a.N < 256)) continue;
@@ -796,14 +809,26 @@ Plan plan_3xtf32(fb_ctx* ctx, const fb_gemm_args& a, bool force_pair) {
     for (int lg = 0; lg < 4; ++lg) {
       const int s = 1 << lg;
       double t;
+      bool tail = false;
       int seg = SEG_KB, drains = 0;   // of a launch of one wave: accumulation segment, segments before the last
       if (s == 1) {
         const int64_t slots = sms / ranks > 0 ? sms / ranks : 1;
-        double waves = (double)((tiles + slots - 1) / slots);
-        const int64_t rest = tiles % slots;
-        if (tiles > slots && rest != 0 && 4 * rest < 3 * slots && num_kb > UNIT_KB) waves = (double)tiles / (double)slots + 0.15;   // the tail is split
-        t = 5.0 + waves * (num_kb * t_kb[sh] + t_tile[sh]);
-        if (tiles <= slots && gw != nullptr) seg = segment_kblocks(a, num_kb, num_kb, sms, &drains);
+        const int64_t full = tiles / slots, rest = tiles % slots;
+        t = 5.0 + full * (num_kb * t_kb[sh] + t_tile[sh]);
+        const double whole = num_kb * t_kb[sh] + t_tile[sh];
+        if (full == 0) {
+          // one wave: whole tiles, or their units over all CTAs
+          if (gw != nullptr) seg = segment_kblocks(a, num_kb, num_kb, sms, &drains);
+          const double cut = tail_time(rest, slots, num_kb, t_kb[sh], t_tile[sh]);
+          tail = cut < whole + 2.5 * drains;
+          if (tail) { seg = SEG_KB; drains = 0; }
+          t += tail ? cut : whole;
+        } else if (rest != 0) {
+          // A last wave that fills less than 3/4 of the machine is always cut.  (Fuller waves gain nothing: the kernel runs at
+          // the power limit, where idle SMs let the busy ones clock higher.)
+          tail = 4 * rest < 3 * slots && num_kb > UNIT_KB && gw != nullptr;
+          t += tail ? tail_time(rest, slots, num_kb, t_kb[sh], t_tile[sh]) : whole;
+        }
       } else {
         if (sh == 2 || gw == nullptr || ctx->reserved_sms != 0 || num_kb < 2 * s || tiles > gw->clusters[lg]) break;
         const int part_kb = (num_kb + s - 1) / s;
@@ -811,7 +836,7 @@ Plan plan_3xtf32(fb_ctx* ctx, const fb_gemm_args& a, bool force_pair) {
         seg = segment_kblocks(a, num_kb, part_kb, sms, &drains);
       }
       t += 2.5 * drains;
-      if (t < best_t) { best_t = t; best = {sh, s, seg, s > 1 || drains > 0}; }
+      if (t < best_t) { best_t = t; best = {sh, s, seg, s > 1 || drains > 0, tail}; }
     }
   }
   return best;
@@ -864,7 +889,9 @@ int32_t fb_gemm_tc_launch(fb_ctx* ctx, cudaStream_t stream, const fb_gemm_args& 
   if (!fb_gemm_tc_supported(a)) return FB_ERR_UNSUPPORTED;
   if (passes == 1) {
     const bool narrow1 = (a.N <= 128) || (2 * ((a.M + BM - 1) / BM) * ((a.N + 255) / 256) <= ctx->sm_count);
-    const Plan whole = {0, 1, SEG_KB, false};
+    // (TF32 in one pass: the last wave is cut as it always was)
+    const int64_t slots = ctx->sm_count - ctx->reserved_sms, rest = (((a.M + BM - 1) / BM) * ((a.N + (narrow1 ? 127 : 255)) / (narrow1 ? 128 : 256))) % slots;
+    const Plan whole = {0, 1, SEG_KB, false, ctx->gemm_ws != nullptr && rest != 0 && 4 * rest < 3 * slots && a.K > BK * UNIT_KB};
     return narrow1 ? launch_layout_sg<128, 1, false, 2, false>(ctx, stream, a, whole) : launch_layout_sg<256, 1, false, 2, false>(ctx, stream, a, whole);
   }
   const Plan p = plan_3xtf32(ctx, a, passes == 32);

@@ -52,7 +52,7 @@ def test_gemm_f32_cuts(ctx, ta, tb, m, n, k, pad, accumulate):
 
 # few tiles and long K: K split over 8, 4 and 2 CTAs, whole tiles of one wave, pairs
 @pytest.mark.parametrize("m,n,k,even", [(104, 1032, 12256, 745), (240, 736, 12624, 1023), (192, 104, 5760, 512), (64, 4096, 4096, 885),
-                                        (512, 512, 16384, 1664), (1024, 1024, 16384, 1664), (1296, 2216, 1528, 1115),
+                                        (512, 512, 16384, 1664), (1024, 1024, 16384, 1664), (1296, 2216, 1528, 1115), (5184, 512, 1216, 690),
                                         (672, 4288, 6008, 1664), (4096, 1024, 4096, 2048)])
 def test_truncating_sums_are_no_longer_than_an_even_cut(ctx, m, n, k, even):
     """The tensor core truncates while it accumulates: 7.3e-9 of the result's norm per k-value of one accumulation (measured
@@ -67,6 +67,37 @@ def test_truncating_sums_are_no_longer_than_an_even_cut(ctx, m, n, k, even):
                  0, 0)
         err = float((out.double() - ref).norm() / ref.norm())
         assert err < 8.5e-9 * even, err
+
+
+def test_reserved_sms_keep_the_k_split(ctx):
+    """With SMs left to communication kernels no clusters are used; 16 tiles of 1024 k-blocks still spread over the others
+    (a whole tile each takes six times as long), and the results are those of a product."""
+    from fluxb200 import lib
+    m = n = 512
+    A, B, ref = _operands(0, 0, m, n, 16384, 0, torch.float32)
+    out = torch.empty(n, m, device="cuda")
+
+    def product():
+        lib.call("fb_gemm_f32", ctx.handle, ctx.stream, 0, 0, m, n, 16384, A.data_ptr(), m, B.data_ptr(), 16384, out.data_ptr(), m, 0, 0)
+
+    def time_us():
+        for _ in range(3):
+            product()
+        start, end = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+        start.record()
+        for _ in range(10):
+            product()
+        end.record()
+        torch.cuda.synchronize()
+        return start.elapsed_time(end) * 100
+    free = time_us()
+    ctx.set_reserved_sms(8)
+    try:
+        reserved = time_us()
+        assert ((out.double() - ref).norm() / ref.norm()) < 3e-5
+    finally:
+        ctx.set_reserved_sms(0)
+    assert reserved < 3 * free, (reserved, free)
 
 
 # an odd leading dimension of one operand, of the result alone, and a start off the 16-byte boundary
