@@ -236,6 +236,9 @@ int32_t fb_gemm_simt_launch(fb_ctx* ctx, cudaStream_t stream, const fb_gemm_args
 // alignment is outside what the kernel handles, so the dispatcher can pick the FMA kernel.
 int32_t fb_gemm_tc_launch(fb_ctx* ctx, cudaStream_t stream, const fb_gemm_args& a, int passes);
 bool fb_gemm_tc_supported(const fb_gemm_args& a);
+// the time (us) that the kernel's own plan expects
+double fb_gemm_tc_time(fb_ctx* ctx, const fb_gemm_args& a);
+double fb_gemm_simt_time(const fb_ctx* ctx, const fb_gemm_args& a);
 int32_t fb_gemm_dispatch(fb_ctx* ctx, cudaStream_t stream, const fb_gemm_args& a, int precision);
 void fb_gemm_workspace_destroy(fb_ctx* ctx);
 // clusters of `size` (2, 4, 8) CTAs that hold an SM each and are resident at once

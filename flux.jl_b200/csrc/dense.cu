@@ -49,12 +49,15 @@ int32_t fb_gemm_dispatch(fb_ctx* ctx, cudaStream_t stream, const fb_gemm_args& a
       // Below about 1e8 multiply-adds the FMA kernel ends before the tensor-core kernel's fixed cost (barriers, tensor
       // memory, operand split, read-back: ~9 us with a split K range) is paid: 231 x 512 x 512 9 us against 12, 512 x 512
       // x 512 14.6 against 12.7, 1024 x 512 x 784 32 against 16.  With fewer than 32 rows, columns or k-values most of a
-      // 128-wide tile is padding.
+      // 128-wide tile is padding; 17 to 31 rows, for which the FMA kernel pads too, go to the kernel whose plan expects the
+      // shorter time (24 x 8192 x 8192: FMA 190 us, tensor cores 93; 24 x 4096 x 1024: 21 against 23).
       // Operands or results whose rows are not 16-byte aligned stay on the FMA kernel: copies with padded rows would let the
       // tensor cores take them faster (1001 x 1003 x 1005 in 48 us against 87, 4095^3 in 1.06 ms against 3.9), but with
       // 3xTF32's errors (2.1e-6 against 5.7e-7, 1.5e-5 against 1.1e-6) and a NaN for every product with an infinite factor.
       const double macs = (double)a.M * (double)a.N * (double)a.K;
-      if (macs >= 1.0e8 && a.K >= 32 && a.N >= 32 && a.M >= 32 && fb_gemm_tc_supported(a)) return fb_gemm_tc_launch(ctx, stream, a, 3);
+      if (macs >= 1.0e8 && a.K >= 32 && a.N >= 32 && a.M > 16 && fb_gemm_tc_supported(a) &&
+          (a.M >= 32 || fb_gemm_tc_time(ctx, a) < fb_gemm_simt_time(ctx, a)))
+        return fb_gemm_tc_launch(ctx, stream, a, 3);
       return fb_gemm_simt_launch(ctx, stream, a);
     }
     default:

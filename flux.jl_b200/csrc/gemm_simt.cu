@@ -271,8 +271,12 @@ int32_t launch_fma_layout(fb_ctx* ctx, cudaStream_t stream, const fb_gemm_args& 
 // measured on B200 at 1.0 us for a 64 x 64 tile, 0.55 for 32 x 64 and 0.3 for the 16-wide ones (taken where a dimension
 // is at most 16 and a wider tile would compute padding), plus 1 us for a cluster's reduction.  About 15 / 33 / 74 clusters
 // of 8 / 4 / 2 CTAs with an SM each are resident at once.
-int32_t fb_gemm_simt_launch(fb_ctx* ctx, cudaStream_t stream, const fb_gemm_args& a) {
-  if (a.M == 0 || a.N == 0) return FB_OK;
+namespace {
+struct FmaPlan {
+  int thin, half, splits;   // 16-wide tile of rows (1) or columns (2); 32 x 64 instead of 64 x 64; CTAs that share K
+  double time;
+};
+FmaPlan plan_fma(const fb_ctx* ctx, const fb_gemm_args& a) {
   const int thin = a.M <= 16 ? 1 : a.N <= 16 ? 2 : 0;
   const int64_t stages = (a.K + BK - 1) / BK;
   const int slots[4] = {ctx->sm_count, ctx->sm_count / 2, ctx->sm_count * 33 / 148, ctx->sm_count * 15 / 148};
@@ -291,8 +295,17 @@ int32_t fb_gemm_simt_launch(fb_ctx* ctx, cudaStream_t stream, const fb_gemm_args
       if (t < best_t) { best_t = t; best_half = half; best_splits = s; }
     }
   }
-  if (thin == 1) return launch_fma_layout<16, 64, 4, 4>(ctx, stream, a, best_splits);
-  if (thin == 2) return launch_fma_layout<64, 16, 4, 4>(ctx, stream, a, best_splits);
-  if (best_half) return launch_fma_layout<32, 64, 4, 4>(ctx, stream, a, best_splits);
-  return launch_fma_layout<64, 64, 4, 4>(ctx, stream, a, best_splits);
+  return {thin, best_half, best_splits, best_t};
+}
+}  // namespace
+
+double fb_gemm_simt_time(const fb_ctx* ctx, const fb_gemm_args& a) { return plan_fma(ctx, a).time; }
+
+int32_t fb_gemm_simt_launch(fb_ctx* ctx, cudaStream_t stream, const fb_gemm_args& a) {
+  if (a.M == 0 || a.N == 0) return FB_OK;
+  const FmaPlan p = plan_fma(ctx, a);
+  if (p.thin == 1) return launch_fma_layout<16, 64, 4, 4>(ctx, stream, a, p.splits);
+  if (p.thin == 2) return launch_fma_layout<64, 16, 4, 4>(ctx, stream, a, p.splits);
+  if (p.half) return launch_fma_layout<32, 64, 4, 4>(ctx, stream, a, p.splits);
+  return launch_fma_layout<64, 64, 4, 4>(ctx, stream, a, p.splits);
 }

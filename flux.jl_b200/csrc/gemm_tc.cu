@@ -625,6 +625,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
 // --------------------------------------------------------------------------- host side ---
 // Workspace of the split-tile schedule, owned by the context: slots for partial sums and the tickets.
 struct Plan {
+  double time;              // modelled, us
   int shape, ksplit, seg;   // tile shape (0, 1, 2: see plan_3xtf32), CTAs that share a tile, k-blocks per accumulation segment
   bool split;               // the SPLIT kernel: one wave of shared tiles, or of tiles of several segments
   bool tail;                // the last wave is cut along K and dealt out over all CTAs
@@ -798,11 +799,10 @@ Plan plan_3xtf32(fb_ctx* ctx, const fb_gemm_args& a, bool force_pair) {
   const int num_kb = (int)((a.K + BK - 1) / BK);
   static const int bm[3] = {128, 128, 256}, bn[3] = {128, 256, 256};
   static const double t_kb[3] = {0.53, 0.62, 0.62}, t_tile[3] = {0.5, 2.5, 2.5};
-  Plan best = {0, 1, SEG_KB, false, false};
-  double best_t = 1e30;
+  Plan best = {1e30, 0, 1, SEG_KB, false, false};
   for (int sh = 2; sh >= 0; --sh) {
     if (sh == 2 && (a.M < 256 || a.N < 256)) continue;
-    if (force_pair && sh != 2 && best_t < 1e30) continue;
+    if (force_pair && sh != 2 && best.time < 1e30) continue;
     if (sh == 1 && a.N <= 128) continue;
     const int ranks = sh == 2 ? 2 : 1;
     const int64_t tiles = ((a.M + bm[sh] - 1) / bm[sh]) * ((a.N + bn[sh] - 1) / bn[sh]);
@@ -836,7 +836,7 @@ Plan plan_3xtf32(fb_ctx* ctx, const fb_gemm_args& a, bool force_pair) {
         seg = segment_kblocks(a, num_kb, part_kb, sms, &drains);
       }
       t += 2.5 * drains;
-      if (t < best_t) { best_t = t; best = {sh, s, seg, s > 1 || drains > 0, tail}; }
+      if (t < best.time) best = {t, sh, s, seg, s > 1 || drains > 0, tail};
     }
   }
   return best;
@@ -884,6 +884,8 @@ bool fb_gemm_tc_supported(const fb_gemm_args& a) {
   return true;
 }
 
+double fb_gemm_tc_time(fb_ctx* ctx, const fb_gemm_args& a) { return plan_3xtf32(ctx, a, false).time; }
+
 // passes: 3 = 3xTF32, 1 = one TF32 pass, 32 = 3xTF32 on two-CTA tiles where the shape allows
 int32_t fb_gemm_tc_launch(fb_ctx* ctx, cudaStream_t stream, const fb_gemm_args& a, int passes) {
   if (!fb_gemm_tc_supported(a)) return FB_ERR_UNSUPPORTED;
@@ -891,7 +893,7 @@ int32_t fb_gemm_tc_launch(fb_ctx* ctx, cudaStream_t stream, const fb_gemm_args& 
     const bool narrow1 = (a.N <= 128) || (2 * ((a.M + BM - 1) / BM) * ((a.N + 255) / 256) <= ctx->sm_count);
     // (TF32 in one pass: the last wave is cut as it always was)
     const int64_t slots = ctx->sm_count - ctx->reserved_sms, rest = (((a.M + BM - 1) / BM) * ((a.N + (narrow1 ? 127 : 255)) / (narrow1 ? 128 : 256))) % slots;
-    const Plan whole = {0, 1, SEG_KB, false, ctx->gemm_ws != nullptr && rest != 0 && 4 * rest < 3 * slots && a.K > BK * UNIT_KB};
+    const Plan whole = {0.0, 0, 1, SEG_KB, false, ctx->gemm_ws != nullptr && rest != 0 && 4 * rest < 3 * slots && a.K > BK * UNIT_KB};
     return narrow1 ? launch_layout_sg<128, 1, false, 2, false>(ctx, stream, a, whole) : launch_layout_sg<256, 1, false, 2, false>(ctx, stream, a, whole);
   }
   const Plan p = plan_3xtf32(ctx, a, passes == 32);

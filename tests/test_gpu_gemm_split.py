@@ -100,6 +100,33 @@ def test_reserved_sms_keep_the_k_split(ctx):
     assert reserved < 3 * free, (reserved, free)
 
 
+@pytest.mark.parametrize("rows", [17, 31])
+@pytest.mark.parametrize("out_dim,in_dim", [(8192, 8192), (16384, 4096), (4096, 1024)])
+def test_few_rows_go_to_the_faster_kernel(ctx, rows, out_dim, in_dim):
+    """17 to 31 rows: the default precision takes no more than 1.3 times what the better of the two kernels takes (the FMA
+    kernel needs twice the tensor cores' time at the largest of these sizes)."""
+    from fluxb200 import lib
+    A, B, ref = _operands(0, 0, out_dim, rows, in_dim, 0, torch.float32)
+    out = torch.empty(rows, out_dim, device="cuda")
+
+    def time_us(precision):
+        def product():
+            lib.call("fb_gemm_f32", ctx.handle, ctx.stream, 0, 0, out_dim, rows, in_dim, A.data_ptr(), out_dim, B.data_ptr(), in_dim,
+                     out.data_ptr(), out_dim, 0, precision)
+        for _ in range(3):
+            product()
+        start, end = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+        start.record()
+        for _ in range(20):
+            product()
+        end.record()
+        torch.cuda.synchronize()
+        return start.elapsed_time(end) * 50
+    fma, tc, default = time_us(lib.PREC["fp32_simt"]), time_us(lib.PREC["3xtf32"]), time_us(lib.PREC["default"])
+    assert default < 1.3 * min(fma, tc), (fma, tc, default)
+    assert ((out.double() - ref).norm() / ref.norm()) < 3e-5
+
+
 # an odd leading dimension of one operand, of the result alone, and a start off the 16-byte boundary
 @pytest.mark.parametrize("ta,tb", [(0, 0), (1, 0), (0, 1), (1, 1)])
 @pytest.mark.parametrize("m,n,k,lda,ldb,ldc,shift", [(1001, 1003, 1005, 0, 0, 0, 0), (512, 1024, 2048, 1, 0, 0, 0), (512, 1024, 2048, 0, 3, 0, 0),
