@@ -1063,7 +1063,8 @@ int32_t fb_attn_fwd_tc(fb_ctx* ctx, cudaStream_t stream, const float* q, const f
 }
 
 // *did_kv, *did_q: which part was done.  dQ, dK and dV accumulate in tensor memory with truncating adds; beyond 2048 keys
-// (queries), and for the other head sizes, the FMA kernels are the more accurate ones.
+// (queries), for the other head sizes and for unaligned arrays, the FMA kernels are the more accurate ones (8 heads of 64,
+// 512 x 512: dQ 4e-7, dK and dV 6e-7 of the norm in 245 us, here 1.4e-6 and 5e-6 in 87).
 int32_t fb_attn_bwd_tc(fb_ctx* ctx, cudaStream_t stream, const float* q, const float* k, const float* v, const uint8_t* mask, const float* o,
                        const float* lse, const float* dout, float* dq, float* dk, float* dv, int64_t e_dim, int64_t ev_dim, int64_t lq,
                        int64_t lk, int64_t batch, int nheads, int causal, bool* did_kv, bool* did_q) {
@@ -1072,11 +1073,11 @@ int32_t fb_attn_bwd_tc(fb_ctx* ctx, cudaStream_t stream, const float* q, const f
   if (!attn_tc_enabled() || !attn_bwd_tc_enabled() || mask != nullptr || !make_plan(&P, 3, e_dim, ev_dim, lq, lk, batch, nheads, causal) ||
       P.D.d != HD || P.D.dv != HD)
     return FB_ERR_UNSUPPORTED;
-  const bool kv = lq <= BWD_MAX_BLOCKS * KT, qq = lk <= BWD_MAX_BLOCKS * KT;
+  // (arrays off the 16-byte boundary have always been the FMA kernels')
+  if (!fb_aligned16(q) || !fb_aligned16(k) || !fb_aligned16(v) || !fb_aligned16(dout)) return FB_ERR_UNSUPPORTED;
+  const bool kv = lq <= BWD_MAX_BLOCKS * KT && fb_aligned16(dk) && fb_aligned16(dv), qq = lk <= BWD_MAX_BLOCKS * KT && fb_aligned16(dq);
   if (!kv && !qq) return FB_ERR_UNSUPPORTED;
-  if (!fb_aligned16(q) || !fb_aligned16(k) || !fb_aligned16(v) || !fb_aligned16(o) || !fb_aligned16(dout) || !fb_aligned16(dq) ||
-      !fb_aligned16(dk) || !fb_aligned16(dv))
-    P.D.vec = 0;
+  if (!fb_aligned16(o)) P.D.vec = 0;
   const int32_t st = bwd_impl<3>(ctx, stream, (const uint8_t*)q, (const uint8_t*)k, (const uint8_t*)v, o, lse, (const uint8_t*)dout,
                                  (uint8_t*)dq, (uint8_t*)dk, (uint8_t*)dv, P, batch, kv, qq);
   if (st == FB_OK) {
@@ -1088,7 +1089,8 @@ int32_t fb_attn_bwd_tc(fb_ctx* ctx, cudaStream_t stream, const float* q, const f
 
 // The same for bf16 q, k, v (and dO): one plane each, outputs rounded to bf16 once.  o32 (optional in the forward call) keeps
 // the Float32 output for the backward pass.  FB_ERR_UNSUPPORTED, without a message, for every call these kernels do not
-// take: the caller then casts and takes the Float32 entry points, which also report what is wrong with a bad one.
+// take: the caller then casts and takes the Float32 entry points, which also report what is wrong with a bad one.  The
+// backward call takes the head size of the Float32 one, for the same reason.
 FB_API int32_t fb_attn_fwd_bf16(fb_ctx* ctx, void* stream, const uint16_t* q, const uint16_t* k, const uint16_t* v, float* o32, uint16_t* o,
                                 float* lse, int64_t e_dim, int64_t ev_dim, int64_t lq, int64_t lk, int64_t batch, int32_t nheads,
                                 int32_t causal) {
@@ -1108,7 +1110,7 @@ FB_API int32_t fb_attn_bwd_bf16(fb_ctx* ctx, void* stream, const uint16_t* q, co
   AtcPlan P;
   if (!attn_tc_enabled() || !attn_bwd_tc_enabled() || !q || !k || !v || !o32 || !lse || !dout || !dq || !dk || !dv || nheads < 1 ||
       e_dim % nheads != 0 || ev_dim % nheads != 0 || batch * nheads > 65535 || lq > BWD_MAX_BLOCKS * KT || lk > BWD_MAX_BLOCKS * KT ||
-      !make_plan(&P, 1, e_dim, ev_dim, lq, lk, batch, nheads, causal))
+      !make_plan(&P, 1, e_dim, ev_dim, lq, lk, batch, nheads, causal) || P.D.d != HD || P.D.dv != HD)
     return FB_ERR_UNSUPPORTED;
   if (!fb_aligned16(q) || !fb_aligned16(k) || !fb_aligned16(v) || !fb_aligned16(o32) || !fb_aligned16(dout) || !fb_aligned16(dq) ||
       !fb_aligned16(dk) || !fb_aligned16(dv))

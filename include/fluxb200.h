@@ -438,8 +438,8 @@ int32_t fb_attn_scores_ex(fb_ctx* ctx, void* stream, const float* q, const float
 /* fb_attn_fwd / fb_attn_bwd on bf16 q, k, v, o and gradients (16-bit storage, Float32 arithmetic; every product of
  * probabilities keeps their 24 bits), without mask, bias and dropout.  o32 is the Float32 output that the backward pass
  * reads (the forward call takes NULL where none follows).  FB_ERR_UNSUPPORTED for shapes these kernels do not take (head
- * sizes above 64 or not multiples of 8, in the backward pass more than 2048 queries or keys, unaligned arrays): cast and
- * use the calls above. */
+ * sizes above 64 or not multiples of 8, in the backward pass other than 64 or more than 2048 queries or keys, unaligned
+ * arrays): cast and use the calls above. */
 int32_t fb_attn_fwd_bf16(fb_ctx* ctx, void* stream, const uint16_t* q, const uint16_t* k, const uint16_t* v, float* o32,
                          uint16_t* o, float* lse, int64_t e_dim, int64_t ev_dim, int64_t lq, int64_t lk, int64_t batch,
                          int32_t nheads, int32_t causal);

@@ -89,6 +89,55 @@ def test_attention_bf16(d, heads, lq, lk, causal):
     assert float((a.sum(-1) - 1).abs().max()) < 1e-4
 
 
+@pytest.mark.parametrize("lq,lk,causal", [(512, 512, 1), (130, 700, 0)])
+def test_backward_of_unaligned_arrays_keeps_float32_sums(lq, lk, causal):
+    """Arrays 4 bytes past a 16-byte boundary are the FMA kernels' in the backward pass: two chained sums of at most 700 terms
+    with rounding to nearest, sqrt(700) * 2^-24 each = 1.6e-6 of the norm (the plane kernels' truncated sums: 5e-6)."""
+    import fluxb200 as F
+    from fluxb200 import lib
+    g = torch.Generator(device="cuda")
+    g.manual_seed(lq)
+    heads, d, batch = 4, 64, 2
+    mk = lambda n: torch.randn(batch * n * heads * d + 4, device="cuda", generator=g)[1:1 + batch * n * heads * d].view(batch, n, heads * d)
+    q, k, v, do, o, dq, dk, dv = (mk(n) for n in (lq, lk, lk, lq, lq, lq, lk, lk))
+    lse = torch.empty(batch * heads * lq, device="cuda")
+    ctx = F.context()
+    dims = (heads * d, heads * d, lq, lk, batch, heads, causal)
+    p = [t.data_ptr() for t in (q, k, v)]
+    lib.call("fb_attn_fwd", ctx.handle, ctx.stream, *p, None, o.data_ptr(), lse.data_ptr(), *dims)
+    lib.call("fb_attn_bwd", ctx.handle, ctx.stream, *p, None, o.data_ptr(), lse.data_ptr(), do.data_ptr(), dq.data_ptr(), dk.data_ptr(),
+             dv.data_ptr(), *dims)
+    for name, got, ref in zip(("dq", "dk", "dv"), (dq, dk, dv), _reference(q, k, v, do, d, d, heads, causal)[1:]):
+        assert _err(got, ref) < 1.6e-6, (name, _err(got, ref))
+
+
+@pytest.mark.parametrize("d,lq,lk,causal", [(32, 300, 300, 1), (8, 70, 131, 0), (56, 65, 200, 0)])
+def test_bf16_backward_of_small_heads_is_the_float32_one(d, lq, lk, causal):
+    """Head sizes below 64: the gradients are those of the Float32 kernels on the widened operands, rounded once."""
+    import fluxb200 as F
+    from fluxb200 import lib
+    g = torch.Generator(device="cuda")
+    g.manual_seed(d)
+    heads, batch = 2, 2
+    E = heads * d
+    low = tuple(F.B200Array(torch.randn(batch * n * E, device="cuda", generator=g).bfloat16(), (E, n, batch)) for n in (lq, lk, lk))
+    mask = F.make_causal_mask() if causal else None
+    ctx = F.context()
+    dims = (E, E, lq, lk, batch, heads, causal)
+    (_, y), (grads,) = F.withgradient(lambda a: (lambda y: (F.sum_abs2(y), y))(F.dot_product_attention(*a, nheads=heads, mask=mask)[0]), low)
+    q, k, v = (t.t.float() for t in low)
+    o32, o16 = torch.empty(batch * lq * E, device="cuda"), torch.empty(batch * lq * E, device="cuda", dtype=torch.bfloat16)
+    lse = torch.empty(batch * heads * lq, device="cuda")
+    lib.call("fb_attn_fwd_bf16", ctx.handle, ctx.stream, *[t.ptr for t in low], o32.data_ptr(), o16.data_ptr(), lse.data_ptr(), *dims)
+    assert torch.equal(o16, y.t)
+    do = (2 * y.t.float()).bfloat16().float()
+    out = [torch.empty_like(t) for t in (q, k, v)]
+    lib.call("fb_attn_bwd", ctx.handle, ctx.stream, *[t.data_ptr() for t in (q, k, v)], None, o32.data_ptr(), lse.data_ptr(), do.data_ptr(),
+             *[t.data_ptr() for t in out], *dims)
+    for got, ref in zip(grads, out):
+        assert torch.equal(got.t, ref.bfloat16())
+
+
 def test_attention_two_streams():
     """Calls of one thread on two streams share the context's operand arena: neither may read the other's copies."""
     import fluxb200 as F
