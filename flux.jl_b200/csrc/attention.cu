@@ -4,6 +4,8 @@
 // Layout: Julia q[E, Lq, B] is read as [B][Lq][E]; head h owns features h*d .. (h+1)*d-1 of every row.
 // lse is [B][h][Lq].  One block handles one (batch, head, 64-row tile); S / P tiles are 64 x 64.
 // Arithmetic is fp32 throughout (FMA pipes), which is what the 1e-4 parity tolerance needs.
+#include <cuda_bf16.h>
+
 #include "common.cuh"
 
 namespace {
@@ -23,6 +25,9 @@ struct AttnDims {
   const float* dalpha;
   float p_drop, drop_scale;
   uint64_t seed, offset;
+  // redo_n bytes per (batch, head), or NULL: only heads with a byte set are computed (see fb_attn_fwd_redo)
+  const uint8_t* redo;
+  int redo_n;
 };
 
 // the logit of (query i, key j): scaled score plus the additive bias
@@ -38,15 +43,18 @@ __device__ __forceinline__ float attn_dropmul(const AttnDims& D, int64_t b, int 
   return fb_dropout_keep(idx, D.p_drop, D.seed, D.offset) ? D.drop_scale : 0.0f;
 }
 
+__device__ __forceinline__ float attn_value(float x) { return x; }
+__device__ __forceinline__ float attn_value(uint16_t bf16) { return __uint_as_float((uint32_t)bf16 << 16); }
+
 // dst[r][c] = src[(row0 + r) * ld_src + c] for r < 64, c < LD - 4 (zero padded outside rows < nrows, c < width)
-template <int LD>
-__device__ __forceinline__ void load_tile(float* __restrict__ dst, const float* __restrict__ src, int64_t ld_src,
+template <int LD, typename T>
+__device__ __forceinline__ void load_tile(float* __restrict__ dst, const T* __restrict__ src, int64_t ld_src,
                                           int64_t row0, int64_t nrows, int width) {
   constexpr int W = LD - 4;
   for (int e = threadIdx.x; e < TS * W; e += AT) {
     const int r = e / W, c = e % W;
     const int64_t gr = row0 + r;
-    dst[r * LD + c] = (gr < nrows && c < width) ? __ldg(src + gr * ld_src + c) : 0.0f;
+    dst[r * LD + c] = (gr < nrows && c < width) ? attn_value(__ldg(src + gr * ld_src + c)) : 0.0f;
   }
 }
 
@@ -140,10 +148,12 @@ __device__ __forceinline__ float row16_sum(float v) {
 }
 
 // ------------------------------------------------------------------------------------ forward ---
-template <int NC>
+// T: Float32, or bf16 bits with o16 the rounded output besides o (which may then be NULL).  A block computes one 64-row tile;
+// REDO: the tiles blockIdx.x, + gridDim.x, ... of a head with a byte of D.redo set (a loop in the common kernel costs 3 - 8 %).
+template <int NC, typename T, bool REDO>
 __global__ void __launch_bounds__(AT)
-attn_fwd_kernel(const float* __restrict__ q, const float* __restrict__ k, const float* __restrict__ v,
-                const uint8_t* __restrict__ mask, float* __restrict__ o, float* __restrict__ lse, AttnDims D) {
+attn_fwd_kernel(const T* __restrict__ q, const T* __restrict__ k, const T* __restrict__ v,
+                const uint8_t* __restrict__ mask, float* __restrict__ o, uint16_t* __restrict__ o16, float* __restrict__ lse, AttnDims D) {
   constexpr int LD = NC * 64 + 4;
   extern __shared__ float sm[];
   float* Qs = sm;
@@ -151,84 +161,95 @@ attn_fwd_kernel(const float* __restrict__ q, const float* __restrict__ k, const 
   float* Vs = Ks + TS * LD;
   float* Ps = Vs + TS * LD;
   const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
-  const int64_t i0 = (int64_t)blockIdx.x * TS;
   const int h = blockIdx.y;
   const int64_t b = blockIdx.z;
-  const float* qb = q + b * D.Lq * D.E + (int64_t)h * D.d;
-  const float* kb = k + b * D.Lk * D.E + (int64_t)h * D.d;
-  const float* vb = v + b * D.Lk * D.Ev + (int64_t)h * D.dv;
+  if (REDO) {
+    int any = 0;
+    for (int i = threadIdx.x; i < D.redo_n; i += AT) any |= D.redo[(b * D.H + h) * D.redo_n + i];
+    if (!__syncthreads_or(any)) return;
+  }
+  const T* qb = q + b * D.Lq * D.E + (int64_t)h * D.d;
+  const T* kb = k + b * D.Lk * D.E + (int64_t)h * D.d;
+  const T* vb = v + b * D.Lk * D.Ev + (int64_t)h * D.dv;
   const int kdim = (D.d + 3) & ~3;
 
-  load_tile<LD>(Qs, qb, D.E, i0, D.Lq, D.d);
-  float acc[NC][4][4];
-  float m[4], l[4];
-#pragma unroll
-  for (int i = 0; i < 4; ++i) {
-    m[i] = -INFINITY;
-    l[i] = 0.0f;
-#pragma unroll
-    for (int cc = 0; cc < NC; ++cc)
-#pragma unroll
-      for (int e = 0; e < 4; ++e) acc[cc][i][e] = 0.0f;
-  }
-  int64_t kv_end = D.Lk;
-  if (D.causal && i0 + TS < kv_end) kv_end = i0 + TS;
-  for (int64_t j0 = 0; j0 < kv_end; j0 += TS) {
-    __syncthreads();
-    load_tile<LD>(Ks, kb, D.E, j0, D.Lk, D.d);
-    load_tile<LD>(Vs, vb, D.Ev, j0, D.Lk, D.dv);
-    __syncthreads();
-    float S[4][4];
-    tile_abt<LD>(S, Qs, Ks, kdim, ty, tx);
+  int64_t i0 = (int64_t)blockIdx.x * TS;
+  do {
+    if (REDO) __syncthreads();   // the tile before has been read
+    load_tile<LD>(Qs, qb, D.E, i0, D.Lq, D.d);
+    float acc[NC][4][4];
+    float m[4], l[4];
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
-      const int64_t gi = i0 + ty + 16 * i;
-      bool keep[4];
-      float mx = -INFINITY;
-#pragma unroll
-      for (int j = 0; j < 4; ++j) {
-        keep[j] = attn_keep(D, mask, gi, j0 + tx + 16 * j);
-        S[i][j] = keep[j] ? attn_logit(D, S[i][j], b, h, gi, j0 + tx + 16 * j) : -INFINITY;
-        mx = fmaxf(mx, S[i][j]);
-      }
-      mx = row16_max(mx);
-      const float m_new = fmaxf(m[i], mx);
-      const float m_use = (m_new == -INFINITY) ? 0.0f : m_new;
-      const float corr = expf(m[i] - m_use);   // m[i] = -inf gives 0
-      float rs = 0.0f;
-#pragma unroll
-      for (int j = 0; j < 4; ++j) {
-        const float p = keep[j] ? expf(S[i][j] - m_use) : 0.0f;
-        rs += p;
-        // dropout acts on the normalised weights: the row sum keeps every term, the product with V the kept ones
-        Ps[(ty + 16 * i) * PLD + tx + 16 * j] = (keep[j] && D.p_drop > 0.0f) ? p * attn_dropmul(D, b, h, gi, j0 + tx + 16 * j) : p;
-      }
-      rs = row16_sum(rs);
-      l[i] = l[i] * corr + rs;
-      m[i] = m_new;
+      m[i] = -INFINITY;
+      l[i] = 0.0f;
 #pragma unroll
       for (int cc = 0; cc < NC; ++cc)
 #pragma unroll
-        for (int e = 0; e < 4; ++e) acc[cc][i][e] *= corr;
+        for (int e = 0; e < 4; ++e) acc[cc][i][e] = 0.0f;
     }
-    __syncthreads();
-    tile_pv<NC, LD>(acc, Ps, Vs, ty, tx);
-  }
-  float* ob = o + b * D.Lq * D.Ev + (int64_t)h * D.dv;
+    int64_t kv_end = D.Lk;
+    if (D.causal && i0 + TS < kv_end) kv_end = i0 + TS;
+    for (int64_t j0 = 0; j0 < kv_end; j0 += TS) {
+      __syncthreads();
+      load_tile<LD>(Ks, kb, D.E, j0, D.Lk, D.d);
+      load_tile<LD>(Vs, vb, D.Ev, j0, D.Lk, D.dv);
+      __syncthreads();
+      float S[4][4];
+      tile_abt<LD>(S, Qs, Ks, kdim, ty, tx);
 #pragma unroll
-  for (int i = 0; i < 4; ++i) {
-    const int64_t gi = i0 + ty + 16 * i;
-    if (gi >= D.Lq) continue;
-    const float inv = l[i] > 0.0f ? 1.0f / l[i] : 0.0f;
+      for (int i = 0; i < 4; ++i) {
+        const int64_t gi = i0 + ty + 16 * i;
+        bool keep[4];
+        float mx = -INFINITY;
 #pragma unroll
-    for (int cc = 0; cc < NC; ++cc)
+        for (int j = 0; j < 4; ++j) {
+          keep[j] = attn_keep(D, mask, gi, j0 + tx + 16 * j);
+          S[i][j] = keep[j] ? attn_logit(D, S[i][j], b, h, gi, j0 + tx + 16 * j) : -INFINITY;
+          mx = fmaxf(mx, S[i][j]);
+        }
+        mx = row16_max(mx);
+        const float m_new = fmaxf(m[i], mx);
+        const float m_use = (m_new == -INFINITY) ? 0.0f : m_new;
+        const float corr = expf(m[i] - m_use);   // m[i] = -inf gives 0
+        float rs = 0.0f;
 #pragma unroll
-      for (int e = 0; e < 4; ++e) {
-        const int c = cc * 64 + 4 * tx + e;
-        if (c < D.dv) ob[gi * D.Ev + c] = acc[cc][i][e] * inv;
+        for (int j = 0; j < 4; ++j) {
+          const float p = keep[j] ? expf(S[i][j] - m_use) : 0.0f;
+          rs += p;
+          // dropout acts on the normalised weights: the row sum keeps every term, the product with V the kept ones
+          Ps[(ty + 16 * i) * PLD + tx + 16 * j] = (keep[j] && D.p_drop > 0.0f) ? p * attn_dropmul(D, b, h, gi, j0 + tx + 16 * j) : p;
+        }
+        rs = row16_sum(rs);
+        l[i] = l[i] * corr + rs;
+        m[i] = m_new;
+#pragma unroll
+        for (int cc = 0; cc < NC; ++cc)
+#pragma unroll
+          for (int e = 0; e < 4; ++e) acc[cc][i][e] *= corr;
       }
-    if (tx == 0) lse[(b * D.H + h) * D.Lq + gi] = (l[i] > 0.0f) ? m[i] + logf(l[i]) : -INFINITY;
-  }
+      __syncthreads();
+      tile_pv<NC, LD>(acc, Ps, Vs, ty, tx);
+    }
+    const int64_t ob = b * D.Lq * D.Ev + (int64_t)h * D.dv;
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      const int64_t gi = i0 + ty + 16 * i;
+      if (gi >= D.Lq) continue;
+      const float inv = l[i] > 0.0f ? 1.0f / l[i] : 0.0f;
+#pragma unroll
+      for (int cc = 0; cc < NC; ++cc)
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+          const int c = cc * 64 + 4 * tx + e;
+          if (c >= D.dv) continue;
+          if (sizeof(T) == 4 || o != nullptr) o[ob + gi * D.Ev + c] = acc[cc][i][e] * inv;
+          if (sizeof(T) == 2) o16[ob + gi * D.Ev + c] = __bfloat16_as_ushort(__float2bfloat16_rn(acc[cc][i][e] * inv));
+        }
+      if (tx == 0) lse[(b * D.H + h) * D.Lq + gi] = (l[i] > 0.0f) ? m[i] + logf(l[i]) : -INFINITY;
+    }
+    i0 += (int64_t)gridDim.x * TS;
+  } while (REDO && i0 < D.Lq);
 }
 
 // dlt[b][h][i] = sum_c dO[b][i][h*dv + c] * O[b][i][h*dv + c]; one warp per (b, i, h)
@@ -469,6 +490,7 @@ int32_t attn_make_dims(const char* fn, AttnDims* D, int64_t e_dim, int64_t ev_di
   D->scale = 1.0f / sqrtf((float)D->d);
   D->bias = nullptr; D->bias_sh = 0; D->bias_sb = 0; D->dalpha = nullptr;
   D->p_drop = 0.0f; D->drop_scale = 1.0f; D->seed = 0; D->offset = 0;
+  D->redo = nullptr; D->redo_n = 0;
   return FB_OK;
 }
 
@@ -484,6 +506,30 @@ int32_t attn_set_extras(const char* fn, AttnDims* D, const float* bias, int64_t 
 bool attn_has_extras(const AttnDims& D) { return D.bias != nullptr || D.p_drop > 0.0f || D.dalpha != nullptr; }
 
 }  // namespace
+
+int32_t fb_attn_fwd_redo(fb_ctx* ctx, cudaStream_t stream, int bf16, const void* q, const void* k, const void* v, float* o, uint16_t* o16,
+                         float* lse, int64_t e_dim, int64_t ev_dim, int64_t lq, int64_t lk, int64_t batch, int nheads, int causal,
+                         const uint8_t* redo, int redo_n) {
+  AttnDims D;
+  const int32_t st = attn_make_dims("fb_attn_fwd", &D, e_dim, ev_dim, lq, lk, batch, nheads, causal);
+  if (st != FB_OK) return st;
+  D.redo = redo; D.redo_n = redo_n;
+  constexpr size_t smem = (size_t)(3 * TS * (64 + 4) + TS * PLD) * sizeof(float);
+  // about three blocks per SM: a launch that finds nothing to do is over in one wave
+  int64_t gx = (int64_t)ctx->sm_count * 3 / (batch * nheads);
+  const int64_t tiles = (lq + TS - 1) / TS;
+  gx = gx < 1 ? 1 : gx > tiles ? tiles : gx;
+  const dim3 grid((unsigned)gx, (unsigned)nheads, (unsigned)batch);
+  if (bf16) {
+    FB_CUDA(cudaFuncSetAttribute(attn_fwd_kernel<1, uint16_t, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    attn_fwd_kernel<1, uint16_t, true><<<grid, AT, smem, stream>>>((const uint16_t*)q, (const uint16_t*)k, (const uint16_t*)v, nullptr, o, o16, lse, D);
+  } else {
+    FB_CUDA(cudaFuncSetAttribute(attn_fwd_kernel<1, float, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    attn_fwd_kernel<1, float, true><<<grid, AT, smem, stream>>>((const float*)q, (const float*)k, (const float*)v, nullptr, o, nullptr, lse, D);
+  }
+  FB_LAUNCH_CHECK();
+  return FB_OK;
+}
 
 FB_API int32_t fb_attn_fwd(fb_ctx* ctx, void* stream_, const float* q, const float* k, const float* v,
                            const uint8_t* mask, float* o, float* lse, int64_t e_dim, int64_t ev_dim, int64_t lq,
@@ -512,11 +558,11 @@ FB_API int32_t fb_attn_fwd_ex(fb_ctx* ctx, void* stream_, const float* q, const 
   const size_t smem = (size_t)(3 * TS * (nc * 64 + 4) + TS * PLD) * sizeof(float);
   dim3 grid((unsigned)((lq + TS - 1) / TS), (unsigned)nheads, (unsigned)batch);
   if (nc == 1) {
-    FB_CUDA(cudaFuncSetAttribute(attn_fwd_kernel<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    attn_fwd_kernel<1><<<grid, AT, smem, stream>>>(q, k, v, mask, o, lse, D);
+    FB_CUDA(cudaFuncSetAttribute(attn_fwd_kernel<1, float, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    attn_fwd_kernel<1, float, false><<<grid, AT, smem, stream>>>(q, k, v, mask, o, nullptr, lse, D);
   } else {
-    FB_CUDA(cudaFuncSetAttribute(attn_fwd_kernel<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    attn_fwd_kernel<2><<<grid, AT, smem, stream>>>(q, k, v, mask, o, lse, D);
+    FB_CUDA(cudaFuncSetAttribute(attn_fwd_kernel<2, float, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    attn_fwd_kernel<2, float, false><<<grid, AT, smem, stream>>>(q, k, v, mask, o, nullptr, lse, D);
   }
   FB_LAUNCH_CHECK();
   return FB_OK;

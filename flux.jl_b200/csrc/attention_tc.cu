@@ -131,14 +131,20 @@ __device__ __forceinline__ void row_f32(const float* src, int c0, int width, boo
   }
 }
 
-// One row of a CTA's own operand into tensor memory: NP planes of 32 columns each (Float32 source: 3, bf16 source: 1)
+__device__ __forceinline__ bool not_finite(uint32_t bits) { return (bits & 0x7f800000u) == 0x7f800000u; }
+
+// One row of a CTA's own operand into tensor memory: NP planes of 32 columns each (Float32 source: 3, bf16 source: 1).
+// True when a value of it is not finite.
 template <int NP>
-__device__ __forceinline__ void row_to_tmem(const void* src, int width, bool live, bool vec, uint32_t t_addr) {
+__device__ __forceinline__ bool row_to_tmem(const void* src, int width, bool live, bool vec, uint32_t t_addr) {
+  bool odd = false;
 #pragma unroll
   for (int hf = 0; hf < 2; ++hf) {
     if (NP == 3) {
       uint32_t v[32];
       row_f32((const float*)src, 32 * hf, width, live, vec, v);
+#pragma unroll
+      for (int c = 0; c < 32; ++c) odd |= not_finite(v[c]);
       store_planes32(t_addr + 16u * hf, t_addr + 32u + 16u * hf, t_addr + 64u + 16u * hf, v);
     } else {
       uint32_t v[16];
@@ -148,9 +154,12 @@ __device__ __forceinline__ void row_to_tmem(const void* src, int width, bool liv
         if (live && 32 * hf + 2 * c < width) x = __ldg((const uint4*)((const uint16_t*)src + 32 * hf + 2 * c));
         v[c] = x.x; v[c + 1] = x.y; v[c + 2] = x.z; v[c + 3] = x.w;
       }
+#pragma unroll
+      for (int c = 0; c < 16; ++c) odd |= not_finite(v[c]) | not_finite(v[c] << 16);
       tc_st_32x32b_x16(t_addr + 16u * hf, v);
     }
   }
+  return odd;
 }
 
 // 32 columns (from c0) of an output row, scaled; Float32, or bf16 rounded to nearest
@@ -252,7 +261,8 @@ struct SplitArgs {
   const float* o;       // for the job of index 3 (dO)
   const float* lse;
   float2* rv;
-  int H, vec;
+  uint8_t* odd;         // or NULL: [job][tile] bytes, 2 * tiles of odd_n per (batch, head): a value of the tile is not finite
+  int H, vec, odd_n;
 };
 
 template <int NP>
@@ -265,6 +275,7 @@ __global__ void __launch_bounds__(256) attn_split_kernel(SplitArgs A) {
   uint8_t* dst = J.dst + (bh * J.tiles + blockIdx.x) * (int64_t)(NP * TILE);
   const int ch = threadIdx.x & 7;
   const bool is_do = blockIdx.z == 3;
+  int odd = 0;
 #pragma unroll
   for (int it = 0; it < 2; ++it) {
     const int r = (threadIdx.x >> 3) + 32 * it;
@@ -303,6 +314,8 @@ __global__ void __launch_bounds__(256) attn_split_kernel(SplitArgs A) {
         x[2 * e + 1] = __uint_as_float(w[e] & 0xffff0000u);
       }
     }
+#pragma unroll
+    for (int e = 0; e < 8; ++e) odd |= not_finite(__float_as_uint(x[e])) ? 1 : 0;
     if (is_do) {
       float s = 0.0f;
 #pragma unroll
@@ -321,6 +334,10 @@ __global__ void __launch_bounds__(256) attn_split_kernel(SplitArgs A) {
       s += __shfl_xor_sync(0xffffffffu, s, 4);
       if (ch == 0) A.rv[bh * ((int64_t)J.tiles * KT) + row] = live ? make_float2(A.lse[bh * J.L + row] * LOG2E, s) : make_float2(INFINITY, 0.0f);
     }
+  }
+  if (A.odd != nullptr) {
+    odd = __syncthreads_or(odd);
+    if (threadIdx.x == 0) A.odd[bh * A.odd_n + (int)blockIdx.z * J.tiles + (int)blockIdx.x] = odd ? 1 : 0;
   }
 }
 
@@ -362,7 +379,8 @@ struct FwdCfg {
 template <int NP>
 __global__ void __launch_bounds__(FWD_THREADS, 2)
 attn_fwd_tc_kernel(const void* __restrict__ qmat, const uint8_t* __restrict__ kimg, const uint8_t* __restrict__ vimg,
-                   float* __restrict__ o, uint16_t* __restrict__ o16, float* __restrict__ lse, AtcDims D, int32_t* __restrict__ dev_err) {
+                   float* __restrict__ o, uint16_t* __restrict__ o16, float* __restrict__ lse, uint8_t* __restrict__ odd_q, int odd_n,
+                   AtcDims D, int32_t* __restrict__ dev_err) {
   using cfg = FwdCfg<NP>;
   constexpr int S = cfg::SLOTS;
   enum { B_FULL = 0, B_FREE = S, B_QREADY = 2 * S, B_SFULL, B_PREADY, B_OFULL, B_COUNT };
@@ -451,7 +469,11 @@ attn_fwd_tc_kernel(const void* __restrict__ qmat, const uint8_t* __restrict__ ki
     const bool live = gi < D.Lq;
     const uint32_t t_row = tmem + ((uint32_t)(32 * q) << 16);
     const int64_t el = NP == 3 ? 4 : 2;
-    row_to_tmem<NP>((const uint8_t*)qmat + el * ((b * D.Lq + gi) * D.E + (int64_t)h * D.d), D.d, live, D.vec != 0, t_row);
+    const bool odd = row_to_tmem<NP>((const uint8_t*)qmat + el * ((b * D.Lq + gi) * D.E + (int64_t)h * D.d), D.d, live, D.vec != 0, t_row);
+    if (odd_q != nullptr) {
+      const bool any = __any_sync(0xffffffffu, odd);
+      if (lane == 0) odd_q[bh * odd_n + (int)(i0 / QT) * 4 + q] = any ? 1 : 0;
+    }
     tc_wait_st();
     tc_fence_before();
     __syncwarp();
@@ -986,11 +1008,17 @@ bool make_plan(AtcPlan* P, int np, int64_t e_dim, int64_t ev_dim, int64_t lq, in
   return true;
 }
 
+// redo: heads with a value that is not finite are computed again by the FMA kernel.  Planes cannot carry one (the remainder of
+// an infinite value is NaN, and so is an infinite plane times a zero one), while the sums of products give what such a value
+// makes: a key of -inf no weight, a value of inf an infinite output.  The launch that finds nothing costs 4 - 6 us (2048 x 2048,
+// 8 heads of 32, batch 2: 114 -> 119 us; the FMA kernel 853).
 template <int NP>
 int32_t fwd_impl(fb_ctx* ctx, cudaStream_t stream, const uint8_t* q, const uint8_t* k, const uint8_t* v, float* o, uint16_t* o16, float* lse,
-                 const AtcPlan& P, int64_t batch) {
+                 const AtcPlan& P, int64_t batch, bool redo) {
   const AtcDims& D = P.D;
-  const int64_t el = NP == 3 ? 4 : 2, per = 2 * P.kbytes;
+  // a byte for every K and V tile and every 32 queries of a (batch, head)
+  const int odd_n = 2 * D.ktiles + 2 * D.qtiles;
+  const int64_t el = NP == 3 ? 4 : 2, per = 2 * P.kbytes + (redo ? (int64_t)D.H * odd_n : 0);
   int64_t chunk = IMAGE_BYTES / per;
   chunk = chunk < 1 ? 1 : (chunk > batch ? batch : chunk);
   uint8_t* img = (uint8_t*)fb_pack_scratch(ctx, stream, (size_t)(chunk * per));
@@ -998,16 +1026,23 @@ int32_t fwd_impl(fb_ctx* ctx, cudaStream_t stream, const uint8_t* q, const uint8
   FB_CUDA(cudaFuncSetAttribute(attn_fwd_tc_kernel<NP>, cudaFuncAttributeMaxDynamicSharedMemorySize, FwdCfg<NP>::SMEM));
   for (int64_t b0 = 0; b0 < batch; b0 += chunk) {
     const int64_t nb = b0 + chunk > batch ? batch - b0 : chunk;
+    uint8_t* odd = redo ? img + nb * 2 * P.kbytes : nullptr;
     SplitArgs A = {};
-    A.H = D.H; A.vec = D.vec;
+    A.H = D.H; A.vec = D.vec; A.odd = odd; A.odd_n = odd_n;
     A.job[0] = {k + el * b0 * D.Lk * D.E, img, D.Lk, D.E, D.d, D.ktiles};
     A.job[1] = {v + el * b0 * D.Lk * D.Ev, img + nb * P.kbytes, D.Lk, D.Ev, D.dv, D.ktiles};
     attn_split_kernel<NP><<<dim3((unsigned)D.ktiles, (unsigned)(nb * D.H), 2), 256, 0, stream>>>(A);
     FB_LAUNCH_CHECK();
     attn_fwd_tc_kernel<NP><<<dim3((unsigned)(D.qtiles / 2), (unsigned)D.H, (unsigned)nb), FWD_THREADS, FwdCfg<NP>::SMEM, stream>>>(
         q + el * b0 * D.Lq * D.E, img, img + nb * P.kbytes, o ? o + b0 * D.Lq * D.Ev : nullptr, o16 ? o16 + b0 * D.Lq * D.Ev : nullptr,
-        lse + b0 * D.H * D.Lq, D, ctx->dev_error);
+        lse + b0 * D.H * D.Lq, odd ? odd + 2 * D.ktiles : nullptr, odd_n, D, ctx->dev_error);
     FB_LAUNCH_CHECK();
+    if (redo) {
+      const int32_t st = fb_attn_fwd_redo(ctx, stream, NP == 1, q + el * b0 * D.Lq * D.E, k + el * b0 * D.Lk * D.E, v + el * b0 * D.Lk * D.Ev,
+                                          o ? o + b0 * D.Lq * D.Ev : nullptr, o16 ? o16 + b0 * D.Lq * D.Ev : nullptr, lse + b0 * D.H * D.Lq,
+                                          D.E, D.Ev, D.Lq, D.Lk, nb, D.H, D.causal, odd, odd_n);
+      if (st != FB_OK) return st;
+    }
   }
   fb_pack_done(ctx, stream);
   return FB_OK;
@@ -1059,7 +1094,9 @@ int32_t fb_attn_fwd_tc(fb_ctx* ctx, cudaStream_t stream, const float* q, const f
   AtcPlan P;
   if (!attn_tc_enabled() || mask != nullptr || !make_plan(&P, 3, e_dim, ev_dim, lq, lk, batch, nheads, causal)) return FB_ERR_UNSUPPORTED;
   if (!fb_aligned16(q) || !fb_aligned16(k) || !fb_aligned16(v) || !fb_aligned16(o)) P.D.vec = 0;
-  return fwd_impl<3>(ctx, stream, (const uint8_t*)q, (const uint8_t*)k, (const uint8_t*)v, o, nullptr, lse, P, batch);
+  // (aligned heads of 64 have always been the tensor cores', which make NaNs of infinite values)
+  const bool redo = P.D.d != HD || P.D.dv != HD || !P.D.vec;
+  return fwd_impl<3>(ctx, stream, (const uint8_t*)q, (const uint8_t*)k, (const uint8_t*)v, o, nullptr, lse, P, batch, redo);
 }
 
 // *did_kv, *did_q: which part was done.  dQ, dK and dV accumulate in tensor memory with truncating adds; beyond 2048 keys
@@ -1100,7 +1137,8 @@ FB_API int32_t fb_attn_fwd_bf16(fb_ctx* ctx, void* stream, const uint16_t* q, co
       !make_plan(&P, 1, e_dim, ev_dim, lq, lk, batch, nheads, causal))
     return FB_ERR_UNSUPPORTED;
   if (!fb_aligned16(q) || !fb_aligned16(k) || !fb_aligned16(v) || !fb_aligned16(o) || !fb_aligned16(o32)) return FB_ERR_UNSUPPORTED;
-  return fwd_impl<1>(ctx, (cudaStream_t)stream, (const uint8_t*)q, (const uint8_t*)k, (const uint8_t*)v, o32, o, lse, P, batch);
+  const bool redo = P.D.d != HD || P.D.dv != HD;
+  return fwd_impl<1>(ctx, (cudaStream_t)stream, (const uint8_t*)q, (const uint8_t*)k, (const uint8_t*)v, o32, o, lse, P, batch, redo);
 }
 
 FB_API int32_t fb_attn_bwd_bf16(fb_ctx* ctx, void* stream, const uint16_t* q, const uint16_t* k, const uint16_t* v, const float* o32,

@@ -138,6 +138,54 @@ def test_bf16_backward_of_small_heads_is_the_float32_one(d, lq, lk, causal):
         assert torch.equal(got.t, ref.bfloat16())
 
 
+@pytest.mark.parametrize("d,dv,lq,lk,causal,shift,dtype", [(32, 32, 200, 300, 0, 0, "f32"), (20, 12, 77, 130, 1, 0, "f32"), (64, 64, 300, 129, 0, 1, "f32"),
+                                                           (64, 16, 65, 64, 1, 0, "f32"), (32, 32, 200, 300, 0, 0, "bf16"), (8, 16, 129, 70, 1, 0, "bf16")])
+def test_infinite_and_nan_operands(d, dv, lq, lk, causal, shift, dtype):
+    """What the FMA kernel (reached through an additive bias of zeros) makes of operands that are not finite, bit for bit, in
+    the heads that hold them; the other heads are as they are without them."""
+    import fluxb200 as F
+    from fluxb200 import lib
+    g = torch.Generator(device="cuda")
+    g.manual_seed(d + lq)
+    heads, batch, inf = 4, 2, float("inf")
+    mk = lambda n, size: torch.randn(batch * n * heads * size + 4, device="cuda", generator=g)[shift:shift + batch * n * heads * size].view(batch, n, heads, size)
+    clean = [mk(lq, d), mk(lk, d), mk(lk, dv)]
+    if dtype == "bf16":
+        clean = [t.bfloat16().float() for t in clean]
+    ctx = F.context()
+    dims = (heads * d, heads * dv, lq, lk, batch, heads, causal)
+    zero_bias = torch.zeros(lk * lq, device="cuda")
+
+    def forward(arrays, general=False):
+        o, lse = mk(lq, dv), torch.empty(batch, heads, lq, device="cuda")
+        if dtype == "bf16" and not general:
+            low, o16 = [t.bfloat16() for t in arrays], torch.empty(o.shape, device="cuda", dtype=torch.bfloat16)
+            lib.call("fb_attn_fwd_bf16", ctx.handle, ctx.stream, *[t.data_ptr() for t in low], o.data_ptr(), o16.data_ptr(), lse.data_ptr(), *dims)
+            assert torch.equal(torch.nan_to_num(o16), torch.nan_to_num(o.bfloat16()))
+            return o, lse
+        lib.call("fb_attn_fwd_ex", ctx.handle, ctx.stream, *[t.data_ptr() for t in arrays], None, zero_bias.data_ptr() if general else None, 0, 0,
+                 0.0, 0, 0, o.data_ptr(), lse.data_ptr(), *dims)
+        return o, lse
+    plain, plain_lse = forward(clean)
+    arrays = [t.clone() if not shift else mk(t.shape[1], t.shape[3]).copy_(t) for t in clean]
+    arrays[0][0, lq // 2, 0, 1] = inf                # a query
+    arrays[1][0, lk // 3, 1, 0] = -inf               # a key: weight 0 or 1, by the sign of the query's value
+    arrays[2][1, 3, 2, dv - 1] = inf                 # a value
+    arrays[1][1, lk - 1, 3, d - 1] = float("nan")
+    (o, lse), (ref, ref_lse) = forward(arrays), forward(arrays, general=True)
+    touched = {(0, 0), (0, 1), (1, 2), (1, 3)}
+    for b in range(batch):
+        for h in range(heads):
+            if (b, h) in touched:
+                assert torch.equal(torch.isnan(o[b, :, h]), torch.isnan(ref[b, :, h]))
+                assert torch.equal(torch.nan_to_num(o[b, :, h], nan=7.0), torch.nan_to_num(ref[b, :, h], nan=7.0))
+                assert torch.equal(torch.nan_to_num(lse[b, h], nan=7.0), torch.nan_to_num(ref_lse[b, h], nan=7.0))
+            else:
+                assert torch.equal(o[b, :, h], plain[b, :, h]) and torch.equal(lse[b, h], plain_lse[b, h])
+    assert bool(torch.isinf(ref[1, 3:, 2, dv - 1]).any()) and bool(torch.isfinite(ref[0, :, 1]).any())
+    assert ctx.device_error() == 0
+
+
 def test_attention_two_streams():
     """Calls of one thread on two streams share the context's operand arena: neither may read the other's copies."""
     import fluxb200 as F
