@@ -51,10 +51,6 @@ FB_API int32_t fb_ctx_create(int32_t device, fb_ctx** out) {
   c->smem_optin = prop.sharedMemPerBlockOptin;
   c->scratch = nullptr;
   c->scratch_bytes = 0;
-  c->pack = nullptr;
-  c->pack_bytes = 0;
-  c->pack_stream = nullptr;
-  c->pack_used = false;
   c->retired_count = 0;
   c->dev_error = nullptr;
   c->gemm_ws = nullptr;
@@ -72,18 +68,26 @@ FB_API int32_t fb_ctx_create(int32_t device, fb_ctx** out) {
     return fb_fail(FB_ERR_ALLOC, "fb_ctx_create: cudaHostAlloc failed");
   }
   memset((void*)c->host_page, 0, 64);
-  if (cudaEventCreateWithFlags(&c->pack_event, cudaEventDisableTiming) != cudaSuccess) {
+  // What a call's own memory leaves behind is kept up to POOL_KEEP and goes back to the device beyond that.
+  constexpr uint64_t POOL_KEEP = uint64_t(1) << 30;
+  cudaMemPoolProps pool;
+  memset(&pool, 0, sizeof(pool));
+  pool.allocType = cudaMemAllocationTypePinned;
+  pool.location.type = cudaMemLocationTypeDevice;
+  pool.location.id = device;
+  uint64_t keep = POOL_KEEP;
+  if (cudaMemPoolCreate(&c->pool, &pool) != cudaSuccess || cudaMemPoolSetAttribute(c->pool, cudaMemPoolAttrReleaseThreshold, &keep) != cudaSuccess) {
     cudaGetLastError();
     cudaFree(c->dev_error);
     cudaFreeHost((void*)c->host_page);
     delete c;
-    return fb_fail(FB_ERR_CUDA, "fb_ctx_create: cudaEventCreate failed");
+    return fb_fail(FB_ERR_ALLOC, "fb_ctx_create: cudaMemPoolCreate failed");
   }
   int32_t ws_status = fb_side_kernels_prepare_elementwise();
   if (ws_status == FB_OK) ws_status = fb_side_kernels_prepare_peer();
   if (ws_status == FB_OK) ws_status = fb_gemm_workspace_create(c);
   if (ws_status != FB_OK) {
-    cudaEventDestroy(c->pack_event);
+    cudaMemPoolDestroy(c->pool);
     cudaFree(c->dev_error);
     cudaFreeHost((void*)c->host_page);
     delete c;
@@ -106,8 +110,7 @@ FB_API int32_t fb_ctx_destroy(fb_ctx* ctx) {
   cudaSetDevice(ctx->device);
   cudaDeviceSynchronize();
   if (ctx->scratch) cudaFree(ctx->scratch);
-  if (ctx->pack) cudaFree(ctx->pack);
-  cudaEventDestroy(ctx->pack_event);
+  cudaMemPoolDestroy(ctx->pool);
   for (int i = 0; i < ctx->retired_count; ++i) cudaFree(ctx->retired[i]);
   if (ctx->dev_error) cudaFree(ctx->dev_error);
   cudaFreeHost((void*)ctx->host_page);
@@ -116,12 +119,13 @@ FB_API int32_t fb_ctx_destroy(fb_ctx* ctx) {
   return FB_OK;
 }
 
-static void* arena_get(fb_ctx* ctx, void** block, size_t* have, size_t bytes) {
-  if (bytes <= *have && *block != nullptr) return *block;
+void* fb_scratch(fb_ctx* ctx, cudaStream_t stream, size_t bytes) {
+  (void)stream;
+  if (bytes <= ctx->scratch_bytes && ctx->scratch != nullptr) return ctx->scratch;
   // grow geometrically; the outgrown block stays allocated until the context is destroyed, because work already
   // enqueued - or captured in a CUDA graph - may still name it
   size_t want = bytes < (size_t(1) << 22) ? (size_t(1) << 22) : bytes;
-  if (want < 2 * *have) want = 2 * *have;
+  if (want < 2 * ctx->scratch_bytes) want = 2 * ctx->scratch_bytes;
   want = (want + 255) & ~size_t(255);
   void* p = nullptr;
   if (cudaMalloc(&p, want) != cudaSuccess) {
@@ -129,44 +133,10 @@ static void* arena_get(fb_ctx* ctx, void** block, size_t* have, size_t bytes) {
     fb_set_error("scratch arena: cudaMalloc of %zu bytes failed", want);
     return nullptr;
   }
-  if (*block != nullptr && ctx->retired_count < FB_MAX_RETIRED) ctx->retired[ctx->retired_count++] = *block;
-  *block = p;
-  *have = want;
+  if (ctx->scratch != nullptr && ctx->retired_count < FB_MAX_RETIRED) ctx->retired[ctx->retired_count++] = ctx->scratch;
+  ctx->scratch = p;
+  ctx->scratch_bytes = want;
   return p;
-}
-
-void* fb_scratch(fb_ctx* ctx, cudaStream_t stream, size_t bytes) {
-  (void)stream;
-  return arena_get(ctx, &ctx->scratch, &ctx->scratch_bytes, bytes);
-}
-
-static bool stream_capturing(cudaStream_t stream) {
-  cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
-  if (cudaStreamIsCapturing(stream, &cs) != cudaSuccess) {
-    cudaGetLastError();
-    return true;
-  }
-  return cs != cudaStreamCaptureStatusNone;
-}
-
-void* fb_pack_scratch(fb_ctx* ctx, cudaStream_t stream, size_t bytes) {
-  const bool capturing = stream_capturing(stream);
-  if (bytes > ctx->pack_bytes && capturing) return nullptr;
-  if (ctx->pack_used && ctx->pack_stream != stream && !capturing && cudaStreamWaitEvent(stream, ctx->pack_event, 0) != cudaSuccess) {
-    cudaGetLastError();
-    return nullptr;
-  }
-  return arena_get(ctx, &ctx->pack, &ctx->pack_bytes, bytes);
-}
-
-void fb_pack_done(fb_ctx* ctx, cudaStream_t stream) {
-  if (stream_capturing(stream)) return;
-  if (cudaEventRecord(ctx->pack_event, stream) != cudaSuccess) {
-    cudaGetLastError();
-    return;
-  }
-  ctx->pack_stream = stream;
-  ctx->pack_used = true;
 }
 
 FB_API int32_t fb_malloc(fb_ctx* ctx, int64_t bytes, void** out) {

@@ -978,8 +978,8 @@ bool attn_bwd_tc_enabled() {
   return on;
 }
 
-// plane images of one call take at most this much scratch memory unless one batch entry needs more: a call is cut along
-// the batch otherwise
+// the plane images of one call take at most this much memory unless one batch entry needs more: a call is cut along the batch
+// otherwise
 constexpr int64_t IMAGE_BYTES = (int64_t)512 << 20;
 
 struct AtcPlan {
@@ -1021,7 +1021,8 @@ int32_t fwd_impl(fb_ctx* ctx, cudaStream_t stream, const uint8_t* q, const uint8
   const int64_t el = NP == 3 ? 4 : 2, per = 2 * P.kbytes + (redo ? (int64_t)D.H * odd_n : 0);
   int64_t chunk = IMAGE_BYTES / per;
   chunk = chunk < 1 ? 1 : (chunk > batch ? batch : chunk);
-  uint8_t* img = (uint8_t*)fb_pack_scratch(ctx, stream, (size_t)(chunk * per));
+  const fb_temp images(ctx, stream, (size_t)(chunk * per));
+  uint8_t* img = (uint8_t*)images.p;
   if (!img) return FB_ERR_UNSUPPORTED;
   FB_CUDA(cudaFuncSetAttribute(attn_fwd_tc_kernel<NP>, cudaFuncAttributeMaxDynamicSharedMemorySize, FwdCfg<NP>::SMEM));
   for (int64_t b0 = 0; b0 < batch; b0 += chunk) {
@@ -1044,7 +1045,6 @@ int32_t fwd_impl(fb_ctx* ctx, cudaStream_t stream, const uint8_t* q, const uint8
       if (st != FB_OK) return st;
     }
   }
-  fb_pack_done(ctx, stream);
   return FB_OK;
 }
 
@@ -1055,7 +1055,8 @@ int32_t bwd_impl(fb_ctx* ctx, cudaStream_t stream, const uint8_t* q, const uint8
   const int64_t el = NP == 3 ? 4 : 2, per = 2 * P.kbytes + 2 * P.qbytes + P.rvbytes;
   int64_t chunk = IMAGE_BYTES / per;
   chunk = chunk < 1 ? 1 : (chunk > batch ? batch : chunk);
-  uint8_t* img = (uint8_t*)fb_pack_scratch(ctx, stream, (size_t)(chunk * per));
+  const fb_temp images(ctx, stream, (size_t)(chunk * per));
+  uint8_t* img = (uint8_t*)images.p;
   if (!img) return FB_ERR_UNSUPPORTED;
   FB_CUDA(cudaFuncSetAttribute(attn_bwd_dkdv_tc_kernel<NP>, cudaFuncAttributeMaxDynamicSharedMemorySize, KvCfg<NP>::SMEM));
   FB_CUDA(cudaFuncSetAttribute(attn_bwd_dq_tc_kernel<NP>, cudaFuncAttributeMaxDynamicSharedMemorySize, DqCfg<NP>::SMEM));
@@ -1081,7 +1082,6 @@ int32_t bwd_impl(fb_ctx* ctx, cudaStream_t stream, const uint8_t* q, const uint8
         q + el * qoff, dout + el * qvoff, ki, vi, rv, dq + el * qoff, D, ctx->dev_error);
     FB_LAUNCH_CHECK();
   }
-  fb_pack_done(ctx, stream);
   return FB_OK;
 }
 

@@ -20,11 +20,7 @@ struct fb_ctx {
   size_t smem_optin;
   void* scratch;         // device arena, grown on demand, reused by every call on this context
   size_t scratch_bytes;
-  void* pack;            // second arena: images of attention operands (a caller's scratch stays untouched)
-  size_t pack_bytes;
-  cudaEvent_t pack_event;     // behind the last work that reads the arena, enqueued on pack_stream
-  cudaStream_t pack_stream;
-  bool pack_used;
+  cudaMemPool_t pool;    // stream-ordered memory of single calls (fb_temp)
   void* retired[FB_MAX_RETIRED];   // outgrown arena blocks, released with the context
   int retired_count;
   int32_t* dev_error;    // device error word written by kernels whose bounded waits ran out
@@ -40,11 +36,24 @@ int32_t fb_fail(int32_t code, const char* fmt, ...);
 // Returns a pointer into the context arena of at least `bytes` (256-byte aligned); grows the arena when it is
 // too small (outgrown blocks are kept until fb_ctx_destroy).  NULL on allocation failure.
 void* fb_scratch(fb_ctx* ctx, cudaStream_t stream, size_t bytes);
-// The same from the operand-copy arena; NULL (without an error) also when it would have to grow inside a stream capture.
-// Work enqueued on another stream waits for the last use of the arena (not inside a capture, whose replays the caller
-// orders): call fb_pack_done behind the last kernel that reads the copies.
-void* fb_pack_scratch(fb_ctx* ctx, cudaStream_t stream, size_t bytes);
-void fb_pack_done(fb_ctx* ctx, cudaStream_t stream);
+// Device memory of one call, from its stream's order: work on another stream never gets it before this call's kernels are done,
+// and inside a capture it is the graph's own, whatever runs beside a replay.  p is NULL (without an error message) when there
+// is none.  Costs the host about 1 us eagerly; a captured graph holds its own addresses.
+struct fb_temp {
+  void* p;
+  cudaStream_t stream;
+  fb_temp(fb_ctx* ctx, cudaStream_t s, size_t bytes) : p(nullptr), stream(s) {
+    if (bytes != 0 && cudaMallocFromPoolAsync(&p, bytes, ctx->pool, s) != cudaSuccess) {
+      cudaGetLastError();
+      p = nullptr;
+    }
+  }
+  ~fb_temp() {
+    if (p != nullptr && cudaFreeAsync(p, stream) != cudaSuccess) cudaGetLastError();
+  }
+  fb_temp(const fb_temp&) = delete;
+  fb_temp& operator=(const fb_temp&) = delete;
+};
 
 #define FB_CHECK_CTX(ctx)                                                   \
   do {                                                                      \

@@ -17,7 +17,11 @@
  *  - `stream` is a cudaStream_t passed as void* (NULL = the default stream).  Calls enqueue work
  *    and return; only fb_sync, fb_memcpy_d2h and the fb_comm_* bootstrap calls block;
  *  - the caller owns all tensors, including the saved-for-backward buffers (statistics, gates,
- *    log-sum-exp); the library owns only a per-context scratch arena that grows on demand.
+ *    log-sum-exp); the library owns a per-context scratch arena that grows on demand and a memory pool that
+ *    single calls take their operand images from in their stream's order (up to 1 GiB stays with the context).
+ *    Pool memory is safe on any number of streams and in captured graphs.  The scratch arena (partial sums of
+ *    losses, bias gradients and normalisation layers, projections of recurrent layers) is not: calls of one
+ *    context that overlap on several streams, or with a replayed graph, need one context per stream.
  */
 #ifndef FLUXB200_H
 #define FLUXB200_H

@@ -187,7 +187,7 @@ def test_infinite_and_nan_operands(d, dv, lq, lk, causal, shift, dtype):
 
 
 def test_attention_two_streams():
-    """Calls of one thread on two streams share the context's operand arena: neither may read the other's copies."""
+    """Calls of one thread on two streams take their operand images from one pool: neither may read the other's."""
     import fluxb200 as F
     from fluxb200 import lib
     heads, d, n, batch = 8, 64, 512, 4
@@ -213,3 +213,73 @@ def test_attention_two_streams():
     torch.cuda.synchronize()
     for s in sets:
         assert torch.equal(s[3], s[5])
+
+
+def _forward_set(g, batch, n, heads, d):
+    q, k, v = (torch.randn(batch, n, heads * d, device="cuda", generator=g) for _ in range(3))
+    return q, k, v, torch.empty_like(q), torch.empty(batch * heads * n, device="cuda"), torch.empty_like(q)
+
+
+def test_attention_replay_beside_eager_calls():
+    """A replayed graph and eager calls (or another replay) on two streams: a captured call's images are its graph's own."""
+    import fluxb200 as F
+    from fluxb200 import lib
+    heads, d, n, batch = 8, 64, 512, 4
+    g = torch.Generator(device="cuda")
+    g.manual_seed(6)
+    dims = (heads * d, heads * d, n, n, batch, heads, 0)
+    ctx = F.context()
+    sets = [_forward_set(g, batch, n, heads, d) for _ in range(3)]
+
+    def forward(s, out):
+        lib.call("fb_attn_fwd", ctx.handle, ctx.stream, *[t.data_ptr() for t in s[:3]], None, out.data_ptr(), s[4].data_ptr(), *dims)
+    for s in sets:
+        forward(s, s[5])
+    torch.cuda.synchronize()
+    graphs = []
+    for s in sets[:2]:
+        graphs.append(torch.cuda.CUDAGraph())
+        with torch.cuda.graph(graphs[-1]):
+            for _ in range(3):
+                forward(s, s[3])
+    streams = [torch.cuda.Stream() for _ in range(3)]
+    for _ in range(10):
+        for graph, st in zip(graphs, streams):
+            with torch.cuda.stream(st):
+                graph.replay()
+        with torch.cuda.stream(streams[2]):
+            for _ in range(3):
+                forward(sets[2], sets[2][3])
+    torch.cuda.synchronize()
+    for s in sets:
+        assert torch.equal(s[3], s[5])
+
+
+def test_attention_captured_without_warm_up():
+    """A context whose first attention call of a size is inside a capture runs the same kernels there as eagerly."""
+    import fluxb200 as F
+    from fluxb200 import core, lib
+    heads, d, n, batch = 4, 64, 700, 3
+    g = torch.Generator(device="cuda")
+    g.manual_seed(7)
+    dims = (heads * d, heads * d, n, n, batch, heads, 1)
+    ctx, fresh = F.context(), core.Context(0)
+    q, k, v, o, lse, ref = _forward_set(g, batch, n, heads, d)
+    do = torch.randn(q.shape, device="cuda", generator=g)
+    grads, ref_grads = [[torch.empty_like(q) for _ in range(3)] for _ in range(2)]
+
+    def both(handle, out, gr):
+        p = [t.data_ptr() for t in (q, k, v)]
+        lib.call("fb_attn_fwd", handle, ctx.stream, *p, None, out.data_ptr(), lse.data_ptr(), *dims)
+        lib.call("fb_attn_bwd", handle, ctx.stream, *p, None, out.data_ptr(), lse.data_ptr(), do.data_ptr(), *[t.data_ptr() for t in gr], *dims)
+    both(ctx.handle, ref, ref_grads)
+    torch.cuda.synchronize()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        both(fresh.handle, o, grads)
+    for _ in range(2):
+        graph.replay()
+    torch.cuda.synchronize()
+    assert torch.equal(o, ref) and all(torch.equal(a, b) for a, b in zip(grads, ref_grads))
+    del graph
+    lib.call("fb_ctx_destroy", fresh.handle)
