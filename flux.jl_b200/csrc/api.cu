@@ -53,7 +53,6 @@ FB_API int32_t fb_ctx_create(int32_t device, fb_ctx** out) {
   c->scratch_bytes = 0;
   c->retired_count = 0;
   c->dev_error = nullptr;
-  c->gemm_ws = nullptr;
   e = cudaMalloc(&c->dev_error, 256);
   if (e != cudaSuccess) {
     delete c;
@@ -83,15 +82,15 @@ FB_API int32_t fb_ctx_create(int32_t device, fb_ctx** out) {
     delete c;
     return fb_fail(FB_ERR_ALLOC, "fb_ctx_create: cudaMemPoolCreate failed");
   }
-  int32_t ws_status = fb_side_kernels_prepare_elementwise();
-  if (ws_status == FB_OK) ws_status = fb_side_kernels_prepare_peer();
-  if (ws_status == FB_OK) ws_status = fb_gemm_workspace_create(c);
-  if (ws_status != FB_OK) {
+  int32_t status = fb_side_kernels_prepare_elementwise();
+  if (status == FB_OK) status = fb_side_kernels_prepare_peer();
+  fb_gemm_query_clusters(c);
+  if (status != FB_OK) {
     cudaMemPoolDestroy(c->pool);
     cudaFree(c->dev_error);
     cudaFreeHost((void*)c->host_page);
     delete c;
-    return ws_status;
+    return status;
   }
   *out = c;
   return FB_OK;
@@ -114,7 +113,6 @@ FB_API int32_t fb_ctx_destroy(fb_ctx* ctx) {
   for (int i = 0; i < ctx->retired_count; ++i) cudaFree(ctx->retired[i]);
   if (ctx->dev_error) cudaFree(ctx->dev_error);
   cudaFreeHost((void*)ctx->host_page);
-  fb_gemm_workspace_destroy(ctx);
   delete ctx;
   return FB_OK;
 }
@@ -207,11 +205,7 @@ FB_API int32_t fb_device_error(fb_ctx* ctx, void* stream, int32_t* out_host) {
   FB_REQUIRE(out_host, FB_ERR_INVALID_ARG, "fb_device_error: out is NULL");
   FB_CUDA(cudaMemcpyAsync(out_host, ctx->dev_error, sizeof(int32_t), cudaMemcpyDeviceToHost, (cudaStream_t)stream));
   FB_CUDA(cudaStreamSynchronize((cudaStream_t)stream));
-  if (*out_host != 0) {
-    // a kernel that gave up may have left GEMM tickets drawn: start the next launch from a clean state
-    fb_gemm_workspace_reset(ctx, (cudaStream_t)stream);
-    FB_CUDA(cudaMemsetAsync(ctx->dev_error, 0, sizeof(int32_t), (cudaStream_t)stream));
-  }
+  if (*out_host != 0) FB_CUDA(cudaMemsetAsync(ctx->dev_error, 0, sizeof(int32_t), (cudaStream_t)stream));
   return FB_OK;
 }
 

@@ -26,7 +26,7 @@ struct fb_ctx {
   int32_t* dev_error;    // device error word written by kernels whose bounded waits ran out
   uint32_t* host_page;   // pinned page that fb_read_scalar's kernel writes
   uint32_t host_seq;
-  void* gemm_ws;      // opaque (gemm_tc.cu): workspace of the split-tile GEMM schedule
+  int clusters[4];       // clusters of 1, 2, 4, 8 CTAs that hold an SM each (GEMM kernels) and are resident at once
 };
 
 // thread-local last-error message
@@ -249,9 +249,7 @@ bool fb_gemm_tc_supported(const fb_gemm_args& a);
 double fb_gemm_tc_time(fb_ctx* ctx, const fb_gemm_args& a);
 double fb_gemm_simt_time(const fb_ctx* ctx, const fb_gemm_args& a);
 int32_t fb_gemm_dispatch(fb_ctx* ctx, cudaStream_t stream, const fb_gemm_args& a, int precision);
-void fb_gemm_workspace_destroy(fb_ctx* ctx);
-// clusters of `size` (2, 4, 8) CTAs that hold an SM each and are resident at once
-int fb_gemm_resident_clusters(fb_ctx* ctx, int size);
+void fb_gemm_query_clusters(fb_ctx* ctx);
 // attention_tc.cu: tensor-core attention; FB_ERR_UNSUPPORTED when the call is not taken
 int32_t fb_attn_fwd_tc(fb_ctx* ctx, cudaStream_t stream, const float* q, const float* k, const float* v, const uint8_t* mask,
                        float* o, float* lse, int64_t e_dim, int64_t ev_dim, int64_t lq, int64_t lk, int64_t batch, int nheads,
@@ -263,13 +261,11 @@ int32_t fb_attn_fwd_redo(fb_ctx* ctx, cudaStream_t stream, int bf16, const void*
 int32_t fb_attn_bwd_tc(fb_ctx* ctx, cudaStream_t stream, const float* q, const float* k, const float* v, const uint8_t* mask, const float* o,
                        const float* lse, const float* dout, float* dq, float* dk, float* dv, int64_t e_dim, int64_t ev_dim, int64_t lq,
                        int64_t lk, int64_t batch, int nheads, int causal, bool* did_kv, bool* did_q);
-int32_t fb_gemm_workspace_create(fb_ctx* ctx);
 // Kernels that run on a communication stream beside a resident GEMM CTA (update, peer exchange, time marks) ask for
 // the same shared-memory carve-out as the GEMM: an SM runs CTAs of different kernels together only when they agree
 // on how its L1 / shared memory is split.
 int32_t fb_side_kernels_prepare_elementwise();
 int32_t fb_side_kernels_prepare_peer();
-void fb_gemm_workspace_reset(fb_ctx* ctx, cudaStream_t stream);
 
 // delta = dy .* act'(.) and db[j] = sum_rows delta[row][j]   (rows x cols row-major; cols = out_dim)
 int32_t fb_act_bwd_colsum(fb_ctx* ctx, cudaStream_t stream, int act, const float* dy, const float* y,

@@ -521,7 +521,7 @@ int32_t fb_gemm_bf16_launch(fb_ctx* ctx, cudaStream_t stream, const fb_gemm_bf16
         const int64_t slots = sms / ranks > 0 ? sms / ranks : 1;
         t = 5.0 + (double)((tiles + slots - 1) / slots) * (num_kb * t_kb[sh] + t_tile[sh]);
       } else {
-        if (ctx->reserved_sms != 0 || num_kb < 2 * s || s * ranks > 8 || tiles > fb_gemm_resident_clusters(ctx, s * ranks)) break;
+        if (ctx->reserved_sms != 0 || num_kb < 2 * s || s * ranks > 8 || tiles > ctx->clusters[lg + ranks - 1]) break;
         t = 8.0 + ((num_kb + s - 1) / s) * t_kb[sh] + t_tile[sh];
       }
       if (t < best_t) { best_t = t; best_sh = sh; best_s = s; }

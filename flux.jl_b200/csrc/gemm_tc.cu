@@ -62,7 +62,7 @@ struct Sched {
   int ksplit;        // CTAs of one cluster that share a tile, each with a part of its K range (1: no split)
   int seg;           // k-blocks per accumulation segment
   float* ws;         // [2 * G * ranks] slots of BM x 256 floats
-  int* tickets;      // [G * ranks * 4], zero between launches
+  int* tickets;      // [G * ranks * 4], zero at the start
 };
 struct Portion {
   int tile, kb0, kb1;
@@ -511,10 +511,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
         }
       }
       if (!SPLIT && p.partial && ok) {
-        if (fused) {
-          __syncwarp();
-          if (lane == 0) *ticket = 0;   // every part is accounted for: ready for the next launch
-        } else {
+        if (!fused) {
           // whoever draws the last ticket adds the slots up, in k order (the same sums as the fused path makes)
           __threadfence();
           __syncwarp();
@@ -534,8 +531,6 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
 #pragma unroll
               for (int j = 0; j < 4; ++j) emit4(row, v + 4 * j, nb + 4 * j, accumulate != 0, true);
             }
-            __syncwarp();
-            if (lane == 0) *ticket = 0;   // ready for the next launch
           }
         }
       }
@@ -631,12 +626,6 @@ struct Plan {
   bool tail;                // the last wave is cut along K and dealt out over all CTAs
 };
 
-struct GemmWorkspace {
-  float* ws;
-  int* tickets;
-  int clusters[4];   // clusters of 1, 2, 4, 8 CTAs that are resident at once
-};
-
 // Accumulation segment of a launch of one wave.  An even cut of all k-blocks over the SMs gives each of them num_kb * tiles / SMs
 // (tiles: 256 x 256 by two SMs, 128 x 256 or 128 x 128, the largest that occupy half of the GPU); no truncating sum is longer
 // than that, nor than 1664 k-values, and where the tiles fill 3/4 of the SMs by themselves 2048: a shared tile is then at
@@ -720,15 +709,23 @@ int32_t launch_variant(fb_ctx* ctx, cudaStream_t stream, const fb_gemm_args& a, 
   sch.tickets = nullptr;
   int64_t G = Gmax < num_tiles ? Gmax : num_tiles;
   const int64_t rest = num_tiles % Gmax;
-  const GemmWorkspace* gw = (const GemmWorkspace*)ctx->gemm_ws;
-  if (SPLIT) {
-    G = num_tiles * plan.ksplit;
-    sch.ws = gw->ws;
-  } else if (plan.tail && rest * sch.nu < 0x40000000) {
+  const bool tail = !SPLIT && plan.tail && rest * sch.nu < 0x40000000;
+  if (SPLIT) G = num_tiles * plan.ksplit;
+  // slots for segments that wait (one per CTA), or for the parts of a tail (two per CTA, and the tickets)
+  constexpr size_t SLOT = (size_t)BM * 256 * sizeof(float);
+  const size_t tickets = (size_t)ctx->sm_count * 4 * sizeof(int);
+  const size_t need = SPLIT ? ((num_kb + plan.ksplit - 1) / plan.ksplit > plan.seg ? SLOT * (size_t)(G * (PAIR ? 2 : 1)) : 0)
+                            : tail ? SLOT * 2 * (size_t)(Gmax * (PAIR ? 2 : 1)) + tickets : 0;
+  const fb_temp ws(ctx, stream, need);
+  sch.ws = (float*)ws.p;
+  if (need != 0 && ws.p == nullptr) {
+    // no memory: whole tiles, whose segments meet in C
+    if (SPLIT) return launch_variant<A_MN, B_MN, BN, PASSES, PAIR, SG, false>(ctx, stream, a, {plan.time, plan.shape, 1, plan.seg, false, false});
+  } else if (tail) {
     sch.dp_tiles = (int)(num_tiles - rest);
     sch.U = (int)(rest * sch.nu);
-    sch.ws = gw->ws;
-    sch.tickets = gw->tickets;
+    sch.tickets = (int*)((char*)ws.p + need - tickets);
+    FB_CUDA(cudaMemsetAsync(sch.tickets, 0, tickets, stream));
     G = Gmax;
   }
   cudaLaunchConfig_t lc;
@@ -794,7 +791,6 @@ double tail_time(int64_t rest, int64_t slots, int num_kb, double t_kb, double t_
 }
 
 Plan plan_3xtf32(fb_ctx* ctx, const fb_gemm_args& a, bool force_pair) {
-  const GemmWorkspace* gw = (const GemmWorkspace*)ctx->gemm_ws;
   const int sms = ctx->sm_count - ctx->reserved_sms;
   const int num_kb = (int)((a.K + BK - 1) / BK);
   static const int bm[3] = {128, 128, 256}, bn[3] = {128, 256, 256};
@@ -818,7 +814,7 @@ Plan plan_3xtf32(fb_ctx* ctx, const fb_gemm_args& a, bool force_pair) {
         const double whole = num_kb * t_kb[sh] + t_tile[sh];
         if (full == 0) {
           // one wave: whole tiles, or their units over all CTAs
-          if (gw != nullptr) seg = segment_kblocks(a, num_kb, num_kb, sms, &drains);
+          seg = segment_kblocks(a, num_kb, num_kb, sms, &drains);
           const double cut = tail_time(rest, slots, num_kb, t_kb[sh], t_tile[sh]);
           tail = cut < whole + 2.5 * drains;
           if (tail) { seg = SEG_KB; drains = 0; }
@@ -826,11 +822,11 @@ Plan plan_3xtf32(fb_ctx* ctx, const fb_gemm_args& a, bool force_pair) {
         } else if (rest != 0) {
           // A last wave that fills less than 3/4 of the machine is always cut.  (Fuller waves gain nothing: the kernel runs at
           // the power limit, where idle SMs let the busy ones clock higher.)
-          tail = 4 * rest < 3 * slots && num_kb > UNIT_KB && gw != nullptr;
+          tail = 4 * rest < 3 * slots && num_kb > UNIT_KB;
           t += tail ? tail_time(rest, slots, num_kb, t_kb[sh], t_tile[sh]) : whole;
         }
       } else {
-        if (sh == 2 || gw == nullptr || ctx->reserved_sms != 0 || num_kb < 2 * s || tiles > gw->clusters[lg]) break;
+        if (sh == 2 || ctx->reserved_sms != 0 || num_kb < 2 * s || tiles > ctx->clusters[lg]) break;
         const int part_kb = (num_kb + s - 1) / s;
         t = 8.5 + part_kb * t_kb[sh] + t_tile[sh];
         seg = segment_kblocks(a, num_kb, part_kb, sms, &drains);
@@ -840,33 +836,6 @@ Plan plan_3xtf32(fb_ctx* ctx, const fb_gemm_args& a, bool force_pair) {
     }
   }
   return best;
-}
-
-// How many clusters of 2, 4 and 8 CTAs with the GEMM's shared memory are resident at once.
-void query_clusters(fb_ctx* ctx, int* clusters) {
-  auto kern = gemm_tc_kernel<false, true, 256, 3, false, 2, true>;
-  using cfg = Cfg<256, 3, false, 2>;
-  clusters[0] = ctx->sm_count;
-  for (int lg = 1; lg < 4; ++lg) {
-    clusters[lg] = 0;
-    cudaLaunchConfig_t lc;
-    memset(&lc, 0, sizeof(lc));
-    lc.gridDim = dim3((unsigned)(ctx->sm_count / (1 << lg) * (1 << lg)), 1, 1);
-    lc.blockDim = dim3(cfg::NUM_THREADS, 1, 1);
-    lc.dynamicSmemBytes = cfg::SMEM_BYTES;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeClusterDimension;
-    attr[0].val.clusterDim.x = 1u << lg;
-    attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
-    lc.attrs = attr;
-    lc.numAttrs = 1;
-    int n = 0;
-    if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, cfg::SMEM_BYTES) == cudaSuccess &&
-        cudaOccupancyMaxActiveClusters(&n, kern, &lc) == cudaSuccess)
-      clusters[lg] = n;
-    else
-      cudaGetLastError();
-  }
 }
 
 }  // namespace
@@ -893,7 +862,7 @@ int32_t fb_gemm_tc_launch(fb_ctx* ctx, cudaStream_t stream, const fb_gemm_args& 
     const bool narrow1 = (a.N <= 128) || (2 * ((a.M + BM - 1) / BM) * ((a.N + 255) / 256) <= ctx->sm_count);
     // (TF32 in one pass: the last wave is cut as it always was)
     const int64_t slots = ctx->sm_count - ctx->reserved_sms, rest = (((a.M + BM - 1) / BM) * ((a.N + (narrow1 ? 127 : 255)) / (narrow1 ? 128 : 256))) % slots;
-    const Plan whole = {0.0, 0, 1, SEG_KB, false, ctx->gemm_ws != nullptr && rest != 0 && 4 * rest < 3 * slots && a.K > BK * UNIT_KB};
+    const Plan whole = {0.0, 0, 1, SEG_KB, false, rest != 0 && 4 * rest < 3 * slots && a.K > BK * UNIT_KB};
     return narrow1 ? launch_layout_sg<128, 1, false, 2, false>(ctx, stream, a, whole) : launch_layout_sg<256, 1, false, 2, false>(ctx, stream, a, whole);
   }
   const Plan p = plan_3xtf32(ctx, a, passes == 32);
@@ -902,42 +871,29 @@ int32_t fb_gemm_tc_launch(fb_ctx* ctx, cudaStream_t stream, const fb_gemm_args& 
   return launch_layout<256, true>(ctx, stream, a, p);
 }
 
-// Called by fb_ctx_create / fb_ctx_destroy.  The workspace is allocated up front (2 slots of 128 x 256 floats per
-// SM, 37 MiB on 148 SMs) so that no launch allocates; calls that share a context must be ordered on one stream.
-int32_t fb_gemm_workspace_create(fb_ctx* ctx) {
-  GemmWorkspace* gw = new GemmWorkspace();
-  gw->ws = nullptr;
-  gw->tickets = nullptr;
-  const size_t slots = (size_t)2 * (size_t)ctx->sm_count;
-  const size_t tickets = (size_t)ctx->sm_count * 4;
-  if (cudaMalloc(&gw->ws, slots * BM * 256 * sizeof(float)) != cudaSuccess ||
-      cudaMalloc(&gw->tickets, tickets * sizeof(int)) != cudaSuccess) {
-    cudaGetLastError();
-    if (gw->ws) cudaFree(gw->ws);
-    delete gw;
-    return fb_fail(FB_ERR_ALLOC, "fb_ctx_create: GEMM workspace allocation failed");
+// How many clusters of 2, 4 and 8 CTAs with the GEMM's shared memory are resident at once (called by fb_ctx_create).
+void fb_gemm_query_clusters(fb_ctx* ctx) {
+  auto kern = gemm_tc_kernel<false, true, 256, 3, false, 2, true>;
+  using cfg = Cfg<256, 3, false, 2>;
+  ctx->clusters[0] = ctx->sm_count;
+  for (int lg = 1; lg < 4; ++lg) {
+    ctx->clusters[lg] = 0;
+    cudaLaunchConfig_t lc;
+    memset(&lc, 0, sizeof(lc));
+    lc.gridDim = dim3((unsigned)(ctx->sm_count / (1 << lg) * (1 << lg)), 1, 1);
+    lc.blockDim = dim3(cfg::NUM_THREADS, 1, 1);
+    lc.dynamicSmemBytes = cfg::SMEM_BYTES;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = 1u << lg;
+    attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+    lc.attrs = attr;
+    lc.numAttrs = 1;
+    int n = 0;
+    if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, cfg::SMEM_BYTES) == cudaSuccess &&
+        cudaOccupancyMaxActiveClusters(&n, kern, &lc) == cudaSuccess)
+      ctx->clusters[lg] = n;
+    else
+      cudaGetLastError();
   }
-  cudaMemset(gw->tickets, 0, tickets * sizeof(int));
-  query_clusters(ctx, gw->clusters);
-  ctx->gemm_ws = gw;
-  return FB_OK;
-}
-
-void fb_gemm_workspace_reset(fb_ctx* ctx, cudaStream_t stream) {
-  GemmWorkspace* gw = (GemmWorkspace*)ctx->gemm_ws;
-  if (gw != nullptr && gw->tickets != nullptr) cudaMemsetAsync(gw->tickets, 0, (size_t)ctx->sm_count * 4 * sizeof(int), stream);
-}
-
-int fb_gemm_resident_clusters(fb_ctx* ctx, int size) {
-  const GemmWorkspace* gw = (const GemmWorkspace*)ctx->gemm_ws;
-  return gw == nullptr ? 0 : gw->clusters[size == 8 ? 3 : size == 4 ? 2 : size == 2 ? 1 : 0];
-}
-
-void fb_gemm_workspace_destroy(fb_ctx* ctx) {
-  GemmWorkspace* gw = (GemmWorkspace*)ctx->gemm_ws;
-  if (gw == nullptr) return;
-  if (gw->ws) cudaFree(gw->ws);
-  if (gw->tickets) cudaFree(gw->tickets);
-  delete gw;
-  ctx->gemm_ws = nullptr;
 }

@@ -189,3 +189,39 @@ def test_dense_forward_epilogues_of_cut_tiles(ctx, act, out_dim, in_dim, n):
     assert ((z.double() - zr).norm() / zr.norm()) < 3e-5
     assert ((y.double() - yr).norm() / yr.norm()) < 3e-5
     assert ctx.device_error() == 0
+
+
+@pytest.mark.parametrize("m,n,k", [(512, 512, 32768), (1000, 2048, 4096), (1024, 5120, 2048)])
+def test_split_products_on_several_streams(ctx, m, n, k):
+    """Products that park segments or the parts of a cut last wave in memory of their own, on two streams and beside the
+    replays of a graph on a third: every result is the serial one, bit for bit."""
+    from fluxb200 import lib
+    sets = []
+    for i in range(3):
+        g = torch.Generator(device="cuda").manual_seed(i)
+        A, B = (torch.randn(k, d, generator=g, device="cuda") for d in (m, n))
+        sets.append((A, B.T.contiguous(), torch.empty(n, m, device="cuda"), torch.empty(n, m, device="cuda")))
+
+    def product(s, out):
+        lib.call("fb_gemm_f32", ctx.handle, ctx.stream, 0, 0, m, n, k, s[0].data_ptr(), m, s[1].data_ptr(), k, out.data_ptr(), m, 0, 0)
+    for s in sets:
+        product(s, s[3])
+    torch.cuda.synchronize()
+    ref = sets[0][1].double() @ sets[0][0].double()
+    assert ((sets[0][3].double() - ref).norm() / ref.norm()) < 3e-5
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        product(sets[2], sets[2][2])
+        product(sets[2], sets[2][2])
+    streams = [torch.cuda.Stream() for _ in range(3)]
+    for _ in range(10):
+        for s, st in zip(sets[:2], streams):
+            with torch.cuda.stream(st):
+                product(s, s[2])
+                product(s, s[2])
+        with torch.cuda.stream(streams[2]):
+            graph.replay()
+    torch.cuda.synchronize()
+    for s in sets:
+        assert torch.equal(s[2], s[3])
+    assert ctx.device_error() == 0
