@@ -85,20 +85,29 @@ static PyObject* w_{name}(PyObject* self, PyObject* const* a, Py_ssize_t n) {{
     return "".join(out)
 
 
-def build_fastcall(force: bool = False) -> str:
-    """The native call wrappers, generated from the header and compiled with the host compiler."""
+def build_fastcall(force: bool = False):
+    """The native call wrappers, generated from the header and compiled with the host compiler.  Optional: without the Python
+    headers or a C compiler nothing is built (nor left from an older header), calls go through ctypes, and None is returned."""
     header = os.path.join(HERE, "..", "include", "fluxb200.h")
     head = os.path.join(HERE, "csrc", "fastcall_head.h")
     out = os.path.join(HERE, "fluxb200", "_fastcall" + sysconfig.get_config_var("EXT_SUFFIX"))
-    if force or _newer([header, head, os.path.abspath(__file__)], out):
-        src = os.path.join(OBJ, "fastcall.c")
-        with open(src, "w") as f:
-            f.write(_fastcall_source(header))
-        cmd = [os.environ.get("CC") or "gcc", "-O2", "-shared", "-fPIC", "-I", sysconfig.get_paths()["include"], src, "-o", out]
-        r = subprocess.run(cmd, capture_output=True, text=True)
-        if r.returncode != 0:
-            print(r.stdout + r.stderr)
-            raise RuntimeError("building the native call wrappers failed")
+    if not force and not _newer([header, head, os.path.abspath(__file__)], out):
+        return out
+    include, cc = sysconfig.get_paths()["include"], os.environ.get("CC") or "gcc"
+    missing = "Python.h" if not os.path.exists(os.path.join(include, "Python.h")) else cc if shutil.which(cc.split()[0]) is None else None
+    if missing is not None:
+        print(f"no {missing}: the native call wrappers are not built, calls go through ctypes")
+        if os.path.exists(out):
+            os.remove(out)
+        return None
+    src = os.path.join(OBJ, "fastcall.c")
+    with open(src, "w") as f:
+        f.write(_fastcall_source(header))
+    cmd = cc.split() + ["-O2", "-shared", "-fPIC", "-I", include, src, "-o", out]
+    r = subprocess.run(cmd, capture_output=True, text=True)
+    if r.returncode != 0:
+        print(r.stdout + r.stderr)
+        raise RuntimeError("building the native call wrappers failed")
     return out
 
 

@@ -77,3 +77,28 @@ def test_product_never_imports_the_oracle():
             if f.endswith((".py", ".cu", ".cuh", ".jl")):
                 txt = open(os.path.join(dirpath, f), errors="replace").read()
                 assert "flux_oracle" not in txt and "oracle/" not in txt, f
+
+
+@pytest.mark.parametrize("missing", ["headers", "compiler"])
+def test_build_without_python_headers_or_compiler(monkeypatch, tmp_path, missing):
+    """The native call wrappers are optional: a machine that cannot compile them still builds, and keeps no stale ones."""
+    import importlib.util
+    import shutil
+    pkg = os.path.join(ROOT, "flux.jl_b200")
+    spec = importlib.util.spec_from_file_location("fluxb200_build_copy", os.path.join(pkg, "build.py"))
+    build = importlib.util.module_from_spec(spec)
+    spec.loader.exec_module(build)
+    here = tmp_path / "pkg"
+    for d in (here / "csrc", here / "fluxb200", tmp_path / "include", tmp_path / "obj", tmp_path / "empty"):
+        d.mkdir(parents=True)
+    shutil.copy(os.path.join(pkg, "csrc", "fastcall_head.h"), here / "csrc")
+    shutil.copy(HEADER, tmp_path / "include")
+    monkeypatch.setattr(build, "HERE", str(here))
+    monkeypatch.setattr(build, "OBJ", str(tmp_path / "obj"))
+    out = here / "fluxb200" / ("_fastcall" + build.sysconfig.get_config_var("EXT_SUFFIX"))
+    out.write_bytes(b"of an older header")
+    if missing == "headers":
+        monkeypatch.setattr(build.sysconfig, "get_paths", lambda: {"include": str(tmp_path / "empty")})
+    else:
+        monkeypatch.setenv("CC", str(tmp_path / "empty" / "cc"))
+    assert build.build_fastcall(force=True) is None and not out.exists()
