@@ -71,11 +71,13 @@ __device__ __forceinline__ uint32_t pack_bf16(float lo, float hi) {
 __device__ __forceinline__ float bf16_lo(uint32_t w) { return __uint_as_float(w << 16); }
 __device__ __forceinline__ float bf16_hi(uint32_t w) { return __uint_as_float(w & 0xffff0000u); }
 
-template <bool A_MN, bool B_MN, int BN, bool PAIR>
+// SPLIT: the CTAs (pairs) of a cluster share one tile, each with a part of its K range.  A kernel of its own: shared with the
+// plain launches it is in their way, as are they in its.
+template <bool A_MN, bool B_MN, int BN, bool PAIR, bool SPLIT>
 __global__ void __launch_bounds__(HCfg<BN, PAIR>::NUM_THREADS, 1)
 gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB, void* __restrict__ Cv,
                  int64_t ldc, uint16_t* __restrict__ Z, const uint16_t* __restrict__ bias_n, int M, int N, int K, int act,
-                 int accumulate, int out_f32, int32_t* __restrict__ dev_err, int a3d, int b3d, int num_tiles, int tiles_n, int ksplit) {
+                 int accumulate, int out_f32, int32_t* __restrict__ dev_err, int a3d, int b3d, int num_tiles, int tiles_n, int nsplit) {
   using cfg = HCfg<BN, PAIR>;
   constexpr int STAGES = cfg::STAGES;
   extern __shared__ uint8_t smem_raw[];
@@ -93,16 +95,17 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
   volatile int* s_skip = (volatile int*)(bars + 3 * STAGES + 6);   // [0] mine, [1] written by the peer CTA
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  // ksplit > 1: the CTAs (pairs) of a cluster share one tile, each with a part of its K range
-  const uint32_t crank = (PAIR || ksplit > 1) ? cluster_ctarank() : 0u;
+  const int ksplit = SPLIT ? nsplit : 1;
+  const uint32_t crank = (PAIR || SPLIT) ? cluster_ctarank() : 0u;
   const uint32_t rank = PAIR ? (crank & 1u) : 0u;
   const uint32_t lead_rank = crank - rank;
   const bool leader = (rank == 0);
   const int cid = PAIR ? (int)(blockIdx.x >> 1) : (int)blockIdx.x;
   const int G = PAIR ? (int)(gridDim.x >> 1) : (int)gridDim.x;
-  const int all_kb = (K + HBK - 1) / HBK, part = cid % ksplit;
-  const int kb0 = (int)((long long)all_kb * part / ksplit), num_kb = (int)((long long)all_kb * (part + 1) / ksplit) - kb0;
-  const int tile_beg = cid / ksplit, tile_step = ksplit > 1 ? num_tiles : G;
+  const int all_kb = (K + HBK - 1) / HBK, part = SPLIT ? cid % ksplit : 0;
+  const int kb0 = SPLIT ? (int)((long long)all_kb * part / ksplit) : 0;
+  const int num_kb = SPLIT ? (int)((long long)all_kb * (part + 1) / ksplit) - kb0 : all_kb;
+  const int tile_beg = SPLIT ? cid / ksplit : cid, tile_step = SPLIT ? num_tiles : G;
   auto tile_m0 = [&](int t) { return PAIR ? (t / tiles_n) * 256 + 128 * (int)rank : (t / tiles_n) * HBM_; };
   auto tile_n0 = [&](int t) { return (t % tiles_n) * BN; };
 
@@ -121,7 +124,7 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     fence_proxy_async();
   }
-  if (PAIR || ksplit > 1) {
+  if (PAIR || SPLIT) {
     __syncwarp();
     cluster_sync_all();   // all CTAs of the cluster run and their barriers exist: remote accesses may start
     if (threadIdx.x == 0 && crank == 0) {
@@ -193,11 +196,15 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
         *(uint4*)crow = make_uint4(pack_bf16(u[0], u[1]), pack_bf16(u[2], u[3]), pack_bf16(u[4], u[5]), pack_bf16(u[6], u[7]));
       }
     } else {
+      constexpr int TAIL_UNROLL = SPLIT ? 1 : 8;   // rolled, the cluster's reduction is 1.5 us shorter (less code to fetch)
+      float t[8];
 #pragma unroll
+      for (int e = 0; e < 8; ++e) t[e] = u[e];
+#pragma unroll TAIL_UNROLL
       for (int e = 0; e < 8; ++e) {
         if (n + e >= N) break;
         const int64_t o = (int64_t)row * ldc + n + e;
-        float x = u[e];
+        float x = t[e];
         if (accumulate) x += out_f32 ? ((float*)Cv)[o] : bf16_lo((uint32_t)((uint16_t*)Cv)[o]);
         if (bias_n) x += bf16_lo((uint32_t)bias_n[n + e]);
         if (Z) Z[o] = (uint16_t)(pack_bf16(x, 0.0f) & 0xffffu);
@@ -326,13 +333,40 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
         tc_ld_32x32b_x32(tmem_base + ((uint32_t)(32 * q) << 16) + (uint32_t)(buf * BN + cc * 32), r);
         tc_wait_ld();
         float* v = reinterpret_cast<float*>(r);
-        if (ksplit > 1) {   // all MMAs have read their stages: the sums go where the cluster can add them up
+        if (SPLIT) {   // all MMAs have read their stages: the sums go where the cluster can add them up
           float4* d4 = (float4*)((float*)smem + (32 * q + lane) * (BN + 4) + cc * 32);
 #pragma unroll
           for (int j = 0; j < 8; ++j) d4[j] = make_float4(v[4 * j], v[4 * j + 1], v[4 * j + 2], v[4 * j + 3]);
-        } else {
+        } else if (out_f32 || nb + 31 >= N) {
 #pragma unroll
           for (int j = 0; j < 4; ++j) emit8(row, v + 8 * j, nb + 8 * j);
+        } else if (row < M) {
+          // the usual case apart from emit8, whose code for the others between the pieces costs 1 - 2 us a launch (608 x 64 x
+          // 376: 10.3 us, so 8.3; 4096 x 2048 x 4096 with gelu 77 and 72)
+          uint16_t* crow = (uint16_t*)Cv + (int64_t)row * ldc + nb;
+          uint16_t* zrow = Z ? Z + (int64_t)row * ldc + nb : nullptr;
+#pragma unroll
+          for (int j = 0; j < 4; ++j) {       // 8 columns = one 16-byte store
+            float u[8];
+#pragma unroll
+            for (int e = 0; e < 8; ++e) u[e] = v[8 * j + e];
+            if (accumulate) {
+              const uint4 c4 = *(const uint4*)(crow + 8 * j);
+              u[0] += bf16_lo(c4.x); u[1] += bf16_hi(c4.x); u[2] += bf16_lo(c4.y); u[3] += bf16_hi(c4.y);
+              u[4] += bf16_lo(c4.z); u[5] += bf16_hi(c4.z); u[6] += bf16_lo(c4.w); u[7] += bf16_hi(c4.w);
+            }
+            if (bias_n) {
+              const uint4 b4 = __ldg((const uint4*)(bias_n + nb + 8 * j));
+              u[0] += bf16_lo(b4.x); u[1] += bf16_hi(b4.x); u[2] += bf16_lo(b4.y); u[3] += bf16_hi(b4.y);
+              u[4] += bf16_lo(b4.z); u[5] += bf16_hi(b4.z); u[6] += bf16_lo(b4.w); u[7] += bf16_hi(b4.w);
+            }
+            if (zrow) *(uint4*)(zrow + 8 * j) = make_uint4(pack_bf16(u[0], u[1]), pack_bf16(u[2], u[3]), pack_bf16(u[4], u[5]), pack_bf16(u[6], u[7]));
+            if (act != FB_ACT_IDENTITY) {
+#pragma unroll
+              for (int e = 0; e < 8; ++e) u[e] = fb_act_apply(act, u[e]);
+            }
+            *(uint4*)(crow + 8 * j) = make_uint4(pack_bf16(u[0], u[1]), pack_bf16(u[2], u[3]), pack_bf16(u[4], u[5]), pack_bf16(u[6], u[7]));
+          }
         }
       }
       // this buffer may be overwritten once every epilogue warp (of both CTAs) has read its quadrant
@@ -346,7 +380,7 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
   }
 
   // ---------------------------------------------- split K: the cluster adds up its parts ---
-  if (ksplit > 1) {
+  if (SPLIT) {
     __syncwarp();
     cluster_sync_all();
     const int rows = HBM_ / ksplit, m0 = tile_m0(tile_beg), n0 = tile_n0(tile_beg);
@@ -379,7 +413,7 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
   // ---------------------------------------------------------------------- teardown ---
   tc_fence_before();
   __syncthreads();
-  if (PAIR || ksplit > 1) cluster_sync_all();   // no CTA may release its tensor or shared memory while a peer can still touch it
+  if (PAIR || SPLIT) cluster_sync_all();   // no CTA may release its tensor or shared memory while a peer can still touch it
   if (warp == 1) {
     __syncwarp();
     if (PAIR)
@@ -416,7 +450,7 @@ bool encode_map_bf16_mn3d(CUtensorMap* map, const uint16_t* base, int64_t K, int
             CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
-template <bool A_MN, bool B_MN, int BN, bool PAIR>
+template <bool A_MN, bool B_MN, int BN, bool PAIR, bool SPLIT>
 int32_t launch_bf16(fb_ctx* ctx, cudaStream_t stream, const fb_gemm_bf16_args& a, int ksplit) {
   using cfg = HCfg<BN, PAIR>;
   CUtensorMap tmA, tmB;
@@ -438,7 +472,7 @@ int32_t launch_bf16(fb_ctx* ctx, cudaStream_t stream, const fb_gemm_bf16_args& a
   }
   if (!ok) return fb_fail(FB_ERR_CUDA, "bf16 gemm: cuTensorMapEncodeTiled failed (M=%lld N=%lld K=%lld lda=%lld ldb=%lld)",
                           (long long)a.M, (long long)a.N, (long long)a.K, (long long)a.lda, (long long)a.ldb);
-  auto kern = gemm_bf16_kernel<A_MN, B_MN, BN, PAIR>;
+  auto kern = gemm_bf16_kernel<A_MN, B_MN, BN, PAIR, SPLIT>;
   FB_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, cfg::SMEM_BYTES));
   // the whole L1 / shared array as shared memory: the communication-stream kernels ask for the same split, and an SM
   // takes CTAs of two kernels together only when their splits agree
@@ -449,7 +483,7 @@ int32_t launch_bf16(fb_ctx* ctx, cudaStream_t stream, const fb_gemm_bf16_args& a
   if (num_tiles > 0x7fffffff) return fb_fail(FB_ERR_UNSUPPORTED, "bf16 gemm: too many tiles");
   const int sms = ctx->sm_count - ctx->reserved_sms;
   const int64_t Gmax = PAIR ? (sms / 2 > 0 ? sms / 2 : 1) : sms;
-  const int64_t G = ksplit > 1 ? num_tiles * ksplit : Gmax < num_tiles ? Gmax : num_tiles;
+  const int64_t G = SPLIT ? num_tiles * ksplit : Gmax < num_tiles ? Gmax : num_tiles;
   cudaLaunchConfig_t lc;
   memset(&lc, 0, sizeof(lc));
   lc.gridDim = dim3((unsigned)(PAIR ? 2 * G : G), 1, 1);
@@ -469,14 +503,14 @@ int32_t launch_bf16(fb_ctx* ctx, cudaStream_t stream, const fb_gemm_bf16_args& a
   return FB_OK;
 }
 
-template <int BN, bool PAIR>
+template <int BN, bool PAIR, bool SPLIT>
 int32_t launch_bf16_layout(fb_ctx* ctx, cudaStream_t stream, const fb_gemm_bf16_args& a, int ksplit) {
   if (a.a_mn_major) {
-    if (a.b_mn_major) return launch_bf16<true, true, BN, PAIR>(ctx, stream, a, ksplit);
-    return launch_bf16<true, false, BN, PAIR>(ctx, stream, a, ksplit);
+    if (a.b_mn_major) return launch_bf16<true, true, BN, PAIR, SPLIT>(ctx, stream, a, ksplit);
+    return launch_bf16<true, false, BN, PAIR, SPLIT>(ctx, stream, a, ksplit);
   }
-  if (a.b_mn_major) return launch_bf16<false, true, BN, PAIR>(ctx, stream, a, ksplit);
-  return launch_bf16<false, false, BN, PAIR>(ctx, stream, a, ksplit);
+  if (a.b_mn_major) return launch_bf16<false, true, BN, PAIR, SPLIT>(ctx, stream, a, ksplit);
+  return launch_bf16<false, false, BN, PAIR, SPLIT>(ctx, stream, a, ksplit);
 }
 
 }  // namespace
@@ -527,7 +561,12 @@ int32_t fb_gemm_bf16_launch(fb_ctx* ctx, cudaStream_t stream, const fb_gemm_bf16
       if (t < best_t) { best_t = t; best_sh = sh; best_s = s; }
     }
   }
-  if (best_sh == 2) return launch_bf16_layout<256, true>(ctx, stream, a, best_s);
-  if (best_sh == 1) return launch_bf16_layout<256, false>(ctx, stream, a, best_s);
-  return launch_bf16_layout<128, false>(ctx, stream, a, best_s);
+  if (best_s > 1) {
+    if (best_sh == 2) return launch_bf16_layout<256, true, true>(ctx, stream, a, best_s);
+    if (best_sh == 1) return launch_bf16_layout<256, false, true>(ctx, stream, a, best_s);
+    return launch_bf16_layout<128, false, true>(ctx, stream, a, best_s);
+  }
+  if (best_sh == 2) return launch_bf16_layout<256, true, false>(ctx, stream, a, 1);
+  if (best_sh == 1) return launch_bf16_layout<256, false, false>(ctx, stream, a, 1);
+  return launch_bf16_layout<128, false, false>(ctx, stream, a, 1);
 }

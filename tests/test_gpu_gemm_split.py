@@ -172,6 +172,20 @@ def test_gemm_bf16_cuts(ctx, ta, tb, m, n, k, f32):
     assert ctx.device_error() == 0
 
 
+@pytest.mark.parametrize("m,n,k", [(509, 104, 784), (77, 200, 64), (1021, 2048, 4096), (250, 300, 5000)])
+@pytest.mark.parametrize("f32", [0, 1])
+def test_gemm_bf16_ragged_rows(ctx, m, n, k, f32):
+    """rows of the result that are no multiple of 8 long, in plain and shared tiles; the padding of a row stays as it is"""
+    from fluxb200 import lib
+    ld = (m + 7) // 8 * 8
+    A, B, ref = _operands(0, 0, m, n, k, 0, torch.bfloat16)
+    A = torch.nn.functional.pad(A, (0, ld - m))
+    out = torch.full((n, ld), 3.0, device="cuda", dtype=torch.float32 if f32 else torch.bfloat16)
+    lib.call("fb_gemm_bf16", ctx.handle, ctx.stream, 0, 0, m, n, k, A.data_ptr(), ld, B.data_ptr(), B.shape[1], out.data_ptr(), ld, 0, f32)
+    assert float((out[:, :m].double() - ref).norm() / ref.norm()) < (3e-5 if f32 else 2.0 ** -9)
+    assert bool((out[:, m:] == 3.0).all()) and ctx.device_error() == 0
+
+
 @pytest.mark.parametrize("act", ["identity", "relu", "gelu_tanh"])
 @pytest.mark.parametrize("out_dim,in_dim,n", [(512, 784, 1), (10, 512, 100), (513, 300, 70), (512, 784, 1024), (1001, 520, 500)])
 def test_dense_forward_epilogues_of_cut_tiles(ctx, act, out_dim, in_dim, n):
