@@ -45,3 +45,62 @@ def test_sequence_kernels(cell, I, H, T, B):
     close(F.cpu(c["Wh"]), rWh, name="dWh", **tol)
     close(F.cpu(c["bias" if cell == "lstm" else "b"]), rb, name="db", **tol)
     assert F.context().device_error() == 0
+
+
+# (a CTA walks several chunks of columns for many steps; hidden sizes beyond 512 that are no multiple of 4: scalar loads in
+# several 512-wide pieces; three chunks of a small layer)
+LONG = [("lstm", 3, 772, 40, 70), ("gru", 3, 772, 40, 70), ("gru", 5, 515, 30, 40), ("lstm", 4, 530, 30, 33), ("lstm", 6, 200, 60, 300),
+        ("gru", 6, 203, 60, 300)]
+
+
+def _rnn(cell, I, H, T, B):
+    import fluxb200 as F
+    rng = np.random.default_rng(I + H + T + B)
+    ng = 4 if cell == "lstm" else 3
+    Wi, Wh = O.glorot_uniform(rng, ng * H, I), O.glorot_uniform(rng, ng * H, H)
+    b = (rng.normal(size=ng * H) * 0.1).astype(np.float32)
+    x = rng.normal(size=(I, T, B)).astype(np.float32)
+    state = tuple(rng.normal(size=(H, B)).astype(np.float32) for _ in range(2 if cell == "lstm" else 1))
+    return (F.LSTM if cell == "lstm" else F.GRU)(Wi, Wh, b.copy()), (Wi, Wh, b, x), state
+
+
+def _autograd(cell, arrays, state, out):
+    """dWi, dWh, db of sum(abs2, out) in float64 (the oracle's reverse sweeps start from zero states)."""
+    import torch
+    Wi, Wh, b = (torch.tensor(v, requires_grad=True) for v in arrays[:3])
+    x, h, c = torch.tensor(arrays[3]), torch.tensor(state[0]), torch.tensor(state[-1])
+    total, worst = 0.0, 0.0
+    for t in range(x.shape[1]):
+        if cell == "lstm":
+            i, f, g, o = (Wi @ x[:, t] + Wh @ h + b[:, None]).chunk(4)
+            c = torch.sigmoid(f) * c + torch.sigmoid(i) * torch.tanh(g)
+            h = torch.sigmoid(o) * torch.tanh(c)
+        else:
+            gx, gh = (Wi @ x[:, t] + b[:, None]).chunk(3), (Wh @ h).chunk(3)
+            r, z = torch.sigmoid(gx[0] + gh[0]), torch.sigmoid(gx[1] + gh[1])
+            h = (1 - z) * torch.tanh(gx[2] + r * gh[2]) + z * h
+        total = total + (h * h).sum()
+        worst = max(worst, float((h.detach() - torch.tensor(out[:, t])).abs().max()))
+    assert worst < 1e-10      # the same recurrence as the oracle's
+    total.backward()
+    return [v.grad.numpy() for v in (Wi, Wh, b)]
+
+
+@pytest.mark.parametrize("cell,I,H,T,B", LONG)
+def test_long_sequences_with_initial_state(cell, I, H, T, B):
+    import fluxb200 as F
+    rnn, arrays, state = _rnn(cell, I, H, T, B)
+    xg, sg = F.gpu(arrays[3]), tuple(F.gpu(s) for s in state)
+    start = sg if cell == "lstm" else sg[0]
+    a64, s64 = [v.astype(np.float64) for v in arrays], [v.astype(np.float64) for v in state]
+    ref = (O.lstm_scan_fwd if cell == "lstm" else O.gru_scan_fwd)(*a64, *s64)[0]
+    close(F.cpu(rnn(xg, start)), ref, name="out")
+    _, (g,) = F.withgradient(lambda m: F.sum_abs2(m(xg, start)), rnn)
+    grads = _autograd(cell, a64, s64, ref)
+    # two chained reductions as above, over T * B columns
+    tol = dict(rtol=2e-4, atol_scale=2e-4)
+    c = g["cell"]
+    close(F.cpu(c["Wi"]), grads[0], name="dWi", **tol)
+    close(F.cpu(c["Wh"]), grads[1], name="dWh", **tol)
+    close(F.cpu(c["bias" if cell == "lstm" else "b"]), grads[2], name="db", **tol)
+    assert F.context().device_error() == 0
