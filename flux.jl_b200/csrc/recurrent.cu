@@ -490,22 +490,9 @@ bool persistent_enabled() {
   return on != 0;
 }
 
-// The blocks of the sequence kernels wait for one another's results (bounded), which needs every block resident at
-// once.  Outside a stream capture they are launched cooperatively (the runtime then guarantees it, or
-// refuses).  A cooperative launch cannot be recorded into a CUDA graph, so under capture the same kernel is launched
-// plainly: its grid was sized by the occupancy query to fit the GPU, and a replayed graph starts it when the stream's
-// previous kernel has ended; should another stream hold SMs at that moment, the limit of the polls ends the launch with
-// code 3002 or 3003 in the device error word instead of waiting for ever.
-
-cudaError_t launch_persistent(const void* kern, dim3 grid, dim3 block, void** args, size_t smem, cudaStream_t stream) {
-  cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
-  if (cudaStreamIsCapturing(stream, &cs) != cudaSuccess) {
-    cudaGetLastError();
-    cs = cudaStreamCaptureStatusNone;
-  }
-  if (cs == cudaStreamCaptureStatusNone) return cudaLaunchCooperativeKernel(kern, grid, block, args, smem, stream);
-  return cudaLaunchKernel(kern, grid, block, args, smem, stream);
-}
+// The blocks of the sequence kernels wait for one another's results (bounded), which needs every block resident at once.
+// They are launched cooperatively, inside a stream capture too: the graph's kernel node keeps the attribute, so that two
+// replays on two streams, or a replay beside other work, never hold half of the SMs each until the polls run out.
 
 // Units and batch columns of a CTA of the sequence kernels, by the smallest modelled time of a step (us): the FMAs of the
 // CTA's chunks at 60 % of the FMA rate (40 % for the narrow tiles), 0.8 per chunk (loads, reduction, gates), 1.3 for the
@@ -563,7 +550,7 @@ int32_t launch_fwd_seq(fb_ctx* ctx, cudaStream_t stream, const float* Wh, const 
   void* args[] = {(void*)&Wh, (void*)&gx, (void*)&h0, (void*)&c0, (void*)&out, (void*)&cache, (void*)&cst, (void*)&cached, (void*)&hT,
                   (void*)&cT, (void*)&H, (void*)&B, (void*)&T, (void*)&nbg, (void*)&dev_err};
   FB_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)p.smem));
-  FB_CUDA(launch_persistent(kern, dim3((unsigned)p.grid), dim3(SQ_THREADS), args, p.smem, stream));
+  FB_CUDA(cudaLaunchCooperativeKernel(kern, dim3((unsigned)p.grid), dim3(SQ_THREADS), args, p.smem, stream));
   FB_LAUNCH_CHECK();
   return FB_OK;
 }
@@ -581,7 +568,7 @@ int32_t launch_bwd_seq(fb_ctx* ctx, cudaStream_t stream, const float* Wh, const 
   void* args[] = {(void*)&Wh, (void*)&keep, (void*)&cst, (void*)&s0, (void*)&hout, (void*)&dout, (void*)&dhT, (void*)&dcT, (void*)&dg,
                   (void*)&dgx, (void*)&H, (void*)&B, (void*)&T, (void*)&nbg, (void*)&dev_err};
   FB_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)p.smem));
-  FB_CUDA(launch_persistent(kern, dim3((unsigned)p.grid), dim3(SQ_THREADS), args, p.smem, stream));
+  FB_CUDA(cudaLaunchCooperativeKernel(kern, dim3((unsigned)p.grid), dim3(SQ_THREADS), args, p.smem, stream));
   FB_LAUNCH_CHECK();
   return FB_OK;
 }

@@ -463,8 +463,7 @@ class GraphedGradient:
 
     `f(model)` must close over device arrays that are updated in place between calls.  `graph()` replays the captured
     launch sequence and returns the loss array (device scalar) and the gradient tree, whose arrays are the same
-    buffers on every call.  BatchNorm running statistics advance on every replay, as they would in eager calls.
-    (Recurrent layers run one launch per time step inside a captured step: a cooperative launch cannot be recorded.)"""
+    buffers on every call.  BatchNorm running statistics advance on every replay, as they would in eager calls."""
 
     def __init__(self, f, model):
         side = torch.cuda.Stream()

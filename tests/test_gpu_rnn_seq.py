@@ -104,3 +104,52 @@ def test_long_sequences_with_initial_state(cell, I, H, T, B):
     close(F.cpu(c["Wh"]), grads[1], name="dWh", **tol)
     close(F.cpu(c["bias" if cell == "lstm" else "b"]), grads[2], name="db", **tol)
     assert F.context().device_error() == 0
+
+
+@pytest.mark.parametrize("cell,I,H,T,B", [("lstm", 64, 512, 24, 64), ("gru", 17, 203, 40, 90)])
+def test_captured_sequences_replay_like_eager_calls(cell, I, H, T, B):
+    """Forward and backward pass recorded into graphs and replayed on two streams at once (each wants more than half of the
+    SMs): bit for bit the eager results."""
+    import torch
+
+    import fluxb200 as F
+    from fluxb200 import lib
+    ctx, sets = F.context(), []
+    for i in range(2):
+        _, (Wi, Wh, b, x), _ = _rnn(cell, I, H, T + i, B)
+        arrays = [F.gpu(v) for v in (Wi, Wh, b, x)]
+        steps = T + i
+        cache = torch.empty(getattr(lib.raw(), f"fb_{cell}_cache_bytes")(I, H, steps, B) // 4, device="cuda")
+        out, dout = F.empty((H, steps, B)), F.gpu(np.random.default_rng(i).normal(size=(H, steps, B)).astype(np.float32))
+        grads = [F.empty(Wi.shape), F.empty(Wh.shape), F.empty(x.shape)]
+
+        def run(arrays=arrays, cache=cache, out=out, dout=dout, grads=grads, steps=steps):
+            Wi, Wh, b, x = (v.ptr for v in arrays)
+            none, dims = (None,) * 2, (I, H, steps, B)
+            if cell == "lstm":
+                lib.call("fb_lstm_fwd", ctx.handle, ctx.stream, Wi, Wh, b, x, *none, out.ptr, *none, cache.data_ptr(), *dims)
+                lib.call("fb_lstm_bwd", ctx.handle, ctx.stream, Wi, Wh, x, *none, out.ptr, cache.data_ptr(), dout.ptr, *none, grads[0].ptr,
+                         grads[1].ptr, None, grads[2].ptr, *dims)
+            else:
+                lib.call("fb_gru_fwd", ctx.handle, ctx.stream, Wi, Wh, b, x, None, out.ptr, None, cache.data_ptr(), *dims)
+                lib.call("fb_gru_bwd", ctx.handle, ctx.stream, Wi, Wh, x, None, out.ptr, cache.data_ptr(), dout.ptr, None, grads[0].ptr,
+                         grads[1].ptr, None, grads[2].ptr, *dims)
+        run()
+        eager = [v.t.clone() for v in [out] + grads]
+        torch.cuda.synchronize()
+        graph = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(graph):
+            run()
+        for v in [out] + grads:
+            v.t.zero_()
+        sets.append((graph, [out] + grads, eager, arrays, cache, dout))
+    streams = [torch.cuda.Stream() for _ in sets]
+    torch.cuda.synchronize()
+    for _ in range(5):
+        for (graph, *_), st in zip(sets, streams):
+            with torch.cuda.stream(st):
+                graph.replay()
+    torch.cuda.synchronize()
+    for _, results, eager, *_ in sets:
+        assert all(torch.equal(a.t, b) for a, b in zip(results, eager))
+    assert ctx.device_error() == 0
