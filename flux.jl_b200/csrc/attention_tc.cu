@@ -56,16 +56,22 @@ __device__ __forceinline__ void tc_st_32x32b_x16(uint32_t taddr, const uint32_t*
 }
 __device__ __forceinline__ void tc_wait_st() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
 
+// Shared-memory descriptors travel as their low word (start address / 16 in its 14 low bits, leading offset above), to which a
+// step's offset is added, and a high word that all steps share.  A tile ends below 228 KB, so that the sum never leaves the
+// 14 bits.  (As 64-bit sums for A and B under a run-time step count one form of the product below gave wrong low-order terms;
+// where the compiler went wrong there is not known, so no form adds to 64 bits.)
+//
 // D[tmem] (+)= A[tmem] * B[smem]: the A tile (128 rows x 16 bf16 values) sits in 8 consecutive TMEM columns, two values each
-__device__ __forceinline__ void tc_mma_bf16_ta(uint32_t d_tmem, uint32_t a_tmem, uint64_t b_desc, uint32_t idesc, uint32_t accumulate) {
+__device__ __forceinline__ void tc_mma_bf16_ta(uint32_t d_tmem, uint32_t a_tmem, uint32_t b_lo, uint32_t hi, uint32_t idesc, uint32_t accumulate) {
   asm volatile(
-      "{\n\t.reg .pred p;\n\t"
+      "{\n\t.reg .pred p;\n\t.reg .b64 db;\n\t"
       "setp.ne.b32 p, %4, 0;\n\t"
-      "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, {%5, %6, %7, %8}, p;\n\t}"
-      ::"r"(d_tmem), "r"(a_tmem), "l"(b_desc), "r"(idesc), "r"(accumulate), "r"(0u), "r"(0u), "r"(0u), "r"(0u)
+      "mov.b64 db, {%2, %9};\n\t"
+      "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], db, %3, {%5, %6, %7, %8}, p;\n\t}"
+      ::"r"(d_tmem), "r"(a_tmem), "r"(b_lo), "r"(idesc), "r"(accumulate), "r"(0u), "r"(0u), "r"(0u), "r"(0u), "r"(hi)
       : "memory");
 }
-// the same with A from shared memory; both descriptors by their low words (address, leading offset), `hi` above both
+// the same with A from shared memory
 __device__ __forceinline__ void tc_mma_bf16_sa(uint32_t d_tmem, uint32_t a_lo, uint32_t b_lo, uint32_t hi, uint32_t idesc, uint32_t accumulate) {
   asm volatile(
       "{\n\t.reg .pred p;\n\t.reg .b64 da, db;\n\t"
@@ -203,14 +209,14 @@ __device__ __forceinline__ uint64_t desc_mn(uint32_t saddr) { return make_smem_d
 template <int NP>
 __device__ __forceinline__ void mma_rows_t(uint32_t d, uint32_t a_tmem, uint32_t b_smem, int nks) {
   const uint64_t b0 = desc_k(b_smem);
-  const uint32_t idesc = idesc_bf16(KT, false);
+  const uint32_t idesc = idesc_bf16(KT, false), hi = (uint32_t)(b0 >> 32);
   using P = Prod<NP, NP>;
 #pragma unroll
   for (int i = 0; i < P::N; ++i)
 #pragma unroll
     for (int ks = 0; ks < 4; ++ks)
       if (ks < nks)
-        tc_mma_bf16_ta(d, a_tmem + (uint32_t)(32 * P::a(i) + 8 * ks), b0 + (uint64_t)((P::b(i) * TILE + ks * 32) >> 4), idesc,
+        tc_mma_bf16_ta(d, a_tmem + (uint32_t)(32 * P::a(i) + 8 * ks), (uint32_t)b0 + (uint32_t)((P::b(i) * TILE + ks * 32) >> 4), hi, idesc,
                        (i > 0 || ks > 0) ? 1u : 0u);
 }
 // the same with A in shared memory: planes of 128 rows, 2 * TILE apart, all four steps (head sizes are zero-padded)
@@ -232,7 +238,7 @@ __device__ __forceinline__ void mma_rows_s(uint32_t d, uint32_t a_smem, uint32_t
 template <int NP>
 __device__ __forceinline__ void mma_planes(uint32_t d, uint32_t t01, uint32_t t2, uint32_t hstep2, uint32_t b_smem, int n, bool accumulate) {
   const uint64_t b0 = desc_mn(b_smem);
-  const uint32_t idesc = idesc_bf16(n, true);
+  const uint32_t idesc = idesc_bf16(n, true), hi = (uint32_t)(b0 >> 32);
   using P = Prod<3, NP>;
 #pragma unroll
   for (int i = 0; i < P::N; ++i)
@@ -240,7 +246,7 @@ __device__ __forceinline__ void mma_planes(uint32_t d, uint32_t t01, uint32_t t2
     for (int ks = 0; ks < 4; ++ks) {
       const uint32_t hf = (uint32_t)(ks >> 1), in = (uint32_t)(8 * (ks & 1));
       const uint32_t a = P::a(i) == 2 ? t2 + hstep2 * hf + in : t01 + 32u * hf + 16u * (uint32_t)P::a(i) + in;
-      tc_mma_bf16_ta(d, a, b0 + (uint64_t)((P::b(i) * TILE + ks * 2048) >> 4), idesc, (accumulate || i > 0 || ks > 0) ? 1u : 0u);
+      tc_mma_bf16_ta(d, a, (uint32_t)b0 + (uint32_t)((P::b(i) * TILE + ks * 2048) >> 4), hi, idesc, (accumulate || i > 0 || ks > 0) ? 1u : 0u);
     }
 }
 

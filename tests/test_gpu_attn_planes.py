@@ -89,6 +89,34 @@ def test_attention_bf16(d, heads, lq, lk, causal):
     assert float((a.sum(-1) - 1).abs().max()) < 1e-4
 
 
+@pytest.mark.parametrize("d", [8, 16, 24, 32, 40, 48, 56, 64])
+@pytest.mark.parametrize("causal", [0, 1])
+def test_every_plane_product_is_there(d, causal):
+    """Every number of 16-feature steps, one to four key blocks.  The smallest plane products lie near 2^-16 of the whole: one
+    that were missing or taken from the wrong place would show as 5e-6 and more.  Forward: 2^-24 for the cut and a few
+    roundings to nearest, 5e-7.  Backward at head size 64: 24 truncating adds of 2^-24 a block, 3e-6 for two blocks."""
+    import fluxb200 as F
+    from fluxb200 import lib
+    g = torch.Generator(device="cuda")
+    g.manual_seed(d)
+    heads, batch = 3, 2
+    ctx = F.context()
+    for lq, lk in ((128, 64), (200, 120), (64, 250)):
+        q, k, v, do = (torch.randn(batch, n, heads * d, device="cuda", generator=g) for n in (lq, lk, lk, lq))
+        o, dq, dk, dv = (torch.empty_like(t) for t in (q, q, k, v))
+        lse = torch.empty(batch * heads * lq, device="cuda")
+        dims = (heads * d, heads * d, lq, lk, batch, heads, causal)
+        p = [t.data_ptr() for t in (q, k, v)]
+        lib.call("fb_attn_fwd", ctx.handle, ctx.stream, *p, None, o.data_ptr(), lse.data_ptr(), *dims)
+        ref = _reference(q, k, v, do, d, d, heads, causal)
+        assert _err(o, ref[0]) < 5e-7, _err(o, ref[0])
+        if d == 64 and lk <= 128 and lq <= 128:
+            lib.call("fb_attn_bwd", ctx.handle, ctx.stream, *p, None, o.data_ptr(), lse.data_ptr(), do.data_ptr(), dq.data_ptr(), dk.data_ptr(),
+                     dv.data_ptr(), *dims)
+            for name, got, want in zip(("dq", "dk", "dv"), (dq, dk, dv), ref[1:]):
+                assert _err(got, want) < 3e-6, (name, _err(got, want))
+
+
 @pytest.mark.parametrize("lq,lk,causal", [(512, 512, 1), (130, 700, 0)])
 def test_backward_of_unaligned_arrays_keeps_float32_sums(lq, lk, causal):
     """Arrays 4 bytes past a 16-byte boundary are the FMA kernels' in the backward pass: two chained sums of at most 700 terms
