@@ -649,10 +649,13 @@ MHA_DTYPES = ("f32", "bf16")
 CASES = """gemm_fwd    Dense 4096=>4096 forward at --batch (3xTF32 tcgen05 GEMM, K-major x MN-major)
 gemm_dw     the dW GEMM of the same layer (MN-major x MN-major, K = batch)
 gemm_dx     the dX GEMM of the same layer (K-major x K-major)
+gemm_split  1024 x 1024 x 16384, Float32: 64 tiles whose K range two CTAs of a cluster share
+gemm_fma    2049 x 2047 x 2045, Float32: rows off the 16-byte boundary, FMA kernel
 gemm_bf16_fwd / gemm_bf16_dw / gemm_bf16_dx   the same three products with BFloat16 storage (tcgen05 kind::f16)
 layernorm   LayerNorm(4096) forward + backward on 4096 x 8192
 batchnorm   BatchNorm(256, relu) training forward + backward on 32 x 32 x 256 x 128
 adam        Adam step over 32 Mi parameters in 4 leaves
+adam_bf16   the same for bf16 parameters with Float32 masters
 attention   causal attention forward + backward, E = 1024, 16 heads, S = 1024, B = 2
 lstm        LSTM(512=>512) forward + backward, T = 32, B = 64
 gru         GRU(512=>512) forward + backward, T = 32, B = 64
@@ -688,6 +691,11 @@ def run_case(args):
         else:
             fn = lambda: call("fb_gemm_f32", 1, 0, d, n, d, P(W), d, P(dy), d, P(dx), d, 0, 0)       # dx = W' * dy
         work = (2.0 * n * d * d, "TFLOP/s")
+    elif case in ("gemm_split", "gemm_fma"):
+        m, n, k = (1024, 1024, 16384) if case == "gemm_split" else (2049, 2047, 2045)
+        A, B, out = rn(m * k), rn(n * k), em(m * n)
+        fn = lambda: call("fb_gemm_f32", 0, 1, m, n, k, P(A), m, P(B), n, P(out), m, 0, 0)
+        work = (2.0 * m * n * k, "TFLOP/s")
     elif case in ("gemm_bf16_fwd", "gemm_bf16_dw", "gemm_bf16_dx"):
         n, d = args.batch, 4096
         bfr = lambda k: rn(k).to(torch.bfloat16)
@@ -729,6 +737,15 @@ def run_case(args):
         counts = (C.c_int64 * k)(*([cnt] * k))
         fn = lambda: call("fb_adam_step", k, tabs[0], tabs[1], tabs[2], tabs[3], counts, 1e-3, 0.9, 0.999, 1e-8, 0.9, 0.999, 1.0)
         work = (7.0 * k * cnt * 4, "GB/s")
+    elif case == "adam_bf16":
+        k, cnt = 4, 8 << 20
+        w, m, v = ([rn(cnt) for _ in range(k)] for _ in range(3))
+        p, gr = ([rn(cnt).to(torch.bfloat16) for _ in range(k)] for _ in range(2))
+        arr = C.c_void_p * k
+        tabs = [arr(*[t.data_ptr() for t in ts]) for ts in (p, w, gr, m, v)]
+        counts = (C.c_int64 * k)(*([cnt] * k))
+        fn = lambda: call("fb_adam_step_bf16", k, *tabs, counts, 1e-3, 0.9, 0.999, 1e-8, 0.9, 0.999, 1.0)
+        work = (28.0 * k * cnt, "GB/s")
     elif case == "attention":
         E, S, B, H = 1024, args.seq, 2, 16
         q, k_, v_, do = rn(E * S * B), rn(E * S * B), rn(E * S * B), rn(E * S * B)
