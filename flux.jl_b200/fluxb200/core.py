@@ -77,6 +77,7 @@ class B200Array:
     """
 
     __slots__ = ("t", "size", "_node", "__weakref__")
+    backed = True   # (a cotangent whose value is known has no memory before somebody reads it)
 
     def __init__(self, t: torch.Tensor, size):
         self.t = t
@@ -236,29 +237,21 @@ class Tape:
         cls.tracked = set()
 
 
-def accumulate(grads: dict, owned: set, arr: B200Array, g: B200Array, fresh: bool):
+def accumulate(grads: dict, arr: B200Array, g: B200Array):
     """grads[id(arr)] += g (tangent accumulation, Zygote's `accum`).
 
-    Only memory that belongs to this one gradient is added to in place: `owned` holds the keys for which that is so.
-    `fresh` says that g's memory was handed over to `arr` alone; a pullback may also pass its cotangent's memory on
-    (reshape, add), which other gradients then share, so that the sum needs memory of its own."""
+    A pullback may pass its cotangent's memory on (reshape, add): several of the sweep's gradients then share it, and the sum
+    needs memory of its own.  `grads` holds every gradient of the sweep, so one look at it says whether that is so."""
     k = id(arr)
     if k not in grads:
         grads[k] = g
-        if fresh:
-            owned.add(k)
+        return
+    ctx, acc = context(), grads[k]
+    ptr = acc.t.data_ptr()
+    if any(key != k and other.backed and other.t.data_ptr() == ptr for key, other in grads.items()):
+        acc = grads[k] = _wrap(acc.t.clone(), acc.size)
+    if acc.t.dtype == torch.bfloat16:
+        g = to_bf16(g)
+        lib.call("fb_axpy_bf16", ctx.handle, ctx.stream, 1.0, g.ptr, acc.ptr, g.numel())
     else:
-        own_gradient(grads, owned, k)
-        ctx, acc = context(), grads[k]
-        if acc.t.dtype == torch.bfloat16:
-            g = to_bf16(g)
-            lib.call("fb_axpy_bf16", ctx.handle, ctx.stream, 1.0, g.ptr, acc.ptr, g.numel())
-        else:
-            lib.call("fb_axpy", ctx.handle, ctx.stream, 1.0, to_f32(g).ptr, acc.ptr, g.numel())
-
-
-def own_gradient(grads: dict, owned: set, k: int):
-    """Gives grads[k] memory that no other gradient shares."""
-    if k not in owned:
-        grads[k] = _wrap(grads[k].t.clone(), grads[k].size)
-        owned.add(k)
+        lib.call("fb_axpy", ctx.handle, ctx.stream, 1.0, to_f32(g).ptr, acc.ptr, g.numel())

@@ -14,7 +14,7 @@ import numpy as np
 import torch
 
 from . import lib
-from .core import B200Array, Tape, accumulate, context, empty, gpu, own_gradient, to_bf16, to_f32, zeros
+from .core import B200Array, Tape, accumulate, context, empty, gpu, to_bf16, to_f32, zeros
 from .layers import DimensionMismatch, Layer, trainables
 
 
@@ -182,9 +182,7 @@ def _withgradient_device(f, model, grad_sink=None):
                     if a is not None and id(a) in pid:
                         counts[id(a)] = counts.get(id(a), 0) + 1
             grad_sink.expect_uses(counts)
-        one = _One(loss.t.device)
-        grads: dict = {id(loss): one}
-        owned: set = set()
+        grads: dict = {id(loss): _One(loss.t.device)}
         # gradient averaging runs beside the reverse sweep: leave it the SMs it needs
         reserve = int(getattr(grad_sink, "reserved_sms", 0) or 0)
         if reserve:
@@ -193,17 +191,20 @@ def _withgradient_device(f, model, grad_sink=None):
             gs = [grads.get(id(o)) for o in outs]
             if all(g is None for g in gs):
                 continue
-            res = [(arr, g) for arr, g in pullback(gs) if arr is not None and g is not None]
-            # memory that the pullback passed on from its cotangents, or gave to two inputs, is shared
-            given = [g.t.data_ptr() for g in gs if g is not None and not (g is one and one.untouched)]
-            ptrs = [None if g is one else g.t.data_ptr() for _, g in res]
-            for (arr, g), ptr in zip(res, ptrs):
-                accumulate(grads, owned, arr, g, ptr is not None and ptr not in given and ptrs.count(ptr) == 1)
+            for arr, g in pullback(gs):
+                if arr is None or g is None:
+                    continue
+                accumulate(grads, arr, g)
                 if grad_sink is not None:
                     grad_sink.ready(arr)
-        for p in params:   # a gradient that is handed out is its receiver's alone
-            if id(p) in grads:
-                own_gradient(grads, owned, id(p))
+        handed: set = set()
+        for k in {id(p): None for p in params}:   # what is handed out shares no memory
+            g = grads.get(k)
+            if g is not None:
+                ptr = g.t.data_ptr()
+                if ptr in handed or isinstance(g, _One):
+                    grads[k] = B200Array(g.t.clone(), g.size)
+                handed.add(ptr)
         tree = _grad_tree(model, grads)
     finally:
         if int(getattr(grad_sink, "reserved_sms", 0) or 0):
@@ -245,8 +246,8 @@ class _One(B200Array):
         self._is_one, self._device, self._value = True, device, None
 
     @property
-    def untouched(self) -> bool:
-        return self._value is None
+    def backed(self) -> bool:
+        return self._value is not None
 
     @property
     def t(self):
