@@ -631,7 +631,7 @@ def small_config_lines(config, steps, warmup):
                 8, ms, clocks,
                 {"bound": "tensor", "achieved": flops / ms / 1e9, "peak": peak, "unit": "TFLOP/s", "frac": flops / ms / 1e9 / peak, "traffic": None,
                  "flops_per_step": flops,
-                 "note": ("projections and the attention core (forward, dQ, dK/dV) on tcgen05 with 3xTF32; softmax and dS on TMEM read-back; "
+                 "note": ("projections on tcgen05 with 3xTF32, the attention core (forward, dQ, dK/dV) on three bf16 planes per operand; softmax and dS on TMEM read-back; "
                           if dtype == "f32" else "the opt-in bf16 path (fluxb200.bf16); ") + how},
                 ms_e2e, h2d, (1 * (512 / 2048) ** 2 * 1.0) / cpu,
                 "1 of 8 samples at seq 512 (1/16 of a sample's attention work, 1/4 of its projections), Float32, 1 run", dtype=dtype)
@@ -649,7 +649,7 @@ MHA_DTYPES = ("f32", "bf16")
 CASES = """gemm_fwd    Dense 4096=>4096 forward at --batch (3xTF32 tcgen05 GEMM, K-major x MN-major)
 gemm_dw     the dW GEMM of the same layer (MN-major x MN-major, K = batch)
 gemm_dx     the dX GEMM of the same layer (K-major x K-major)
-gemm_split  1024 x 1024 x 16384, Float32: 64 tiles whose K range two CTAs of a cluster share
+gemm_split  1024 x 1024 x 16384, Float32: 32 tiles whose K range the four CTAs of a cluster share
 gemm_fma    2049 x 2047 x 2045, Float32: rows off the 16-byte boundary, FMA kernel
 gemm_bf16_fwd / gemm_bf16_dw / gemm_bf16_dx   the same three products with BFloat16 storage (tcgen05 kind::f16)
 layernorm   LayerNorm(4096) forward + backward on 4096 x 8192

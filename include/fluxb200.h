@@ -15,10 +15,12 @@
  *  - arrays are dense and column-major exactly as Julia stores them: a Julia `W[out,in]` is read by
  *    the kernels as row-major `[in][out]`, `x[in,N]` as `[N][in]`, WHCN images as `[N][C][H*W]`;
  *  - `stream` is a cudaStream_t passed as void* (NULL = the default stream).  Calls enqueue work
- *    and return; only fb_sync, fb_memcpy_d2h and the fb_comm_* bootstrap calls block;
+ *    and return; only fb_sync, fb_memcpy_d2h, fb_device_error, fb_read_scalar and the fb_comm_* bootstrap calls
+ *    block;
+ *  - a context is used by one thread at a time;
  *  - the caller owns all tensors, including the saved-for-backward buffers (statistics, gates,
  *    log-sum-exp); the library owns a per-context scratch arena that grows on demand and a memory pool that
- *    single calls take their operand images from in their stream's order (up to 1 GiB stays with the context).
+ *    single calls take operand images and GEMM sums from in their stream's order (up to 1 GiB stays with it).
  *    Pool memory is safe on any number of streams and in captured graphs.  The scratch arena (partial sums of
  *    losses, bias gradients and normalisation layers, projections of recurrent layers) is not: calls of one
  *    context that overlap on several streams, or with a replayed graph, need one context per stream.
@@ -105,7 +107,8 @@ int32_t fb_device_error(fb_ctx* ctx, void* stream, int32_t* out_host);
 
 /* Reads one device Float32 (a loss) together with the device error word: a one-thread kernel on `stream` stores both in
  * a host page that this call watches, which is several us quicker than a copy and a stream synchronisation each.
- * Returns when the stream has reached this point.  The error word is left as it is (fb_device_error clears it).  Not
+ * Returns when the stream has reached this point (the calling thread spins until then).  The page belongs to the
+ * context: two threads need a context each.  The error word is left as it is (fb_device_error clears it).  Not
  * for a stream that is being captured.  Replaces the implicit device-to-host read of a loss (src/train.jl:377). */
 int32_t fb_read_scalar(fb_ctx* ctx, void* stream, const float* x, float* value_host, int32_t* error_host);
 

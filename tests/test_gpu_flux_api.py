@@ -519,7 +519,7 @@ def test_read_scalar_sees_the_stream_and_the_error_word():
     lib.call("fb_selftest_bounded_wait", ctx.handle, ctx.stream, 16)
     assert ctx.read_scalar(x)[1] == 9001 and ctx.read_scalar(x)[1] == 9001
     assert ctx.device_error() == 9001 and ctx.read_scalar(x)[1] == 0
-    # the constant cotangent of the loss is shared and must not change when a loss receives a second contribution
+    # a loss that receives a second contribution, twice over
     d = F.Dense(np.ones((1, 1), np.float32), False)
     xg = F.gpu(np.full((1, 1), 3.0, np.float32))
 
