@@ -69,6 +69,37 @@ def test_truncating_sums_are_no_longer_than_an_even_cut(ctx, m, n, k, even):
         assert err < 8.5e-9 * even, err
 
 
+# tiles of several accumulation segments that meet in the workspace: pairs, one-CTA tiles, tiles shared by a cluster
+@pytest.mark.parametrize("out_dim,in_dim,n", [(512, 1216, 5184), (10240, 3000, 200), (264, 9000, 520)])
+@pytest.mark.parametrize("act", ["identity", "gelu_tanh"])
+def test_epilogues_behind_parked_segments(ctx, out_dim, in_dim, n, act):
+    from fluxb200 import lib
+    g = torch.Generator(device="cuda").manual_seed(n)
+    W = torch.randn(in_dim, out_dim, generator=g, device="cuda") / in_dim ** 0.5
+    b, x = torch.randn(out_dim, generator=g, device="cuda"), torch.randn(n, in_dim, generator=g, device="cuda")
+    y, z = torch.empty(n, out_dim, device="cuda"), torch.empty(n, out_dim, device="cuda")
+    lib.call("fb_dense_fwd", ctx.handle, ctx.stream, lib.ACT[act], 0, W.data_ptr(), b.data_ptr(), x.data_ptr(), y.data_ptr(), z.data_ptr(),
+             out_dim, in_dim, n)
+    zr = x.double() @ W.double() + b.double()
+    yr = zr if act == "identity" else torch.nn.functional.gelu(zr, approximate="tanh")
+    assert ((z.double() - zr).norm() / zr.norm()) < 3e-5 and ((y.double() - yr).norm() / yr.norm()) < 3e-5
+    before = y.clone()
+    lib.call("fb_gemm_f32", ctx.handle, ctx.stream, 0, 0, out_dim, n, in_dim, W.data_ptr(), out_dim, x.data_ptr(), in_dim, y.data_ptr(), out_dim, 1, 0)
+    ref = before.double() + zr - b.double()
+    assert ((y.double() - ref).norm() / ref.norm()) < 3e-5 and ctx.device_error() == 0
+
+
+def test_the_tensor_core_kernel_refuses_unaligned_results(ctx):
+    from fluxb200 import lib
+    A, B, _ = _operands(0, 0, 512, 512, 512, 0, torch.float32)
+    out = torch.zeros(512, 513, device="cuda")
+    for precision in ("3xtf32", "tf32", "3xtf32_pair"):
+        with pytest.raises(lib.FluxB200Error):
+            lib.call("fb_gemm_f32", ctx.handle, ctx.stream, 0, 0, 512, 512, 512, A.data_ptr(), 512, B.data_ptr(), 512, out.data_ptr(), 513, 0,
+                     lib.PREC[precision])
+    assert not bool(out.any())
+
+
 def test_reserved_sms_keep_the_k_split(ctx):
     """With SMs left to communication kernels no clusters are used; 16 tiles of 1024 k-blocks still spread over the others
     (a whole tile each takes six times as long), and the results are those of a product."""
