@@ -237,19 +237,22 @@ class Tape:
         cls.tracked = set()
 
 
-def accumulate(grads: dict, arr: B200Array, g: B200Array):
+def accumulate(grads: dict, owned: set, arr: B200Array, g: B200Array):
     """grads[id(arr)] += g (tangent accumulation, Zygote's `accum`).
 
     A pullback may pass its cotangent's memory on (reshape, add): several of the sweep's gradients then share it, and the sum
-    needs memory of its own.  `grads` holds every gradient of the sweep, so one look at it says whether that is so."""
+    needs memory of its own.  `grads` holds every gradient of the sweep, so one look at it says whether that is so; `owned`
+    remembers the keys that have been looked at (an array's gradient is passed on only after its last contribution)."""
     k = id(arr)
     if k not in grads:
         grads[k] = g
         return
     ctx, acc = context(), grads[k]
-    ptr = acc.t.data_ptr()
-    if any(key != k and other.backed and other.t.data_ptr() == ptr for key, other in grads.items()):
-        acc = grads[k] = _wrap(acc.t.clone(), acc.size)
+    if k not in owned:
+        owned.add(k)
+        ptr = acc.t.data_ptr()
+        if any(key != k and other.backed and other.t.data_ptr() == ptr for key, other in grads.items()):
+            acc = grads[k] = _wrap(acc.t.clone(), acc.size)
     if acc.t.dtype == torch.bfloat16:
         g = to_bf16(g)
         lib.call("fb_axpy_bf16", ctx.handle, ctx.stream, 1.0, g.ptr, acc.ptr, g.numel())

@@ -183,6 +183,7 @@ def _withgradient_device(f, model, grad_sink=None):
                         counts[id(a)] = counts.get(id(a), 0) + 1
             grad_sink.expect_uses(counts)
         grads: dict = {id(loss): _One(loss.t.device)}
+        owned: set = set()
         # gradient averaging runs beside the reverse sweep: leave it the SMs it needs
         reserve = int(getattr(grad_sink, "reserved_sms", 0) or 0)
         if reserve:
@@ -194,7 +195,7 @@ def _withgradient_device(f, model, grad_sink=None):
             for arr, g in pullback(gs):
                 if arr is None or g is None:
                     continue
-                accumulate(grads, arr, g)
+                accumulate(grads, owned, arr, g)
                 if grad_sink is not None:
                     grad_sink.ready(arr)
         handed: set = set()
