@@ -50,7 +50,7 @@ constexpr int SEG_KB = 128;          // the longest accumulation segment in k-bl
 
 // Work schedule of one launch.  Tiles [0, dp_tiles) are taken whole: CTA (pair) cid of G takes cid, cid + G, ...
 // (n fastest, so the tiles in flight are neighbours and share operand panels in L2).  The remaining tiles - a
-// last wave that would leave most SMs idle - are cut along K into units of UNIT_KB k-blocks; the U units are
+// last wave that would leave most SMs idle (the only one where the plan expects a gain) - are cut along K into units of UNIT_KB k-blocks; the U units are
 // dealt out as G contiguous ranges, so a tile may be computed by several CTAs ("parts").  Each part writes its
 // partial sums to a workspace slot; the part that finishes last (an atomic ticket per tile, no waiting) adds the
 // slots in k order and applies the epilogue.
@@ -770,6 +770,7 @@ int32_t launch_layout(fb_ctx* ctx, cudaStream_t stream, const fb_gemm_args& a, c
 // all 256 B columns from shared memory), two-CTA 256 x 256 tiles 215-232 TFLOP/s (each CTA reads only its 128 B
 // columns).  At 1024 x 4096 x 4096 (one wave of 64 two-CTA tiles on 74 SM pairs) both, and cutting every tile along
 // K over all pairs, take 0.204-0.207 ms: what is left there is the unoverlapped prologue and epilogue of a single tile.
+//
 // How a 3xTF32 product is cut.  Shapes: 128 x 128 (0) and 128 x 256 (1) tiles of one CTA, 256 x 256 tiles of a CTA pair
 // (2); ksplit CTAs of one cluster share a tile's K range where whole tiles would leave SMs idle.  The choice is
 // the smallest of the modelled times; its constants (us) are fitted to measurements on B200: a k-block of 16 costs
