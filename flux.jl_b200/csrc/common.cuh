@@ -248,6 +248,18 @@ bool fb_gemm_tc_supported(const fb_gemm_args& a);
 // the time (us) that the kernel's own plan expects
 double fb_gemm_tc_time(fb_ctx* ctx, const fb_gemm_args& a);
 double fb_gemm_simt_time(const fb_ctx* ctx, const fb_gemm_args& a);
+// planes.cu: both operands of a product as images of two half-precision planes
+struct fb_planes {
+  uint16_t* img[2];
+  int32_t* exps[2];      // per row, padded to a multiple of 128: the exponent that undoes its scale
+  int64_t rows[2];       // 128-byte rows of an operand's images
+};
+size_t fb_planes_bytes(const fb_gemm_args& a);
+// gemm_planes.cu: the product of such images for arguments that fb_gemm_tc_supported takes; FB_ERR_UNSUPPORTED (without an error
+// message) when there is no memory for them.  The time is what the kernel's own plan expects, as above.
+int32_t fb_gemm_planes_launch(fb_ctx* ctx, cudaStream_t stream, const fb_gemm_args& a);
+double fb_gemm_planes_time(const fb_ctx* ctx, const fb_gemm_args& a);
+int32_t fb_planes_split(cudaStream_t stream, const fb_gemm_args& a, void* mem, fb_planes* out);
 int32_t fb_gemm_dispatch(fb_ctx* ctx, cudaStream_t stream, const fb_gemm_args& a, int precision);
 void fb_gemm_query_clusters(fb_ctx* ctx);
 // attention_tc.cu: tensor-core attention; FB_ERR_UNSUPPORTED when the call is not taken

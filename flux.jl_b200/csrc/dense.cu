@@ -17,7 +17,7 @@ static int default_precision_override() {
     const char* e = getenv("FLUXB200_PRECISION");
     if (e != nullptr) {
       if (strcmp(e, "fp32_simt") == 0) cached = FB_PREC_FP32_SIMT;
-      else if (strcmp(e, "3xtf32") == 0) cached = FB_PREC_DEFAULT;
+      else if (strcmp(e, "3xtf32") == 0) cached = FB_PREC_3XTF32;
       else if (strcmp(e, "tf32") == 0) cached = FB_PREC_TF32;
     }
   }
@@ -56,8 +56,16 @@ int32_t fb_gemm_dispatch(fb_ctx* ctx, cudaStream_t stream, const fb_gemm_args& a
       // 3xTF32's errors (2.1e-6 against 5.7e-7, 1.5e-5 against 1.1e-6) and a NaN for every product with an infinite factor.
       const double macs = (double)a.M * (double)a.N * (double)a.K;
       if (macs >= 1.0e8 && a.K >= 32 && a.N >= 32 && a.M > 16 && fb_gemm_tc_supported(a) &&
-          (a.M >= 32 || fb_gemm_tc_time(ctx, a) < fb_gemm_simt_time(ctx, a)))
+          (a.M >= 32 || fb_gemm_tc_time(ctx, a) < fb_gemm_simt_time(ctx, a))) {
+        // Two half-precision planes per operand and products at twice the rate, for a pass over both operands first: where the two
+        // plans expect them to be faster, from about 2e9 multiply-adds on (1024 x 1024 x 1024: 26.6 us as 3xTF32, 29 - 35 as
+        // planes; 2048 x 2048 x 2048: 97 and 76; 8192 x 4096 x 4096: 1043 and 584).
+        if (default_precision_override() != FB_PREC_3XTF32 && fb_gemm_planes_time(ctx, a) < fb_gemm_tc_time(ctx, a)) {
+          const int32_t st = fb_gemm_planes_launch(ctx, stream, a);
+          if (st != FB_ERR_UNSUPPORTED) return st;
+        }
         return fb_gemm_tc_launch(ctx, stream, a, 3);
+      }
       return fb_gemm_simt_launch(ctx, stream, a);
     }
     default:

@@ -1,0 +1,68 @@
+// Work schedule of the Float32 tensor-core GEMM kernels (gemm_tc.cu, gemm_planes.cu).  File-local to the translation unit that
+// includes it.
+#pragma once
+
+namespace {
+
+// Work schedule of one launch.  Tiles [0, dp_tiles) are taken whole: CTA (pair) cid of G takes cid, cid + G, ...
+// (n fastest, so the tiles in flight are neighbours and share operand panels in L2).  The remaining tiles - a
+// last wave that would leave most SMs idle (the only one where the plan expects a gain) - are cut along K into units of
+// UNIT k-blocks; the U units are dealt out as G contiguous ranges, so a tile may be computed by several CTAs ("parts").
+// Each part writes its partial sums to a workspace slot; the part that finishes last (an atomic ticket per tile, no waiting)
+// adds the slots in k order and applies the epilogue.
+struct Sched {
+  int num_tiles, tiles_n, dp_tiles;
+  int nu;            // units per tile
+  int U;             // units in the tail: (num_tiles - dp_tiles) * nu
+  int ksplit;        // CTAs of one cluster that share a tile, each with a part of its K range (1: no split)
+  int seg;           // k-blocks per accumulation segment
+  float* ws;         // [2 * G * ranks] slots of BM x 256 floats
+  int* tickets;      // [G * ranks * 4], zero at the start
+};
+struct Portion {
+  int tile, kb0, kb1;
+  int partial;       // 0: the whole tile, results go to C
+  int tail_tile;     // index of the tile inside the tail (partial only)
+  int trail;         // 1 when this CTA's range began before the tile's first unit (names the slot)
+};
+template <bool SPLIT, int UNIT>   // UNIT: k-blocks of a unit
+struct WorkIter {
+  int w, ta, tb, t0;
+  __device__ WorkIter(const Sched& s, int cid, int G) : w(0) {
+    if (SPLIT) return;
+    ta = t0 = (int)((long long)cid * s.U / G);
+    tb = (int)((long long)(cid + 1) * s.U / G);
+  }
+  __device__ bool next(const Sched& s, int cid, int G, int num_kb, Portion& p) {
+    if (SPLIT) {   // one portion per CTA (pair): part cid % ksplit of tile cid / ksplit
+      if (w++ != 0) return false;
+      const int part = cid % s.ksplit;
+      p.tile = cid / s.ksplit;
+      p.kb0 = (int)((long long)num_kb * part / s.ksplit);
+      p.kb1 = (int)((long long)num_kb * (part + 1) / s.ksplit);
+      p.partial = 0; p.tail_tile = 0; p.trail = 0;
+      return true;
+    }
+    if (w * G + cid < s.dp_tiles) {
+      p.tile = w * G + cid; p.kb0 = 0; p.kb1 = num_kb; p.partial = 0; p.tail_tile = 0; p.trail = 0;
+      ++w;
+      return true;
+    }
+    if (ta < tb) {
+      const int tr = ta / s.nu, ua = ta % s.nu;
+      const int rem = tb - ta;
+      const int ub = (ua + rem < s.nu) ? ua + rem : s.nu;
+      p.tile = s.dp_tiles + tr;
+      p.kb0 = ua * UNIT;
+      p.kb1 = (ub == s.nu) ? num_kb : ub * UNIT;
+      p.partial = (ua == 0 && ub == s.nu) ? 0 : 1;
+      p.tail_tile = tr;
+      p.trail = (t0 < tr * s.nu) ? 1 : 0;
+      ta += ub - ua;
+      return true;
+    }
+    return false;
+  }
+};
+
+}  // namespace

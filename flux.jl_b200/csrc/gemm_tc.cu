@@ -40,75 +40,15 @@
 #include <stdlib.h>
 
 #include "common.cuh"
+#include "gemm_sched.cuh"
 #include "tc_common.cuh"
 
 namespace {
 
 constexpr int BM = 128;
 constexpr int BK = 16;               // floats per k-block (64 bytes)
+constexpr int UNIT_KB = 32;            // k-blocks of a unit of the tail split (gemm_sched.cuh)
 constexpr int SEG_KB = 128;          // the longest accumulation segment in k-blocks (2048 k-values)
-
-// Work schedule of one launch.  Tiles [0, dp_tiles) are taken whole: CTA (pair) cid of G takes cid, cid + G, ...
-// (n fastest, so the tiles in flight are neighbours and share operand panels in L2).  The remaining tiles - a
-// last wave that would leave most SMs idle (the only one where the plan expects a gain) - are cut along K into units of UNIT_KB k-blocks; the U units are
-// dealt out as G contiguous ranges, so a tile may be computed by several CTAs ("parts").  Each part writes its
-// partial sums to a workspace slot; the part that finishes last (an atomic ticket per tile, no waiting) adds the
-// slots in k order and applies the epilogue.
-constexpr int UNIT_KB = 32;
-struct Sched {
-  int num_tiles, tiles_n, dp_tiles;
-  int nu;            // units per tile
-  int U;             // units in the tail: (num_tiles - dp_tiles) * nu
-  int ksplit;        // CTAs of one cluster that share a tile, each with a part of its K range (1: no split)
-  int seg;           // k-blocks per accumulation segment
-  float* ws;         // [2 * G * ranks] slots of BM x 256 floats
-  int* tickets;      // [G * ranks * 4], zero at the start
-};
-struct Portion {
-  int tile, kb0, kb1;
-  int partial;       // 0: the whole tile, results go to C
-  int tail_tile;     // index of the tile inside the tail (partial only)
-  int trail;         // 1 when this CTA's range began before the tile's first unit (names the slot)
-};
-template <bool SPLIT>
-struct WorkIter {
-  int w, ta, tb, t0;
-  __device__ WorkIter(const Sched& s, int cid, int G) : w(0) {
-    if (SPLIT) return;
-    ta = t0 = (int)((long long)cid * s.U / G);
-    tb = (int)((long long)(cid + 1) * s.U / G);
-  }
-  __device__ bool next(const Sched& s, int cid, int G, int num_kb, Portion& p) {
-    if (SPLIT) {   // one portion per CTA (pair): part cid % ksplit of tile cid / ksplit
-      if (w++ != 0) return false;
-      const int part = cid % s.ksplit;
-      p.tile = cid / s.ksplit;
-      p.kb0 = (int)((long long)num_kb * part / s.ksplit);
-      p.kb1 = (int)((long long)num_kb * (part + 1) / s.ksplit);
-      p.partial = 0; p.tail_tile = 0; p.trail = 0;
-      return true;
-    }
-    if (w * G + cid < s.dp_tiles) {
-      p.tile = w * G + cid; p.kb0 = 0; p.kb1 = num_kb; p.partial = 0; p.tail_tile = 0; p.trail = 0;
-      ++w;
-      return true;
-    }
-    if (ta < tb) {
-      const int tr = ta / s.nu, ua = ta % s.nu;
-      const int rem = tb - ta;
-      const int ub = (ua + rem < s.nu) ? ua + rem : s.nu;
-      p.tile = s.dp_tiles + tr;
-      p.kb0 = ua * UNIT_KB;
-      p.kb1 = (ub == s.nu) ? num_kb : ub * UNIT_KB;
-      p.partial = (ua == 0 && ub == s.nu) ? 0 : 1;
-      p.tail_tile = tr;
-      p.trail = (t0 < tr * s.nu) ? 1 : 0;
-      ta += ub - ua;
-      return true;
-    }
-    return false;
-  }
-};
 
 template <int BN, int PASSES, bool PAIR, int SG>
 struct Cfg {
@@ -264,7 +204,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
       int m0 = 0, nb0 = 0;
       int it = 0;   // k-blocks issued so far over all tiles: names the stage and its phase
       bool ok = true;
-      WorkIter<SPLIT> wi(sch, cid, G);
+      WorkIter<SPLIT, UNIT_KB> wi(sch, cid, G);
       Portion p;
       while (ok && wi.next(sch, cid, G, num_kb, p)) {
         m0 = tile_m0(p.tile);
@@ -309,7 +249,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
                              ((uint32_t)(BN >> 3) << 17) | ((uint32_t)((PAIR ? 256 : BM) >> 4) << 24);
       bool ok = true;
       int it = 0, sc = 0;   // k-blocks and accumulation segments issued so far over all tiles
-      WorkIter<SPLIT> wi(sch, cid, G);
+      WorkIter<SPLIT, UNIT_KB> wi(sch, cid, G);
       Portion p;
       while (ok && wi.next(sch, cid, G, num_kb, p))
       for (int kb = p.kb0, kb_in_seg = 0; kb < p.kb1 && ok; ++kb, ++it) {
@@ -375,7 +315,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
     constexpr int RANKS = PAIR ? 2 : 1;
     bool ok = true;
     int sc = 0;                             // segments drained so far over all tiles
-    WorkIter<SPLIT> wi(sch, cid, G);
+    WorkIter<SPLIT, UNIT_KB> wi(sch, cid, G);
     Portion p;
     while (ok && wi.next(sch, cid, G, num_kb, p)) {
       const int n0 = tile_n0(p.tile);
@@ -542,7 +482,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
     bool ok = true;
     int total_kb = 0;   // the stage ring runs on across tiles
     {
-      WorkIter<SPLIT> wi(sch, cid, G);
+      WorkIter<SPLIT, UNIT_KB> wi(sch, cid, G);
       Portion p;
       while (wi.next(sch, cid, G, num_kb, p)) total_kb += p.kb1 - p.kb0;
     }

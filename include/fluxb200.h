@@ -55,7 +55,7 @@ extern "C" {
 #define FB_ACT_GELU_ERF 5
 
 /* matmul precision for Float32 data */
-#define FB_PREC_DEFAULT 0 /* 3xTF32 on the tensor cores when the shape allows, else fp32 FMA */
+#define FB_PREC_DEFAULT 0 /* two half-precision planes per operand or 3xTF32 on the tensor cores when the shape allows, else fp32 FMA */
 #define FB_PREC_FP32_SIMT 1 /* always the fp32 FMA kernel */
 #define FB_PREC_3XTF32 2  /* tcgen05 tensor cores, error-compensated TF32 (fp32-level accuracy) */
 #define FB_PREC_TF32 3    /* tcgen05 tensor cores, single TF32 pass */

@@ -1,0 +1,156 @@
+"""GPU tests of the Float32 products on two half-precision planes per operand, which the default precision takes where their
+plan expects them to be faster than 3xTF32.  Reference: the product in float64.
+
+Bounds: a product of planes is off by at most 2 * 2^-23 + 2^-22 of |a||b| per term (operand rounding, the dropped product of the
+lower planes), which for N(0, 1) operands averages out below 1e-7 of the result's norm; the tensor core truncates while it
+accumulates, 3.5e-9 of the norm per k-value over at most 512 of them: 1.8e-6, and 3e-6 leaves room for the sums' own
+rounding.  3xTF32 is off by 7.3e-9 per k-value over up to 2048: it would not pass at the longer sums here."""
+import ctypes as C
+
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+TOL = 3e-6
+
+
+@pytest.fixture(scope="module")
+def ctx():
+    import fluxb200 as F
+    return F.context(0)
+
+
+def _mat(g, rows, k, mn, pad):
+    """op(X)[rows, k] as float64 and the row-major storage: [rows][k] or, MN-major, [k][rows], `pad` values behind each row."""
+    s = torch.randn((k, rows + pad) if mn else (rows, k + pad), generator=g, device="cuda")
+    return s, (s[:, :rows].T if mn else s[:, :k]).double()
+
+
+def _product(ctx, a, a_mn, b, b_mn, out, m, n, k, accumulate=0):
+    """row-major out[m][n] (the entry point is column-major: its first operand is b)"""
+    from fluxb200 import lib
+    lib.call("fb_gemm_f32", ctx.handle, ctx.stream, 0 if b_mn else 1, 1 if a_mn else 0, n, m, k, C.c_void_p(b.data_ptr()), b.shape[1],
+             C.c_void_p(a.data_ptr()), a.shape[1], C.c_void_p(out.data_ptr()), out.shape[1], accumulate, 0)
+
+
+# pairs: whole waves, a ragged last row and column of tiles, a last wave cut along K; one-CTA tiles, and shared by 2, 4 and 8 CTAs;
+# K that ends inside a k-block and inside its 16-byte pieces, K of more than 8192 (rows no longer held in registers)
+LARGE = [(4312, 2344, 3008, 0), (4100, 2052, 4100, 4), (2500, 1284, 8200, 0), (2052, 2052, 2056, 0), (520, 4100, 8196, 8)]
+FEW = [(1028, 1028, 16388, 0), (200, 544, 12488, 0), (72, 1048, 8960, 0)]     # tiles (planes in the K-major order only)
+
+
+@pytest.mark.parametrize("a_mn,b_mn,m,n,k,pad", [o + s for s in LARGE for o in ((0, 1), (0, 0), (1, 1), (1, 0))] + [(0, 0) + s for s in FEW])
+def test_products_of_planes(ctx, a_mn, b_mn, m, n, k, pad):
+    g = torch.Generator(device="cuda").manual_seed(m + n + k)
+    a, a64 = _mat(g, m, k, a_mn, pad)
+    b, b64 = _mat(g, n, k, b_mn, pad)
+    ref = a64 @ b64.T
+    for accumulate in (0, 1):
+        out = torch.full((m, n + 4), 2.0, device="cuda")
+        _product(ctx, a, a_mn, b, b_mn, out, m, n, k, accumulate)
+        err = (out[:, :n].double() - 2.0 * accumulate - ref).norm() / ref.norm()
+        assert err < TOL, float(err)
+        assert bool((out[:, n:] == 2.0).all()) and ctx.device_error() == 0
+
+
+@pytest.mark.parametrize("out_dim,in_dim,n", [(2344, 3008, 4312), (1032, 4100, 2500), (2052, 2048, 2050)])
+@pytest.mark.parametrize("act", ["identity", "relu", "gelu_tanh", "tanh"])
+def test_epilogues(ctx, out_dim, in_dim, n, act):
+    from fluxb200 import lib
+    g = torch.Generator(device="cuda").manual_seed(n)
+    W = torch.randn(in_dim, out_dim, generator=g, device="cuda") / in_dim ** 0.5
+    b, x = torch.randn(out_dim, generator=g, device="cuda"), torch.randn(n, in_dim, generator=g, device="cuda")
+    zr = x.double() @ W.double() + b.double()
+    yr = {"identity": zr, "relu": zr.relu(), "tanh": zr.tanh(), "gelu_tanh": torch.nn.functional.gelu(zr, approximate="tanh")}[act]
+    for with_z in (True, False):
+        y, z = torch.empty(n, out_dim, device="cuda"), torch.full((n, out_dim), 5.0, device="cuda")
+        lib.call("fb_dense_fwd", ctx.handle, ctx.stream, lib.ACT[act], 0, W.data_ptr(), b.data_ptr(), x.data_ptr(), y.data_ptr(),
+                 z.data_ptr() if with_z else None, out_dim, in_dim, n)
+        assert (y.double() - yr).norm() / yr.norm() < TOL and ctx.device_error() == 0
+        assert (z.double() - zr).norm() / zr.norm() < TOL if with_z else bool((z == 5.0).all())
+
+
+@pytest.mark.parametrize("a_mn,b_mn", [(0, 1), (0, 0), (1, 1)])
+@pytest.mark.parametrize("k", [2048, 9000])
+def test_rows_of_any_magnitude(ctx, a_mn, b_mn, k):
+    """Every row has a scale of its own: rows from 2^-100 to 2^100, zero rows, products that are tiny or huge although their
+    scaled sums are not, and single elements far below their row's largest."""
+    m, n = 2048, 2304
+    g = torch.Generator(device="cuda").manual_seed(k)
+    a, _ = _mat(g, m, k, a_mn, 0)
+    b, _ = _mat(g, n, k, b_mn, 0)
+    ea = torch.randint(-100, 101, (m,), generator=g, device="cuda").double()
+    eb = torch.minimum(torch.maximum(torch.randint(-100, 101, (n,), generator=g, device="cuda").double(), torch.tensor(-100.0)), torch.tensor(20.0))
+    sa, sb = (2.0 ** ea).float(), (2.0 ** eb).float()
+    sa[5], sb[7] = 0.0, 0.0
+    a *= sa[None, :] if a_mn else sa[:, None]
+    b *= sb[None, :] if b_mn else sb[:, None]
+    small = torch.rand(a.shape, generator=g, device="cuda") < 0.3
+    a = torch.where(small, a * 2.0 ** -16, a)
+    a64, b64 = (a.T if a_mn else a).double(), (b.T if b_mn else b).double()
+    ref = a64 @ b64.T
+    out = torch.empty(m, n, device="cuda")
+    _product(ctx, a, a_mn, b, b_mn, out, m, n, k)
+    scale = a64.norm(dim=1)[:, None] * b64.norm(dim=1)[None, :]      # a row's and a column's norms bound an element's terms
+    fits = (scale < 1e36) & (scale > 1e-30)
+    assert int(fits.sum()) > m * n // 3
+    err = ((out.double() - ref).abs() / scale.clamp_min(1e-300))[fits].max()
+    assert err < 2 * TOL, float(err)            # the largest of 4e6 elements, each against the norm of its own terms
+    assert bool((out[5] == 0).all()) and bool((out[:, 7] == 0).all()) and ctx.device_error() == 0
+
+
+def test_values_that_are_not_finite_stay_in_their_rows(ctx):
+    m, n, k = 2048, 2304, 2048
+    g = torch.Generator(device="cuda").manual_seed(1)
+    a, a64 = _mat(g, m, k, 0, 0)
+    b, b64 = _mat(g, n, k, 1, 0)
+    ref = a64 @ b64.T
+    a[3, 100], a[700, 5], b[9, 17] = float("inf"), float("nan"), float("-inf")
+    out = torch.empty(m, n, device="cuda")
+    _product(ctx, a, 0, b, 1, out, m, n, k)
+    bad = ~torch.isfinite(out)
+    want = torch.zeros_like(bad)
+    want[3], want[700], want[:, 17] = True, True, True
+    assert bool((bad == want).all())
+    assert float((out.double() - ref)[~want].norm() / ref[~want].norm()) < TOL
+
+
+def test_operands_whose_images_are_made_in_pieces(ctx):
+    m, n, k = 49160, 4104, 4096                 # 805 MB of images for the larger operand
+    g = torch.Generator(device="cuda").manual_seed(2)
+    for shape in ((m, n), (n, m)):
+        a, _ = _mat(g, shape[0], k, 0, 0)
+        b, _ = _mat(g, shape[1], k, 1, 0)
+        out = torch.empty(shape, device="cuda")
+        _product(ctx, a, 0, b, 1, out, shape[0], shape[1], k)
+        rows = torch.randint(0, shape[0], (64,), generator=g, device="cuda")
+        cols = torch.cat([torch.randint(0, shape[1], (62,), generator=g, device="cuda"), torch.tensor([0, shape[1] - 1], device="cuda")])
+        ref = a[rows].double() @ b[:, cols].double()
+        assert float((out[rows][:, cols].double() - ref).norm() / ref.norm()) < TOL
+        ref = a[-1].double() @ b.double()
+        assert float((out[-1].double() - ref).norm() / ref.norm()) < TOL and ctx.device_error() == 0
+
+
+def test_products_of_planes_inside_a_graph_and_beside_one(ctx):
+    """Images belong to their call: a replay on one stream and eager products on another do not meet."""
+    m, n, k = 2048, 2048, 4096
+    g = torch.Generator(device="cuda").manual_seed(3)
+    a, a64 = _mat(g, m, k, 0, 0)
+    b, b64 = _mat(g, n, k, 1, 0)
+    c, c64 = _mat(g, m, k, 0, 0)
+    out, out2 = torch.empty(m, n, device="cuda"), torch.empty(m, n, device="cuda")
+    _product(ctx, a, 0, b, 1, out, m, n, k)
+    graph, side = torch.cuda.CUDAGraph(), torch.cuda.Stream()
+    torch.cuda.synchronize()
+    with torch.cuda.graph(graph):
+        _product(ctx, a, 0, b, 1, out, m, n, k)
+    torch.cuda.synchronize()
+    for _ in range(10):
+        graph.replay()
+        with torch.cuda.stream(side):
+            _product(ctx, c, 0, b, 1, out2, m, n, k)
+    torch.cuda.synchronize()
+    for got, x in ((out, a64), (out2, c64)):
+        ref = x @ b64.T
+        assert float((got.double() - ref).norm() / ref.norm()) < TOL
+    assert ctx.device_error() == 0
