@@ -1,378 +1,607 @@
 // BatchNorm forward (training / inference) and backward (memory-bound).
 //
-// Data layout: x is [n][c][s] row-major (Julia WHCN with s = W*H; a 2-D input [C, N] has s == 1).
-// Training forward = statistics pass (read x) + finaliser (tiny) + normalise pass (read x, write y):
-// 2 reads + 1 write.  Backward = reduction pass (read x, dy) + finaliser + dx pass (read x, dy, write
-// dx): 4 reads + 1 write; the activation mask is recomputed from x instead of reading y.
-// Statistics use a shifted sum / sum-of-squares per thread, converted to (count, mean, M2) and merged
-// with Chan's (Welford) update through warp shuffles, so large |mean|/std inputs stay accurate.
+// Data layout: x is [n][c][s] row-major (Julia WHCN with s = W*H; a 2-D input [C, N] has s == 1).  A block of 256 threads takes
+// rows (one sample's s values of a channel) with tpr threads side by side on one row (a power of two) and 256 / tpr rows at a
+// time; W = 4 floats a piece where rows are whole aligned float4, else one.
+//
+// Training forward: a cluster of up to 8 CTAs owns a channel at a time.  Its values are read once, into shared memory, where their
+// statistics are taken; the CTAs' sums meet in distributed shared memory, and y is written from there: 1 read + 1 write.  The
+// kernel is persistent: while a channel is worked on the next two are on their way.  Channels that do not fit
+// (more than 8 x 200 KB) take statistics first and normalise in a second pass.  32 x 32 x 256 x 128: 76 -> 63 us (statistics, a
+// finaliser and a second pass before; 41 would be two passes at the HBM rate: 15 clusters of 8 fit the GPU, 120 of 148 SMs,
+// and 256 channels are 17.1 rounds of them); 7 x 7 x 512 x 256: 136 -> 21; 512 x 256: 103 -> 7.
+// Backward: sums of dz and dz xhat per channel (a cluster again, no second launch), then, if dx is wanted, a pass that writes
+// it; the activation mask is recomputed from x instead of reading y.
+// Statistics are sums of x - shift and of its square with one of the channel's values as the shift, so large |mean|/std inputs
+// stay accurate.
 #include "common.cuh"
+#include "tc_common.cuh"
 
 namespace {
 
 constexpr int BN_THREADS = 256;
+constexpr int BN_FWD_THREADS = 512;          // of a channel cached in shared memory: more loads of one CTA in flight
+constexpr int BN_MAX_CLUSTER = 8;
+constexpr size_t BN_CACHE_MAX = 200 * 1024;  // of one CTA, the only one of its SM
 
-struct Wf { float n, mean, m2; };
-
-__device__ __forceinline__ Wf wf_warp_merge(Wf a) {
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) {
-    const float nb = __shfl_xor_sync(0xffffffffu, a.n, o);
-    const float mb = __shfl_xor_sync(0xffffffffu, a.mean, o);
-    const float qb = __shfl_xor_sync(0xffffffffu, a.m2, o);
-    fb_welford_merge(a.n, a.mean, a.m2, nb, mb, qb);
-  }
-  return a;
-}
-
-// Block merge; result valid in thread 0.
-__device__ __forceinline__ Wf wf_block_merge(Wf a, float* sh /* 96 floats */) {
-  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, nw = blockDim.x >> 5;
-  a = wf_warp_merge(a);
-  __syncthreads();
-  if (lane == 0) { sh[w] = a.n; sh[32 + w] = a.mean; sh[64 + w] = a.m2; }
-  __syncthreads();
-  Wf r;
-  r.n = (lane < nw) ? sh[lane] : 0.0f;
-  r.mean = (lane < nw) ? sh[32 + lane] : 0.0f;
-  r.m2 = (lane < nw) ? sh[64 + lane] : 0.0f;
-  return wf_warp_merge(r);
-}
-
-// --------------------------------------------------------------------------- statistics pass ---
-// grid (c, split): block (ch, p) covers samples p, p+split, ... of channel ch.
-template <bool VEC>
-__global__ void __launch_bounds__(BN_THREADS)
-bn_stats_kernel(const float* __restrict__ x, float* __restrict__ part /* [c][split][3] */, int64_t s,
-                int64_t c, int64_t n) {
-  __shared__ float sh[96];
-  const int64_t ch = blockIdx.x;
-  const int split = gridDim.y, p = blockIdx.y;
-  const float shift = __ldg(x + ch * s);  // a value inside the channel's range
-  float cnt = 0.0f, s1 = 0.0f, s2 = 0.0f;
-  if (VEC) {
-    // four rows per pass: four independent 128-bit loads in flight per thread
-    const int64_t s4 = s >> 2;
-    for (int64_t i = p; i < n; i += 4 * (int64_t)split) {
-      const float4* r4[4];
-      bool ok[4];
-#pragma unroll
-      for (int u = 0; u < 4; ++u) {
-        const int64_t ii = i + (int64_t)u * split;
-        ok[u] = ii < n;
-        r4[u] = (const float4*)(x + ((ok[u] ? ii : i) * c + ch) * s);
-      }
-      for (int64_t j = threadIdx.x; j < s4; j += BN_THREADS) {
-        float4 v[4];
-#pragma unroll
-        for (int u = 0; u < 4; ++u) v[u] = ok[u] ? __ldcs(r4[u] + j) : make_float4(shift, shift, shift, shift);
-#pragma unroll
-        for (int u = 0; u < 4; ++u) {
-          const float a = v[u].x - shift, b = v[u].y - shift, cc = v[u].z - shift, d = v[u].w - shift;
-          s1 += (a + b) + (cc + d);
-          s2 += (a * a + b * b) + (cc * cc + d * d);
-          cnt += ok[u] ? 4.0f : 0.0f;
-        }
-      }
-    }
+template <int W>
+__device__ __forceinline__ void ld_piece(const float* p, float* v) {
+  if (W == 4) {
+    const float4 q = *(const float4*)p;
+    v[0] = q.x; v[1] = q.y; v[2] = q.z; v[3] = q.w;
   } else {
-    for (int64_t i = p; i < n; i += split) {
-      const float* row = x + (i * c + ch) * s;
-      for (int64_t j = threadIdx.x; j < s; j += BN_THREADS) {
-        const float a = row[j] - shift;
-        s1 += a;
-        s2 += a * a;
-        cnt += 1.0f;
-      }
+    v[0] = *p;
+  }
+}
+// the same for values that are not looked at again soon (whole passes over tensors that may exceed L2)
+template <int W>
+__device__ __forceinline__ void ld_stream(const float* p, float* v) {
+  if (W == 4) {
+    const float4 q = __ldcs((const float4*)p);
+    v[0] = q.x; v[1] = q.y; v[2] = q.z; v[3] = q.w;
+  } else {
+    v[0] = *p;
+  }
+}
+template <int W>
+__device__ __forceinline__ void st_stream(float* p, const float* v) {
+  if (W == 4) __stcs((float4*)p, make_float4(v[0], v[1], v[2], v[3]));
+  else *p = v[0];
+}
+template <int W>
+__device__ __forceinline__ void st_piece(float* p, const float* v) {
+  if (W == 4) *(float4*)p = make_float4(v[0], v[1], v[2], v[3]);
+  else *p = v[0];
+}
+
+struct Dims {
+  int64_t s, c, n;
+  int split;   // CTAs per channel
+  int tpr;     // threads side by side on one row
+};
+
+// The pieces of a channel that this thread owns: `mine` rows, `step` floats apart, in each of `cols` columns of pieces, `col_step`
+// floats apart, the first of channel 0 at `base`.
+struct Walk {
+  int64_t base, step;
+  int mine, cols, col_step;
+};
+template <int W>
+__device__ __forceinline__ Walk make_walk(const Dims& g, int p) {
+  const int tx = threadIdx.x & (g.tpr - 1), ty = threadIdx.x / g.tpr, nr = (int)blockDim.x / g.tpr;
+  const int64_t first = (int64_t)p * nr + ty, rows = (int64_t)g.split * nr, mine = (g.n - first + rows - 1) / rows;
+  const int64_t at = (int64_t)tx * W, cols = (g.s - at + (int64_t)g.tpr * W - 1) / ((int64_t)g.tpr * W);
+  Walk w;
+  w.base = first * g.c * g.s + at;
+  w.step = rows * g.c * g.s;
+  w.mine = first < g.n ? (int)mine : 0;
+  w.cols = at < g.s ? (int)cols : 0;
+  w.col_step = g.tpr * W;
+  return w;
+}
+// f(k, off, m), U rows at a time, in an order that a second call repeats: pieces k .. k + m - 1 (m <= U) of channel ch lie at off,
+// off + w.step, ...
+template <int U, typename F>
+__device__ __forceinline__ void each_piece(const Walk& w, int64_t ch_off, F f) {
+  int k = 0;
+  for (int j = 0; j < w.cols; ++j) {
+    int64_t off = w.base + ch_off + (int64_t)j * w.col_step;
+    for (int i = 0; i < w.mine; i += U, off += U * w.step) {
+      const int m = w.mine - i < U ? w.mine - i : U;
+      f(k, off, m);
+      k += m;
     }
   }
-  Wf w;
-  w.n = cnt;
-  w.mean = cnt > 0.0f ? s1 / cnt : 0.0f;
-  w.m2 = cnt > 0.0f ? fmaxf(s2 - s1 * w.mean, 0.0f) : 0.0f;
-  w.mean += shift;
-  w = wf_block_merge(w, sh);
+}
+
+// Sums over a cluster of `split` CTAs.  Every CTA sends its own to all of them with st.async, which an mbarrier of the receiver
+// counts: a cluster barrier would first wait for every store to y that is still on its way (its release covers them): that cost
+// 1 - 2 us of the 5 us a channel of 32 x 32 x 128 values took.  Two sets of slots in turn: a CTA sends to a set again only after
+// everybody's next sums have reached it, which are sent after this set was read.
+struct Exchange {
+  float2 slots[2][BN_MAX_CLUSTER];
+  uint64_t bar[2];
+  float sh[64];
+};
+__device__ __forceinline__ void exchange_init(Exchange& x, int split) {
+  if (split == 1) return;
   if (threadIdx.x == 0) {
-    float* o = part + (ch * split + p) * 3;
-    o[0] = w.n; o[1] = w.mean; o[2] = w.m2;
+    mbar_init(smem_u32(&x.bar[0]), 1);
+    mbar_init(smem_u32(&x.bar[1]), 1);
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
+  __syncwarp();
+  cluster_sync_all();
+}
+// Both sums, valid in every thread.  `round` counts the calls.  False when a wait ran out (bounded: error code 2101).
+__device__ __forceinline__ bool channel_sums(Exchange& x, float& a, float& b, int split, uint32_t mine, int round) {
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, nw = (int)blockDim.x >> 5;
+  a = fb_warp_sum(a);
+  b = fb_warp_sum(b);
+  if (lane == 0) { x.sh[w] = a; x.sh[32 + w] = b; }
+  __syncthreads();
+  if (split == 1) {
+    a = fb_warp_sum(lane < nw ? x.sh[lane] : 0.0f);
+    b = fb_warp_sum(lane < nw ? x.sh[32 + lane] : 0.0f);
+    __syncthreads();   // sh may be written again
+    return true;
+  }
+  const int turn = round & 1;
+  const uint32_t bar = smem_u32(&x.bar[turn]);
+  if (w == 0) {
+    a = fb_warp_sum(lane < nw ? x.sh[lane] : 0.0f);
+    b = fb_warp_sum(lane < nw ? x.sh[32 + lane] : 0.0f);
+    if (lane == 0) mbar_arrive_expect_tx(bar, 8u * (uint32_t)split);
+    if (lane < split)
+      asm volatile("st.async.shared::cluster.mbarrier::complete_tx::bytes.v2.f32 [%0], {%1, %2}, [%3];"
+                   ::"r"(map_to_cta(smem_u32(&x.slots[turn][mine]), (uint32_t)lane)), "f"(a), "f"(b), "r"(map_to_cta(bar, (uint32_t)lane))
+                   : "memory");
+  }
+  uint32_t ok = 0;
+  for (uint32_t it = 0; it < WAIT_LIMIT && !ok; ++it)
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n\t"
+        "selp.u32 %0, 1, 0, p;\n\t}"
+        : "=r"(ok)
+        : "r"(bar), "r"((uint32_t)(round >> 1) & 1u)
+        : "memory");
+  a = b = 0.0f;
+  for (int r = 0; r < split; ++r) {
+    const float2 v = x.slots[turn][r];
+    a += v.x;
+    b += v.y;
+  }
+  return ok != 0;
 }
 
-// One thread per channel: merge the split partials, write mean / rstd, update running statistics.
-__global__ void bn_stats_finalize_kernel(const float* __restrict__ part, int split, int64_t c, float eps,
-                                         float momentum, float* __restrict__ save_mean,
-                                         float* __restrict__ save_rstd, float* __restrict__ running_mean,
-                                         float* __restrict__ running_var) {
-  const int64_t ch = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (ch >= c) return;
-  float n = 0.0f, mean = 0.0f, m2 = 0.0f;
-  for (int p = 0; p < split; ++p) {
-    const float* q = part + (ch * split + p) * 3;
-    fb_welford_merge(n, mean, m2, q[0], q[1], q[2]);
+// mean, 1 / std and running statistics from the shifted sums of a channel of cnt values
+struct ChannelStats { float mean, rs; };
+__device__ __forceinline__ ChannelStats channel_stats(float s1, float s2, float shift, float cnt, float eps, bool write, int64_t ch,
+                                                      float momentum, float* save_mean, float* save_rstd, float* running_mean,
+                                                      float* running_var) {
+  const float d = s1 / cnt, m2 = fmaxf(s2 - s1 * d, 0.0f), mean = shift + d;
+  const float var = m2 / cnt;  // biased
+  const float rs = rsqrtf(var + eps);
+  if (write) {
+    save_mean[ch] = mean;
+    save_rstd[ch] = rs;
+    if (running_mean != nullptr) {
+      running_mean[ch] = (1.0f - momentum) * running_mean[ch] + momentum * mean;
+      running_var[ch] = (1.0f - momentum) * running_var[ch] + momentum * var * (cnt / (cnt - 1.0f));
+    }
   }
-  const float var = m2 / n;  // biased
-  save_mean[ch] = mean;
-  save_rstd[ch] = rsqrtf(var + eps);
-  if (running_mean != nullptr) {
-    running_mean[ch] = (1.0f - momentum) * running_mean[ch] + momentum * mean;
-    running_var[ch] = (1.0f - momentum) * running_var[ch] + momentum * var * (n / (n - 1.0f));
-  }
+  return {mean, rs};
 }
 
-// rstd from running variance (inference)
-__global__ void bn_infer_prepare_kernel(const float* __restrict__ running_mean, const float* __restrict__ running_var,
-                                        float eps, int64_t c, float* __restrict__ mean, float* __restrict__ rstd) {
-  const int64_t ch = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (ch >= c) return;
-  mean[ch] = running_mean[ch];
-  rstd[ch] = 1.0f / sqrtf(running_var[ch] + eps);
+// ------------------------------------------------------------------------------ statistics ---
+// One cluster of `split` CTAs per channel.
+template <int W>
+__global__ void __launch_bounds__(BN_THREADS)
+bn_stats_kernel(const float* __restrict__ x, const Dims g, float eps, float momentum, float* __restrict__ save_mean,
+                float* __restrict__ save_rstd, float* __restrict__ running_mean, float* __restrict__ running_var,
+                int32_t* __restrict__ dev_err) {
+  constexpr int U = 4;
+  __shared__ Exchange ex;
+  const int64_t ch = blockIdx.x / (unsigned)g.split;
+  const int p = (int)(blockIdx.x % (unsigned)g.split);
+  exchange_init(ex, g.split);
+  const float shift = __ldg(x + ch * g.s);  // a value inside the channel's range
+  float s1 = 0.0f, s2 = 0.0f;
+  const Walk wk = make_walk<W>(g, p);
+  each_piece<U>(wk, ch * g.s, [&](int, int64_t off, int m) {
+    float v[U][W];
+#pragma unroll
+    for (int u = 0; u < U; ++u)
+      if (u < m) ld_piece<W>(x + off + u * wk.step, v[u]);
+#pragma unroll
+    for (int u = 0; u < U; ++u)
+      if (u < m)
+#pragma unroll
+        for (int e = 0; e < W; ++e) {
+          const float a = v[u][e] - shift;
+          s1 += a;
+          s2 = fmaf(a, a, s2);
+        }
+  });
+  const bool ok = channel_sums(ex, s1, s2, g.split, (uint32_t)p, 0);
+  channel_stats(s1, s2, shift, (float)(g.s * g.n), eps, p == 0 && threadIdx.x == 0, ch, momentum, save_mean, save_rstd, running_mean, running_var);
+  if (!ok && threadIdx.x == 0) atomicExch(dev_err, 2101);
+  if (g.split > 1) cluster_sync_all();   // (no CTA leaves while another may still send to it)
+}
+
+// ------------------------------------------------------------- the whole training forward pass ---
+// Cluster q of Q takes channels q, q + Q, ...; `depth` (1 .. 3) channels are held: each thread brings its own pieces with cp.async and
+// reads nobody else's, so the copies need no barrier.
+template <int W, int ACT>
+__global__ void __launch_bounds__(BN_FWD_THREADS, 1)
+bn_fwd_kernel(const float* __restrict__ x, const float* __restrict__ gamma, const float* __restrict__ beta, float* __restrict__ y,
+              const Dims g, int depth, int slab, float eps, float momentum, float* __restrict__ save_mean, float* __restrict__ save_rstd,
+              float* __restrict__ running_mean, float* __restrict__ running_var, int act, int32_t* __restrict__ dev_err) {
+  extern __shared__ __align__(16) float cache[];   // [depth][piece][thread][W]
+  __shared__ Exchange ex;
+  const int p = (int)(blockIdx.x % (unsigned)g.split);
+  const int64_t Q = gridDim.x / (unsigned)g.split, first = blockIdx.x / (unsigned)g.split;
+  const float cnt = (float)(g.s * g.n);
+  exchange_init(ex, g.split);
+  const Walk wk = make_walk<W>(g, p);
+  const int pieces = wk.mine * wk.cols, per = (int)blockDim.x * W;
+  float* const own = cache + threadIdx.x * W;
+  auto fetch = [&](int64_t ch, float* to) {
+    if (ch < g.c) {
+      uint32_t dst = smem_u32(to);
+      each_piece<1>(wk, ch * g.s, [&](int, int64_t off, int) {
+        if (W == 4) asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(x + off) : "memory");
+        else asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(dst), "l"(x + off) : "memory");
+        dst += (uint32_t)per * 4u;
+      });
+    }
+    asm volatile("cp.async.commit_group;" ::: "memory");
+  };
+  for (int d = 0; d < depth; ++d) fetch(first + d * Q, own + d * slab);
+  // a value inside the channel's range, scale and bias: one channel ahead
+  auto ahead = [&](const float* a, int64_t ch, int64_t stride, float otherwise) { return a != nullptr && ch < g.c ? __ldg(a + ch * stride) : otherwise; };
+  float shift = ahead(x, first, g.s, 0.0f), ga = ahead(gamma, first, 1, 1.0f), be = ahead(beta, first, 1, 0.0f);
+  int d = 0, round = 0;
+  bool ok = true;
+  for (int64_t ch = first; ch < g.c; ch += Q, ++round) {
+    const float shift1 = ahead(x, ch + Q, g.s, 0.0f), ga1 = ahead(gamma, ch + Q, 1, 1.0f), be1 = ahead(beta, ch + Q, 1, 0.0f);
+    if (depth == 3) asm volatile("cp.async.wait_group 2;" ::: "memory");
+    else if (depth == 2) asm volatile("cp.async.wait_group 1;" ::: "memory");
+    else asm volatile("cp.async.wait_group 0;" ::: "memory");
+    float* const here = own + d * slab;
+    float s1 = 0.0f, s2 = 0.0f;
+#pragma unroll 4
+    for (int k = 0; k < pieces; ++k) {
+      float v[W];
+      ld_piece<W>(here + k * per, v);
+#pragma unroll
+      for (int e = 0; e < W; ++e) {
+        const float a = v[e] - shift;
+        s1 += a;
+        s2 = fmaf(a, a, s2);
+      }
+    }
+    ok = channel_sums(ex, s1, s2, g.split, (uint32_t)p, round) && ok;
+    const ChannelStats st = channel_stats(s1, s2, shift, cnt, eps, p == 0 && threadIdx.x == 0, ch, momentum, save_mean, save_rstd, running_mean, running_var);
+    const float sc = st.rs * ga;
+    const float* src = here;
+    each_piece<1>(wk, ch * g.s, [&](int, int64_t off, int) {
+      float o[W];
+      ld_piece<W>(src, o);
+      src += per;
+#pragma unroll
+      for (int e = 0; e < W; ++e) o[e] = fb_act_apply_k<ACT>(act, fmaf(o[e] - st.mean, sc, be));
+      st_piece<W>(y + off, o);
+    });
+    fetch(ch + depth * Q, here);
+    d = d + 1 == depth ? 0 : d + 1;
+    shift = shift1; ga = ga1; be = be1;
+  }
+  if (!ok && threadIdx.x == 0) atomicExch(dev_err, 2101);
+  if (g.split > 1) cluster_sync_all();   // (no CTA leaves while another may still send to it)
 }
 
 // ----------------------------------------------------------------------------- normalise pass ---
-template <bool VEC>
+// rows of one chunk
+__host__ __device__ __forceinline__ int bn_chunk(int nr) { return 8 * nr < BN_THREADS ? 8 * nr : BN_THREADS; }
+
+// mean and rstd per channel; VAR: a variance is given instead of rstd
+template <int W, bool VAR, int ACT>
 __global__ void __launch_bounds__(BN_THREADS)
 bn_apply_kernel(const float* __restrict__ x, const float* __restrict__ gamma, const float* __restrict__ beta,
-                const float* __restrict__ mean, const float* __restrict__ rstd, float* __restrict__ y, int64_t s,
-                int64_t c, int64_t total, int act) {
-  if (VEC) {
-    const int64_t total4 = total >> 2;
-    const float4* x4 = (const float4*)x;
-    float4* y4 = (float4*)y;
-    for (int64_t i = (int64_t)blockIdx.x * BN_THREADS + threadIdx.x; i < total4; i += (int64_t)gridDim.x * BN_THREADS) {
-      const int64_t ch = ((i << 2) / s) % c;
-      const float mu = __ldg(mean + ch);
-      const float sc = __ldg(rstd + ch) * (gamma ? __ldg(gamma + ch) : 1.0f);
-      const float sf = beta ? __ldg(beta + ch) : 0.0f;
-      const float4 v = __ldcs(x4 + i);
-      float4 o;
-      o.x = fmaf(v.x - mu, sc, sf); o.y = fmaf(v.y - mu, sc, sf); o.z = fmaf(v.z - mu, sc, sf); o.w = fmaf(v.w - mu, sc, sf);
-      if (act != FB_ACT_IDENTITY) {
-        o.x = fb_act_apply(act, o.x); o.y = fb_act_apply(act, o.y); o.z = fb_act_apply(act, o.z); o.w = fb_act_apply(act, o.w);
-      }
-      __stcs(y4 + i, o);
+                const float* __restrict__ mean, const float* __restrict__ rstd, float eps, float* __restrict__ y, int64_t s, int64_t c,
+                int64_t rows, int tpr, int act) {
+  constexpr int U = 4;
+  __shared__ float3 par[BN_THREADS];   // mean, scale, shift of a chunk of rows: one thread each, not all threads for every row
+  const int tx = threadIdx.x & (tpr - 1), ty = threadIdx.x / tpr, nr = BN_THREADS / tpr;
+  const int chunk = bn_chunk(nr);
+  for (int64_t r0 = (int64_t)blockIdx.x * chunk; r0 < rows; r0 += (int64_t)gridDim.x * chunk) {
+    const int m = rows - r0 < chunk ? (int)(rows - r0) : chunk;
+    __syncthreads();
+    if ((int)threadIdx.x < m) {
+      const int64_t r = r0 + threadIdx.x, ch = rows <= 0x7fffffff ? (int64_t)((uint32_t)r % (uint32_t)c) : r % c;
+      const float q = __ldg(rstd + ch);
+      par[threadIdx.x] = make_float3(__ldg(mean + ch), (VAR ? 1.0f / sqrtf(q + eps) : q) * (gamma ? __ldg(gamma + ch) : 1.0f), beta ? __ldg(beta + ch) : 0.0f);
     }
-  } else {
-    for (int64_t i = (int64_t)blockIdx.x * BN_THREADS + threadIdx.x; i < total; i += (int64_t)gridDim.x * BN_THREADS) {
-      const int64_t ch = (i / s) % c;
-      const float sc = rstd[ch] * (gamma ? gamma[ch] : 1.0f);
-      const float o = fmaf(x[i] - mean[ch], sc, beta ? beta[ch] : 0.0f);
-      y[i] = fb_act_apply(act, o);
-    }
-  }
-}
-
-// Row-structured variants for long contiguous rows (s4 >= 32 float4): one (sample, channel) row per block pass, so
-// the per-element channel lookup (an integer division) disappears; two rows per pass for memory-level parallelism.
-__global__ void __launch_bounds__(BN_THREADS)
-bn_apply_rows_kernel(const float4* __restrict__ x, const float* __restrict__ gamma, const float* __restrict__ beta,
-                     const float* __restrict__ mean, const float* __restrict__ rstd, float4* __restrict__ y, int64_t s4,
-                     int64_t c, int64_t rows, int act) {
-  for (int64_t r0 = (int64_t)blockIdx.x * 2; r0 < rows; r0 += (int64_t)gridDim.x * 2) {
-    const bool ok2 = r0 + 1 < rows;
-    const int64_t ch0 = r0 % c, ch1 = (r0 + 1) % c;
-    const float mu0 = __ldg(mean + ch0), sc0 = __ldg(rstd + ch0) * (gamma ? __ldg(gamma + ch0) : 1.0f), sf0 = beta ? __ldg(beta + ch0) : 0.0f;
-    const float mu1 = __ldg(mean + ch1), sc1 = __ldg(rstd + ch1) * (gamma ? __ldg(gamma + ch1) : 1.0f), sf1 = beta ? __ldg(beta + ch1) : 0.0f;
-    const float4* xa = x + r0 * s4;
-    float4* ya = y + r0 * s4;
-    for (int64_t j = threadIdx.x; j < s4; j += BN_THREADS) {
-      const float4 va = __ldcs(xa + j);
-      float4 vb = make_float4(0.f, 0.f, 0.f, 0.f);
-      if (ok2) vb = __ldcs(xa + s4 + j);
-      float4 oa, ob;
-      oa.x = fmaf(va.x - mu0, sc0, sf0); oa.y = fmaf(va.y - mu0, sc0, sf0); oa.z = fmaf(va.z - mu0, sc0, sf0); oa.w = fmaf(va.w - mu0, sc0, sf0);
-      ob.x = fmaf(vb.x - mu1, sc1, sf1); ob.y = fmaf(vb.y - mu1, sc1, sf1); ob.z = fmaf(vb.z - mu1, sc1, sf1); ob.w = fmaf(vb.w - mu1, sc1, sf1);
-      if (act != FB_ACT_IDENTITY) {
-        oa.x = fb_act_apply(act, oa.x); oa.y = fb_act_apply(act, oa.y); oa.z = fb_act_apply(act, oa.z); oa.w = fb_act_apply(act, oa.w);
-        ob.x = fb_act_apply(act, ob.x); ob.y = fb_act_apply(act, ob.y); ob.z = fb_act_apply(act, ob.z); ob.w = fb_act_apply(act, ob.w);
-      }
-      __stcs(ya + j, oa);
-      if (ok2) __stcs(ya + s4 + j, ob);
-    }
-  }
-}
-
-__global__ void __launch_bounds__(BN_THREADS)
-bn_bwd_apply_rows_kernel(const float4* __restrict__ x, const float4* __restrict__ dy, const float* __restrict__ gamma,
-                         const float* __restrict__ beta, const float* __restrict__ mean, const float* __restrict__ rstd,
-                         const float* __restrict__ coef, float4* __restrict__ dx, int64_t s4, int64_t c, int64_t rows, int act) {
-  for (int64_t r = blockIdx.x; r < rows; r += gridDim.x) {
-    const int64_t ch = r % c;
-    const float mu = __ldg(mean + ch), rs = __ldg(rstd + ch);
-    const float ga = gamma ? __ldg(gamma + ch) : 1.0f, be = beta ? __ldg(beta + ch) : 0.0f;
-    const float m1 = __ldg(coef + ch * 2), m2 = __ldg(coef + ch * 2 + 1), k = ga * rs;
-    const float4* xa = x + r * s4;
-    const float4* da = dy + r * s4;
-    float4* oa = dx + r * s4;
-    for (int64_t j = threadIdx.x; j < s4; j += 2 * BN_THREADS) {
-      const int64_t j2 = j + BN_THREADS;
-      const bool ok2 = j2 < s4;
-      float4 xv[2], dz[2];
-      xv[0] = __ldcs(xa + j); dz[0] = __ldcs(da + j);
-      if (ok2) { xv[1] = __ldcs(xa + j2); dz[1] = __ldcs(da + j2); }
+    __syncthreads();
+    for (int k = ty; k < m; k += U * nr) {
+      const float* xr = x + (r0 + k) * s;
+      float* yr = y + (r0 + k) * s;
+      for (int64_t j = (int64_t)tx * W; j < s; j += (int64_t)tpr * W) {
+        float v[U][W];
 #pragma unroll
-      for (int u = 0; u < 2; ++u) {
-        if (u == 1 && !ok2) break;
-        const float h0 = (xv[u].x - mu) * rs, h1 = (xv[u].y - mu) * rs, h2 = (xv[u].z - mu) * rs, h3 = (xv[u].w - mu) * rs;
-        if (act != FB_ACT_IDENTITY) {
-          dz[u].x *= fb_act_grad_z(act, fmaf(h0, ga, be)); dz[u].y *= fb_act_grad_z(act, fmaf(h1, ga, be));
-          dz[u].z *= fb_act_grad_z(act, fmaf(h2, ga, be)); dz[u].w *= fb_act_grad_z(act, fmaf(h3, ga, be));
+        for (int u = 0; u < U; ++u)
+          if (k + u * nr < m) ld_stream<W>(xr + u * nr * s + j, v[u]);
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+          if (k + u * nr >= m) break;
+          const float3 q = par[k + u * nr];
+#pragma unroll
+          for (int e = 0; e < W; ++e) v[u][e] = fb_act_apply_k<ACT>(act, fmaf(v[u][e] - q.x, q.y, q.z));
+          st_stream<W>(yr + u * nr * s + j, v[u]);
         }
-        float4 o;
-        o.x = k * (dz[u].x - m1 - h0 * m2); o.y = k * (dz[u].y - m1 - h1 * m2);
-        o.z = k * (dz[u].z - m1 - h2 * m2); o.w = k * (dz[u].w - m1 - h3 * m2);
-        __stcs(oa + (u == 0 ? j : j2), o);
       }
     }
   }
 }
 
-// --------------------------------------------------------------------------- backward reduce ---
-// part[c][split][2] = (sum dz, sum dz*xhat) with dz = dy * act'(gamma*xhat+beta)
-template <bool VEC>
+// Short rows (less than 128 floats) whatever their alignment: the tensor as one run of float4 pieces, which may span rows.  s and
+// c divide by multiplication (Granlund and Montgomery, "Division by invariant integers using multiplication").
+struct FastDiv {
+  uint32_t d, mul, sh1, sh2;
+};
+FastDiv fast_div(uint32_t d) {
+  uint32_t l = 0;
+  while (l < 32 && ((uint64_t)1 << l) < d) ++l;
+  const uint64_t m = ((((uint64_t)1 << l) - d) << 32) / d + 1;
+  return {d, (uint32_t)m, l < 1 ? l : 1, l < 1 ? 0 : l - 1};
+}
+__device__ __forceinline__ uint32_t quotient(const FastDiv& f, uint32_t n) {
+  const uint32_t t = __umulhi(f.mul, n);
+  return (t + ((n - t) >> f.sh1)) >> f.sh2;
+}
+
+template <bool VAR, int ACT>
 __global__ void __launch_bounds__(BN_THREADS)
-bn_bwd_reduce_kernel(const float* __restrict__ x, const float* __restrict__ dy, const float* __restrict__ gamma,
-                     const float* __restrict__ beta, const float* __restrict__ mean, const float* __restrict__ rstd,
-                     float* __restrict__ part, int64_t s, int64_t c, int64_t n, int act) {
-  __shared__ float sh[64];
-  const int64_t ch = blockIdx.x;
-  const int split = gridDim.y, p = blockIdx.y;
-  const float mu = mean[ch], rs = rstd[ch];
-  const float ga = gamma ? gamma[ch] : 1.0f, be = beta ? beta[ch] : 0.0f;
+bn_apply_flat_kernel(const float* __restrict__ x, const float* __restrict__ gamma, const float* __restrict__ beta,
+                     const float* __restrict__ mean, const float* __restrict__ rstd, float eps, float* __restrict__ y, const FastDiv fs,
+                     const FastDiv fc, uint32_t total, int act) {
+  constexpr int U = 2;
+  for (uint32_t i = blockIdx.x * (U * BN_THREADS) + threadIdx.x; i < (total + 3) / 4; i += gridDim.x * (U * BN_THREADS)) {
+    float v[U][4];
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      const uint32_t at = 4 * (i + u * BN_THREADS);
+      if (at + 3 < total) {
+        ld_piece<4>(x + at, v[u]);
+      } else {
+#pragma unroll
+        for (int e = 0; e < 4; ++e) v[u][e] = at + e < total ? x[at + e] : 0.0f;
+      }
+    }
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      const uint32_t at = 4 * (i + u * BN_THREADS);
+      if (at >= total) break;
+      const uint32_t row = quotient(fs, at);
+      uint32_t pos = at - row * fs.d, ch = row - quotient(fc, row) * fc.d;
+      float mu = 0.0f, sc = 0.0f, sf = 0.0f;
+#pragma unroll
+      for (int e = 0; e < 4; ++e) {
+        if (e == 0 || pos == 0) {
+          const float q = __ldg(rstd + ch);
+          mu = __ldg(mean + ch);
+          sc = (VAR ? 1.0f / sqrtf(q + eps) : q) * (gamma ? __ldg(gamma + ch) : 1.0f);
+          sf = beta ? __ldg(beta + ch) : 0.0f;
+        }
+        v[u][e] = fb_act_apply_k<ACT>(act, fmaf(v[u][e] - mu, sc, sf));
+        if (++pos == fs.d) {
+          pos = 0;
+          if (++ch == fc.d) ch = 0;
+        }
+      }
+      if (at + 3 < total) {
+        st_piece<4>(y + at, v[u]);
+      } else {
+#pragma unroll
+        for (int e = 0; e < 4; ++e)
+          if (at + e < total) y[at + e] = v[u][e];
+      }
+    }
+  }
+}
+
+// ----------------------------------------------------------------------------------- backward ---
+// dgamma, dbeta and (coef != NULL) the means of dz and dz * xhat, with dz = dy_scale * dy * act'(gamma * xhat + beta); one cluster
+// per channel
+template <int W, int ACT>
+__global__ void __launch_bounds__(BN_THREADS, 5)
+bn_bwd_sums_kernel(const float* __restrict__ x, const float* __restrict__ dy, float dy_scale, const float* __restrict__ gamma,
+                   const float* __restrict__ beta, const float* __restrict__ mean, const float* __restrict__ rstd, const Dims g,
+                   float* __restrict__ coef, float* __restrict__ dgamma, float* __restrict__ dbeta, int act, int32_t* __restrict__ dev_err) {
+  constexpr int U = 2;
+  __shared__ Exchange ex;
+  exchange_init(ex, g.split);
+  const int64_t ch = blockIdx.x / (unsigned)g.split;
+  const int p = (int)(blockIdx.x % (unsigned)g.split);
+  const float mu = __ldg(mean + ch), rs = __ldg(rstd + ch);
+  const float ga = gamma ? __ldg(gamma + ch) : 1.0f, be = beta ? __ldg(beta + ch) : 0.0f;
   float a1 = 0.0f, a2 = 0.0f;
-  if (VEC) {
-    const int64_t s4 = s >> 2;
-    for (int64_t i = p; i < n; i += 2 * (int64_t)split) {
-      const int64_t i2 = i + split;
-      const bool ok2 = i2 < n;
-      const float4* xa = (const float4*)(x + (i * c + ch) * s);
-      const float4* da = (const float4*)(dy + (i * c + ch) * s);
-      const float4* xb = (const float4*)(x + ((ok2 ? i2 : i) * c + ch) * s);
-      const float4* db = (const float4*)(dy + ((ok2 ? i2 : i) * c + ch) * s);
-      for (int64_t j = threadIdx.x; j < s4; j += BN_THREADS) {
-        float4 xv[2], dz[2];
-        xv[0] = __ldcs(xa + j); dz[0] = __ldcs(da + j);
-        if (ok2) { xv[1] = __ldcs(xb + j); dz[1] = __ldcs(db + j); }
-        else { xv[1] = make_float4(mu, mu, mu, mu); dz[1] = make_float4(0.f, 0.f, 0.f, 0.f); }
+  const Walk wk = make_walk<W>(g, p);
+  each_piece<U>(wk, ch * g.s, [&](int, int64_t off, int m) {
+    float v[U][W], d[U][W];
 #pragma unroll
-        for (int u = 0; u < 2; ++u) {
-          const float h0 = (xv[u].x - mu) * rs, h1 = (xv[u].y - mu) * rs, h2 = (xv[u].z - mu) * rs, h3 = (xv[u].w - mu) * rs;
-          if (act != FB_ACT_IDENTITY) {
-            dz[u].x *= fb_act_grad_z(act, fmaf(h0, ga, be)); dz[u].y *= fb_act_grad_z(act, fmaf(h1, ga, be));
-            dz[u].z *= fb_act_grad_z(act, fmaf(h2, ga, be)); dz[u].w *= fb_act_grad_z(act, fmaf(h3, ga, be));
-          }
-          a1 += (dz[u].x + dz[u].y) + (dz[u].z + dz[u].w);
-          a2 += (dz[u].x * h0 + dz[u].y * h1) + (dz[u].z * h2 + dz[u].w * h3);
-        }
+    for (int u = 0; u < U; ++u)
+      if (u < m) {
+        ld_piece<W>(x + off + u * wk.step, v[u]);
+        ld_piece<W>(dy + off + u * wk.step, d[u]);
       }
-    }
-  } else {
-    for (int64_t i = p; i < n; i += split) {
-      const int64_t base = (i * c + ch) * s;
-      for (int64_t j = threadIdx.x; j < s; j += BN_THREADS) {
-        const float h = (x[base + j] - mu) * rs;
-        const float dz = dy[base + j] * fb_act_grad_z(act, fmaf(h, ga, be));
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      if (u >= m) break;
+#pragma unroll
+      for (int e = 0; e < W; ++e) {
+        const float h = (v[u][e] - mu) * rs;
+        float dz = d[u][e] * dy_scale;
+        if (ACT != 0) dz = fb_act_bwd_k<ACT>(act, fmaf(h, ga, be), dz);
         a1 += dz;
-        a2 += dz * h;
+        a2 = fmaf(dz, h, a2);
       }
     }
-  }
-  a1 = fb_warp_sum(a1);
-  a2 = fb_warp_sum(a2);
-  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-  if (lane == 0) { sh[w] = a1; sh[32 + w] = a2; }
-  __syncthreads();
-  if (w == 0) {
-    float r1 = lane < (BN_THREADS / 32) ? sh[lane] : 0.0f;
-    float r2 = lane < (BN_THREADS / 32) ? sh[32 + lane] : 0.0f;
-    r1 = fb_warp_sum(r1);
-    r2 = fb_warp_sum(r2);
-    if (lane == 0) {
-      part[(ch * split + p) * 2 + 0] = r1;
-      part[(ch * split + p) * 2 + 1] = r2;
+  });
+  if (!channel_sums(ex, a1, a2, g.split, (uint32_t)p, 0) && threadIdx.x == 0) atomicExch(dev_err, 2101);
+  if (p == 0 && threadIdx.x == 0) {
+    if (dbeta) dbeta[ch] = a1;
+    if (dgamma) dgamma[ch] = a2;
+    if (coef) {
+      const float cnt = (float)(g.s * g.n);
+      coef[ch * 2 + 0] = a1 / cnt;
+      coef[ch * 2 + 1] = a2 / cnt;
     }
   }
+  if (g.split > 1) cluster_sync_all();   // (no CTA leaves while another may still send to it)
 }
 
-// coef[c][2] = (sum dz / cnt, sum dz*xhat / cnt); dgamma, dbeta
-__global__ void bn_bwd_finalize_kernel(const float* __restrict__ part, int split, int64_t c, float cnt,
-                                       float* __restrict__ coef, float* __restrict__ dgamma,
-                                       float* __restrict__ dbeta) {
-  const int64_t ch = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (ch >= c) return;
-  float a1 = 0.0f, a2 = 0.0f;
-  for (int p = 0; p < split; ++p) {
-    a1 += part[(ch * split + p) * 2 + 0];
-    a2 += part[(ch * split + p) * 2 + 1];
-  }
-  if (dbeta) dbeta[ch] = a1;
-  if (dgamma) dgamma[ch] = a2;
-  coef[ch * 2 + 0] = a1 / cnt;
-  coef[ch * 2 + 1] = a2 / cnt;
-}
-
-template <bool VEC>
+template <int W, int ACT>
 __global__ void __launch_bounds__(BN_THREADS)
 bn_bwd_apply_kernel(const float* __restrict__ x, const float* __restrict__ dy, const float* __restrict__ gamma,
                     const float* __restrict__ beta, const float* __restrict__ mean, const float* __restrict__ rstd,
-                    const float* __restrict__ coef, float* __restrict__ dx, int64_t s, int64_t c, int64_t total,
-                    int act) {
-  if (VEC) {
-    const int64_t total4 = total >> 2;
-    const float4* x4 = (const float4*)x;
-    const float4* d4 = (const float4*)dy;
-    float4* o4 = (float4*)dx;
-    for (int64_t i = (int64_t)blockIdx.x * BN_THREADS + threadIdx.x; i < total4; i += (int64_t)gridDim.x * BN_THREADS) {
-      const int64_t ch = ((i << 2) / s) % c;
-      const float mu = __ldg(mean + ch), rs = __ldg(rstd + ch);
-      const float ga = gamma ? __ldg(gamma + ch) : 1.0f, be = beta ? __ldg(beta + ch) : 0.0f;
-      const float m1 = __ldg(coef + ch * 2), m2 = __ldg(coef + ch * 2 + 1);
-      const float4 xv = __ldcs(x4 + i);
-      float4 dz = __ldcs(d4 + i);
-      const float h0 = (xv.x - mu) * rs, h1 = (xv.y - mu) * rs, h2 = (xv.z - mu) * rs, h3 = (xv.w - mu) * rs;
-      if (act != FB_ACT_IDENTITY) {
-        dz.x *= fb_act_grad_z(act, fmaf(h0, ga, be)); dz.y *= fb_act_grad_z(act, fmaf(h1, ga, be));
-        dz.z *= fb_act_grad_z(act, fmaf(h2, ga, be)); dz.w *= fb_act_grad_z(act, fmaf(h3, ga, be));
+                    const float* __restrict__ coef, float* __restrict__ dx, int64_t s, int64_t c, int64_t rows, int tpr, int act) {
+  constexpr int U = 2;
+  const int tx = threadIdx.x & (tpr - 1), ty = threadIdx.x / tpr, nr = BN_THREADS / tpr;
+  for (int64_t r = (int64_t)blockIdx.x * nr + ty; r < rows; r += (int64_t)gridDim.x * nr) {
+    const int64_t ch = rows <= 0x7fffffff ? (int64_t)((uint32_t)r % (uint32_t)c) : r % c;
+    const float mu = __ldg(mean + ch), rs = __ldg(rstd + ch);
+    const float ga = gamma ? __ldg(gamma + ch) : 1.0f, be = beta ? __ldg(beta + ch) : 0.0f;
+    const float m1 = __ldg(coef + ch * 2), m2 = __ldg(coef + ch * 2 + 1), k = ga * rs;
+    const int64_t base = r * s;
+    for (int64_t j = (int64_t)tx * W; j < s; j += (int64_t)U * tpr * W) {
+      float v[U][W], d[U][W];
+#pragma unroll
+      for (int u = 0; u < U; ++u) {
+        const int64_t ju = j + (int64_t)u * tpr * W;
+        if (ju < s) {
+          ld_stream<W>(x + base + ju, v[u]);
+          ld_stream<W>(dy + base + ju, d[u]);
+        }
       }
-      const float k = ga * rs;
-      float4 o;
-      o.x = k * (dz.x - m1 - h0 * m2); o.y = k * (dz.y - m1 - h1 * m2);
-      o.z = k * (dz.z - m1 - h2 * m2); o.w = k * (dz.w - m1 - h3 * m2);
-      __stcs(o4 + i, o);
-    }
-  } else {
-    for (int64_t i = (int64_t)blockIdx.x * BN_THREADS + threadIdx.x; i < total; i += (int64_t)gridDim.x * BN_THREADS) {
-      const int64_t ch = (i / s) % c;
-      const float rs = rstd[ch], ga = gamma ? gamma[ch] : 1.0f, be = beta ? beta[ch] : 0.0f;
-      const float h = (x[i] - mean[ch]) * rs;
-      const float dz = dy[i] * fb_act_grad_z(act, fmaf(h, ga, be));
-      dx[i] = ga * rs * (dz - coef[ch * 2] - h * coef[ch * 2 + 1]);
+#pragma unroll
+      for (int u = 0; u < U; ++u) {
+        const int64_t ju = j + (int64_t)u * tpr * W;
+        if (ju >= s) break;
+        float o[W];
+#pragma unroll
+        for (int e = 0; e < W; ++e) {
+          const float h = (v[u][e] - mu) * rs;
+          const float dz = ACT == 0 ? d[u][e] : fb_act_bwd_k<ACT>(act, fmaf(h, ga, be), d[u][e]);
+          o[e] = k * (dz - m1 - h * m2);
+        }
+        st_stream<W>(dx + base + ju, o);
+      }
     }
   }
 }
 
-int bn_pick_split(const fb_ctx* ctx, int64_t c, int64_t n) {
-  int64_t target = (int64_t)ctx->sm_count * 8;
-  int64_t split = (target + c - 1) / c;
-  if (split < 1) split = 1;
-  if (split > n) split = n;
-  if (split > 65535) split = 65535;
-  return (int)split;
+// ------------------------------------------------------------------------------------ launches ---
+int bn_tpr(int64_t pieces, int nt) {
+  int t = 1;
+  while (t < nt && t < pieces) t *= 2;
+  return t;
+}
+// More CTAs per channel while the GPU has room for blocks and a block has four rows for each of its threads.
+Dims bn_dims(const fb_ctx* ctx, int64_t s, int64_t c, int64_t n, int W, int nt, int64_t blocks) {
+  Dims g = {s, c, n, 1, bn_tpr(s / W, nt)};
+  while (g.split < BN_MAX_CLUSTER && c * g.split < blocks * ctx->sm_count && n >= 8 * (int64_t)g.split * (nt / g.tpr)) g.split *= 2;
+  return g;
 }
 
-unsigned bn_elem_grid(const fb_ctx* ctx, int64_t work_items) {
-  int64_t blocks = (work_items + BN_THREADS - 1) / BN_THREADS;
-  const int64_t cap = (int64_t)ctx->sm_count * 32;
-  if (blocks > cap) blocks = cap;
-  if (blocks < 1) blocks = 1;
-  return (unsigned)blocks;
+// A launch of so many clusters of g.split CTAs
+template <typename K, typename... A>
+int32_t bn_launch(K kern, cudaStream_t stream, const Dims& g, int64_t clusters, int nt, size_t smem, A... args) {
+  FB_REQUIRE(clusters * g.split <= 0x7fffffff, FB_ERR_SHAPE, "batchnorm: too many channels");
+  if (smem > 48 * 1024) FB_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  cudaLaunchConfig_t lc;
+  memset(&lc, 0, sizeof(lc));
+  lc.gridDim = dim3((unsigned)(clusters * g.split), 1, 1);
+  lc.blockDim = dim3((unsigned)nt, 1, 1);
+  lc.dynamicSmemBytes = smem;
+  lc.stream = stream;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = (unsigned)g.split;
+  attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+  lc.attrs = attr;
+  lc.numAttrs = 1;
+  FB_CUDA(cudaLaunchKernelEx(&lc, kern, args...));
+  FB_LAUNCH_CHECK();
+  return FB_OK;
 }
 
-unsigned bn_row_grid(const fb_ctx* ctx, int64_t rows) {
-  int64_t blocks = (rows + 1) / 2;
+unsigned bn_row_grid(const fb_ctx* ctx, int64_t rows, int tpr) {
+  const int64_t nr = BN_THREADS / tpr;
+  int64_t blocks = (rows + 2 * nr - 1) / (2 * nr);
   const int64_t cap = (int64_t)ctx->sm_count * 16;
   if (blocks > cap) blocks = cap;
   if (blocks < 1) blocks = 1;
   return (unsigned)blocks;
+}
+
+// f(W, activation kind) as compile-time constants
+template <typename F>
+auto bn_kind(bool vec, int act, F f) {
+  return fb_act_kind(act, [&](auto k) {
+    return vec ? f(std::integral_constant<int, 4>(), k) : f(std::integral_constant<int, 1>(), k);
+  });
+}
+
+template <bool VAR>
+int32_t bn_apply(fb_ctx* ctx, cudaStream_t stream, bool vec, const float* x, const float* gamma, const float* beta, const float* mean,
+                 const float* rstd, float eps, float* y, int64_t s, int64_t c, int64_t n, int act) {
+  if (s < 128 && s * c * n <= 0x7fffffff && fb_aligned16(x) && fb_aligned16(y)) {
+    const int64_t pieces = (s * c * n + 3) / 4, per = 2 * BN_THREADS, blocks = (pieces + per - 1) / per, cap = (int64_t)ctx->sm_count * 16;
+    fb_act_kind(act, [&](auto k) {
+      bn_apply_flat_kernel<VAR, k.value><<<(unsigned)(blocks < cap ? blocks : cap), BN_THREADS, 0, stream>>>(
+          x, gamma, beta, mean, rstd, eps, y, fast_div((uint32_t)s), fast_div((uint32_t)c), (uint32_t)(s * c * n), act);
+    });
+    FB_LAUNCH_CHECK();
+    return FB_OK;
+  }
+  const int tpr = bn_tpr(vec ? s / 4 : s, BN_THREADS);
+  bn_kind(vec, act, [&](auto W, auto k) {
+    const int64_t chunk = bn_chunk(BN_THREADS / tpr), blocks = (c * n + chunk - 1) / chunk, cap = (int64_t)ctx->sm_count * 32;
+    bn_apply_kernel<W.value, VAR, k.value><<<(unsigned)(blocks < cap ? blocks : cap), BN_THREADS, 0, stream>>>(x, gamma, beta, mean, rstd, eps, y, s, c, c * n, tpr, act);
+  });
+  FB_LAUNCH_CHECK();
+  return FB_OK;
+}
+
+// y = act(BatchNorm(x)) with batch statistics, which are saved; running statistics are updated where given
+int32_t bn_fwd_batch(fb_ctx* ctx, cudaStream_t stream, const float* x, const float* gamma, const float* beta, float* running_mean,
+                     float* running_var, float* y, float* save_mean, float* save_rstd, int64_t s, int64_t c, int64_t n, float eps,
+                     float momentum, int act) {
+  const bool vec = (s % 4 == 0) && fb_aligned16(x) && fb_aligned16(y);
+  const int W = vec ? 4 : 1;
+  // few values per channel: smaller blocks
+  const int nt = s * n > 2048 * W ? BN_FWD_THREADS : BN_THREADS;
+  Dims g = {s, c, n, 1, bn_tpr(s / W, nt)};
+  auto bytes = [&] {
+    const int64_t rows = (int64_t)g.split * (nt / g.tpr);
+    return (size_t)((n + rows - 1) / rows * ((s / W + g.tpr - 1) / g.tpr)) * nt * W * sizeof(float);
+  };
+  int lg = 0;
+  // two channels at least in a CTA's shared memory, and every SM with a CTA
+  while (g.split < BN_MAX_CLUSTER && (2 * bytes() > BN_CACHE_MAX || (c * g.split < ctx->sm_count && n >= 8 * (int64_t)g.split * (nt / g.tpr)))) {
+    g.split *= 2;
+    ++lg;
+  }
+  const size_t slab = bytes();
+  if (slab <= BN_CACHE_MAX) {
+    const int64_t resident = ctx->clusters[lg] > 0 ? ctx->clusters[lg] : 1, clusters = c < resident ? c : resident;
+    const int64_t rounds = (c + clusters - 1) / clusters;
+    int depth = (int)(BN_CACHE_MAX / slab);
+    depth = depth > 3 ? 3 : depth;
+    depth = depth > rounds ? (int)rounds : depth;
+    return bn_kind(vec, act, [&](auto w, auto k) {
+      return bn_launch(bn_fwd_kernel<w.value, k.value>, stream, g, clusters, nt, slab * depth, x, gamma, beta, y, g, depth, (int)(slab / sizeof(float)), eps,
+                       momentum, save_mean, save_rstd, running_mean, running_var, act, ctx->dev_error);
+    });
+  }
+  g = bn_dims(ctx, s, c, n, W, BN_THREADS, 12);
+  const int32_t st = bn_kind(vec, FB_ACT_IDENTITY, [&](auto w, auto) {
+    return bn_launch(bn_stats_kernel<w.value>, stream, g, c, BN_THREADS, 0, x, g, eps, momentum, save_mean, save_rstd, running_mean, running_var,
+                     ctx->dev_error);
+  });
+  return st != FB_OK ? st : bn_apply<false>(ctx, stream, vec, x, gamma, beta, save_mean, save_rstd, eps, y, s, c, n, act);
+}
+
+int32_t bn_bwd_sums(fb_ctx* ctx, cudaStream_t stream, bool vec, const float* x, const float* dy, float dy_scale, const float* gamma,
+                    const float* beta, const float* mean, const float* rstd, float* coef, float* dgamma, float* dbeta, int64_t s,
+                    int64_t c, int64_t n, int act) {
+  const Dims g = bn_dims(ctx, s, c, n, vec ? 4 : 1, BN_THREADS, 12);
+  return bn_kind(vec, act, [&](auto w, auto k) {
+    return bn_launch(bn_bwd_sums_kernel<w.value, k.value>, stream, g, c, BN_THREADS, 0, x, dy, dy_scale, gamma, beta, mean, rstd, g, coef, dgamma, dbeta, act, ctx->dev_error);
+  });
 }
 
 int32_t bn_check(const char* fn, int64_t s, int64_t c, int64_t n, int act) {
@@ -399,25 +628,9 @@ FB_API int32_t fb_batchnorm_fwd_train(fb_ctx* ctx, void* stream_, const float* x
              (long long)(s * n));
   FB_REQUIRE(x && y && save_mean && save_rstd, FB_ERR_INVALID_ARG, "fb_batchnorm_fwd_train: NULL pointer");
   FB_REQUIRE((running_mean == nullptr) == (running_var == nullptr), FB_ERR_INVALID_ARG, "fb_batchnorm_fwd_train: running_mean and running_var must both be given or both NULL");
-  const int split = bn_pick_split(ctx, c, n);
-  float* part = (float*)fb_scratch(ctx, stream, (size_t)c * split * 3 * sizeof(float));
-  if (!part) return FB_ERR_ALLOC;
-  const bool vec = (s % 4 == 0) && fb_aligned16(x) && fb_aligned16(y);
-  dim3 grid((unsigned)c, (unsigned)split);
-  if (vec) bn_stats_kernel<true><<<grid, BN_THREADS, 0, stream>>>(x, part, s, c, n);
-  else bn_stats_kernel<false><<<grid, BN_THREADS, 0, stream>>>(x, part, s, c, n);
-  FB_LAUNCH_CHECK();
   const bool upd = track_stats != 0 && running_mean != nullptr;
-  bn_stats_finalize_kernel<<<(unsigned)((c + 127) / 128), 128, 0, stream>>>(part, split, c, eps, momentum, save_mean,
-                                                                           save_rstd, upd ? running_mean : nullptr,
-                                                                           upd ? running_var : nullptr);
-  FB_LAUNCH_CHECK();
-  const int64_t total = s * c * n;
-  if (vec && s >= 128) bn_apply_rows_kernel<<<bn_row_grid(ctx, c * n), BN_THREADS, 0, stream>>>((const float4*)x, gamma, beta, save_mean, save_rstd, (float4*)y, s / 4, c, c * n, act);
-  else if (vec) bn_apply_kernel<true><<<bn_elem_grid(ctx, total / 4), BN_THREADS, 0, stream>>>(x, gamma, beta, save_mean, save_rstd, y, s, c, total, act);
-  else bn_apply_kernel<false><<<bn_elem_grid(ctx, total), BN_THREADS, 0, stream>>>(x, gamma, beta, save_mean, save_rstd, y, s, c, total, act);
-  FB_LAUNCH_CHECK();
-  return FB_OK;
+  return bn_fwd_batch(ctx, stream, x, gamma, beta, upd ? running_mean : nullptr, upd ? running_var : nullptr, y, save_mean, save_rstd, s,
+                      c, n, eps, momentum, act);
 }
 
 FB_API int32_t fb_batchnorm_fwd_infer(fb_ctx* ctx, void* stream_, const float* x, const float* gamma,
@@ -430,29 +643,13 @@ FB_API int32_t fb_batchnorm_fwd_infer(fb_ctx* ctx, void* stream_, const float* x
   FB_REQUIRE((gamma == nullptr) == (beta == nullptr), FB_ERR_INVALID_ARG, "fb_batchnorm_fwd_infer: gamma and beta must both be given or both NULL");
   if (n == 0) return FB_OK;
   FB_REQUIRE(x && y, FB_ERR_INVALID_ARG, "fb_batchnorm_fwd_infer: NULL pointer");
-  const int split = bn_pick_split(ctx, c, n);
-  float* ws = (float*)fb_scratch(ctx, stream, (size_t)c * (split * 3 + 2) * sizeof(float));
-  if (!ws) return FB_ERR_ALLOC;
-  float* mean = ws;
-  float* rstd = ws + c;
-  float* part = ws + 2 * c;
-  const bool vec = (s % 4 == 0) && fb_aligned16(x) && fb_aligned16(y);
   if (running_mean != nullptr && running_var != nullptr) {
-    bn_infer_prepare_kernel<<<(unsigned)((c + 127) / 128), 128, 0, stream>>>(running_mean, running_var, eps, c, mean, rstd);
-  } else {
-    dim3 grid((unsigned)c, (unsigned)split);
-    if (vec) bn_stats_kernel<true><<<grid, BN_THREADS, 0, stream>>>(x, part, s, c, n);
-    else bn_stats_kernel<false><<<grid, BN_THREADS, 0, stream>>>(x, part, s, c, n);
-    FB_LAUNCH_CHECK();
-    bn_stats_finalize_kernel<<<(unsigned)((c + 127) / 128), 128, 0, stream>>>(part, split, c, eps, 0.0f, mean, rstd, nullptr, nullptr);
+    const bool vec = (s % 4 == 0) && fb_aligned16(x) && fb_aligned16(y);
+    return bn_apply<true>(ctx, stream, vec, x, gamma, beta, running_mean, running_var, eps, y, s, c, n, act);
   }
-  FB_LAUNCH_CHECK();
-  const int64_t total = s * c * n;
-  if (vec && s >= 128) bn_apply_rows_kernel<<<bn_row_grid(ctx, c * n), BN_THREADS, 0, stream>>>((const float4*)x, gamma, beta, mean, rstd, (float4*)y, s / 4, c, c * n, act);
-  else if (vec) bn_apply_kernel<true><<<bn_elem_grid(ctx, total / 4), BN_THREADS, 0, stream>>>(x, gamma, beta, mean, rstd, y, s, c, total, act);
-  else bn_apply_kernel<false><<<bn_elem_grid(ctx, total), BN_THREADS, 0, stream>>>(x, gamma, beta, mean, rstd, y, s, c, total, act);
-  FB_LAUNCH_CHECK();
-  return FB_OK;
+  float* ws = (float*)fb_scratch(ctx, stream, (size_t)c * 2 * sizeof(float));
+  if (!ws) return FB_ERR_ALLOC;
+  return bn_fwd_batch(ctx, stream, x, gamma, beta, nullptr, nullptr, y, ws, ws + c, s, c, n, eps, 0.0f, act);
 }
 
 FB_API int32_t fb_batchnorm_bwd(fb_ctx* ctx, void* stream_, const float* x, const float* gamma,
@@ -466,22 +663,28 @@ FB_API int32_t fb_batchnorm_bwd(fb_ctx* ctx, void* stream_, const float* x, cons
   FB_REQUIRE((gamma == nullptr) == (beta == nullptr), FB_ERR_INVALID_ARG, "fb_batchnorm_bwd: gamma and beta must both be given or both NULL");
   FB_REQUIRE(n >= 1, FB_ERR_SHAPE, "fb_batchnorm_bwd: empty batch");
   FB_REQUIRE(x && save_mean && save_rstd && dy && dx, FB_ERR_INVALID_ARG, "fb_batchnorm_bwd: NULL pointer");
-  const int split = bn_pick_split(ctx, c, n);
-  float* ws = (float*)fb_scratch(ctx, stream, (size_t)c * (split * 2 + 2) * sizeof(float));
-  if (!ws) return FB_ERR_ALLOC;
-  float* coef = ws;
-  float* part = ws + 2 * c;
+  float* coef = (float*)fb_scratch(ctx, stream, (size_t)c * 2 * sizeof(float));
+  if (!coef) return FB_ERR_ALLOC;
   const bool vec = (s % 4 == 0) && fb_aligned16(x) && fb_aligned16(dy) && fb_aligned16(dx);
-  dim3 grid((unsigned)c, (unsigned)split);
-  if (vec) bn_bwd_reduce_kernel<true><<<grid, BN_THREADS, 0, stream>>>(x, dy, gamma, beta, save_mean, save_rstd, part, s, c, n, act);
-  else bn_bwd_reduce_kernel<false><<<grid, BN_THREADS, 0, stream>>>(x, dy, gamma, beta, save_mean, save_rstd, part, s, c, n, act);
-  FB_LAUNCH_CHECK();
-  bn_bwd_finalize_kernel<<<(unsigned)((c + 127) / 128), 128, 0, stream>>>(part, split, c, (float)(s * n), coef, dgamma, dbeta);
-  FB_LAUNCH_CHECK();
-  const int64_t total = s * c * n;
-  if (vec && s >= 128) bn_bwd_apply_rows_kernel<<<bn_row_grid(ctx, c * n), BN_THREADS, 0, stream>>>((const float4*)x, (const float4*)dy, gamma, beta, save_mean, save_rstd, coef, (float4*)dx, s / 4, c, c * n, act);
-  else if (vec) bn_bwd_apply_kernel<true><<<bn_elem_grid(ctx, total / 4), BN_THREADS, 0, stream>>>(x, dy, gamma, beta, save_mean, save_rstd, coef, dx, s, c, total, act);
-  else bn_bwd_apply_kernel<false><<<bn_elem_grid(ctx, total), BN_THREADS, 0, stream>>>(x, dy, gamma, beta, save_mean, save_rstd, coef, dx, s, c, total, act);
+  st = bn_bwd_sums(ctx, stream, vec, x, dy, 1.0f, gamma, beta, save_mean, save_rstd, coef, dgamma, dbeta, s, c, n, act);
+  if (st != FB_OK) return st;
+  const int tpr = bn_tpr(vec ? s / 4 : s, BN_THREADS);
+  bn_kind(vec, act, [&](auto w, auto k) {
+    bn_bwd_apply_kernel<w.value, k.value><<<bn_row_grid(ctx, c * n, tpr), BN_THREADS, 0, stream>>>(x, dy, gamma, beta, save_mean, save_rstd, coef, dx, s, c, c * n, tpr, act);
+  });
   FB_LAUNCH_CHECK();
   return FB_OK;
+}
+
+FB_API int32_t fb_batchnorm_bwd_params(fb_ctx* ctx, void* stream_, const float* x, const float* gamma, const float* beta,
+                                       const float* save_mean, const float* save_rstd, const float* dy, float dy_scale,
+                                       float* dgamma, float* dbeta, int64_t s, int64_t c, int64_t n, int32_t act) {
+  FB_CHECK_CTX(ctx);
+  int32_t st = bn_check("fb_batchnorm_bwd_params", s, c, n, act);
+  if (st != FB_OK) return st;
+  FB_REQUIRE((gamma == nullptr) == (beta == nullptr), FB_ERR_INVALID_ARG, "fb_batchnorm_bwd_params: gamma and beta must both be given or both NULL");
+  FB_REQUIRE(n >= 1, FB_ERR_SHAPE, "fb_batchnorm_bwd_params: empty batch");
+  FB_REQUIRE(x && save_mean && save_rstd && dy && dgamma && dbeta, FB_ERR_INVALID_ARG, "fb_batchnorm_bwd_params: NULL pointer");
+  const bool vec = (s % 4 == 0) && fb_aligned16(x) && fb_aligned16(dy);
+  return bn_bwd_sums(ctx, (cudaStream_t)stream_, vec, x, dy, dy_scale, gamma, beta, save_mean, save_rstd, nullptr, dgamma, dbeta, s, c, n, act);
 }

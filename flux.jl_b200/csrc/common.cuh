@@ -6,6 +6,8 @@
 #include <stdio.h>
 #include <string.h>
 
+#include <type_traits>
+
 #include "../../include/fluxb200.h"
 
 #define FB_API extern "C" __attribute__((visibility("default")))
@@ -132,6 +134,24 @@ __device__ __forceinline__ float fb_act_grad_y(int act, float y) {
     case FB_ACT_SIGMOID: return y * (1.0f - y);
     default: return 1.0f;
   }
+}
+
+// Kernels that unroll over many elements take the activation's kind as a template argument: none, relu, or any (whose code per
+// element is long enough to cost registers and instruction fetches even where it is not executed).
+template <int KIND>
+__device__ __forceinline__ float fb_act_apply_k(int act, float z) {
+  return KIND == 0 ? z : KIND == 1 ? fmaxf(z, 0.0f) : fb_act_apply(act, z);
+}
+// d * act'(z)
+template <int KIND>
+__device__ __forceinline__ float fb_act_bwd_k(int act, float z, float d) {
+  return KIND == 0 ? d : KIND == 1 ? (z > 0.0f ? d : d * 0.0f) : d * fb_act_grad_z(act, z);
+}
+template <typename F>
+static inline auto fb_act_kind(int act, F f) {
+  if (act == FB_ACT_IDENTITY) return f(std::integral_constant<int, 0>());
+  if (act == FB_ACT_RELU) return f(std::integral_constant<int, 1>());
+  return f(std::integral_constant<int, 2>());
 }
 
 static inline bool fb_act_valid(int act) { return act >= FB_ACT_IDENTITY && act <= FB_ACT_GELU_ERF; }

@@ -4,6 +4,10 @@
 // row.  Forward: one read of x, one write of y (the row lives in registers between the two reductions).
 // Backward: one read each of x and dy, one write of dx; dgamma / dbeta are accumulated per thread in
 // registers across the rows a block owns and reduced in a second, small kernel from per-block partials.
+// Where only dgamma / dbeta are wanted the backward pass is a sum over columns and needs no row sums at all.
+//
+// Rows of up to 1024 features belong to one warp each (no block barriers, every load of a row in flight at once), longer ones to
+// a block.  Rows that are no whole number of aligned float4 are read float by float, up to 8192 features in registers too.
 #include "common.cuh"
 
 namespace {
@@ -83,6 +87,254 @@ ln_fwd_vec_kernel(const float4* __restrict__ x, const float4* __restrict__ gamma
         st_stream(yr + c, o);
       }
     }
+  }
+}
+
+// ------------------------------------------------- rows in registers, any alignment ---
+// T threads per row (a warp, or the block of 256), V pieces of W = VEC ? 4 : 1 floats each.  Bound: HBM and the latency of a row's
+// loads and sums.  Forward, from a cold cache: 1001 features x 3000 rows 16 -> 13 us (a block per row that read it three times),
+// 1024 x 16384 34 -> 24, 64 x 16384 24 -> 4 (a block per row of 16 pieces), 8191 x 2000 55 -> 37.
+template <int W>
+__device__ __forceinline__ void ld_piece(const float* p, float* v) {
+  if (W == 4) {
+    const float4 q = *(const float4*)p;
+    v[0] = q.x; v[1] = q.y; v[2] = q.z; v[3] = q.w;
+  } else {
+    v[0] = *p;
+  }
+}
+template <int W>
+__device__ __forceinline__ void st_piece(float* p, const float* v) {
+  if (W == 4) *(float4*)p = make_float4(v[0], v[1], v[2], v[3]);
+  else *p = v[0];
+}
+template <int T>
+__device__ __forceinline__ float row_sum(float v, float* sh) {
+  return T == 32 ? fb_warp_sum(v) : fb_block_sum(v, sh);
+}
+
+template <int V, int T, bool VEC, int ACT>
+__global__ void __launch_bounds__(LN_THREADS)
+ln_fwd_rows_kernel(const float* __restrict__ x, const float* __restrict__ gamma, const float* __restrict__ beta,
+                   float* __restrict__ y, float* __restrict__ mean, float* __restrict__ rstd, int d, int64_t n, float eps, int act) {
+  constexpr int W = VEC ? 4 : 1;
+  __shared__ float sh[64];
+  const int t = threadIdx.x % T;
+  const float inv_d = 1.0f / (float)d;
+  for (int64_t row = (int64_t)blockIdx.x * (LN_THREADS / T) + threadIdx.x / T; row < n; row += (int64_t)gridDim.x * (LN_THREADS / T)) {
+    const float* xr = x + row * d;
+    float v[V][W];
+    float s = 0.0f;
+#pragma unroll
+    for (int i = 0; i < V; ++i) {
+      const int c = (t + i * T) * W;
+      if (c < d) ld_piece<W>(xr + c, v[i]);
+    }
+#pragma unroll
+    for (int i = 0; i < V; ++i)
+      if ((t + i * T) * W < d)
+#pragma unroll
+        for (int e = 0; e < W; ++e) s += v[i][e];
+    const float mu = row_sum<T>(s, sh) * inv_d;
+    float q = 0.0f;
+#pragma unroll
+    for (int i = 0; i < V; ++i)
+      if ((t + i * T) * W < d)
+#pragma unroll
+        for (int e = 0; e < W; ++e) { const float a = v[i][e] - mu; q = fmaf(a, a, q); }
+    const float rs = rsqrtf(row_sum<T>(q, sh) * inv_d + eps);
+    if (t == 0) {
+      mean[row] = mu;
+      rstd[row] = rs;
+    }
+    float* yr = y + row * d;
+    constexpr int B = V < 8 ? V : 8;   // pieces whose gamma and beta are loaded together
+#pragma unroll
+    for (int i0 = 0; i0 < V; i0 += B) {
+      float g[B][W], b[B][W];
+      if (gamma != nullptr) {
+#pragma unroll
+        for (int k = 0; k < B; ++k) {
+          const int c = (t + (i0 + k) * T) * W;
+          if (c < d) {
+            ld_piece<W>(gamma + c, g[k]);
+            ld_piece<W>(beta + c, b[k]);
+          }
+        }
+      }
+#pragma unroll
+      for (int k = 0; k < B; ++k) {
+        const int c = (t + (i0 + k) * T) * W;
+        float o[W];
+#pragma unroll
+        for (int e = 0; e < W; ++e) {
+          o[e] = (v[i0 + k][e] - mu) * rs;
+          if (gamma != nullptr) o[e] = fmaf(o[e], g[k][e], b[k][e]);
+          o[e] = fb_act_apply_k<ACT>(act, o[e]);
+        }
+        if (c < d) st_piece<W>(yr + c, o);
+      }
+    }
+  }
+}
+
+// Backward with dx.  A block's partial dgamma / dbeta: every thread's columns summed over its rows, then (T = 32) over the eight
+// warps.  With the second kernel: 1001 features x 3000 rows 60 -> 42 us, 64 x 16384 58 -> 17, 3001 x 3000 163 -> 54, 8191 x 2000 331
+// -> 114 (partials in global memory, rows read twice before).
+template <int V, int T, bool VEC, int ACT>
+__global__ void __launch_bounds__(LN_THREADS)
+ln_bwd_rows_kernel(const float* __restrict__ x, const float* __restrict__ gamma, const float* __restrict__ beta,
+                   const float* __restrict__ mean, const float* __restrict__ rstd, const float* __restrict__ dy, float* __restrict__ dx,
+                   float* __restrict__ part_dg, float* __restrict__ part_db, int d, int64_t n, int act) {
+  constexpr int W = VEC ? 4 : 1;
+  __shared__ float sh[64];
+  __shared__ float red[T == 32 ? 8 * V * W * 32 : 1];
+  const int t = threadIdx.x % T, w = threadIdx.x / T;
+  const float inv_d = 1.0f / (float)d;
+  float ag[V][W], ab[V][W];
+#pragma unroll
+  for (int i = 0; i < V; ++i)
+#pragma unroll
+    for (int e = 0; e < W; ++e) ag[i][e] = ab[i][e] = 0.0f;
+  for (int64_t row = (int64_t)blockIdx.x * (LN_THREADS / T) + w; row < n; row += (int64_t)gridDim.x * (LN_THREADS / T)) {
+    const float mu = __ldg(mean + row), rs = __ldg(rstd + row);
+    const float* xr = x + row * d;
+    const float* dyr = dy + row * d;
+    float xh[V][W], g[V][W];
+#pragma unroll
+    for (int i = 0; i < V; ++i) {
+      const int c = (t + i * T) * W;
+      if (c < d) {
+        ld_piece<W>(xr + c, xh[i]);
+        ld_piece<W>(dyr + c, g[i]);
+      }
+    }
+    float s1 = 0.0f, s2 = 0.0f;
+#pragma unroll
+    for (int i = 0; i < V; ++i) {
+      const int c = (t + i * T) * W;
+      if (c < d) {
+        float ga[W], be[W];
+        if (gamma != nullptr) {
+          ld_piece<W>(gamma + c, ga);
+          if (ACT != 0) ld_piece<W>(beta + c, be);
+        }
+#pragma unroll
+        for (int e = 0; e < W; ++e) {
+          if (gamma == nullptr) { ga[e] = 1.0f; be[e] = 0.0f; }
+          const float h = (xh[i][e] - mu) * rs;
+          const float dz = ACT == 0 ? g[i][e] : fb_act_bwd_k<ACT>(act, fmaf(h, ga[e], be[e]), g[i][e]);
+          ag[i][e] = fmaf(dz, h, ag[i][e]);
+          ab[i][e] += dz;
+          xh[i][e] = h;
+          g[i][e] = dz * ga[e];
+          s1 += g[i][e];
+          s2 = fmaf(g[i][e], h, s2);
+        }
+      }
+    }
+    if (T == 32) {
+      s1 = fb_warp_sum(s1);
+      s2 = fb_warp_sum(s2);
+    } else {
+      block_sum2(s1, s2, sh);
+    }
+    const float m1 = s1 * inv_d, m2 = s2 * inv_d;
+    float* dxr = dx + row * d;
+#pragma unroll
+    for (int i = 0; i < V; ++i) {
+      const int c = (t + i * T) * W;
+      if (c < d) {
+        float o[W];
+#pragma unroll
+        for (int e = 0; e < W; ++e) o[e] = rs * (g[i][e] - m1 - xh[i][e] * m2);
+        st_piece<W>(dxr + c, o);
+      }
+    }
+  }
+  if (part_dg == nullptr) return;
+  float* pg = part_dg + (int64_t)blockIdx.x * d;
+  float* pb = part_db + (int64_t)blockIdx.x * d;
+  if (T != 32) {
+#pragma unroll
+    for (int i = 0; i < V; ++i) {
+      const int c = (t + i * T) * W;
+      if (c < d) {
+        st_piece<W>(pg + c, ag[i]);
+        st_piece<W>(pb + c, ab[i]);
+      }
+    }
+    return;
+  }
+#pragma unroll
+  for (int k = 0; k < 2; ++k) {
+    __syncthreads();
+#pragma unroll
+    for (int i = 0; i < V; ++i) st_piece<W>(red + w * (V * W * 32) + (t + i * 32) * W, k == 0 ? ag[i] : ab[i]);
+    __syncthreads();
+    for (int c = threadIdx.x; c < d; c += LN_THREADS) {
+      float a = 0.0f;
+#pragma unroll
+      for (int r = 0; r < 8; ++r) a += red[r * (V * W * 32) + c];
+      (k == 0 ? pg : pb)[c] = a;
+    }
+  }
+}
+
+// Only dgamma / dbeta: lx lanes side by side cover lx * W columns, 256 / lx rows at a time; grid (column blocks, row groups).
+// dy counts dy_scale times.  Bound: one read of x and dy (1024 x 16384: 77 us with a dx, 38; 1001 x 3000: 60 and 17).
+template <bool VEC, int ACT>
+__global__ void __launch_bounds__(LN_THREADS)
+ln_bwd_params_kernel(const float* __restrict__ x, const float* __restrict__ gamma, const float* __restrict__ beta,
+                     const float* __restrict__ mean, const float* __restrict__ rstd, const float* __restrict__ dy, float dy_scale,
+                     float* __restrict__ part_dg, float* __restrict__ part_db, int64_t d, int64_t n, int act, int lx) {
+  constexpr int W = VEC ? 4 : 1, U = 4;
+  __shared__ float sa[LN_THREADS * W], sb[LN_THREADS * W];
+  const int tx = threadIdx.x & (lx - 1), ty = threadIdx.x / lx, ny = LN_THREADS / lx;
+  const int64_t c = ((int64_t)blockIdx.x * lx + tx) * W;
+  float ag[W], ab[W], ga[W], be[W];
+#pragma unroll
+  for (int e = 0; e < W; ++e) { ag[e] = ab[e] = be[e] = 0.0f; ga[e] = 1.0f; }
+  if (c < d) {
+    if (ACT != 0 && gamma != nullptr) {
+      ld_piece<W>(gamma + c, ga);
+      ld_piece<W>(beta + c, be);
+    }
+    const int64_t step = (int64_t)gridDim.y * ny;
+    for (int64_t row = (int64_t)blockIdx.y * ny + ty; row < n; row += U * step) {
+      float xv[U][W], dv[U][W], mu[U], rs[U];
+#pragma unroll
+      for (int u = 0; u < U; ++u) {
+        const int64_t r = row + u * step;
+        const int64_t rr = r < n ? r : row;
+        mu[u] = __ldg(mean + rr);
+        rs[u] = __ldg(rstd + rr);
+        ld_piece<W>(x + rr * d + c, xv[u]);
+        ld_piece<W>(dy + rr * d + c, dv[u]);
+      }
+#pragma unroll
+      for (int u = 0; u < U; ++u)
+#pragma unroll
+        for (int e = 0; e < W; ++e) {
+          if (row + u * step >= n) continue;
+          const float h = (xv[u][e] - mu[u]) * rs[u];
+          float dz = dv[u][e] * dy_scale;
+          if (ACT != 0) dz = fb_act_bwd_k<ACT>(act, fmaf(h, ga[e], be[e]), dz);
+          ag[e] = fmaf(dz, h, ag[e]);
+          ab[e] += dz;
+        }
+    }
+  }
+#pragma unroll
+  for (int e = 0; e < W; ++e) { sa[threadIdx.x * W + e] = ag[e]; sb[threadIdx.x * W + e] = ab[e]; }
+  __syncthreads();
+  for (int k = threadIdx.x; k < lx * W; k += LN_THREADS) {
+    const int64_t col = (int64_t)blockIdx.x * lx * W + k;
+    if (col >= d) break;
+    float a = 0.0f, b = 0.0f;
+    for (int r = 0; r < ny; ++r) { a += sa[r * lx * W + k]; b += sb[r * lx * W + k]; }
+    part_dg[(int64_t)blockIdx.y * d + col] = a;
+    part_db[(int64_t)blockIdx.y * d + col] = b;
   }
 }
 
@@ -380,9 +632,34 @@ fb_colreduce2_kernel(const float* __restrict__ part_a, const float* __restrict__
   }
 }
 
+// f(V, T, VEC) as compile-time constants for the kernels that hold rows of d features in registers; false: none does.  Aligned
+// rows of more than 1024 features keep the kernels above, whose rows stream past L2.
+template <typename F>
+static bool ln_rows_dispatch(int64_t d, bool vec, F f) {
+  using std::integral_constant;
+  using std::true_type;
+  using std::false_type;
+  if (vec) {
+    if (d <= 128) f(integral_constant<int, 1>(), integral_constant<int, 32>(), true_type());
+    else if (d <= 256) f(integral_constant<int, 2>(), integral_constant<int, 32>(), true_type());
+    else if (d <= 512) f(integral_constant<int, 4>(), integral_constant<int, 32>(), true_type());
+    else if (d <= 1024) f(integral_constant<int, 8>(), integral_constant<int, 32>(), true_type());
+    else return false;
+    return true;
+  }
+  if (d <= 128) f(integral_constant<int, 4>(), integral_constant<int, 32>(), false_type());
+  else if (d <= 256) f(integral_constant<int, 8>(), integral_constant<int, 32>(), false_type());
+  else if (d <= 512) f(integral_constant<int, 16>(), integral_constant<int, 32>(), false_type());
+  else if (d <= 1024) f(integral_constant<int, 32>(), integral_constant<int, 32>(), false_type());
+  else if (d <= 2048) f(integral_constant<int, 8>(), integral_constant<int, 256>(), false_type());
+  else if (d <= 4096) f(integral_constant<int, 16>(), integral_constant<int, 256>(), false_type());
+  else if (d <= 8192) f(integral_constant<int, 32>(), integral_constant<int, 256>(), false_type());
+  else return false;
+  return true;
+}
+
 static int ln_pick_v(int64_t d4) {
   const int64_t per = (d4 + LN_THREADS - 1) / LN_THREADS;
-  if (per <= 1) return 1;
   if (per <= 2) return 2;
   if (per <= 4) return 4;
   if (per <= 8) return 8;
@@ -402,7 +679,15 @@ FB_API int32_t fb_layernorm_fwd(fb_ctx* ctx, void* stream_, const float* x, cons
   const bool vec = (d % 4 == 0) && fb_aligned16(x) && fb_aligned16(y) && (!gamma || (fb_aligned16(gamma) && fb_aligned16(beta)));
   const int v = vec ? ln_pick_v(d / 4) : 0;
   const unsigned grid = (unsigned)(n < (int64_t)ctx->sm_count * 64 ? n : (int64_t)ctx->sm_count * 64);
-  if (v == 0) {
+  const bool rows = ln_rows_dispatch(d, vec, [&](auto V, auto T, auto vc) {
+    const int64_t per = LN_THREADS / T.value, blocks = (n + per - 1) / per;
+    fb_act_kind(act, [&](auto k) {
+      ln_fwd_rows_kernel<V.value, T.value, vc.value, k.value><<<(unsigned)(blocks < 0x7fffffff ? blocks : 0x7fffffff), LN_THREADS, 0, stream>>>(
+          x, gamma, beta, y, mean, rstd, (int)d, n, eps, act);
+    });
+  });
+  if (rows) {
+  } else if (v == 0) {
     ln_fwd_generic_kernel<<<grid, LN_THREADS, 0, stream>>>(x, gamma, beta, y, mean, rstd, d, n, eps, act);
   } else {
     const float4 *x4 = (const float4*)x, *g4 = (const float4*)gamma, *b4 = (const float4*)beta;
@@ -410,7 +695,6 @@ FB_API int32_t fb_layernorm_fwd(fb_ctx* ctx, void* stream_, const float* x, cons
     const int d4 = (int)(d / 4);
     const unsigned gridv = (unsigned)(n < 0x7fffffff ? n : 0x7fffffff);
     switch (v) {
-      case 1: ln_fwd_vec_kernel<1><<<gridv, LN_THREADS, 0, stream>>>(x4, g4, b4, y4, mean, rstd, d4, n, eps, act); break;
       case 2: ln_fwd_vec_kernel<2><<<gridv, LN_THREADS, 0, stream>>>(x4, g4, b4, y4, mean, rstd, d4, n, eps, act); break;
       case 4: ln_fwd_vec_kernel<4><<<gridv, LN_THREADS, 0, stream>>>(x4, g4, b4, y4, mean, rstd, d4, n, eps, act); break;
       default: ln_fwd_vec_kernel<8><<<gridv, LN_THREADS, 0, stream>>>(x4, g4, b4, y4, mean, rstd, d4, n, eps, act); break;
@@ -426,13 +710,21 @@ int32_t fb_layernorm_bwd_impl(cudaStream_t stream, int sm_count, float* part, in
                               const float* dy, float* dx, float* dgamma, float* dbeta, int64_t d, int64_t n,
                               int32_t act, int32_t* dev_err, bool allow_ring = true) {
   (void)sm_count;
+  if (d <= 1024 && groups > (n + 7) / 8) groups = (n + 7) / 8;   // (eight rows a block)
   const bool want_param = (dgamma != nullptr);
   float* part_dg = want_param ? part : nullptr;
   float* part_db = want_param ? part + groups * d : nullptr;
   const bool vec = (d % 4 == 0) && fb_aligned16(x) && fb_aligned16(dy) && fb_aligned16(dx) &&
                    (!gamma || (fb_aligned16(gamma) && fb_aligned16(beta)));
   const int v = vec ? ln_pick_v(d / 4) : 0;
-  if (v == 0) {
+  const bool rows = ln_rows_dispatch(d, vec, [&](auto V, auto T, auto vc) {
+    fb_act_kind(act, [&](auto k) {
+      ln_bwd_rows_kernel<V.value, T.value, vc.value, k.value><<<(unsigned)groups, LN_THREADS, 0, stream>>>(
+          x, gamma, beta, mean, rstd, dy, dx, part_dg, part_db, (int)d, n, act);
+    });
+  });
+  if (rows) {
+  } else if (v == 0) {
     ln_bwd_generic_kernel<<<(unsigned)groups, LN_THREADS, 0, stream>>>(x, gamma, beta, mean, rstd, dy, dx, part_dg,
                                                                        part_db, d, n, act);
   } else {
@@ -462,7 +754,6 @@ int32_t fb_layernorm_bwd_impl(cudaStream_t stream, int sm_count, float* part, in
       }
     } else {
       switch (v) {
-        case 1: ln_bwd_vec_kernel<1><<<g, LN_THREADS, 0, stream>>>(x4, g4, b4, mean, rstd, dy4, dx4, pg4, pb4, d4, n, act); break;
         case 2: ln_bwd_vec_kernel<2><<<g, LN_THREADS, 0, stream>>>(x4, g4, b4, mean, rstd, dy4, dx4, pg4, pb4, d4, n, act); break;
         case 4: ln_bwd_vec_kernel<4><<<g, LN_THREADS, 0, stream>>>(x4, g4, b4, mean, rstd, dy4, dx4, pg4, pb4, d4, n, act); break;
         default: ln_bwd_vec_kernel<8><<<g, LN_THREADS, 0, stream>>>(x4, g4, b4, mean, rstd, dy4, dx4, pg4, pb4, d4, n, act); break;
@@ -509,6 +800,46 @@ FB_API int32_t fb_layernorm_bwd(fb_ctx* ctx, void* stream_, const float* x, cons
   }
   return fb_layernorm_bwd_impl(stream, ctx->sm_count, part, groups, x, gamma, beta, mean, rstd, dy, dx, dgamma, dbeta,
                                d, n, act, ctx->dev_error);
+}
+
+FB_API int32_t fb_layernorm_bwd_params(fb_ctx* ctx, void* stream_, const float* x, const float* gamma, const float* beta,
+                                       const float* mean, const float* rstd, const float* dy, float dy_scale, float* dgamma,
+                                       float* dbeta, int64_t d, int64_t n, int32_t act) {
+  FB_CHECK_CTX(ctx);
+  cudaStream_t stream = (cudaStream_t)stream_;
+  FB_REQUIRE(d >= 1 && n >= 0, FB_ERR_SHAPE, "fb_layernorm_bwd_params: bad shape d=%lld n=%lld", (long long)d, (long long)n);
+  FB_REQUIRE(fb_act_valid(act), FB_ERR_INVALID_ARG, "fb_layernorm_bwd_params: unknown activation %d", act);
+  FB_REQUIRE((gamma == nullptr) == (beta == nullptr), FB_ERR_INVALID_ARG, "fb_layernorm_bwd_params: gamma and beta must both be given or both NULL");
+  FB_REQUIRE(dgamma && dbeta, FB_ERR_INVALID_ARG, "fb_layernorm_bwd_params: NULL pointer");
+  if (n == 0) {
+    FB_CUDA(cudaMemsetAsync(dgamma, 0, d * sizeof(float), stream));
+    FB_CUDA(cudaMemsetAsync(dbeta, 0, d * sizeof(float), stream));
+    return FB_OK;
+  }
+  FB_REQUIRE(x && mean && rstd && dy, FB_ERR_INVALID_ARG, "fb_layernorm_bwd_params: NULL pointer");
+  const bool vec = (d % 4 == 0) && fb_aligned16(x) && fb_aligned16(dy) && (!gamma || (fb_aligned16(gamma) && fb_aligned16(beta)));
+  const int64_t pieces = vec ? d / 4 : d;
+  int lx = 32;
+  while (lx > 1 && lx / 2 >= pieces) lx /= 2;
+  // about eight blocks per SM, each with at least four rows a thread
+  const int64_t col_blocks = (pieces + lx - 1) / lx, ny = LN_THREADS / lx;
+  int64_t groups = ((int64_t)ctx->sm_count * 8 + col_blocks - 1) / col_blocks;
+  const int64_t most = (n + 4 * ny - 1) / (4 * ny);
+  groups = groups > most ? most : groups;
+  groups = groups > 65535 ? 65535 : groups;
+  FB_REQUIRE(col_blocks <= 0x7fffffff, FB_ERR_UNSUPPORTED, "fb_layernorm_bwd_params: too many features");
+  float* part = (float*)fb_scratch(ctx, stream, (size_t)(2 * groups * d) * sizeof(float));
+  if (!part) return FB_ERR_ALLOC;
+  float *pg = part, *pb = part + groups * d;
+  const dim3 grid((unsigned)col_blocks, (unsigned)groups);
+  fb_act_kind(act, [&](auto k) {
+    if (vec) ln_bwd_params_kernel<true, k.value><<<grid, LN_THREADS, 0, stream>>>(x, gamma, beta, mean, rstd, dy, dy_scale, pg, pb, d, n, act, lx);
+    else ln_bwd_params_kernel<false, k.value><<<grid, LN_THREADS, 0, stream>>>(x, gamma, beta, mean, rstd, dy, dy_scale, pg, pb, d, n, act, lx);
+  });
+  FB_LAUNCH_CHECK();
+  fb_colreduce2_kernel<<<(unsigned)((d + 31) / 32), 256, 0, stream>>>(pg, pb, dgamma, dbeta, groups, d);
+  FB_LAUNCH_CHECK();
+  return FB_OK;
 }
 
 // ------------------------------------------------------------- LayerNorm backward without allocation ---

@@ -203,6 +203,36 @@ def to_f32(a: B200Array) -> B200Array:
     return out
 
 
+class Scaled(B200Array):
+    """A cotangent that is known to be `factor` times the Float32 array `base`.  Its memory exists from the first reader on;
+    kernels that take a factor with their cotangent read `base` itself (`unscaled`)."""
+
+    __slots__ = ("base", "factor", "_value")
+
+    def __init__(self, base: B200Array, factor: float):
+        self.size, self._node = base.size, None
+        self.base, self.factor, self._value = base, factor, None
+
+    @property
+    def backed(self) -> bool:
+        return self._value is not None
+
+    @property
+    def t(self):
+        if self._value is None:
+            ctx, out = context(), empty(self.size)
+            lib.call("fb_scale", ctx.handle, ctx.stream, self.base.ptr, self.factor, out.ptr, out.numel())
+            self._value = out.t
+        return self._value
+
+
+def unscaled(g: B200Array):
+    """(array, factor) whose product is the cotangent `g`, without making memory for it."""
+    if isinstance(g, Scaled) and not g.backed:
+        return g.base, g.factor
+    return to_f32(g), 1.0
+
+
 # ------------------------------------------------------------------------------------- tape ---
 class Tape:
     """Reverse-mode tape: a list of (output, inputs, pullback) recorded while `Tape.active`."""

@@ -14,7 +14,7 @@ import numpy as np
 import torch
 
 from . import lib
-from .core import B200Array, Tape, context, empty, gpu, is_bf16, to_bf16, to_f32, zeros
+from .core import B200Array, Tape, context, empty, gpu, is_bf16, to_bf16, to_f32, unscaled, zeros
 from .init import glorot_uniform
 
 
@@ -327,12 +327,20 @@ class LayerNorm(Layer):
             def pullback(gs, x=x):
                 dy = gs[0]
                 sink = Tape.grad_sink
-                dx = empty(x.size)
+                need_dx = Tape.needs(x)
+                if g is None and not need_dx:
+                    return []
+                dx = empty(x.size) if need_dx else None
                 dg = ((sink.buffer_for(g) if sink else None) or empty(g.size)) if g is not None else None
                 dbeta = ((sink.buffer_for(b) if sink else None) or empty(b.size)) if b is not None else None
-                lib.call("fb_layernorm_bwd", ctx.handle, ctx.stream, x.ptr, _ptr(g), _ptr(b), mean.ptr, rstd.ptr, dy.ptr,
-                         dx.ptr, _ptr(dg), _ptr(dbeta), d, n, act)
-                res = [(x, dx)] if Tape.needs(x) else []
+                if need_dx:
+                    lib.call("fb_layernorm_bwd", ctx.handle, ctx.stream, x.ptr, _ptr(g), _ptr(b), mean.ptr, rstd.ptr, dy.ptr,
+                             dx.ptr, _ptr(dg), _ptr(dbeta), d, n, act)
+                else:
+                    dy, factor = unscaled(dy)
+                    lib.call("fb_layernorm_bwd_params", ctx.handle, ctx.stream, x.ptr, g.ptr, b.ptr, mean.ptr, rstd.ptr, dy.ptr, factor,
+                             dg.ptr, dbeta.ptr, d, n, act)
+                res = [(x, dx)] if need_dx else []
                 if g is not None:
                     res += [(g, dg), (b, dbeta)]
                 return res
@@ -395,12 +403,20 @@ class BatchNorm(Layer):
 
             def pullback(gs, x=x):
                 dy = gs[0]
-                dx = empty(x.size)
+                need_dx = Tape.needs(x)
+                if g is None and not need_dx:
+                    return []
+                dx = empty(x.size) if need_dx else None
                 dg = empty((c,)) if g is not None else None
                 dbeta = empty((c,)) if b is not None else None
-                lib.call("fb_batchnorm_bwd", ctx.handle, ctx.stream, x.ptr, _ptr(g), _ptr(b), mean.ptr, rstd.ptr, dy.ptr,
-                         dx.ptr, _ptr(dg), _ptr(dbeta), s, c, n, act)
-                res = [(x, dx)] if Tape.needs(x) else []
+                if need_dx:
+                    lib.call("fb_batchnorm_bwd", ctx.handle, ctx.stream, x.ptr, _ptr(g), _ptr(b), mean.ptr, rstd.ptr, dy.ptr,
+                             dx.ptr, _ptr(dg), _ptr(dbeta), s, c, n, act)
+                else:
+                    dy, factor = unscaled(dy)
+                    lib.call("fb_batchnorm_bwd_params", ctx.handle, ctx.stream, x.ptr, g.ptr, b.ptr, mean.ptr, rstd.ptr, dy.ptr, factor,
+                             dg.ptr, dbeta.ptr, s, c, n, act)
+                res = [(x, dx)] if need_dx else []
                 if g is not None:
                     res += [(g, dg), (b, dbeta)]
                 return res

@@ -14,7 +14,7 @@ import numpy as np
 import torch
 
 from . import lib
-from .core import B200Array, Tape, accumulate, context, empty, gpu, to_bf16, to_f32, zeros
+from .core import B200Array, Scaled, Tape, accumulate, context, empty, gpu, to_bf16, to_f32, zeros
 from .layers import DimensionMismatch, Layer, trainables
 
 
@@ -83,9 +83,7 @@ def sum_abs2(y: B200Array) -> B200Array:
         def pullback(gs):
             g = gs[0]
             s = 2.0 if (g is None or getattr(g, "_is_one", False)) else 2.0 * float(g.t.item())
-            dy = empty(y.size)
-            lib.call("fb_scale", ctx.handle, ctx.stream, y.ptr, s, dy.ptr, y.numel())
-            return [(y, dy)]
+            return [(y, Scaled(y, s))]
 
         Tape.record(out, [y], pullback)
     return out

@@ -179,6 +179,11 @@ int32_t fb_layernorm_bwd(fb_ctx* ctx, void* stream, const float* x, const float*
                          const float* beta, const float* mean, const float* rstd, const float* dy,
                          float* dx, float* dgamma, float* dbeta, int64_t d, int64_t n, int32_t act);
 
+/* fb_layernorm_bwd without dx, for an input that has no gradient: dgamma[d], dbeta[d] for the cotangent dy_scale * dy. */
+int32_t fb_layernorm_bwd_params(fb_ctx* ctx, void* stream, const float* x, const float* gamma, const float* beta,
+                                const float* mean, const float* rstd, const float* dy, float dy_scale,
+                                float* dgamma, float* dbeta, int64_t d, int64_t n, int32_t act);
+
 /* fb_layernorm_bwd for callers that may not allocate device memory (a process whose memory budget is fixed at
  * start-up, code inside a stream capture, runtime threads that must not risk the implicit synchronisation of
  * cudaMalloc / cudaFree).  No counterpart in the reference; same arguments and results as fb_layernorm_bwd minus the
@@ -218,6 +223,11 @@ int32_t fb_batchnorm_bwd(fb_ctx* ctx, void* stream, const float* x, const float*
                          const float* beta, const float* save_mean, const float* save_rstd,
                          const float* dy, float* dx, float* dgamma, float* dbeta, int64_t s, int64_t c,
                          int64_t n, int32_t act);
+
+/* fb_batchnorm_bwd without dx, for an input that has no gradient: dgamma[c], dbeta[c] for the cotangent dy_scale * dy. */
+int32_t fb_batchnorm_bwd_params(fb_ctx* ctx, void* stream, const float* x, const float* gamma, const float* beta,
+                                const float* save_mean, const float* save_rstd, const float* dy, float dy_scale,
+                                float* dgamma, float* dbeta, int64_t s, int64_t c, int64_t n, int32_t act);
 
 /* ------------------------------------------------------------------- GroupNorm / InstanceNorm -- */
 
