@@ -9,6 +9,8 @@
 // backward, ordered by the stream.
 #include <stdlib.h>
 
+#include <cuda_fp16.h>
+
 #include "common.cuh"
 
 namespace {
@@ -446,6 +448,7 @@ rnn_bwd_dh2d_kernel(const float* __restrict__ Wh, const float* __restrict__ dg, 
 constexpr size_t DH2D_SMEM = (size_t)2 * DH_U * DH_LD * sizeof(float);
 
 #include "rnn_seq.cuh"
+#include "rnn_mma.cuh"
 
 // hprev_all[(b, t)] = t == 0 ? h0[b] (or 0) : out[(b, t-1)]
 __global__ void __launch_bounds__(RT)
@@ -536,17 +539,69 @@ const void* seq_bwd_kernel(int ug, int bg) {
   return bg == 16 ? (const void*)rnn_bwd_seq_kernel<NG, 8, 16, VEC> : bg == 8 ? (const void*)rnn_bwd_seq_kernel<NG, 8, 8, VEC> : (const void*)rnn_bwd_seq_kernel<NG, 8, 4, VEC>;
 }
 
+// The same for the tensor-core kernels (16 units x 8 or 16 columns a CTA).  Hidden sizes from 48 up to 512 (beyond, the fragments of the
+// weights do not fit the registers), and sequences long enough to pay for the start (fragments, the buffer's fill).  Against the
+// FMA kernels (us, forward and backward with their bulk products): LSTM 512 x 64 columns, 256 steps 1650 + 2390 -> 890 + 1550; 4
+// steps 46 + 78 -> 39 + 75, 2 steps 35 + 67 -> 35 + 68, 1 step 25 + 48 -> 28 + 50; GRU 257 x 128, 50 steps 231 + 463 -> 156 + 360;
+// 200 x 20, 50 steps 105 + 169 -> 97 + 162; 100 x 20, 3 steps 22 + 40 -> 27 + 43; LSTM 48 x 128, 50 steps 103 + 166 -> 97 + 148;
+// 32 x 128, 20 steps 45 + 74 -> 48 + 76; 16 x 1, 100 steps 143 + 167 -> 145 + 160.
+bool plan_mma(const fb_ctx* ctx, int ng, int H, int64_t B, int64_t T, bool bwd, SeqPlan* best) {
+  if (!persistent_enabled() || B > (1 << 20) || H < 48 || H > 512 || T * H < 1536) return false;
+  const int ugroups = (H + MQ_UG - 1) / MQ_UG;
+  double best_t = 1e30;
+  for (int bg = 16; bg >= 8; bg /= 2) {
+    const int64_t nch = (B + bg - 1) / bg;
+    const int nbg = (int)(nch < ctx->sm_count / ugroups ? nch : ctx->sm_count / ugroups);
+    if (nbg < 1) continue;
+    const int64_t chunks = (nch + nbg - 1) / nbg;
+    if (chunks > 64) continue;
+    const double t = chunks * (0.8 + 0.02 * bg) + 1.3;   // us of a step
+    if (t < best_t) {
+      best_t = t;
+      best->ug = MQ_UG; best->bg = bg; best->nbg = nbg; best->grid = ugroups * nbg;
+      best->smem = bwd ? mq_bwd_smem(bg, (ng * mq_pad(H) + 511) / 512, (int)chunks) : mq_fwd_smem(ng, bg, H <= 128 ? 1 : H <= 256 ? 2 : 4, (int)chunks);
+    }
+  }
+  return best_t < 1e30 && best->smem <= ctx->smem_optin;
+}
+template <int NG>
+const void* mma_fwd_kernel(int bg, int H) {
+  if (bg == 16) return H <= 128 ? (const void*)rnn_fwd_mma_kernel<NG, 16, 1> : H <= 256 ? (const void*)rnn_fwd_mma_kernel<NG, 16, 2> : (const void*)rnn_fwd_mma_kernel<NG, 16, 4>;
+  return H <= 128 ? (const void*)rnn_fwd_mma_kernel<NG, 8, 1> : H <= 256 ? (const void*)rnn_fwd_mma_kernel<NG, 8, 2> : (const void*)rnn_fwd_mma_kernel<NG, 8, 4>;
+}
+template <int NG, int BG>
+const void* mma_bwd_kernel(int np) {
+  return np == 1 ? (const void*)rnn_bwd_mma_kernel<NG, BG, 1> : np == 2 ? (const void*)rnn_bwd_mma_kernel<NG, BG, 2>
+       : np == 3 ? (const void*)rnn_bwd_mma_kernel<NG, BG, 3> : (const void*)rnn_bwd_mma_kernel<NG, BG, 4>;
+}
+
 // Launches the whole forward / backward time loop; FB_ERR_UNSUPPORTED (without a message) when the hidden size does not fit.
 template <int NG>
 int32_t launch_fwd_seq(fb_ctx* ctx, cudaStream_t stream, const float* Wh, const float* gx, const float* h0, const float* c0, float* out,
                        float* cache, float* cst, float* hT, float* cT, int H, int64_t B64, int64_t T64) {
   SeqPlan p;
+  int B = (int)B64, T = (int)T64, cached = cache != nullptr ? 1 : 0;
+  int32_t* dev_err = ctx->dev_error;
+  if (plan_mma(ctx, NG, H, B64, T64, false, &p)) {
+    const size_t bytes = (size_t)(T64 - 1) * mq_run(B64, p.bg, mq_pad(H)) * sizeof(float);
+    const fb_temp mem(ctx, stream, bytes);
+    if (bytes == 0 || mem.p != nullptr) {
+      if (bytes != 0) FB_CUDA(cudaMemsetAsync(mem.p, 0xff, bytes, stream));
+      const void* kern = mma_fwd_kernel<NG>(p.bg, H);
+      float* ex = (float*)mem.p;
+      void* args[] = {(void*)&Wh, (void*)&gx, (void*)&h0, (void*)&c0, (void*)&out, (void*)&cache, (void*)&cst, (void*)&cached, (void*)&hT,
+                      (void*)&cT, (void*)&ex, (void*)&H, (void*)&B, (void*)&T, (void*)&p.nbg, (void*)&dev_err};
+      FB_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)p.smem));
+      FB_CUDA(cudaLaunchCooperativeKernel(kern, dim3((unsigned)p.grid), dim3(SQ_THREADS), args, p.smem, stream));
+      FB_LAUNCH_CHECK();
+      return FB_OK;
+    }
+  }
   if (!plan_seq(ctx, NG, H, B64, false, &p)) return FB_ERR_UNSUPPORTED;
   const bool vec = H % 4 == 0 && fb_aligned16(out) && fb_aligned16(h0);
   const void* kern = vec ? seq_fwd_kernel<NG, true>(p.ug, p.bg) : seq_fwd_kernel<NG, false>(p.ug, p.bg);
   if (T64 > 1) FB_CUDA(cudaMemsetAsync(out, 0xff, (size_t)(T64 * B64 * H) * sizeof(float), stream));
-  int B = (int)B64, T = (int)T64, cached = cache != nullptr ? 1 : 0, nbg = p.nbg;
-  int32_t* dev_err = ctx->dev_error;
+  int nbg = p.nbg;
   void* args[] = {(void*)&Wh, (void*)&gx, (void*)&h0, (void*)&c0, (void*)&out, (void*)&cache, (void*)&cst, (void*)&cached, (void*)&hT,
                   (void*)&cT, (void*)&H, (void*)&B, (void*)&T, (void*)&nbg, (void*)&dev_err};
   FB_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)p.smem));
@@ -559,12 +614,29 @@ int32_t launch_bwd_seq(fb_ctx* ctx, cudaStream_t stream, const float* Wh, const 
                        const float* hout, const float* dout, const float* dhT, const float* dcT, float* dg, float* dgx, int H, int64_t B64,
                        int64_t T64) {
   SeqPlan p;
+  int B = (int)B64, T = (int)T64;
+  int32_t* dev_err = ctx->dev_error;
+  if (plan_mma(ctx, NG, H, B64, T64, true, &p)) {
+    const size_t bytes = T64 > 1 ? (size_t)T64 * mq_run(B64, p.bg, NG * mq_pad(H)) * sizeof(float) : 0;   // (step 0 sends nothing)
+    const fb_temp mem(ctx, stream, bytes);
+    if (bytes == 0 || mem.p != nullptr) {
+      if (bytes != 0) FB_CUDA(cudaMemsetAsync(mem.p, 0xff, bytes, stream));
+      const int np = (NG * mq_pad(H) + 511) / 512;
+      const void* kern = p.bg == 16 ? mma_bwd_kernel<NG, 16>(np) : mma_bwd_kernel<NG, 8>(np);
+      float* ex = (float*)mem.p;
+      void* args[] = {(void*)&Wh, (void*)&keep, (void*)&cst, (void*)&s0, (void*)&hout, (void*)&dout, (void*)&dhT, (void*)&dcT, (void*)&dg,
+                      (void*)&dgx, (void*)&ex, (void*)&H, (void*)&B, (void*)&T, (void*)&p.nbg, (void*)&dev_err};
+      FB_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)p.smem));
+      FB_CUDA(cudaLaunchCooperativeKernel(kern, dim3((unsigned)p.grid), dim3(SQ_THREADS), args, p.smem, stream));
+      FB_LAUNCH_CHECK();
+      return FB_OK;
+    }
+  }
   if (!plan_seq(ctx, NG, H, B64, true, &p)) return FB_ERR_UNSUPPORTED;
   const bool vec = NG * H % 4 == 0 && fb_aligned16(dg);
   const void* kern = vec ? seq_bwd_kernel<NG, true>(p.ug, p.bg) : seq_bwd_kernel<NG, false>(p.ug, p.bg);
   if (T64 > 1) FB_CUDA(cudaMemsetAsync(dg, 0xff, (size_t)(T64 * B64 * NG * H) * sizeof(float), stream));
-  int B = (int)B64, T = (int)T64, nbg = p.nbg;
-  int32_t* dev_err = ctx->dev_error;
+  int nbg = p.nbg;
   void* args[] = {(void*)&Wh, (void*)&keep, (void*)&cst, (void*)&s0, (void*)&hout, (void*)&dout, (void*)&dhT, (void*)&dcT, (void*)&dg,
                   (void*)&dgx, (void*)&H, (void*)&B, (void*)&T, (void*)&nbg, (void*)&dev_err};
   FB_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)p.smem));

@@ -1,0 +1,494 @@
+// The time loop of an LSTM / GRU in one launch with the per-step products on the warp-level tensor cores (included by recurrent.cu
+// behind rnn_seq.cuh, whose way of exchanging results it shares: words are polled in place until none is the empty pattern).
+//
+// CTA (unit group, batch group): 16 hidden units x BG = 8 or 16 columns.  Eight warps share k, and every warp keeps its
+// part of the CTA's weight rows in registers for the whole launch, as mma.m16n8k16 fragments of two half-precision planes
+// (W 2^s = hi + lo with a power of two per row, 23 bits).  Three products (lo hi, hi lo, hi hi) replace one Float32 product; a
+// warp's sum has at most 64 k-values (backward: sums of 64 are added up in Float32), then the warps' sums are added in Float32.
+//
+// Exchange.  A step's results go to a buffer of their own in the order of the fragments: [t][columns of a CTA][16 k-values]
+// [8 columns][lane][4], so that a lane polls exactly the 16-byte pieces that it multiplies, a warp reads whole 512-byte runs
+// and a CTA writes one: no shared memory and no barrier between the arrival of h and the product, and a warp waits for its own
+// part only.  (The four k-values of a lane are neighbours; the order within a fragment is the same for both operands and does not
+// matter to the sum.)  Read from `out`, whose rows lie T * H apart, the same pieces took 1.6 us of a step of 3.9 (L2: 8 rows of 64
+// bytes a request, every row 512 KB from the next).  |h| <= 1, in a GRU at most the largest of its column's initial state, so h
+// is exchanged as the two halves of 2^14 h (less in such a column), which its reader need not convert; the initial state itself is
+// multiplied in Float32.  Gate derivatives are exchanged in Float32: a column's scale is taken from the largest of the values that
+// the warp multiplies, anew for every 64 of them.
+//
+// What bounds it: T dependent steps: one store -> load flight through L2, then about 100 mma per warp (0.4 us), the sum over the
+// warps (0.3 us) and the gates (0.6 us).  H 512, B 64, T 256: forward 6.0 -> 3.0 us a step, backward 7.8 -> 4.5 (Float32 FMAs from
+// shared memory before: 2.3 us of a step by themselves).  Error against float64 is that of the FMA kernel.
+#pragma once
+
+constexpr int MQ_UG = 16;
+
+__device__ __forceinline__ void mq_mma(float (&c)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
+  asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%0, %1, %2, %3};"
+               : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
+               : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
+}
+// two values -> their upper and lower halves
+__device__ __forceinline__ void mq_split(float x, float y, uint32_t& hi, uint32_t& lo) {
+  const __half2 h = __floats2half2_rn(x, y);
+  const float2 f = __half22float2(h);
+  const __half2 l = __floats2half2_rn(x - f.x, y - f.y);
+  hi = *reinterpret_cast<const uint32_t*>(&h);
+  lo = *reinterpret_cast<const uint32_t*>(&l);
+}
+// 2^s that puts a largest magnitude (its bits) into [2^14, 2^15), as s
+__device__ __forceinline__ int mq_shift(uint32_t max_bits) {
+  const int s = 141 - (int)(max_bits >> 23);
+  return max_bits == 0 ? 0 : s > 126 ? 126 : s < -113 ? -113 : s;
+}
+__device__ __forceinline__ float mq_pow2(int s) { return __int_as_float((s + 127) << 23); }
+
+// A fragment of one k-step: rows r and r + 8 of Ws, k-values 4 q .. 4 q + 3 of the step
+__device__ __forceinline__ void mq_load_a(const float* Ws, int ld, int r, int k, float s0, float s8, uint32_t (&hi)[4], uint32_t (&lo)[4]) {
+  const float4 x = *(const float4*)(Ws + (size_t)r * ld + k), y = *(const float4*)(Ws + (size_t)(r + 8) * ld + k);
+  mq_split(x.x * s0, x.y * s0, hi[0], lo[0]);
+  mq_split(y.x * s8, y.y * s8, hi[1], lo[1]);
+  mq_split(x.z * s0, x.w * s0, hi[2], lo[2]);
+  mq_split(y.z * s8, y.w * s8, hi[3], lo[3]);
+}
+
+// The pieces of one lane, k-steps ks .. ks + KS - 1 of a step's run (of `steps` of them), polled until all are there.  AGAIN asks only
+// for those that were missing.
+template <int NT, int KS>
+struct MqPieces {
+  uint4 v[NT][KS];
+  static __device__ __forceinline__ bool empty(const uint4& x) {
+    return (x.x == SQ_EMPTY) | (x.y == SQ_EMPTY) | (x.z == SQ_EMPTY) | (x.w == SQ_EMPTY);
+  }
+  template <bool AGAIN>
+  __device__ __forceinline__ void load(const float* run, int ncols, int ks, int steps) {
+    const int lane = threadIdx.x & 31;
+    const float* p = run + (size_t)ks * (NT * 128) + 4 * lane;
+#pragma unroll
+    for (int s = 0; s < KS; ++s)
+#pragma unroll
+      for (int n = 0; n < NT; ++n) {
+        if (AGAIN && !empty(v[n][s])) continue;
+        uint4 x = make_uint4(0u, 0u, 0u, 0u);
+        if (8 * n + (lane >> 2) < ncols && ks + s < steps) x = sq_peek4(p + (s * NT + n) * 128);
+        v[n][s] = x;
+      }
+  }
+  __device__ __forceinline__ bool complete() const {
+    bool missing = false;
+#pragma unroll
+    for (int n = 0; n < NT; ++n)
+#pragma unroll
+      for (int s = 0; s < KS; ++s) missing |= empty(v[n][s]);
+    return !missing;
+  }
+  __device__ __forceinline__ bool wait(const float* run, int ncols, int ks, int steps, const int32_t* dev_err) {
+    uint32_t spins = 0;
+    while (!complete()) {
+      if (++spins > SQ_POLL_LIMIT || ((spins & 255u) == 255u && *(const volatile int32_t*)dev_err != 0)) return false;
+      load<true>(run, ncols, ks, steps);
+    }
+    return true;
+  }
+};
+// words of a run: `batch` columns in whole groups of bg, k in whole k-steps
+inline size_t mq_run(int64_t batch, int bg, int k) { return (size_t)((batch + bg - 1) / bg) * bg * k; }
+inline int mq_pad(int n) { return (n + 15) / 16 * 16; }
+
+// word (k-step ks, k-value gu of it, column gb) of a CTA's run
+__device__ __forceinline__ void mq_publish(float* run, int bg, int ks, int gu, int gb, uint32_t w) {
+  float* p = run + (size_t)ks * (bg * 16) + (gb >> 3) * 128 + (gb & 7) * 16 + gu;
+  asm volatile("st.relaxed.gpu.global.u32 [%0], %1;" ::"l"(p), "r"(w) : "memory");
+}
+// x, a scaled h, as (upper half, lower half); a conversion never makes the half 0xffff, so no word is the empty pattern.  An infinite
+// one (from a GRU's initial state) is sent as the largest half: it saturates gates all the same.
+__device__ __forceinline__ uint32_t mq_halves(float x) {
+  x = x > 65504.0f ? 65504.0f : x < -65504.0f ? -65504.0f : x;
+  const __half a = __float2half_rn(x);
+  const __half b = __float2half_rn(x - __half2float(a));
+  return (uint32_t)__half_as_ushort(a) | ((uint32_t)__half_as_ushort(b) << 16);
+}
+__device__ __forceinline__ uint32_t mq_word(float v) {
+  const uint32_t w = __float_as_uint(v);
+  return w == SQ_EMPTY ? 0x7fffffffu : w;
+}
+
+// rowf[r] = 2^-shift of row r, from the largest magnitude of Ws[r][0 .. n)
+__device__ __forceinline__ void mq_row_scales(const float* Ws, int ld, int rows, int n, float* rowf) {
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  for (int r = warp; r < rows; r += SQ_THREADS / 32) {
+    uint32_t m = 0;
+    for (int k = lane; k < n; k += 32) m = max(m, __float_as_uint(Ws[(size_t)r * ld + k]) & 0x7fffffffu);
+    m = __reduce_max_sync(0xffffffffu, m);
+    if (lane == 0) rowf[r] = mq_pow2(-mq_shift(m));
+  }
+}
+
+inline size_t mq_fwd_smem(int ng, int bg, int ks, int chunks) {
+  const size_t w = (size_t)ng * MQ_UG * (128 * ks + 4), red = (size_t)2 * 8 * bg * (ng * MQ_UG + 4);
+  return (w + red + ng * MQ_UG + (size_t)chunks * (MQ_UG + 1) * bg) * 4;
+}
+inline size_t mq_bwd_smem(int bg, int np, int chunks) {
+  const size_t w = (size_t)MQ_UG * (512 * np + 4), red = (size_t)2 * 8 * bg * (MQ_UG + 4);
+  return ((w > red ? w : red) + MQ_UG + (size_t)chunks * MQ_UG * bg) * 4;
+}
+
+// Arguments as for rnn_fwd_seq_kernel, and the exchange buffer (T - 1 runs); KS k-steps of 16 per warp: hidden sizes up to 128 KS.
+template <int NG, int BG, int KS>
+__global__ void __launch_bounds__(SQ_THREADS, 1)
+rnn_fwd_mma_kernel(const float* __restrict__ Wh, const float* __restrict__ gx, const float* __restrict__ h0, const float* __restrict__ c0,
+                   float* __restrict__ out, float* __restrict__ cache, float* __restrict__ cst, int cached, float* __restrict__ hT,
+                   float* __restrict__ cT, float* ex, int H, int B, int T, int nbg, int32_t* dev_err) {
+  constexpr int UG = MQ_UG, R = NG * UG, NT = BG / 8, LD = 128 * KS + 4, LR = R + 4;
+  extern __shared__ __align__(16) float sm[];
+  float* Ws = sm;                            // [R][LD], until the initial state has been multiplied
+  float* red = Ws + R * LD;                  // [2][8][BG][LR]
+  float* rowf = red + 2 * 8 * BG * LR;       // [R]
+  float* colf = rowf + R;                    // [chunks][BG]: what undoes a column's scale
+  const int ugroups = (H + UG - 1) / UG;
+  const int u0 = ((int)blockIdx.x % ugroups) * UG, bgrp = (int)blockIdx.x / ugroups;
+  const int nchunks = (B + BG - 1) / BG;
+  const int64_t ldrow = (int64_t)T * H, ldgx = (int64_t)T * NG * H, ldc = (int64_t)T * 4 * H;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, q = lane & 3;
+  const int gu = threadIdx.x % UG, gb = threadIdx.x / UG;   // gates: unit, column (threads below UG * BG)
+  const int u = u0 + gu, ks0 = warp * KS, steps = (H + 15) / 16;
+  const size_t run = (size_t)nchunks * BG * steps * 16;
+  float* cs = colf + (nchunks + nbg - 1) / nbg * BG;   // [chunks][BG * UG]: LSTM c, GRU h
+  for (int e = threadIdx.x; e < R * 128 * KS; e += SQ_THREADS) {
+    const int rr = e % R, k = e / R, g = rr / UG, uu = rr % UG;
+    Ws[(size_t)rr * LD + k] = (k < H && u0 + uu < H) ? __ldg(Wh + (int64_t)k * (NG * H) + g * H + u0 + uu) : 0.0f;
+  }
+  for (int ch = bgrp, i = 0; ch < nchunks; ch += nbg, ++i) {
+    const int b = ch * BG + gb;
+    const float* s0 = NG == 4 ? c0 : h0;
+    if (threadIdx.x < UG * BG) cs[i * UG * BG + threadIdx.x] = (s0 && b < B && u < H) ? s0[(int64_t)b * H + u] : 0.0f;
+    for (int c = warp; c < BG; c += SQ_THREADS / 32) {
+      uint32_t m = 0x3f800000u;   // 1
+      if (NG == 3 && h0 != nullptr && ch * BG + c < B)
+        for (int k = lane; k < H; k += 32) m = max(m, __float_as_uint(__ldg(h0 + (int64_t)(ch * BG + c) * H + k)) & 0x7fffffffu);
+      m = __reduce_max_sync(0xffffffffu, m);
+      if (lane == 0) colf[i * BG + c] = mq_pow2((int)(m >> 23) - 127 - 14 < 100 ? (int)(m >> 23) - 127 - 14 : 100);
+    }
+  }
+  __syncthreads();
+  mq_row_scales(Ws, LD, R, 128 * KS, rowf);
+  __syncthreads();
+  uint32_t ahi[NG][KS][4], alo[NG][KS][4];
+#pragma unroll
+  for (int g = 0; g < NG; ++g) {
+    const int r = g * UG + (lane >> 2);
+    const float s0 = 1.0f / rowf[r], s8 = 1.0f / rowf[r + 8];   // powers of two
+#pragma unroll
+    for (int s = 0; s < KS; ++s) mq_load_a(Ws, LD, r, 16 * (ks0 + s) + 4 * q, s0, s8, ahi[g][s], alo[g][s]);
+  }
+  __syncthreads();
+  int turn = 0;
+  // the input projection of the next (step, chunk), on its way while this one waits for h
+  float gxn[NG];
+  auto ahead = [&](int t, int ch) {
+    const int b = ch * BG + gb;
+    const bool there = threadIdx.x < UG * BG && b < B && u < H && t < T;
+#pragma unroll
+    for (int g = 0; g < NG; ++g) gxn[g] = there ? __ldg(gx + (int64_t)b * ldgx + (int64_t)t * NG * H + g * H + u) : 0.0f;
+  };
+  ahead(0, bgrp);
+  for (int t = 0; t < T; ++t) {
+    for (int ch = bgrp, ci = 0; ch < nchunks; ch += nbg, ++ci, turn ^= 1) {
+      const int b0 = ch * BG, nb = B - b0 < BG ? B - b0 : BG;
+      const int b = b0 + gb;
+      const bool mine = threadIdx.x < UG * BG && gb < nb && u < H;
+      float gxv[NG];
+#pragma unroll
+      for (int g = 0; g < NG; ++g) gxv[g] = gxn[g];
+      if (ch + nbg < nchunks) ahead(t, ch + nbg);
+      else ahead(t + 1, bgrp);
+      float pre[NG];
+#pragma unroll
+      for (int g = 0; g < NG; ++g) pre[g] = 0.0f;
+      if (t > 0) {
+        const float* src = ex + (size_t)(t - 1) * run + (size_t)ch * (BG * 16) * steps;
+        MqPieces<NT, KS> pc;
+        pc.template load<false>(src, nb, ks0, steps);
+        const bool ok = pc.wait(src, nb, ks0, steps, dev_err);
+        float acc[NG][NT][4];
+#pragma unroll
+        for (int g = 0; g < NG; ++g)
+#pragma unroll
+          for (int n = 0; n < NT; ++n)
+#pragma unroll
+            for (int e = 0; e < 4; ++e) acc[g][n][e] = 0.0f;
+        // The cross terms of all k-steps first: an add into the accumulator truncates, so the fewer behind the large terms the
+        // better.  Product by product over all accumulators, so that an mma does not follow the one that it adds to.
+#pragma unroll
+        for (int s = 0; s < KS; ++s) {
+          uint32_t hi[NT][2], lo[NT][2];   // words are (hi, lo)
+#pragma unroll
+          for (int n = 0; n < NT; ++n) {
+            const uint4 x = pc.v[n][s];
+            hi[n][0] = __byte_perm(x.x, x.y, 0x5410); lo[n][0] = __byte_perm(x.x, x.y, 0x7632);
+            hi[n][1] = __byte_perm(x.z, x.w, 0x5410); lo[n][1] = __byte_perm(x.z, x.w, 0x7632);
+          }
+#pragma unroll
+          for (int n = 0; n < NT; ++n)
+#pragma unroll
+            for (int g = 0; g < NG; ++g) mq_mma(acc[g][n], alo[g][s], hi[n][0], hi[n][1]);
+#pragma unroll
+          for (int n = 0; n < NT; ++n)
+#pragma unroll
+            for (int g = 0; g < NG; ++g) mq_mma(acc[g][n], ahi[g][s], lo[n][0], lo[n][1]);
+        }
+#pragma unroll
+        for (int s = 0; s < KS; ++s) {
+          uint32_t hi[NT][2];
+#pragma unroll
+          for (int n = 0; n < NT; ++n) {
+            const uint4 x = pc.v[n][s];
+            hi[n][0] = __byte_perm(x.x, x.y, 0x5410);
+            hi[n][1] = __byte_perm(x.z, x.w, 0x5410);
+          }
+#pragma unroll
+          for (int n = 0; n < NT; ++n)
+#pragma unroll
+            for (int g = 0; g < NG; ++g) mq_mma(acc[g][n], ahi[g][s], hi[n][0], hi[n][1]);
+        }
+        float* rw = red + (size_t)(turn * 8 + warp) * BG * LR;
+#pragma unroll
+        for (int g = 0; g < NG; ++g)
+#pragma unroll
+          for (int n = 0; n < NT; ++n)
+#pragma unroll
+            for (int e = 0; e < 4; ++e) rw[(8 * n + 2 * q + (e & 1)) * LR + g * UG + (lane >> 2) + 8 * (e >> 1)] = acc[g][n][e];
+        // One barrier a step: sums of the step after next come behind the next one's, where this step's have been read.
+        if (!__syncthreads_and(ok ? 1 : 0)) {
+          if (threadIdx.x == 0) atomicCAS(dev_err, 0, 3002);
+          return;
+        }
+        if (mine) {
+#pragma unroll
+          for (int g = 0; g < NG; ++g) {
+            float s = 0.0f;
+#pragma unroll
+            for (int w = 0; w < 8; ++w) s += red[((size_t)(turn * 8 + w) * BG + gb) * LR + g * UG + gu];
+            pre[g] = s * rowf[g * UG + gu] * colf[ci * BG + gb];
+          }
+        }
+      } else if (h0 != nullptr && mine) {
+#pragma unroll 4
+        for (int k = 0; k < H; ++k) {
+          const float h = __ldg(h0 + (int64_t)b * H + k);
+#pragma unroll
+          for (int g = 0; g < NG; ++g) pre[g] = fmaf(Ws[(g * UG + gu) * LD + k], h, pre[g]);
+        }
+      }
+      if (mine) {
+        float hn, cn = 0.0f;
+        float4 keep;
+        float* c = cs + ci * UG * BG + threadIdx.x;
+        if (NG == 4) {
+          const float zi = pre[0] + gxv[0], zf = pre[1] + gxv[1], zg = pre[2] + gxv[2], zo = pre[NG - 1] + gxv[NG - 1];
+          const float ig = 1.0f / (1.0f + expf(-zi)), fg = 1.0f / (1.0f + expf(-zf));
+          const float gg = tanhf(zg), og = 1.0f / (1.0f + expf(-zo));
+          cn = fg * *c + ig * gg;
+          *c = cn;
+          hn = og * tanhf(cn);
+          keep = make_float4(ig, fg, gg, og);
+        } else {
+          const float gh3 = pre[2];
+          const float r = 1.0f / (1.0f + expf(-(gxv[0] + pre[0])));
+          const float z = 1.0f / (1.0f + expf(-(gxv[1] + pre[1])));
+          const float hc = tanhf(gxv[2] + r * gh3);
+          hn = (1.0f - z) * hc + z * *c;
+          *c = hn;
+          keep = make_float4(r, z, hc, gh3);
+        }
+        if (t + 1 < T) mq_publish(ex + (size_t)t * run + (size_t)ch * (BG * 16) * steps, BG, u0 / 16, gu, gb, mq_halves(hn * (1.0f / colf[ci * BG + gb])));
+        out[(int64_t)t * H + (int64_t)b * ldrow + u] = hn;
+        if (cache) {
+          float* gr = cache + (int64_t)t * 4 * H + (int64_t)b * ldc;
+          gr[u] = keep.x; gr[H + u] = keep.y; gr[2 * H + u] = keep.z; gr[3 * H + u] = keep.w;
+        }
+        if (NG == 4 && cached) cst[(int64_t)t * H + (int64_t)b * ldrow + u] = cn;
+        if (t == T - 1 && hT) {
+          hT[(int64_t)b * H + u] = hn;
+          if (NG == 4) cT[(int64_t)b * H + u] = cn;
+        }
+      } else if (t + 1 < T && threadIdx.x < UG * BG && gb < nb) {
+        mq_publish(ex + (size_t)t * run + (size_t)ch * (BG * 16) * steps, BG, u0 / 16, gu, gb, 0u);   // (units that do not exist)
+      }
+    }
+  }
+}
+
+// Arguments as for rnn_bwd_seq_kernel, and the exchange buffer (T runs); NP pieces of four k-steps per warp: NG * H, each gate's rows in
+// whole k-steps, up to 512 NP.
+template <int NG, int BG, int NP>
+__global__ void __launch_bounds__(SQ_THREADS, 1)
+rnn_bwd_mma_kernel(const float* __restrict__ Wh, const float* __restrict__ keep, const float* __restrict__ cst,
+                   const float* __restrict__ s0, const float* __restrict__ hout, const float* __restrict__ dout,
+                   const float* __restrict__ dhT, const float* __restrict__ dcT, float* __restrict__ dg, float* __restrict__ dgx,
+                   float* ex, int H, int B, int T, int nbg, int32_t* dev_err) {
+  constexpr int UG = MQ_UG, NT = BG / 8, LD = 512 * NP + 4, LR = UG + 4;
+  constexpr int WSZ = UG * LD > 2 * 8 * BG * LR ? UG * LD : 2 * 8 * BG * LR;
+  extern __shared__ __align__(16) float sm[];
+  float* Ws = sm;                                 // [UG][LD], only before the loop
+  float* red = sm;                                // [2][8][BG][LR]
+  float* rowf = sm + WSZ;                         // [UG]
+  float* carry = rowf + UG;                       // [chunks][UG * BG]: LSTM dc, GRU dh * z
+  const int K = NG * H;
+  const int ugroups = (H + UG - 1) / UG;
+  const int u0 = ((int)blockIdx.x % ugroups) * UG, bgrp = (int)blockIdx.x / ugroups;
+  const int nchunks = (B + BG - 1) / BG;
+  const int64_t ldrow = (int64_t)T * H, ldd = (int64_t)T * K, ldk = (int64_t)T * 4 * H;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, q = lane & 3;
+  const int gu = threadIdx.x % UG, gb = threadIdx.x / UG;
+  const int Hp = (H + 15) & ~15;                  // a gate's rows in the exchange: whole k-steps
+  const int u = u0 + gu, ks0 = warp * 4 * NP, steps = NG * Hp / 16;
+  const size_t run = (size_t)nchunks * BG * steps * 16;
+  for (int e = threadIdx.x; e < UG * 512 * NP; e += SQ_THREADS) {
+    const int r = e % (512 * NP), uu = e / (512 * NP), g = r / Hp, w = r - g * Hp;
+    Ws[(size_t)uu * LD + r] = (g < NG && w < H && u0 + uu < H) ? __ldg(Wh + (int64_t)(u0 + uu) * K + g * H + w) : 0.0f;
+  }
+  for (int ch = bgrp, i = 0; ch < nchunks; ch += nbg, ++i) {
+    const int b = ch * BG + gb;
+    if (threadIdx.x < UG * BG) carry[i * UG * BG + threadIdx.x] = (NG == 4 && dcT && b < B && u < H) ? dcT[(int64_t)b * H + u] : 0.0f;
+  }
+  __syncthreads();
+  mq_row_scales(Ws, LD, UG, 512 * NP, rowf);
+  __syncthreads();
+  uint32_t ahi[NP][4][4], alo[NP][4][4];
+  {
+    const int r = lane >> 2;
+    const float f0 = 1.0f / rowf[r], f8 = 1.0f / rowf[r + 8];   // powers of two
+#pragma unroll
+    for (int p = 0; p < NP; ++p)
+#pragma unroll
+      for (int s = 0; s < 4; ++s) mq_load_a(Ws, LD, r, 16 * (ks0 + 4 * p + s) + 4 * q, f0, f8, ahi[p][s], alo[p][s]);
+  }
+  __syncthreads();
+  int turn = 0;
+  for (int t = T - 1; t >= 0; --t) {
+    for (int ch = bgrp, ci = 0; ch < nchunks; ch += nbg, ++ci, turn ^= 1) {
+      const int b0 = ch * BG, nb = B - b0 < BG ? B - b0 : BG;
+      const int b = b0 + gb;
+      const bool mine = threadIdx.x < UG * BG && gb < nb && u < H;
+      float k0 = 0.f, k1 = 0.f, k2 = 0.f, k3 = 0.f, ct = 0.f, sp = 0.f, dh = 0.f;
+      if (mine) {
+        const float* kr = keep + (int64_t)t * 4 * H + (int64_t)b * ldk;
+        k0 = __ldg(kr + u); k1 = __ldg(kr + H + u); k2 = __ldg(kr + 2 * H + u); k3 = __ldg(kr + 3 * H + u);
+        const float* prev = NG == 4 ? cst : hout;   // c_{t-1} or h_{t-1}
+        if (NG == 4) ct = __ldg(cst + (int64_t)t * H + (int64_t)b * ldrow + u);
+        sp = t > 0 ? __ldg(prev + (int64_t)(t - 1) * H + (int64_t)b * ldrow + u) : s0 ? __ldg(s0 + (int64_t)b * H + u) : 0.0f;
+        dh = __ldg(dout + (int64_t)t * H + (int64_t)b * ldrow + u);
+        if (t == T - 1 && dhT) dh += __ldg(dhT + (int64_t)b * H + u);
+      }
+      if (t < T - 1) {
+        const float* src = ex + (size_t)(t + 1) * run + (size_t)ch * (BG * 16) * steps;
+        float sum[NT][4];
+#pragma unroll
+        for (int n = 0; n < NT; ++n)
+#pragma unroll
+          for (int e = 0; e < 4; ++e) sum[n][e] = 0.0f;
+        bool ok = true;
+        MqPieces<NT, 4> pc[2];
+        pc[0].template load<false>(src, nb, ks0, steps);
+#pragma unroll
+        for (int p = 0; p < NP; ++p) {
+          MqPieces<NT, 4>& now = pc[p & 1];
+          ok = now.wait(src, nb, ks0 + 4 * p, steps, dev_err) && ok;
+          if (p + 1 < NP) pc[(p + 1) & 1].template load<false>(src, nb, ks0 + 4 * (p + 1), steps);
+          int sh[NT];
+          float sc[NT];
+          float hh[NT][4], cr[NT][4];   // hi hi, and the cross terms
+#pragma unroll
+          for (int n = 0; n < NT; ++n) {
+            uint32_t m = 0;
+#pragma unroll
+            for (int s = 0; s < 4; ++s) {
+              const uint4 x = now.v[n][s];
+              m = max(m, max(max(x.x & 0x7fffffffu, x.y & 0x7fffffffu), max(x.z & 0x7fffffffu, x.w & 0x7fffffffu)));
+            }
+            m = max(m, __shfl_xor_sync(0xffffffffu, m, 1));
+            m = max(m, __shfl_xor_sync(0xffffffffu, m, 2));
+            sh[n] = mq_shift(m);
+            sc[n] = mq_pow2(sh[n]);
+#pragma unroll
+            for (int e = 0; e < 4; ++e) hh[n][e] = cr[n][e] = 0.0f;
+          }
+#pragma unroll
+          for (int s = 0; s < 4; ++s) {
+            uint32_t hi[NT][2], lo[NT][2];
+#pragma unroll
+            for (int n = 0; n < NT; ++n) {
+              const uint4 x = now.v[n][s];
+              mq_split(__uint_as_float(x.x) * sc[n], __uint_as_float(x.y) * sc[n], hi[n][0], lo[n][0]);
+              mq_split(__uint_as_float(x.z) * sc[n], __uint_as_float(x.w) * sc[n], hi[n][1], lo[n][1]);
+            }
+            // (in an order that keeps an mma away from the one that it adds to)
+#pragma unroll
+            for (int n = 0; n < NT; ++n) mq_mma(cr[n], alo[p][s], hi[n][0], hi[n][1]);
+#pragma unroll
+            for (int n = 0; n < NT; ++n) mq_mma(hh[n], ahi[p][s], hi[n][0], hi[n][1]);
+#pragma unroll
+            for (int n = 0; n < NT; ++n) mq_mma(cr[n], ahi[p][s], lo[n][0], lo[n][1]);
+          }
+          // columns 2 q and 2 q + 1 were scaled by the lanes that hold them
+#pragma unroll
+          for (int n = 0; n < NT; ++n) {
+            const float f0 = mq_pow2(-__shfl_sync(0xffffffffu, sh[n], 8 * q)), f1 = mq_pow2(-__shfl_sync(0xffffffffu, sh[n], 8 * q + 4));
+#pragma unroll
+            for (int e = 0; e < 4; ++e) sum[n][e] = fmaf(hh[n][e] + cr[n][e], (e & 1) ? f1 : f0, sum[n][e]);
+          }
+        }
+        float* rw = red + (size_t)(turn * 8 + warp) * BG * LR;
+#pragma unroll
+        for (int n = 0; n < NT; ++n)
+#pragma unroll
+          for (int e = 0; e < 4; ++e) rw[(8 * n + 2 * q + (e & 1)) * LR + (lane >> 2) + 8 * (e >> 1)] = sum[n][e];
+        if (!__syncthreads_and(ok ? 1 : 0)) {
+          if (threadIdx.x == 0) atomicCAS(dev_err, 0, 3003);
+          return;
+        }
+        if (mine) {
+          float s = 0.0f;
+#pragma unroll
+          for (int w = 0; w < 8; ++w) s += red[((size_t)(turn * 8 + w) * BG + gb) * LR + gu];
+          dh = fmaf(s, rowf[gu], dh);
+        }
+      }
+      float d[NG];
+#pragma unroll
+      for (int g = 0; g < NG; ++g) d[g] = 0.0f;
+      if (mine) {
+        float* cy = carry + ci * UG * BG + threadIdx.x;
+        float* row = dg + (int64_t)t * K + (int64_t)b * ldd;
+        if (NG == 4) {
+          const float tc = tanhf(ct);
+          const float d_o = dh * tc;
+          const float dcc = *cy + dh * k3 * (1.0f - tc * tc);
+          d[0] = dcc * k2 * k0 * (1.0f - k0);
+          d[1] = dcc * sp * k1 * (1.0f - k1);
+          d[2] = dcc * k0 * (1.0f - k2 * k2);
+          d[NG - 1] = d_o * k3 * (1.0f - k3);
+          *cy = dcc * k1;
+        } else {
+          if (t < T - 1) dh += *cy;
+          const float r = k0, z = k1, hc = k2, gh3 = k3;
+          const float da3 = dh * (1.0f - z) * (1.0f - hc * hc);
+          const float da2 = dh * (sp - hc) * z * (1.0f - z);
+          const float da1 = da3 * gh3 * r * (1.0f - r);
+          d[0] = da1; d[1] = da2; d[2] = da3 * r;
+          float* x = dgx + (int64_t)t * K + (int64_t)b * ldd;
+          x[u] = da1; x[H + u] = da2; x[2 * H + u] = da3;
+          *cy = dh * z;
+        }
+#pragma unroll
+        for (int g = 0; g < NG; ++g) row[g * H + u] = d[g];
+      }
+      if (t > 0 && threadIdx.x < UG * BG && gb < nb) {   // (zeros for units that do not exist)
+#pragma unroll
+        for (int g = 0; g < NG; ++g)
+          mq_publish(ex + (size_t)t * run + (size_t)ch * (BG * 16) * steps, BG, (g * Hp + u0) / 16, gu, gb, mq_word(d[g]));
+      }
+    }
+  }
+}

@@ -1,0 +1,121 @@
+"""GPU tests of the tensor-core recurrences at the edges of their cuts: hidden sizes around 16 units, 128 / 256 / 512 (k-steps per warp)
+and the backward pieces of 64, batches around 8 and 16 columns and of several chunks per CTA, initial states, steps that
+send nothing.  Reference: float64 autograd.
+
+Tolerance: operands rounded to 23 bits and sums of up to 2048 Float32 products, partly truncated, through up to 40 dependent steps
+whose gates have slopes below one: 5e-6 of the largest value; 2e-5 on what is summed over steps and batch."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+# (sequences of T * H >= 1536 and 48 <= H <= 512 take them; the others here are the neighbours across those lines)
+SHAPES = [(1, 1, 2), (47, 7, 33), (48, 8, 32), (49, 9, 32), (64, 17, 24), (127, 5, 13), (128, 16, 12), (129, 33, 12), (255, 3, 7), (256, 65, 6),
+          (257, 8, 6), (340, 40, 5), (511, 20, 4), (512, 64, 4), (512, 150, 3), (512, 2, 2), (500, 1, 40), (96, 12, 17), (80, 300, 20), (48, 700, 32),
+          (200, 20, 8), (513, 9, 3)]
+
+
+def _reference(cell, wi, wh, b, x, h, c):
+    out, gx = [], x @ wi + b
+    for t in range(x.shape[1]):
+        gh = h @ wh
+        if cell == "lstm":
+            i, f, g, o = (gx[:, t] + gh).chunk(4, 1)
+            c = torch.sigmoid(f) * c + torch.sigmoid(i) * torch.tanh(g)
+            h = torch.sigmoid(o) * torch.tanh(c)
+        else:
+            (a1, a2, a3), (g1, g2, g3) = gx[:, t].chunk(3, 1), gh.chunk(3, 1)
+            r, z = torch.sigmoid(a1 + g1), torch.sigmoid(a2 + g2)
+            h = (1 - z) * torch.tanh(a3 + r * g3) + z * h
+        out.append(h)
+    return torch.stack(out, 1), h, c
+
+
+@pytest.mark.parametrize("cell", ["lstm", "gru"])
+@pytest.mark.parametrize("states", [False, True])
+@pytest.mark.parametrize("H,B,T", SHAPES)
+def test_recurrences(cell, states, H, B, T):
+    import fluxb200 as F
+    from fluxb200 import lib
+    ctx, I, ng = F.context(0), 12, 4 if cell == "lstm" else 3
+    g = torch.Generator(device="cuda").manual_seed(H + B + T)
+    new = lambda *s: torch.randn(*s, generator=g, device="cuda")
+    p = lambda t: None if t is None else t.data_ptr()
+    wi, wh, b = new(I, ng * H) / I ** 0.5, new(H, ng * H) / H ** 0.5, new(ng * H) * 0.1
+    wh[:, ::7] *= 2.0 ** -20                          # gate rows of very different magnitude
+    x, dout = new(B, T, I), new(B, T, H)
+    dout[B // 2] *= 2.0 ** 30                         # and columns
+    h0, c0 = (new(B, H) * 3, new(B, H) if cell == "lstm" else None) if states else (None, None)
+    dhT, dcT = (new(B, H), new(B, H)) if states else (None, None)
+    out, hT, cT = torch.empty(B, T, H, device="cuda"), torch.empty(B, H, device="cuda"), torch.empty(B, H, device="cuda")
+    dwi, dwh, db, dx = (torch.empty_like(t) for t in (wi, wh, b, x))
+    alone = torch.empty_like(out)
+    if cell == "lstm":
+        cache = torch.empty(lib.raw().fb_lstm_cache_bytes(I, H, T, B) // 4, device="cuda")
+        lib.call("fb_lstm_fwd", ctx.handle, ctx.stream, p(wi), p(wh), p(b), p(x), p(h0), p(c0), p(out), p(hT), p(cT), p(cache), I, H, T, B)
+        lib.call("fb_lstm_bwd", ctx.handle, ctx.stream, p(wi), p(wh), p(x), p(h0), p(c0), p(out), p(cache), p(dout), p(dhT), p(dcT), p(dwi), p(dwh),
+                 p(db), p(dx), I, H, T, B)
+        lib.call("fb_lstm_fwd", ctx.handle, ctx.stream, p(wi), p(wh), p(b), p(x), p(h0), p(c0), p(alone), None, None, None, I, H, T, B)
+    else:
+        cache = torch.empty(lib.raw().fb_gru_cache_bytes(I, H, T, B) // 4, device="cuda")
+        lib.call("fb_gru_fwd", ctx.handle, ctx.stream, p(wi), p(wh), p(b), p(x), p(h0), p(out), p(hT), p(cache), I, H, T, B)
+        lib.call("fb_gru_bwd", ctx.handle, ctx.stream, p(wi), p(wh), p(x), p(h0), p(out), p(cache), p(dout), p(dhT), p(dwi), p(dwh), p(db), p(dx), I, H, T, B)
+        lib.call("fb_gru_fwd", ctx.handle, ctx.stream, p(wi), p(wh), p(b), p(x), p(h0), p(alone), None, None, I, H, T, B)
+    assert ctx.device_error() == 0 and torch.equal(alone, out)
+    leaf = lambda t: t.double().requires_grad_()
+    rwi, rwh, rb, rx = map(leaf, (wi, wh, b, x))
+    zero = torch.zeros(B, H, device="cuda", dtype=torch.double)
+    ref, rh, rc = _reference(cell, rwi, rwh, rb, rx, h0.double() if states else zero, c0.double() if c0 is not None else zero)
+    total = (ref * dout.double()).sum()
+    if states:
+        total = total + (rh * dhT.double()).sum() + ((rc * dcT.double()).sum() if cell == "lstm" else 0.0)
+    total.backward()
+
+    def close(got, want, tol, name):
+        err = float((got.double() - want).abs().max() / want.abs().max())
+        assert err < tol, (name, err)
+    close(out, ref.detach(), 5e-6, "out")
+    close(hT, rh.detach(), 5e-6, "hT")
+    if cell == "lstm":
+        close(cT, rc.detach(), 5e-6, "cT")
+    for got, want, name in ((dwi, rwi, "dWi"), (dwh, rwh, "dWh"), (db, rb, "db")):
+        if name != "dWh" or T > 1 or states:
+            close(got, want.grad, 2e-5, name)
+    for i in range(B):                                # every column by its own largest value
+        close(dx[i], rx.grad[i], 2e-5, "dx")
+
+
+def test_a_sequence_inside_a_graph_beside_another_stream():
+    """The exchange buffer belongs to the call: replays and eager calls on another stream give what each gives alone."""
+    import fluxb200 as F
+    from fluxb200 import lib
+    ctx = F.context(0)
+    g = torch.Generator(device="cuda").manual_seed(0)
+    H, B, T, I = 96, 12, 20, 16
+    new = lambda *s: torch.randn(*s, generator=g, device="cuda")
+    wi, wh, b = new(I, 4 * H) / 4, new(H, 4 * H) / 10, new(4 * H) * 0.1
+    xs = [new(B, T, I), new(B, T, I)]
+    outs = [torch.empty(B, T, H, device="cuda") for _ in range(2)]
+    caches = [torch.empty(lib.raw().fb_lstm_cache_bytes(I, H, T, B) // 4, device="cuda") for _ in range(2)]
+
+    def call(k):
+        lib.call("fb_lstm_fwd", ctx.handle, ctx.stream, wi.data_ptr(), wh.data_ptr(), b.data_ptr(), xs[k].data_ptr(), None, None, outs[k].data_ptr(), None, None,
+                 caches[k].data_ptr(), I, H, T, B)
+    want = []
+    for k in range(2):
+        call(k)
+        torch.cuda.synchronize()
+        want.append(outs[k].clone())
+    graph, side = torch.cuda.CUDAGraph(), torch.cuda.Stream()
+    with torch.cuda.graph(graph):
+        call(0)
+    torch.cuda.synchronize()
+    for _ in range(5):
+        outs[0].zero_()
+        outs[1].zero_()
+        torch.cuda.synchronize()
+        graph.replay()
+        with torch.cuda.stream(side):
+            call(1)
+        torch.cuda.synchronize()
+        assert torch.equal(outs[0], want[0]) and torch.equal(outs[1], want[1]) and ctx.device_error() == 0
