@@ -11,8 +11,8 @@
 // stage ring and the two accumulator buffers in tensor memory run on across tiles, so the epilogue of one tile
 // overlaps the main loop of the next.
 //
-// Warp roles: warp 0 issues the TMA loads, warp 1 owns tensor memory and issues the MMAs, warps 2-5 are the
-// epilogue (one TMEM lane quadrant each).  In a pair the leader's MMA reads both CTAs' shared memory, so both CTAs'
+// Warp roles: warp 0 issues the TMA loads, warp 1 owns tensor memory and issues the MMAs, warps 2-9 are the
+// epilogue (warp w: TMEM lane quadrant w % 4, one half of the columns).  In a pair the leader's MMA reads both CTAs' shared memory, so both CTAs'
 // loads (cta_group::2 form) complete on the LEADER's full barrier, which expects the bytes of both halves.
 //
 // Operand layouts in shared memory are the canonical 128-byte-swizzle layouts the MMA descriptors name: K-major
@@ -31,6 +31,7 @@ namespace {
 constexpr int HBM_ = 128;            // rows of A per CTA
 constexpr int HBK = 64;              // bf16 values per k-block (128 bytes)
 constexpr uint32_t LAYOUT_SW128 = 2;
+constexpr int EPI_WARPS = 8;         // two per TMEM lane quadrant, each with half of the tile's columns
 
 template <int BN, bool PAIR>
 struct HCfg {
@@ -39,11 +40,12 @@ struct HCfg {
   static constexpr int B_BYTES = BNC * HBK * 2;               // 16 KB at 128 columns
   static constexpr int STAGE_BYTES = A_BYTES + B_BYTES;
   static constexpr int STAGES = (196608 / STAGE_BYTES) > 8 ? 8 : (196608 / STAGE_BYTES);
-  static constexpr int BAR_OFFSET = STAGES * STAGE_BYTES;
+  static constexpr int OUT_OFFSET = STAGES * STAGE_BYTES;     // 4 KB of each epilogue warp on their way to C
+  static constexpr int BAR_OFFSET = OUT_OFFSET + EPI_WARPS * 4096;
   static constexpr int SMEM_BYTES = BAR_OFFSET + 512 + 1024;  // barriers + alignment slack
   static constexpr int TMEM_COLS = 2 * BN;                    // two accumulator buffers
-  static constexpr int NUM_THREADS = 32 * 6;
-  static constexpr uint32_t ARRIVALS = PAIR ? 8 : 4;          // epilogue warps arriving on tmem_empty
+  static constexpr int NUM_THREADS = 32 * (2 + EPI_WARPS);
+  static constexpr uint32_t ARRIVALS = (PAIR ? 2 : 1) * EPI_WARPS;   // epilogue warps arriving on tmem_empty
 };
 
 __device__ __forceinline__ uint32_t pack_bf16(float lo, float hi) {
@@ -298,6 +300,8 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
   } else {
     // -------------------------------------------------------------- epilogue warps ---
     const int q = warp & 3;                 // TMEM lane quadrant this warp may read
+    const int half = (warp - 2) >> 2;       // its half of the columns
+    uint4* stage = (uint4*)(smem + cfg::OUT_OFFSET) + (warp - 2) * 256;
     bool ok = true;
     int tc = 0;
     for (int t = tile_beg; t < num_tiles && ok; t += tile_step, ++tc) {
@@ -308,47 +312,75 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
       if (!ok) break;
       tc_fence_after();
 #pragma unroll 1
-      for (int cc = 0; cc < BN / 32; ++cc) {
-        const int nb = n0 + cc * 32;
+      for (int cc = 0; cc < BN / 128; ++cc) {     // 64 columns at a time
+        const int c0 = half * (BN / 2) + cc * 64, nb = n0 + c0;
         if (nb >= N) break;   // warp-uniform
-        uint32_t r[32];
-        tc_ld_32x32b_x32(tmem_base + ((uint32_t)(32 * q) << 16) + (uint32_t)(buf * BN + cc * 32), r);
-        tc_wait_ld();
-        float* v = reinterpret_cast<float*>(r);
+        const uint32_t acc = tmem_base + ((uint32_t)(32 * q) << 16) + (uint32_t)(buf * BN + c0);
         if (SPLIT) {   // all MMAs have read their stages: the sums go where the cluster can add them up
-          float4* d4 = (float4*)((float*)smem + (32 * q + lane) * (BN + 4) + cc * 32);
 #pragma unroll
-          for (int j = 0; j < 8; ++j) d4[j] = make_float4(v[4 * j], v[4 * j + 1], v[4 * j + 2], v[4 * j + 3]);
-        } else if (out_f32 || nb + 31 >= N) {
+          for (int h = 0; h < 2; ++h) {
+            uint32_t r[32];
+            tc_ld_32x32b_x32(acc + 32u * (uint32_t)h, r);
+            tc_wait_ld();
+            const float* v = reinterpret_cast<const float*>(r);
+            float4* d4 = (float4*)((float*)smem + (32 * q + lane) * (BN + 4) + c0 + 32 * h);
 #pragma unroll
-          for (int j = 0; j < 4; ++j) emit8(row, v + 8 * j, nb + 8 * j);
-        } else if (row < M) {
-          // the usual case apart from emit8, whose code for the others between the pieces costs 1 - 2 us a launch (608 x 64 x
-          // 376: 10.3 us, so 8.3; 4096 x 2048 x 4096 with gelu 77 and 72)
-          uint16_t* crow = (uint16_t*)Cv + (int64_t)row * ldc + nb;
-          uint16_t* zrow = Z ? Z + (int64_t)row * ldc + nb : nullptr;
-#pragma unroll
-          for (int j = 0; j < 4; ++j) {       // 8 columns = one 16-byte store
-            float u[8];
-#pragma unroll
-            for (int e = 0; e < 8; ++e) u[e] = v[8 * j + e];
-            if (accumulate) {
-              const uint4 c4 = *(const uint4*)(crow + 8 * j);
-              u[0] += bf16_lo(c4.x); u[1] += bf16_hi(c4.x); u[2] += bf16_lo(c4.y); u[3] += bf16_hi(c4.y);
-              u[4] += bf16_lo(c4.z); u[5] += bf16_hi(c4.z); u[6] += bf16_lo(c4.w); u[7] += bf16_hi(c4.w);
-            }
-            if (bias_n) {
-              const uint4 b4 = __ldg((const uint4*)(bias_n + nb + 8 * j));
-              u[0] += bf16_lo(b4.x); u[1] += bf16_hi(b4.x); u[2] += bf16_lo(b4.y); u[3] += bf16_hi(b4.y);
-              u[4] += bf16_lo(b4.z); u[5] += bf16_hi(b4.z); u[6] += bf16_lo(b4.w); u[7] += bf16_hi(b4.w);
-            }
-            if (zrow) *(uint4*)(zrow + 8 * j) = make_uint4(pack_bf16(u[0], u[1]), pack_bf16(u[2], u[3]), pack_bf16(u[4], u[5]), pack_bf16(u[6], u[7]));
-            if (act != FB_ACT_IDENTITY) {
-#pragma unroll
-              for (int e = 0; e < 8; ++e) u[e] = fb_act_apply(act, u[e]);
-            }
-            *(uint4*)(crow + 8 * j) = make_uint4(pack_bf16(u[0], u[1]), pack_bf16(u[2], u[3]), pack_bf16(u[4], u[5]), pack_bf16(u[6], u[7]));
+            for (int j = 0; j < 8; ++j) d4[j] = make_float4(v[4 * j], v[4 * j + 1], v[4 * j + 2], v[4 * j + 3]);
           }
+        } else if (out_f32 || accumulate || nb + 63 >= N) {
+#pragma unroll 1
+          for (int h = 0; h < 2; ++h) {
+            if (nb + 32 * h >= N) break;
+            uint32_t r[32];
+            tc_ld_32x32b_x32(acc + 32u * (uint32_t)h, r);
+            tc_wait_ld();
+            float* v = reinterpret_cast<float*>(r);
+#pragma unroll
+            for (int j = 0; j < 4; ++j) emit8(row, v + 8 * j, nb + 32 * h + 8 * j);
+          }
+        } else {
+          // The usual case: a lane rounds 64 values of its row, and eight lanes store a row's 128 bytes (16384 x 1024 x 1024: 41.5
+          // -> 39.3 us against 16 bytes of 32 rows at a time by four warps; longer sums hide their stores).
+          const int r0 = tile_m0(t) + 32 * q + (lane >> 3);
+          auto store = [&](uint16_t* to, const uint4 (&w)[8]) {
+#pragma unroll
+            for (int j = 0; j < 8; ++j) stage[lane * 8 + (j ^ (lane & 7))] = w[j];
+            __syncwarp();
+            uint16_t* dst = to + (int64_t)r0 * ldc + nb + 8 * (lane & 7);
+#pragma unroll
+            for (int i = 0; i < 8; ++i) {
+              const int r = 4 * i + (lane >> 3);
+              const uint4 x = stage[r * 8 + ((lane & 7) ^ (r & 7))];
+              if (r0 + 4 * i < M) *(uint4*)(dst + (int64_t)(4 * i) * ldc) = x;
+            }
+            __syncwarp();
+          };
+          uint4 w[8], wa[8];   // before and behind the activation
+#pragma unroll
+          for (int h = 0; h < 2; ++h) {
+            uint32_t r[32];
+            tc_ld_32x32b_x32(acc + 32u * (uint32_t)h, r);
+            tc_wait_ld();
+            float* v = reinterpret_cast<float*>(r);
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+              float* u = v + 8 * j;
+              if (bias_n) {
+                const uint4 b4 = __ldg((const uint4*)(bias_n + nb + 32 * h + 8 * j));
+                u[0] += bf16_lo(b4.x); u[1] += bf16_hi(b4.x); u[2] += bf16_lo(b4.y); u[3] += bf16_hi(b4.y);
+                u[4] += bf16_lo(b4.z); u[5] += bf16_hi(b4.z); u[6] += bf16_lo(b4.w); u[7] += bf16_hi(b4.w);
+              }
+              w[4 * h + j] = make_uint4(pack_bf16(u[0], u[1]), pack_bf16(u[2], u[3]), pack_bf16(u[4], u[5]), pack_bf16(u[6], u[7]));
+              if (act != FB_ACT_IDENTITY) {
+#pragma unroll
+                for (int e = 0; e < 8; ++e) u[e] = fb_act_apply(act, u[e]);
+                wa[4 * h + j] = make_uint4(pack_bf16(u[0], u[1]), pack_bf16(u[2], u[3]), pack_bf16(u[4], u[5]), pack_bf16(u[6], u[7]));
+              }
+            }
+          }
+          if (Z) store(Z, w);
+          if (act == FB_ACT_IDENTITY) store((uint16_t*)Cv, w);
+          else store((uint16_t*)Cv, wa);
         }
       }
       // this buffer may be overwritten once every epilogue warp (of both CTAs) has read its quadrant
