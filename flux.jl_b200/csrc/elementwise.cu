@@ -483,6 +483,53 @@ FB_API int32_t fb_round_bf16(fb_ctx* ctx, void* stream, const float* x, float* y
   return FB_OK;
 }
 
+// out = a + b in Float32, each term Float32 or BFloat16 (out may be one of them): a sum of two arrays in one pass
+template <bool AB, bool BB>
+__global__ void __launch_bounds__(EW_THREADS)
+add_kernel(const void* a, const void* b, float* out, int64_t count, int vec) {
+  const int64_t tid = (int64_t)blockIdx.x * EW_THREADS + threadIdx.x, stride = (int64_t)gridDim.x * EW_THREADS;
+  auto four = [](const void* p, bool low, int64_t i, float (&v)[4]) {
+    if (low) {
+      const uint2 w = ((const uint2*)p)[i];
+      v[0] = __uint_as_float(w.x << 16); v[1] = __uint_as_float(w.x & 0xffff0000u);
+      v[2] = __uint_as_float(w.y << 16); v[3] = __uint_as_float(w.y & 0xffff0000u);
+    } else {
+      const float4 q = ((const float4*)p)[i];
+      v[0] = q.x; v[1] = q.y; v[2] = q.z; v[3] = q.w;
+    }
+  };
+  auto one = [](const void* p, bool low, int64_t i) {
+    return low ? __uint_as_float((uint32_t)((const uint16_t*)p)[i] << 16) : ((const float*)p)[i];
+  };
+  int64_t done = 0;
+  if (vec) {
+    done = count & ~int64_t(3);
+    for (int64_t i = tid; i < (count >> 2); i += stride) {
+      float x[4], y[4];
+      four(a, AB, i, x);
+      four(b, BB, i, y);
+      ((float4*)out)[i] = make_float4(x[0] + y[0], x[1] + y[1], x[2] + y[2], x[3] + y[3]);
+    }
+  }
+  for (int64_t i = done + tid; i < count; i += stride) out[i] = one(a, AB, i) + one(b, BB, i);
+}
+
+FB_API int32_t fb_add_mixed(fb_ctx* ctx, void* stream_, const void* a, int32_t a_bf16, const void* b, int32_t b_bf16, float* out, int64_t count) {
+  FB_CHECK_CTX(ctx);
+  FB_REQUIRE(count >= 0, FB_ERR_INVALID_ARG, "fb_add_mixed: negative count");
+  if (count == 0) return FB_OK;
+  FB_REQUIRE(a && b && out, FB_ERR_INVALID_ARG, "fb_add_mixed: NULL pointer");
+  cudaStream_t stream = (cudaStream_t)stream_;
+  const int vec = fb_aligned16(a) && fb_aligned16(b) && fb_aligned16(out);
+  const unsigned grid = ew_grid(ctx, vec ? (count + 3) / 4 : count);
+  if (a_bf16 && b_bf16) add_kernel<true, true><<<grid, EW_THREADS, 0, stream>>>(a, b, out, count, vec);
+  else if (a_bf16) add_kernel<true, false><<<grid, EW_THREADS, 0, stream>>>(a, b, out, count, vec);
+  else if (b_bf16) add_kernel<false, true><<<grid, EW_THREADS, 0, stream>>>(a, b, out, count, vec);
+  else add_kernel<false, false><<<grid, EW_THREADS, 0, stream>>>(a, b, out, count, vec);
+  FB_LAUNCH_CHECK();
+  return FB_OK;
+}
+
 FB_API int32_t fb_cast_f32_bf16(fb_ctx* ctx, void* stream, const float* x, uint16_t* y, int64_t count) {
   FB_CHECK_CTX(ctx);
   FB_REQUIRE(count >= 0, FB_ERR_INVALID_ARG, "fb_cast_f32_bf16: negative count");

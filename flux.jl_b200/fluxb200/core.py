@@ -94,7 +94,7 @@ class B200Array:
         return len(self.size)
 
     def numel(self):
-        return self.t.numel()
+        return math.prod(self.size)
 
     def reshape(self, *size):
         """Julia `reshape`: same memory, new column-major shape (no tape entry needed: identity pullback)."""
@@ -175,25 +175,38 @@ def cpu(x):
 
 
 def is_bf16(a) -> bool:
-    return isinstance(a, B200Array) and a.t.dtype == torch.bfloat16
+    return isinstance(a, B200Array) and not isinstance(a, (Scaled, Widened)) and a.t.dtype == torch.bfloat16
 
 
 def to_bf16(a: B200Array) -> B200Array:
     """Float32 -> BFloat16 storage (round to nearest even, bit-exact with Flux._to_bf16, src/functor.jl:161-166).
     Under `withgradient` the cast is recorded: the cotangent comes back in the input's element type."""
-    if a is None or a.t.dtype == torch.bfloat16:
+    if a is None or is_bf16(a):
         return a
+    if isinstance(a, Widened) and not a.backed:
+        return a.base     # (the cast back is exact)
     ctx = context()
     out = empty(a.size, torch.bfloat16)
     lib.call("fb_cast_f32_bf16", ctx.handle, ctx.stream, a.ptr, out.ptr, a.numel())
     if Tape.needs(a):
-        Tape.record(out, [a], lambda gs, src=a: [(src, to_f32(gs[0]))])
+        Tape.record(out, [a], lambda gs, src=a: [(src, widened(gs[0]))])
     return out
+
+
+def shared_bf16(a: B200Array, n: int):
+    """n results of to_bf16(a) that share one cast; each has its own place in the tape, so that their cotangents are added up in
+    Float32 as those of n casts are."""
+    first = to_bf16(a)
+    rest = [_wrap(first.t, first.size) for _ in range(n - 1)]
+    if Tape.needs(a):
+        for out in rest:
+            Tape.record(out, [a], lambda gs, src=a: [(src, widened(gs[0]))])
+    return [first] + rest
 
 
 def to_f32(a: B200Array) -> B200Array:
     """BFloat16 -> Float32 storage (exact)."""
-    if a is None or a.t.dtype != torch.bfloat16:
+    if a is None or not is_bf16(a):
         return a
     ctx = context()
     out = empty(a.size)
@@ -224,6 +237,39 @@ class Scaled(B200Array):
             lib.call("fb_scale", ctx.handle, ctx.stream, self.base.ptr, self.factor, out.ptr, out.numel())
             self._value = out.t
         return self._value
+
+
+class Widened(B200Array):
+    """A Float32 cotangent whose values are those of the BFloat16 array `base`.  Its memory exists from the first reader on;
+    what adds it to another gradient or can read BFloat16 takes `base` itself (`narrow`)."""
+
+    __slots__ = ("base", "_value")
+
+    def __init__(self, base: B200Array):
+        self.size, self._node = base.size, None
+        self.base, self._value = base, None
+
+    @property
+    def backed(self) -> bool:
+        return self._value is not None
+
+    @property
+    def t(self):
+        if self._value is None:
+            ctx, out = context(), empty(self.size)
+            lib.call("fb_cast_bf16_f32", ctx.handle, ctx.stream, self.base.ptr, out.ptr, out.numel())
+            self._value = out.t
+        return self._value
+
+
+def widened(g: B200Array) -> B200Array:
+    """to_f32 of a cotangent, as late as possible."""
+    return Widened(g) if is_bf16(g) else g
+
+
+def narrow(g: B200Array) -> B200Array:
+    """The array behind a cotangent that is a BFloat16 array's values, or the cotangent."""
+    return g.base if isinstance(g, Widened) and not g.backed else g
 
 
 def unscaled(g: B200Array):
@@ -287,4 +333,8 @@ def accumulate(grads: dict, owned: set, arr: B200Array, g: B200Array):
         g = to_bf16(g)
         lib.call("fb_axpy_bf16", ctx.handle, ctx.stream, 1.0, g.ptr, acc.ptr, g.numel())
     else:
-        lib.call("fb_axpy", ctx.handle, ctx.stream, 1.0, to_f32(g).ptr, acc.ptr, g.numel())
+        g = narrow(g)
+        if is_bf16(g):
+            lib.call("fb_add_mixed", ctx.handle, ctx.stream, acc.ptr, 0, g.ptr, 1, acc.ptr, g.numel())
+        else:
+            lib.call("fb_axpy", ctx.handle, ctx.stream, 1.0, g.ptr, acc.ptr, g.numel())

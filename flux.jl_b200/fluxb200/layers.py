@@ -14,7 +14,7 @@ import numpy as np
 import torch
 
 from . import lib
-from .core import B200Array, Tape, context, empty, gpu, is_bf16, to_bf16, to_f32, unscaled, zeros
+from .core import B200Array, Tape, context, empty, gpu, is_bf16, narrow, shared_bf16, to_bf16, to_f32, unscaled, zeros
 from .init import glorot_uniform
 
 
@@ -100,8 +100,13 @@ class Chain(Layer):
         self.layers = tuple(layers)
 
     def __call__(self, x):
-        for l in self.layers:
-            x = l(x)
+        last = len(self.layers) - 1
+        for i, l in enumerate(self.layers):
+            # the normalised rows that only a bf16 Dense reads are stored as it reads them
+            if type(l) is LayerNorm and i < last and type(self.layers[i + 1]) is Dense and is_bf16(self.layers[i + 1].weight):
+                x = l(x, low=True)
+            else:
+                x = l(x)
         return x
 
     def __getitem__(self, i):
@@ -306,13 +311,17 @@ class LayerNorm(Layer):
     def __repr__(self):
         return f"LayerNorm({', '.join(map(str, self.size))})"
 
-    def __call__(self, x: B200Array) -> B200Array:
-        x = to_f32(x)
+    def __call__(self, x: B200Array, low=False) -> B200Array:
+        """`low`: y as a BFloat16 array (for Chain, in front of a layer that would cast it)."""
+        d = math.prod(self.size)
+        mixed = (low or is_bf16(x)) and d % 8 == 0 and d <= 8192 and x.ptr % 16 == 0 and (
+            not self.affine or (self.diag.scale.ptr | self.diag.bias.ptr) % 16 == 0)
+        if not mixed:
+            x = to_f32(x)
         if self.affine:
             _wait_params(self.diag.scale, self.diag.bias)
-            for d, s in enumerate(self.size):
-                _size_check(self, x, d + 1, s)
-        d = math.prod(self.size)
+            for i, s in enumerate(self.size):
+                _size_check(self, x, i + 1, s)
         if x.numel() % d != 0 or x.size[:len(self.size)] != self.size:
             raise DimensionMismatch(f"layer {self} expects leading dims {self.size}, got {x}")
         n = x.numel() // d
@@ -320,7 +329,10 @@ class LayerNorm(Layer):
         act = lib.ACT[self.λ]
         g = self.diag.scale if self.affine else None
         b = self.diag.bias if self.affine else None
-        y, mean, rstd = empty(x.size), empty((n,)), empty((n,))
+        mean, rstd = empty((n,)), empty((n,))
+        if mixed:
+            return self._call_mixed(x, low, mean, rstd, d, n, g, b)
+        y = empty(x.size)
         lib.call("fb_layernorm_fwd", ctx.handle, ctx.stream, x.ptr, _ptr(g), _ptr(b), y.ptr, mean.ptr, rstd.ptr, d, n,
                  self.ε, act)
         if Tape.active:
@@ -347,6 +359,36 @@ class LayerNorm(Layer):
 
             Tape.record(y, [x, g, b], pullback)
         return y
+
+
+def _layernorm_call_mixed(self, x, low, mean, rstd, d, n, g, b):
+    """The LayerNorm call where x is a BFloat16 array or y becomes one: what the casts around the Float32 kernels would give."""
+    ctx, act = context(), lib.ACT[self.λ]
+    y = empty(x.size, torch.bfloat16 if low else torch.float32)
+    lib.call("fb_layernorm_fwd_mixed", ctx.handle, ctx.stream, x.ptr, int(is_bf16(x)), _ptr(g), _ptr(b), y.ptr, int(low), mean.ptr, rstd.ptr,
+             d, n, self.ε, act)
+    if Tape.active:
+        def pullback(gs, x=x):
+            dy = narrow(gs[0])
+            sink = Tape.grad_sink
+            need_dx = Tape.needs(x)
+            if g is None and not need_dx:
+                return []
+            dx = empty(x.size, x.t.dtype) if need_dx else None
+            dg = ((sink.buffer_for(g) if sink else None) or empty(g.size)) if g is not None else None
+            dbeta = ((sink.buffer_for(b) if sink else None) or empty(b.size)) if b is not None else None
+            lib.call("fb_layernorm_bwd_mixed", ctx.handle, ctx.stream, x.ptr, int(is_bf16(x)), _ptr(g), _ptr(b), mean.ptr, rstd.ptr, dy.ptr,
+                     int(is_bf16(dy)), _ptr(dx), _ptr(dg), _ptr(dbeta), d, n, act)
+            res = [(x, dx)] if need_dx else []
+            if g is not None:
+                res += [(g, dg), (b, dbeta)]
+            return res
+
+        Tape.record(y, [x, g, b], pullback)
+    return y
+
+
+LayerNorm._call_mixed = _layernorm_call_mixed
 
 
 # -------------------------------------------------------------------------------- BatchNorm ---
@@ -798,6 +840,8 @@ class MultiHeadAttention(Layer):
         for a in (q_in, k_in, v_in):
             if a.ndim != 3:
                 raise TypeError("MethodError: MultiHeadAttention expects 3-d arrays (features, len, batch)")
+        if not is_bf16(q_in) and q_in is k_in and k_in is v_in and all(type(p) is Dense and is_bf16(p.weight) for p in (self.q_proj, self.k_proj, self.v_proj)):
+            q_in, k_in, v_in = shared_bf16(q_in, 3)     # one cast for the three
         q = self.q_proj(q_in)
         k = self.k_proj(k_in)
         v = self.v_proj(v_in)

@@ -67,6 +67,8 @@ PROTOTYPES = {
     "fb_layernorm_fwd": (_i32, [_p, _p, _p, _p, _p, _p, _p, _p, _i64, _i64, _f, _i32]),
     "fb_layernorm_bwd": (_i32, [_p, _p, _p, _p, _p, _p, _p, _p, _p, _p, _p, _i64, _i64, _i32]),
     "fb_layernorm_bwd_params": (_i32, [_p] * 8 + [_f, _p, _p, _i64, _i64, _i32]),
+    "fb_layernorm_fwd_mixed": (_i32, [_p, _p, _p, _i32, _p, _p, _p, _i32, _p, _p, _i64, _i64, _f, _i32]),
+    "fb_layernorm_bwd_mixed": (_i32, [_p, _p, _p, _i32, _p, _p, _p, _p, _p, _i32, _p, _p, _p, _i64, _i64, _i32]),
     "fb_layernorm_bwd_noalloc": (_i32, [_p, _p, _p, _p, _p, _p, _p, _p, _p, _p, _i64, _i64, _i32]),
     "fb_batchnorm_fwd_train": (_i32, [_p, _p, _p, _p, _p, _p, _p, _p, _p, _p, _i64, _i64, _i64, _f, _f, _i32, _i32]),
     "fb_batchnorm_fwd_infer": (_i32, [_p, _p, _p, _p, _p, _p, _p, _p, _i64, _i64, _i64, _f, _i32]),
@@ -86,6 +88,7 @@ PROTOTYPES = {
     "fb_fill": (_i32, [_p, _p, _p, _f, _i64]),
     "fb_scale": (_i32, [_p, _p, _p, _f, _p, _i64]),
     "fb_axpy": (_i32, [_p, _p, _f, _p, _p, _i64]),
+    "fb_add_mixed": (_i32, [_p, _p, _p, _i32, _p, _i32, _p, _i64]),
     "fb_cast_f32_bf16": (_i32, [_p, _p, _p, _p, _i64]),
     "fb_cast_bf16_f32": (_i32, [_p, _p, _p, _p, _i64]),
     "fb_round_bf16": (_i32, [_p, _p, _p, _p, _i64]),

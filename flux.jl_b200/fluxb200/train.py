@@ -14,7 +14,7 @@ import numpy as np
 import torch
 
 from . import lib
-from .core import B200Array, Scaled, Tape, accumulate, context, empty, gpu, to_bf16, to_f32, zeros
+from .core import B200Array, Scaled, Tape, accumulate, context, empty, gpu, is_bf16, to_bf16, to_f32, zeros
 from .layers import DimensionMismatch, Layer, trainables
 
 
@@ -109,14 +109,18 @@ def sum_all(y: B200Array) -> B200Array:
 
 def add(a: B200Array, b: B200Array) -> B200Array:
     """a + b for two arrays of one size (e.g. two loss terms); the cotangent goes to both."""
-    a, b = to_f32(a), to_f32(b)
     if a.size != b.size:
         raise DimensionMismatch(f"dimensions must match: a has dims {a.size}, b has dims {b.size}")
     ctx = context()
-    out = B200Array(a.t.clone(), a.size)
-    lib.call("fb_axpy", ctx.handle, ctx.stream, 1.0, b.ptr, out.ptr, out.numel())
+    if is_bf16(a) or is_bf16(b):
+        out = empty(a.size)
+        lib.call("fb_add_mixed", ctx.handle, ctx.stream, a.ptr, int(is_bf16(a)), b.ptr, int(is_bf16(b)), out.ptr, out.numel())
+    else:
+        out = B200Array(a.t.clone(), a.size)
+        lib.call("fb_axpy", ctx.handle, ctx.stream, 1.0, b.ptr, out.ptr, out.numel())
     if Tape.needs(a, b):
-        Tape.record(out, [a, b], lambda gs: [(a, gs[0]), (b, gs[0])])
+        # (a BFloat16 term's cotangent is the cast's; one that nothing needs is not cast)
+        Tape.record(out, [a, b], lambda gs: [(v, to_bf16(gs[0]) if is_bf16(v) and Tape.needs(v) else gs[0]) for v in (a, b)])
     return out
 
 

@@ -184,6 +184,16 @@ int32_t fb_layernorm_bwd_params(fb_ctx* ctx, void* stream, const float* x, const
                                 const float* mean, const float* rstd, const float* dy, float dy_scale,
                                 float* dgamma, float* dbeta, int64_t d, int64_t n, int32_t act);
 
+/* fb_layernorm_fwd / fb_layernorm_bwd where x (and dx with it), y and dy may be BFloat16 arrays (raw bits in uint16): x_bf16,
+ * y_bf16, dy_bf16 say which.  Parameters, statistics and all arithmetic are Float32, as if the arrays were cast on the
+ * way.  dx may be NULL.  Arrays must be 16-byte aligned and d a multiple of 8 up to 8192 (FB_ERR_UNSUPPORTED otherwise). */
+int32_t fb_layernorm_fwd_mixed(fb_ctx* ctx, void* stream, const void* x, int32_t x_bf16, const float* gamma,
+                               const float* beta, void* y, int32_t y_bf16, float* mean, float* rstd, int64_t d, int64_t n,
+                               float eps, int32_t act);
+int32_t fb_layernorm_bwd_mixed(fb_ctx* ctx, void* stream, const void* x, int32_t x_bf16, const float* gamma,
+                               const float* beta, const float* mean, const float* rstd, const void* dy, int32_t dy_bf16,
+                               void* dx, float* dgamma, float* dbeta, int64_t d, int64_t n, int32_t act);
+
 /* fb_layernorm_bwd for callers that may not allocate device memory (a process whose memory budget is fixed at
  * start-up, code inside a stream capture, runtime threads that must not risk the implicit synchronisation of
  * cudaMalloc / cudaFree).  No counterpart in the reference; same arguments and results as fb_layernorm_bwd minus the
@@ -297,6 +307,8 @@ int32_t fb_timestamp(fb_ctx* ctx, void* stream, uint64_t* out_dev);
 int32_t fb_scale(fb_ctx* ctx, void* stream, const float* x, float alpha, float* y, int64_t count);
 /* y += alpha * x (tangent accumulation `+` of Zygote; `x .-= dx` of Optimisers.update!). */
 int32_t fb_axpy(fb_ctx* ctx, void* stream, float alpha, const float* x, float* y, int64_t count);
+/* out = a + b, each term a Float32 or (a_bf16 / b_bf16 != 0) a BFloat16 array; out may be a Float32 term. */
+int32_t fb_add_mixed(fb_ctx* ctx, void* stream, const void* a, int32_t a_bf16, const void* b, int32_t b_bf16, float* out, int64_t count);
 /* Float32 -> BFloat16 bits, round-to-nearest-even in the integer domain, NaN -> 0x7fc0; bit-exact
  * with Flux._to_bf16 (src/functor.jl:161-166). */
 int32_t fb_cast_f32_bf16(fb_ctx* ctx, void* stream, const float* x, uint16_t* y, int64_t count);

@@ -1,0 +1,108 @@
+"""GPU tests of the bf16 path where it makes no Float32 copies: LayerNorm on BFloat16 arrays in and out, casts and sums of both types
+at the edges of their pieces.  References are computed in
+float64 from the same rounded arrays; a BFloat16 result may be off by one rounding (2^-8 of the value) where a Float32
+result lies within 1e-5 of a tie, so these compare with 2^-8 of the element plus 1e-5 of the largest."""
+import ctypes as C
+
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+ACTS = {"identity": lambda v: v, "relu": torch.relu, "gelu_tanh": lambda v: torch.nn.functional.gelu(v, approximate="tanh")}
+BF = torch.bfloat16
+
+
+@pytest.fixture(scope="module")
+def ctx():
+    import fluxb200 as F
+    return F.context(0)
+
+
+def _p(t):
+    return C.c_void_p(t.data_ptr()) if t is not None else None
+
+
+def _close(got, ref, name, tol=1e-5):
+    lim = tol * ref.abs().max() + (2.0 ** -8 * ref.abs() if got.dtype == BF else 0.0)
+    assert bool(((got.double() - ref).abs() <= lim).all()), (name, float((got.double() - ref).abs().max()), float(ref.abs().max()))
+
+
+@pytest.mark.parametrize("d", [8, 248, 256, 264, 512, 520, 1024, 1032, 2048, 2056, 4096, 4104, 8192])
+@pytest.mark.parametrize("n,act", [(1, "identity"), (37, "gelu_tanh"), (600, "relu")])
+@pytest.mark.parametrize("xb,yb", [(0, 1), (1, 0), (1, 1), (0, 0)])
+def test_layernorm_mixed(ctx, d, n, act, xb, yb):
+    from fluxb200 import lib
+    g = torch.Generator(device="cuda").manual_seed(d + n)
+    new = lambda *s: torch.randn(*s, generator=g, device="cuda")
+    xt, yt = (BF if xb else torch.float32), (BF if yb else torch.float32)
+    x, dy, gamma, beta = (new(n, d) * 2 + 0.5).to(xt), new(n, d), new(d) * 0.1 + 1, new(d) * 0.1
+    xr, gr, br = (t.double().requires_grad_() for t in (x, gamma, beta))
+    z = torch.nn.functional.layer_norm(xr, (d,), gr, br, 1e-5)
+    if act == "relu":       # an element within rounding of zero may take either side
+        dy = torch.where(z.detach().abs() < 1e-4, 0.0, dy.double()).float()
+    dy = dy.to(yt)
+    y, dx = torch.empty(n, d, device="cuda", dtype=yt), torch.empty(n, d, device="cuda", dtype=xt)
+    mean, rstd, dg, db, dg2, db2 = (torch.empty(k, device="cuda") for k in (n, n, d, d, d, d))
+    a = lib.ACT[act]
+    lib.call("fb_layernorm_fwd_mixed", ctx.handle, ctx.stream, _p(x), xb, _p(gamma), _p(beta), _p(y), yb, _p(mean), _p(rstd), d, n, 1e-5, a)
+    lib.call("fb_layernorm_bwd_mixed", ctx.handle, ctx.stream, _p(x), xb, _p(gamma), _p(beta), _p(mean), _p(rstd), _p(dy), yb, _p(dx), _p(dg), _p(db), d, n, a)
+    lib.call("fb_layernorm_bwd_mixed", ctx.handle, ctx.stream, _p(x), xb, _p(gamma), _p(beta), _p(mean), _p(rstd), _p(dy), yb, None, _p(dg2), _p(db2), d, n, a)
+    ref = ACTS[act](z)
+    ref.backward(dy.double())
+    _close(y, ref.detach(), "y")
+    _close(dx, xr.grad, "dx", 2e-5)
+    _close(dg, gr.grad, "dgamma", 2e-5)
+    _close(db, br.grad, "dbeta", 2e-5)
+    assert torch.equal(dg, dg2) and torch.equal(db, db2)
+
+
+@pytest.mark.parametrize("n", [1, 7, 8, 9, 4099, 100000])
+@pytest.mark.parametrize("shift", [0, 1])
+def test_casts_and_sums(ctx, n, shift):
+    from fluxb200 import lib
+    g = torch.Generator(device="cuda").manual_seed(n)
+    a = torch.randn(n + shift, generator=g, device="cuda")[shift:]
+    if n > 8:
+        a[3], a[5] = float("inf"), float("nan")
+    low, back, out = torch.empty(n + shift, device="cuda", dtype=BF)[shift:], torch.empty(n + shift, device="cuda")[shift:], torch.empty(n, device="cuda")
+    lib.call("fb_cast_f32_bf16", ctx.handle, ctx.stream, _p(a), _p(low), n)
+    lib.call("fb_cast_bf16_f32", ctx.handle, ctx.stream, _p(low), _p(back), n)
+    assert torch.equal(low.isnan(), a.isnan()) and torch.equal(low[~a.isnan()], a.to(BF)[~a.isnan()]) and torch.equal(back[~a.isnan()], low.float()[~a.isnan()])
+    for x, y in ((a, low), (low, a), (low, low), (a, a)):
+        lib.call("fb_add_mixed", ctx.handle, ctx.stream, _p(x), int(x.dtype == BF), _p(y), int(y.dtype == BF), _p(out), n)
+        assert torch.equal(out.nan_to_num(7.0), (x.float() + y.float()).nan_to_num(7.0))
+
+
+def test_chain_without_copies_is_the_chain_with_them(ctx):
+    """LayerNorm -> bf16 Dense blocks in a Chain (no Float32 copies) and the same layers called one by one with casts between them: the
+    same bits in every result and gradient."""
+    import numpy as np
+
+    import fluxb200 as F
+    rng = np.random.default_rng(0)
+    d = 64
+    layers = []
+    for _ in range(2):
+        layers += [F.LayerNorm(d), F.Dense(rng.standard_normal((d, d), dtype=np.float32) / 8, rng.standard_normal(d, dtype=np.float32), "gelu")]
+    model = F.bf16(F.Chain(*layers))
+    x = F.gpu(rng.standard_normal((d, 40), dtype=np.float32))
+
+    def by_hand(m):
+        y = x
+        for layer in m.layers:
+            y = layer(F.f32(y))
+        return F.sum_abs2(y)
+    la, (ga,) = F.withgradient(lambda m: F.sum_abs2(m(x)), model)
+    lb, (gb,) = F.withgradient(by_hand, model)
+    assert la == lb
+
+    def flat(t):
+        if isinstance(t, dict):
+            return [v for k in t for v in flat(t[k])]
+        if isinstance(t, (tuple, list)):
+            return [v for k in t for v in flat(k)]
+        return [t.t] if isinstance(t, F.B200Array) else []
+    assert len(flat(ga)) == 8
+    for a, b in zip(flat(ga), flat(gb)):
+        assert a.dtype == b.dtype and float((a.double() - b.double()).abs().max()) <= 2e-6 * float(b.double().abs().max()) + (
+            2.0 ** -8 * float(b.double().abs().max()) if a.dtype == BF else 0.0)
