@@ -140,6 +140,24 @@ __device__ __forceinline__ uint32_t map_to_cta(uint32_t local_addr, uint32_t ran
   asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(local_addr), "r"(rank));
   return r;
 }
+// out[k] = sum over the cluster's CTAs, in rank order, of the n floats that each of them holds at `mine` in its shared memory, for
+// k < limit; a CTA adds up one slice.  Ends with every CTA past its reads.
+__device__ __forceinline__ void cluster_column_sums(const float* mine, int n, float* out, int64_t limit, uint32_t size) {
+  __syncwarp();
+  cluster_sync_all();
+  const int per = (n + (int)size - 1) / (int)size, k0 = (int)cluster_ctarank() * per;
+  for (int k = k0 + (int)threadIdx.x; k < n && k < k0 + per && k < limit; k += (int)blockDim.x) {
+    float s = 0.0f;
+    for (uint32_t r = 0; r < size; ++r) {
+      float v;
+      asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v) : "r"(map_to_cta(smem_u32(mine + k), r)) : "memory");
+      s += v;
+    }
+    out[k] = s;
+  }
+  __syncwarp();
+  cluster_sync_all();
+}
 __device__ __forceinline__ void mbar_arrive_cluster(uint32_t cluster_addr) {
   asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(cluster_addr) : "memory");
 }

@@ -94,7 +94,7 @@ class B200Array:
         return len(self.size)
 
     def numel(self):
-        return math.prod(self.size)
+        return self.t.numel()
 
     def reshape(self, *size):
         """Julia `reshape`: same memory, new column-major shape (no tape entry needed: identity pullback)."""
@@ -175,7 +175,7 @@ def cpu(x):
 
 
 def is_bf16(a) -> bool:
-    return isinstance(a, B200Array) and not isinstance(a, (Scaled, Widened)) and a.t.dtype == torch.bfloat16
+    return type(a) is B200Array and a.t.dtype == torch.bfloat16     # (a cotangent whose memory may not exist is Float32)
 
 
 def to_bf16(a: B200Array) -> B200Array:
@@ -206,7 +206,7 @@ def shared_bf16(a: B200Array, n: int):
 
 def to_f32(a: B200Array) -> B200Array:
     """BFloat16 -> Float32 storage (exact)."""
-    if a is None or not is_bf16(a):
+    if type(a) is not B200Array or a.t.dtype != torch.bfloat16:
         return a
     ctx = context()
     out = empty(a.size)
@@ -225,6 +225,9 @@ class Scaled(B200Array):
     def __init__(self, base: B200Array, factor: float):
         self.size, self._node = base.size, None
         self.base, self.factor, self._value = base, factor, None
+
+    def numel(self):
+        return self.base.numel()
 
     @property
     def backed(self) -> bool:
@@ -248,6 +251,9 @@ class Widened(B200Array):
     def __init__(self, base: B200Array):
         self.size, self._node = base.size, None
         self.base, self._value = base, None
+
+    def numel(self):
+        return self.base.numel()
 
     @property
     def backed(self) -> bool:

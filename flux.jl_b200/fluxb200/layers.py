@@ -100,10 +100,10 @@ class Chain(Layer):
         self.layers = tuple(layers)
 
     def __call__(self, x):
-        last = len(self.layers) - 1
-        for i, l in enumerate(self.layers):
+        layers = self.layers
+        for i, l in enumerate(layers):
             # the normalised rows that only a bf16 Dense reads are stored as it reads them
-            if type(l) is LayerNorm and i < last and type(self.layers[i + 1]) is Dense and is_bf16(self.layers[i + 1].weight):
+            if type(l) is LayerNorm and i + 1 < len(layers) and type(layers[i + 1]) is Dense and is_bf16(layers[i + 1].weight):
                 x = l(x, low=True)
             else:
                 x = l(x)
