@@ -9,6 +9,8 @@
 // backward, ordered by the stream.
 #include <stdlib.h>
 
+#include <type_traits>
+
 #include <cuda_fp16.h>
 
 #include "common.cuh"
@@ -554,12 +556,12 @@ bool plan_mma(const fb_ctx* ctx, int ng, int H, int64_t B, int64_t T, bool bwd, 
     const int nbg = (int)(nch < ctx->sm_count / ugroups ? nch : ctx->sm_count / ugroups);
     if (nbg < 1) continue;
     const int64_t chunks = (nch + nbg - 1) / nbg;
-    if (chunks > 64) continue;
+    if (chunks > MQ_CHUNKS) continue;
     const double t = chunks * (0.8 + 0.02 * bg) + 1.3;   // us of a step
     if (t < best_t) {
       best_t = t;
       best->ug = MQ_UG; best->bg = bg; best->nbg = nbg; best->grid = ugroups * nbg;
-      best->smem = bwd ? mq_bwd_smem(bg, (ng * mq_pad(H) + 511) / 512, (int)chunks) : mq_fwd_smem(ng, bg, H <= 128 ? 1 : H <= 256 ? 2 : 4, (int)chunks);
+      best->smem = bwd ? mq_bwd_smem((int)chunks, bg) : mq_fwd_smem(ng, bg, H <= 128 ? 1 : H <= 256 ? 2 : 4, (int)chunks);
     }
   }
   return best_t < 1e30 && best->smem <= ctx->smem_optin;
@@ -569,10 +571,10 @@ const void* mma_fwd_kernel(int bg, int H) {
   if (bg == 16) return H <= 128 ? (const void*)rnn_fwd_mma_kernel<NG, 16, 1> : H <= 256 ? (const void*)rnn_fwd_mma_kernel<NG, 16, 2> : (const void*)rnn_fwd_mma_kernel<NG, 16, 4>;
   return H <= 128 ? (const void*)rnn_fwd_mma_kernel<NG, 8, 1> : H <= 256 ? (const void*)rnn_fwd_mma_kernel<NG, 8, 2> : (const void*)rnn_fwd_mma_kernel<NG, 8, 4>;
 }
-template <int NG, int BG>
-const void* mma_bwd_kernel(int np) {
-  return np == 1 ? (const void*)rnn_bwd_mma_kernel<NG, BG, 1> : np == 2 ? (const void*)rnn_bwd_mma_kernel<NG, BG, 2>
-       : np == 3 ? (const void*)rnn_bwd_mma_kernel<NG, BG, 3> : (const void*)rnn_bwd_mma_kernel<NG, BG, 4>;
+template <int NG>
+const void* mma_bwd_kernel(int bg, int H) {
+  if (bg == 16) return H <= 128 ? (const void*)rnn_bwd_mma_kernel<NG, 16, 1> : H <= 256 ? (const void*)rnn_bwd_mma_kernel<NG, 16, 2> : (const void*)rnn_bwd_mma_kernel<NG, 16, 4>;
+  return H <= 128 ? (const void*)rnn_bwd_mma_kernel<NG, 8, 1> : H <= 256 ? (const void*)rnn_bwd_mma_kernel<NG, 8, 2> : (const void*)rnn_bwd_mma_kernel<NG, 8, 4>;
 }
 
 // Launches the whole forward / backward time loop; FB_ERR_UNSUPPORTED (without a message) when the hidden size does not fit.
@@ -617,16 +619,17 @@ int32_t launch_bwd_seq(fb_ctx* ctx, cudaStream_t stream, const float* Wh, const 
   int B = (int)B64, T = (int)T64;
   int32_t* dev_err = ctx->dev_error;
   if (plan_mma(ctx, NG, H, B64, T64, true, &p)) {
-    const size_t bytes = T64 > 1 ? (size_t)T64 * mq_run(B64, p.bg, NG * mq_pad(H)) * sizeof(float) : 0;   // (step 0 sends nothing)
+    const size_t slot = mq_part_run(B64, p.bg, H) * sizeof(float);
+    int ring = T64 < MQ_RING || T64 * slot <= MQ_ALL_STEPS ? T : MQ_RING;
+    const size_t bytes = T64 > 1 ? ring * slot : 0;
     const fb_temp mem(ctx, stream, bytes);
     if (bytes == 0 || mem.p != nullptr) {
       if (bytes != 0) FB_CUDA(cudaMemsetAsync(mem.p, 0xff, bytes, stream));
-      const int np = (NG * mq_pad(H) + 511) / 512;
-      const void* kern = p.bg == 16 ? mma_bwd_kernel<NG, 16>(np) : mma_bwd_kernel<NG, 8>(np);
+      const void* kern = mma_bwd_kernel<NG>(p.bg, H);
       float* ex = (float*)mem.p;
       void* args[] = {(void*)&Wh, (void*)&keep, (void*)&cst, (void*)&s0, (void*)&hout, (void*)&dout, (void*)&dhT, (void*)&dcT, (void*)&dg,
-                      (void*)&dgx, (void*)&ex, (void*)&H, (void*)&B, (void*)&T, (void*)&p.nbg, (void*)&dev_err};
-      FB_CUDA(fb_allow_smem(kern, ctx->smem_optin));
+                      (void*)&dgx, (void*)&ex, (void*)&H, (void*)&B, (void*)&T, (void*)&p.nbg, (void*)&ring, (void*)&dev_err};
+      FB_CUDA(fb_allow_smem(kern, mq_bwd_smem(MQ_CHUNKS, 16)));
       FB_CUDA(cudaLaunchCooperativeKernel(kern, dim3((unsigned)p.grid), dim3(SQ_THREADS), args, p.smem, stream));
       FB_LAUNCH_CHECK();
       return FB_OK;

@@ -18,12 +18,12 @@
 // A warp that meets a weight or a value that is not finite, or an |h| of 16 or more (a GRU's initial state; |h| <= 1 otherwise), sums the
 // products of that step in Float32 instead, from memory.
 //
-// What bounds it: T dependent steps: one store -> load flight through L2, then about 100 mma per warp (0.4 us), the sum over the
-// warps (0.3 us) and the gates (0.6 us).  H 512, B 64, T 256: forward 6.0 -> 3.0 us a step, backward 7.8 -> 4.5 (Float32 FMAs from
-// shared memory before: 2.3 us of a step by themselves).  Error against float64 is that of the FMA kernel.
+// What bounds it: T dependent steps (H 512, B 64: 5100 clocks): one store -> load flight through L2 (1200), the planes of h and 192 mma per
+// SM partition at 8.7 clocks each (2250), the sum over the warps and the gates (1300).  FMA kernels 6.0 us a step, here 2.8.  Error against
+// float64 is that of the FMA kernel.
 #pragma once
 
-constexpr int MQ_UG = 16;
+constexpr int MQ_UG = 16, MQ_CHUNKS = 64;   // units of a CTA, its chunks of columns at most
 
 __device__ __forceinline__ void mq_mma(float (&c)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
   asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%0, %1, %2, %3};"
@@ -59,6 +59,7 @@ __device__ __forceinline__ uint32_t mq_max_lanes(uint32_t m) {
   return max(m, __shfl_xor_sync(0xffffffffu, m, 2));
 }
 constexpr uint32_t MQ_INF = 0x7f800000u;
+constexpr int MQ_MODERATE = 56;   // shifts whose powers of two can be multiplied with each other
 
 // A fragments of KS k-steps: rows r and r + 8 of Ws, k-values k + 4 q .. of each step (k: the lane's first).  sh: the rows' shifts.
 // Returns whether all of them are finite.
@@ -134,6 +135,9 @@ __device__ __forceinline__ void mq_publish(float* run, int bg, int ks, int gu, i
   float* p = run + (size_t)ks * (bg * 16) + (gb >> 3) * 128 + (gb & 7) * 16 + gu;
   asm volatile("st.relaxed.gpu.global.u32 [%0], %1;" ::"l"(p), "r"(w) : "memory");
 }
+__device__ __forceinline__ void mq_put4(float* p, uint32_t a, uint32_t b, uint32_t c, uint32_t d) {
+  asm volatile("st.relaxed.gpu.global.v4.u32 [%0], {%1, %2, %3, %4};" ::"l"(p), "r"(a), "r"(b), "r"(c), "r"(d) : "memory");
+}
 // k-value k of column c of a run, as the exchange holds it
 template <int NT>
 __device__ __forceinline__ float mq_at(const float* run, int k, int c) {
@@ -145,12 +149,8 @@ __device__ __forceinline__ uint32_t mq_word(float v) {
 }
 
 inline size_t mq_fwd_smem(int ng, int bg, int ks, int chunks) {
-  const size_t w = (size_t)ng * MQ_UG * (128 * ks + 4), red = (size_t)2 * 8 * bg * (ng * MQ_UG + 4);
+  const size_t w = (size_t)ng * MQ_UG * (128 * ks + 4), red = (size_t)2 * 8 * bg * (MQ_UG + 1) * 4;
   return (w + red + (size_t)chunks * MQ_UG * bg) * 4;
-}
-inline size_t mq_bwd_smem(int bg, int np, int chunks) {
-  const size_t w = (size_t)MQ_UG * (512 * np + 4), red = (size_t)2 * 8 * bg * (MQ_UG + 4);
-  return ((w > red ? w : red) + (size_t)chunks * MQ_UG * bg) * 4;
 }
 
 // Arguments as for rnn_fwd_seq_kernel, and the exchange buffer (T - 1 runs); KS k-steps of 16 per warp: hidden sizes up to 128 KS.
@@ -159,11 +159,11 @@ __global__ void __launch_bounds__(SQ_THREADS, 1)
 rnn_fwd_mma_kernel(const float* __restrict__ Wh, const float* __restrict__ gx, const float* __restrict__ h0, const float* __restrict__ c0,
                    float* __restrict__ out, float* __restrict__ cache, float* __restrict__ cst, int cached, float* __restrict__ hT,
                    float* __restrict__ cT, float* ex, int H, int B, int T, int nbg, int32_t* dev_err) {
-  constexpr int UG = MQ_UG, R = NG * UG, NT = BG / 8, LD = 128 * KS + 4, LR = R + 4;
+  constexpr int UG = MQ_UG, R = NG * UG, NT = BG / 8, LD = 128 * KS + 4, LU = UG + 1;
   extern __shared__ __align__(16) float sm[];
   float* Ws = sm;                            // [R][LD], until the initial state has been multiplied
-  float* red = Ws + R * LD;                  // [2][8][BG][LR]
-  float* cs = red + 2 * 8 * BG * LR;         // [chunks][BG * UG]: LSTM c, GRU h
+  float4* red = (float4*)(Ws + R * LD);      // [2][8][BG][LU]: the gates of a unit and column side by side, in 16-byte accesses without conflicts
+  float* cs = (float*)(red + 2 * 8 * BG * LU);   // [chunks][BG * UG]: LSTM c, GRU h
   const int ugroups = (H + UG - 1) / UG;
   const int u0 = ((int)blockIdx.x % ugroups) * UG, bgrp = (int)blockIdx.x / ugroups;
   const int nchunks = (B + BG - 1) / BG;
@@ -188,8 +188,12 @@ rnn_fwd_mma_kernel(const float* __restrict__ Wh, const float* __restrict__ gx, c
 #pragma unroll
   for (int g = 0; g < NG; ++g) finite = mq_load_a<KS>(Ws, LD, g * UG + (lane >> 2), 16 * ks0 + 4 * q, ahi[g], alo[g], ash[g]) && finite;
   finite = __all_sync(0xffffffffu, finite);
+  bool moderate = true;
+#pragma unroll
+  for (int g = 0; g < NG; ++g) moderate = moderate && abs(ash[g][0]) <= MQ_MODERATE && abs(ash[g][1]) <= MQ_MODERATE;
   int turn = 0;
-  // the input projection of the next (step, chunk), on its way while this one waits for h
+  // The input projection of the next (step, chunk).  Asked for behind the poll: a poll that follows a load from DRAM returns no sooner
+  // than that (LSTM 512, batch 64: the wait for h 2200 -> 1150 clocks).
   float gxn[NG];
   auto ahead = [&](int t, int ch) {
     const int b = ch * BG + gb;
@@ -206,8 +210,6 @@ rnn_fwd_mma_kernel(const float* __restrict__ Wh, const float* __restrict__ gx, c
       float gxv[NG];
 #pragma unroll
       for (int g = 0; g < NG; ++g) gxv[g] = gxn[g];
-      if (ch + nbg < nchunks) ahead(t, ch + nbg);
-      else ahead(t + 1, bgrp);
       float pre[NG];
 #pragma unroll
       for (int g = 0; g < NG; ++g) pre[g] = 0.0f;
@@ -216,6 +218,7 @@ rnn_fwd_mma_kernel(const float* __restrict__ Wh, const float* __restrict__ gx, c
         MqPieces<NT, KS> pc;
         pc.template load<false>(src, nb, ks0, steps);
         const bool ok = pc.wait(src, nb, ks0, steps, dev_err);
+        ahead(ch + nbg < nchunks ? t : t + 1, ch + nbg < nchunks ? ch + nbg : bgrp);
         float acc[NG][NT][4];
 #pragma unroll
         for (int g = 0; g < NG; ++g)
@@ -234,7 +237,10 @@ rnn_fwd_mma_kernel(const float* __restrict__ Wh, const float* __restrict__ gx, c
           hsh[n] = mq_shift(m);
           small = small && m < 0x41800000u;   // 16
         }
-        float* rw = red + (size_t)(turn * 8 + warp) * BG * LR;
+        float4* rw = red + (turn * 8 + warp) * BG * LU + (lane >> 2);
+        auto put = [&](int n, int e) {   // column 8 n + 2 q + (e & 1), unit (lane >> 2) + 8 (e >> 1)
+          rw[(8 * n + 2 * q + (e & 1)) * LU + 8 * (e >> 1)] = make_float4(acc[0][n][e], acc[1][n][e], acc[2][n][e], NG == 4 ? acc[NG - 1][n][e] : 0.0f);
+        };
         if (__all_sync(0xffffffffu, small || !ok)) {
           // The cross terms of all k-steps first: an add into the accumulator truncates, so the fewer behind the large terms the
           // better.  Product by product over all accumulators, so that an mma does not follow the one that it adds to.
@@ -268,11 +274,22 @@ rnn_fwd_mma_kernel(const float* __restrict__ Wh, const float* __restrict__ gx, c
 #pragma unroll
           for (int n = 0; n < NT; ++n) {
             const int c0 = __shfl_sync(0xffffffffu, hsh[n], 8 * q), c1 = __shfl_sync(0xffffffffu, hsh[n], 8 * q + 4);
+            if (moderate && (c0 <= MQ_MODERATE) & (c1 <= MQ_MODERATE)) {   // (c >= 10, as |h| < 16) factors that no product of them leaves the range with
+              const float f0 = mq_pow2(-c0), f1 = mq_pow2(-c1);
 #pragma unroll
-            for (int g = 0; g < NG; ++g)
+              for (int e = 0; e < 4; ++e) {
 #pragma unroll
-              for (int e = 0; e < 4; ++e)
-                rw[(8 * n + 2 * q + (e & 1)) * LR + g * UG + (lane >> 2) + 8 * (e >> 1)] = mq_unscale(acc[g][n][e], -(ash[g][e >> 1] + ((e & 1) ? c1 : c0)));
+                for (int g = 0; g < NG; ++g) acc[g][n][e] *= mq_pow2(-ash[g][e >> 1]) * ((e & 1) ? f1 : f0);
+                put(n, e);
+              }
+            } else {
+#pragma unroll
+              for (int e = 0; e < 4; ++e) {
+#pragma unroll
+                for (int g = 0; g < NG; ++g) acc[g][n][e] = mq_unscale(acc[g][n][e], -(ash[g][e >> 1] + ((e & 1) ? c1 : c0)));
+                put(n, e);
+              }
+            }
           }
         } else {
           for (int k = 16 * ks0; k < 16 * (ks0 + KS) && k < H; ++k)
@@ -287,11 +304,9 @@ rnn_fwd_mma_kernel(const float* __restrict__ Wh, const float* __restrict__ gx, c
                   if (u0 + uu < H) acc[g][n][e] = fmaf(__ldg(Wh + (int64_t)k * (NG * H) + g * H + u0 + uu), h, acc[g][n][e]);
               }
 #pragma unroll
-          for (int g = 0; g < NG; ++g)
+          for (int n = 0; n < NT; ++n)
 #pragma unroll
-            for (int n = 0; n < NT; ++n)
-#pragma unroll
-              for (int e = 0; e < 4; ++e) rw[(8 * n + 2 * q + (e & 1)) * LR + g * UG + (lane >> 2) + 8 * (e >> 1)] = acc[g][n][e];
+            for (int e = 0; e < 4; ++e) put(n, e);
         }
         // One barrier a step: sums of the step after next come behind the next one's, where this step's have been read.
         if (!__syncthreads_and(ok ? 1 : 0)) {
@@ -300,19 +315,23 @@ rnn_fwd_mma_kernel(const float* __restrict__ Wh, const float* __restrict__ gx, c
         }
         if (mine) {
 #pragma unroll
-          for (int g = 0; g < NG; ++g) {
-            float s = 0.0f;
-#pragma unroll
-            for (int w = 0; w < 8; ++w) s += red[((size_t)(turn * 8 + w) * BG + gb) * LR + g * UG + gu];
-            pre[g] = s;
+          for (int w = 0; w < 8; ++w) {
+            const float4 s = red[((turn * 8 + w) * BG + gb) * LU + gu];
+            pre[0] += s.x;
+            pre[1] += s.y;
+            pre[2] += s.z;
+            if (NG == 4) pre[NG - 1] += s.w;
           }
         }
-      } else if (h0 != nullptr && mine) {
+      } else {
+        ahead(ch + nbg < nchunks ? t : t + 1, ch + nbg < nchunks ? ch + nbg : bgrp);
+        if (h0 != nullptr && mine) {
 #pragma unroll 4
-        for (int k = 0; k < H; ++k) {
-          const float h = __ldg(h0 + (int64_t)b * H + k);
+          for (int k = 0; k < H; ++k) {
+            const float h = __ldg(h0 + (int64_t)b * H + k);
 #pragma unroll
-          for (int g = 0; g < NG; ++g) pre[g] = fmaf(Ws[(g * UG + gu) * LD + k], h, pre[g]);
+            for (int g = 0; g < NG; ++g) pre[g] = fmaf(Ws[(g * UG + gu) * LD + k], h, pre[g]);
+          }
         }
       }
       if (mine) {
@@ -354,155 +373,170 @@ rnn_fwd_mma_kernel(const float* __restrict__ Wh, const float* __restrict__ gx, c
   }
 }
 
-// Arguments as for rnn_bwd_seq_kernel, and the exchange buffer (T runs); NP pieces of four k-steps per warp: NG * H, each gate's rows in
-// whole k-steps, up to 512 NP.
-template <int NG, int BG, int NP>
+// Backward.  The same CTAs; a CTA turns dh_t of its units into its own gate derivatives dg_t (NG * 16 rows x BG columns, one k-step per
+// gate) and multiplies them at once with its rows of Wh', for ALL units: a warp owns the 16-unit groups warp, warp + 8, ... and keeps
+// their fragments in registers.  What travels is the product: each group's CTA gets one partial sum per producer, polled in place
+// and added up in the producers' order.  (With dg itself exchanged a CTA read 4 H words per column and step, 128 KB at H 512, and cut
+// all of them into planes.)  H 512, B 64, T 256: 4.8 -> 3.35 us a step; what bounds it: 192 mma per SM partition (0.9 us), the sums'
+// way through L2 (32 KB out, in and reset per CTA: 1.3 us), gates and planes (0.5 us).
+//
+// Exchange: [slot][chunk][consumer group][producer group][BG / 8][lane][4], a lane's accumulators as it holds them.  Up to MQ_ALL_STEPS
+// bytes every step has a slot of its own.  Beyond, MQ_RING slots take the steps in turn, so that they stay in L2: a consumer puts the
+// empty pattern back over what it has read, and the slot is written again MQ_RING steps later.  That the pattern is there by then: every
+// thread fences in every MQ_FENCE-th step (steps count down), behind the barrier that follows the resets and ahead of the one before
+// the CTA sends.  A reset of step s lies before its CTA's fence of a step f, s >= f > s - MQ_FENCE, and so before what that CTA sends in f;
+// who has received that fences in step f - MQ_FENCE, before it writes to the same slot in step s + 1 - MQ_RING.
+// (Rings of 4, 8 and 16: 885, 847, 868 us at B 64; 1746, 1677, 1637 at B 128.  Resets behind the products or by bulk copies delay what is
+// sent: 910 - 1040 us.)
+constexpr int MQ_FENCE = 6, MQ_RING = 2 * MQ_FENCE;
+constexpr size_t MQ_ALL_STEPS = (size_t)32 << 20;   // bytes up to which every step gets a slot of its own, and nothing is reset
+constexpr int MQ_BAD = 1000;   // in the place of a column's shift: a value of it is not finite
+
+inline size_t mq_part_run(int64_t batch, int bg, int H) {
+  const size_t groups = (size_t)(H + MQ_UG - 1) / MQ_UG;
+  return (size_t)((batch + bg - 1) / bg) * groups * groups * (MQ_UG * bg);
+}
+inline size_t mq_bwd_smem(int chunks, int bg) { return (size_t)chunks * MQ_UG * bg * sizeof(float); }   // beside the kernel's own
+
+template <int NG, int BG, int MT>
 __global__ void __launch_bounds__(SQ_THREADS, 1)
 rnn_bwd_mma_kernel(const float* __restrict__ Wh, const float* __restrict__ keep, const float* __restrict__ cst,
                    const float* __restrict__ s0, const float* __restrict__ hout, const float* __restrict__ dout,
                    const float* __restrict__ dhT, const float* __restrict__ dcT, float* __restrict__ dg, float* __restrict__ dgx,
-                   float* ex, int H, int B, int T, int nbg, int32_t* dev_err) {
-  constexpr int UG = MQ_UG, NT = BG / 8, LD = 512 * NP + 4, LR = UG + 4;
-  constexpr int WSZ = UG * LD > 2 * 8 * BG * LR ? UG * LD : 2 * 8 * BG * LR;
-  extern __shared__ __align__(16) float sm[];
-  float* Ws = sm;                                 // [UG][LD], only before the loop
-  float* red = sm;                                // [2][8][BG][LR]
-  float* carry = sm + WSZ;                        // [chunks][UG * BG]: LSTM dc, GRU dh * z
+                   float* ex, int H, int B, int T, int nbg, int ring, int32_t* dev_err) {
+  constexpr int UG = MQ_UG, NT = BG / 8, BLOCK = UG * BG;
+  constexpr int PIECES = 32 * NT, GRP = SQ_THREADS / PIECES, PER = 8 * MT / GRP;   // GRP sets of threads share the producers
+  constexpr int LS = 20;                          // words of the sums per 16: the gates' threads read them without bank conflicts
+  __shared__ __align__(16) float sums[GRP][NT][8 * LS];
+  __shared__ __align__(16) uint4 frag[NG][NT][32];   // {hi, hi, lo, lo} of a lane's four k-values
+  __shared__ float dval[BG][NG * UG];             // the values themselves
+  __shared__ int csh[BG];                         // the columns' shifts
+  extern __shared__ float carry[];                // [chunks][UG * BG]: LSTM dc, GRU dh * z
   const int K = NG * H;
   const int ugroups = (H + UG - 1) / UG;
-  const int u0 = ((int)blockIdx.x % ugroups) * UG, bgrp = (int)blockIdx.x / ugroups;
+  const int ug = (int)blockIdx.x % ugroups, bgrp = (int)blockIdx.x / ugroups, u0 = ug * UG;
   const int nchunks = (B + BG - 1) / BG;
-  const int64_t ldrow = (int64_t)T * H, ldd = (int64_t)T * K, ldk = (int64_t)T * 4 * H;
+  const int64_t ldd = (int64_t)T * K;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, q = lane & 3;
   const int gu = threadIdx.x % UG, gb = threadIdx.x / UG;
-  const int Hp = (H + 15) & ~15;                  // a gate's rows in the exchange: whole k-steps
-  const int u = u0 + gu, ks0 = warp * 4 * NP, steps = NG * Hp / 16;
-  const size_t run = (size_t)nchunks * BG * steps * 16;
-  for (int e = threadIdx.x; e < UG * 512 * NP; e += SQ_THREADS) {
-    const int r = e % (512 * NP), uu = e / (512 * NP), g = r / Hp, w = r - g * Hp;
-    Ws[(size_t)uu * LD + r] = (g < NG && w < H && u0 + uu < H) ? __ldg(Wh + (int64_t)(u0 + uu) * K + g * H + w) : 0.0f;
-  }
+  const int u = u0 + gu;
+  const bool gates = threadIdx.x < BLOCK;
+  const size_t run = (size_t)nchunks * ugroups * ugroups * BLOCK;
   for (int ch = bgrp, i = 0; ch < nchunks; ch += nbg, ++i) {
     const int b = ch * BG + gb;
-    if (threadIdx.x < UG * BG) carry[i * UG * BG + threadIdx.x] = (NG == 4 && dcT && b < B && u < H) ? dcT[(int64_t)b * H + u] : 0.0f;
+    if (gates) carry[i * BLOCK + threadIdx.x] = (NG == 4 && dcT && b < B && u < H) ? dcT[(int64_t)b * H + u] : 0.0f;
+  }
+  // fragments of Wh': rows (lane >> 2) and 8 more of each group, this CTA's NG * 16 k-values
+  uint32_t ahi[MT][NG][4], alo[MT][NG][4];
+  int ash[MT][2];
+  bool finite = true, moderate = true;
+#pragma unroll
+  for (int m = 0; m < MT; ++m) {
+    float v[2][NG][4];
+    uint32_t mx[2] = {0u, 0u};
+#pragma unroll
+    for (int i = 0; i < 2; ++i) {
+      const int row = (warp + 8 * m) * UG + (lane >> 2) + 8 * i;
+#pragma unroll
+      for (int g = 0; g < NG; ++g)
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+          v[i][g][e] = (row < H && u0 + 4 * q + e < H) ? __ldg(Wh + (int64_t)row * K + g * H + u0 + 4 * q + e) : 0.0f;
+          mx[i] = max(mx[i], __float_as_uint(v[i][g][e]) & 0x7fffffffu);
+        }
+      mx[i] = mq_max_lanes(mx[i]);
+      ash[m][i] = mq_shift(mx[i]);
+      moderate = moderate && abs(ash[m][i]) <= MQ_MODERATE;
+      const float sc = mq_pow2(ash[m][i]);
+#pragma unroll
+      for (int g = 0; g < NG; ++g) {
+        mq_split(v[i][g][0] * sc, v[i][g][1] * sc, ahi[m][g][i], alo[m][g][i]);
+        mq_split(v[i][g][2] * sc, v[i][g][3] * sc, ahi[m][g][2 + i], alo[m][g][2 + i]);
+      }
+    }
+    finite = finite && mx[0] < MQ_INF && mx[1] < MQ_INF;
   }
   __syncthreads();
-  uint32_t ahi[NP][4][4], alo[NP][4][4];
-  int ash[NP][2];
-  bool finite[NP];
+  // What a step reads of its own units, asked for a step ahead and behind the poll (as in the forward kernel).  No branch around the loads:
+  // where paths meet, the compiler waits for what is on its way.
+  float nk[4], nct = 0.0f, nsp = 0.0f, ndh = 0.0f;
+  auto ahead = [&](int t, int ch) {
+    const int b = ch * BG + gb;
+    const bool there = gates && b < B && u < H && t >= 0;
+    const int64_t row = there ? (int64_t)b * T + t : 0;
+    const float *kr = keep + row * 4 * H + u, *prev = NG == 4 ? cst : hout;   // c_{t-1} or h_{t-1}
 #pragma unroll
-  for (int p = 0; p < NP; ++p)
-    finite[p] = __all_sync(0xffffffffu, mq_load_a<4>(Ws, LD, lane >> 2, 16 * (ks0 + 4 * p) + 4 * q, ahi[p], alo[p], ash[p]));
-  __syncthreads();
-  int turn = 0;
+    for (int i = 0; i < 4; ++i) nk[i] = there ? __ldg(kr + i * H) : 0.0f;
+    if (NG == 4) nct = there ? __ldg(cst + row * H + u) : 0.0f;
+    nsp = there && t > 0 ? __ldg(prev + (row - 1) * H + u) : 0.0f;
+    ndh = there ? __ldg(dout + row * H + u) : 0.0f;
+  };
+  ahead(T - 1, bgrp);
+  const int grp = threadIdx.x / PIECES, piece = threadIdx.x % PIECES;
   for (int t = T - 1; t >= 0; --t) {
-    for (int ch = bgrp, ci = 0; ch < nchunks; ch += nbg, ++ci, turn ^= 1) {
+    for (int ch = bgrp, ci = 0; ch < nchunks; ch += nbg, ++ci) {
       const int b0 = ch * BG, nb = B - b0 < BG ? B - b0 : BG;
       const int b = b0 + gb;
-      const bool mine = threadIdx.x < UG * BG && gb < nb && u < H;
-      float k0 = 0.f, k1 = 0.f, k2 = 0.f, k3 = 0.f, ct = 0.f, sp = 0.f, dh = 0.f;
-      if (mine) {
-        const float* kr = keep + (int64_t)t * 4 * H + (int64_t)b * ldk;
-        k0 = __ldg(kr + u); k1 = __ldg(kr + H + u); k2 = __ldg(kr + 2 * H + u); k3 = __ldg(kr + 3 * H + u);
-        const float* prev = NG == 4 ? cst : hout;   // c_{t-1} or h_{t-1}
-        if (NG == 4) ct = __ldg(cst + (int64_t)t * H + (int64_t)b * ldrow + u);
-        sp = t > 0 ? __ldg(prev + (int64_t)(t - 1) * H + (int64_t)b * ldrow + u) : s0 ? __ldg(s0 + (int64_t)b * H + u) : 0.0f;
-        dh = __ldg(dout + (int64_t)t * H + (int64_t)b * ldrow + u);
-        if (t == T - 1 && dhT) dh += __ldg(dhT + (int64_t)b * H + u);
-      }
+      const bool mine = gates && gb < nb && u < H;
+      const float k0 = nk[0], k1 = nk[1], k2 = nk[2], k3 = nk[3], ct = nct;
+      float sp = nsp, dh = ndh;
+      if (t == 0 && s0 && mine) sp = __ldg(s0 + (int64_t)b * H + u);
+      if (t == T - 1 && dhT && mine) dh += __ldg(dhT + (int64_t)b * H + u);
       if (t < T - 1) {
-        const float* src = ex + (size_t)(t + 1) * run + (size_t)ch * (BG * 16) * steps;
-        float sum[NT][4];
+        float* src = ex + (size_t)((t + 1) % ring) * run + ((size_t)ch * ugroups + ug) * ugroups * BLOCK + 4 * piece;
+        uint4 v[PER];
+        bool missing = false;
 #pragma unroll
-        for (int n = 0; n < NT; ++n)
-#pragma unroll
-          for (int e = 0; e < 4; ++e) sum[n][e] = 0.0f;
-        bool ok = true;
-        MqPieces<NT, 4> pc[2];
-        pc[0].template load<false>(src, nb, ks0, steps);
-#pragma unroll
-        for (int p = 0; p < NP; ++p) {
-          MqPieces<NT, 4>& now = pc[p & 1];
-          ok = now.wait(src, nb, ks0 + 4 * p, steps, dev_err) && ok;
-          if (p + 1 < NP) pc[(p + 1) & 1].template load<false>(src, nb, ks0 + 4 * (p + 1), steps);
-          int sh[NT];
-          bool fine = finite[p];
-#pragma unroll
-          for (int n = 0; n < NT; ++n) {
-            uint32_t m = 0u;
-#pragma unroll
-            for (int s = 0; s < 4; ++s) m = mq_max4(m, now.v[n][s]);
-            m = mq_max_lanes(m);
-            sh[n] = mq_shift(m);
-            fine = fine && m < MQ_INF;
-          }
-          if (__all_sync(0xffffffffu, fine || !ok)) {
-            float hh[NT][4], cr[NT][4];   // hi hi, and the cross terms
-#pragma unroll
-            for (int n = 0; n < NT; ++n)
-#pragma unroll
-              for (int e = 0; e < 4; ++e) hh[n][e] = cr[n][e] = 0.0f;
-#pragma unroll
-            for (int s = 0; s < 4; ++s) {
-              uint32_t hi[NT][2], lo[NT][2];
-#pragma unroll
-              for (int n = 0; n < NT; ++n) {
-                const uint4 x = now.v[n][s];
-                const float sc = mq_pow2(sh[n]);
-                mq_split(__uint_as_float(x.x) * sc, __uint_as_float(x.y) * sc, hi[n][0], lo[n][0]);
-                mq_split(__uint_as_float(x.z) * sc, __uint_as_float(x.w) * sc, hi[n][1], lo[n][1]);
-              }
-              // (in an order that keeps an mma away from the one that it adds to)
-#pragma unroll
-              for (int n = 0; n < NT; ++n) mq_mma(cr[n], alo[p][s], hi[n][0], hi[n][1]);
-#pragma unroll
-              for (int n = 0; n < NT; ++n) mq_mma(hh[n], ahi[p][s], hi[n][0], hi[n][1]);
-#pragma unroll
-              for (int n = 0; n < NT; ++n) mq_mma(cr[n], ahi[p][s], lo[n][0], lo[n][1]);
-            }
-            // columns 2 q and 2 q + 1 were scaled by the lanes that hold them
-#pragma unroll
-            for (int n = 0; n < NT; ++n) {
-              const int c0 = __shfl_sync(0xffffffffu, sh[n], 8 * q), c1 = __shfl_sync(0xffffffffu, sh[n], 8 * q + 4);
-#pragma unroll
-              for (int e = 0; e < 4; ++e) sum[n][e] += mq_unscale(hh[n][e] + cr[n][e], -(ash[p][e >> 1] + ((e & 1) ? c1 : c0)));
-            }
-          } else {
-            for (int k = 16 * (ks0 + 4 * p); k < 16 * (ks0 + 4 * p + 4) && k < 16 * steps; ++k) {
-              const int g = k / Hp, w = k - g * Hp;
-              if (w >= H) continue;
-#pragma unroll
-              for (int n = 0; n < NT; ++n)
-#pragma unroll
-                for (int e = 0; e < 4; ++e) {
-                  const int c = 8 * n + 2 * q + (e & 1), uu = (lane >> 2) + 8 * (e >> 1);
-                  if (c < nb && u0 + uu < H) sum[n][e] = fmaf(__ldg(Wh + (int64_t)(u0 + uu) * K + g * H + w), mq_at<NT>(src, k, c), sum[n][e]);
-                }
-            }
-          }
+        for (int i = 0; i < PER; ++i) {
+          const int p = grp + GRP * i;
+          v[i] = p < ugroups ? sq_peek4(src + (size_t)p * BLOCK) : make_uint4(0u, 0u, 0u, 0u);
         }
-        float* rw = red + (size_t)(turn * 8 + warp) * BG * LR;
 #pragma unroll
-        for (int n = 0; n < NT; ++n)
+        for (int i = 0; i < PER; ++i) missing |= MqPieces<1, 1>::empty(v[i]);
+        bool ok = true;
+        uint32_t spins = 0;
+        while (missing) {
+          if (++spins > SQ_POLL_LIMIT || ((spins & 255u) == 255u && *(const volatile int32_t*)dev_err != 0)) {
+            ok = false;
+            break;
+          }
+          missing = false;
 #pragma unroll
-          for (int e = 0; e < 4; ++e) rw[(8 * n + 2 * q + (e & 1)) * LR + (lane >> 2) + 8 * (e >> 1)] = sum[n][e];
+          for (int i = 0; i < PER; ++i)
+            if (MqPieces<1, 1>::empty(v[i])) v[i] = sq_peek4(src + (size_t)(grp + GRP * i) * BLOCK);
+#pragma unroll
+          for (int i = 0; i < PER; ++i) missing |= MqPieces<1, 1>::empty(v[i]);
+        }
+        float4 s = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+#pragma unroll
+        for (int i = 0; i < PER; ++i) {
+          s.x += __uint_as_float(v[i].x);
+          s.y += __uint_as_float(v[i].y);
+          s.z += __uint_as_float(v[i].z);
+          s.w += __uint_as_float(v[i].w);
+          if (ring < T && grp + GRP * i < ugroups) mq_put4(src + (size_t)(grp + GRP * i) * BLOCK, SQ_EMPTY, SQ_EMPTY, SQ_EMPTY, SQ_EMPTY);
+        }
+        *(float4*)&sums[grp][piece >> 5][((piece & 31) >> 2) * LS + 4 * (piece & 3)] = s;
+        ahead(ch + nbg < nchunks ? t : t - 1, ch + nbg < nchunks ? ch + nbg : bgrp);
         if (!__syncthreads_and(ok ? 1 : 0)) {
           if (threadIdx.x == 0) atomicCAS(dev_err, 0, 3003);
           return;
         }
+        if (ring < T && t % MQ_FENCE == 0) __threadfence();
         if (mine) {
-          float s = 0.0f;
+          float r = 0.0f;
 #pragma unroll
-          for (int w = 0; w < 8; ++w) s += red[((size_t)(turn * 8 + w) * BG + gb) * LR + gu];
-          dh += s;
+          for (int w = 0; w < GRP; ++w) r += sums[w][gb >> 3][(gu & 7) * LS + 4 * ((gb & 7) >> 1) + (gb & 1) + 2 * (gu >> 3)];
+          dh += r;
         }
+      } else {
+        ahead(ch + nbg < nchunks ? t : t - 1, ch + nbg < nchunks ? ch + nbg : bgrp);
       }
       float d[NG];
 #pragma unroll
       for (int g = 0; g < NG; ++g) d[g] = 0.0f;
       if (mine) {
-        float* cy = carry + ci * UG * BG + threadIdx.x;
-        float* row = dg + (int64_t)t * K + (int64_t)b * ldd;
+        float* cy = carry + ci * BLOCK + threadIdx.x;
         if (NG == 4) {
           const float tc = tanhf(ct);
           const float d_o = dh * tc;
@@ -523,13 +557,117 @@ rnn_bwd_mma_kernel(const float* __restrict__ Wh, const float* __restrict__ keep,
           x[u] = da1; x[H + u] = da2; x[2 * H + u] = da3;
           *cy = dh * z;
         }
+      }
+      if (t > 0 && gates) {
+        // this column's planes (zeros for units and columns that do not exist), scaled by its largest value
+        uint32_t m = 0u;
+#pragma unroll
+        for (int g = 0; g < NG; ++g) m = max(m, __float_as_uint(d[g]) & 0x7fffffffu);
+#pragma unroll
+        for (int o = 1; o < UG; o *= 2) m = max(m, __shfl_xor_sync(0xffffffffu, m, o));
+        const int sh = mq_shift(m);
+        const float sc = mq_pow2(sh);
+        if (gu == 0) csh[gb] = m < MQ_INF ? sh : MQ_BAD;
+#pragma unroll
+        for (int g = 0; g < NG; ++g) {
+          const float x = d[g] * sc;
+          const __half hi = __float2half_rn(x), lo = __float2half_rn(x - __half2float(hi));
+          __half* f = (__half*)&frag[g][gb >> 3][4 * (gb & 7) + (gu >> 2)] + (gu & 3);
+          f[0] = hi;
+          f[4] = lo;
+          dval[gb][g * UG + gu] = d[g];
+        }
+      }
+      if (t > 0) __syncthreads();
+      if (mine) {
+        float* row = dg + (int64_t)t * K + (int64_t)b * ldd;
 #pragma unroll
         for (int g = 0; g < NG; ++g) row[g * H + u] = d[g];
       }
-      if (t > 0 && threadIdx.x < UG * BG && gb < nb) {   // (zeros for units that do not exist)
+      if (t == 0) continue;
+      uint4 bf[NG][NT];
+      int sh[NT][2];
+      bool cols = true;
 #pragma unroll
-        for (int g = 0; g < NG; ++g)
-          mq_publish(ex + (size_t)t * run + (size_t)ch * (BG * 16) * steps, BG, (g * Hp + u0) / 16, gu, gb, mq_word(d[g]));
+      for (int n = 0; n < NT; ++n) {
+#pragma unroll
+        for (int g = 0; g < NG; ++g) bf[g][n] = frag[g][n][lane];
+#pragma unroll
+        for (int i = 0; i < 2; ++i) {
+          sh[n][i] = csh[8 * n + 2 * q + i];
+          cols = cols && sh[n][i] != MQ_BAD;
+        }
+      }
+      float* dst = ex + (size_t)(t % ring) * run + ((size_t)ch * ugroups * ugroups + ug) * BLOCK + 4 * lane;
+      auto send = [&](int m, int n, const float (&v)[4]) {
+        if (warp + 8 * m < ugroups) mq_put4(dst + (size_t)(warp + 8 * m) * ugroups * BLOCK + 128 * n, mq_word(v[0]), mq_word(v[1]), mq_word(v[2]), mq_word(v[3]));
+      };
+      // (groups that do not exist have rows of zeros: no branch between the products, so that one group's sums are scaled and sent under
+      // the next one's products)
+      auto products = [&](auto is_plain) {
+        float f[NT][2];
+#pragma unroll
+        for (int n = 0; n < NT; ++n)
+#pragma unroll
+          for (int i = 0; i < 2; ++i) f[n][i] = mq_pow2(-sh[n][i]);
+#pragma unroll
+        for (int m = 0; m < MT; ++m) {
+          constexpr int CR = MT < 4 ? 2 : 1;   // (four groups leave no registers for more)
+          float hh[NT][4], cr[CR][NT][4];      // hi hi, and the cross terms: sums of their own, as an mma waits for the one that it adds to
+#pragma unroll
+          for (int n = 0; n < NT; ++n)
+#pragma unroll
+            for (int e = 0; e < 4; ++e) hh[n][e] = cr[0][n][e] = cr[CR - 1][n][e] = 0.0f;
+#pragma unroll
+          for (int g = 0; g < NG; ++g) {
+#pragma unroll
+            for (int n = 0; n < NT; ++n) mq_mma(cr[0][n], alo[m][g], bf[g][n].x, bf[g][n].y);
+#pragma unroll
+            for (int n = 0; n < NT; ++n) mq_mma(hh[n], ahi[m][g], bf[g][n].x, bf[g][n].y);
+#pragma unroll
+            for (int n = 0; n < NT; ++n) mq_mma(cr[CR - 1][n], ahi[m][g], bf[g][n].z, bf[g][n].w);
+          }
+          const float a0 = mq_pow2(-ash[m][0]), a1 = mq_pow2(-ash[m][1]);
+#pragma unroll
+          for (int n = 0; n < NT; ++n) {
+            float v[4];
+#pragma unroll
+            for (int e = 0; e < 4; ++e) {
+              const float x = CR == 2 ? hh[n][e] + (cr[0][n][e] + cr[CR - 1][n][e]) : hh[n][e] + cr[0][n][e];
+              v[e] = decltype(is_plain)::value ? x * ((e >> 1 ? a1 : a0) * f[n][e & 1]) : mq_unscale(x, -(ash[m][e >> 1] + sh[n][e & 1]));
+            }
+            send(m, n, v);
+          }
+        }
+      };
+      bool plain = moderate;
+#pragma unroll
+      for (int n = 0; n < NT; ++n) plain = plain && abs(sh[n][0]) <= MQ_MODERATE && abs(sh[n][1]) <= MQ_MODERATE;
+      plain = __all_sync(0xffffffffu, plain);
+      if (__all_sync(0xffffffffu, cols && finite)) {
+        if (plain) products(std::true_type());
+        else products(std::false_type());
+      } else {
+        for (int m = 0; m < MT; ++m) {
+          float v[NT][4];
+#pragma unroll
+          for (int n = 0; n < NT; ++n)
+#pragma unroll
+            for (int e = 0; e < 4; ++e) v[n][e] = 0.0f;
+          for (int k = 0; k < NG * UG; ++k) {
+            const int g = k / UG, w = u0 + k % UG;
+            if (w >= H) continue;
+#pragma unroll
+            for (int n = 0; n < NT; ++n)
+#pragma unroll
+              for (int e = 0; e < 4; ++e) {
+                const int c = 8 * n + 2 * q + (e & 1), row = (warp + 8 * m) * UG + (lane >> 2) + 8 * (e >> 1);
+                if (c < nb && row < H) v[n][e] = fmaf(__ldg(Wh + (int64_t)row * K + g * H + w), dval[c][k], v[n][e]);
+              }
+          }
+#pragma unroll
+          for (int n = 0; n < NT; ++n) send(m, n, v[n]);
+        }
       }
     }
   }

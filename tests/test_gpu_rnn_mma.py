@@ -85,6 +85,13 @@ def test_recurrences(cell, states, H, B, T):
         close(dx[i], rx.grad[i], 2e-5, "dx")
 
 
+@pytest.mark.parametrize("cell", ["lstm", "gru"])
+@pytest.mark.parametrize("H,B,T", [(512, 40, 37), (400, 130, 27), (500, 9, 130), (512, 150, 13)])
+def test_backward_slots_that_are_reset(cell, H, B, T):
+    """Exchanges of more than 32 MB: twelve slots take the steps in turn (the last shape: one slot is used twice)."""
+    test_recurrences(cell, False, H, B, T)
+
+
 def test_a_sequence_inside_a_graph_beside_another_stream():
     """The exchange buffer belongs to the call: replays and eager calls on another stream give what each gives alone."""
     import fluxb200 as F
