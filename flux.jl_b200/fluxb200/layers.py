@@ -9,6 +9,7 @@ LSTMCell :383-419, GRUCell :586-628, LSTM :491-524, GRU :685-718), attention.jl 
 from __future__ import annotations
 
 import math
+from array import array
 
 import numpy as np
 import torch
@@ -101,6 +102,10 @@ class Chain(Layer):
 
     def __call__(self, x):
         layers = self.layers
+        if not Tape.active and len(layers) > 1 and type(x) is B200Array and x.ndim <= 2 and Tape.grad_sink is None:
+            y = _dense_chain(layers, x)
+            if y is not None:
+                return y
         for i, l in enumerate(layers):
             # the normalised rows that only a bf16 Dense reads are stored as it reads them
             if type(l) is LayerNorm and i + 1 < len(layers) and type(layers[i + 1]) is Dense and is_bf16(layers[i + 1].weight):
@@ -114,6 +119,33 @@ class Chain(Layer):
 
     def __repr__(self):
         return "Chain(" + ", ".join(map(repr, self.layers)) + ")"
+
+
+def _dense_chain(layers, x):
+    """A Chain of Float32 Dense layers applied to a few columns, as one launch; None where that is not what the call is, or not the
+    faster way (the layers are then called one by one, and say what is wrong with a bad call)."""
+    size = x.size
+    n, d = size[1] if len(size) == 2 else 1, size[0]
+    if n > _CHAIN_COLUMNS or x.t.dtype != torch.float32:
+        return None
+    table = []
+    for l in layers:
+        if type(l) is not Dense or l.precision != "default":
+            return None
+        W, b = l.weight, l.bias
+        if W.size[1] != d or W.t.dtype != torch.float32 or (b is not False and b.t.dtype != torch.float32):
+            return None
+        d = W.size[0]
+        table += (W.t.data_ptr(), 0 if b is False else b.t.data_ptr(), W.size[1], d, lib.ACT[l.σ])
+    ctx = context()
+    y = empty((d,) + size[1:])
+    rows = array("q", table)
+    if lib.supported("fb_dense_chain_fwd", ctx.handle, ctx.stream, rows.buffer_info()[0], len(layers), x.t.data_ptr(), y.t.data_ptr(), n):
+        return y
+    return None
+
+
+_CHAIN_COLUMNS = 28   # seven clusters of four columns
 
 
 def _round_bf16(a: B200Array) -> B200Array:

@@ -59,6 +59,7 @@ PROTOTYPES = {
     "fb_selftest_bounded_wait": (_i32, [_p, _p, _i32]),
     "fb_gemm_f32": (_i32, [_p, _p, _i32, _i32, _i64, _i64, _i64, _p, _i64, _p, _i64, _p, _i64, _i32, _i32]),
     "fb_dense_fwd": (_i32, [_p, _p, _i32, _i32, _p, _p, _p, _p, _p, _i64, _i64, _i64]),
+    "fb_dense_chain_fwd": (_i32, [_p, _p, _p, _i32, _p, _p, _i64]),
     "fb_dense_bwd": (_i32, [_p, _p, _i32, _i32, _p, _p, _p, _p, _p, _p, _p, _p, _p, _i64, _i64, _i64]),
     "fb_gemm_bf16": (_i32, [_p, _p, _i32, _i32, _i64, _i64, _i64, _p, _i64, _p, _i64, _p, _i64, _i32, _i32]),
     "fb_axpy_bf16": (_i32, [_p, _p, _f, _p, _p, _i64]),
@@ -183,6 +184,19 @@ def check(status: int) -> None:
 
 
 PROFILE = None   # optional {"names": set, "events": list}: CUDA events recorded around the named entry points
+
+
+def supported(name: str, *args) -> bool:
+    """Calls an entry point that may answer FB_ERR_UNSUPPORTED without a message: whether it did what was asked."""
+    f = _fast.get(name)
+    status = f(*args) if f is not None else None
+    if status is None:
+        status = getattr(_lib, name)(*args)
+    if status == 0:
+        return True
+    if status != ERR_UNSUPPORTED:
+        check(status)
+    return False
 
 
 def call(name: str, *args):

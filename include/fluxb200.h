@@ -137,6 +137,12 @@ int32_t fb_dense_fwd(fb_ctx* ctx, void* stream, int32_t act, int32_t precision, 
                      const float* b, const float* x, float* y, float* z, int64_t out_dim,
                      int64_t in_dim, int64_t n);
 
+/* Consecutive Dense layers for a few columns in one launch: y[out_last,n] = layer_last(...layer_1(x[in_1,n])).  `table` (host memory,
+ * read during the call) has five int64 per layer: weight pointer, bias pointer or 0, in, out, activation.  FB_ERR_UNSUPPORTED, without
+ * a message, for calls that are better served layer by layer (the caller then does that).  Inference only: nothing between
+ * the layers is stored.  Replaces the loop of (c::Chain)(x) (src/layers/basic.jl:49-81) over Dense layers. */
+int32_t fb_dense_chain_fwd(fb_ctx* ctx, void* stream, const int64_t* table, int32_t layers, const float* x, float* y, int64_t n);
+
 /* Reverse of fb_dense_fwd (the Zygote pullback of basic.jl:199; external rrules of `*` and
  * NNlib.bias_act!): delta = dy .* act'(.), dW = delta * x', db = sum_n delta, dx = W' * delta.
  * `y` is the forward output (used by relu/tanh/sigmoid), `z` the saved pre-activation (gelu; may be
