@@ -486,18 +486,19 @@ bn_apply_flat_kernel(const float* __restrict__ x, const float* __restrict__ gamm
 // ----------------------------------------------------------------------------------- backward ---
 // dgamma, dbeta and (coef != NULL) the means of dz and dz * xhat, with dz = dy_scale * dy * act'(gamma * xhat + beta); one cluster
 // per channel
-template <int W, int ACT>
+template <int W, int ACT, bool OWN>
 __global__ void __launch_bounds__(BN_THREADS, 5)
 bn_bwd_sums_kernel(const float* __restrict__ x, const float* __restrict__ dy, float dy_scale, const float* __restrict__ gamma,
                    const float* __restrict__ beta, const float* __restrict__ mean, const float* __restrict__ rstd, const Dims g,
                    float* __restrict__ coef, float* __restrict__ dgamma, float* __restrict__ dbeta, int act, int32_t* __restrict__ dev_err) {
-  constexpr int U = 2;
+  constexpr int U = OWN ? 4 : 2;
   __shared__ Exchange ex;
   exchange_init(ex, g.split);
   const int64_t ch = blockIdx.x / (unsigned)g.split;
   const int p = (int)(blockIdx.x % (unsigned)g.split);
   const float mu = __ldg(mean + ch), rs = __ldg(rstd + ch);
   const float ga = gamma ? __ldg(gamma + ch) : 1.0f, be = beta ? __ldg(beta + ch) : 0.0f;
+  const float sc = rs * ga;   // (as the forward pass scales)
   float a1 = 0.0f, a2 = 0.0f;
   const Walk wk = make_walk<W>(g, p);
   each_piece<U>(wk, ch * g.s, [&](int, int64_t off, int m) {
@@ -506,7 +507,7 @@ bn_bwd_sums_kernel(const float* __restrict__ x, const float* __restrict__ dy, fl
     for (int u = 0; u < U; ++u)
       if (u < m) {
         ld_piece<W>(x + off + u * wk.step, v[u]);
-        ld_piece<W>(dy + off + u * wk.step, d[u]);
+        if (!OWN) ld_piece<W>(dy + off + u * wk.step, d[u]);
       }
 #pragma unroll
     for (int u = 0; u < U; ++u) {
@@ -514,7 +515,7 @@ bn_bwd_sums_kernel(const float* __restrict__ x, const float* __restrict__ dy, fl
 #pragma unroll
       for (int e = 0; e < W; ++e) {
         const float h = (v[u][e] - mu) * rs;
-        float dz = d[u][e] * dy_scale;
+        float dz = (OWN ? fb_act_apply_k<ACT>(act, fmaf(v[u][e] - mu, sc, be)) : d[u][e]) * dy_scale;
         if (ACT != 0) dz = fb_act_bwd_k<ACT>(act, fmaf(h, ga, be), dz);
         a1 += dz;
         a2 = fmaf(dz, h, a2);
@@ -688,12 +689,14 @@ int32_t bn_fwd_batch(fb_ctx* ctx, cudaStream_t stream, const float* x, const flo
   return st != FB_OK ? st : bn_apply<false>(ctx, stream, vec, x, gamma, beta, save_mean, save_rstd, eps, y, s, c, n, act);
 }
 
+// dy == NULL: the cotangent is dy_scale times the layer's output, which the kernel makes from x instead of reading it
 int32_t bn_bwd_sums(fb_ctx* ctx, cudaStream_t stream, bool vec, const float* x, const float* dy, float dy_scale, const float* gamma,
                     const float* beta, const float* mean, const float* rstd, float* coef, float* dgamma, float* dbeta, int64_t s,
                     int64_t c, int64_t n, int act) {
   const Dims g = bn_dims(ctx, s, c, n, vec ? 4 : 1, BN_THREADS, 12);
   return bn_kind(vec, act, [&](auto w, auto k) {
-    return bn_launch(bn_bwd_sums_kernel<w.value, k.value>, stream, g, c, BN_THREADS, 0, x, dy, dy_scale, gamma, beta, mean, rstd, g, coef, dgamma, dbeta, act, ctx->dev_error);
+    return bn_launch(dy != nullptr ? bn_bwd_sums_kernel<w.value, k.value, false> : bn_bwd_sums_kernel<w.value, k.value, true>, stream, g, c, BN_THREADS, 0, x, dy,
+                     dy_scale, gamma, beta, mean, rstd, g, coef, dgamma, dbeta, act, ctx->dev_error);
   });
 }
 
@@ -780,4 +783,17 @@ FB_API int32_t fb_batchnorm_bwd_params(fb_ctx* ctx, void* stream_, const float* 
   FB_REQUIRE(x && save_mean && save_rstd && dy && dgamma && dbeta, FB_ERR_INVALID_ARG, "fb_batchnorm_bwd_params: NULL pointer");
   const bool vec = (s % 4 == 0) && fb_aligned16(x) && fb_aligned16(dy);
   return bn_bwd_sums(ctx, (cudaStream_t)stream_, vec, x, dy, dy_scale, gamma, beta, save_mean, save_rstd, nullptr, dgamma, dbeta, s, c, n, act);
+}
+
+FB_API int32_t fb_batchnorm_bwd_params_own(fb_ctx* ctx, void* stream_, const float* x, const float* gamma, const float* beta,
+                                           const float* save_mean, const float* save_rstd, float y_scale, float* dgamma, float* dbeta,
+                                           int64_t s, int64_t c, int64_t n, int32_t act) {
+  FB_CHECK_CTX(ctx);
+  int32_t st = bn_check("fb_batchnorm_bwd_params_own", s, c, n, act);
+  if (st != FB_OK) return st;
+  FB_REQUIRE((gamma == nullptr) == (beta == nullptr), FB_ERR_INVALID_ARG, "fb_batchnorm_bwd_params_own: gamma and beta must both be given or both NULL");
+  FB_REQUIRE(n >= 1, FB_ERR_SHAPE, "fb_batchnorm_bwd_params_own: empty batch");
+  FB_REQUIRE(x && save_mean && save_rstd && dgamma && dbeta, FB_ERR_INVALID_ARG, "fb_batchnorm_bwd_params_own: NULL pointer");
+  const bool vec = (s % 4 == 0) && fb_aligned16(x);
+  return bn_bwd_sums(ctx, (cudaStream_t)stream_, vec, x, nullptr, y_scale, gamma, beta, save_mean, save_rstd, nullptr, dgamma, dbeta, s, c, n, act);
 }

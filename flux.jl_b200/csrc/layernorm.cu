@@ -373,7 +373,7 @@ ln_bwd_rows_kernel(const float* __restrict__ x, const float* __restrict__ gamma,
 // Only dgamma / dbeta: lx lanes side by side cover lx * W columns, 256 / lx rows at a time; grid (column blocks, row groups).
 // dy counts dy_scale times.  Bound: one read of x and dy (1024 x 16384: 77 us with a dx, 38; 1001 x 3000: 60 and 17).
 // CL: the row groups of a column block are a cluster, which adds its sums up itself (part_dg and part_db are dgamma and dbeta).
-template <bool VEC, int ACT, bool CL>
+template <bool VEC, int ACT, bool CL, bool OWN>
 __global__ void __launch_bounds__(LN_THREADS)
 ln_bwd_params_kernel(const float* __restrict__ x, const float* __restrict__ gamma, const float* __restrict__ beta,
                      const float* __restrict__ mean, const float* __restrict__ rstd, const float* __restrict__ dy, float dy_scale,
@@ -386,7 +386,7 @@ ln_bwd_params_kernel(const float* __restrict__ x, const float* __restrict__ gamm
 #pragma unroll
   for (int e = 0; e < W; ++e) { ag[e] = ab[e] = be[e] = 0.0f; ga[e] = 1.0f; }
   if (c < d) {
-    if (ACT != 0 && gamma != nullptr) {
+    if ((OWN || ACT != 0) && gamma != nullptr) {
       ld_piece<W>(gamma + c, ga);
       ld_piece<W>(beta + c, be);
     }
@@ -400,7 +400,7 @@ ln_bwd_params_kernel(const float* __restrict__ x, const float* __restrict__ gamm
         mu[u] = __ldg(mean + rr);
         rs[u] = __ldg(rstd + rr);
         ld_piece<W>(x + rr * d + c, xv[u]);
-        ld_piece<W>(dy + rr * d + c, dv[u]);
+        if (!OWN) ld_piece<W>(dy + rr * d + c, dv[u]);
       }
 #pragma unroll
       for (int u = 0; u < U; ++u)
@@ -408,8 +408,9 @@ ln_bwd_params_kernel(const float* __restrict__ x, const float* __restrict__ gamm
         for (int e = 0; e < W; ++e) {
           if (row + u * step >= n) continue;
           const float h = (xv[u][e] - mu[u]) * rs[u];
-          float dz = dv[u][e] * dy_scale;
-          if (ACT != 0) dz = fb_act_bwd_k<ACT>(act, fmaf(h, ga[e], be[e]), dz);
+          const float z = fmaf(h, ga[e], be[e]);
+          float dz = (OWN ? fb_act_apply_k<ACT>(act, z) : dv[u][e]) * dy_scale;
+          if (ACT != 0) dz = fb_act_bwd_k<ACT>(act, z, dz);
           ag[e] = fmaf(dz, h, ag[e]);
           ab[e] += dz;
         }
@@ -1129,22 +1130,21 @@ FB_API int32_t fb_layernorm_bwd(fb_ctx* ctx, void* stream_, const float* x, cons
                                d, n, act, ctx->dev_error);
 }
 
-FB_API int32_t fb_layernorm_bwd_params(fb_ctx* ctx, void* stream_, const float* x, const float* gamma, const float* beta,
-                                       const float* mean, const float* rstd, const float* dy, float dy_scale, float* dgamma,
-                                       float* dbeta, int64_t d, int64_t n, int32_t act) {
-  FB_CHECK_CTX(ctx);
-  cudaStream_t stream = (cudaStream_t)stream_;
-  FB_REQUIRE(d >= 1 && n >= 0, FB_ERR_SHAPE, "fb_layernorm_bwd_params: bad shape d=%lld n=%lld", (long long)d, (long long)n);
-  FB_REQUIRE(fb_act_valid(act), FB_ERR_INVALID_ARG, "fb_layernorm_bwd_params: unknown activation %d", act);
-  FB_REQUIRE((gamma == nullptr) == (beta == nullptr), FB_ERR_INVALID_ARG, "fb_layernorm_bwd_params: gamma and beta must both be given or both NULL");
-  FB_REQUIRE(dgamma && dbeta, FB_ERR_INVALID_ARG, "fb_layernorm_bwd_params: NULL pointer");
+// dy == NULL: the cotangent is dy_scale times the layer's output, which the kernel makes from x instead of reading it
+static int32_t ln_bwd_params(const char* fn, fb_ctx* ctx, cudaStream_t stream, const float* x, const float* gamma, const float* beta,
+                             const float* mean, const float* rstd, const float* dy, float dy_scale, float* dgamma,
+                             float* dbeta, int64_t d, int64_t n, int32_t act) {
+  FB_REQUIRE(d >= 1 && n >= 0, FB_ERR_SHAPE, "%s: bad shape d=%lld n=%lld", fn, (long long)d, (long long)n);
+  FB_REQUIRE(fb_act_valid(act), FB_ERR_INVALID_ARG, "%s: unknown activation %d", fn, act);
+  FB_REQUIRE((gamma == nullptr) == (beta == nullptr), FB_ERR_INVALID_ARG, "%s: gamma and beta must both be given or both NULL", fn);
+  FB_REQUIRE(dgamma && dbeta, FB_ERR_INVALID_ARG, "%s: NULL pointer", fn);
   if (n == 0) {
     FB_CUDA(cudaMemsetAsync(dgamma, 0, d * sizeof(float), stream));
     FB_CUDA(cudaMemsetAsync(dbeta, 0, d * sizeof(float), stream));
     return FB_OK;
   }
-  FB_REQUIRE(x && mean && rstd && dy, FB_ERR_INVALID_ARG, "fb_layernorm_bwd_params: NULL pointer");
-  const bool vec = (d % 4 == 0) && fb_aligned16(x) && fb_aligned16(dy) && (!gamma || (fb_aligned16(gamma) && fb_aligned16(beta)));
+  FB_REQUIRE(x && mean && rstd, FB_ERR_INVALID_ARG, "%s: NULL pointer", fn);
+  const bool vec = (d % 4 == 0) && fb_aligned16(x) && (dy == nullptr || fb_aligned16(dy)) && (!gamma || (fb_aligned16(gamma) && fb_aligned16(beta)));
   const int64_t pieces = vec ? d / 4 : d;
   int lx = 32;
   while (lx > 1 && lx / 2 >= pieces) lx /= 2;
@@ -1157,7 +1157,7 @@ FB_API int32_t fb_layernorm_bwd_params(fb_ctx* ctx, void* stream_, const float* 
   const int64_t most = (n + 4 * ny - 1) / (4 * ny);
   groups = groups > most ? most : groups;
   groups = groups > 65535 ? 65535 : groups;
-  FB_REQUIRE(col_blocks <= 0x7fffffff, FB_ERR_UNSUPPORTED, "fb_layernorm_bwd_params: too many features");
+  FB_REQUIRE(col_blocks <= 0x7fffffff, FB_ERR_UNSUPPORTED, "%s: too many features", fn);
   if (one) {
     cudaLaunchConfig_t lc;
     memset(&lc, 0, sizeof(lc));
@@ -1171,8 +1171,9 @@ FB_API int32_t fb_layernorm_bwd_params(fb_ctx* ctx, void* stream_, const float* 
     lc.attrs = attr;
     lc.numAttrs = 1;
     const cudaError_t e = fb_act_kind(act, [&](auto k) {
-      return cudaLaunchKernelEx(&lc, vec ? ln_bwd_params_kernel<true, k.value, true> : ln_bwd_params_kernel<false, k.value, true>, x, gamma, beta, mean,
-                                rstd, dy, dy_scale, dgamma, dbeta, d, n, (int)act, lx);
+      return cudaLaunchKernelEx(&lc, dy == nullptr ? (vec ? ln_bwd_params_kernel<true, k.value, true, true> : ln_bwd_params_kernel<false, k.value, true, true>)
+                                                   : (vec ? ln_bwd_params_kernel<true, k.value, true, false> : ln_bwd_params_kernel<false, k.value, true, false>),
+                                x, gamma, beta, mean, rstd, dy, dy_scale, dgamma, dbeta, d, n, (int)act, lx);
     });
     FB_CUDA(e);
     FB_LAUNCH_CHECK();
@@ -1183,13 +1184,29 @@ FB_API int32_t fb_layernorm_bwd_params(fb_ctx* ctx, void* stream_, const float* 
   float *pg = part, *pb = part + groups * d;
   const dim3 grid((unsigned)col_blocks, (unsigned)groups);
   fb_act_kind(act, [&](auto k) {
-    if (vec) ln_bwd_params_kernel<true, k.value, false><<<grid, LN_THREADS, 0, stream>>>(x, gamma, beta, mean, rstd, dy, dy_scale, pg, pb, d, n, act, lx);
-    else ln_bwd_params_kernel<false, k.value, false><<<grid, LN_THREADS, 0, stream>>>(x, gamma, beta, mean, rstd, dy, dy_scale, pg, pb, d, n, act, lx);
+    auto kern = dy == nullptr ? (vec ? ln_bwd_params_kernel<true, k.value, false, true> : ln_bwd_params_kernel<false, k.value, false, true>)
+                              : (vec ? ln_bwd_params_kernel<true, k.value, false, false> : ln_bwd_params_kernel<false, k.value, false, false>);
+    kern<<<grid, LN_THREADS, 0, stream>>>(x, gamma, beta, mean, rstd, dy, dy_scale, pg, pb, d, n, act, lx);
   });
   FB_LAUNCH_CHECK();
   fb_colreduce2_kernel<<<(unsigned)((d + 31) / 32), 256, 0, stream>>>(pg, pb, dgamma, dbeta, groups, d);
   FB_LAUNCH_CHECK();
   return FB_OK;
+}
+
+FB_API int32_t fb_layernorm_bwd_params(fb_ctx* ctx, void* stream, const float* x, const float* gamma, const float* beta,
+                                       const float* mean, const float* rstd, const float* dy, float dy_scale, float* dgamma,
+                                       float* dbeta, int64_t d, int64_t n, int32_t act) {
+  FB_CHECK_CTX(ctx);
+  FB_REQUIRE(dy != nullptr || n <= 0, FB_ERR_INVALID_ARG, "fb_layernorm_bwd_params: NULL pointer");
+  return ln_bwd_params("fb_layernorm_bwd_params", ctx, (cudaStream_t)stream, x, gamma, beta, mean, rstd, dy, dy_scale, dgamma, dbeta, d, n, act);
+}
+
+FB_API int32_t fb_layernorm_bwd_params_own(fb_ctx* ctx, void* stream, const float* x, const float* gamma, const float* beta,
+                                           const float* mean, const float* rstd, float y_scale, float* dgamma, float* dbeta, int64_t d,
+                                           int64_t n, int32_t act) {
+  FB_CHECK_CTX(ctx);
+  return ln_bwd_params("fb_layernorm_bwd_params_own", ctx, (cudaStream_t)stream, x, gamma, beta, mean, rstd, nullptr, y_scale, dgamma, dbeta, d, n, act);
 }
 
 static bool ln_low_ok(const void* x, const float* gamma, const float* beta, const void* b, const void* c, int64_t d) {

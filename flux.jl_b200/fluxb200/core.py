@@ -289,6 +289,11 @@ def unscaled(g: B200Array):
     return to_f32(g), 1.0
 
 
+def is_scaled(g: B200Array, y: B200Array) -> bool:
+    """Whether the cotangent `g` is a factor times `y` itself, and nobody has read it."""
+    return isinstance(g, Scaled) and not g.backed and g.base is y
+
+
 # ------------------------------------------------------------------------------------- tape ---
 class Tape:
     """Reverse-mode tape: a list of (output, inputs, pullback) recorded while `Tape.active`."""

@@ -15,7 +15,7 @@ import numpy as np
 import torch
 
 from . import lib
-from .core import B200Array, Tape, context, empty, gpu, is_bf16, narrow, shared_bf16, to_bf16, to_f32, unscaled, zeros
+from .core import B200Array, Tape, context, empty, gpu, is_bf16, is_scaled, narrow, shared_bf16, to_bf16, to_f32, unscaled, zeros
 from .init import glorot_uniform
 
 
@@ -380,6 +380,9 @@ class LayerNorm(Layer):
                 if need_dx:
                     lib.call("fb_layernorm_bwd", ctx.handle, ctx.stream, x.ptr, _ptr(g), _ptr(b), mean.ptr, rstd.ptr, dy.ptr,
                              dx.ptr, _ptr(dg), _ptr(dbeta), d, n, act)
+                elif is_scaled(dy, y):
+                    lib.call("fb_layernorm_bwd_params_own", ctx.handle, ctx.stream, x.ptr, g.ptr, b.ptr, mean.ptr, rstd.ptr, dy.factor, dg.ptr, dbeta.ptr,
+                             d, n, act)
                 else:
                     dy, factor = unscaled(dy)
                     lib.call("fb_layernorm_bwd_params", ctx.handle, ctx.stream, x.ptr, g.ptr, b.ptr, mean.ptr, rstd.ptr, dy.ptr, factor,
@@ -486,6 +489,9 @@ class BatchNorm(Layer):
                 if need_dx:
                     lib.call("fb_batchnorm_bwd", ctx.handle, ctx.stream, x.ptr, _ptr(g), _ptr(b), mean.ptr, rstd.ptr, dy.ptr,
                              dx.ptr, _ptr(dg), _ptr(dbeta), s, c, n, act)
+                elif is_scaled(dy, y):
+                    lib.call("fb_batchnorm_bwd_params_own", ctx.handle, ctx.stream, x.ptr, g.ptr, b.ptr, mean.ptr, rstd.ptr, dy.factor, dg.ptr, dbeta.ptr,
+                             s, c, n, act)
                 else:
                     dy, factor = unscaled(dy)
                     lib.call("fb_batchnorm_bwd_params", ctx.handle, ctx.stream, x.ptr, g.ptr, b.ptr, mean.ptr, rstd.ptr, dy.ptr, factor,

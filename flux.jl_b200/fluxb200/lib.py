@@ -75,6 +75,8 @@ PROTOTYPES = {
     "fb_batchnorm_fwd_infer": (_i32, [_p, _p, _p, _p, _p, _p, _p, _p, _i64, _i64, _i64, _f, _i32]),
     "fb_batchnorm_bwd": (_i32, [_p, _p, _p, _p, _p, _p, _p, _p, _p, _p, _p, _i64, _i64, _i64, _i32]),
     "fb_batchnorm_bwd_params": (_i32, [_p] * 8 + [_f, _p, _p, _i64, _i64, _i64, _i32]),
+    "fb_batchnorm_bwd_params_own": (_i32, [_p] * 7 + [_f, _p, _p, _i64, _i64, _i64, _i32]),
+    "fb_layernorm_bwd_params_own": (_i32, [_p] * 7 + [_f, _p, _p, _i64, _i64, _i32]),
     "fb_groupnorm_fwd": (_i32, [_p, _p, _p, _p, _p, _p, _p, _p, _i64, _i64, _i64, _i64, _f, _i32]),
     "fb_groupnorm_bwd": (_i32, [_p, _p, _p, _p, _p, _p, _p, _p, _p, _p, _p, _i64, _i64, _i64, _i64, _i32]),
     "fb_instancenorm_update_stats": (_i32, [_p, _p, _p, _p, _p, _p, _i64, _i64, _i64, _f, _f]),

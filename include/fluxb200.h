@@ -189,6 +189,10 @@ int32_t fb_layernorm_bwd(fb_ctx* ctx, void* stream, const float* x, const float*
 int32_t fb_layernorm_bwd_params(fb_ctx* ctx, void* stream, const float* x, const float* gamma, const float* beta,
                                 const float* mean, const float* rstd, const float* dy, float dy_scale,
                                 float* dgamma, float* dbeta, int64_t d, int64_t n, int32_t act);
+/* The same where the cotangent is y_scale times the layer's own output (that of sum(abs2, y) is 2 y): y is made from x again instead of
+ * being read. */
+int32_t fb_layernorm_bwd_params_own(fb_ctx* ctx, void* stream, const float* x, const float* gamma, const float* beta, const float* mean,
+                                    const float* rstd, float y_scale, float* dgamma, float* dbeta, int64_t d, int64_t n, int32_t act);
 
 /* fb_layernorm_fwd / fb_layernorm_bwd where x (and dx with it), y and dy may be BFloat16 arrays (raw bits in uint16): x_bf16,
  * y_bf16, dy_bf16 say which.  Parameters, statistics and all arithmetic are Float32, as if the arrays were cast on the
@@ -244,6 +248,11 @@ int32_t fb_batchnorm_bwd(fb_ctx* ctx, void* stream, const float* x, const float*
 int32_t fb_batchnorm_bwd_params(fb_ctx* ctx, void* stream, const float* x, const float* gamma, const float* beta,
                                 const float* save_mean, const float* save_rstd, const float* dy, float dy_scale,
                                 float* dgamma, float* dbeta, int64_t s, int64_t c, int64_t n, int32_t act);
+/* The same where the cotangent is y_scale times the layer's own output (that of sum(abs2, y) is 2 y): y is made from x again instead of
+ * being read. */
+int32_t fb_batchnorm_bwd_params_own(fb_ctx* ctx, void* stream, const float* x, const float* gamma, const float* beta,
+                                    const float* save_mean, const float* save_rstd, float y_scale, float* dgamma, float* dbeta,
+                                    int64_t s, int64_t c, int64_t n, int32_t act);
 
 /* ------------------------------------------------------------------- GroupNorm / InstanceNorm -- */
 
