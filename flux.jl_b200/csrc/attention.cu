@@ -28,6 +28,7 @@ struct AttnDims {
   // redo_n bytes per (batch, head), or NULL: only heads with a byte set are computed (see fb_attn_fwd_redo)
   const uint8_t* redo;
   int redo_n;
+  int64_t dlt_ld;   // REDO kernels of the backward pass: words from one head's deltas to the next one's, which lie two words apart
 };
 
 // the logit of (query i, key j): scaled score plus the additive bias
@@ -271,8 +272,11 @@ attn_delta_kernel(const float* __restrict__ o, const float* __restrict__ dout, f
   if (lane == 0) dlt[(b * D.H + h) * D.Lq + i] = s;
 }
 
-// P and dS tiles for (q tile i0, kv tile j0) from staged Q, K, V, dO.
-template <int LD>
+__device__ __forceinline__ void attn_put(float* p, float v) { *p = v; }
+__device__ __forceinline__ void attn_put(uint16_t* p, float v) { *p = __bfloat16_as_ushort(__float2bfloat16_rn(v)); }
+
+// P and dS tiles for (q tile i0, kv tile j0) from staged Q, K, V, dO.  dlt_bh: words DSTEP apart.
+template <int LD, int DSTEP>
 __device__ __forceinline__ void recompute_p_ds(const AttnDims& D, const uint8_t* mask, const float* Qs, const float* Ks,
                                                const float* Vs, const float* dOs, const float* lse_bh,
                                                const float* dlt_bh, int64_t i0, int64_t j0, int ty, int tx,
@@ -285,7 +289,7 @@ __device__ __forceinline__ void recompute_p_ds(const AttnDims& D, const uint8_t*
   for (int i = 0; i < 4; ++i) {
     const int64_t gi = i0 + ty + 16 * i;
     const float ls = gi < D.Lq ? lse_bh[gi] : -INFINITY;
-    const float dl = gi < D.Lq ? dlt_bh[gi] : 0.0f;
+    const float dl = gi < D.Lq ? dlt_bh[DSTEP * gi] : 0.0f;
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
       const bool keep = attn_keep(D, mask, gi, j0 + tx + 16 * j) && (ls != -INFINITY);
@@ -301,11 +305,11 @@ __device__ __forceinline__ void recompute_p_ds(const AttnDims& D, const uint8_t*
 }
 
 // ------------------------------------------------------------------------- backward: dK, dV ---
-template <int NC>
+template <int NC, typename T, bool REDO>
 __global__ void __launch_bounds__(AT)
-attn_bwd_dkdv_kernel(const float* __restrict__ q, const float* __restrict__ k, const float* __restrict__ v,
+attn_bwd_dkdv_kernel(const T* __restrict__ q, const T* __restrict__ k, const T* __restrict__ v,
                      const uint8_t* __restrict__ mask, const float* __restrict__ lse, const float* __restrict__ dlt,
-                     const float* __restrict__ dout, float* __restrict__ dk, float* __restrict__ dv, AttnDims D) {
+                     const T* __restrict__ dout, T* __restrict__ dk, T* __restrict__ dv, AttnDims D) {
   constexpr int LD = NC * 64 + 4;
   extern __shared__ float sm[];
   float* Ks = sm;
@@ -315,58 +319,67 @@ attn_bwd_dkdv_kernel(const float* __restrict__ q, const float* __restrict__ k, c
   float* Ps = dOs + TS * LD;
   float* dSs = Ps + TS * PLD;
   const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
-  const int64_t j0 = (int64_t)blockIdx.x * TS;
+  int64_t j0 = (int64_t)blockIdx.x * TS;
   const int h = blockIdx.y;
   const int64_t b = blockIdx.z;
-  const float* qb = q + b * D.Lq * D.E + (int64_t)h * D.d;
-  const float* kb = k + b * D.Lk * D.E + (int64_t)h * D.d;
-  const float* vb = v + b * D.Lk * D.Ev + (int64_t)h * D.dv;
-  const float* dob = dout + b * D.Lq * D.Ev + (int64_t)h * D.dv;
+  const T* qb = q + b * D.Lq * D.E + (int64_t)h * D.d;
+  const T* kb = k + b * D.Lk * D.E + (int64_t)h * D.d;
+  const T* vb = v + b * D.Lk * D.Ev + (int64_t)h * D.dv;
+  const T* dob = dout + b * D.Lq * D.Ev + (int64_t)h * D.dv;
   const float* lse_bh = lse + (b * D.H + h) * D.Lq;
-  const float* dlt_bh = dlt + (b * D.H + h) * D.Lq;
-  load_tile<LD>(Ks, kb, D.E, j0, D.Lk, D.d);
-  load_tile<LD>(Vs, vb, D.Ev, j0, D.Lk, D.dv);
-  float adk[NC][4][4], adv[NC][4][4];
-#pragma unroll
-  for (int cc = 0; cc < NC; ++cc)
-#pragma unroll
-    for (int i = 0; i < 4; ++i)
-#pragma unroll
-      for (int e = 0; e < 4; ++e) { adk[cc][i][e] = 0.0f; adv[cc][i][e] = 0.0f; }
-  const int64_t i_begin = D.causal ? j0 : 0;   // queries i < j0 never see keys of this tile
-  for (int64_t i0 = i_begin; i0 < D.Lq; i0 += TS) {
-    __syncthreads();
-    load_tile<LD>(Qs, qb, D.E, i0, D.Lq, D.d);
-    load_tile<LD>(dOs, dob, D.Ev, i0, D.Lq, D.dv);
-    __syncthreads();
-    recompute_p_ds<LD>(D, mask, Qs, Ks, Vs, dOs, lse_bh, dlt_bh, i0, j0, ty, tx, Ps, dSs, b, h);
-    __syncthreads();
-    tile_ptx<NC, LD>(adv, Ps, dOs, ty, tx);
-    tile_ptx<NC, LD>(adk, dSs, Qs, ty, tx);
+  const float* dlt_bh = dlt + (b * D.H + h) * (REDO ? D.dlt_ld : D.Lq);
+  if (REDO) {
+    int any = 0;
+    for (int i = threadIdx.x; i < D.redo_n; i += AT) any |= D.redo[(b * D.H + h) * D.redo_n + i];
+    if (!__syncthreads_or(any)) return;
   }
-  float* dkb = dk + b * D.Lk * D.E + (int64_t)h * D.d;
-  float* dvb = dv + b * D.Lk * D.Ev + (int64_t)h * D.dv;
-#pragma unroll
-  for (int jj = 0; jj < 4; ++jj) {
-    const int64_t gj = j0 + ty + 16 * jj;
-    if (gj >= D.Lk) continue;
+  do {
+    if (REDO) __syncthreads();
+    load_tile<LD>(Ks, kb, D.E, j0, D.Lk, D.d);
+    load_tile<LD>(Vs, vb, D.Ev, j0, D.Lk, D.dv);
+    float adk[NC][4][4], adv[NC][4][4];
 #pragma unroll
     for (int cc = 0; cc < NC; ++cc)
 #pragma unroll
-      for (int e = 0; e < 4; ++e) {
-        const int c = cc * 64 + 4 * tx + e;
-        if (c < D.d) dkb[gj * D.E + c] = adk[cc][jj][e] * D.scale;
-        if (c < D.dv) dvb[gj * D.Ev + c] = adv[cc][jj][e];
-      }
-  }
+      for (int i = 0; i < 4; ++i)
+#pragma unroll
+        for (int e = 0; e < 4; ++e) { adk[cc][i][e] = 0.0f; adv[cc][i][e] = 0.0f; }
+    const int64_t i_begin = D.causal ? j0 : 0;   // queries i < j0 never see keys of this tile
+    for (int64_t i0 = i_begin; i0 < D.Lq; i0 += TS) {
+      __syncthreads();
+      load_tile<LD>(Qs, qb, D.E, i0, D.Lq, D.d);
+      load_tile<LD>(dOs, dob, D.Ev, i0, D.Lq, D.dv);
+      __syncthreads();
+      recompute_p_ds<LD, REDO ? 2 : 1>(D, mask, Qs, Ks, Vs, dOs, lse_bh, dlt_bh, i0, j0, ty, tx, Ps, dSs, b, h);
+      __syncthreads();
+      tile_ptx<NC, LD>(adv, Ps, dOs, ty, tx);
+      tile_ptx<NC, LD>(adk, dSs, Qs, ty, tx);
+    }
+    T* dkb = dk + b * D.Lk * D.E + (int64_t)h * D.d;
+    T* dvb = dv + b * D.Lk * D.Ev + (int64_t)h * D.dv;
+#pragma unroll
+    for (int jj = 0; jj < 4; ++jj) {
+      const int64_t gj = j0 + ty + 16 * jj;
+      if (gj >= D.Lk) continue;
+#pragma unroll
+      for (int cc = 0; cc < NC; ++cc)
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+          const int c = cc * 64 + 4 * tx + e;
+          if (c < D.d) attn_put(dkb + gj * D.E + c, adk[cc][jj][e] * D.scale);
+          if (c < D.dv) attn_put(dvb + gj * D.Ev + c, adv[cc][jj][e]);
+        }
+    }
+    j0 += (int64_t)gridDim.x * TS;
+  } while (REDO && j0 < D.Lk);
 }
 
 // ----------------------------------------------------------------------------- backward: dQ ---
-template <int NC>
+template <int NC, typename T, bool REDO>
 __global__ void __launch_bounds__(AT)
-attn_bwd_dq_kernel(const float* __restrict__ q, const float* __restrict__ k, const float* __restrict__ v,
+attn_bwd_dq_kernel(const T* __restrict__ q, const T* __restrict__ k, const T* __restrict__ v,
                    const uint8_t* __restrict__ mask, const float* __restrict__ lse, const float* __restrict__ dlt,
-                   const float* __restrict__ dout, float* __restrict__ dq, AttnDims D) {
+                   const T* __restrict__ dout, T* __restrict__ dq, AttnDims D) {
   constexpr int LD = NC * 64 + 4;
   extern __shared__ float sm[];
   float* Qs = sm;
@@ -375,48 +388,57 @@ attn_bwd_dq_kernel(const float* __restrict__ q, const float* __restrict__ k, con
   float* Vs = Ks + TS * LD;
   float* dSs = Vs + TS * LD;
   const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
-  const int64_t i0 = (int64_t)blockIdx.x * TS;
+  int64_t i0 = (int64_t)blockIdx.x * TS;
   const int h = blockIdx.y;
   const int64_t b = blockIdx.z;
-  const float* qb = q + b * D.Lq * D.E + (int64_t)h * D.d;
-  const float* kb = k + b * D.Lk * D.E + (int64_t)h * D.d;
-  const float* vb = v + b * D.Lk * D.Ev + (int64_t)h * D.dv;
-  const float* dob = dout + b * D.Lq * D.Ev + (int64_t)h * D.dv;
+  const T* qb = q + b * D.Lq * D.E + (int64_t)h * D.d;
+  const T* kb = k + b * D.Lk * D.E + (int64_t)h * D.d;
+  const T* vb = v + b * D.Lk * D.Ev + (int64_t)h * D.dv;
+  const T* dob = dout + b * D.Lq * D.Ev + (int64_t)h * D.dv;
   const float* lse_bh = lse + (b * D.H + h) * D.Lq;
-  const float* dlt_bh = dlt + (b * D.H + h) * D.Lq;
-  load_tile<LD>(Qs, qb, D.E, i0, D.Lq, D.d);
-  load_tile<LD>(dOs, dob, D.Ev, i0, D.Lq, D.dv);
-  float adq[NC][4][4];
-#pragma unroll
-  for (int cc = 0; cc < NC; ++cc)
-#pragma unroll
-    for (int i = 0; i < 4; ++i)
-#pragma unroll
-      for (int e = 0; e < 4; ++e) adq[cc][i][e] = 0.0f;
-  int64_t kv_end = D.Lk;
-  if (D.causal && i0 + TS < kv_end) kv_end = i0 + TS;
-  for (int64_t j0 = 0; j0 < kv_end; j0 += TS) {
-    __syncthreads();
-    load_tile<LD>(Ks, kb, D.E, j0, D.Lk, D.d);
-    load_tile<LD>(Vs, vb, D.Ev, j0, D.Lk, D.dv);
-    __syncthreads();
-    recompute_p_ds<LD>(D, mask, Qs, Ks, Vs, dOs, lse_bh, dlt_bh, i0, j0, ty, tx, nullptr, dSs, b, h);
-    __syncthreads();
-    tile_pv<NC, LD>(adq, dSs, Ks, ty, tx);
+  const float* dlt_bh = dlt + (b * D.H + h) * (REDO ? D.dlt_ld : D.Lq);
+  if (REDO) {
+    int any = 0;
+    for (int i = threadIdx.x; i < D.redo_n; i += AT) any |= D.redo[(b * D.H + h) * D.redo_n + i];
+    if (!__syncthreads_or(any)) return;
   }
-  float* dqb = dq + b * D.Lq * D.E + (int64_t)h * D.d;
-#pragma unroll
-  for (int i = 0; i < 4; ++i) {
-    const int64_t gi = i0 + ty + 16 * i;
-    if (gi >= D.Lq) continue;
+  do {
+    if (REDO) __syncthreads();
+    load_tile<LD>(Qs, qb, D.E, i0, D.Lq, D.d);
+    load_tile<LD>(dOs, dob, D.Ev, i0, D.Lq, D.dv);
+    float adq[NC][4][4];
 #pragma unroll
     for (int cc = 0; cc < NC; ++cc)
 #pragma unroll
-      for (int e = 0; e < 4; ++e) {
-        const int c = cc * 64 + 4 * tx + e;
-        if (c < D.d) dqb[gi * D.E + c] = adq[cc][i][e] * D.scale;
-      }
-  }
+      for (int i = 0; i < 4; ++i)
+#pragma unroll
+        for (int e = 0; e < 4; ++e) adq[cc][i][e] = 0.0f;
+    int64_t kv_end = D.Lk;
+    if (D.causal && i0 + TS < kv_end) kv_end = i0 + TS;
+    for (int64_t j0 = 0; j0 < kv_end; j0 += TS) {
+      __syncthreads();
+      load_tile<LD>(Ks, kb, D.E, j0, D.Lk, D.d);
+      load_tile<LD>(Vs, vb, D.Ev, j0, D.Lk, D.dv);
+      __syncthreads();
+      recompute_p_ds<LD, REDO ? 2 : 1>(D, mask, Qs, Ks, Vs, dOs, lse_bh, dlt_bh, i0, j0, ty, tx, nullptr, dSs, b, h);
+      __syncthreads();
+      tile_pv<NC, LD>(adq, dSs, Ks, ty, tx);
+    }
+    T* dqb = dq + b * D.Lq * D.E + (int64_t)h * D.d;
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      const int64_t gi = i0 + ty + 16 * i;
+      if (gi >= D.Lq) continue;
+#pragma unroll
+      for (int cc = 0; cc < NC; ++cc)
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+          const int c = cc * 64 + 4 * tx + e;
+          if (c < D.d) attn_put(dqb + gi * D.E + c, adq[cc][i][e] * D.scale);
+        }
+    }
+    i0 += (int64_t)gridDim.x * TS;
+  } while (REDO && i0 < D.Lq);
 }
 
 // --------------------------------------------------------------------- scores on demand ---
@@ -490,7 +512,7 @@ int32_t attn_make_dims(const char* fn, AttnDims* D, int64_t e_dim, int64_t ev_di
   D->scale = 1.0f / sqrtf((float)D->d);
   D->bias = nullptr; D->bias_sh = 0; D->bias_sb = 0; D->dalpha = nullptr;
   D->p_drop = 0.0f; D->drop_scale = 1.0f; D->seed = 0; D->offset = 0;
-  D->redo = nullptr; D->redo_n = 0;
+  D->redo = nullptr; D->redo_n = 0; D->dlt_ld = 0;
   return FB_OK;
 }
 
@@ -529,6 +551,41 @@ int32_t fb_attn_fwd_redo(fb_ctx* ctx, cudaStream_t stream, int bf16, const void*
   }
   FB_LAUNCH_CHECK();
   return FB_OK;
+}
+
+template <typename T>
+static int32_t bwd_redo(fb_ctx* ctx, cudaStream_t stream, const void* q, const void* k, const void* v, const float* lse, const float* dlt, const void* dout, void* dq,
+                        void* dk, void* dv, int64_t batch, const AttnDims& D) {
+  constexpr size_t smem_kv = (size_t)(4 * TS * (64 + 4) + 2 * TS * PLD) * sizeof(float), smem_q = (size_t)(4 * TS * (64 + 4) + TS * PLD) * sizeof(float);
+  // about two blocks per SM: a launch that finds nothing to do is over in one wave
+  const int64_t fit = (int64_t)ctx->sm_count * 2 / (batch * D.H);
+  auto blocks = [&](int64_t len) {
+    const int64_t tiles = (len + TS - 1) / TS;
+    return (unsigned)(fit < 1 ? 1 : fit > tiles ? tiles : fit);
+  };
+  if (dk != nullptr) {
+    FB_CUDA(cudaFuncSetAttribute(attn_bwd_dkdv_kernel<1, T, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_kv));
+    attn_bwd_dkdv_kernel<1, T, true><<<dim3(blocks(D.Lk), (unsigned)D.H, (unsigned)batch), AT, smem_kv, stream>>>(
+        (const T*)q, (const T*)k, (const T*)v, nullptr, lse, dlt, (const T*)dout, (T*)dk, (T*)dv, D);
+    FB_LAUNCH_CHECK();
+  }
+  if (dq != nullptr) {
+    FB_CUDA(cudaFuncSetAttribute(attn_bwd_dq_kernel<1, T, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_q));
+    attn_bwd_dq_kernel<1, T, true><<<dim3(blocks(D.Lq), (unsigned)D.H, (unsigned)batch), AT, smem_q, stream>>>(
+        (const T*)q, (const T*)k, (const T*)v, nullptr, lse, dlt, (const T*)dout, (T*)dq, D);
+    FB_LAUNCH_CHECK();
+  }
+  return FB_OK;
+}
+int32_t fb_attn_bwd_redo(fb_ctx* ctx, cudaStream_t stream, int bf16, const void* q, const void* k, const void* v, const float* lse, const float* dlt,
+                         int64_t dlt_rows, const void* dout, void* dq, void* dk, void* dv, int64_t e_dim, int64_t ev_dim, int64_t lq, int64_t lk,
+                         int64_t batch, int nheads, int causal, const uint8_t* redo, int redo_n) {
+  AttnDims D;
+  const int32_t st = attn_make_dims("fb_attn_bwd", &D, e_dim, ev_dim, lq, lk, batch, nheads, causal);
+  if (st != FB_OK) return st;
+  D.redo = redo; D.redo_n = redo_n; D.dlt_ld = 2 * dlt_rows;
+  return bf16 ? bwd_redo<uint16_t>(ctx, stream, q, k, v, lse, dlt, dout, dq, dk, dv, batch, D)
+              : bwd_redo<float>(ctx, stream, q, k, v, lse, dlt, dout, dq, dk, dv, batch, D);
 }
 
 FB_API int32_t fb_attn_fwd(fb_ctx* ctx, void* stream_, const float* q, const float* k, const float* v,
@@ -626,20 +683,20 @@ FB_API int32_t fb_attn_bwd_ex(fb_ctx* ctx, void* stream_, const float* q, const 
   dim3 grid_kv((unsigned)((lk + TS - 1) / TS), (unsigned)nheads, (unsigned)batch);
   dim3 grid_q((unsigned)((lq + TS - 1) / TS), (unsigned)nheads, (unsigned)batch);
   if (nc == 1) {
-    FB_CUDA(cudaFuncSetAttribute(attn_bwd_dkdv_kernel<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_kv));
-    FB_CUDA(cudaFuncSetAttribute(attn_bwd_dq_kernel<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_q));
+    FB_CUDA(cudaFuncSetAttribute(attn_bwd_dkdv_kernel<1, float, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_kv));
+    FB_CUDA(cudaFuncSetAttribute(attn_bwd_dq_kernel<1, float, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_q));
     if (!did_kv) {
-      attn_bwd_dkdv_kernel<1><<<grid_kv, AT, smem_kv, stream>>>(q, k, v, mask, lse, dlt, dout, dk, dv, D);
+      attn_bwd_dkdv_kernel<1, float, false><<<grid_kv, AT, smem_kv, stream>>>(q, k, v, mask, lse, dlt, dout, dk, dv, D);
       FB_LAUNCH_CHECK();
     }
     if (did_q) return FB_OK;
-    attn_bwd_dq_kernel<1><<<grid_q, AT, smem_q, stream>>>(q, k, v, mask, lse, dlt, dout, dq, D);
+    attn_bwd_dq_kernel<1, float, false><<<grid_q, AT, smem_q, stream>>>(q, k, v, mask, lse, dlt, dout, dq, D);
   } else {
-    FB_CUDA(cudaFuncSetAttribute(attn_bwd_dkdv_kernel<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_kv));
-    FB_CUDA(cudaFuncSetAttribute(attn_bwd_dq_kernel<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_q));
-    attn_bwd_dkdv_kernel<2><<<grid_kv, AT, smem_kv, stream>>>(q, k, v, mask, lse, dlt, dout, dk, dv, D);
+    FB_CUDA(cudaFuncSetAttribute(attn_bwd_dkdv_kernel<2, float, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_kv));
+    FB_CUDA(cudaFuncSetAttribute(attn_bwd_dq_kernel<2, float, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_q));
+    attn_bwd_dkdv_kernel<2, float, false><<<grid_kv, AT, smem_kv, stream>>>(q, k, v, mask, lse, dlt, dout, dk, dv, D);
     FB_LAUNCH_CHECK();
-    attn_bwd_dq_kernel<2><<<grid_q, AT, smem_q, stream>>>(q, k, v, mask, lse, dlt, dout, dq, D);
+    attn_bwd_dq_kernel<2, float, false><<<grid_q, AT, smem_q, stream>>>(q, k, v, mask, lse, dlt, dout, dq, D);
   }
   FB_LAUNCH_CHECK();
   return FB_OK;

@@ -313,6 +313,10 @@ int32_t fb_attn_fwd_tc(fb_ctx* ctx, cudaStream_t stream, const float* q, const f
 int32_t fb_attn_fwd_redo(fb_ctx* ctx, cudaStream_t stream, int bf16, const void* q, const void* k, const void* v, float* o, uint16_t* o16,
                          float* lse, int64_t e_dim, int64_t ev_dim, int64_t lq, int64_t lk, int64_t batch, int nheads, int causal,
                          const uint8_t* redo, int redo_n);
+// the same for the backward pass: dlt in every second word from the one given, dlt_rows of them per (batch, head); dq or dk and dv may be NULL
+int32_t fb_attn_bwd_redo(fb_ctx* ctx, cudaStream_t stream, int bf16, const void* q, const void* k, const void* v, const float* lse, const float* dlt,
+                         int64_t dlt_rows, const void* dout, void* dq, void* dk, void* dv, int64_t e_dim, int64_t ev_dim, int64_t lq, int64_t lk,
+                         int64_t batch, int nheads, int causal, const uint8_t* redo, int redo_n);
 int32_t fb_attn_bwd_tc(fb_ctx* ctx, cudaStream_t stream, const float* q, const float* k, const float* v, const uint8_t* mask, const float* o,
                        const float* lse, const float* dout, float* dq, float* dk, float* dv, int64_t e_dim, int64_t ev_dim, int64_t lq,
                        int64_t lk, int64_t batch, int nheads, int causal, bool* did_kv, bool* did_q);
