@@ -60,10 +60,6 @@ __device__ __forceinline__ void tc_wait_st() { asm volatile("tcgen05.wait::st.sy
 // 14 bits.  (As 64-bit sums for A and B under a run-time step count one form of the product below gave wrong low-order terms;
 // where the compiler went wrong there is not known, so no form adds to 64 bits.)
 //
-// The issuing warp runs as a whole, and one elected lane of it issues: where the compiler sees that all lanes agree, addresses stay in
-// uniform registers, which the instruction reads.  Under `if (lane == 0)` every operand of every MMA was moved there one by one, 88
-// clocks an MMA whose multiplications take 32.
-//
 // D[tmem] (+)= A[tmem] * B[smem]: the A tile (128 rows x 16 halves) sits in 8 consecutive TMEM columns, two values each
 __device__ __forceinline__ void tc_mma_ta(uint32_t d_tmem, uint32_t a_tmem, uint32_t b_lo, uint32_t hi, uint32_t idesc, uint32_t accumulate) {
   asm volatile(
@@ -110,19 +106,6 @@ __device__ __forceinline__ void tc_mma_sa_down(uint32_t d_tmem, uint32_t a_lo, u
       ::"r"(d_tmem), "r"(a_lo), "r"(b_lo), "r"(idesc), "r"(0u), "r"(hi)
       : "memory");
 }
-// arrives at the barrier when the MMAs issued so far are done
-__device__ __forceinline__ void tc_commit_one(uint32_t bar) {
-  asm volatile(
-      "{\n\t.reg .pred q;\n\telect.sync _|q, 0xffffffff;\n\t"
-      "@q tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n\t}"
-      ::"r"(bar)
-      : "memory");
-}
-// a wait of a whole warp whose result every lane shares
-__device__ __forceinline__ bool warp_wait(uint32_t bar, uint32_t parity, volatile int* s_abort) {
-  return __all_sync(0xffffffffu, mbar_wait(bar, parity, s_abort)) != 0;
-}
-
 // plain bulk copy of a piece of a plane image (both addresses and the size are multiples of 16 bytes)
 __device__ __forceinline__ void bulk_load(uint32_t dst, const void* src, uint32_t bytes, uint32_t bar) {
   asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
@@ -523,7 +506,7 @@ attn_fwd_tc_kernel(const void* __restrict__ qmat, const uint8_t* __restrict__ ki
   volatile int* s_abort = (volatile int*)(s_tmem + 1);
   volatile int* s_skip = (volatile int*)(s_tmem + 2);
 
-  const int warp = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0), lane = threadIdx.x & 31;
+  const int warp = uniform_warp(), lane = threadIdx.x & 31;
   // causal: the last query tiles have the most key blocks, so they are scheduled first
   const int64_t i0 = (int64_t)(D.causal ? gridDim.x - 1 - blockIdx.x : blockIdx.x) * QT;
   const int h = blockIdx.y;
@@ -576,8 +559,8 @@ attn_fwd_tc_kernel(const void* __restrict__ qmat, const uint8_t* __restrict__ ki
         if (!warp_wait(bar(B_FULL + s), (uint32_t)(n / S) & 1u, s_abort)) return false;
         tc_fence_after();
         mma_rows_t<NP>(tmem + T_R, tmem, sb + (uint32_t)(s * cfg::SLOT_BYTES), nks);
-        tc_commit_one(bar(B_SFULL));
-        tc_commit_one(bar(B_FREE + s));
+        tc_commit(bar(B_SFULL));
+        tc_commit(bar(B_FREE + s));
         return true;
       };
       bool ok = warp_wait(bar(B_QREADY), 0u, s_abort) && issue_s(0);
@@ -587,8 +570,8 @@ attn_fwd_tc_kernel(const void* __restrict__ qmat, const uint8_t* __restrict__ ki
         if (!ok) break;
         tc_fence_after();
         mma_planes<NP>(tmem + T_O, tmem + T_R, sb + (uint32_t)(s * cfg::SLOT_BYTES), nv);
-        tc_commit_one(bar(B_OFULL));
-        tc_commit_one(bar(B_FREE + s));
+        tc_commit(bar(B_OFULL));
+        tc_commit(bar(B_FREE + s));
         // the next scores go where the weights are: the tensor pipe runs in order
         if (j + 1 < nkb) ok = issue_s(j + 1);
       }
@@ -792,7 +775,7 @@ attn_bwd_dq_tc_kernel(const void* __restrict__ q, const void* __restrict__ dout,
 
   __shared__ HeadShifts hs;
   __shared__ int16_t row_q[QT], row_d[QT];
-  const int warp = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0), lane = threadIdx.x & 31;
+  const int warp = uniform_warp(), lane = threadIdx.x & 31;
   const int64_t i0 = (int64_t)(D.causal ? gridDim.x - 1 - blockIdx.x : blockIdx.x) * QT;
   const int h = blockIdx.y;
   const int64_t b = blockIdx.z, bh = b * D.H + h;
@@ -854,8 +837,8 @@ attn_bwd_dq_tc_kernel(const void* __restrict__ q, const void* __restrict__ dout,
           tc_fence_after();
           const uint32_t r = tmem + T_R + (uint32_t)(128 * (j & 1));
           mma_planes_sum<NP>(tmem + T_DQ, tmem + T_DX, r, sb + (uint32_t)((j % S) * cfg::SLOT_BYTES), nd, j > 0);
-          tc_commit_one(bar(B_FREE + j % S));
-          if (j == nkb - 1) tc_commit_one(bar(B_DONE));
+          tc_commit(bar(B_FREE + j % S));
+          if (j == nkb - 1) tc_commit(bar(B_DONE));
         }
         const int t = j + 2, s = t % S;
         if (t < nkb) {
@@ -865,7 +848,7 @@ attn_bwd_dq_tc_kernel(const void* __restrict__ q, const void* __restrict__ dout,
           const uint32_t base = sb + (uint32_t)(s * cfg::SLOT_BYTES), r = tmem + T_R + (uint32_t)(128 * (t & 1));
           mma_rows_t<NP>(r, tmem, base, nks);
           mma_rows_t<NP>(r + 64u, tmem + T_DO, base + NP * TILE, nvs);
-          tc_commit_one(bar(B_SFULL + (t & 1)));
+          tc_commit(bar(B_SFULL + (t & 1)));
         }
       }
     }
@@ -995,7 +978,7 @@ attn_bwd_dkdv_tc_kernel(const uint8_t* __restrict__ qimg, const uint8_t* __restr
   volatile int* s_skip = (volatile int*)(s_tmem + 2);
 
   __shared__ HeadShifts hs;
-  const int warp = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0), lane = threadIdx.x & 31;
+  const int warp = uniform_warp(), lane = threadIdx.x & 31;
   const int64_t j0 = (int64_t)blockIdx.x * QT;   // first key of this CTA
   const int h = blockIdx.y;
   const int64_t b = blockIdx.z, bh = b * D.H + h;
@@ -1068,10 +1051,10 @@ attn_bwd_dkdv_tc_kernel(const uint8_t* __restrict__ qimg, const uint8_t* __restr
           tc_fence_after();
           const uint32_t r = tmem + (uint32_t)(128 * (i & 1));
           mma_planes_sum<NP>(tmem + T_DV, tmem + T_DV + 64u, r, slot(2 * i), nv, i > 0);
-          tc_commit_one(bar(B_FREE + (2 * i) % S));
+          tc_commit(bar(B_FREE + (2 * i) % S));
           mma_planes_sum<NP>(tmem + T_DK, tmem + T_DK + 64u, r + 64u, slot(2 * i + 1), nd, i > 0);
-          tc_commit_one(bar(B_FREE + (2 * i + 1) % S));
-          if (i == nqb - 1) tc_commit_one(bar(B_DONE));
+          tc_commit(bar(B_FREE + (2 * i + 1) % S));
+          if (i == nqb - 1) tc_commit(bar(B_DONE));
         }
         const int t = i + 2;
         if (t < nqb) {
@@ -1084,7 +1067,7 @@ attn_bwd_dkdv_tc_kernel(const uint8_t* __restrict__ qimg, const uint8_t* __restr
           if (!ok) break;
           tc_fence_after();
           mma_rows_s<NP>(r, sb + cfg::K_OFF, slot(2 * t + 1));
-          tc_commit_one(bar(B_SFULL + (t & 1)));
+          tc_commit(bar(B_SFULL + (t & 1)));
         }
       }
     }

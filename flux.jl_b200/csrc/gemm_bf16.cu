@@ -78,7 +78,7 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
   volatile int* s_abort = (volatile int*)(bars + 3 * STAGES + 5);
   volatile int* s_skip = (volatile int*)(bars + 3 * STAGES + 6);   // [0] mine, [1] written by the peer CTA
 
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = uniform_warp(), lane = threadIdx.x & 31;
   const int ksplit = SPLIT ? nsplit : 1;
   const uint32_t crank = (PAIR || SPLIT) ? cluster_ctarank() : 0u;
   const uint32_t rank = PAIR ? (crank & 1u) : 0u;
@@ -141,7 +141,7 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
-  const uint32_t tmem_base = *s_tmem;
+  const uint32_t tmem_base = __reduce_or_sync(0xffffffffu, *s_tmem);
 
   // 8 consecutive columns of one row: accumulate, bias, pre-activation, activation, store
   auto emit8 = [&](int row, float* u, int n) {
@@ -251,7 +251,7 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
     }
   } else if (warp == 1) {
     // -------------------------------------------------- MMA issuer (the leader CTA of a pair) ---
-    if (lane == 0 && leader) {
+    if (leader) {
       // instruction descriptor: D = F32, A = B = BF16, operand majors, N >> 3, M >> 4
       const uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((A_MN ? 1u : 0u) << 15) | ((B_MN ? 1u : 0u) << 16) |
                              ((uint32_t)(BN >> 3) << 17) | ((uint32_t)((PAIR ? 256 : HBM_) >> 4) << 24);
@@ -261,14 +261,14 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
         const int buf = tc & 1, use = tc >> 1;
         if (use > 0) {
           // the epilogue warps must have drained this accumulator buffer's previous tile
-          ok = mbar_wait_cluster(tmem_empty_bar(buf), (uint32_t)(use - 1) & 1u, s_abort);
+          ok = warp_wait_cluster(tmem_empty_bar(buf), (uint32_t)(use - 1) & 1u, s_abort);
           if (!ok) break;
         }
         const uint32_t d_tmem = tmem_base + (uint32_t)(buf * BN);
         for (int kb = 0; kb < num_kb && ok; ++kb, ++it) {
           const int s = it % STAGES;
           const uint32_t ph = (uint32_t)(it / STAGES) & 1u;
-          ok = mbar_wait_cluster(full_bar(s), ph, s_abort);
+          ok = warp_wait_cluster(full_bar(s), ph, s_abort);
           if (!ok) break;
           tc_fence_after();
           const uint32_t a_s = smem_base + (uint32_t)(s * cfg::STAGE_BYTES);

@@ -209,7 +209,7 @@ gemm_planes_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constan
   volatile int* s_abort = (volatile int*)(bars + 2 * STAGES + 5);
   volatile int* s_skip = (volatile int*)(bars + 2 * STAGES + 6);   // [0] mine, [1] written by the cluster's first CTA
 
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = uniform_warp(), lane = threadIdx.x & 31;
   const int ksplit = SPLIT ? sch.ksplit : 1;
   const uint32_t crank = (PAIR || SPLIT) ? cluster_ctarank() : 0u;
   const uint32_t rank = PAIR ? (crank & 1u) : 0u;   // half of the pair's tile
@@ -271,7 +271,7 @@ gemm_planes_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constan
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
-  const uint32_t tmem_base = *s_tmem;
+  const uint32_t tmem_base = __reduce_or_sync(0xffffffffu, *s_tmem);
 
   if (warp == 0) {
     // ------------------------------------------------------------------ TMA producer ---
@@ -303,7 +303,7 @@ gemm_planes_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constan
     }
   } else if (warp == 1) {
     // -------------------------------------------------- MMA issuer (the leader CTA of a pair) ---
-    if (lane == 0 && leader) {
+    if (leader) {
       // instruction descriptor: D = F32, A = B = F16 (code 0), operand majors, N >> 3, M >> 4
       const uint32_t idesc = (1u << 4) | ((uint32_t)a_mn << 15) | ((uint32_t)b_mn << 16) | ((uint32_t)(BN >> 3) << 17) |
                              ((uint32_t)((BM * RANKS) >> 4) << 24);
@@ -323,10 +323,10 @@ gemm_planes_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constan
           const int buf = sc & 1, use = sc >> 1;
           if (kb_in_seg == 0 && use > 0) {
             // the epilogue warps must have drained this accumulator buffer's previous segment
-            ok = mbar_wait_cluster(tmem_empty_bar(buf), (uint32_t)(use - 1) & 1u, s_abort);
+            ok = warp_wait_cluster(tmem_empty_bar(buf), (uint32_t)(use - 1) & 1u, s_abort);
             if (!ok) break;
           }
-          ok = mbar_wait_cluster(full_bar(s), ph, s_abort);
+          ok = warp_wait_cluster(full_bar(s), ph, s_abort);
           if (!ok) break;
           tc_fence_after();
           const uint32_t d_tmem = tmem_base + (uint32_t)(buf * BN);

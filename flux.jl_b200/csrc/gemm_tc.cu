@@ -94,7 +94,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
   volatile int* s_abort = (volatile int*)(bars + 3 * STAGES + 5);
   volatile int* s_skip = (volatile int*)(bars + 3 * STAGES + 6);   // [0] mine, [1] written by the peer CTA
 
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = uniform_warp(), lane = threadIdx.x & 31;
   const bool ksplit = SPLIT && !PAIR && sch.ksplit > 1;   // (pairs take whole tiles: the spare registers of their 22 warps are few)
   const uint32_t crank = (PAIR || ksplit) ? cluster_ctarank() : 0u;
   const uint32_t rank = PAIR ? crank : 0u;   // half of the pair's tile
@@ -157,7 +157,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
-  const uint32_t tmem_base = *s_tmem;
+  const uint32_t tmem_base = __reduce_or_sync(0xffffffffu, *s_tmem);
 
   // u: 4 consecutive columns starting at n of one row.  add_c: add what C holds; fin: this is the tile's final value,
   // so bias, pre-activation store and activation apply.
@@ -243,7 +243,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
     }
   } else if (warp == 1) {
     // -------------------------------------------------- MMA issuer (the leader CTA of a pair) ---
-    if (lane == 0 && leader) {
+    if (leader) {
       // instruction descriptor: D = F32, A = B = TF32, operand majors, N >> 3, M >> 4
       const uint32_t idesc = (1u << 4) | (2u << 7) | (2u << 10) | ((A_MN ? 1u : 0u) << 15) | ((B_MN ? 1u : 0u) << 16) |
                              ((uint32_t)(BN >> 3) << 17) | ((uint32_t)((PAIR ? 256 : BM) >> 4) << 24);
@@ -258,10 +258,10 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
         const int buf = sc & 1, use = sc >> 1;
         if (kb_in_seg == 0 && use > 0) {
           // the epilogue warps must have drained this accumulator buffer's previous segment
-          ok = mbar_wait_cluster(tmem_empty_bar(buf), (uint32_t)(use - 1) & 1u, s_abort);
+          ok = warp_wait_cluster(tmem_empty_bar(buf), (uint32_t)(use - 1) & 1u, s_abort);
           if (!ok) break;
         }
-        ok = mbar_wait_cluster(PASSES == 3 ? ready_bar(s) : full_bar(s), ph, s_abort);
+        ok = warp_wait_cluster(PASSES == 3 ? ready_bar(s) : full_bar(s), ph, s_abort);
         if (!ok) break;
         tc_fence_after();
         const uint32_t d_tmem = tmem_base + (uint32_t)(buf * BN);
