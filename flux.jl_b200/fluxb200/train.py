@@ -343,60 +343,58 @@ def update(opt_state: OptState, model, grad_tree):
     outer = getattr(opt_state, "outer", None)
     if isinstance(outer, DistributedOptimizerBase):
         outer.average_gradients(opt_state, gmap)
-    ctx = context()
-    rule = opt_state.rule
-    ps = [p for p in opt_state.params if id(p) in gmap]
-    seen = set()
-    ps = [p for p in ps if not (id(p) in seen or seen.add(id(p)))]
-    if not ps:
-        return opt_state, model
+    _run_update(opt_state, _plan_update(opt_state, gmap))
+    return opt_state, model
+
+
+def _plan_update(opt_state: OptState, gmap: dict):
+    """The calls that apply the gradients `gmap`, and the leaves' next powers of beta; nothing of the state is touched yet."""
+    rule, calls, powers = opt_state.rule, [], []
+    leaves = opt_state.leaves
+    ps = list({id(p): p for p in opt_state.params if id(p) in gmap}.values())
     # BFloat16 parameters: the rule runs on the Float32 master copy with the gradient widened to Float32; the
     # parameter is the master rounded back
-    low = [p for p in ps if opt_state.leaves[id(p)].master is not None]
-    wmap = {id(p): (opt_state.leaves[id(p)].master if opt_state.leaves[id(p)].master is not None else p) for p in ps}
+    low = [p for p in ps if leaves[id(p)].master is not None]
+    wmap = {id(p): (leaves[id(p)].master if leaves[id(p)].master is not None else p) for p in ps}
     # (in one pass where the gradient is bf16 and the rule Adam)
     fused = {id(p) for p in low if isinstance(rule, Adam) and gmap[id(p)].t.dtype == torch.bfloat16}
-    low = [p for p in low if id(p) not in fused]
     gmap = {k: g if k in fused else to_f32(g) for k, g in gmap.items()}
     if isinstance(rule, Descent):
+        calls = [("fb_axpy", (-rule.eta, gmap[id(p)].ptr, wmap[id(p)].ptr, p.numel())) for p in ps]
+    else:
+        # leaves share (β1ᵗ, β2ᵗ) when they have seen the same number of steps: group by that pair
+        groups: dict = {}
         for p in ps:
-            lib.call("fb_axpy", ctx.handle, ctx.stream, -rule.eta, gmap[id(p)].ptr, wmap[id(p)].ptr, p.numel())
-        _write_back(low, wmap)
-        return opt_state, model
-    # leaves share (β1ᵗ, β2ᵗ) when they have seen the same number of steps: group by that pair
-    groups: dict = {}
-    for p in ps:
-        groups.setdefault((opt_state.leaves[id(p)].state[2], id(p) in fused), []).append(p)
-    for ((b1t, b2t), one_pass), plist in groups.items():
-        k = len(plist)
-        arr_t = C.c_void_p * k
-        w = arr_t(*[wmap[id(p)].t.data_ptr() for p in plist])
-        g = arr_t(*[gmap[id(p)].t.data_ptr() for p in plist])
-        m = arr_t(*[opt_state.leaves[id(p)].state[0].t.data_ptr() for p in plist])
-        v = arr_t(*[opt_state.leaves[id(p)].state[1].t.data_ptr() for p in plist])
-        cnt = (C.c_int64 * k)(*[p.numel() for p in plist])
-        rest = (w, g, m, v, cnt, rule.eta, rule.beta[0], rule.beta[1], rule.epsilon, b1t, b2t, 1.0)
-        if one_pass:
-            lib.call("fb_adam_step_bf16", ctx.handle, ctx.stream, k, arr_t(*[p.t.data_ptr() for p in plist]), *rest)
-        else:
-            lib.call("fb_adam_step", ctx.handle, ctx.stream, k, *rest)
-        nb = _advance_powers((b1t, b2t), rule.beta)
+            groups.setdefault((leaves[id(p)].state[2], id(p) in fused), []).append(p)
+        for ((b1t, b2t), one_pass), plist in groups.items():
+            k = len(plist)
+            table, states = C.c_void_p * k, [leaves[id(p)].state for p in plist]
+            rest = (table(*[wmap[id(p)].t.data_ptr() for p in plist]), table(*[gmap[id(p)].t.data_ptr() for p in plist]),
+                    table(*[s[0].t.data_ptr() for s in states]), table(*[s[1].t.data_ptr() for s in states]), (C.c_int64 * k)(*[p.numel() for p in plist]),
+                    rule.eta, rule.beta[0], rule.beta[1], rule.epsilon, b1t, b2t, 1.0)
+            if one_pass:
+                calls.append(("fb_adam_step_bf16", (k, table(*[p.t.data_ptr() for p in plist])) + rest))
+            else:
+                calls.append(("fb_adam_step", (k,) + rest))
+            powers.append((plist, _advance_powers((b1t, b2t), rule.beta)))
+    calls += [("fb_cast_f32_bf16", (wmap[id(p)].ptr, p.ptr, p.numel())) for p in low if id(p) not in fused]
+    return calls, powers, gmap   # (the gradients live until the calls are made)
+
+
+def _run_update(opt_state: OptState, plan):
+    calls, powers, _ = plan
+    ctx = context()
+    for name, args in calls:
+        lib.call(name, ctx.handle, ctx.stream, *args)
+    for plist, nb in powers:
         for p in plist:
             opt_state.leaves[id(p)].state[2] = nb
-    _write_back(low, wmap)
-    return opt_state, model
 
 
 def _advance_powers(bt, beta):
     """(β1ᵗ, β2ᵗ) of the next step, in Float32 as the rule's state keeps them."""
     f32 = np.float32
     return (float(f32(bt[0]) * f32(beta[0])), float(f32(bt[1]) * f32(beta[1])))
-
-
-def _write_back(low, wmap):
-    ctx = context()
-    for p in low:
-        lib.call("fb_cast_f32_bf16", ctx.handle, ctx.stream, wmap[id(p)].ptr, p.ptr, p.numel())
 
 
 def trainstep(loss, model, batch, opt_state):
@@ -410,18 +408,24 @@ def trainstep(loss, model, batch, opt_state):
         outer.check_async_error()
     if sink is not None:
         sink.begin_step()
+    if not isinstance(outer, DistributedOptimizerBase):
+        value, aux, grads = _withgradient_device(lambda m: loss(m, *batch), model, grad_sink=sink)
+        gmap: dict = {}
+        _flat_grads(model, grads, gmap)
+        plan = _plan_update(opt_state, gmap)   # (while the device is at work; behind the read it would wait for this)
+        lv, err = context().read_scalar(to_f32(value))
+        if err != 0:   # a kernel left its gradients unwritten: they must not reach the parameters
+            _raise_on_device_error()
+        if math.isfinite(lv):
+            _run_update(opt_state, plan)
+        return lv if aux is None else (lv,) + tuple(aux)
     (l, gs), err = _withgradient(lambda m: loss(m, *batch), model, grad_sink=sink)
-    lv = l[0] if isinstance(l, tuple) else l
-    shared = isinstance(outer, DistributedOptimizerBase)
-    if err != 0 and not shared:   # a kernel left its gradients unwritten: they must not reach the parameters
-        _raise_on_device_error()
-    finite = outer.all_finite(lv) if shared else math.isfinite(lv)
-    if finite:
+    if outer.all_finite(l[0] if isinstance(l, tuple) else l):
         update(opt_state, model, gs[0])
     elif sink is not None:
         sink.finish()   # the collectives already started must be matched on every worker
-    if shared:   # (the other workers' collectives had to be matched first; an update alone contains no bounded wait)
-        _raise_on_device_error()
+    # (the other workers' collectives had to be matched first; an update alone contains no bounded wait)
+    _raise_on_device_error()
     return l
 
 
