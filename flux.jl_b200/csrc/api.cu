@@ -211,6 +211,7 @@ FB_API int32_t fb_device_error(fb_ctx* ctx, void* stream, int32_t* out_host) {
 
 // host page: [0] value bits, [1] error word, [2] sequence number
 __global__ void read_scalar_kernel(const float* x, const int32_t* dev_err, volatile uint32_t* page, uint32_t seq) {
+  fb_after_previous();
   page[0] = __float_as_uint(*x);
   page[1] = (uint32_t)*(const volatile int32_t*)dev_err;
   __threadfence_system();
@@ -223,7 +224,7 @@ FB_API int32_t fb_read_scalar(fb_ctx* ctx, void* stream_, const float* x, float*
   cudaStream_t stream = (cudaStream_t)stream_;
   volatile uint32_t* page = ctx->host_page;
   const uint32_t seq = ++ctx->host_seq;
-  read_scalar_kernel<<<1, 1, 0, stream>>>(x, ctx->dev_error, page, seq);
+  fb_launch(read_scalar_kernel, 1, 1, 0, stream, x, ctx->dev_error, page, seq);
   FB_LAUNCH_CHECK();
   for (uint32_t spin = 0; page[2] != seq; ++spin) {
     if ((spin & 4095u) != 4095u) continue;

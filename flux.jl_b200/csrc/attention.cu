@@ -155,6 +155,7 @@ template <int NC, typename T, bool REDO>
 __global__ void __launch_bounds__(AT)
 attn_fwd_kernel(const T* __restrict__ q, const T* __restrict__ k, const T* __restrict__ v,
                 const uint8_t* __restrict__ mask, float* __restrict__ o, uint16_t* __restrict__ o16, float* __restrict__ lse, AttnDims D) {
+  fb_after_previous();
   constexpr int LD = NC * 64 + 4;
   extern __shared__ float sm[];
   float* Qs = sm;
@@ -257,6 +258,7 @@ attn_fwd_kernel(const T* __restrict__ q, const T* __restrict__ k, const T* __res
 __global__ void __launch_bounds__(AT)
 attn_delta_kernel(const float* __restrict__ o, const float* __restrict__ dout, float* __restrict__ dlt, AttnDims D,
                   int64_t B) {
+  fb_after_previous();
   const int lane = threadIdx.x & 31;
   const int64_t w = (int64_t)blockIdx.x * (AT / 32) + (threadIdx.x >> 5);
   const int64_t total = B * D.Lq * D.H;
@@ -310,6 +312,7 @@ __global__ void __launch_bounds__(AT)
 attn_bwd_dkdv_kernel(const T* __restrict__ q, const T* __restrict__ k, const T* __restrict__ v,
                      const uint8_t* __restrict__ mask, const float* __restrict__ lse, const float* __restrict__ dlt,
                      const T* __restrict__ dout, T* __restrict__ dk, T* __restrict__ dv, AttnDims D) {
+  fb_after_previous();
   constexpr int LD = NC * 64 + 4;
   extern __shared__ float sm[];
   float* Ks = sm;
@@ -380,6 +383,7 @@ __global__ void __launch_bounds__(AT)
 attn_bwd_dq_kernel(const T* __restrict__ q, const T* __restrict__ k, const T* __restrict__ v,
                    const uint8_t* __restrict__ mask, const float* __restrict__ lse, const float* __restrict__ dlt,
                    const T* __restrict__ dout, T* __restrict__ dq, AttnDims D) {
+  fb_after_previous();
   constexpr int LD = NC * 64 + 4;
   extern __shared__ float sm[];
   float* Qs = sm;
@@ -447,6 +451,7 @@ template <int NC>
 __global__ void __launch_bounds__(AT)
 attn_scores_kernel(const float* __restrict__ q, const float* __restrict__ k, const uint8_t* __restrict__ mask,
                    const float* __restrict__ lse, float* __restrict__ alpha, float* __restrict__ extra_dlt, AttnDims D) {
+  fb_after_previous();
   // With extra_dlt the kernel does not write alpha: it adds sum_j alpha_ij * dalpha_ij to extra_dlt[b][h][i] (the
   // share of an alpha cotangent in the softmax backward's row term).
   constexpr int LD = NC * 64 + 4;
@@ -544,10 +549,10 @@ int32_t fb_attn_fwd_redo(fb_ctx* ctx, cudaStream_t stream, int bf16, const void*
   const dim3 grid((unsigned)gx, (unsigned)nheads, (unsigned)batch);
   if (bf16) {
     FB_CUDA(cudaFuncSetAttribute(attn_fwd_kernel<1, uint16_t, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    attn_fwd_kernel<1, uint16_t, true><<<grid, AT, smem, stream>>>((const uint16_t*)q, (const uint16_t*)k, (const uint16_t*)v, nullptr, o, o16, lse, D);
+    fb_launch(attn_fwd_kernel<1, uint16_t, true>, grid, AT, smem, stream, (const uint16_t*)q, (const uint16_t*)k, (const uint16_t*)v, nullptr, o, o16, lse, D);
   } else {
     FB_CUDA(cudaFuncSetAttribute(attn_fwd_kernel<1, float, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    attn_fwd_kernel<1, float, true><<<grid, AT, smem, stream>>>((const float*)q, (const float*)k, (const float*)v, nullptr, o, nullptr, lse, D);
+    fb_launch(attn_fwd_kernel<1, float, true>, grid, AT, smem, stream, (const float*)q, (const float*)k, (const float*)v, nullptr, o, nullptr, lse, D);
   }
   FB_LAUNCH_CHECK();
   return FB_OK;
@@ -565,14 +570,12 @@ static int32_t bwd_redo(fb_ctx* ctx, cudaStream_t stream, const void* q, const v
   };
   if (dk != nullptr) {
     FB_CUDA(cudaFuncSetAttribute(attn_bwd_dkdv_kernel<1, T, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_kv));
-    attn_bwd_dkdv_kernel<1, T, true><<<dim3(blocks(D.Lk), (unsigned)D.H, (unsigned)batch), AT, smem_kv, stream>>>(
-        (const T*)q, (const T*)k, (const T*)v, nullptr, lse, dlt, (const T*)dout, (T*)dk, (T*)dv, D);
+    fb_launch(attn_bwd_dkdv_kernel<1, T, true>, dim3(blocks(D.Lk), (unsigned)D.H, (unsigned)batch), AT, smem_kv, stream, (const T*)q, (const T*)k, (const T*)v, nullptr, lse, dlt, (const T*)dout, (T*)dk, (T*)dv, D);
     FB_LAUNCH_CHECK();
   }
   if (dq != nullptr) {
     FB_CUDA(cudaFuncSetAttribute(attn_bwd_dq_kernel<1, T, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_q));
-    attn_bwd_dq_kernel<1, T, true><<<dim3(blocks(D.Lq), (unsigned)D.H, (unsigned)batch), AT, smem_q, stream>>>(
-        (const T*)q, (const T*)k, (const T*)v, nullptr, lse, dlt, (const T*)dout, (T*)dq, D);
+    fb_launch(attn_bwd_dq_kernel<1, T, true>, dim3(blocks(D.Lq), (unsigned)D.H, (unsigned)batch), AT, smem_q, stream, (const T*)q, (const T*)k, (const T*)v, nullptr, lse, dlt, (const T*)dout, (T*)dq, D);
     FB_LAUNCH_CHECK();
   }
   return FB_OK;
@@ -616,10 +619,10 @@ FB_API int32_t fb_attn_fwd_ex(fb_ctx* ctx, void* stream_, const float* q, const 
   dim3 grid((unsigned)((lq + TS - 1) / TS), (unsigned)nheads, (unsigned)batch);
   if (nc == 1) {
     FB_CUDA(cudaFuncSetAttribute(attn_fwd_kernel<1, float, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    attn_fwd_kernel<1, float, false><<<grid, AT, smem, stream>>>(q, k, v, mask, o, nullptr, lse, D);
+    fb_launch(attn_fwd_kernel<1, float, false>, grid, AT, smem, stream, q, k, v, mask, o, nullptr, lse, D);
   } else {
     FB_CUDA(cudaFuncSetAttribute(attn_fwd_kernel<2, float, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    attn_fwd_kernel<2, float, false><<<grid, AT, smem, stream>>>(q, k, v, mask, o, nullptr, lse, D);
+    fb_launch(attn_fwd_kernel<2, float, false>, grid, AT, smem, stream, q, k, v, mask, o, nullptr, lse, D);
   }
   FB_LAUNCH_CHECK();
   return FB_OK;
@@ -659,7 +662,7 @@ FB_API int32_t fb_attn_bwd_ex(fb_ctx* ctx, void* stream_, const float* q, const 
   float* dlt = (float*)fb_scratch(ctx, stream, (size_t)(batch * nheads * lq) * sizeof(float));
   if (!dlt) return FB_ERR_ALLOC;
   const int64_t warps = batch * lq * nheads;
-  attn_delta_kernel<<<(unsigned)((warps + AT / 32 - 1) / (AT / 32)), AT, 0, stream>>>(o, dout, dlt, D, batch);
+  fb_launch(attn_delta_kernel, (unsigned)((warps + AT / 32 - 1) / (AT / 32)), AT, 0, stream, o, dout, dlt, D, batch);
   FB_LAUNCH_CHECK();
   const int nc = (D.d > 64 || D.dv > 64) ? 2 : 1;
   const int ld = nc * 64 + 4;
@@ -671,10 +674,10 @@ FB_API int32_t fb_attn_bwd_ex(fb_ctx* ctx, void* stream_, const float* q, const 
     dim3 grid_s((unsigned)((lk + TS - 1) / TS), (unsigned)((lq + TS - 1) / TS), (unsigned)(batch * nheads));
     if (ncs == 1) {
       FB_CUDA(cudaFuncSetAttribute(attn_scores_kernel<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_s));
-      attn_scores_kernel<1><<<grid_s, AT, smem_s, stream>>>(q, k, mask, lse, nullptr, dlt, D);
+      fb_launch(attn_scores_kernel<1>, grid_s, AT, smem_s, stream, q, k, mask, lse, nullptr, dlt, D);
     } else {
       FB_CUDA(cudaFuncSetAttribute(attn_scores_kernel<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_s));
-      attn_scores_kernel<2><<<grid_s, AT, smem_s, stream>>>(q, k, mask, lse, nullptr, dlt, D);
+      fb_launch(attn_scores_kernel<2>, grid_s, AT, smem_s, stream, q, k, mask, lse, nullptr, dlt, D);
     }
     FB_LAUNCH_CHECK();
   }
@@ -686,17 +689,17 @@ FB_API int32_t fb_attn_bwd_ex(fb_ctx* ctx, void* stream_, const float* q, const 
     FB_CUDA(cudaFuncSetAttribute(attn_bwd_dkdv_kernel<1, float, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_kv));
     FB_CUDA(cudaFuncSetAttribute(attn_bwd_dq_kernel<1, float, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_q));
     if (!did_kv) {
-      attn_bwd_dkdv_kernel<1, float, false><<<grid_kv, AT, smem_kv, stream>>>(q, k, v, mask, lse, dlt, dout, dk, dv, D);
+      fb_launch(attn_bwd_dkdv_kernel<1, float, false>, grid_kv, AT, smem_kv, stream, q, k, v, mask, lse, dlt, dout, dk, dv, D);
       FB_LAUNCH_CHECK();
     }
     if (did_q) return FB_OK;
-    attn_bwd_dq_kernel<1, float, false><<<grid_q, AT, smem_q, stream>>>(q, k, v, mask, lse, dlt, dout, dq, D);
+    fb_launch(attn_bwd_dq_kernel<1, float, false>, grid_q, AT, smem_q, stream, q, k, v, mask, lse, dlt, dout, dq, D);
   } else {
     FB_CUDA(cudaFuncSetAttribute(attn_bwd_dkdv_kernel<2, float, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_kv));
     FB_CUDA(cudaFuncSetAttribute(attn_bwd_dq_kernel<2, float, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_q));
-    attn_bwd_dkdv_kernel<2, float, false><<<grid_kv, AT, smem_kv, stream>>>(q, k, v, mask, lse, dlt, dout, dk, dv, D);
+    fb_launch(attn_bwd_dkdv_kernel<2, float, false>, grid_kv, AT, smem_kv, stream, q, k, v, mask, lse, dlt, dout, dk, dv, D);
     FB_LAUNCH_CHECK();
-    attn_bwd_dq_kernel<2, float, false><<<grid_q, AT, smem_q, stream>>>(q, k, v, mask, lse, dlt, dout, dq, D);
+    fb_launch(attn_bwd_dq_kernel<2, float, false>, grid_q, AT, smem_q, stream, q, k, v, mask, lse, dlt, dout, dq, D);
   }
   FB_LAUNCH_CHECK();
   return FB_OK;
@@ -727,10 +730,10 @@ FB_API int32_t fb_attn_scores_ex(fb_ctx* ctx, void* stream_, const float* q, con
   dim3 grid((unsigned)((lk + TS - 1) / TS), (unsigned)((lq + TS - 1) / TS), (unsigned)(batch * nheads));
   if (nc == 1) {
     FB_CUDA(cudaFuncSetAttribute(attn_scores_kernel<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    attn_scores_kernel<1><<<grid, AT, smem, stream>>>(q, k, mask, lse, alpha, nullptr, D);
+    fb_launch(attn_scores_kernel<1>, grid, AT, smem, stream, q, k, mask, lse, alpha, nullptr, D);
   } else {
     FB_CUDA(cudaFuncSetAttribute(attn_scores_kernel<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    attn_scores_kernel<2><<<grid, AT, smem, stream>>>(q, k, mask, lse, alpha, nullptr, D);
+    fb_launch(attn_scores_kernel<2>, grid, AT, smem, stream, q, k, mask, lse, alpha, nullptr, D);
   }
   FB_LAUNCH_CHECK();
   return FB_OK;

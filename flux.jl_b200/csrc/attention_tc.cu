@@ -361,6 +361,7 @@ struct SplitArgs {
 
 template <int NP>
 __global__ void __launch_bounds__(256) attn_split_kernel(SplitArgs A) {
+  fb_after_previous();
   __shared__ uint32_t top[8];
   const SplitJob J = A.job[blockIdx.z];
   if ((int)blockIdx.x >= J.tiles) return;
@@ -495,6 +496,7 @@ __global__ void __launch_bounds__(FWD_THREADS, 2)
 attn_fwd_tc_kernel(const void* __restrict__ qmat, const uint8_t* __restrict__ kimg, const uint8_t* __restrict__ vimg,
                    const int16_t* __restrict__ shifts, float* __restrict__ o, uint16_t* __restrict__ o16, float* __restrict__ lse,
                    uint8_t* __restrict__ odd_q, int odd_n, AtcDims D, int32_t* __restrict__ dev_err) {
+  fb_after_previous();
   using cfg = FwdCfg<NP>;
   constexpr int S = cfg::SLOTS;
   enum { B_FULL = 0, B_FREE = S, B_QREADY = 2 * S, B_SFULL, B_PREADY, B_OFULL, B_COUNT };
@@ -762,6 +764,7 @@ __global__ void __launch_bounds__(BWD_THREADS, 1)
 attn_bwd_dq_tc_kernel(const void* __restrict__ q, const void* __restrict__ dout, const uint8_t* __restrict__ kimg,
                       const uint8_t* __restrict__ vimg, const float2* __restrict__ rv, const int16_t* __restrict__ shifts,
                       uint8_t* __restrict__ odd_spread, int odd_n, void* __restrict__ dq, AtcDims D, int32_t* __restrict__ dev_err) {
+  fb_after_previous();
   using cfg = DqCfg<NP>;
   constexpr int S = cfg::SLOTS;
   enum { B_FULL = 0, B_FREE = S, B_QREADY = 2 * S, B_SFULL, B_DSREADY = B_SFULL + 2, B_DONE = B_DSREADY + 2, B_COUNT };
@@ -966,6 +969,7 @@ attn_bwd_dkdv_tc_kernel(const uint8_t* __restrict__ qimg, const uint8_t* __restr
                         const uint8_t* __restrict__ vimg, const float2* __restrict__ rv, const int16_t* __restrict__ shifts,
                         uint8_t* __restrict__ odd_spread, int odd_n, void* __restrict__ dk, void* __restrict__ dv, AtcDims D,
                         int32_t* __restrict__ dev_err) {
+  fb_after_previous();
   using cfg = KvCfg<NP>;
   constexpr int S = cfg::SLOTS;
   enum { B_FULL = 0, B_FREE = S, B_KV = 2 * S, B_SFULL, B_PREADY = B_SFULL + 2, B_DONE = B_PREADY + 2, B_COUNT };
@@ -1235,10 +1239,9 @@ int32_t fwd_impl(fb_ctx* ctx, cudaStream_t stream, const uint8_t* q, const uint8
     A.H = D.H; A.vec = D.vec; A.odd = odd; A.odd_n = odd_n; A.shifts = shifts; A.jobs = 2; A.max_tiles = D.ktiles;
     A.job[0] = {k + el * b0 * D.Lk * D.E, img, D.Lk, D.E, D.d, D.ktiles, SH_QK};
     A.job[1] = {v + el * b0 * D.Lk * D.Ev, img + nb * P.kbytes, D.Lk, D.Ev, D.dv, D.ktiles, SH_V};
-    attn_split_kernel<NP><<<dim3((unsigned)D.ktiles, (unsigned)(nb * D.H), 2), 256, 0, stream>>>(A);
+    fb_launch(attn_split_kernel<NP>, dim3((unsigned)D.ktiles, (unsigned)(nb * D.H), 2), 256, 0, stream, A);
     FB_LAUNCH_CHECK();
-    attn_fwd_tc_kernel<NP><<<dim3((unsigned)(D.qtiles / 2), (unsigned)D.H, (unsigned)nb), FWD_THREADS, FwdCfg<NP>::SMEM, stream>>>(
-        q + el * b0 * D.Lq * D.E, img, img + nb * P.kbytes, shifts, o ? o + b0 * D.Lq * D.Ev : nullptr, o16 ? o16 + b0 * D.Lq * D.Ev : nullptr,
+    fb_launch(attn_fwd_tc_kernel<NP>, dim3((unsigned)(D.qtiles / 2), (unsigned)D.H, (unsigned)nb), FWD_THREADS, FwdCfg<NP>::SMEM, stream, q + el * b0 * D.Lq * D.E, img, img + nb * P.kbytes, shifts, o ? o + b0 * D.Lq * D.Ev : nullptr, o16 ? o16 + b0 * D.Lq * D.Ev : nullptr,
         lse + b0 * D.H * D.Lq, odd + 2 * D.ktiles, odd_n, D, ctx->dev_error);
     FB_LAUNCH_CHECK();
     const int32_t st = fb_attn_fwd_redo(ctx, stream, NP == 1, q + el * b0 * D.Lq * D.E, k + el * b0 * D.Lk * D.E, v + el * b0 * D.Lk * D.Ev,
@@ -1279,13 +1282,11 @@ int32_t bwd_impl(fb_ctx* ctx, cudaStream_t stream, const uint8_t* q, const uint8
     A.o = o + qvoff; A.lse = lse + b0 * D.H * D.Lq; A.rv = rv;
     // (tiles that one operand has and another has not keep no byte)
     if (D.qtiles != D.ktiles) FB_CUDA(cudaMemsetAsync(odd, 0, (size_t)(nb * D.H * odd_n), stream));
-    attn_split_kernel<NP><<<dim3((unsigned)D.max_tiles, (unsigned)(nb * D.H), 4), 256, 0, stream>>>(A);
+    fb_launch(attn_split_kernel<NP>, dim3((unsigned)D.max_tiles, (unsigned)(nb * D.H), 4), 256, 0, stream, A);
     FB_LAUNCH_CHECK();
-    if (do_kv) attn_bwd_dkdv_tc_kernel<NP><<<dim3((unsigned)(D.ktiles / 2), (unsigned)D.H, (unsigned)nb), KvCfg<NP>::THREADS, KvCfg<NP>::SMEM, stream>>>(
-        qi, doi, ki, vi, rv, shifts, odd + 4 * D.max_tiles, odd_n, dk + el * koff, dv + el * kvoff, D, ctx->dev_error);
+    if (do_kv) fb_launch(attn_bwd_dkdv_tc_kernel<NP>, dim3((unsigned)(D.ktiles / 2), (unsigned)D.H, (unsigned)nb), KvCfg<NP>::THREADS, KvCfg<NP>::SMEM, stream, qi, doi, ki, vi, rv, shifts, odd + 4 * D.max_tiles, odd_n, dk + el * koff, dv + el * kvoff, D, ctx->dev_error);
     FB_LAUNCH_CHECK();
-    if (do_q) attn_bwd_dq_tc_kernel<NP><<<dim3((unsigned)(D.qtiles / 2), (unsigned)D.H, (unsigned)nb), BWD_THREADS, DqCfg<NP>::SMEM, stream>>>(
-        q + el * qoff, dout + el * qvoff, ki, vi, rv, shifts, odd + 4 * D.max_tiles, odd_n, dq + el * qoff, D, ctx->dev_error);
+    if (do_q) fb_launch(attn_bwd_dq_tc_kernel<NP>, dim3((unsigned)(D.qtiles / 2), (unsigned)D.H, (unsigned)nb), BWD_THREADS, DqCfg<NP>::SMEM, stream, q + el * qoff, dout + el * qvoff, ki, vi, rv, shifts, odd + 4 * D.max_tiles, odd_n, dq + el * qoff, D, ctx->dev_error);
     FB_LAUNCH_CHECK();
     const int32_t st = fb_attn_bwd_redo(ctx, stream, NP == 1, q + el * qoff, k + el * koff, v + el * kvoff, lse + b0 * D.H * D.Lq, (const float*)rv + 1,
                                         (int64_t)D.qtiles * KT, dout + el * qvoff, do_q ? dq + el * qoff : nullptr, do_kv ? dk + el * koff : nullptr,

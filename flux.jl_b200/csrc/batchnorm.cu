@@ -255,6 +255,7 @@ __global__ void __launch_bounds__(BN_THREADS)
 bn_stats_kernel(const float* __restrict__ x, const Dims g, float eps, float momentum, float* __restrict__ save_mean,
                 float* __restrict__ save_rstd, float* __restrict__ running_mean, float* __restrict__ running_var,
                 int32_t* __restrict__ dev_err) {
+  fb_after_previous();
   constexpr int U = 4;
   __shared__ Exchange ex;
   const int64_t ch = blockIdx.x / (unsigned)g.split;
@@ -306,6 +307,7 @@ __global__ void __launch_bounds__(BN_FWD_THREADS, 1)
 bn_fwd_kernel(const float* __restrict__ x, const float* __restrict__ gamma, const float* __restrict__ beta, float* __restrict__ y,
               const Dims g, int depth, int slab, float eps, float momentum, float* __restrict__ save_mean, float* __restrict__ save_rstd,
               float* __restrict__ running_mean, float* __restrict__ running_var, int act, int32_t* __restrict__ dev_err) {
+  fb_after_previous();
   extern __shared__ __align__(16) float cache[];   // [depth][piece][thread][W]
   __shared__ Exchange ex;
   const int p = (int)(blockIdx.x % (unsigned)g.split);
@@ -383,6 +385,7 @@ __global__ void __launch_bounds__(BN_THREADS)
 bn_apply_kernel(const float* __restrict__ x, const float* __restrict__ gamma, const float* __restrict__ beta,
                 const float* __restrict__ mean, const float* __restrict__ rstd, float eps, float* __restrict__ y, int64_t s, int64_t c,
                 int64_t rows, int tpr, int act) {
+  fb_after_previous();
   constexpr int U = 4;
   __shared__ float3 par[BN_THREADS];   // mean, scale, shift of a chunk of rows: one thread each, not all threads for every row
   const int tx = threadIdx.x & (tpr - 1), ty = threadIdx.x / tpr, nr = BN_THREADS / tpr;
@@ -438,6 +441,7 @@ __global__ void __launch_bounds__(BN_THREADS)
 bn_apply_flat_kernel(const float* __restrict__ x, const float* __restrict__ gamma, const float* __restrict__ beta,
                      const float* __restrict__ mean, const float* __restrict__ rstd, float eps, float* __restrict__ y, const FastDiv fs,
                      const FastDiv fc, uint32_t total, int act) {
+  fb_after_previous();
   constexpr int U = 2;
   for (uint32_t i = blockIdx.x * (U * BN_THREADS) + threadIdx.x; i < (total + 3) / 4; i += gridDim.x * (U * BN_THREADS)) {
     float v[U][4];
@@ -491,6 +495,7 @@ __global__ void __launch_bounds__(BN_THREADS, 5)
 bn_bwd_sums_kernel(const float* __restrict__ x, const float* __restrict__ dy, float dy_scale, const float* __restrict__ gamma,
                    const float* __restrict__ beta, const float* __restrict__ mean, const float* __restrict__ rstd, const Dims g,
                    float* __restrict__ coef, float* __restrict__ dgamma, float* __restrict__ dbeta, int act, int32_t* __restrict__ dev_err) {
+  fb_after_previous();
   constexpr int U = OWN ? 4 : 2;
   __shared__ Exchange ex;
   exchange_init(ex, g.split);
@@ -540,6 +545,7 @@ __global__ void __launch_bounds__(BN_THREADS)
 bn_bwd_apply_kernel(const float* __restrict__ x, const float* __restrict__ dy, const float* __restrict__ gamma,
                     const float* __restrict__ beta, const float* __restrict__ mean, const float* __restrict__ rstd,
                     const float* __restrict__ coef, float* __restrict__ dx, int64_t s, int64_t c, int64_t rows, int tpr, int act) {
+  fb_after_previous();
   constexpr int U = 2;
   const int tx = threadIdx.x & (tpr - 1), ty = threadIdx.x / tpr, nr = BN_THREADS / tpr;
   for (int64_t r = (int64_t)blockIdx.x * nr + ty; r < rows; r += (int64_t)gridDim.x * nr) {
@@ -599,12 +605,13 @@ int32_t bn_launch(K kern, cudaStream_t stream, const Dims& g, int64_t clusters, 
   lc.blockDim = dim3((unsigned)nt, 1, 1);
   lc.dynamicSmemBytes = smem;
   lc.stream = stream;
-  cudaLaunchAttribute attr[1];
+  cudaLaunchAttribute attr[2];
+  attr[1] = fb_early_start();
   attr[0].id = cudaLaunchAttributeClusterDimension;
   attr[0].val.clusterDim.x = (unsigned)g.split;
   attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
   lc.attrs = attr;
-  lc.numAttrs = 1;
+  lc.numAttrs = 2;
   FB_CUDA(cudaLaunchKernelEx(&lc, kern, args...));
   FB_LAUNCH_CHECK();
   return FB_OK;
@@ -633,8 +640,7 @@ int32_t bn_apply(fb_ctx* ctx, cudaStream_t stream, bool vec, const float* x, con
   if (s < 128 && s * c * n <= 0x7fffffff && fb_aligned16(x) && fb_aligned16(y)) {
     const int64_t pieces = (s * c * n + 3) / 4, per = 2 * BN_THREADS, blocks = (pieces + per - 1) / per, cap = (int64_t)ctx->sm_count * 16;
     fb_act_kind(act, [&](auto k) {
-      bn_apply_flat_kernel<VAR, k.value><<<(unsigned)(blocks < cap ? blocks : cap), BN_THREADS, 0, stream>>>(
-          x, gamma, beta, mean, rstd, eps, y, fast_div((uint32_t)s), fast_div((uint32_t)c), (uint32_t)(s * c * n), act);
+      fb_launch(bn_apply_flat_kernel<VAR, k.value>, (unsigned)(blocks < cap ? blocks : cap), BN_THREADS, 0, stream, x, gamma, beta, mean, rstd, eps, y, fast_div((uint32_t)s), fast_div((uint32_t)c), (uint32_t)(s * c * n), act);
     });
     FB_LAUNCH_CHECK();
     return FB_OK;
@@ -642,7 +648,7 @@ int32_t bn_apply(fb_ctx* ctx, cudaStream_t stream, bool vec, const float* x, con
   const int tpr = bn_tpr(vec ? s / 4 : s, BN_THREADS);
   bn_kind(vec, act, [&](auto W, auto k) {
     const int64_t chunk = bn_chunk(BN_THREADS / tpr), blocks = (c * n + chunk - 1) / chunk, cap = (int64_t)ctx->sm_count * 32;
-    bn_apply_kernel<W.value, VAR, k.value><<<(unsigned)(blocks < cap ? blocks : cap), BN_THREADS, 0, stream>>>(x, gamma, beta, mean, rstd, eps, y, s, c, c * n, tpr, act);
+    fb_launch(bn_apply_kernel<W.value, VAR, k.value>, (unsigned)(blocks < cap ? blocks : cap), BN_THREADS, 0, stream, x, gamma, beta, mean, rstd, eps, y, s, c, c * n, tpr, act);
   });
   FB_LAUNCH_CHECK();
   return FB_OK;
@@ -766,7 +772,7 @@ FB_API int32_t fb_batchnorm_bwd(fb_ctx* ctx, void* stream_, const float* x, cons
   if (st != FB_OK) return st;
   const int tpr = bn_tpr(vec ? s / 4 : s, BN_THREADS);
   bn_kind(vec, act, [&](auto w, auto k) {
-    bn_bwd_apply_kernel<w.value, k.value><<<bn_row_grid(ctx, c * n, tpr), BN_THREADS, 0, stream>>>(x, dy, gamma, beta, save_mean, save_rstd, coef, dx, s, c, c * n, tpr, act);
+    fb_launch(bn_bwd_apply_kernel<w.value, k.value>, bn_row_grid(ctx, c * n, tpr), BN_THREADS, 0, stream, x, dy, gamma, beta, save_mean, save_rstd, coef, dx, s, c, c * n, tpr, act);
   });
   FB_LAUNCH_CHECK();
   return FB_OK;

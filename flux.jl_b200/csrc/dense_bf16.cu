@@ -43,6 +43,7 @@ template <int KIND>
 __global__ void __launch_bounds__(256)
 act_bwd_colsum_bf16_kernel(int act, const uint16_t* __restrict__ dy, const uint16_t* __restrict__ y, const uint16_t* __restrict__ z,
                            uint16_t* __restrict__ delta, float* __restrict__ part, int64_t rows, int64_t cols, int64_t rpb) {
+  fb_after_previous();
   __shared__ float sh[4][64];
   const int tx = threadIdx.x & 63, ty = threadIdx.x >> 6;
   const int64_t col = (int64_t)blockIdx.x * 64 + tx;
@@ -69,6 +70,7 @@ template <int KIND>
 __global__ void __launch_bounds__(256)
 act_bwd_colsum_bf16x8_kernel(int act, const uint16_t* __restrict__ dy, const uint16_t* __restrict__ y, const uint16_t* __restrict__ z,
                              uint16_t* __restrict__ delta, float* __restrict__ part, int64_t rows, int64_t cols, int64_t rpb) {
+  fb_after_previous();
   __shared__ float4 sh[2][32][16];       // [row][half of eight columns][piece]: no bank conflicts on either side
   const int lx = threadIdx.x & 7, ly = threadIdx.x >> 3;
   const int64_t col = (int64_t)blockIdx.x * 64 + lx * 8;
@@ -125,6 +127,8 @@ act_bwd_colsum_bf16x8_kernel(int act, const uint16_t* __restrict__ dy, const uin
 
 // the groups' sums in turn: 32 columns a block, 64 groups at a time on their way through shared memory
 __global__ void __launch_bounds__(256) colsum_parts_bf16_kernel(const float* __restrict__ part, uint16_t* __restrict__ out, int64_t groups, int64_t cols) {
+  fb_after_previous();
+  fb_let_next_start();
   __shared__ float sh[64][33];
   const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
   const int64_t c = (int64_t)blockIdx.x * 32 + tx;
@@ -146,6 +150,7 @@ __global__ void __launch_bounds__(256) colsum_parts_bf16_kernel(const float* __r
 }
 
 __global__ void __launch_bounds__(256) axpy_bf16_kernel(float alpha, const uint16_t* __restrict__ x, uint16_t* __restrict__ y, int64_t count) {
+  fb_after_previous();
   for (int64_t i = (int64_t)blockIdx.x * 256 + threadIdx.x; i < count; i += (int64_t)gridDim.x * 256)
     y[i] = f2bf(fmaf(alpha, bf2f(x[i]), bf2f(y[i])));
 }
@@ -159,7 +164,7 @@ FB_API int32_t fb_axpy_bf16(fb_ctx* ctx, void* stream, float alpha, const uint16
   FB_REQUIRE(x && y, FB_ERR_INVALID_ARG, "fb_axpy_bf16: NULL pointer");
   int64_t blocks = (count + 255) / 256;
   if (blocks > (int64_t)ctx->sm_count * 16) blocks = (int64_t)ctx->sm_count * 16;
-  axpy_bf16_kernel<<<(unsigned)blocks, 256, 0, (cudaStream_t)stream>>>(alpha, x, y, count);
+  fb_launch(axpy_bf16_kernel, (unsigned)blocks, 256, 0, (cudaStream_t)stream, alpha, x, y, count);
   FB_LAUNCH_CHECK();
   return FB_OK;
 }
@@ -231,12 +236,12 @@ FB_API int32_t fb_dense_bwd_bf16(fb_ctx* ctx, void* stream_, int32_t act, const 
     }
     fb_act_kind(act, [&](auto k) {
       const dim3 grid((unsigned)gx, (unsigned)gy);
-      if (vec && rpb >= 32) act_bwd_colsum_bf16x8_kernel<k.value><<<grid, 256, 0, stream>>>(act, dy, y, z, delta, part, n, out_dim, rpb);
-      else act_bwd_colsum_bf16_kernel<k.value><<<grid, 256, 0, stream>>>(act, dy, y, z, delta, part, n, out_dim, rpb);
+      if (vec && rpb >= 32) fb_launch(act_bwd_colsum_bf16x8_kernel<k.value>, grid, 256, 0, stream, act, dy, y, z, delta, part, n, out_dim, rpb);
+      else fb_launch(act_bwd_colsum_bf16_kernel<k.value>, grid, 256, 0, stream, act, dy, y, z, delta, part, n, out_dim, rpb);
     });
     FB_LAUNCH_CHECK();
     if (db != nullptr) {
-      colsum_parts_bf16_kernel<<<(unsigned)((out_dim + 31) / 32), 256, 0, stream>>>(part, db, gy, out_dim);
+      fb_launch(colsum_parts_bf16_kernel, (unsigned)((out_dim + 31) / 32), 256, 0, stream, part, db, gy, out_dim);
       FB_LAUNCH_CHECK();
     }
   }

@@ -46,6 +46,7 @@ __device__ __forceinline__ void dc_copy4(void* dst, const void* src, int bytes) 
 // NB: columns of a cluster
 template <int NB>
 __global__ void __launch_bounds__(DC_THREADS, 1) dense_chain_kernel(const __grid_constant__ DcArgs A) {
+  fb_after_previous();
   extern __shared__ __align__(16) uint8_t dc_smem[];
   __shared__ float bias[DC_MAX_LAYERS][DC_MAX_SLICE];               // this CTA's slices
   __shared__ __align__(16) float sent[DC_WIDTH / DC_CTAS];
@@ -188,7 +189,8 @@ __global__ void __launch_bounds__(DC_THREADS, 1) dense_chain_kernel(const __grid
 template <int NB>
 int32_t launch(fb_ctx* ctx, cudaStream_t stream, const DcArgs& A) {
   cudaLaunchConfig_t lc = {};
-  cudaLaunchAttribute at[1];
+  cudaLaunchAttribute at[2];
+  at[1] = fb_early_start();
   at[0].id = cudaLaunchAttributeClusterDimension;
   at[0].val.clusterDim.x = DC_CTAS;
   at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
@@ -197,7 +199,7 @@ int32_t launch(fb_ctx* ctx, cudaStream_t stream, const DcArgs& A) {
   lc.dynamicSmemBytes = DC_SMEM;
   lc.stream = stream;
   lc.attrs = at;
-  lc.numAttrs = 1;
+  lc.numAttrs = 2;
   FB_CUDA(fb_allow_smem(dense_chain_kernel<NB>, DC_SMEM));
   FB_CUDA(cudaFuncSetAttribute(dense_chain_kernel<NB>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
   FB_CUDA(cudaLaunchKernelEx(&lc, dense_chain_kernel<NB>, A));

@@ -18,6 +18,7 @@ unsigned ew_grid(const fb_ctx* ctx, int64_t items) {
 
 __global__ void __launch_bounds__(EW_THREADS)
 scale_kernel(const float* __restrict__ x, float alpha, float* __restrict__ y, int64_t count, int vec) {
+  fb_after_previous();
   const int64_t tid = (int64_t)blockIdx.x * EW_THREADS + threadIdx.x, stride = (int64_t)gridDim.x * EW_THREADS;
   if (vec) {
     const float4* x4 = (const float4*)x;
@@ -35,6 +36,7 @@ scale_kernel(const float* __restrict__ x, float alpha, float* __restrict__ y, in
 
 __global__ void __launch_bounds__(EW_THREADS)
 axpy_kernel(float alpha, const float* __restrict__ x, float* __restrict__ y, int64_t count, int vec) {
+  fb_after_previous();
   const int64_t tid = (int64_t)blockIdx.x * EW_THREADS + threadIdx.x, stride = (int64_t)gridDim.x * EW_THREADS;
   if (vec) {
     const float4* x4 = (const float4*)x;
@@ -53,6 +55,7 @@ axpy_kernel(float alpha, const float* __restrict__ x, float* __restrict__ y, int
 
 __global__ void __launch_bounds__(EW_THREADS)
 cast_f32_bf16_kernel(const float* __restrict__ x, uint16_t* __restrict__ y, int64_t count, int vec) {
+  fb_after_previous();
   const int64_t tid = (int64_t)blockIdx.x * EW_THREADS + threadIdx.x, stride = (int64_t)gridDim.x * EW_THREADS;
   // eight values a thread where both arrays allow it (16.8 M values: 21 -> 14.7 us, 2 M values 9.2 -> 4.7)
   int64_t done = 0;
@@ -72,6 +75,7 @@ cast_f32_bf16_kernel(const float* __restrict__ x, uint16_t* __restrict__ y, int6
 
 __global__ void __launch_bounds__(EW_THREADS)
 cast_bf16_f32_kernel(const uint16_t* __restrict__ x, float* __restrict__ y, int64_t count, int vec) {
+  fb_after_previous();
   const int64_t tid = (int64_t)blockIdx.x * EW_THREADS + threadIdx.x, stride = (int64_t)gridDim.x * EW_THREADS;
   int64_t done = 0;
   if (vec) {
@@ -88,6 +92,7 @@ cast_bf16_f32_kernel(const uint16_t* __restrict__ x, float* __restrict__ y, int6
 // ------------------------------------------------------------------------------- sum of squares ---
 __global__ void __launch_bounds__(EW_THREADS)
 sumsq_partial_kernel(const float* __restrict__ x, int64_t count, float* __restrict__ part, int vec, int square) {
+  fb_after_previous();
   __shared__ float sh[32];
   const int64_t tid = (int64_t)blockIdx.x * EW_THREADS + threadIdx.x, stride = (int64_t)gridDim.x * EW_THREADS;
   float s = 0.0f;
@@ -108,6 +113,8 @@ sumsq_partial_kernel(const float* __restrict__ x, int64_t count, float* __restri
 // out[0] = scale * sum(part[0..m))   (one block; fixed order -> run-to-run deterministic)
 __global__ void __launch_bounds__(1024)
 final_sum_kernel(const float* __restrict__ part, int64_t m, float scale, float* __restrict__ out) {
+  fb_after_previous();
+  fb_let_next_start();
   __shared__ float sh[32];
   float s = 0.0f;
   for (int64_t i = threadIdx.x; i < m; i += 1024) s += part[i];
@@ -121,6 +128,8 @@ template <bool LABELS>
 __global__ void __launch_bounds__(128)
 xent_kernel(const float* __restrict__ yhat, const int32_t* __restrict__ labels, const float* __restrict__ ydense,
             float* __restrict__ loss_part, float* __restrict__ dyhat, int64_t c, int64_t n, float gscale) {
+  fb_after_previous();
+  fb_let_next_start();
   const int lane = threadIdx.x & 31;
   const int64_t row = (int64_t)blockIdx.x * 4 + (threadIdx.x >> 5);
   if (row >= n) return;
@@ -184,6 +193,7 @@ template <int ADAM_THREADS, int MIN_BLOCKS>
 __global__ void __launch_bounds__(ADAM_THREADS, MIN_BLOCKS)
 adam_kernel(const __grid_constant__ AdamTable tab, float eta, float beta1, float beta2, float eps, float inv_c1,
             float inv_c2, float grad_scale, const float* __restrict__ bt_dev, const float* __restrict__ guard) {
+  fb_after_previous();
   // device-resident step state (used when the step is replayed from a CUDA graph): the running beta powers
   // and an optional guard scalar (the loss) whose non-finite value skips the update
   if (guard != nullptr && !isfinite(__ldg(guard))) return;
@@ -254,6 +264,7 @@ __device__ __forceinline__ uint16_t adam_round(float w) {
 __global__ void __launch_bounds__(256)
 adam_bf16_kernel(const __grid_constant__ AdamLowTable tab, float eta, float beta1, float beta2, float eps, float inv_c1, float inv_c2,
                  float grad_scale) {
+  fb_after_previous();
   int t = 0;
   while (t + 1 < tab.t.ntensors && (int)blockIdx.x >= tab.t.block_start[t + 1]) ++t;
   const int64_t begin = (int64_t)(blockIdx.x - tab.t.block_start[t]) * ADAM_CHUNK;
@@ -309,6 +320,8 @@ __global__ void __launch_bounds__(256)
 act_bwd_colsum_kernel(int act, const float* __restrict__ dy, const float* __restrict__ y, const float* __restrict__ z,
                       float* __restrict__ delta, float* __restrict__ part, int64_t rows, int64_t cols,
                       int64_t rows_per_block) {
+  fb_after_previous();
+  fb_let_next_start();
   constexpr int U = CL ? 4 : 1;
   __shared__ float sh[8][32 * VEC + 1];
   const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
@@ -429,11 +442,11 @@ int32_t fb_act_bwd_colsum(fb_ctx* ctx, cudaStream_t stream, int act, const float
     part = (float*)fb_scratch(ctx, stream, (size_t)(gy * cols) * sizeof(float));
     if (!part) return FB_ERR_ALLOC;
   }
-  if (vec) act_bwd_colsum_kernel<4, false><<<grid, 256, 0, stream>>>(act, dy, y, z, dout, part, rows, cols, rpb);
-  else act_bwd_colsum_kernel<1, false><<<grid, 256, 0, stream>>>(act, dy, y, z, dout, part, rows, cols, rpb);
+  if (vec) fb_launch(act_bwd_colsum_kernel<4, false>, grid, 256, 0, stream, act, dy, y, z, dout, part, rows, cols, rpb);
+  else fb_launch(act_bwd_colsum_kernel<1, false>, grid, 256, 0, stream, act, dy, y, z, dout, part, rows, cols, rpb);
   FB_LAUNCH_CHECK();
   if (db != nullptr) {
-    fb_colreduce2_kernel<<<(unsigned)((cols + 31) / 32), 256, 0, stream>>>(part, nullptr, db, nullptr, gy, cols);
+    fb_launch(fb_colreduce2_kernel, (unsigned)((cols + 31) / 32), 256, 0, stream, part, nullptr, db, nullptr, gy, cols);
     FB_LAUNCH_CHECK();
   }
   return FB_OK;
@@ -445,12 +458,13 @@ FB_API int32_t fb_scale(fb_ctx* ctx, void* stream, const float* x, float alpha, 
   if (count == 0) return FB_OK;
   FB_REQUIRE(x && y, FB_ERR_INVALID_ARG, "fb_scale: NULL pointer");
   const int vec = fb_aligned16(x) && fb_aligned16(y);
-  scale_kernel<<<ew_grid(ctx, vec ? (count + 3) / 4 : count), EW_THREADS, 0, (cudaStream_t)stream>>>(x, alpha, y, count, vec);
+  fb_launch(scale_kernel, ew_grid(ctx, vec ? (count + 3) / 4 : count), EW_THREADS, 0, (cudaStream_t)stream, x, alpha, y, count, vec);
   FB_LAUNCH_CHECK();
   return FB_OK;
 }
 
 __global__ void __launch_bounds__(256) fill_kernel(float* __restrict__ x, float value, int64_t count) {
+  fb_after_previous();
   for (int64_t i = (int64_t)blockIdx.x * 256 + threadIdx.x; i < count; i += (int64_t)gridDim.x * 256) x[i] = value;
 }
 
@@ -461,7 +475,7 @@ FB_API int32_t fb_fill(fb_ctx* ctx, void* stream, float* x, float value, int64_t
   FB_REQUIRE(x, FB_ERR_INVALID_ARG, "fb_fill: NULL pointer");
   int64_t blocks = (count + 255) / 256;
   if (blocks > (int64_t)ctx->sm_count * 32) blocks = (int64_t)ctx->sm_count * 32;
-  fill_kernel<<<(unsigned)blocks, 256, 0, (cudaStream_t)stream>>>(x, value, count);
+  fb_launch(fill_kernel, (unsigned)blocks, 256, 0, (cudaStream_t)stream, x, value, count);
   FB_LAUNCH_CHECK();
   return FB_OK;
 }
@@ -469,6 +483,7 @@ FB_API int32_t fb_fill(fb_ctx* ctx, void* stream, float* x, float value, int64_t
 // One thread stores the GPU's nanosecond timer: a stream-ordered time mark that also works inside a captured graph
 // (where events cannot be timed).
 __global__ void timestamp_kernel(uint64_t* out) {
+  fb_after_previous();
   uint64_t t;
   asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
   *out = t;
@@ -484,7 +499,7 @@ int32_t fb_side_kernels_prepare_elementwise() {
 FB_API int32_t fb_timestamp(fb_ctx* ctx, void* stream, uint64_t* out_dev) {
   FB_CHECK_CTX(ctx);
   FB_REQUIRE(out_dev, FB_ERR_INVALID_ARG, "fb_timestamp: NULL pointer");
-  timestamp_kernel<<<1, 1, 0, (cudaStream_t)stream>>>(out_dev);
+  fb_launch(timestamp_kernel, 1, 1, 0, (cudaStream_t)stream, out_dev);
   FB_LAUNCH_CHECK();
   return FB_OK;
 }
@@ -495,13 +510,14 @@ FB_API int32_t fb_axpy(fb_ctx* ctx, void* stream, float alpha, const float* x, f
   if (count == 0) return FB_OK;
   FB_REQUIRE(x && y, FB_ERR_INVALID_ARG, "fb_axpy: NULL pointer");
   const int vec = fb_aligned16(x) && fb_aligned16(y);
-  axpy_kernel<<<ew_grid(ctx, vec ? (count + 3) / 4 : count), EW_THREADS, 0, (cudaStream_t)stream>>>(alpha, x, y, count, vec);
+  fb_launch(axpy_kernel, ew_grid(ctx, vec ? (count + 3) / 4 : count), EW_THREADS, 0, (cudaStream_t)stream, alpha, x, y, count, vec);
   FB_LAUNCH_CHECK();
   return FB_OK;
 }
 
 __global__ void __launch_bounds__(EW_THREADS)
 round_bf16_kernel(const float* __restrict__ x, float* __restrict__ y, int64_t count) {
+  fb_after_previous();
   const int64_t tid = (int64_t)blockIdx.x * blockDim.x + threadIdx.x, stride = (int64_t)gridDim.x * blockDim.x;
   for (int64_t i = tid; i < count; i += stride) y[i] = __uint_as_float((uint32_t)fb_bf16_bits(x[i]) << 16);
 }
@@ -511,7 +527,7 @@ FB_API int32_t fb_round_bf16(fb_ctx* ctx, void* stream, const float* x, float* y
   FB_REQUIRE(count >= 0, FB_ERR_INVALID_ARG, "fb_round_bf16: negative count");
   if (count == 0) return FB_OK;
   FB_REQUIRE(x && y, FB_ERR_INVALID_ARG, "fb_round_bf16: NULL pointer");
-  round_bf16_kernel<<<ew_grid(ctx, count), EW_THREADS, 0, (cudaStream_t)stream>>>(x, y, count);
+  fb_launch(round_bf16_kernel, ew_grid(ctx, count), EW_THREADS, 0, (cudaStream_t)stream, x, y, count);
   FB_LAUNCH_CHECK();
   return FB_OK;
 }
@@ -520,6 +536,7 @@ FB_API int32_t fb_round_bf16(fb_ctx* ctx, void* stream, const float* x, float* y
 template <bool AB, bool BB>
 __global__ void __launch_bounds__(EW_THREADS)
 add_kernel(const void* a, const void* b, float* out, int64_t count, int vec) {
+  fb_after_previous();
   const int64_t tid = (int64_t)blockIdx.x * EW_THREADS + threadIdx.x, stride = (int64_t)gridDim.x * EW_THREADS;
   auto four = [](const void* p, bool low, int64_t i, float (&v)[4]) {
     if (low) {
@@ -555,10 +572,10 @@ FB_API int32_t fb_add_mixed(fb_ctx* ctx, void* stream_, const void* a, int32_t a
   cudaStream_t stream = (cudaStream_t)stream_;
   const int vec = fb_aligned16(a) && fb_aligned16(b) && fb_aligned16(out);
   const unsigned grid = ew_grid(ctx, vec ? (count + 3) / 4 : count);
-  if (a_bf16 && b_bf16) add_kernel<true, true><<<grid, EW_THREADS, 0, stream>>>(a, b, out, count, vec);
-  else if (a_bf16) add_kernel<true, false><<<grid, EW_THREADS, 0, stream>>>(a, b, out, count, vec);
-  else if (b_bf16) add_kernel<false, true><<<grid, EW_THREADS, 0, stream>>>(a, b, out, count, vec);
-  else add_kernel<false, false><<<grid, EW_THREADS, 0, stream>>>(a, b, out, count, vec);
+  if (a_bf16 && b_bf16) fb_launch(add_kernel<true, true>, grid, EW_THREADS, 0, stream, a, b, out, count, vec);
+  else if (a_bf16) fb_launch(add_kernel<true, false>, grid, EW_THREADS, 0, stream, a, b, out, count, vec);
+  else if (b_bf16) fb_launch(add_kernel<false, true>, grid, EW_THREADS, 0, stream, a, b, out, count, vec);
+  else fb_launch(add_kernel<false, false>, grid, EW_THREADS, 0, stream, a, b, out, count, vec);
   FB_LAUNCH_CHECK();
   return FB_OK;
 }
@@ -569,7 +586,7 @@ FB_API int32_t fb_cast_f32_bf16(fb_ctx* ctx, void* stream, const float* x, uint1
   if (count == 0) return FB_OK;
   FB_REQUIRE(x && y, FB_ERR_INVALID_ARG, "fb_cast_f32_bf16: NULL pointer");
   const int vec = fb_aligned16(x) && fb_aligned16(y);
-  cast_f32_bf16_kernel<<<ew_grid(ctx, vec ? (count + 7) / 8 : count), EW_THREADS, 0, (cudaStream_t)stream>>>(x, y, count, vec);
+  fb_launch(cast_f32_bf16_kernel, ew_grid(ctx, vec ? (count + 7) / 8 : count), EW_THREADS, 0, (cudaStream_t)stream, x, y, count, vec);
   FB_LAUNCH_CHECK();
   return FB_OK;
 }
@@ -580,7 +597,7 @@ FB_API int32_t fb_cast_bf16_f32(fb_ctx* ctx, void* stream, const uint16_t* x, fl
   if (count == 0) return FB_OK;
   FB_REQUIRE(x && y, FB_ERR_INVALID_ARG, "fb_cast_bf16_f32: NULL pointer");
   const int vec = fb_aligned16(x) && fb_aligned16(y);
-  cast_bf16_f32_kernel<<<ew_grid(ctx, vec ? (count + 7) / 8 : count), EW_THREADS, 0, (cudaStream_t)stream>>>(x, y, count, vec);
+  fb_launch(cast_bf16_f32_kernel, ew_grid(ctx, vec ? (count + 7) / 8 : count), EW_THREADS, 0, (cudaStream_t)stream, x, y, count, vec);
   FB_LAUNCH_CHECK();
   return FB_OK;
 }
@@ -600,9 +617,9 @@ static int32_t sum_common(fb_ctx* ctx, cudaStream_t stream, const float* x, int6
   if (blocks < 1) blocks = 1;
   float* part = (float*)fb_scratch(ctx, stream, (size_t)blocks * sizeof(float));
   if (!part) return FB_ERR_ALLOC;
-  sumsq_partial_kernel<<<(unsigned)blocks, EW_THREADS, 0, stream>>>(x, count, part, vec, square);
+  fb_launch(sumsq_partial_kernel, (unsigned)blocks, EW_THREADS, 0, stream, x, count, part, vec, square);
   FB_LAUNCH_CHECK();
-  final_sum_kernel<<<1, 1024, 0, stream>>>(part, blocks, 1.0f, out);
+  fb_launch(final_sum_kernel, 1, 1024, 0, stream, part, blocks, 1.0f, out);
   FB_LAUNCH_CHECK();
   return FB_OK;
 }
@@ -625,10 +642,10 @@ static int32_t xent_common(fb_ctx* ctx, cudaStream_t stream, const float* yhat, 
   if (!part) return FB_ERR_ALLOC;
   const unsigned grid = (unsigned)((n + 3) / 4);
   const float gscale = dloss / (float)n;
-  if (labels) xent_kernel<true><<<grid, 128, 0, stream>>>(yhat, labels, nullptr, part, dyhat, c, n, gscale);
-  else xent_kernel<false><<<grid, 128, 0, stream>>>(yhat, nullptr, y, part, dyhat, c, n, gscale);
+  if (labels) fb_launch(xent_kernel<true>, grid, 128, 0, stream, yhat, labels, nullptr, part, dyhat, c, n, gscale);
+  else fb_launch(xent_kernel<false>, grid, 128, 0, stream, yhat, nullptr, y, part, dyhat, c, n, gscale);
   FB_LAUNCH_CHECK();
-  final_sum_kernel<<<1, 1024, 0, stream>>>(part, n, 1.0f / (float)n, loss);
+  fb_launch(final_sum_kernel, 1, 1024, 0, stream, part, n, 1.0f / (float)n, loss);
   FB_LAUNCH_CHECK();
   return FB_OK;
 }
@@ -691,7 +708,7 @@ FB_API int32_t fb_adam_step_bf16(fb_ctx* ctx, void* stream_, int32_t ntensors, u
     if (k == 0) continue;
     tab.t.block_start[k] = blocks;
     tab.t.ntensors = k;
-    adam_bf16_kernel<<<(unsigned)blocks, 256, 0, (cudaStream_t)stream_>>>(tab, eta, beta1, beta2, eps, inv_c1, inv_c2, grad_scale);
+    fb_launch(adam_bf16_kernel, (unsigned)blocks, 256, 0, (cudaStream_t)stream_, tab, eta, beta1, beta2, eps, inv_c1, inv_c2, grad_scale);
     FB_LAUNCH_CHECK();
   }
   return FB_OK;
@@ -716,6 +733,8 @@ FB_API int32_t fb_adam_block_dev(fb_ctx* ctx, void* stream_, float* w, const flo
 }
 
 __global__ void adam_advance_kernel(float* __restrict__ bt, float beta1, float beta2, const float* __restrict__ guard) {
+  fb_after_previous();
+  fb_let_next_start();
   if (guard != nullptr && !isfinite(*guard)) return;
   bt[0] *= beta1;
   bt[1] *= beta2;
@@ -724,7 +743,7 @@ __global__ void adam_advance_kernel(float* __restrict__ bt, float beta1, float b
 FB_API int32_t fb_adam_advance(fb_ctx* ctx, void* stream_, float* bt_dev, float beta1, float beta2, const float* guard_dev) {
   FB_CHECK_CTX(ctx);
   FB_REQUIRE(bt_dev != nullptr, FB_ERR_INVALID_ARG, "fb_adam_advance: bt_dev is NULL");
-  adam_advance_kernel<<<1, 1, 0, (cudaStream_t)stream_>>>(bt_dev, beta1, beta2, guard_dev);
+  fb_launch(adam_advance_kernel, 1, 1, 0, (cudaStream_t)stream_, bt_dev, beta1, beta2, guard_dev);
   FB_LAUNCH_CHECK();
   return FB_OK;
 }
@@ -766,7 +785,7 @@ static int32_t adam_common(fb_ctx* ctx, cudaStream_t stream, int32_t ntensors, f
       adam_kernel<ADAM_SIDE_THREADS, 2048 / ADAM_SIDE_THREADS><<<(unsigned)blocks, ADAM_SIDE_THREADS, 0, stream>>>(
           tab, eta, beta1, beta2, eps, inv_c1, inv_c2, grad_scale, bt_dev, guard);
     else
-      adam_kernel<EW_THREADS, 1><<<(unsigned)blocks, EW_THREADS, 0, stream>>>(tab, eta, beta1, beta2, eps, inv_c1, inv_c2, grad_scale,
+      fb_launch(adam_kernel<EW_THREADS, 1>, (unsigned)blocks, EW_THREADS, 0, stream, tab, eta, beta1, beta2, eps, inv_c1, inv_c2, grad_scale,
                                                                               bt_dev, guard);
     FB_LAUNCH_CHECK();
   }

@@ -62,6 +62,7 @@ __global__ void __launch_bounds__(HCfg<BN, PAIR>::NUM_THREADS, 1)
 gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB, void* __restrict__ Cv,
                  int64_t ldc, uint16_t* __restrict__ Z, const uint16_t* __restrict__ bias_n, int M, int N, int K, int act,
                  int accumulate, int out_f32, int32_t* __restrict__ dev_err, int a3d, int b3d, int num_tiles, int tiles_n, int nsplit) {
+  fb_after_previous();
   using cfg = HCfg<BN, PAIR>;
   constexpr int STAGES = cfg::STAGES;
   extern __shared__ uint8_t smem_raw[];
@@ -504,13 +505,14 @@ int32_t launch_bf16(fb_ctx* ctx, cudaStream_t stream, const fb_gemm_bf16_args& a
   lc.blockDim = dim3(cfg::NUM_THREADS, 1, 1);
   lc.dynamicSmemBytes = cfg::SMEM_BYTES;
   lc.stream = stream;
-  cudaLaunchAttribute attr[1];
+  cudaLaunchAttribute attr[2];
+  attr[1] = fb_early_start();
   attr[0].id = cudaLaunchAttributeClusterDimension;
   attr[0].val.clusterDim.x = (PAIR ? 2 : 1) * ksplit;
   attr[0].val.clusterDim.y = 1;
   attr[0].val.clusterDim.z = 1;
   lc.attrs = attr;
-  lc.numAttrs = 1;
+  lc.numAttrs = 2;
   FB_CUDA(cudaLaunchKernelEx(&lc, kern, tmA, tmB, a.C, a.ldc, a.Z, a.bias_n, (int)a.M, (int)a.N, (int)a.K, a.act, a.accumulate,
                              a.out_f32, ctx->dev_error, a3d, b3d, (int)num_tiles, tiles_n, ksplit));
   FB_LAUNCH_CHECK();

@@ -191,6 +191,7 @@ template <bool PAIR, bool SPLIT>
 __global__ void __launch_bounds__(NUM_THREADS, 1)
 gemm_planes_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB, const __grid_constant__ Out out, int K,
                    int32_t* __restrict__ dev_err, int a_mn, int b_mn, const Sched sch) {
+  fb_after_previous();
   constexpr int BN = PAIR ? 256 : 128;
   constexpr int TMEM_COLS = 2 * BN;                 // two accumulator buffers
   constexpr int RANKS = PAIR ? 2 : 1;
@@ -671,13 +672,14 @@ int32_t launch(fb_ctx* ctx, cudaStream_t stream, const fb_gemm_args& a, const Pl
   lc.blockDim = dim3(NUM_THREADS, 1, 1);
   lc.dynamicSmemBytes = SMEM_BYTES;
   lc.stream = stream;
-  cudaLaunchAttribute attr[1];
+  cudaLaunchAttribute attr[2];
+  attr[1] = fb_early_start();
   attr[0].id = cudaLaunchAttributeClusterDimension;
   attr[0].val.clusterDim.x = RANKS * plan.ksplit;
   attr[0].val.clusterDim.y = 1;
   attr[0].val.clusterDim.z = 1;
   lc.attrs = attr;
-  lc.numAttrs = 1;
+  lc.numAttrs = 2;
   FB_CUDA(cudaLaunchKernelEx(&lc, kern, tmA, tmB, out, (int)a.K, ctx->dev_error, a.a_mn_major, a.b_mn_major, sch));
   FB_LAUNCH_CHECK();
   return fb_gemm_tc_launch(ctx, stream, a, 3, planes.over);

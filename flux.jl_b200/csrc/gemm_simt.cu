@@ -87,6 +87,8 @@ __global__ void __launch_bounds__(THREADS)
 gemm_fma_kernel(const float* __restrict__ A, int64_t lda, const float* __restrict__ B, int64_t ldb, float* __restrict__ C, int64_t ldc,
                 float* __restrict__ Z, const float* __restrict__ bias_n, const float* __restrict__ bias_m, int64_t M, int64_t N,
                 int64_t K, int act, int accumulate, int splits, int64_t kper, int64_t tiles_n) {
+  fb_after_previous();
+  fb_let_next_start();
   constexpr int TR = BM / TM, TC = BN / TN, KG = THREADS / (TR * TC), KPG = BK / KG;
   static_assert(KG >= 1 && KPG >= 4, "a group needs four k values per stage");
   constexpr int AS = A_MN ? BK * (BM + 4) : BM * (BK + 4), BS = B_MN ? BK * (BN + 4) : BN * (BK + 4);
@@ -240,12 +242,13 @@ int32_t launch_fma_variant(fb_ctx* ctx, cudaStream_t stream, const fb_gemm_args&
   // gives every CTA an SM of its own.
   lc.dynamicSmemBytes = splits > 1 ? 118 * 1024 : SMEM;
   lc.stream = stream;
-  cudaLaunchAttribute attr[1];
+  cudaLaunchAttribute attr[2];
+  attr[1] = fb_early_start();
   attr[0].id = cudaLaunchAttributeClusterDimension;
   attr[0].val.clusterDim.x = (unsigned)splits;
   attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
-  lc.attrs = attr;
-  lc.numAttrs = splits > 1 ? 1 : 0;
+  lc.attrs = splits > 1 ? attr : attr + 1;
+  lc.numAttrs = splits > 1 ? 2 : 1;
   FB_CUDA(cudaLaunchKernelEx(&lc, kern, a.A, a.lda, a.B, a.ldb, a.C, a.ldc, a.Z, a.bias_n, a.bias_m, a.M, a.N, a.K, a.act, a.accumulate,
                              splits, kper, tiles_n));
   FB_LAUNCH_CHECK();

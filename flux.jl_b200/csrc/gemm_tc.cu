@@ -76,6 +76,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
                float* __restrict__ C, int64_t ldc, float* __restrict__ Z, const float* __restrict__ bias_n, int M,
                int N, int K, int act, int accumulate, int32_t* __restrict__ dev_err, int a3d, int b3d,
                const Sched sch) {
+  fb_after_previous();
   using cfg = Cfg<BN, PASSES, PAIR, SG>;
   constexpr int SPLIT_GROUPS = SG;
   constexpr int STAGES = cfg::STAGES;
@@ -676,13 +677,14 @@ int32_t launch_variant(fb_ctx* ctx, cudaStream_t stream, const fb_gemm_args& a, 
   lc.blockDim = dim3(cfg::NUM_THREADS, 1, 1);
   lc.dynamicSmemBytes = cfg::SMEM_BYTES;
   lc.stream = stream;
-  cudaLaunchAttribute attr[1];
+  cudaLaunchAttribute attr[2];
+  attr[1] = fb_early_start();
   attr[0].id = cudaLaunchAttributeClusterDimension;
   attr[0].val.clusterDim.x = (PAIR ? 2 : 1) * plan.ksplit;
   attr[0].val.clusterDim.y = 1;
   attr[0].val.clusterDim.z = 1;
   lc.attrs = attr;
-  lc.numAttrs = 1;
+  lc.numAttrs = 2;
   FB_CUDA(cudaLaunchKernelEx(&lc, kern, tmA, tmB, a.C, a.ldc, a.Z, a.bias_n, (int)a.M, (int)a.N, (int)a.K, a.act,
                              a.accumulate, ctx->dev_error, a3d, b3d, sch));
   FB_LAUNCH_CHECK();

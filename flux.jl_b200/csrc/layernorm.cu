@@ -38,6 +38,7 @@ __global__ void __launch_bounds__(LN_THREADS)
 ln_fwd_vec_kernel(const float4* __restrict__ x, const float4* __restrict__ gamma,
                   const float4* __restrict__ beta, float4* __restrict__ y, float* __restrict__ mean,
                   float* __restrict__ rstd, int d4, int64_t n, float eps, int act) {
+  fb_after_previous();
   __shared__ float sh[64];
   const float inv_d = 1.0f / (4.0f * (float)d4);
   for (int64_t row = blockIdx.x; row < n; row += gridDim.x) {
@@ -193,6 +194,7 @@ template <int V, int T, bool VEC, int ACT>
 __global__ void __launch_bounds__(LN_THREADS, VEC && V == 8 ? 2 : VEC && V == 4 ? 3 : 1)
 ln_fwd_rows_kernel(const float* __restrict__ x, const float* __restrict__ gamma, const float* __restrict__ beta,
                    float* __restrict__ y, float* __restrict__ mean, float* __restrict__ rstd, int d, int64_t n, float eps, int act) {
+  fb_after_previous();
   constexpr int W = VEC ? 4 : 1;
   __shared__ float sh[64];
   const int t = threadIdx.x % T;
@@ -263,6 +265,7 @@ __global__ void __launch_bounds__(LN_THREADS)
 ln_bwd_rows_kernel(const float* __restrict__ x, const float* __restrict__ gamma, const float* __restrict__ beta,
                    const float* __restrict__ mean, const float* __restrict__ rstd, const float* __restrict__ dy, float* __restrict__ dx,
                    float* __restrict__ part_dg, float* __restrict__ part_db, int d, int64_t n, int act) {
+  fb_after_previous();
   constexpr int W = VEC ? 4 : 1;
   __shared__ float sh[64];
   __shared__ float red[T == 32 ? 8 * V * W * 32 : 1];
@@ -378,6 +381,7 @@ __global__ void __launch_bounds__(LN_THREADS)
 ln_bwd_params_kernel(const float* __restrict__ x, const float* __restrict__ gamma, const float* __restrict__ beta,
                      const float* __restrict__ mean, const float* __restrict__ rstd, const float* __restrict__ dy, float dy_scale,
                      float* __restrict__ part_dg, float* __restrict__ part_db, int64_t d, int64_t n, int act, int lx) {
+  fb_after_previous();
   constexpr int W = VEC ? 4 : 1, U = 4;
   __shared__ float sa[LN_THREADS * W], sb[LN_THREADS * W];
   const int tx = threadIdx.x & (lx - 1), ty = threadIdx.x / lx, ny = LN_THREADS / lx;
@@ -487,6 +491,7 @@ template <int V, int T, int ACT, bool XB, bool YB>
 __global__ void __launch_bounds__(LN_THREADS)
 ln_fwd_low_kernel(const void* __restrict__ x, const float* __restrict__ gamma, const float* __restrict__ beta, void* __restrict__ y,
                   float* __restrict__ mean, float* __restrict__ rstd, int d, int64_t n, float eps, int act) {
+  fb_after_previous();
   constexpr int P = T == 32 ? 2 : 1, W = 4 * P;
   __shared__ float sh[64];
   const int t = threadIdx.x % T;
@@ -534,6 +539,7 @@ __global__ void __launch_bounds__(LN_THREADS)
 ln_bwd_low_kernel(const void* __restrict__ x, const float* __restrict__ gamma, const float* __restrict__ beta, const float* __restrict__ mean,
                   const float* __restrict__ rstd, const void* __restrict__ dy, void* __restrict__ dx, float* __restrict__ part_dg,
                   float* __restrict__ part_db, int d, int64_t n, int act) {
+  fb_after_previous();
   constexpr int P = T == 32 ? 2 : 1, W = 4 * P;
   __shared__ float sh[64];
   __shared__ float red[T == 32 ? 8 * V * 32 * W : 1];
@@ -670,6 +676,7 @@ __global__ void __launch_bounds__(LN_THREADS)
 ln_fwd_generic_kernel(const float* __restrict__ x, const float* __restrict__ gamma,
                       const float* __restrict__ beta, float* __restrict__ y, float* __restrict__ mean,
                       float* __restrict__ rstd, int64_t d, int64_t n, float eps, int act) {
+  fb_after_previous();
   __shared__ float sh[64];
   for (int64_t row = blockIdx.x; row < n; row += gridDim.x) {
     const float* xr = x + row * d;
@@ -697,6 +704,7 @@ ln_bwd_vec_kernel(const float4* __restrict__ x, const float4* __restrict__ gamma
                   const float4* __restrict__ beta, const float* __restrict__ mean,
                   const float* __restrict__ rstd, const float4* __restrict__ dy, float4* __restrict__ dx,
                   float4* __restrict__ part_dg, float4* __restrict__ part_db, int d4, int64_t n, int act) {
+  fb_after_previous();
   __shared__ float sh[64];
   const float inv_d = 1.0f / (4.0f * (float)d4);
   float4 ag[V], ab[V], gam[V], bet[V];
@@ -777,6 +785,7 @@ ln_bwd_pipe_kernel(const float* __restrict__ x, const float4* __restrict__ gamma
                    const float* __restrict__ mean, const float* __restrict__ rstd, const float* __restrict__ dy,
                    float4* __restrict__ dx, float4* __restrict__ part_dg, float4* __restrict__ part_db, int d4,
                    int64_t n, int act, int nstages, int32_t* __restrict__ dev_err) {
+  fb_after_previous();
   extern __shared__ __align__(128) uint8_t ln_smem[];
   __shared__ float sh[64];
   __shared__ __align__(8) uint64_t bar[LN_PIPE_MAX];
@@ -893,6 +902,7 @@ ln_bwd_generic_kernel(const float* __restrict__ x, const float* __restrict__ gam
                       const float* __restrict__ beta, const float* __restrict__ mean,
                       const float* __restrict__ rstd, const float* __restrict__ dy, float* __restrict__ dx,
                       float* __restrict__ part_dg, float* __restrict__ part_db, int64_t d, int64_t n, int act) {
+  fb_after_previous();
   __shared__ float sh[64];
   float* pg = part_dg ? part_dg + (int64_t)blockIdx.x * d : nullptr;
   float* pb = part_db ? part_db + (int64_t)blockIdx.x * d : nullptr;
@@ -930,6 +940,8 @@ ln_bwd_generic_kernel(const float* __restrict__ x, const float* __restrict__ gam
 __global__ void __launch_bounds__(256)
 fb_colreduce2_kernel(const float* __restrict__ part_a, const float* __restrict__ part_b,
                      float* __restrict__ out_a, float* __restrict__ out_b, int64_t groups, int64_t d) {
+  fb_after_previous();
+  fb_let_next_start();
   __shared__ float sa[8][33], sb[8][33];
   const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
   const int64_t col = (int64_t)blockIdx.x * 32 + tx;
@@ -1010,22 +1022,21 @@ FB_API int32_t fb_layernorm_fwd(fb_ctx* ctx, void* stream_, const float* x, cons
   const bool rows = ln_rows_dispatch(d, vec, [&](auto V, auto T, auto vc) {
     const int64_t per = LN_THREADS / T.value, blocks = (n + per - 1) / per;
     fb_act_kind(act, [&](auto k) {
-      ln_fwd_rows_kernel<V.value, T.value, vc.value, k.value><<<(unsigned)(blocks < 0x7fffffff ? blocks : 0x7fffffff), LN_THREADS, 0, stream>>>(
-          x, gamma, beta, y, mean, rstd, (int)d, n, eps, act);
+      fb_launch(ln_fwd_rows_kernel<V.value, T.value, vc.value, k.value>, (unsigned)(blocks < 0x7fffffff ? blocks : 0x7fffffff), LN_THREADS, 0, stream, x, gamma, beta, y, mean, rstd, (int)d, n, eps, act);
     });
   });
   if (rows) {
   } else if (v == 0) {
-    ln_fwd_generic_kernel<<<grid, LN_THREADS, 0, stream>>>(x, gamma, beta, y, mean, rstd, d, n, eps, act);
+    fb_launch(ln_fwd_generic_kernel, grid, LN_THREADS, 0, stream, x, gamma, beta, y, mean, rstd, d, n, eps, act);
   } else {
     const float4 *x4 = (const float4*)x, *g4 = (const float4*)gamma, *b4 = (const float4*)beta;
     float4* y4 = (float4*)y;
     const int d4 = (int)(d / 4);
     const unsigned gridv = (unsigned)(n < 0x7fffffff ? n : 0x7fffffff);
     switch (v) {
-      case 2: ln_fwd_vec_kernel<2><<<gridv, LN_THREADS, 0, stream>>>(x4, g4, b4, y4, mean, rstd, d4, n, eps, act); break;
-      case 4: ln_fwd_vec_kernel<4><<<gridv, LN_THREADS, 0, stream>>>(x4, g4, b4, y4, mean, rstd, d4, n, eps, act); break;
-      default: ln_fwd_vec_kernel<8><<<gridv, LN_THREADS, 0, stream>>>(x4, g4, b4, y4, mean, rstd, d4, n, eps, act); break;
+      case 2: fb_launch(ln_fwd_vec_kernel<2>, gridv, LN_THREADS, 0, stream, x4, g4, b4, y4, mean, rstd, d4, n, eps, act); break;
+      case 4: fb_launch(ln_fwd_vec_kernel<4>, gridv, LN_THREADS, 0, stream, x4, g4, b4, y4, mean, rstd, d4, n, eps, act); break;
+      default: fb_launch(ln_fwd_vec_kernel<8>, gridv, LN_THREADS, 0, stream, x4, g4, b4, y4, mean, rstd, d4, n, eps, act); break;
     }
   }
   FB_LAUNCH_CHECK();
@@ -1047,13 +1058,12 @@ int32_t fb_layernorm_bwd_impl(cudaStream_t stream, int sm_count, float* part, in
   const int v = vec ? ln_pick_v(d / 4) : 0;
   const bool rows = ln_rows_dispatch(d, vec, [&](auto V, auto T, auto vc) {
     fb_act_kind(act, [&](auto k) {
-      ln_bwd_rows_kernel<V.value, T.value, vc.value, k.value><<<(unsigned)groups, LN_THREADS, 0, stream>>>(
-          x, gamma, beta, mean, rstd, dy, dx, part_dg, part_db, (int)d, n, act);
+      fb_launch(ln_bwd_rows_kernel<V.value, T.value, vc.value, k.value>, (unsigned)groups, LN_THREADS, 0, stream, x, gamma, beta, mean, rstd, dy, dx, part_dg, part_db, (int)d, n, act);
     });
   });
   if (rows) {
   } else if (v == 0) {
-    ln_bwd_generic_kernel<<<(unsigned)groups, LN_THREADS, 0, stream>>>(x, gamma, beta, mean, rstd, dy, dx, part_dg,
+    fb_launch(ln_bwd_generic_kernel, (unsigned)groups, LN_THREADS, 0, stream, x, gamma, beta, mean, rstd, dy, dx, part_dg,
                                                                        part_db, d, n, act);
   } else {
     const float4 *x4 = (const float4*)x, *g4 = (const float4*)gamma, *b4 = (const float4*)beta, *dy4 = (const float4*)dy;
@@ -1069,28 +1079,28 @@ int32_t fb_layernorm_bwd_impl(cudaStream_t stream, int sm_count, float* part, in
       switch (v) {
         case 2:
           FB_CUDA(fb_allow_smem(ln_bwd_pipe_kernel<2>, LN_PIPE_BYTES));
-          ln_bwd_pipe_kernel<2><<<g, LN_THREADS, smem, stream>>>(x, g4, b4, mean, rstd, dy, dx4, pg4, pb4, d4, n, act, nst, dev_err);
+          fb_launch(ln_bwd_pipe_kernel<2>, g, LN_THREADS, smem, stream, x, g4, b4, mean, rstd, dy, dx4, pg4, pb4, d4, n, act, nst, dev_err);
           break;
         case 4:
           FB_CUDA(fb_allow_smem(ln_bwd_pipe_kernel<4>, LN_PIPE_BYTES));
-          ln_bwd_pipe_kernel<4><<<g, LN_THREADS, smem, stream>>>(x, g4, b4, mean, rstd, dy, dx4, pg4, pb4, d4, n, act, nst, dev_err);
+          fb_launch(ln_bwd_pipe_kernel<4>, g, LN_THREADS, smem, stream, x, g4, b4, mean, rstd, dy, dx4, pg4, pb4, d4, n, act, nst, dev_err);
           break;
         default:
           FB_CUDA(fb_allow_smem(ln_bwd_pipe_kernel<8>, LN_PIPE_BYTES));
-          ln_bwd_pipe_kernel<8><<<g, LN_THREADS, smem, stream>>>(x, g4, b4, mean, rstd, dy, dx4, pg4, pb4, d4, n, act, nst, dev_err);
+          fb_launch(ln_bwd_pipe_kernel<8>, g, LN_THREADS, smem, stream, x, g4, b4, mean, rstd, dy, dx4, pg4, pb4, d4, n, act, nst, dev_err);
           break;
       }
     } else {
       switch (v) {
-        case 2: ln_bwd_vec_kernel<2><<<g, LN_THREADS, 0, stream>>>(x4, g4, b4, mean, rstd, dy4, dx4, pg4, pb4, d4, n, act); break;
-        case 4: ln_bwd_vec_kernel<4><<<g, LN_THREADS, 0, stream>>>(x4, g4, b4, mean, rstd, dy4, dx4, pg4, pb4, d4, n, act); break;
-        default: ln_bwd_vec_kernel<8><<<g, LN_THREADS, 0, stream>>>(x4, g4, b4, mean, rstd, dy4, dx4, pg4, pb4, d4, n, act); break;
+        case 2: fb_launch(ln_bwd_vec_kernel<2>, g, LN_THREADS, 0, stream, x4, g4, b4, mean, rstd, dy4, dx4, pg4, pb4, d4, n, act); break;
+        case 4: fb_launch(ln_bwd_vec_kernel<4>, g, LN_THREADS, 0, stream, x4, g4, b4, mean, rstd, dy4, dx4, pg4, pb4, d4, n, act); break;
+        default: fb_launch(ln_bwd_vec_kernel<8>, g, LN_THREADS, 0, stream, x4, g4, b4, mean, rstd, dy4, dx4, pg4, pb4, d4, n, act); break;
       }
     }
   }
   FB_LAUNCH_CHECK();
   if (want_param) {
-    fb_colreduce2_kernel<<<(unsigned)((d + 31) / 32), 256, 0, stream>>>(part_dg, part_db, dgamma, dbeta, groups, d);
+    fb_launch(fb_colreduce2_kernel, (unsigned)((d + 31) / 32), 256, 0, stream, part_dg, part_db, dgamma, dbeta, groups, d);
     FB_LAUNCH_CHECK();
   }
   return FB_OK;
@@ -1186,10 +1196,10 @@ static int32_t ln_bwd_params(const char* fn, fb_ctx* ctx, cudaStream_t stream, c
   fb_act_kind(act, [&](auto k) {
     auto kern = dy == nullptr ? (vec ? ln_bwd_params_kernel<true, k.value, false, true> : ln_bwd_params_kernel<false, k.value, false, true>)
                               : (vec ? ln_bwd_params_kernel<true, k.value, false, false> : ln_bwd_params_kernel<false, k.value, false, false>);
-    kern<<<grid, LN_THREADS, 0, stream>>>(x, gamma, beta, mean, rstd, dy, dy_scale, pg, pb, d, n, act, lx);
+    fb_launch(kern, grid, LN_THREADS, 0, stream, x, gamma, beta, mean, rstd, dy, dy_scale, pg, pb, d, n, act, lx);
   });
   FB_LAUNCH_CHECK();
-  fb_colreduce2_kernel<<<(unsigned)((d + 31) / 32), 256, 0, stream>>>(pg, pb, dgamma, dbeta, groups, d);
+  fb_launch(fb_colreduce2_kernel, (unsigned)((d + 31) / 32), 256, 0, stream, pg, pb, dgamma, dbeta, groups, d);
   FB_LAUNCH_CHECK();
   return FB_OK;
 }
@@ -1228,7 +1238,7 @@ FB_API int32_t fb_layernorm_fwd_mixed(fb_ctx* ctx, void* stream_, const void* x,
     const unsigned grid = (unsigned)(blocks < 0x7fffffff ? blocks : 0x7fffffff);
     fb_act_kind(act, [&](auto k) {
       ln_flags(x_bf16 != 0, y_bf16 != 0, [&](auto xb, auto yb) {
-        ln_fwd_low_kernel<V.value, T.value, k.value, xb.value, yb.value><<<grid, LN_THREADS, 0, stream>>>(x, gamma, beta, y, mean, rstd, (int)d, n, eps, act);
+        fb_launch(ln_fwd_low_kernel<V.value, T.value, k.value, xb.value, yb.value>, grid, LN_THREADS, 0, stream, x, gamma, beta, y, mean, rstd, (int)d, n, eps, act);
       });
     });
   });
@@ -1264,14 +1274,13 @@ FB_API int32_t fb_layernorm_bwd_mixed(fb_ctx* ctx, void* stream_, const void* x,
   ln_low_dispatch(d, [&](auto V, auto T) {
     fb_act_kind(act, [&](auto k) {
       ln_flags(x_bf16 != 0, dy_bf16 != 0, [&](auto xb, auto db) {
-        ln_bwd_low_kernel<V.value, T.value, k.value, xb.value, db.value><<<(unsigned)groups, LN_THREADS, 0, stream>>>(
-            x, gamma, beta, mean, rstd, dy, dx, pg, pb, (int)d, n, act);
+        fb_launch(ln_bwd_low_kernel<V.value, T.value, k.value, xb.value, db.value>, (unsigned)groups, LN_THREADS, 0, stream, x, gamma, beta, mean, rstd, dy, dx, pg, pb, (int)d, n, act);
       });
     });
   });
   FB_LAUNCH_CHECK();
   if (dgamma) {
-    fb_colreduce2_kernel<<<(unsigned)((d + 31) / 32), 256, 0, stream>>>(pg, pb, dgamma, dbeta, groups, d);
+    fb_launch(fb_colreduce2_kernel, (unsigned)((d + 31) / 32), 256, 0, stream, pg, pb, dgamma, dbeta, groups, d);
     FB_LAUNCH_CHECK();
   }
   return FB_OK;

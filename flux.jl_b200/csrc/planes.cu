@@ -242,6 +242,7 @@ __device__ void split_rows_any(const PlaneOp& op, int block) {
 
 // first kernel: K-major operands are split, MN-major ones get their maxima; second: MN-major ones are split
 __global__ void __launch_bounds__(256, 4) planes_first_kernel(const PlaneOp a, const PlaneOp b) {
+  fb_after_previous();
   const bool first = (int)blockIdx.x < a.blocks1;
   const PlaneOp& op = first ? a : b;
   const int block = first ? (int)blockIdx.x : (int)blockIdx.x - a.blocks1;
@@ -249,6 +250,7 @@ __global__ void __launch_bounds__(256, 4) planes_first_kernel(const PlaneOp a, c
   else split_rows_any(op, block);
 }
 __global__ void __launch_bounds__(256, 4) planes_second_kernel(const PlaneOp a, const PlaneOp b) {
+  fb_after_previous();
   const bool first = (int)blockIdx.x < a.blocks2;
   split_cols(first ? a : b, first ? (int)blockIdx.x : (int)blockIdx.x - a.blocks2);
 }
@@ -323,10 +325,10 @@ int32_t fb_planes_split(cudaStream_t stream, const fb_gemm_args& g, void* mem, f
     out->rows[i] = tiles * o.num_kb * 2 * IMG_ROWS;
   }
   if (blocks1 > 0x7fffffff || blocks2 > 0x7fffffff) return fb_fail(FB_ERR_UNSUPPORTED, "gemm: operands too large to split");
-  planes_first_kernel<<<(unsigned)blocks1, 256, 0, stream>>>(op[0], op[1]);
+  fb_launch(planes_first_kernel, (unsigned)blocks1, 256, 0, stream, op[0], op[1]);
   FB_LAUNCH_CHECK();
   if (blocks2 > 0) {
-    planes_second_kernel<<<(unsigned)blocks2, 256, 0, stream>>>(op[0], op[1]);
+    fb_launch(planes_second_kernel, (unsigned)blocks2, 256, 0, stream, op[0], op[1]);
     FB_LAUNCH_CHECK();
   }
   return FB_OK;

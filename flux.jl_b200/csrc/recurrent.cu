@@ -456,6 +456,7 @@ constexpr size_t DH2D_SMEM = (size_t)2 * DH_U * DH_LD * sizeof(float);
 __global__ void __launch_bounds__(RT)
 shift_prev_kernel(const float* __restrict__ out, const float* __restrict__ h0, float* __restrict__ hprev_all, int H,
                   int64_t T, int64_t B) {
+  fb_after_previous();
   const int64_t total = B * T * H;
   for (int64_t e = (int64_t)blockIdx.x * RT + threadIdx.x; e < total; e += (int64_t)gridDim.x * RT) {
     const int64_t row = e / H;
@@ -813,7 +814,7 @@ FB_API int32_t fb_lstm_bwd(fb_ctx* ctx, void* stream_, const float* Wi, const fl
   {
     int64_t sb = (rows * H + RT - 1) / RT;
     if (sb > (int64_t)ctx->sm_count * 16) sb = (int64_t)ctx->sm_count * 16;
-    shift_prev_kernel<<<(unsigned)sb, RT, 0, stream>>>(out, h0, hprev_all, H, T, batch);
+    fb_launch(shift_prev_kernel, (unsigned)sb, RT, 0, stream, out, h0, hprev_all, H, T, batch);
     FB_LAUNCH_CHECK();
     a.A = hprev_all; a.lda = hidden; a.a_mn_major = 1;
     a.B = dg; a.ldb = 4 * hidden; a.b_mn_major = 1;
@@ -941,7 +942,7 @@ FB_API int32_t fb_gru_bwd(fb_ctx* ctx, void* stream_, const float* Wi, const flo
     float* hprev_all = dgh + rows * 3 * H;
     int64_t sb = (rows * H + RT - 1) / RT;
     if (sb > (int64_t)ctx->sm_count * 16) sb = (int64_t)ctx->sm_count * 16;
-    shift_prev_kernel<<<(unsigned)sb, RT, 0, stream>>>(out, h0, hprev_all, H, T, batch);
+    fb_launch(shift_prev_kernel, (unsigned)sb, RT, 0, stream, out, h0, hprev_all, H, T, batch);
     FB_LAUNCH_CHECK();
     a.A = hprev_all; a.lda = hidden; a.a_mn_major = 1;
     a.B = dgh; a.ldb = 3 * hidden; a.b_mn_major = 1;
