@@ -548,10 +548,10 @@ int32_t fb_attn_fwd_redo(fb_ctx* ctx, cudaStream_t stream, int bf16, const void*
   gx = gx < 1 ? 1 : gx > tiles ? tiles : gx;
   const dim3 grid((unsigned)gx, (unsigned)nheads, (unsigned)batch);
   if (bf16) {
-    FB_CUDA(cudaFuncSetAttribute(attn_fwd_kernel<1, uint16_t, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    FB_ONCE(ctx, FB_CUDA(cudaFuncSetAttribute(attn_fwd_kernel<1, uint16_t, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem)));
     fb_launch(attn_fwd_kernel<1, uint16_t, true>, grid, AT, smem, stream, (const uint16_t*)q, (const uint16_t*)k, (const uint16_t*)v, nullptr, o, o16, lse, D);
   } else {
-    FB_CUDA(cudaFuncSetAttribute(attn_fwd_kernel<1, float, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    FB_ONCE(ctx, FB_CUDA(cudaFuncSetAttribute(attn_fwd_kernel<1, float, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem)));
     fb_launch(attn_fwd_kernel<1, float, true>, grid, AT, smem, stream, (const float*)q, (const float*)k, (const float*)v, nullptr, o, nullptr, lse, D);
   }
   FB_LAUNCH_CHECK();
@@ -569,12 +569,12 @@ static int32_t bwd_redo(fb_ctx* ctx, cudaStream_t stream, const void* q, const v
     return (unsigned)(fit < 1 ? 1 : fit > tiles ? tiles : fit);
   };
   if (dk != nullptr) {
-    FB_CUDA(cudaFuncSetAttribute(attn_bwd_dkdv_kernel<1, T, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_kv));
+    FB_ONCE(ctx, FB_CUDA(cudaFuncSetAttribute(attn_bwd_dkdv_kernel<1, T, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_kv)));
     fb_launch(attn_bwd_dkdv_kernel<1, T, true>, dim3(blocks(D.Lk), (unsigned)D.H, (unsigned)batch), AT, smem_kv, stream, (const T*)q, (const T*)k, (const T*)v, nullptr, lse, dlt, (const T*)dout, (T*)dk, (T*)dv, D);
     FB_LAUNCH_CHECK();
   }
   if (dq != nullptr) {
-    FB_CUDA(cudaFuncSetAttribute(attn_bwd_dq_kernel<1, T, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_q));
+    FB_ONCE(ctx, FB_CUDA(cudaFuncSetAttribute(attn_bwd_dq_kernel<1, T, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_q)));
     fb_launch(attn_bwd_dq_kernel<1, T, true>, dim3(blocks(D.Lq), (unsigned)D.H, (unsigned)batch), AT, smem_q, stream, (const T*)q, (const T*)k, (const T*)v, nullptr, lse, dlt, (const T*)dout, (T*)dq, D);
     FB_LAUNCH_CHECK();
   }

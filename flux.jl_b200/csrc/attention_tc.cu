@@ -1230,7 +1230,7 @@ int32_t fwd_impl(fb_ctx* ctx, cudaStream_t stream, const uint8_t* q, const uint8
   const fb_temp images(ctx, stream, (size_t)(chunk * per + 512));
   uint8_t* img = (uint8_t*)images.p;
   if (!img) return FB_ERR_UNSUPPORTED;
-  FB_CUDA(cudaFuncSetAttribute(attn_fwd_tc_kernel<NP>, cudaFuncAttributeMaxDynamicSharedMemorySize, FwdCfg<NP>::SMEM));
+  FB_ONCE(ctx, FB_CUDA(cudaFuncSetAttribute(attn_fwd_tc_kernel<NP>, cudaFuncAttributeMaxDynamicSharedMemorySize, FwdCfg<NP>::SMEM)));
   for (int64_t b0 = 0; b0 < batch; b0 += chunk) {
     const int64_t nb = b0 + chunk > batch ? batch - b0 : chunk;
     int16_t* shifts = (int16_t*)(img + nb * 2 * P.kbytes);
@@ -1264,8 +1264,8 @@ int32_t bwd_impl(fb_ctx* ctx, cudaStream_t stream, const uint8_t* q, const uint8
   const fb_temp images(ctx, stream, (size_t)(chunk * per + 512));
   uint8_t* img = (uint8_t*)images.p;
   if (!img) return FB_ERR_UNSUPPORTED;
-  FB_CUDA(cudaFuncSetAttribute(attn_bwd_dkdv_tc_kernel<NP>, cudaFuncAttributeMaxDynamicSharedMemorySize, KvCfg<NP>::SMEM));
-  FB_CUDA(cudaFuncSetAttribute(attn_bwd_dq_tc_kernel<NP>, cudaFuncAttributeMaxDynamicSharedMemorySize, DqCfg<NP>::SMEM));
+  FB_ONCE(ctx, FB_CUDA(cudaFuncSetAttribute(attn_bwd_dkdv_tc_kernel<NP>, cudaFuncAttributeMaxDynamicSharedMemorySize, KvCfg<NP>::SMEM)));
+  FB_ONCE(ctx, FB_CUDA(cudaFuncSetAttribute(attn_bwd_dq_tc_kernel<NP>, cudaFuncAttributeMaxDynamicSharedMemorySize, DqCfg<NP>::SMEM)));
   for (int64_t b0 = 0; b0 < batch; b0 += chunk) {
     const int64_t nb = b0 + chunk > batch ? batch - b0 : chunk;
     uint8_t *ki = img, *vi = ki + nb * P.kbytes, *qi = vi + nb * P.kbytes, *doi = qi + nb * P.qbytes;

@@ -121,6 +121,17 @@ static inline cudaError_t fb_allow_smem(K kern, size_t most) {
   return cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)most);
 }
 
+// Attributes of one kernel (of one instantiation, where it stands in a template): set once per thread and device, as each of these calls
+// takes 1 - 7 us.
+#define FB_ONCE(ctx, ...)                                  \
+  do {                                                     \
+    static thread_local int prepared__ = -1;               \
+    if (prepared__ != (ctx)->device) {                     \
+      __VA_ARGS__;                                         \
+      prepared__ = (ctx)->device;                          \
+    }                                                      \
+  } while (0)
+
 // BFloat16 bits by round-to-nearest-even in the integer domain, NaN -> 0x7fc0 (Flux._to_bf16)
 __device__ __forceinline__ uint16_t fb_bf16_bits(float f) {
   const uint32_t u = __float_as_uint(f);

@@ -200,8 +200,7 @@ int32_t launch(fb_ctx* ctx, cudaStream_t stream, const DcArgs& A) {
   lc.stream = stream;
   lc.attrs = at;
   lc.numAttrs = 2;
-  FB_CUDA(fb_allow_smem(dense_chain_kernel<NB>, DC_SMEM));
-  FB_CUDA(cudaFuncSetAttribute(dense_chain_kernel<NB>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
+  FB_ONCE(ctx, FB_CUDA(fb_allow_smem(dense_chain_kernel<NB>, DC_SMEM)); FB_CUDA(cudaFuncSetAttribute(dense_chain_kernel<NB>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1)));
   FB_CUDA(cudaLaunchKernelEx(&lc, dense_chain_kernel<NB>, A));
   FB_LAUNCH_CHECK();
   return FB_OK;
