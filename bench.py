@@ -631,7 +631,7 @@ def small_config_lines(config, steps, warmup):
                 8, ms, clocks,
                 {"bound": "tensor", "achieved": flops / ms / 1e9, "peak": peak, "unit": "TFLOP/s", "frac": flops / ms / 1e9 / peak, "traffic": None,
                  "flops_per_step": flops,
-                 "note": ("projections on tcgen05 as half-precision planes or 3xTF32, the attention core (forward, dQ, dK/dV) on three bf16 planes per operand; softmax and dS on TMEM read-back; "
+                 "note": ("projections on tcgen05 as half-precision planes or 3xTF32, the attention core (forward, dQ, dK/dV) on two half-precision planes per operand; softmax and dS on TMEM read-back; "
                           if dtype == "f32" else "the opt-in bf16 path (fluxb200.bf16); ") + how},
                 ms_e2e, h2d, (1 * (512 / 2048) ** 2 * 1.0) / cpu,
                 "1 of 8 samples at seq 512 (1/16 of a sample's attention work, 1/4 of its projections), Float32, 1 run", dtype=dtype)

@@ -1,4 +1,4 @@
-"""Tensor-core attention (bf16 planes): head sizes, ragged tiles, unseen keys and slot / region reuse against float64."""
+"""Tensor-core attention (half-precision planes): head sizes, ragged tiles, unseen keys and slot / region reuse against float64."""
 import numpy as np
 import pytest
 
