@@ -1,370 +1,156 @@
-// Flash-style attention on the tensor cores (tcgen05), forward and backward, for head sizes up to 64.
+// Flash-style attention of bf16 operands on the tensor cores (tcgen05), for head sizes up to 64 forward and of 64 backward.
 //
-// Float32 operands are two half-precision planes, x 2^s = hi + lo 2^-11 (23 bits; a power of two per tile or row), and a product is the
-// sum of three plane products: the cross terms first, then hi hi over 2^-11 of them (the MMA scales its accumulator), or, where
-// sums go on over the blocks, in accumulators of their own.  An image in the 128-byte swizzle serves as K-major and as MN-major operand;
-// a small kernel (`attn_split_kernel`) makes the images of K, V, Q and dO once per call, and tiles arrive by plain bulk copies.
-// bf16 operands are one plane, exactly; the probabilities and dS keep two.  Head sizes below 64 are padded with zeros in the images;
-// their zero 16-feature steps are skipped.
+// An operand is one bf16 plane, exactly; the probabilities and dS are Float32 values, cut into three bf16 planes by truncation (8 + 8 + 8
+// mantissa bits: the split is exact), and a product with them is the sum of three plane products, the smallest ones first, accumulated
+// in Float32 in tensor memory.  A bf16 tile in the 128-byte swizzle serves as K-major and as MN-major operand: a small kernel
+// (`attn_split_kernel`) lays K, V, Q and dO out once per call as the images that the MMAs read from shared memory, and tiles arrive by plain
+// bulk copies.  Head sizes below 64 are padded with zeros in those images; their zero 16-feature steps are skipped.
 //
-// Against three bf16 planes per operand and six products (batch 8, 16 heads of 64, 2048 x 2048, causal; us): Float32 images 51 + 114 -> 41
-// + 91, forward 507 -> 350, dK / dV 1113 -> 579, dQ 848 -> 499; bf16 25 + 63 -> 35 + 81, 323 -> 272, 572 -> 442, 374 -> 327.  Errors
-// against float64 (Float32): output 2.3e-7 as before, dQ 4.7e-6 -> 0.9e-6, dK / dV 1.9e-5 -> 3.8e-6 (half as many truncating adds).
-// What bounds them: an MMA with N = 64 takes 53 clocks with A in tensor memory and 74 with A in shared memory, where its multiplications
-// need 32, and between the MMAs of a block the weights' arithmetic (one warp of a set per SM partition, 3700 clocks a block).
+// (Two half-precision planes for the probabilities and dS, as attention_half.cu has them, take a third of these MMAs away, but hold 23 bits
+// of them and, where the scales of a head's tiles differ, fewer.)  What bounds the kernels: an MMA with N = 64 takes 44 clocks where its
+// multiplications need 32, and between the MMAs of a block the weights' arithmetic.
 //
 // A block is 64 keys (64 queries in the dK / dV kernel) against the 128 rows of a CTA; a thread of a compute warp owns
 // one row (one TMEM lane).  Every mbarrier wait is bounded; when one runs out the kernel records 4002 (forward), 4003
 // (dQ) or 4004 (dK / dV) in the context's device error word, all roles leave their loops, tensor memory is released and
 // the kernel returns.
-#include <cuda.h>
-#include <cuda_bf16.h>
-#include <cuda_fp16.h>
-#include <stdlib.h>
+#include "attention_tc.cuh"
 
-#include "common.cuh"
-#include "tc_common.cuh"
+using namespace fb_atc;
 
 namespace {
 
-constexpr int QT = 128;        // rows (queries, or keys in the dK / dV kernel) per CTA
-constexpr int KT = 64;         // keys (queries) per block
-constexpr int HD = 64;         // padded head size
-constexpr int TILE = 8192;     // one plane of a 64 x 64 tile: 64 rows of 128 bytes, 128-byte swizzle
-constexpr uint32_t LAYOUT_SW128 = 2;
-constexpr float LOG2E = 1.4426950408889634f, LN2_HI = 0.693145751953125f, LN2_LO = 1.42860682030941723e-6f;
-
-struct AtcDims {
-  int64_t E, Ev, Lq, Lk;
-  int H, causal, d, dv;
-  int qtiles, ktiles;   // 64-row tiles per (batch, head) in the plane images (even)
-  int max_tiles;        // the larger of both
-  int vec;              // rows can be read and written 16 bytes at a time
-  float scale_log2;     // log2(e) / sqrt(d)
-  float scale;          // 1 / sqrt(d)
-};
-
-// --------------------------------------------------------------------------------------------------- wrappers ---
-__device__ __forceinline__ void tc_st_32x32b_x16(uint32_t taddr, const uint32_t* r) {
-  asm volatile(
-      "tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], "
-      "{%1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16};"
-      ::"r"(taddr), "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]), "r"(r[8]), "r"(r[9]),
-      "r"(r[10]), "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15])
-      : "memory");
+// Two values as three bf16 planes (x in the low half of each word): truncation to the upper 16 bits leaves a remainder of
+// at most 16 significant bits, the same again one of at most 8, which is a bf16 value.
+__device__ __forceinline__ void split3(float x, float y, uint32_t& p0, uint32_t& p1, uint32_t& p2) {
+  const uint32_t xb = __float_as_uint(x), yb = __float_as_uint(y);
+  p0 = __byte_perm(xb, yb, 0x7632);
+  const float rx = x - __uint_as_float(xb & 0xffff0000u), ry = y - __uint_as_float(yb & 0xffff0000u);
+  const uint32_t rxb = __float_as_uint(rx), ryb = __float_as_uint(ry);
+  p1 = __byte_perm(rxb, ryb, 0x7632);
+  p2 = __byte_perm(__float_as_uint(rx - __uint_as_float(rxb & 0xffff0000u)), __float_as_uint(ry - __uint_as_float(ryb & 0xffff0000u)), 0x7632);
 }
-__device__ __forceinline__ void tc_wait_st() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
-
-// Shared-memory descriptors travel as their low word (start address / 16 in its 14 low bits, leading offset above), to which a
-// step's offset is added, and a high word that all steps share.  A tile ends below 228 KB, so that the sum never leaves the
-// 14 bits.  (As 64-bit sums for A and B under a run-time step count one form of the product below gave wrong low-order terms;
-// where the compiler went wrong there is not known, so no form adds to 64 bits.)
-//
-// D[tmem] (+)= A[tmem] * B[smem]: the A tile (128 rows x 16 halves) sits in 8 consecutive TMEM columns, two values each
-__device__ __forceinline__ void tc_mma_ta(uint32_t d_tmem, uint32_t a_tmem, uint32_t b_lo, uint32_t hi, uint32_t idesc, uint32_t accumulate) {
-  asm volatile(
-      "{\n\t.reg .pred p, q;\n\t.reg .b64 db;\n\t"
-      "elect.sync _|q, 0xffffffff;\n\t"
-      "setp.ne.b32 p, %4, 0;\n\t"
-      "mov.b64 db, {%2, %9};\n\t"
-      "@q tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], db, %3, {%5, %6, %7, %8}, p;\n\t}"
-      ::"r"(d_tmem), "r"(a_tmem), "r"(b_lo), "r"(idesc), "r"(accumulate), "r"(0u), "r"(0u), "r"(0u), "r"(0u), "r"(hi)
-      : "memory");
-}
-// the same with A from shared memory
-__device__ __forceinline__ void tc_mma_sa(uint32_t d_tmem, uint32_t a_lo, uint32_t b_lo, uint32_t hi, uint32_t idesc, uint32_t accumulate) {
-  asm volatile(
-      "{\n\t.reg .pred p, q;\n\t.reg .b64 da, db;\n\t"
-      "elect.sync _|q, 0xffffffff;\n\t"
-      "setp.ne.b32 p, %4, 0;\n\t"
-      "mov.b64 da, {%1, %9};\n\t"
-      "mov.b64 db, {%2, %9};\n\t"
-      "@q tcgen05.mma.cta_group::1.kind::f16 [%0], da, db, %3, {%5, %6, %7, %8}, p;\n\t}"
-      ::"r"(d_tmem), "r"(a_lo), "r"(b_lo), "r"(idesc), "r"(accumulate), "r"(0u), "r"(0u), "r"(0u), "r"(0u), "r"(hi)
-      : "memory");
-}
-
-// the same where D is first multiplied by 2^-11 (A from tensor memory; A from shared memory)
-__device__ __forceinline__ void tc_mma_ta_down(uint32_t d_tmem, uint32_t a_tmem, uint32_t b_lo, uint32_t hi, uint32_t idesc) {
-  asm volatile(
-      "{\n\t.reg .pred p, q;\n\t.reg .b64 db;\n\t"
-      "elect.sync _|q, 0xffffffff;\n\t"
-      "setp.eq.b32 p, %4, 0;\n\t"
-      "mov.b64 db, {%2, %5};\n\t"
-      "@q tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], db, %3, {%4, %4, %4, %4}, p, 11;\n\t}"
-      ::"r"(d_tmem), "r"(a_tmem), "r"(b_lo), "r"(idesc), "r"(0u), "r"(hi)
-      : "memory");
-}
-__device__ __forceinline__ void tc_mma_sa_down(uint32_t d_tmem, uint32_t a_lo, uint32_t b_lo, uint32_t hi, uint32_t idesc) {
-  asm volatile(
-      "{\n\t.reg .pred p, q;\n\t.reg .b64 da, db;\n\t"
-      "elect.sync _|q, 0xffffffff;\n\t"
-      "setp.eq.b32 p, %4, 0;\n\t"
-      "mov.b64 da, {%1, %5};\n\t"
-      "mov.b64 db, {%2, %5};\n\t"
-      "@q tcgen05.mma.cta_group::1.kind::f16 [%0], da, db, %3, {%4, %4, %4, %4}, p, 11;\n\t}"
-      ::"r"(d_tmem), "r"(a_lo), "r"(b_lo), "r"(idesc), "r"(0u), "r"(hi)
-      : "memory");
-}
-// plain bulk copy of a piece of a plane image (both addresses and the size are multiples of 16 bytes)
-__device__ __forceinline__ void bulk_load(uint32_t dst, const void* src, uint32_t bytes, uint32_t bar) {
-  asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
-               ::"r"(dst), "l"(src), "r"(bytes), "r"(bar)
-               : "memory");
-}
-
-// 2^x by the special-function unit (relative error ~2^-22, far inside the tolerance of a softmax weight)
-__device__ __forceinline__ float fast_exp2(float x) {
-  float y;
-  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
-  return y;
-}
-
-// Two values as two half-precision planes (x in the low half of each word): the upper one rounded to nearest, the lower one the
-// remainder times 2^11, so that it keeps its bits as long as the upper one does.
-__device__ __forceinline__ void split2(float x, float y, uint32_t& hi, uint32_t& lo) {
-  const __half2 h = __floats2half2_rn(x, y);
-  const float2 f = __half22float2(h);
-  const __half2 l = __floats2half2_rn((x - f.x) * 2048.0f, (y - f.y) * 2048.0f);
-  hi = *reinterpret_cast<const uint32_t*>(&h);
-  lo = *reinterpret_cast<const uint32_t*>(&l);
-}
-__device__ __forceinline__ uint32_t half2_bits(float x, float y) {
-  const __half2 h = __floats2half2_rn(x, y);
-  return *reinterpret_cast<const uint32_t*>(&h);
-}
-
-// Scales are powers of two, as shifts: 2^s puts a largest magnitude (its bits) into [2^14, 2^15).  What is scaled so is held to 2^-23
-// of itself down to 2^-29 of the largest value and to 2^-51 of that below (bf16 values, one plane: exactly down to 2^-32).
-// Three bf16 planes held 2^-25.  It shows where scores are large, whose exponentials turn it into an absolute error: with a key and a
-// value 1e4 times the others errors went 6e-7 -> 4e-6 (o), 1.6e-4 -> 4.3e-3 (dQ), 2.5e-4 -> 1.7e-3 (dV).
-constexpr int SH_ZERO = 1000;    // all values are 0
-__device__ __forceinline__ int shift_of(uint32_t max_bits) { return max_bits == 0 ? SH_ZERO : 141 - (int)(max_bits >> 23); }
-__device__ __forceinline__ float pow2(int e) { return e < -126 ? 0.0f : __int_as_float((e > 127 ? 254 : e + 127) << 23); }
-// v 2^e in two factors, |e| <= 252
-__device__ __forceinline__ float times_pow2(float v, int e) {
-  const int h = e / 2;
-  return v * pow2(h) * pow2(e - h);
-}
-// the line below which an element of a scaled row or tile is badly held; two of them make its head one for the FMA kernels
-template <int NP>
-__device__ __forceinline__ constexpr float faint_line() { return NP == 2 ? 1.9073486328125e-6f : 1.52587890625e-5f; }   // 2^-19, 2^-16
-// largest shifts, up or down, of Q and K, of V and of dO: products of two of their powers of two stay in range
-constexpr int SH_QK = 60, SH_V = 40, SH_DO = 85;
-
-__device__ __forceinline__ uint32_t pack2(float lo, float hi) {
-  const __nv_bfloat162 v = __floats2bfloat162_rn(lo, hi);
-  return *reinterpret_cast<const uint32_t*>(&v);
-}
-
-// 32 values of a thread's row into the two planes of an A operand: 16 columns each at t0 and t1
-__device__ __forceinline__ void store_planes32(uint32_t t0, uint32_t t1, const uint32_t* v) {
-  uint32_t a[16], b[16];
+// 32 values of a thread's row into the three planes of an A operand: 16 columns each at t0, t1 and t2
+__device__ __forceinline__ void store_planes32(uint32_t t0, uint32_t t1, uint32_t t2, const uint32_t* v) {
+  uint32_t a[16], b[16], c[16];
 #pragma unroll
-  for (int e = 0; e < 16; ++e) split2(__uint_as_float(v[2 * e]), __uint_as_float(v[2 * e + 1]), a[e], b[e]);
+  for (int e = 0; e < 16; ++e) split3(__uint_as_float(v[2 * e]), __uint_as_float(v[2 * e + 1]), a[e], b[e], c[e]);
   tc_st_32x32b_x16(t0, a);
   tc_st_32x32b_x16(t1, b);
+  tc_st_32x32b_x16(t2, c);
 }
 
-// 32 consecutive features (from c0) of one row as Float32 values; zero beyond the head size or for a dead row
-__device__ __forceinline__ void row_f32(const float* src, int c0, int width, bool live, bool vec, uint32_t* v) {
-  if (vec) {
-#pragma unroll
-    for (int c = 0; c < 32; c += 4) {
-      float4 x = make_float4(0.f, 0.f, 0.f, 0.f);
-      if (live && c0 + c < width) x = __ldg((const float4*)(src + c0 + c));
-      v[c] = __float_as_uint(x.x); v[c + 1] = __float_as_uint(x.y); v[c + 2] = __float_as_uint(x.z); v[c + 3] = __float_as_uint(x.w);
-    }
-  } else {
-#pragma unroll
-    for (int c = 0; c < 32; ++c) v[c] = (live && c0 + c < width) ? __float_as_uint(__ldg(src + c0 + c)) : 0u;
-  }
-}
-
-__device__ __forceinline__ bool not_finite(uint32_t bits) { return (bits & 0x7f800000u) == 0x7f800000u; }
-
-// One row of a CTA's own operand into tensor memory: NP planes of 32 columns each (Float32 source: 2, bf16 source: 1), scaled by 2^sh.
-// True when the planes cannot hold it.
+// One row of a CTA's own operand into tensor memory: NP planes of 32 columns each (Float32 source: 3, bf16 source: 1).
+// True when a value of it is not finite.
 template <int NP>
-__device__ __forceinline__ bool row_to_tmem(const void* src, int width, bool live, bool vec, uint32_t t_addr, int limit, int& sh) {
-  uint32_t v[2][32];
+__device__ __forceinline__ bool row_to_tmem(const void* src, int width, bool live, bool vec, uint32_t t_addr) {
+  bool odd = false;
 #pragma unroll
   for (int hf = 0; hf < 2; ++hf) {
-    if (NP == 2) {
-      row_f32((const float*)src, 32 * hf, width, live, vec, v[hf]);
+    if (NP == 3) {
+      uint32_t v[32];
+      row_f32((const float*)src, 32 * hf, width, live, vec, v);
+#pragma unroll
+      for (int c = 0; c < 32; ++c) odd |= not_finite(v[c]);
+      store_planes32(t_addr + 16u * hf, t_addr + 32u + 16u * hf, t_addr + 64u + 16u * hf, v);
     } else {
+      uint32_t v[16];
 #pragma unroll
       for (int c = 0; c < 16; c += 4) {   // bf16 head sizes are multiples of 8
         uint4 x = make_uint4(0u, 0u, 0u, 0u);
         if (live && 32 * hf + 2 * c < width) x = __ldg((const uint4*)((const uint16_t*)src + 32 * hf + 2 * c));
-        const uint32_t w[4] = {x.x, x.y, x.z, x.w};
-#pragma unroll
-        for (int e = 0; e < 4; ++e) {
-          v[hf][2 * (c + e)] = w[e] << 16;
-          v[hf][2 * (c + e) + 1] = w[e] & 0xffff0000u;
-        }
+        v[c] = x.x; v[c + 1] = x.y; v[c + 2] = x.z; v[c + 3] = x.w;
       }
+#pragma unroll
+      for (int c = 0; c < 16; ++c) odd |= not_finite(v[c]) | not_finite(v[c] << 16);
+      tc_st_32x32b_x16(t_addr + 16u * hf, v);
     }
   }
-  uint32_t m = 0u;
-#pragma unroll
-  for (int c = 0; c < 64; ++c) m = max(m, v[c >> 5][c & 31] & 0x7fffffffu);
-  sh = shift_of(m);
-  const bool bad = not_finite(m) || sh < -limit;
-  sh = sh == SH_ZERO || bad ? 0 : min(sh, limit);   // (a row far below the others: its elements count as faint ones)
-  const float sc = pow2(sh);
-  int faint = 0;
-#pragma unroll
-  for (int hf = 0; hf < 2; ++hf) {
-#pragma unroll
-    for (int c = 0; c < 32; ++c) {
-      const float x = __uint_as_float(v[hf][c]) * sc;
-      faint += (x != 0.0f && fabsf(x) < faint_line<NP>()) ? 1 : 0;
-      v[hf][c] = __float_as_uint(x);
-    }
-    if (NP == 2) {
-      store_planes32(t_addr + 16u * hf, t_addr + 32u + 16u * hf, v[hf]);
-    } else {
-      uint32_t h[16];
-#pragma unroll
-      for (int e = 0; e < 16; ++e) h[e] = half2_bits(__uint_as_float(v[hf][2 * e]), __uint_as_float(v[hf][2 * e + 1]));
-      tc_st_32x32b_x16(t_addr + 16u * hf, h);
-    }
-  }
-  return bad || faint > 1;
+  return odd;
 }
 
-// 32 columns (from c0) of an output row, scaled; Float32, or bf16 rounded to nearest
-template <bool BF16>
-__device__ __forceinline__ void store_row32(void* dst, int c0, int width, bool vec, const float* v, float sc) {
-  if (BF16) {
-#pragma unroll
-    for (int c = 0; c < 32; c += 8)
-      if (c0 + c < width)
-        *(uint4*)((uint16_t*)dst + c0 + c) = make_uint4(pack2(v[c] * sc, v[c + 1] * sc), pack2(v[c + 2] * sc, v[c + 3] * sc),
-                                                        pack2(v[c + 4] * sc, v[c + 5] * sc), pack2(v[c + 6] * sc, v[c + 7] * sc));
-  } else if (vec) {
-#pragma unroll
-    for (int c = 0; c < 32; c += 4)
-      if (c0 + c < width) *(float4*)((float*)dst + c0 + c) = make_float4(v[c] * sc, v[c + 1] * sc, v[c + 2] * sc, v[c + 3] * sc);
-  } else {
-#pragma unroll
-    for (int c = 0; c < 32; ++c)
-      if (c0 + c < width) ((float*)dst)[c0 + c] = v[c] * sc;
-  }
-}
+// The plane products of A (NA planes) and B (NB planes) from the smallest to the largest: 3 x 3 leaves out the three below
+// 2^-24 of the whole.
+template <int NA, int NB>
+struct Prod {
+  static constexpr int N = NA == 3 && NB == 3 ? 6 : NA == 3 ? 3 : 1;
+  static __device__ __forceinline__ constexpr int a(int i) { return N == 6 ? (i == 0 ? 2 : i == 2 || i == 3 ? 1 : 0) : N == 3 ? 2 - i : 0; }
+  static __device__ __forceinline__ constexpr int b(int i) { return N == 6 ? (i == 1 ? 2 : i == 2 || i == 4 ? 1 : 0) : 0; }
+};
 
-// instruction descriptors: D = F32, A = B = F16, M = 128; B K-major (n columns = rows of the tile) or MN-major
-__device__ __forceinline__ uint32_t idesc_f16(int n, bool b_mn) {
-  return (1u << 4) | ((b_mn ? 1u : 0u) << 16) | ((uint32_t)(n >> 3) << 17) | ((uint32_t)(QT >> 4) << 24);
+// instruction descriptors: D = F32, A = B = BF16, M = 128; B K-major (n columns = rows of the tile) or MN-major
+__device__ __forceinline__ uint32_t idesc_bf16(int n, bool b_mn) {
+  return (1u << 4) | (1u << 7) | (1u << 10) | ((b_mn ? 1u : 0u) << 16) | ((uint32_t)(n >> 3) << 17) | ((uint32_t)(QT >> 4) << 24);
 }
-// operand tiles at 1024-byte boundaries: K-major (one k-step of 16 values = 32 bytes) and MN-major (16 rows of 128 bytes)
-__device__ __forceinline__ uint64_t desc_k(uint32_t saddr) { return make_smem_desc(saddr, 16, 1024, LAYOUT_SW128); }
-__device__ __forceinline__ uint64_t desc_mn(uint32_t saddr) { return make_smem_desc(saddr, KT * 128, 1024, LAYOUT_SW128); }
-
-// The plane products: the cross terms (2^11 too large), then the product of the upper planes over the sum of those times 2^-11.  (The
-// product of the lower planes is below 2^-24 of the whole.)
-//
 // D = A B', A = NP planes in tensor memory (32 columns each), B = NP K-major planes; nks steps of 16 features
 template <int NP>
 __device__ __forceinline__ void mma_rows_t(uint32_t d, uint32_t a_tmem, uint32_t b_smem, int nks) {
   const uint64_t b0 = desc_k(b_smem);
-  const uint32_t idesc = idesc_f16(KT, false), hi = (uint32_t)(b0 >> 32), b = (uint32_t)b0;
-  if (NP == 2) {
+  const uint32_t idesc = idesc_bf16(KT, false), hi = (uint32_t)(b0 >> 32);
+  using P = Prod<NP, NP>;
 #pragma unroll
-    for (int i = 0; i < 2; ++i)
+  for (int i = 0; i < P::N; ++i)
 #pragma unroll
-      for (int ks = 0; ks < 4; ++ks)
-        if (ks < nks)
-          tc_mma_ta(d, a_tmem + (uint32_t)(32 * (1 - i) + 8 * ks), b + (uint32_t)((i * TILE + ks * 32) >> 4), hi, idesc, (i > 0 || ks > 0) ? 1u : 0u);
-  }
-#pragma unroll
-  for (int ks = 0; ks < 4; ++ks)
-    if (ks < nks) {
-      if (NP == 2 && ks == 0) tc_mma_ta_down(d, a_tmem, b, hi, idesc);
-      else tc_mma_ta(d, a_tmem + (uint32_t)(8 * ks), b + (uint32_t)((ks * 32) >> 4), hi, idesc, ks > 0 ? 1u : 0u);
-    }
+    for (int ks = 0; ks < 4; ++ks)
+      if (ks < nks)
+        tc_mma_ta(d, a_tmem + (uint32_t)(32 * P::a(i) + 8 * ks), (uint32_t)b0 + (uint32_t)((P::b(i) * TILE + ks * 32) >> 4), hi, idesc,
+                       (i > 0 || ks > 0) ? 1u : 0u);
 }
 // the same with A in shared memory: planes of 128 rows, 2 * TILE apart, all four steps (head sizes are zero-padded)
 template <int NP>
 __device__ __forceinline__ void mma_rows_s(uint32_t d, uint32_t a_smem, uint32_t b_smem) {
   const uint64_t a0 = desc_k(a_smem), b0 = desc_k(b_smem);
-  const uint32_t idesc = idesc_f16(KT, false), hi = (uint32_t)(a0 >> 32), a = (uint32_t)a0, b = (uint32_t)b0;
-  if (NP == 2) {
+  const uint32_t idesc = idesc_bf16(KT, false), hi = (uint32_t)(a0 >> 32);
+  using P = Prod<NP, NP>;
 #pragma unroll
-    for (int i = 0; i < 2; ++i)
-#pragma unroll
-      for (int ks = 0; ks < 4; ++ks)
-        tc_mma_sa(d, a + (uint32_t)(((1 - i) * 2 * TILE + ks * 32) >> 4), b + (uint32_t)((i * TILE + ks * 32) >> 4), hi, idesc, (i > 0 || ks > 0) ? 1u : 0u);
-  }
-#pragma unroll
-  for (int ks = 0; ks < 4; ++ks) {
-    if (NP == 2 && ks == 0) tc_mma_sa_down(d, a, b, hi, idesc);
-    else tc_mma_sa(d, a + (uint32_t)((ks * 32) >> 4), b + (uint32_t)((ks * 32) >> 4), hi, idesc, ks > 0 ? 1u : 0u);
-  }
-}
-// A = two planes of 64 values in tensor memory that the compute warps stored in halves of 32 values (the upper plane at t + 32 half,
-// the lower one sixteen columns behind it), B = NP MN-major planes whose K rows are the tile's rows; n columns (features, a multiple
-// of 16).  D = A B; or, with sums that go on over the blocks, D += upper A upper B and X += the cross terms, 2^11 too large.
-__device__ __forceinline__ uint32_t plane_step(uint32_t t, int lower, int ks) { return t + (uint32_t)(32 * (ks >> 1) + 16 * lower + 8 * (ks & 1)); }
-template <int NP>
-__device__ __forceinline__ void mma_planes(uint32_t d, uint32_t t, uint32_t b_smem, int n) {
-  const uint64_t b0 = desc_mn(b_smem);
-  const uint32_t idesc = idesc_f16(n, true), hi = (uint32_t)(b0 >> 32), b = (uint32_t)b0;
-#pragma unroll
-  for (int i = 0; i < NP; ++i)
+  for (int i = 0; i < P::N; ++i)
 #pragma unroll
     for (int ks = 0; ks < 4; ++ks)
-      tc_mma_ta(d, plane_step(t, 1 - i, ks), b + (uint32_t)((i * TILE + ks * 2048) >> 4), hi, idesc, (i > 0 || ks > 0) ? 1u : 0u);
-#pragma unroll
-  for (int ks = 0; ks < 4; ++ks) {
-    if (ks == 0) tc_mma_ta_down(d, plane_step(t, 0, 0), b, hi, idesc);
-    else tc_mma_ta(d, plane_step(t, 0, ks), b + (uint32_t)((ks * 2048) >> 4), hi, idesc, 1u);
-  }
+      tc_mma_sa(d, (uint32_t)a0 + (uint32_t)((P::a(i) * 2 * TILE + ks * 32) >> 4), (uint32_t)b0 + (uint32_t)((P::b(i) * TILE + ks * 32) >> 4),
+                     hi, idesc, (i > 0 || ks > 0) ? 1u : 0u);
 }
+// D (+)= A B with A = three planes of 64 values in tensor memory that the compute warps stored in halves of 32 values:
+// plane 0 at t01 + 32 half, plane 1 sixteen columns behind it, plane 2 at t2 + hstep2 half; B = NP MN-major planes whose K
+// rows are the tile's rows; n columns (features, a multiple of 16)
 template <int NP>
-__device__ __forceinline__ void mma_planes_sum(uint32_t d, uint32_t x, uint32_t t, uint32_t b_smem, int n, bool go_on) {
+__device__ __forceinline__ void mma_planes(uint32_t d, uint32_t t01, uint32_t t2, uint32_t hstep2, uint32_t b_smem, int n, bool accumulate) {
   const uint64_t b0 = desc_mn(b_smem);
-  const uint32_t idesc = idesc_f16(n, true), hi = (uint32_t)(b0 >> 32), b = (uint32_t)b0;
+  const uint32_t idesc = idesc_bf16(n, true), hi = (uint32_t)(b0 >> 32);
+  using P = Prod<3, NP>;
 #pragma unroll
-  for (int i = 0; i < NP; ++i)
+  for (int i = 0; i < P::N; ++i)
 #pragma unroll
-    for (int ks = 0; ks < 4; ++ks)
-      tc_mma_ta(x, plane_step(t, 1 - i, ks), b + (uint32_t)((i * TILE + ks * 2048) >> 4), hi, idesc, (go_on || i > 0 || ks > 0) ? 1u : 0u);
-#pragma unroll
-  for (int ks = 0; ks < 4; ++ks)
-    tc_mma_ta(d, plane_step(t, 0, ks), b + (uint32_t)((ks * 2048) >> 4), hi, idesc, (go_on || ks > 0) ? 1u : 0u);
+    for (int ks = 0; ks < 4; ++ks) {
+      const uint32_t hf = (uint32_t)(ks >> 1), in = (uint32_t)(8 * (ks & 1));
+      const uint32_t a = P::a(i) == 2 ? t2 + hstep2 * hf + in : t01 + 32u * hf + 16u * (uint32_t)P::a(i) + in;
+      tc_mma_ta(d, a, (uint32_t)b0 + (uint32_t)((P::b(i) * TILE + ks * 2048) >> 4), hi, idesc, (accumulate || i > 0 || ks > 0) ? 1u : 0u);
+    }
 }
 
 // -------------------------------------------------------------------------------------------- plane images ---
-// One 64 x 64 tile of one (batch, head): rows of Float32 or bf16 values, scaled by a power of two per tile -> NP half-precision planes, each
-// the shared-memory image of the tile (row r at 128 r, its 16-byte chunks permuted by r & 7); rows past the end and features past
-// the head size are 0.  For dO the same pass forms what the softmax backward needs per query: {log2(e) lse, delta = sum_c dO_c O_c};
-// queries past the end get {inf, 0}, which makes their weights 0.
-// shifts: [batch head][job][tile].  A byte of `odd` is set where the planes cannot hold the tile: a value that is not finite, a largest value out of the
-// range of the scales, or two elements and more so far below the largest (faint_line) that their bits are lost; they may be
-// all that counts, where their factors are as far above the others.  The FMA kernels compute the heads of such tiles.
-// Bound by memory: 4 bytes in, 4 out per value (Float32).
+// One 64 x 64 tile of one (batch, head): rows of Float32 or bf16 values -> NP bf16 planes, each the shared-memory image of
+// the tile (row r at 128 r, its 16-byte chunks permuted by r & 7); rows past the end and features past the head size are 0.
+// For dO the same pass forms what the softmax backward needs per query: {log2(e) lse, delta = sum_c dO_c O_c}; queries past
+// the end get {inf, 0}, which makes their weights 0.
+// Bound by memory: 4 bytes in, 6 out per value (Float32).
 struct SplitJob {
   const void* src;
   uint8_t* dst;
   int64_t L, E;
-  int width, tiles, limit;
+  int width, tiles;
 };
 struct SplitArgs {
   SplitJob job[4];
   const float* o;       // for the job of index 3 (dO)
   const float* lse;
   float2* rv;
-  int16_t* shifts;      // [batch head][job][max_tiles]
-  uint8_t* odd;         // the same, odd_n per (batch, head)
-  int H, vec, jobs, max_tiles, odd_n;
+  uint8_t* odd;         // [job][max_tiles] bytes, of odd_n per (batch, head): a value of the tile is not finite
+  int H, vec, max_tiles, odd_n;
 };
 
 template <int NP>
 __global__ void __launch_bounds__(256) attn_split_kernel(SplitArgs A) {
   fb_after_previous();
-  __shared__ uint32_t top[8];
   const SplitJob J = A.job[blockIdx.z];
   if ((int)blockIdx.x >= J.tiles) return;
   const int64_t bh = blockIdx.y;
@@ -373,39 +159,47 @@ __global__ void __launch_bounds__(256) attn_split_kernel(SplitArgs A) {
   uint8_t* dst = J.dst + (bh * J.tiles + blockIdx.x) * (int64_t)(NP * TILE);
   const int ch = threadIdx.x & 7;
   const bool is_do = blockIdx.z == 3;
-  float x[2][8];
-  uint32_t m = 0u;
+  int odd = 0;
 #pragma unroll
   for (int it = 0; it < 2; ++it) {
     const int r = (threadIdx.x >> 3) + 32 * it;
     const int64_t row = (int64_t)blockIdx.x * KT + r;
     const bool live = row < J.L;
     const int64_t off = (b * J.L + row) * J.E + (int64_t)h * J.width;
-    if (NP == 2) {
+    uint8_t* out = dst + r * 128 + ((ch ^ (r & 7)) << 4);
+    float x[8];
+    if (NP == 3) {
       const float* s = (const float*)J.src + off;
       if (A.vec) {
 #pragma unroll
         for (int e = 0; e < 8; e += 4) {
           float4 t = make_float4(0.f, 0.f, 0.f, 0.f);
           if (live && 8 * ch + e < J.width) t = __ldg((const float4*)(s + 8 * ch + e));
-          x[it][e] = t.x; x[it][e + 1] = t.y; x[it][e + 2] = t.z; x[it][e + 3] = t.w;
+          x[e] = t.x; x[e + 1] = t.y; x[e + 2] = t.z; x[e + 3] = t.w;
         }
       } else {
 #pragma unroll
-        for (int e = 0; e < 8; ++e) x[it][e] = (live && 8 * ch + e < J.width) ? __ldg(s + 8 * ch + e) : 0.0f;
+        for (int e = 0; e < 8; ++e) x[e] = (live && 8 * ch + e < J.width) ? __ldg(s + 8 * ch + e) : 0.0f;
       }
+      uint32_t p0[4], p1[4], p2[4];
+#pragma unroll
+      for (int e = 0; e < 4; ++e) split3(x[2 * e], x[2 * e + 1], p0[e], p1[e], p2[e]);
+      *(uint4*)out = make_uint4(p0[0], p0[1], p0[2], p0[3]);
+      *(uint4*)(out + TILE) = make_uint4(p1[0], p1[1], p1[2], p1[3]);
+      *(uint4*)(out + 2 * TILE) = make_uint4(p2[0], p2[1], p2[2], p2[3]);
     } else {
       uint4 t = make_uint4(0u, 0u, 0u, 0u);
       if (live && 8 * ch < J.width) t = __ldg((const uint4*)((const uint16_t*)J.src + off + 8 * ch));
+      *(uint4*)out = t;
       const uint32_t w[4] = {t.x, t.y, t.z, t.w};
 #pragma unroll
       for (int e = 0; e < 4; ++e) {
-        x[it][2 * e] = __uint_as_float(w[e] << 16);
-        x[it][2 * e + 1] = __uint_as_float(w[e] & 0xffff0000u);
+        x[2 * e] = __uint_as_float(w[e] << 16);
+        x[2 * e + 1] = __uint_as_float(w[e] & 0xffff0000u);
       }
     }
 #pragma unroll
-    for (int e = 0; e < 8; ++e) m = max(m, __float_as_uint(x[it][e]) & 0x7fffffffu);
+    for (int e = 0; e < 8; ++e) odd |= not_finite(__float_as_uint(x[e])) ? 1 : 0;
     if (is_do) {
       float s = 0.0f;
 #pragma unroll
@@ -414,9 +208,9 @@ __global__ void __launch_bounds__(256) attn_split_kernel(SplitArgs A) {
         const float* po = A.o + off + 8 * ch + e;
         if (A.vec) {
           const float4 t = __ldg((const float4*)po);
-          s = fmaf(x[it][e], t.x, s); s = fmaf(x[it][e + 1], t.y, s); s = fmaf(x[it][e + 2], t.z, s); s = fmaf(x[it][e + 3], t.w, s);
+          s = fmaf(x[e], t.x, s); s = fmaf(x[e + 1], t.y, s); s = fmaf(x[e + 2], t.z, s); s = fmaf(x[e + 3], t.w, s);
         } else {
-          for (int u = 0; u < 4 && 8 * ch + e + u < J.width; ++u) s = fmaf(x[it][e + u], __ldg(po + u), s);
+          for (int u = 0; u < 4 && 8 * ch + e + u < J.width; ++u) s = fmaf(x[e + u], __ldg(po + u), s);
         }
       }
       s += __shfl_xor_sync(0xffffffffu, s, 1);
@@ -425,69 +219,21 @@ __global__ void __launch_bounds__(256) attn_split_kernel(SplitArgs A) {
       if (ch == 0) A.rv[bh * ((int64_t)J.tiles * KT) + row] = live ? make_float2(A.lse[bh * J.L + row] * LOG2E, s) : make_float2(INFINITY, 0.0f);
     }
   }
-  m = __reduce_max_sync(0xffffffffu, m);
-  if ((threadIdx.x & 31) == 0) top[threadIdx.x >> 5] = m;
-  __syncthreads();
-#pragma unroll
-  for (int w = 0; w < 8; ++w) m = max(m, top[w]);
-  int sh = shift_of(m);
-  const bool bad = not_finite(m) || (sh != SH_ZERO && (sh > J.limit || sh < -J.limit));
-  const float sc = pow2(sh == SH_ZERO || bad ? 0 : sh);
-  int faint = 0;
-#pragma unroll
-  for (int it = 0; it < 2; ++it) {
-    const int r = (threadIdx.x >> 3) + 32 * it;
-    uint8_t* out = dst + r * 128 + ((ch ^ (r & 7)) << 4);
-#pragma unroll
-    for (int e = 0; e < 8; ++e) {
-      x[it][e] *= sc;
-      faint += (x[it][e] != 0.0f && fabsf(x[it][e]) < faint_line<NP>()) ? 1 : 0;
-    }
-    uint32_t p0[4], p1[4];
-#pragma unroll
-    for (int e = 0; e < 4; ++e) split2(x[it][2 * e], x[it][2 * e + 1], p0[e], p1[e]);
-    *(uint4*)out = make_uint4(p0[0], p0[1], p0[2], p0[3]);
-    if (NP == 2) *(uint4*)(out + TILE) = make_uint4(p1[0], p1[1], p1[2], p1[3]);
-  }
-  int some = __syncthreads_count(faint > 0);
-  if (some == 1) some += __syncthreads_or(faint > 1);
-  if (threadIdx.x == 0) {
-    const int at = (int)blockIdx.z * A.max_tiles + (int)blockIdx.x;
-    A.shifts[bh * A.jobs * A.max_tiles + at] = (int16_t)(bad ? 0 : sh);
-    A.odd[bh * A.odd_n + at] = bad || some > 1 ? 1 : 0;
-  }
-}
-
-// ---------------------------------------------------------------------------------- what the kernels share ---
-struct Shared {
-  uint8_t* smem;
-  uint32_t sb;       // its shared-space address (1024-byte aligned)
-};
-__device__ __forceinline__ Shared aligned_smem(uint8_t* raw) {
-  Shared s;
-  s.smem = (uint8_t*)(((uintptr_t)raw + 1023) & ~(uintptr_t)1023);
-  s.sb = smem_u32(s.smem);
-  return s;
-}
-__device__ __forceinline__ void tmem_alloc(volatile uint32_t* slot, uint32_t cols) {
-  asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32((const void*)slot)), "r"(cols) : "memory");
-  asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
-}
-__device__ __forceinline__ void tmem_free(uint32_t base, uint32_t cols) {
-  asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(base), "r"(cols) : "memory");
+  odd = __syncthreads_or(odd);
+  if (threadIdx.x == 0) A.odd[bh * A.odd_n + (int)blockIdx.z * A.max_tiles + (int)blockIdx.x] = odd ? 1 : 0;
 }
 
 // ------------------------------------------------------------------------------------------------------ forward ---
 // One CTA owns 128 queries of one (batch, head); warp 0 copies K and V tiles into a ring of slots (K0 V0 K1 V1 ...),
 // warp 1 issues the MMAs, warps 2-5 are the softmax (thread = query).  S = Q K' lands in 64 columns, the weights replace it
-// as two planes, P V lands in 64 more columns and is added to the thread's registers with round-to-nearest adds.
+// as three planes (96 columns), P V lands in 64 more and is added to the thread's registers with round-to-nearest adds.
 // Within a CTA these steps follow one another; what keeps the tensor pipe busy is the SECOND CTA on the SM: 256 of the 512
 // TMEM columns, half of the registers and of shared memory each.
-//   TMEM columns: Q planes 0..63, S -> P planes 64..127, P V 128..191
+//   TMEM columns: Q planes 0..95, S -> P planes 96..191, P V 192..255
 constexpr int FWD_THREADS = 192;
 template <int NP>
 struct FwdCfg {
-  static constexpr int SLOTS = NP == 2 ? 6 : 8;
+  static constexpr int SLOTS = NP == 3 ? 4 : 8;
   static constexpr int SLOT_BYTES = NP * TILE;
   static constexpr int BAR = SLOTS * SLOT_BYTES;
   static constexpr int SMEM = BAR + 256 + 1024;
@@ -496,8 +242,8 @@ struct FwdCfg {
 template <int NP>
 __global__ void __launch_bounds__(FWD_THREADS, 2)
 attn_fwd_tc_kernel(const void* __restrict__ qmat, const uint8_t* __restrict__ kimg, const uint8_t* __restrict__ vimg,
-                   const int16_t* __restrict__ shifts, float* __restrict__ o, uint16_t* __restrict__ o16, float* __restrict__ lse,
-                   uint8_t* __restrict__ odd_q, int odd_n, AtcDims D, int32_t* __restrict__ dev_err) {
+                   float* __restrict__ o, uint16_t* __restrict__ o16, float* __restrict__ lse, uint8_t* __restrict__ odd_q, int odd_n,
+                   AtcDims D, int32_t* __restrict__ dev_err) {
   fb_after_previous();
   using cfg = FwdCfg<NP>;
   constexpr int S = cfg::SLOTS;
@@ -540,7 +286,7 @@ attn_fwd_tc_kernel(const void* __restrict__ qmat, const uint8_t* __restrict__ ki
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem = __reduce_or_sync(0xffffffffu, *s_tmem);
-  constexpr uint32_t T_R = 64, T_O = 128;
+  constexpr uint32_t T_R = 96, T_O = 192;
 
   if (warp == 0) {
     // ---------------------------------------------------------------- producer ---
@@ -573,7 +319,7 @@ attn_fwd_tc_kernel(const void* __restrict__ qmat, const uint8_t* __restrict__ ki
         ok = warp_wait(bar(B_FULL + s), (uint32_t)(n / S) & 1u, s_abort) && warp_wait(bar(B_PREADY), (uint32_t)j & 1u, s_abort);
         if (!ok) break;
         tc_fence_after();
-        mma_planes<NP>(tmem + T_O, tmem + T_R, sb + (uint32_t)(s * cfg::SLOT_BYTES), nv);
+        mma_planes<NP>(tmem + T_O, tmem + T_R, tmem + T_R + 64u, 16u, sb + (uint32_t)(s * cfg::SLOT_BYTES), nv, false);
         tc_commit(bar(B_OFULL));
         tc_commit(bar(B_FREE + s));
         // the next scores go where the weights are: the tensor pipe runs in order
@@ -586,19 +332,15 @@ attn_fwd_tc_kernel(const void* __restrict__ qmat, const uint8_t* __restrict__ ki
     const int64_t gi = i0 + 32 * q + lane;
     const bool live = gi < D.Lq;
     const uint32_t t_row = tmem + ((uint32_t)(32 * q) << 16);
-    const int64_t el = NP == 2 ? 4 : 2;
-    int sq;
-    const bool odd = row_to_tmem<NP>((const uint8_t*)qmat + el * ((b * D.Lq + gi) * D.E + (int64_t)h * D.d), D.d, live, D.vec != 0, t_row, SH_QK, sq);
+    const int64_t el = NP == 3 ? 4 : 2;
+    const bool odd = row_to_tmem<NP>((const uint8_t*)qmat + el * ((b * D.Lq + gi) * D.E + (int64_t)h * D.d), D.d, live, D.vec != 0, t_row);
     const bool any = __any_sync(0xffffffffu, odd);
     if (lane == 0) odd_q[bh * odd_n + (int)(i0 / QT) * 4 + q] = any ? 1 : 0;
     tc_wait_st();
     tc_fence_before();
     __syncwarp();
     if (lane == 0) mbar_arrive(bar(B_QREADY));
-    const int16_t* sk = shifts + bh * 2 * D.ktiles;   // of the K tiles, then of the V tiles
-    auto shift_at = [&](int i) { const int v = __ldg(sk + i); return v == SH_ZERO ? 0 : v; };
-    int sk_j = shift_at(0), sv_j = shift_at(D.ktiles);
-    float m = -INFINITY, l = 0.0f, fv = 0.0f;         // fv: the scale of the weights and of the V tile whose product is on its way
+    float m = -INFINITY, l = 0.0f;
     float acc[HD];
 #pragma unroll
     for (int c = 0; c < HD; ++c) acc[c] = 0.0f;
@@ -612,7 +354,7 @@ attn_fwd_tc_kernel(const void* __restrict__ qmat, const uint8_t* __restrict__ ki
         tc_ld_32x32b_x32(t_row + T_O + 32u * hf, v);
         tc_wait_ld();
 #pragma unroll
-        for (int c = 0; c < 32; ++c) acc[32 * hf + c] = fmaf(__uint_as_float(v[c]), fv, acc[32 * hf + c]);
+        for (int c = 0; c < 32; ++c) acc[32 * hf + c] += __uint_as_float(v[c]);
       }
       return true;
     };
@@ -644,30 +386,25 @@ attn_fwd_tc_kernel(const void* __restrict__ qmat, const uint8_t* __restrict__ ki
         mx0 = fmaxf(mx0, __uint_as_float(s0[c]));
         mx1 = fmaxf(mx1, __uint_as_float(s1[c]));
       }
-      const float sc = D.scale_log2 * pow2(-(sq + sk_j));
-      fv = pow2(-15 - sv_j);
-      if (j + 1 < nkb) {
-        sk_j = shift_at(j + 1);
-        sv_j = shift_at(D.ktiles + j + 1);
-      }
-      const float m_new = fmaxf(m, fmaxf(mx0, mx1) * sc);
+      const float m_new = fmaxf(m, fmaxf(mx0, mx1));
       const float m_use = (m_new == -INFINITY) ? 0.0f : m_new;
-      const float alpha = fast_exp2(m - m_use);   // m = -inf gives 0
+      const float alpha = fast_exp2((m - m_use) * D.scale_log2);   // m = -inf gives 0
+      const float mc = m_use * D.scale_log2;
       float rs0 = 0.0f, rs1 = 0.0f;
 #pragma unroll
       for (int c = 0; c < 32; ++c) {
-        const float p = fast_exp2(fmaf(__uint_as_float(s0[c]), sc, -m_use));
+        const float p = fast_exp2(fmaf(__uint_as_float(s0[c]), D.scale_log2, -mc));
         rs0 += p;
-        s0[c] = __float_as_uint(p * 32768.0f);
+        s0[c] = __float_as_uint(p);
       }
-      store_planes32(t_row + T_R, t_row + T_R + 16u, s0);
+      store_planes32(t_row + T_R, t_row + T_R + 16u, t_row + T_R + 64u, s0);
 #pragma unroll
       for (int c = 0; c < 32; ++c) {
-        const float p = fast_exp2(fmaf(__uint_as_float(s1[c]), sc, -m_use));
+        const float p = fast_exp2(fmaf(__uint_as_float(s1[c]), D.scale_log2, -mc));
         rs1 += p;
-        s1[c] = __float_as_uint(p * 32768.0f);
+        s1[c] = __float_as_uint(p);
       }
-      store_planes32(t_row + T_R + 32u, t_row + T_R + 48u, s1);
+      store_planes32(t_row + T_R + 32u, t_row + T_R + 48u, t_row + T_R + 80u, s1);
       tc_wait_st();
       tc_fence_before();
       __syncwarp();
@@ -688,7 +425,7 @@ attn_fwd_tc_kernel(const void* __restrict__ qmat, const uint8_t* __restrict__ ki
         if (o != nullptr) store_row32<false>(o + off, 32 * hf, D.dv, D.vec != 0, acc + 32 * hf, inv);
         if (NP == 1) store_row32<true>(o16 + off, 32 * hf, D.dv, true, acc + 32 * hf, inv);
       }
-      lse[bh * D.Lq + gi] = (l > 0.0f) ? fmaf(m, LN2_HI, fmaf(m, LN2_LO, logf(l))) : -INFINITY;
+      lse[bh * D.Lq + gi] = (l > 0.0f) ? m * D.scale + logf(l) : -INFINITY;
     }
   }
 
@@ -707,55 +444,11 @@ attn_fwd_tc_kernel(const void* __restrict__ qmat, const uint8_t* __restrict__ ki
 // P = exp(S / sqrt(d) - lse) and put its planes over them, and dQ += dS K with the same K tile read MN-major.  Two S / dP
 // regions and two sets of four compute warps take the blocks in turn: the tensor cores work on block j + 1 and on dQ of
 // block j - 1 while a set is busy with block j.  dQ accumulates in tensor memory over at most 32 blocks (2048 keys: the
-// adds truncate), upper products and cross terms apart.
-//   TMEM columns: Q planes 0..63, dO planes 64..127, two regions of 128 (S -> dS planes, dP) 128..383, dQ 384..447, cross terms 448..511
-//
-// Scales.  With s the shifts, scores come times 2^(sq + sk), dP times 2^(sdo + sv).  dS is made in units of 2^-(sdo + svmin): |dP| and
-// |delta| are sums of at most 64 products below 2^30, so |dS| < 2^37 there, and 2^-22 of it fits a half; a K tile's shift above the
-// least one goes into it too, so that all blocks add up in one scale.
-constexpr int BWD_THREADS = 320;
-constexpr int BWD_MAX_BLOCKS = 32;
-constexpr int SH_SPREAD = 16;   // what the shifts of a head's K, V, Q and dO tiles may differ by, added up: dS then keeps 2^-19 of itself
-
-// The shifts of a head's tiles (those of tiles of zeros, whatever is multiplied with them, are the least ones), their least ones, and
-// whether they spread too far.  All threads; ends with a barrier.
-struct HeadShifts {
-  int16_t tile[4][BWD_MAX_BLOCKS];   // K, V, Q, dO: as far as there is room (of the operand that a kernel walks there is)
-  int least[4], most[4];
-};
-__device__ __forceinline__ bool head_shifts(HeadShifts& S, const int16_t* shifts, int64_t bh, const AtcDims& D) {
-  if (threadIdx.x < 4) {
-    S.least[threadIdx.x] = SH_ZERO;
-    S.most[threadIdx.x] = -SH_ZERO;
-  }
-  __syncthreads();
-  auto each = [&](auto f) {
-    for (int i = threadIdx.x; i < 4 * D.max_tiles; i += (int)blockDim.x) {
-      const int job = i / D.max_tiles, t = i - job * D.max_tiles;
-      if (t < (job < 2 ? D.ktiles : D.qtiles)) f(job, t, (int)__ldg(shifts + bh * 4 * D.max_tiles + i));
-    }
-  };
-  each([&](int job, int, int v) {
-    if (v == SH_ZERO) return;
-    atomicMin(&S.least[job], v);
-    atomicMax(&S.most[job], v);
-  });
-  __syncthreads();
-  each([&](int job, int t, int v) {
-    if (t < BWD_MAX_BLOCKS) S.tile[job][t] = (int16_t)(v == SH_ZERO ? (S.least[job] == SH_ZERO ? 0 : S.least[job]) : v);
-  });
-  int spread = 0;
-#pragma unroll
-  for (int j = 0; j < 4; ++j)
-    if (S.most[j] >= S.least[j]) spread += S.most[j] - S.least[j];
-  __syncthreads();
-  return spread > SH_SPREAD;
-}
-// the least shift of a job (0 where all tiles are zeros)
-__device__ __forceinline__ int least_of(const HeadShifts& S, int job) { return S.least[job] == SH_ZERO ? 0 : S.least[job]; }
+// adds truncate).
+//   TMEM columns: Q planes 0..95, dO planes 96..191, two regions of 128 (S, dP -> dS planes) 192..447, dQ 448..511
 template <int NP>
 struct DqCfg {
-  static constexpr int SLOTS = 6;
+  static constexpr int SLOTS = NP == 3 ? 4 : 6;
   static constexpr int SLOT_BYTES = 2 * NP * TILE;   // K tile, V tile
   static constexpr int BAR = SLOTS * SLOT_BYTES;
   static constexpr int SMEM = BAR + 256 + 1024;
@@ -764,8 +457,8 @@ struct DqCfg {
 template <int NP>
 __global__ void __launch_bounds__(BWD_THREADS, 1)
 attn_bwd_dq_tc_kernel(const void* __restrict__ q, const void* __restrict__ dout, const uint8_t* __restrict__ kimg,
-                      const uint8_t* __restrict__ vimg, const float2* __restrict__ rv, const int16_t* __restrict__ shifts,
-                      uint8_t* __restrict__ odd_spread, int odd_n, void* __restrict__ dq, AtcDims D, int32_t* __restrict__ dev_err) {
+                      const uint8_t* __restrict__ vimg, const float2* __restrict__ rv, void* __restrict__ dq, AtcDims D,
+                      int32_t* __restrict__ dev_err) {
   fb_after_previous();
   using cfg = DqCfg<NP>;
   constexpr int S = cfg::SLOTS;
@@ -778,8 +471,6 @@ attn_bwd_dq_tc_kernel(const void* __restrict__ q, const void* __restrict__ dout,
   volatile int* s_abort = (volatile int*)(s_tmem + 1);
   volatile int* s_skip = (volatile int*)(s_tmem + 2);
 
-  __shared__ HeadShifts hs;
-  __shared__ int16_t row_q[QT], row_d[QT];
   const int warp = uniform_warp(), lane = threadIdx.x & 31;
   const int64_t i0 = (int64_t)(D.causal ? gridDim.x - 1 - blockIdx.x : blockIdx.x) * QT;
   const int h = blockIdx.y;
@@ -804,15 +495,14 @@ attn_bwd_dq_tc_kernel(const void* __restrict__ q, const void* __restrict__ dout,
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     fence_proxy_async();
   }
-  const bool spread = head_shifts(hs, shifts, bh, D);   // (ends with a barrier)
-  if (blockIdx.x == 0 && threadIdx.x == 0) odd_spread[bh * odd_n] = spread ? 1 : 0;
+  __syncthreads();
   if (*s_skip != 0) return;
   if (warp == 1) tmem_alloc(s_tmem, 512u);
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem = __reduce_or_sync(0xffffffffu, *s_tmem);
-  constexpr uint32_t T_DO = 64, T_R = 128, T_DQ = 384, T_DX = 448;
+  constexpr uint32_t T_DO = 96, T_R = 192, T_DQ = 448;
 
   if (warp == 0) {
     // ---------------------------------------------------------------- producer ---
@@ -841,7 +531,7 @@ attn_bwd_dq_tc_kernel(const void* __restrict__ q, const void* __restrict__ dout,
           if (!ok) break;
           tc_fence_after();
           const uint32_t r = tmem + T_R + (uint32_t)(128 * (j & 1));
-          mma_planes_sum<NP>(tmem + T_DQ, tmem + T_DX, r, sb + (uint32_t)((j % S) * cfg::SLOT_BYTES), nd, j > 0);
+          mma_planes<NP>(tmem + T_DQ, r, r + 64u, 32u, sb + (uint32_t)((j % S) * cfg::SLOT_BYTES), nd, j > 0);
           tc_commit(bar(B_FREE + j % S));
           if (j == nkb - 1) tc_commit(bar(B_DONE));
         }
@@ -863,20 +553,15 @@ attn_bwd_dq_tc_kernel(const void* __restrict__ q, const void* __restrict__ dout,
     const int64_t gi = i0 + 32 * qd + lane;
     const bool live = gi < D.Lq;
     const uint32_t t_row = tmem + ((uint32_t)(32 * qd) << 16);
-    const int64_t el = NP == 2 ? 4 : 2;
+    const int64_t el = NP == 3 ? 4 : 2;
     // the first set brings Q into tensor memory, the second dO
-    int sh;
-    if (set == 0) row_to_tmem<NP>((const uint8_t*)q + el * ((b * D.Lq + gi) * D.E + (int64_t)h * D.d), D.d, live, D.vec != 0, t_row, SH_QK, sh);
-    else row_to_tmem<NP>((const uint8_t*)dout + el * ((b * D.Lq + gi) * D.Ev + (int64_t)h * D.dv), D.dv, live, D.vec != 0, t_row + T_DO, SH_DO, sh);
-    (set == 0 ? row_q : row_d)[32 * qd + lane] = (int16_t)sh;
+    if (set == 0) row_to_tmem<NP>((const uint8_t*)q + el * ((b * D.Lq + gi) * D.E + (int64_t)h * D.d), D.d, live, D.vec != 0, t_row);
+    else row_to_tmem<NP>((const uint8_t*)dout + el * ((b * D.Lq + gi) * D.Ev + (int64_t)h * D.dv), D.dv, live, D.vec != 0, t_row + T_DO);
     tc_wait_st();
     tc_fence_before();
     __syncwarp();
     if (lane == 0) mbar_arrive(bar(B_QREADY));
-    asm volatile("bar.sync 1, 256;" ::: "memory");   // (compute warps: the rows' shifts)
-    const int sq = row_q[32 * qd + lane], sdo = row_d[32 * qd + lane], svmin = least_of(hs, 1), skmin = least_of(hs, 0);
     const float2 ld = rv[bh * ((int64_t)D.qtiles * KT) + gi];   // {inf, 0} past the end: the weights become 0
-    const float delta = times_pow2(ld.y, sdo + svmin);
     bool ok = true;
     for (int j = set; j < nkb && ok; j += 2) {
       ok = mbar_wait(bar(B_SFULL + set), (uint32_t)(j >> 1) & 1u, s_abort);
@@ -887,7 +572,6 @@ attn_bwd_dq_tc_kernel(const void* __restrict__ q, const void* __restrict__ dout,
       if (D.causal && gi - j0 + 1 < lim) lim = gi - j0 + 1;
       const int nvalid = lim < 0 ? 0 : (lim > KT ? KT : (int)lim);
       const uint32_t r = t_row + T_R + (uint32_t)(128 * set);
-      const float sc = D.scale_log2 * pow2(-(sq + hs.tile[0][j])), g = pow2(skmin - hs.tile[0][j] - 22), f = pow2(svmin - hs.tile[1][j]) * g, dg = delta * g;
 #pragma unroll
       for (int hf = 0; hf < 2; ++hf) {
         uint32_t sv[32], dp[32];
@@ -897,16 +581,17 @@ attn_bwd_dq_tc_kernel(const void* __restrict__ q, const void* __restrict__ dout,
         if (nvalid >= KT) {
 #pragma unroll
           for (int c = 0; c < 32; ++c)
-            sv[c] = __float_as_uint(fast_exp2(fmaf(__uint_as_float(sv[c]), sc, -ld.x)) * fmaf(__uint_as_float(dp[c]), f, -dg));
+            sv[c] = __float_as_uint(fast_exp2(fmaf(__uint_as_float(sv[c]), D.scale_log2, -ld.x)) * (__uint_as_float(dp[c]) - ld.y));
         } else {
 #pragma unroll
           for (int c = 0; c < 32; ++c) {
-            float p = fast_exp2(fmaf(__uint_as_float(sv[c]), sc, -ld.x));
+            float p = fast_exp2(fmaf(__uint_as_float(sv[c]), D.scale_log2, -ld.x));
             if (c + 32 * hf >= nvalid) p = 0.0f;
-            sv[c] = __float_as_uint(p * fmaf(__uint_as_float(dp[c]), f, -dg));
+            sv[c] = __float_as_uint(p * (__uint_as_float(dp[c]) - ld.y));
           }
         }
-        store_planes32(r + 32u * hf, r + 32u * hf + 16u, sv);   // (columns this thread has read already)
+        // columns this thread has read already: 32 hf .. and 64 + 32 hf ..
+        store_planes32(r + 32u * hf, r + 32u * hf + 16u, r + 64u + 32u * hf, sv);
       }
       tc_wait_st();
       tc_fence_before();
@@ -917,15 +602,11 @@ attn_bwd_dq_tc_kernel(const void* __restrict__ q, const void* __restrict__ dout,
     if (ok) ok = mbar_wait(bar(B_DONE), 0u, s_abort);
     if (ok) {
       tc_fence_after();
-      uint32_t v[32], w[32];
+      uint32_t v[32];
       tc_ld_32x32b_x32(t_row + T_DQ + 32u * set, v);
-      tc_ld_32x32b_x32(t_row + T_DX + 32u * set, w);
       tc_wait_ld();
-      const int e = 22 - sdo - svmin - skmin;
-#pragma unroll
-      for (int c = 0; c < 32; ++c) v[c] = __float_as_uint(times_pow2(fmaf(__uint_as_float(w[c]), 0.00048828125f, __uint_as_float(v[c])) * D.scale, e));
       if (live)
-        store_row32<NP == 1>((uint8_t*)dq + el * ((b * D.Lq + gi) * D.E + (int64_t)h * D.d), 32 * set, D.d, D.vec != 0, (const float*)v, 1.0f);
+        store_row32<NP == 1>((uint8_t*)dq + el * ((b * D.Lq + gi) * D.E + (int64_t)h * D.d), 32 * set, D.d, D.vec != 0, (const float*)v, D.scale);
     }
   }
 
@@ -944,21 +625,14 @@ attn_bwd_dq_tc_kernel(const void* __restrict__ q, const void* __restrict__ dout,
 //   S' = K Q'  and  dP' = V dO'    (B operands: the Q and dO tiles, K-major)
 //   P' = exp(S' / sqrt(d) - lse_q),  dS' = P' (dP' - delta_q)     (compute warps; planes back into tensor memory)
 //   dV += P' dO  and  dK += dS' Q   (B operands: the same Q and dO tiles, MN-major)
-// As in the dQ kernel two regions and two sets of compute warps take the blocks in turn.  The ring of tile slots holds dO0 Q0 dO1 Q1
-// dO2 ...; dV is issued before dK and dP' before S', so that a slot freed by dV of block i is reloaded under dK of block i and dP' of
-// block i + 2.  K and V in tensor memory would leave room for one region only; from shared memory an MMA of 128 x 64 x 16 takes 48
-// clocks, from tensor memory 44.
-//   TMEM columns: two regions of 128 (S' -> P' planes, dP' -> dS' planes) 0..255, dV 256..319, its cross terms 320..383, dK and its
-//   cross terms 384..511
-// Scales as in the dQ kernel: dS' in units of 2^-(sv of the key's tile + sdomin), P' times 2^15; the shifts of the dO and Q tiles above the
-// least ones go into P' and dS'.
+// As in the dQ kernel two regions and two sets of compute warps take the blocks in turn.  The ring of five tile slots
+// holds dO0 Q0 dO1 Q1 dO2 ...; dV is issued before dK and dP' before S', so that a slot freed by dV of block i is
+// reloaded (with Q of block i + 2) under dK of block i and dP' of block i + 2.  K and V in tensor memory would leave room
+// for one region only; from shared memory an MMA of 128 x 64 x 16 takes 48 clocks, from tensor memory 44.
+//   TMEM columns: two regions of 192 (S', dP', 64 more -> P' and dS' planes) 0..383, dV 384..447, dK 448..511
 template <int NP>
 struct KvCfg {
-  // Compute warps per set: four, a thread with a whole row of a block, or eight with half a row each.  With Float32 operands that is 659
-  // -> 579 us (batch 8, 16 heads, 2048 x 2048, causal); with bf16 ones 442 -> 468, and the dQ kernel gains nothing (499 -> 517).
-  static constexpr int HALVES = NP == 2 ? 2 : 1;
-  static constexpr int THREADS = 64 + 256 * HALVES;
-  static constexpr int SLOTS = 8;
+  static constexpr int SLOTS = NP == 3 ? 5 : 8;
   static constexpr int SLOT_BYTES = NP * TILE + 1024;   // a tile and, behind dO, {lse, delta} of its 64 queries
   static constexpr int K_OFF = SLOTS * SLOT_BYTES, V_OFF = K_OFF + NP * 2 * TILE;
   static constexpr int BAR = V_OFF + NP * 2 * TILE;
@@ -966,11 +640,10 @@ struct KvCfg {
 };
 
 template <int NP>
-__global__ void __launch_bounds__(KvCfg<NP>::THREADS, 1)
+__global__ void __launch_bounds__(BWD_THREADS, 1)
 attn_bwd_dkdv_tc_kernel(const uint8_t* __restrict__ qimg, const uint8_t* __restrict__ doimg, const uint8_t* __restrict__ kimg,
-                        const uint8_t* __restrict__ vimg, const float2* __restrict__ rv, const int16_t* __restrict__ shifts,
-                        uint8_t* __restrict__ odd_spread, int odd_n, void* __restrict__ dk, void* __restrict__ dv, AtcDims D,
-                        int32_t* __restrict__ dev_err) {
+                        const uint8_t* __restrict__ vimg, const float2* __restrict__ rv, void* __restrict__ dk, void* __restrict__ dv,
+                        AtcDims D, int32_t* __restrict__ dev_err) {
   fb_after_previous();
   using cfg = KvCfg<NP>;
   constexpr int S = cfg::SLOTS;
@@ -983,7 +656,6 @@ attn_bwd_dkdv_tc_kernel(const uint8_t* __restrict__ qimg, const uint8_t* __restr
   volatile int* s_abort = (volatile int*)(s_tmem + 1);
   volatile int* s_skip = (volatile int*)(s_tmem + 2);
 
-  __shared__ HeadShifts hs;
   const int warp = uniform_warp(), lane = threadIdx.x & 31;
   const int64_t j0 = (int64_t)blockIdx.x * QT;   // first key of this CTA
   const int h = blockIdx.y;
@@ -1000,7 +672,7 @@ attn_bwd_dkdv_tc_kernel(const uint8_t* __restrict__ qimg, const uint8_t* __restr
     mbar_init(bar(B_KV), 1);
     for (int r = 0; r < 2; ++r) {
       mbar_init(bar(B_SFULL + r), 1);
-      mbar_init(bar(B_PREADY + r), 4 * cfg::HALVES);
+      mbar_init(bar(B_PREADY + r), 4);
     }
     mbar_init(bar(B_DONE), 1);
     *s_abort = 0;
@@ -1008,15 +680,14 @@ attn_bwd_dkdv_tc_kernel(const uint8_t* __restrict__ qimg, const uint8_t* __restr
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     fence_proxy_async();
   }
-  const bool spread = head_shifts(hs, shifts, bh, D);   // (ends with a barrier)
-  if (blockIdx.x == 0 && threadIdx.x == 0) odd_spread[bh * odd_n] = spread ? 1 : 0;
+  __syncthreads();
   if (*s_skip != 0) return;
   if (warp == 1) tmem_alloc(s_tmem, 512u);
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem = __reduce_or_sync(0xffffffffu, *s_tmem);
-  constexpr uint32_t T_DV = 256, T_DK = 384;   // (their cross terms 64 columns behind)
+  constexpr uint32_t T_DV = 384, T_DK = 448;
 
   if (warp == 0) {
     // ---------------------------------------------------------------- producer ---
@@ -1055,16 +726,16 @@ attn_bwd_dkdv_tc_kernel(const uint8_t* __restrict__ qimg, const uint8_t* __restr
           ok = warp_wait(bar(B_PREADY + (i & 1)), (uint32_t)(i >> 1) & 1u, s_abort);
           if (!ok) break;
           tc_fence_after();
-          const uint32_t r = tmem + (uint32_t)(128 * (i & 1));
-          mma_planes_sum<NP>(tmem + T_DV, tmem + T_DV + 64u, r, slot(2 * i), nv, i > 0);
+          const uint32_t r = tmem + (uint32_t)(192 * (i & 1));
+          mma_planes<NP>(tmem + T_DV, r, r + 128u, 32u, slot(2 * i), nv, i > 0);
           tc_commit(bar(B_FREE + (2 * i) % S));
-          mma_planes_sum<NP>(tmem + T_DK, tmem + T_DK + 64u, r + 64u, slot(2 * i + 1), nd, i > 0);
+          mma_planes<NP>(tmem + T_DK, r + 64u, r + 144u, 32u, slot(2 * i + 1), nd, i > 0);
           tc_commit(bar(B_FREE + (2 * i + 1) % S));
           if (i == nqb - 1) tc_commit(bar(B_DONE));
         }
         const int t = i + 2;
         if (t < nqb) {
-          const uint32_t r = tmem + (uint32_t)(128 * (t & 1));
+          const uint32_t r = tmem + (uint32_t)(192 * (t & 1));
           ok = full(2 * t);
           if (!ok) break;
           tc_fence_after();
@@ -1079,19 +750,11 @@ attn_bwd_dkdv_tc_kernel(const uint8_t* __restrict__ qimg, const uint8_t* __restr
     }
   } else {
     // ------------------------------------------------------------ compute warps ---
-    constexpr int HV = cfg::HALVES;
-    const int set = (warp - 2) / (4 * HV), half = ((warp - 2) >> 2) % HV, qd = warp & 3;
+    const int set = (warp - 2) >> 2, qd = warp & 3;
     const int64_t kj = j0 + 32 * qd + lane;   // this thread's key
     const bool live = kj < D.Lk;
     const uint32_t t_row = tmem + ((uint32_t)(32 * qd) << 16);
-    const int64_t el = NP == 2 ? 4 : 2;
-    auto own_shift = [&](int job) {   // (of the two key tiles of this CTA; there may be more than BWD_MAX_BLOCKS)
-      const int v = __ldg(shifts + (bh * 4 + job) * D.max_tiles + 2 * (int64_t)blockIdx.x + (qd >> 1));
-      return v == SH_ZERO ? least_of(hs, job) : v;
-    };
-    const int skr = own_shift(0), svr = own_shift(1);
-    const int sqmin = least_of(hs, 2), sdmin = least_of(hs, 3);
-    const float to_units = pow2(svr + sdmin);
+    const int64_t el = NP == 3 ? 4 : 2;
     bool ok = true;
     for (int i = set; i < nqb && ok; i += 2) {
       const int n = 2 * i;
@@ -1104,13 +767,9 @@ attn_bwd_dkdv_tc_kernel(const uint8_t* __restrict__ qimg, const uint8_t* __restr
       int clo = 0;
       if (D.causal && kj - i0b > 0) clo = (kj - i0b) > KT ? KT : (int)(kj - i0b);
       if (!live) clo = KT;
-      const uint32_t r = t_row + (uint32_t)(128 * set);
-      const int sqi = hs.tile[2][ib0 + i], sdi = hs.tile[3][ib0 + i];
-      const float sc = D.scale_log2 * pow2(-(skr + sqi)), pv = pow2(15 + sdmin - sdi), g = pow2(sqmin - sqi - 22), f = pow2(sdmin - sdi) * g,
-                  dg = to_units * g;
+      const uint32_t r = t_row + (uint32_t)(192 * set);
 #pragma unroll
-      for (int it = 0; it < 2 / HV; ++it) {
-        const int hf = HV == 2 ? half : it;
+      for (int hf = 0; hf < 2; ++hf) {
         uint32_t sv[32], dp[32];
         tc_ld_32x32b_x32(r + 32u * hf, sv);
         tc_ld_32x32b_x32(r + 64u + 32u * hf, dp);
@@ -1118,18 +777,18 @@ attn_bwd_dkdv_tc_kernel(const uint8_t* __restrict__ qimg, const uint8_t* __restr
 #pragma unroll
         for (int c = 0; c < 32; c += 2) {
           const float4 w = row[16 * hf + (c >> 1)];
-          float p0 = fast_exp2(fmaf(__uint_as_float(sv[c]), sc, -w.x));
-          float p1 = fast_exp2(fmaf(__uint_as_float(sv[c + 1]), sc, -w.z));
+          float p0 = fast_exp2(fmaf(__uint_as_float(sv[c]), D.scale_log2, -w.x));
+          float p1 = fast_exp2(fmaf(__uint_as_float(sv[c + 1]), D.scale_log2, -w.z));
           if (c + 32 * hf < clo) p0 = 0.0f;
           if (c + 1 + 32 * hf < clo) p1 = 0.0f;
-          sv[c] = __float_as_uint(p0 * pv);
-          sv[c + 1] = __float_as_uint(p1 * pv);
-          dp[c] = __float_as_uint(p0 * fmaf(__uint_as_float(dp[c]), f, -w.y * dg));
-          dp[c + 1] = __float_as_uint(p1 * fmaf(__uint_as_float(dp[c + 1]), f, -w.w * dg));
+          sv[c] = __float_as_uint(p0);
+          sv[c + 1] = __float_as_uint(p1);
+          dp[c] = __float_as_uint(p0 * (__uint_as_float(dp[c]) - w.y));
+          dp[c + 1] = __float_as_uint(p1 * (__uint_as_float(dp[c + 1]) - w.w));
         }
-        // (over columns this thread has read already)
-        store_planes32(r + 32u * hf, r + 32u * hf + 16u, sv);
-        store_planes32(r + 64u + 32u * hf, r + 80u + 32u * hf, dp);
+        // over columns this thread has read already; the third planes lie behind both
+        store_planes32(r + 32u * hf, r + 32u * hf + 16u, r + 128u + 32u * hf, sv);
+        store_planes32(r + 64u + 32u * hf, r + 80u + 32u * hf, r + 144u + 32u * hf, dp);
       }
       tc_wait_st();
       tc_fence_before();
@@ -1143,22 +802,16 @@ attn_bwd_dkdv_tc_kernel(const uint8_t* __restrict__ qimg, const uint8_t* __restr
       uint8_t* drow = set == 0 ? (uint8_t*)dv + el * ((b * D.Lk + kj) * D.Ev + (int64_t)h * D.dv)
                                : (uint8_t*)dk + el * ((b * D.Lk + kj) * D.E + (int64_t)h * D.d);
 #pragma unroll
-      for (int it = 0; it < 2 / HV; ++it) {
-        const int hf = HV == 2 ? half : it;
-        uint32_t v[32], w[32];
+      for (int hf = 0; hf < 2; ++hf) {
+        uint32_t v[32];
         if (nqb > 0) {
           tc_ld_32x32b_x32(t_row + (set == 0 ? T_DV : T_DK) + 32u * hf, v);
-          tc_ld_32x32b_x32(t_row + (set == 0 ? T_DV : T_DK) + 64u + 32u * hf, w);
           tc_wait_ld();
-          const int e = set == 0 ? -15 - sdmin : 22 - svr - sdmin - sqmin;
-#pragma unroll
-          for (int c = 0; c < 32; ++c)
-            v[c] = __float_as_uint(times_pow2(fmaf(__uint_as_float(w[c]), 0.00048828125f, __uint_as_float(v[c])) * (set == 0 ? 1.0f : D.scale), e));
         } else {
 #pragma unroll
           for (int c = 0; c < 32; ++c) v[c] = 0u;
         }
-        if (live) store_row32<NP == 1>(drow, 32 * hf, set == 0 ? D.dv : D.d, D.vec != 0, (const float*)v, 1.0f);
+        if (live) store_row32<NP == 1>(drow, 32 * hf, set == 0 ? D.dv : D.d, D.vec != 0, (const float*)v, set == 0 ? 1.0f : D.scale);
       }
     }
   }
@@ -1172,127 +825,82 @@ attn_bwd_dkdv_tc_kernel(const uint8_t* __restrict__ qimg, const uint8_t* __restr
   if (threadIdx.x == 0 && *s_abort != 0) atomicExch(dev_err, 4004);
 }
 
-// ------------------------------------------------------------------------------------------------------- host side ---
-// FLUXB200_ATTN_TC = 0 keeps attention on the Float32 FMA kernels, FLUXB200_ATTN_BWD_TC = 0 its backward pass.
-bool env_on(const char* name) {
-  const char* e = getenv(name);
-  return !(e != nullptr && e[0] == '0');
-}
-bool attn_tc_enabled() {
-  static const bool on = env_on("FLUXB200_ATTN_TC");
-  return on;
-}
-bool attn_bwd_tc_enabled() {
-  static const bool on = env_on("FLUXB200_ATTN_BWD_TC");
-  return on;
-}
-
-// the plane images of one call take at most this much memory unless one batch entry needs more: a call is cut along the batch
-// otherwise
-constexpr int64_t IMAGE_BYTES = (int64_t)512 << 20;
-
-struct AtcPlan {
-  AtcDims D;
-  int64_t qbytes, kbytes;   // image of one batch entry's Q (dO), K (V)
-  int64_t rvbytes;
-};
-
-bool make_plan(AtcPlan* P, int np, int64_t e_dim, int64_t ev_dim, int64_t lq, int64_t lk, int64_t batch, int nheads, int causal) {
-  if (nheads < 1 || lq < 1 || lk < 1 || batch < 1 || batch > 65535 || nheads > 65535) return false;
-  const int64_t d = e_dim / nheads, dv = ev_dim / nheads;
-  if (d < 1 || dv < 1 || d > HD || dv > HD) return false;
-  if (np == 1 && (d % 8 != 0 || dv % 8 != 0)) return false;
-  if (lq > 0x3fffff00 || lk > 0x3fffff00) return false;
-  AtcDims& D = P->D;
-  D.E = e_dim; D.Ev = ev_dim; D.Lq = lq; D.Lk = lk; D.H = nheads; D.causal = causal ? 1 : 0;
-  D.d = (int)d; D.dv = (int)dv;
-  D.qtiles = (int)((lq + QT - 1) / QT) * 2;
-  D.ktiles = (int)((lk + QT - 1) / QT) * 2;
-  D.max_tiles = D.qtiles > D.ktiles ? D.qtiles : D.ktiles;
-  D.vec = (d % 4 == 0 && dv % 4 == 0) ? 1 : 0;   // with 16-byte aligned arrays every row of a head is 16-byte aligned
-  D.scale = 1.0f / sqrtf((float)d);
-  D.scale_log2 = D.scale * LOG2E;
-  P->qbytes = (int64_t)nheads * D.qtiles * np * TILE;
-  P->kbytes = (int64_t)nheads * D.ktiles * np * TILE;
-  P->rvbytes = (int64_t)nheads * D.qtiles * KT * (int64_t)sizeof(float2);
-  return true;
-}
-
-// Heads that the planes cannot hold (attn_split_kernel) are computed again by the FMA kernels.  The launch that finds nothing costs 4 - 6
-// us (2048 x 2048, 8 heads of 32, batch 2: 114 -> 119 us; the FMA kernel 853).
-template <int NP>
-int32_t fwd_impl(fb_ctx* ctx, cudaStream_t stream, const uint8_t* q, const uint8_t* k, const uint8_t* v, float* o, uint16_t* o16, float* lse,
+// Heads with a value that is not finite are computed again by the FMA kernels.  Planes cannot carry one (the remainder of an infinite value
+// is NaN, and so is an infinite plane times a zero one), while the sums of products give what such a value makes: a key of -inf no weight, a
+// value of inf an infinite output.  The launch that finds nothing costs 4 - 6 us (2048 x 2048, 8 heads of 32, batch 2: 114 -> 119 us; the
+// FMA kernel 853).
+int32_t fwd_bf16(fb_ctx* ctx, cudaStream_t stream, const uint16_t* q, const uint16_t* k, const uint16_t* v, float* o, uint16_t* o16, float* lse,
                  const AtcPlan& P, int64_t batch) {
   const AtcDims& D = P.D;
   // a byte for every K and V tile and every 32 queries of a (batch, head)
   const int odd_n = 2 * D.ktiles + 2 * D.qtiles;
-  const int64_t el = NP == 2 ? 4 : 2, per = 2 * P.kbytes + (int64_t)D.H * (odd_n + 4 * D.ktiles);
+  const int64_t per = 2 * P.kbytes + (int64_t)D.H * odd_n;
   int64_t chunk = IMAGE_BYTES / per;
   chunk = chunk < 1 ? 1 : (chunk > batch ? batch : chunk);
-  const fb_temp images(ctx, stream, (size_t)(chunk * per + 512));
+  const fb_temp images(ctx, stream, (size_t)(chunk * per));
   uint8_t* img = (uint8_t*)images.p;
   if (!img) return FB_ERR_UNSUPPORTED;
-  FB_ONCE(ctx, FB_CUDA(cudaFuncSetAttribute(attn_fwd_tc_kernel<NP>, cudaFuncAttributeMaxDynamicSharedMemorySize, FwdCfg<NP>::SMEM)));
+  FB_ONCE(ctx, FB_CUDA(cudaFuncSetAttribute(attn_fwd_tc_kernel<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, FwdCfg<1>::SMEM)));
   for (int64_t b0 = 0; b0 < batch; b0 += chunk) {
     const int64_t nb = b0 + chunk > batch ? batch - b0 : chunk;
-    int16_t* shifts = (int16_t*)(img + nb * 2 * P.kbytes);
-    uint8_t* odd = (uint8_t*)(shifts + nb * D.H * 2 * D.ktiles);
+    uint8_t* odd = img + nb * 2 * P.kbytes;
+    const uint16_t *qb = q + b0 * D.Lq * D.E, *kb = k + b0 * D.Lk * D.E, *vb = v + b0 * D.Lk * D.Ev;
+    float *ob = o ? o + b0 * D.Lq * D.Ev : nullptr, *lb = lse + b0 * D.H * D.Lq;
+    uint16_t* ob16 = o16 + b0 * D.Lq * D.Ev;
     SplitArgs A = {};
-    A.H = D.H; A.vec = D.vec; A.odd = odd; A.odd_n = odd_n; A.shifts = shifts; A.jobs = 2; A.max_tiles = D.ktiles;
-    A.job[0] = {k + el * b0 * D.Lk * D.E, img, D.Lk, D.E, D.d, D.ktiles, SH_QK};
-    A.job[1] = {v + el * b0 * D.Lk * D.Ev, img + nb * P.kbytes, D.Lk, D.Ev, D.dv, D.ktiles, SH_V};
-    fb_launch(attn_split_kernel<NP>, dim3((unsigned)D.ktiles, (unsigned)(nb * D.H), 2), 256, 0, stream, A);
+    A.H = D.H; A.vec = D.vec; A.odd = odd; A.odd_n = odd_n; A.max_tiles = D.ktiles;
+    A.job[0] = {kb, img, D.Lk, D.E, D.d, D.ktiles};
+    A.job[1] = {vb, img + nb * P.kbytes, D.Lk, D.Ev, D.dv, D.ktiles};
+    fb_launch(attn_split_kernel<1>, dim3((unsigned)D.ktiles, (unsigned)(nb * D.H), 2), 256, 0, stream, A);
     FB_LAUNCH_CHECK();
-    fb_launch(attn_fwd_tc_kernel<NP>, dim3((unsigned)(D.qtiles / 2), (unsigned)D.H, (unsigned)nb), FWD_THREADS, FwdCfg<NP>::SMEM, stream, q + el * b0 * D.Lq * D.E, img, img + nb * P.kbytes, shifts, o ? o + b0 * D.Lq * D.Ev : nullptr, o16 ? o16 + b0 * D.Lq * D.Ev : nullptr,
-        lse + b0 * D.H * D.Lq, odd + 2 * D.ktiles, odd_n, D, ctx->dev_error);
+    fb_launch(attn_fwd_tc_kernel<1>, dim3((unsigned)(D.qtiles / 2), (unsigned)D.H, (unsigned)nb), FWD_THREADS, FwdCfg<1>::SMEM, stream, qb, img, img + nb * P.kbytes, ob, ob16, lb,
+              odd + 2 * D.ktiles, odd_n, D, ctx->dev_error);
     FB_LAUNCH_CHECK();
-    const int32_t st = fb_attn_fwd_redo(ctx, stream, NP == 1, q + el * b0 * D.Lq * D.E, k + el * b0 * D.Lk * D.E, v + el * b0 * D.Lk * D.Ev,
-                                        o ? o + b0 * D.Lq * D.Ev : nullptr, o16 ? o16 + b0 * D.Lq * D.Ev : nullptr, lse + b0 * D.H * D.Lq,
-                                        D.E, D.Ev, D.Lq, D.Lk, nb, D.H, D.causal, odd, odd_n);
+    const int32_t st = fb_attn_fwd_redo(ctx, stream, 1, qb, kb, vb, ob, ob16, lb, D.E, D.Ev, D.Lq, D.Lk, nb, D.H, D.causal, odd, odd_n);
     if (st != FB_OK) return st;
   }
   return FB_OK;
 }
 
-template <int NP>
-int32_t bwd_impl(fb_ctx* ctx, cudaStream_t stream, const uint8_t* q, const uint8_t* k, const uint8_t* v, const float* o, const float* lse,
-                 const uint8_t* dout, uint8_t* dq, uint8_t* dk, uint8_t* dv, const AtcPlan& P, int64_t batch, bool do_kv, bool do_q) {
+int32_t bwd_bf16(fb_ctx* ctx, cudaStream_t stream, const uint16_t* q, const uint16_t* k, const uint16_t* v, const float* o, const float* lse, const uint16_t* dout,
+                 uint16_t* dq, uint16_t* dk, uint16_t* dv, const AtcPlan& P, int64_t batch) {
   const AtcDims& D = P.D;
-  // a byte for every tile of a (batch, head) and one for its shifts
-  const int odd_n = 4 * D.max_tiles + 1;
-  const int64_t el = NP == 2 ? 4 : 2, per = 2 * P.kbytes + 2 * P.qbytes + P.rvbytes + (int64_t)D.H * (odd_n + 8 * D.max_tiles);
+  const int odd_n = 4 * D.max_tiles;   // a byte for every tile of a (batch, head)
+  const int64_t per = 2 * P.kbytes + 2 * P.qbytes + P.rvbytes + (int64_t)D.H * odd_n;
   int64_t chunk = IMAGE_BYTES / per;
   chunk = chunk < 1 ? 1 : (chunk > batch ? batch : chunk);
-  const fb_temp images(ctx, stream, (size_t)(chunk * per + 512));
+  const fb_temp images(ctx, stream, (size_t)(chunk * per));
   uint8_t* img = (uint8_t*)images.p;
   if (!img) return FB_ERR_UNSUPPORTED;
-  FB_ONCE(ctx, FB_CUDA(cudaFuncSetAttribute(attn_bwd_dkdv_tc_kernel<NP>, cudaFuncAttributeMaxDynamicSharedMemorySize, KvCfg<NP>::SMEM)));
-  FB_ONCE(ctx, FB_CUDA(cudaFuncSetAttribute(attn_bwd_dq_tc_kernel<NP>, cudaFuncAttributeMaxDynamicSharedMemorySize, DqCfg<NP>::SMEM)));
+  FB_ONCE(ctx, FB_CUDA(cudaFuncSetAttribute(attn_bwd_dkdv_tc_kernel<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, KvCfg<1>::SMEM)));
+  FB_ONCE(ctx, FB_CUDA(cudaFuncSetAttribute(attn_bwd_dq_tc_kernel<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, DqCfg<1>::SMEM)));
   for (int64_t b0 = 0; b0 < batch; b0 += chunk) {
     const int64_t nb = b0 + chunk > batch ? batch - b0 : chunk;
     uint8_t *ki = img, *vi = ki + nb * P.kbytes, *qi = vi + nb * P.kbytes, *doi = qi + nb * P.qbytes;
     float2* rv = (float2*)(doi + nb * P.qbytes);
-    int16_t* shifts = (int16_t*)((uint8_t*)rv + nb * P.rvbytes);
-    uint8_t* odd = (uint8_t*)(shifts + nb * D.H * 4 * D.max_tiles);
+    uint8_t* odd = (uint8_t*)rv + nb * P.rvbytes;
     const int64_t qoff = b0 * D.Lq * D.E, qvoff = b0 * D.Lq * D.Ev, koff = b0 * D.Lk * D.E, kvoff = b0 * D.Lk * D.Ev;
+    const uint16_t *qb = q + qoff, *kb = k + koff, *vb = v + kvoff, *dob = dout + qvoff;
+    const float* lb = lse + b0 * D.H * D.Lq;
     SplitArgs A = {};
-    A.H = D.H; A.vec = D.vec; A.odd = odd; A.odd_n = odd_n; A.shifts = shifts; A.jobs = 4; A.max_tiles = D.max_tiles;
-    A.job[0] = {k + el * koff, ki, D.Lk, D.E, D.d, D.ktiles, SH_QK};
-    A.job[1] = {v + el * kvoff, vi, D.Lk, D.Ev, D.dv, D.ktiles, SH_V};
-    A.job[2] = {q + el * qoff, qi, D.Lq, D.E, D.d, D.qtiles, SH_QK};
-    A.job[3] = {dout + el * qvoff, doi, D.Lq, D.Ev, D.dv, D.qtiles, SH_DO};
-    A.o = o + qvoff; A.lse = lse + b0 * D.H * D.Lq; A.rv = rv;
+    A.H = D.H; A.vec = D.vec; A.odd = odd; A.odd_n = odd_n; A.max_tiles = D.max_tiles;
+    A.job[0] = {kb, ki, D.Lk, D.E, D.d, D.ktiles};
+    A.job[1] = {vb, vi, D.Lk, D.Ev, D.dv, D.ktiles};
+    A.job[2] = {qb, qi, D.Lq, D.E, D.d, D.qtiles};
+    A.job[3] = {dob, doi, D.Lq, D.Ev, D.dv, D.qtiles};
+    A.o = o + qvoff; A.lse = lb; A.rv = rv;
     // (tiles that one operand has and another has not keep no byte)
     if (D.qtiles != D.ktiles) FB_CUDA(cudaMemsetAsync(odd, 0, (size_t)(nb * D.H * odd_n), stream));
-    fb_launch(attn_split_kernel<NP>, dim3((unsigned)D.max_tiles, (unsigned)(nb * D.H), 4), 256, 0, stream, A);
+    fb_launch(attn_split_kernel<1>, dim3((unsigned)D.max_tiles, (unsigned)(nb * D.H), 4), 256, 0, stream, A);
     FB_LAUNCH_CHECK();
-    if (do_kv) fb_launch(attn_bwd_dkdv_tc_kernel<NP>, dim3((unsigned)(D.ktiles / 2), (unsigned)D.H, (unsigned)nb), KvCfg<NP>::THREADS, KvCfg<NP>::SMEM, stream, qi, doi, ki, vi, rv, shifts, odd + 4 * D.max_tiles, odd_n, dk + el * koff, dv + el * kvoff, D, ctx->dev_error);
+    fb_launch(attn_bwd_dkdv_tc_kernel<1>, dim3((unsigned)(D.ktiles / 2), (unsigned)D.H, (unsigned)nb), BWD_THREADS, KvCfg<1>::SMEM, stream, qi, doi, ki, vi, rv, dk + koff,
+              dv + kvoff, D, ctx->dev_error);
     FB_LAUNCH_CHECK();
-    if (do_q) fb_launch(attn_bwd_dq_tc_kernel<NP>, dim3((unsigned)(D.qtiles / 2), (unsigned)D.H, (unsigned)nb), BWD_THREADS, DqCfg<NP>::SMEM, stream, q + el * qoff, dout + el * qvoff, ki, vi, rv, shifts, odd + 4 * D.max_tiles, odd_n, dq + el * qoff, D, ctx->dev_error);
+    fb_launch(attn_bwd_dq_tc_kernel<1>, dim3((unsigned)(D.qtiles / 2), (unsigned)D.H, (unsigned)nb), BWD_THREADS, DqCfg<1>::SMEM, stream, qb, dob, ki, vi, rv, dq + qoff, D,
+              ctx->dev_error);
     FB_LAUNCH_CHECK();
-    const int32_t st = fb_attn_bwd_redo(ctx, stream, NP == 1, q + el * qoff, k + el * koff, v + el * kvoff, lse + b0 * D.H * D.Lq, (const float*)rv + 1,
-                                        (int64_t)D.qtiles * KT, dout + el * qvoff, do_q ? dq + el * qoff : nullptr, do_kv ? dk + el * koff : nullptr,
-                                        dv + el * kvoff, D.E, D.Ev, D.Lq, D.Lk, nb, D.H, D.causal, odd, odd_n);
+    const int32_t st = fb_attn_bwd_redo(ctx, stream, 1, qb, kb, vb, lb, (const float*)rv + 1, (int64_t)D.qtiles * KT, dob, dq + qoff, dk + koff, dv + kvoff, D.E, D.Ev,
+                                        D.Lq, D.Lk, nb, D.H, D.causal, odd, odd_n);
     if (st != FB_OK) return st;
   }
   return FB_OK;
@@ -1300,42 +908,7 @@ int32_t bwd_impl(fb_ctx* ctx, cudaStream_t stream, const uint8_t* q, const uint8
 
 }  // namespace
 
-// Both return FB_ERR_UNSUPPORTED when the call is not one these kernels take (the caller then uses the FMA kernels).
-int32_t fb_attn_fwd_tc(fb_ctx* ctx, cudaStream_t stream, const float* q, const float* k, const float* v, const uint8_t* mask,
-                       float* o, float* lse, int64_t e_dim, int64_t ev_dim, int64_t lq, int64_t lk, int64_t batch, int nheads,
-                       int causal) {
-  AtcPlan P;
-  if (!attn_tc_enabled() || mask != nullptr || !make_plan(&P, 2, e_dim, ev_dim, lq, lk, batch, nheads, causal)) return FB_ERR_UNSUPPORTED;
-  if (!fb_aligned16(q) || !fb_aligned16(k) || !fb_aligned16(v) || !fb_aligned16(o)) P.D.vec = 0;
-  return fwd_impl<2>(ctx, stream, (const uint8_t*)q, (const uint8_t*)k, (const uint8_t*)v, o, nullptr, lse, P, batch);
-}
-
-// *did_kv, *did_q: which part was done.  dQ, dK and dV accumulate in tensor memory with truncating adds; beyond 2048 keys
-// (queries), for the other head sizes and for unaligned arrays, the FMA kernels are the more accurate ones (8 heads of 64,
-// 512 x 512: dQ 4e-7, dK and dV 6e-7 of the norm in 245 us, here 1.4e-6 and 5e-6 in 87).
-int32_t fb_attn_bwd_tc(fb_ctx* ctx, cudaStream_t stream, const float* q, const float* k, const float* v, const uint8_t* mask, const float* o,
-                       const float* lse, const float* dout, float* dq, float* dk, float* dv, int64_t e_dim, int64_t ev_dim, int64_t lq,
-                       int64_t lk, int64_t batch, int nheads, int causal, bool* did_kv, bool* did_q) {
-  AtcPlan P;
-  *did_kv = *did_q = false;
-  if (!attn_tc_enabled() || !attn_bwd_tc_enabled() || mask != nullptr || !make_plan(&P, 2, e_dim, ev_dim, lq, lk, batch, nheads, causal) ||
-      P.D.d != HD || P.D.dv != HD)
-    return FB_ERR_UNSUPPORTED;
-  // (arrays off the 16-byte boundary have always been the FMA kernels')
-  if (!fb_aligned16(q) || !fb_aligned16(k) || !fb_aligned16(v) || !fb_aligned16(dout)) return FB_ERR_UNSUPPORTED;
-  const bool kv = lq <= BWD_MAX_BLOCKS * KT && fb_aligned16(dk) && fb_aligned16(dv), qq = lk <= BWD_MAX_BLOCKS * KT && fb_aligned16(dq);
-  if (!kv && !qq) return FB_ERR_UNSUPPORTED;
-  if (!fb_aligned16(o)) P.D.vec = 0;
-  const int32_t st = bwd_impl<2>(ctx, stream, (const uint8_t*)q, (const uint8_t*)k, (const uint8_t*)v, o, lse, (const uint8_t*)dout,
-                                 (uint8_t*)dq, (uint8_t*)dk, (uint8_t*)dv, P, batch, kv, qq);
-  if (st == FB_OK) {
-    *did_kv = kv;
-    *did_q = qq;
-  }
-  return st;
-}
-
-// The same for bf16 q, k, v (and dO): one plane each, outputs rounded to bf16 once.  o32 (optional in the forward call) keeps
+// bf16 q, k, v (and dO): one plane each, outputs rounded to bf16 once.  o32 (optional in the forward call) keeps
 // the Float32 output for the backward pass.  FB_ERR_UNSUPPORTED, without a message, for every call these kernels do not
 // take: the caller then casts and takes the Float32 entry points, which also report what is wrong with a bad one.  The
 // backward call takes the head size of the Float32 one, for the same reason.
@@ -1348,7 +921,7 @@ FB_API int32_t fb_attn_fwd_bf16(fb_ctx* ctx, void* stream, const uint16_t* q, co
       !make_plan(&P, 1, e_dim, ev_dim, lq, lk, batch, nheads, causal))
     return FB_ERR_UNSUPPORTED;
   if (!fb_aligned16(q) || !fb_aligned16(k) || !fb_aligned16(v) || !fb_aligned16(o) || !fb_aligned16(o32)) return FB_ERR_UNSUPPORTED;
-  return fwd_impl<1>(ctx, (cudaStream_t)stream, (const uint8_t*)q, (const uint8_t*)k, (const uint8_t*)v, o32, o, lse, P, batch);
+  return fwd_bf16(ctx, (cudaStream_t)stream, q, k, v, o32, o, lse, P, batch);
 }
 
 FB_API int32_t fb_attn_bwd_bf16(fb_ctx* ctx, void* stream, const uint16_t* q, const uint16_t* k, const uint16_t* v, const float* o32,
@@ -1363,6 +936,5 @@ FB_API int32_t fb_attn_bwd_bf16(fb_ctx* ctx, void* stream, const uint16_t* q, co
   if (!fb_aligned16(q) || !fb_aligned16(k) || !fb_aligned16(v) || !fb_aligned16(o32) || !fb_aligned16(dout) || !fb_aligned16(dq) ||
       !fb_aligned16(dk) || !fb_aligned16(dv))
     return FB_ERR_UNSUPPORTED;
-  return bwd_impl<1>(ctx, (cudaStream_t)stream, (const uint8_t*)q, (const uint8_t*)k, (const uint8_t*)v, o32, lse, (const uint8_t*)dout,
-                     (uint8_t*)dq, (uint8_t*)dk, (uint8_t*)dv, P, batch, true, true);
+  return bwd_bf16(ctx, (cudaStream_t)stream, q, k, v, o32, lse, dout, dq, dk, dv, P, batch);
 }

@@ -365,3 +365,29 @@ def test_inputs_of_very_different_magnitudes(kind, heads, lq, lk, batch, causal,
             got, want = got.reshape(-1, 1), want.reshape(-1, 1)
         err = float(((got - want).norm(dim=0) / want.norm(dim=0).clamp_min(1e-300)).max())
         assert err < tol, (name, err)
+
+
+@pytest.mark.parametrize("scores", [16, 24])
+@pytest.mark.parametrize("heads,n,batch,causal", [(2, 512, 1, 1), (3, 1000, 2, 1)])
+def test_bf16_gradients_of_values_with_small_weights(scores, heads, n, batch, causal):
+    """Scores of standard deviation 16 and 24: keys whose largest weight is as small as 2^-80.  Their own rows of dV are as exact as the
+    others': the one rounding to bf16 (2^-9) and as much again for scores of up to 130 and truncated sums."""
+    import fluxb200 as F
+    from fluxb200 import lib
+    g, E, ctx = torch.Generator(device="cuda").manual_seed(n), 64 * heads, F.context()
+    q, k, v, do = ((torch.randn(batch, n, E, generator=g, device="cuda") * s).bfloat16() for s in (scores ** 0.5, scores ** 0.5, 1.0, 1.0))
+    o, lse, out, dq, dk, dv = torch.empty(batch, n, E, device="cuda"), torch.empty(batch * heads * n, device="cuda"), *(torch.empty_like(q) for _ in range(4))
+    p, dims = lambda t: t.data_ptr(), (E, E, n, n, batch, heads, causal)
+    lib.call("fb_attn_fwd_bf16", ctx.handle, ctx.stream, p(q), p(k), p(v), p(o), p(out), p(lse), *dims)
+    lib.call("fb_attn_bwd_bf16", ctx.handle, ctx.stream, p(q), p(k), p(v), p(o), p(lse), p(do), p(dq), p(dk), p(dv), *dims)
+    assert ctx.device_error() == 0
+    ref = _reference(q, k, v, do, 64, 64, heads, causal)
+    split = lambda t: t.double().view(batch, n, heads, 64).transpose(1, 2)
+    s = split(q) @ split(k).transpose(2, 3) / 8
+    if causal:
+        s = s.masked_fill(torch.arange(n, device="cuda")[None, :] > torch.arange(n, device="cuda")[:, None], -np.inf)
+    counts = torch.softmax(s, -1).amax(2) > 2.0 ** -80     # [batch][head][key]
+    assert bool((torch.softmax(s, -1).amax(2)[counts] < 2.0 ** -50).any())
+    got, want = split(dv)[counts], split(ref[3])[counts]
+    err = float(((got - want).norm(dim=1) / want.norm(dim=1)).max())
+    assert err < 4e-3, err
