@@ -531,6 +531,7 @@ rnn_bwd_mma_kernel(const float* __restrict__ Wh, const float* __restrict__ keep,
         }
       } else {
         ahead(ch + nbg < nchunks ? t : t - 1, ch + nbg < nchunks ? ch + nbg : bgrp);
+        if (ci > 0) __syncthreads();   // (no poll, so no barrier yet: the chunk before may still be read from frag, csh and dval)
       }
       float d[NG];
 #pragma unroll
@@ -578,7 +579,7 @@ rnn_bwd_mma_kernel(const float* __restrict__ Wh, const float* __restrict__ keep,
           dval[gb][g * UG + gu] = d[g];
         }
       }
-      if (t > 0) __syncthreads();
+      __syncthreads();   // planes are there for all; in step 0 nothing is, but the next chunk's partial sums go where these have been read
       if (mine) {
         float* row = dg + (int64_t)t * K + (int64_t)b * ldd;
 #pragma unroll

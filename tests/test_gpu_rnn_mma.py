@@ -226,3 +226,64 @@ def test_gradients_that_are_not_finite_stay_in_their_column(cell):
         # (columns that share fragments with it are summed in Float32 instead of planes)
         assert float((res[0] - res[1])[others].abs().max()) < 2e-5 * float(res[0].abs().max())
         assert not bool(torch.isfinite(res[1][4, :T - 1]).any())
+
+
+def _gradients(cell, wi, wh, b, x, dout):
+    import fluxb200 as F
+    from fluxb200 import lib
+    ctx, (B, T, I), H = F.context(0), x.shape, wh.shape[0]
+    p = lambda t: t.data_ptr()
+    cache, o = torch.empty(getattr(lib.raw(), f"fb_{cell}_cache_bytes")(I, H, T, B) // 4, device="cuda"), torch.empty(B, T, H, device="cuda")
+    g = [torch.empty_like(t) for t in (wi, wh, b, x)]
+    if cell == "lstm":
+        lib.call("fb_lstm_fwd", ctx.handle, ctx.stream, p(wi), p(wh), p(b), p(x), None, None, p(o), None, None, p(cache), I, H, T, B)
+        lib.call("fb_lstm_bwd", ctx.handle, ctx.stream, p(wi), p(wh), p(x), None, None, p(o), p(cache), p(dout), None, None, *map(p, g), I, H, T, B)
+    else:
+        lib.call("fb_gru_fwd", ctx.handle, ctx.stream, p(wi), p(wh), p(b), p(x), None, p(o), None, p(cache), I, H, T, B)
+        lib.call("fb_gru_bwd", ctx.handle, ctx.stream, p(wi), p(wh), p(x), None, p(o), p(cache), p(dout), None, *map(p, g), I, H, T, B)
+    assert ctx.device_error() == 0
+    return g
+
+
+@pytest.mark.parametrize("cell", ["lstm", "gru"])
+@pytest.mark.parametrize("H,B,T", [(400, 130, 4), (400, 130, 30), (512, 150, 3), (512, 70, 40)])
+@pytest.mark.parametrize("bad", [float("inf"), float("nan")])
+def test_chunks_of_columns_do_not_meet(cell, H, B, T, bad):
+    """Several chunks of columns per CTA.  A cotangent that is not finite at the last step sends the warps of its chunk through sums of
+    very different length (25 groups of units: warp 0 alone has a fourth one): no column of another chunk changes a bit."""
+    gen = torch.Generator(device="cuda").manual_seed(H + T)
+    new = lambda *s: torch.randn(*s, generator=gen, device="cuda")
+    ng = 4 if cell == "lstm" else 3
+    wi, wh, b, x, dout = new(16, ng * H) * 0.2, new(H, ng * H) / H ** 0.5, new(ng * H) * 0.1, new(B, T, 16), new(B, T, H)
+    want = _gradients(cell, wi, wh, b, x, dout)[3].clone()
+    for col in (0, 17, B - 1):
+        held = dout[col, T - 1].clone()
+        dout[col, T - 1, ::5] = bad
+        got = _gradients(cell, wi, wh, b, x, dout)[3]
+        dout[col, T - 1] = held
+        others = [i for i in range(B) if i // 16 != col // 16]   # (chunks are of 8 or 16 columns)
+        assert torch.equal(got[others], want[others])
+        assert not bool(torch.isfinite(got[col, T - 1]).all())
+
+
+@pytest.mark.parametrize("cell", ["lstm", "gru"])
+@pytest.mark.parametrize("H,B,T", [(400, 130, 2), (400, 130, 5), (512, 150, 3), (496, 700, 4), (512, 70, 2)])
+def test_chunks_of_columns_repeat_their_bits(cell, H, B, T):
+    """The first step, which waits for nothing, and the last, which sends nothing, again and again; infinite weights of one group of units
+    make the warp that owns it slower than the others.  Finite columns against float64: 2e-5 as above."""
+    gen = torch.Generator(device="cuda").manual_seed(H + B)
+    new = lambda *s: torch.randn(*s, generator=gen, device="cuda")
+    ng = 4 if cell == "lstm" else 3
+    wi, wh, b, x, dout = new(12, ng * H) * 0.2, new(H, ng * H) / H ** 0.5, new(ng * H) * 0.1, new(B, T, 12), new(B, T, H)
+    leaf = [t.double().requires_grad_() for t in (wi, wh, b, x)]
+    zero = torch.zeros(B, H, device="cuda", dtype=torch.double)
+    (_reference(cell, *leaf, zero, zero)[0] * dout.double()).sum().backward()
+    first = [t.clone() for t in _gradients(cell, wi, wh, b, x, dout)]
+    for got, want in zip(first, leaf):
+        assert float((got.double() - want.grad).abs().max() / want.grad.abs().max()) < 2e-5
+    for _ in range(8):
+        assert all(torch.equal(a, c) for a, c in zip(_gradients(cell, wi, wh, b, x, dout), first))
+    wh[20, 3] = float("inf")                                  # (the rows of the second group alone: its warp sums in Float32)
+    slow = [t.clone() for t in _gradients(cell, wi, wh, b, x, dout)]
+    for _ in range(8):
+        assert all(torch.equal(torch.nan_to_num(a), torch.nan_to_num(c)) for a, c in zip(_gradients(cell, wi, wh, b, x, dout), slow))
