@@ -102,7 +102,7 @@ class Chain(Layer):
 
     def __call__(self, x):
         layers = self.layers
-        if not Tape.active and len(layers) > 1 and type(x) is B200Array and x.ndim <= 2 and Tape.grad_sink is None:
+        if not Tape.active and len(layers) > 1 and type(x) is B200Array and 1 <= x.ndim <= 2 and Tape.grad_sink is None:
             y = _dense_chain(layers, x)
             if y is not None:
                 return y

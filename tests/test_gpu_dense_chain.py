@@ -92,3 +92,18 @@ def test_captured_and_beside_another_stream():
             z = m(xs[1])
         torch.cuda.synchronize()
         assert torch.equal(y.t, want[0]) and torch.equal(z.t, want[1])
+
+
+@pytest.mark.parametrize("size", [(), (65,), (65, 1), (65, 40), (65, 1, 1), (1, 64)])
+def test_arrays_of_other_shapes_are_refused_by_the_first_layer(size):
+    import fluxb200 as F
+    m = _chain(F, [64, 32, 8], "relu", torch.Generator(device="cuda").manual_seed(0))
+    n = 1
+    for s in size:
+        n *= s
+    x = F.B200Array(torch.randn(n, device="cuda"), size)
+    with pytest.raises(F.DimensionMismatch) as chain:
+        m(x)
+    with pytest.raises(F.DimensionMismatch) as layer:
+        m.layers[0](x)
+    assert str(chain.value) == str(layer.value)
