@@ -156,6 +156,7 @@ __global__ void __launch_bounds__(AT)
 attn_fwd_kernel(const T* __restrict__ q, const T* __restrict__ k, const T* __restrict__ v,
                 const uint8_t* __restrict__ mask, float* __restrict__ o, uint16_t* __restrict__ o16, float* __restrict__ lse, AttnDims D) {
   fb_after_previous();
+  if (REDO) fb_let_next_start();
   constexpr int LD = NC * 64 + 4;
   extern __shared__ float sm[];
   float* Qs = sm;
@@ -307,12 +308,12 @@ __device__ __forceinline__ void recompute_p_ds(const AttnDims& D, const uint8_t*
 }
 
 // ------------------------------------------------------------------------- backward: dK, dV ---
+// The tile `first` of a head, or REDO: the tiles first, + step, ...
 template <int NC, typename T, bool REDO>
-__global__ void __launch_bounds__(AT)
-attn_bwd_dkdv_kernel(const T* __restrict__ q, const T* __restrict__ k, const T* __restrict__ v,
-                     const uint8_t* __restrict__ mask, const float* __restrict__ lse, const float* __restrict__ dlt,
-                     const T* __restrict__ dout, T* __restrict__ dk, T* __restrict__ dv, AttnDims D) {
-  fb_after_previous();
+__device__ __forceinline__ void
+bwd_dkdv(const T* __restrict__ q, const T* __restrict__ k, const T* __restrict__ v,
+         const uint8_t* __restrict__ mask, const float* __restrict__ lse, const float* __restrict__ dlt,
+         const T* __restrict__ dout, T* __restrict__ dk, T* __restrict__ dv, const AttnDims& D, int first, int step) {
   constexpr int LD = NC * 64 + 4;
   extern __shared__ float sm[];
   float* Ks = sm;
@@ -322,7 +323,7 @@ attn_bwd_dkdv_kernel(const T* __restrict__ q, const T* __restrict__ k, const T* 
   float* Ps = dOs + TS * LD;
   float* dSs = Ps + TS * PLD;
   const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
-  int64_t j0 = (int64_t)blockIdx.x * TS;
+  int64_t j0 = (int64_t)first * TS;
   const int h = blockIdx.y;
   const int64_t b = blockIdx.z;
   const T* qb = q + b * D.Lq * D.E + (int64_t)h * D.d;
@@ -331,11 +332,6 @@ attn_bwd_dkdv_kernel(const T* __restrict__ q, const T* __restrict__ k, const T* 
   const T* dob = dout + b * D.Lq * D.Ev + (int64_t)h * D.dv;
   const float* lse_bh = lse + (b * D.H + h) * D.Lq;
   const float* dlt_bh = dlt + (b * D.H + h) * (REDO ? D.dlt_ld : D.Lq);
-  if (REDO) {
-    int any = 0;
-    for (int i = threadIdx.x; i < D.redo_n; i += AT) any |= D.redo[(b * D.H + h) * D.redo_n + i];
-    if (!__syncthreads_or(any)) return;
-  }
   do {
     if (REDO) __syncthreads();
     load_tile<LD>(Ks, kb, D.E, j0, D.Lk, D.d);
@@ -373,17 +369,24 @@ attn_bwd_dkdv_kernel(const T* __restrict__ q, const T* __restrict__ k, const T* 
           if (c < D.dv) attn_put(dvb + gj * D.Ev + c, adv[cc][jj][e]);
         }
     }
-    j0 += (int64_t)gridDim.x * TS;
+    j0 += (int64_t)step * TS;
   } while (REDO && j0 < D.Lk);
+}
+template <int NC>
+__global__ void __launch_bounds__(AT)
+attn_bwd_dkdv_kernel(const float* __restrict__ q, const float* __restrict__ k, const float* __restrict__ v,
+                     const uint8_t* __restrict__ mask, const float* __restrict__ lse, const float* __restrict__ dlt,
+                     const float* __restrict__ dout, float* __restrict__ dk, float* __restrict__ dv, AttnDims D) {
+  fb_after_previous();
+  bwd_dkdv<NC, float, false>(q, k, v, mask, lse, dlt, dout, dk, dv, D, (int)blockIdx.x, 0);
 }
 
 // ----------------------------------------------------------------------------- backward: dQ ---
 template <int NC, typename T, bool REDO>
-__global__ void __launch_bounds__(AT)
-attn_bwd_dq_kernel(const T* __restrict__ q, const T* __restrict__ k, const T* __restrict__ v,
-                   const uint8_t* __restrict__ mask, const float* __restrict__ lse, const float* __restrict__ dlt,
-                   const T* __restrict__ dout, T* __restrict__ dq, AttnDims D) {
-  fb_after_previous();
+__device__ __forceinline__ void
+bwd_dq(const T* __restrict__ q, const T* __restrict__ k, const T* __restrict__ v,
+       const uint8_t* __restrict__ mask, const float* __restrict__ lse, const float* __restrict__ dlt,
+       const T* __restrict__ dout, T* __restrict__ dq, const AttnDims& D, int first, int step) {
   constexpr int LD = NC * 64 + 4;
   extern __shared__ float sm[];
   float* Qs = sm;
@@ -392,7 +395,7 @@ attn_bwd_dq_kernel(const T* __restrict__ q, const T* __restrict__ k, const T* __
   float* Vs = Ks + TS * LD;
   float* dSs = Vs + TS * LD;
   const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
-  int64_t i0 = (int64_t)blockIdx.x * TS;
+  int64_t i0 = (int64_t)first * TS;
   const int h = blockIdx.y;
   const int64_t b = blockIdx.z;
   const T* qb = q + b * D.Lq * D.E + (int64_t)h * D.d;
@@ -401,11 +404,6 @@ attn_bwd_dq_kernel(const T* __restrict__ q, const T* __restrict__ k, const T* __
   const T* dob = dout + b * D.Lq * D.Ev + (int64_t)h * D.dv;
   const float* lse_bh = lse + (b * D.H + h) * D.Lq;
   const float* dlt_bh = dlt + (b * D.H + h) * (REDO ? D.dlt_ld : D.Lq);
-  if (REDO) {
-    int any = 0;
-    for (int i = threadIdx.x; i < D.redo_n; i += AT) any |= D.redo[(b * D.H + h) * D.redo_n + i];
-    if (!__syncthreads_or(any)) return;
-  }
   do {
     if (REDO) __syncthreads();
     load_tile<LD>(Qs, qb, D.E, i0, D.Lq, D.d);
@@ -441,8 +439,32 @@ attn_bwd_dq_kernel(const T* __restrict__ q, const T* __restrict__ k, const T* __
           if (c < D.d) attn_put(dqb + gi * D.E + c, adq[cc][i][e] * D.scale);
         }
     }
-    i0 += (int64_t)gridDim.x * TS;
+    i0 += (int64_t)step * TS;
   } while (REDO && i0 < D.Lq);
+}
+template <int NC>
+__global__ void __launch_bounds__(AT)
+attn_bwd_dq_kernel(const float* __restrict__ q, const float* __restrict__ k, const float* __restrict__ v,
+                   const uint8_t* __restrict__ mask, const float* __restrict__ lse, const float* __restrict__ dlt,
+                   const float* __restrict__ dout, float* __restrict__ dq, AttnDims D) {
+  fb_after_previous();
+  bwd_dq<NC, float, false>(q, k, v, mask, lse, dlt, dout, dq, D, (int)blockIdx.x, 0);
+}
+
+// Both for the heads with a byte of D.redo set: kv_blocks blocks for dK and dV, the rest for dQ (each may be none).
+template <typename T>
+__global__ void __launch_bounds__(AT)
+attn_bwd_redo_kernel(const T* __restrict__ q, const T* __restrict__ k, const T* __restrict__ v, const float* __restrict__ lse,
+                     const float* __restrict__ dlt, const T* __restrict__ dout, T* __restrict__ dq, T* __restrict__ dk, T* __restrict__ dv,
+                     int kv_blocks, AttnDims D) {
+  fb_after_previous();
+  fb_let_next_start();
+  const int64_t bh = (int64_t)blockIdx.z * D.H + blockIdx.y;
+  int any = 0;
+  for (int i = threadIdx.x; i < D.redo_n; i += AT) any |= D.redo[bh * D.redo_n + i];
+  if (!__syncthreads_or(any)) return;
+  if ((int)blockIdx.x < kv_blocks) bwd_dkdv<1, T, true>(q, k, v, nullptr, lse, dlt, dout, dk, dv, D, (int)blockIdx.x, kv_blocks);
+  else bwd_dq<1, T, true>(q, k, v, nullptr, lse, dlt, dout, dq, D, (int)blockIdx.x - kv_blocks, (int)gridDim.x - kv_blocks);
 }
 
 // --------------------------------------------------------------------- scores on demand ---
@@ -561,23 +583,18 @@ int32_t fb_attn_fwd_redo(fb_ctx* ctx, cudaStream_t stream, int bf16, const void*
 template <typename T>
 static int32_t bwd_redo(fb_ctx* ctx, cudaStream_t stream, const void* q, const void* k, const void* v, const float* lse, const float* dlt, const void* dout, void* dq,
                         void* dk, void* dv, int64_t batch, const AttnDims& D) {
-  constexpr size_t smem_kv = (size_t)(4 * TS * (64 + 4) + 2 * TS * PLD) * sizeof(float), smem_q = (size_t)(4 * TS * (64 + 4) + TS * PLD) * sizeof(float);
+  constexpr size_t smem = (size_t)(4 * TS * (64 + 4) + 2 * TS * PLD) * sizeof(float);
   // about two blocks per SM: a launch that finds nothing to do is over in one wave
-  const int64_t fit = (int64_t)ctx->sm_count * 2 / (batch * D.H);
+  const int64_t fit = (int64_t)ctx->sm_count / (batch * D.H);
   auto blocks = [&](int64_t len) {
     const int64_t tiles = (len + TS - 1) / TS;
-    return (unsigned)(fit < 1 ? 1 : fit > tiles ? tiles : fit);
+    return (int)(fit < 1 ? 1 : fit > tiles ? tiles : fit);
   };
-  if (dk != nullptr) {
-    FB_ONCE(ctx, FB_CUDA(cudaFuncSetAttribute(attn_bwd_dkdv_kernel<1, T, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_kv)));
-    fb_launch(attn_bwd_dkdv_kernel<1, T, true>, dim3(blocks(D.Lk), (unsigned)D.H, (unsigned)batch), AT, smem_kv, stream, (const T*)q, (const T*)k, (const T*)v, nullptr, lse, dlt, (const T*)dout, (T*)dk, (T*)dv, D);
-    FB_LAUNCH_CHECK();
-  }
-  if (dq != nullptr) {
-    FB_ONCE(ctx, FB_CUDA(cudaFuncSetAttribute(attn_bwd_dq_kernel<1, T, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_q)));
-    fb_launch(attn_bwd_dq_kernel<1, T, true>, dim3(blocks(D.Lq), (unsigned)D.H, (unsigned)batch), AT, smem_q, stream, (const T*)q, (const T*)k, (const T*)v, nullptr, lse, dlt, (const T*)dout, (T*)dq, D);
-    FB_LAUNCH_CHECK();
-  }
+  const int kv = dk != nullptr ? blocks(D.Lk) : 0, nq = dq != nullptr ? blocks(D.Lq) : 0;
+  FB_ONCE(ctx, FB_CUDA(cudaFuncSetAttribute(attn_bwd_redo_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem)));
+  fb_launch(attn_bwd_redo_kernel<T>, dim3((unsigned)(kv + nq), (unsigned)D.H, (unsigned)batch), AT, smem, stream, (const T*)q, (const T*)k, (const T*)v, lse, dlt, (const T*)dout,
+            (T*)dq, (T*)dk, (T*)dv, kv, D);
+  FB_LAUNCH_CHECK();
   return FB_OK;
 }
 int32_t fb_attn_bwd_redo(fb_ctx* ctx, cudaStream_t stream, int bf16, const void* q, const void* k, const void* v, const float* lse, const float* dlt,
@@ -686,20 +703,20 @@ FB_API int32_t fb_attn_bwd_ex(fb_ctx* ctx, void* stream_, const float* q, const 
   dim3 grid_kv((unsigned)((lk + TS - 1) / TS), (unsigned)nheads, (unsigned)batch);
   dim3 grid_q((unsigned)((lq + TS - 1) / TS), (unsigned)nheads, (unsigned)batch);
   if (nc == 1) {
-    FB_CUDA(cudaFuncSetAttribute(attn_bwd_dkdv_kernel<1, float, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_kv));
-    FB_CUDA(cudaFuncSetAttribute(attn_bwd_dq_kernel<1, float, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_q));
+    FB_CUDA(cudaFuncSetAttribute(attn_bwd_dkdv_kernel<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_kv));
+    FB_CUDA(cudaFuncSetAttribute(attn_bwd_dq_kernel<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_q));
     if (!did_kv) {
-      fb_launch(attn_bwd_dkdv_kernel<1, float, false>, grid_kv, AT, smem_kv, stream, q, k, v, mask, lse, dlt, dout, dk, dv, D);
+      fb_launch(attn_bwd_dkdv_kernel<1>, grid_kv, AT, smem_kv, stream, q, k, v, mask, lse, dlt, dout, dk, dv, D);
       FB_LAUNCH_CHECK();
     }
     if (did_q) return FB_OK;
-    fb_launch(attn_bwd_dq_kernel<1, float, false>, grid_q, AT, smem_q, stream, q, k, v, mask, lse, dlt, dout, dq, D);
+    fb_launch(attn_bwd_dq_kernel<1>, grid_q, AT, smem_q, stream, q, k, v, mask, lse, dlt, dout, dq, D);
   } else {
-    FB_CUDA(cudaFuncSetAttribute(attn_bwd_dkdv_kernel<2, float, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_kv));
-    FB_CUDA(cudaFuncSetAttribute(attn_bwd_dq_kernel<2, float, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_q));
-    fb_launch(attn_bwd_dkdv_kernel<2, float, false>, grid_kv, AT, smem_kv, stream, q, k, v, mask, lse, dlt, dout, dk, dv, D);
+    FB_CUDA(cudaFuncSetAttribute(attn_bwd_dkdv_kernel<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_kv));
+    FB_CUDA(cudaFuncSetAttribute(attn_bwd_dq_kernel<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_q));
+    fb_launch(attn_bwd_dkdv_kernel<2>, grid_kv, AT, smem_kv, stream, q, k, v, mask, lse, dlt, dout, dk, dv, D);
     FB_LAUNCH_CHECK();
-    fb_launch(attn_bwd_dq_kernel<2, float, false>, grid_q, AT, smem_q, stream, q, k, v, mask, lse, dlt, dout, dq, D);
+    fb_launch(attn_bwd_dq_kernel<2>, grid_q, AT, smem_q, stream, q, k, v, mask, lse, dlt, dout, dq, D);
   }
   FB_LAUNCH_CHECK();
   return FB_OK;

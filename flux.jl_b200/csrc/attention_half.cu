@@ -23,7 +23,8 @@ using namespace fb_atc;
 
 namespace {
 
-constexpr int NP = 2;   // planes of an operand
+constexpr int NP = 2;             // planes of an operand
+constexpr int SLOT = 3 * TILE;    // memory of a tile's images: these two planes, or the three bf16 ones of a head that is left to attention_tc.cu
 
 // the same where D is first multiplied by 2^-11 (A from tensor memory; A from shared memory)
 __device__ __forceinline__ void tc_mma_ta_down(uint32_t d_tmem, uint32_t a_tmem, uint32_t b_lo, uint32_t hi, uint32_t idesc) {
@@ -57,9 +58,17 @@ __device__ __forceinline__ void split2(float x, float y, uint32_t& hi, uint32_t&
   lo = *reinterpret_cast<const uint32_t*>(&l);
 }
 // Scales are powers of two, as shifts: 2^s puts a largest magnitude (its bits) into [2^14, 2^15).  What is scaled so is held to 2^-23
-// of itself down to 2^-29 of the largest value and to 2^-51 of that below.
-// Three bf16 planes held 2^-25.  It shows where scores are large, whose exponentials turn it into an absolute error: with a key and a
-// value 1e4 times the others errors went 6e-7 -> 4e-6 (o), 1.6e-4 -> 4.3e-3 (dQ), 2.5e-4 -> 1.7e-3 (dV).
+// of itself down to 2^-29 of the largest value and to 2^-51 of that below.  Three bf16 planes hold 2^-24 at any exponent, so a head is
+// left to them ("picked") where that would show:
+// - scores that may exceed SCORE_LIMIT, by the row norms of Q and K.  An exponential turns a relative error into an absolute one, and weights below
+//   2^-29 lose bits.  Heads of 512 x 512 with scores of standard deviation 1, 2, 4, 8, 16 (largest bound 16, 31, 62, ...): errors of the output
+//   2.1, 3.4, 3.5, 4.5, 5.7e-7 here and 2.1, 3.3, 3.2, 3.8, 4.8e-7 with three planes, of dQ 0.4 - 2.3e-6 and 1.4 - 2.6e-6; one key and one value
+//   1e4 times the others: output 3.6e-6 and 6.2e-7, dQ 4.3e-3 and 1.6e-4.
+// - a tile with a row or a column (of the operand: a position or a feature) whose largest value is below 2^-19 of the tile's.  So a value
+//   is held to 2^-23 of itself or to 2^-32 of the largest of its row and of its column.
+// - backward, tiles whose scales differ by more than 2^SH_SPREAD: dS is made in one unit for the head.
+// - values out of the range of the scales.
+// Heads with a value that is not finite are the FMA kernels'.
 constexpr int SH_ZERO = 1000;    // all values are 0
 __device__ __forceinline__ int shift_of(uint32_t max_bits) { return max_bits == 0 ? SH_ZERO : 141 - (int)(max_bits >> 23); }
 __device__ __forceinline__ float pow2(int e) { return e < -126 ? 0.0f : __int_as_float((e > 127 ? 254 : e + 127) << 23); }
@@ -68,8 +77,8 @@ __device__ __forceinline__ float times_pow2(float v, int e) {
   const int h = e / 2;
   return v * pow2(h) * pow2(e - h);
 }
-// the line below which an element of a scaled row or tile is badly held; two of them make its head one for the FMA kernels
-constexpr float FAINT_LINE = 1.9073486328125e-6f;   // 2^-19
+constexpr uint32_t FAINT_BITS = 19u << 23;   // 2^-19, as what the bits of a magnitude differ by
+constexpr float SCORE_LIMIT = 32.0f;
 // largest shifts, up or down, of Q and K, of V and of dO: products of two of their powers of two stay in range
 constexpr int SH_QK = 60, SH_V = 40, SH_DO = 85;
 
@@ -83,8 +92,7 @@ __device__ __forceinline__ void store_planes32(uint32_t t0, uint32_t t1, const u
 }
 
 // One row of a CTA's own operand into tensor memory: planes of 32 columns each, scaled by 2^sh.
-// True when the planes cannot hold it.
-__device__ __forceinline__ bool row_to_tmem(const void* src, int width, bool live, bool vec, uint32_t t_addr, int limit, int& sh) {
+__device__ __forceinline__ void row_to_tmem(const void* src, int width, bool live, bool vec, uint32_t t_addr, int limit, int& sh) {
   uint32_t v[2][32];
 #pragma unroll
   for (int hf = 0; hf < 2; ++hf) row_f32((const float*)src, 32 * hf, width, live, vec, v[hf]);
@@ -92,21 +100,14 @@ __device__ __forceinline__ bool row_to_tmem(const void* src, int width, bool liv
 #pragma unroll
   for (int c = 0; c < 64; ++c) m = max(m, v[c >> 5][c & 31] & 0x7fffffffu);
   sh = shift_of(m);
-  const bool bad = not_finite(m) || sh < -limit;
-  sh = sh == SH_ZERO || bad ? 0 : min(sh, limit);   // (a row far below the others: its elements count as faint ones)
+  sh = sh == SH_ZERO ? 0 : min(sh, limit);   // (not below -limit: the head would be picked)
   const float sc = pow2(sh);
-  int faint = 0;
 #pragma unroll
   for (int hf = 0; hf < 2; ++hf) {
 #pragma unroll
-    for (int c = 0; c < 32; ++c) {
-      const float x = __uint_as_float(v[hf][c]) * sc;
-      faint += (x != 0.0f && fabsf(x) < FAINT_LINE) ? 1 : 0;
-      v[hf][c] = __float_as_uint(x);
-    }
+    for (int c = 0; c < 32; ++c) v[hf][c] = __float_as_uint(__uint_as_float(v[hf][c]) * sc);
     store_planes32(t_addr + 16u * hf, t_addr + 32u + 16u * hf, v[hf]);
   }
-  return bad || faint > 1;
 }
 
 // instruction descriptors: D = F32, A = B = F16, M = 128; B K-major (n columns = rows of the tile) or MN-major
@@ -184,10 +185,13 @@ __device__ __forceinline__ void mma_planes_sum(uint32_t d, uint32_t x, uint32_t 
 // the shared-memory image of the tile (row r at 128 r, its 16-byte chunks permuted by r & 7); rows past the end and features past
 // the head size are 0.  For dO the same pass forms what the softmax backward needs per query: {log2(e) lse, delta = sum_c dO_c O_c};
 // queries past the end get {inf, 0}, which makes their weights 0.
-// shifts: [batch head][job][tile].  A byte of `odd` is set where the planes cannot hold the tile: a value that is not finite, a largest value out of the
-// range of the scales, or two elements and more so far below the largest (FAINT_LINE) that their bits are lost; they may be
-// all that counts, where their factors are as far above the others.  The FMA kernels compute the heads of such tiles.
-// Bound by memory: 4 bytes in, 4 out per value (Float32).
+// The notes say what the tile is like.  A job without images (Q ahead of the forward kernel) only gets those.
+// Bound by memory: 4 bytes in, 4 out per value.
+struct TileNote {
+  float norm2;      // largest squared norm of a row
+  int16_t shift;
+  int16_t odd;      // 1: the planes do not hold the tile well, 2: a value is not finite
+};
 struct SplitJob {
   const void* src;
   uint8_t* dst;
@@ -199,95 +203,197 @@ struct SplitArgs {
   const float* o;       // for the job of index 3 (dO)
   const float* lse;
   float2* rv;
-  int16_t* shifts;      // [batch head][job][max_tiles]
-  uint8_t* odd;         // the same, odd_n per (batch, head)
-  int H, vec, jobs, max_tiles, odd_n;
+  TileNote* notes;      // [batch head][job][max_tiles]
+  int H, vec, jobs, max_tiles;
 };
 
-__global__ void __launch_bounds__(256) attn_half_split_kernel(SplitArgs A) {
+constexpr int SPLIT_THREADS = KT * 8, SPLIT_WARPS = SPLIT_THREADS / 32;   // eight values of a row a thread (sixteen of two rows: 78 us for 134 MB of Q, K and V, here 67)
+__global__ void __launch_bounds__(SPLIT_THREADS, 4) attn_half_split_kernel(SplitArgs A) {
   fb_after_previous();
-  __shared__ uint32_t top[8];
+  __shared__ uint32_t top[SPLIT_WARPS];
+  __shared__ float norms[SPLIT_WARPS];
+  __shared__ uint32_t cols[SPLIT_WARPS][KT];
   const SplitJob J = A.job[blockIdx.z];
   if ((int)blockIdx.x >= J.tiles) return;
   const int64_t bh = blockIdx.y;
   const int64_t b = bh / A.H;
   const int h = (int)(bh - b * A.H);
-  uint8_t* dst = J.dst + (bh * J.tiles + blockIdx.x) * (int64_t)(NP * TILE);
-  const int ch = threadIdx.x & 7;
-  const bool is_do = blockIdx.z == 3;
-  float x[2][8];
-  uint32_t m = 0u;
+  const int r = threadIdx.x >> 3, ch = threadIdx.x & 7;
+  const int64_t row = (int64_t)blockIdx.x * KT + r;
+  const bool live = row < J.L;
+  const int64_t off = (b * J.L + row) * J.E + (int64_t)h * J.width;
+  const float* src = (const float*)J.src + off;
+  float x[8];
+  if (A.vec) {
 #pragma unroll
-  for (int it = 0; it < 2; ++it) {
-    const int r = (threadIdx.x >> 3) + 32 * it;
-    const int64_t row = (int64_t)blockIdx.x * KT + r;
-    const bool live = row < J.L;
-    const int64_t off = (b * J.L + row) * J.E + (int64_t)h * J.width;
-    const float* s = (const float*)J.src + off;
-    if (A.vec) {
-#pragma unroll
-      for (int e = 0; e < 8; e += 4) {
-        float4 t = make_float4(0.f, 0.f, 0.f, 0.f);
-        if (live && 8 * ch + e < J.width) t = __ldg((const float4*)(s + 8 * ch + e));
-        x[it][e] = t.x; x[it][e + 1] = t.y; x[it][e + 2] = t.z; x[it][e + 3] = t.w;
-      }
-    } else {
-#pragma unroll
-      for (int e = 0; e < 8; ++e) x[it][e] = (live && 8 * ch + e < J.width) ? __ldg(s + 8 * ch + e) : 0.0f;
+    for (int e = 0; e < 8; e += 4) {
+      float4 t = make_float4(0.f, 0.f, 0.f, 0.f);
+      if (live && 8 * ch + e < J.width) t = __ldg((const float4*)(src + 8 * ch + e));
+      x[e] = t.x; x[e + 1] = t.y; x[e + 2] = t.z; x[e + 3] = t.w;
     }
+  } else {
 #pragma unroll
-    for (int e = 0; e < 8; ++e) m = max(m, __float_as_uint(x[it][e]) & 0x7fffffffu);
-    if (is_do) {
-      float sum = 0.0f;
-#pragma unroll
-      for (int e = 0; e < 8; e += 4) {
-        if (!live || 8 * ch + e >= J.width) break;
-        const float* po = A.o + off + 8 * ch + e;
-        if (A.vec) {
-          const float4 t = __ldg((const float4*)po);
-          sum = fmaf(x[it][e], t.x, sum); sum = fmaf(x[it][e + 1], t.y, sum); sum = fmaf(x[it][e + 2], t.z, sum); sum = fmaf(x[it][e + 3], t.w, sum);
-        } else {
-          for (int u = 0; u < 4 && 8 * ch + e + u < J.width; ++u) sum = fmaf(x[it][e + u], __ldg(po + u), sum);
-        }
-      }
-      sum += __shfl_xor_sync(0xffffffffu, sum, 1);
-      sum += __shfl_xor_sync(0xffffffffu, sum, 2);
-      sum += __shfl_xor_sync(0xffffffffu, sum, 4);
-      if (ch == 0) A.rv[bh * ((int64_t)J.tiles * KT) + row] = live ? make_float2(A.lse[bh * J.L + row] * LOG2E, sum) : make_float2(INFINITY, 0.0f);
-    }
+    for (int e = 0; e < 8; ++e) x[e] = (live && 8 * ch + e < J.width) ? __ldg(src + 8 * ch + e) : 0.0f;
   }
-  m = __reduce_max_sync(0xffffffffu, m);
-  if ((threadIdx.x & 31) == 0) top[threadIdx.x >> 5] = m;
-  __syncthreads();
+  if (blockIdx.z == 3) {   // dO
+    float sum = 0.0f;
 #pragma unroll
-  for (int w = 0; w < 8; ++w) m = max(m, top[w]);
-  int sh = shift_of(m);
-  const bool bad = not_finite(m) || (sh != SH_ZERO && (sh > J.limit || sh < -J.limit));
-  const float sc = pow2(sh == SH_ZERO || bad ? 0 : sh);
-  int faint = 0;
-#pragma unroll
-  for (int it = 0; it < 2; ++it) {
-    const int r = (threadIdx.x >> 3) + 32 * it;
-    uint8_t* out = dst + r * 128 + ((ch ^ (r & 7)) << 4);
-#pragma unroll
-    for (int e = 0; e < 8; ++e) {
-      x[it][e] *= sc;
-      faint += (x[it][e] != 0.0f && fabsf(x[it][e]) < FAINT_LINE) ? 1 : 0;
+    for (int e = 0; e < 8; e += 4) {
+      if (!live || 8 * ch + e >= J.width) break;
+      const float* po = A.o + off + 8 * ch + e;
+      if (A.vec) {
+        const float4 t = __ldg((const float4*)po);
+        sum = fmaf(x[e], t.x, sum); sum = fmaf(x[e + 1], t.y, sum); sum = fmaf(x[e + 2], t.z, sum); sum = fmaf(x[e + 3], t.w, sum);
+      } else {
+        for (int u = 0; u < 4 && 8 * ch + e + u < J.width; ++u) sum = fmaf(x[e + u], __ldg(po + u), sum);
+      }
     }
+    sum += __shfl_xor_sync(0xffffffffu, sum, 1);
+    sum += __shfl_xor_sync(0xffffffffu, sum, 2);
+    sum += __shfl_xor_sync(0xffffffffu, sum, 4);
+    if (ch == 0) A.rv[bh * ((int64_t)J.tiles * KT) + row] = live ? make_float2(A.lse[bh * J.L + row] * LOG2E, sum) : make_float2(INFINITY, 0.0f);
+  }
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  uint32_t m = 0u, least = ~0u;   // the largest magnitude, the least one that is not 0 (less 1)
+#pragma unroll
+  for (int e = 0; e < 8; ++e) {
+    const uint32_t a = __float_as_uint(x[e]) & 0x7fffffffu;
+    m = max(m, a);
+    least = min(least, a - 1u);
+  }
+  const uint32_t own = m;   // the largest of this thread's eight
+  m = __reduce_max_sync(0xffffffffu, m);
+  float norm2 = 0.0f;
+  if ((blockIdx.z & 1) == 0) {   // K and Q
+#pragma unroll
+    for (int e = 0; e < 8; ++e) norm2 = fmaf(x[e], x[e], norm2);
+    norm2 += __shfl_xor_sync(0xffffffffu, norm2, 1);
+    norm2 += __shfl_xor_sync(0xffffffffu, norm2, 2);
+    norm2 += __shfl_xor_sync(0xffffffffu, norm2, 4);
+    norm2 = __uint_as_float(__reduce_max_sync(0xffffffffu, __float_as_uint(norm2)));   // (not negative: the order is that of the bits)
+  }
+  if (lane == 0) {
+    top[warp] = m;
+    norms[warp] = norm2;
+  }
+  __syncthreads();
+  m = __reduce_max_sync(0xffffffffu, top[lane % SPLIT_WARPS]);
+  const int sh = shift_of(m);
+  const bool in_range = sh == SH_ZERO || (sh <= J.limit && sh >= -J.limit);
+  // (few tiles hold a value below the line at all: one of a hundred of normally distributed ones)
+  const uint32_t line = m > FAINT_BITS ? m - FAINT_BITS : 0u;
+  const bool look = __syncthreads_or(least != ~0u && least + 1u < line) != 0;
+  if (J.dst != nullptr) {
+    const float sc = pow2(sh == SH_ZERO || !in_range ? 0 : sh);
+    uint8_t* out = J.dst + (bh * J.tiles + blockIdx.x) * (int64_t)SLOT + r * 128 + ((ch ^ (r & 7)) << 4);
     uint32_t p0[4], p1[4];
 #pragma unroll
-    for (int e = 0; e < 4; ++e) split2(x[it][2 * e], x[it][2 * e + 1], p0[e], p1[e]);
+    for (int e = 0; e < 4; ++e) split2(x[2 * e] * sc, x[2 * e + 1] * sc, p0[e], p1[e]);
     *(uint4*)out = make_uint4(p0[0], p0[1], p0[2], p0[3]);
     *(uint4*)(out + TILE) = make_uint4(p1[0], p1[1], p1[2], p1[3]);
   }
-  int some = __syncthreads_count(faint > 0);
-  if (some == 1) some += __syncthreads_or(faint > 1);
+  bool faint = false;
+  if (look) {
+    uint32_t rmax = own;
+#pragma unroll
+    for (int o = 1; o < 8; o *= 2) rmax = max(rmax, __shfl_xor_sync(0xffffffffu, rmax, o));
+    faint = rmax != 0u && rmax < line;
+#pragma unroll
+    for (int e = 0; e < 8; ++e) {
+      uint32_t col = __float_as_uint(x[e]) & 0x7fffffffu;
+      col = max(col, __shfl_xor_sync(0xffffffffu, col, 8));
+      col = max(col, __shfl_xor_sync(0xffffffffu, col, 16));
+      if (lane < 8) cols[warp][8 * lane + e] = col;
+    }
+    __syncthreads();
+    if (threadIdx.x < KT) {
+      uint32_t col = 0u;
+#pragma unroll 4
+      for (int w = 0; w < SPLIT_WARPS; ++w) col = max(col, cols[w][threadIdx.x]);
+      faint |= col != 0u && col < line;
+    }
+    faint = __syncthreads_or(faint) != 0;
+  }
   if (threadIdx.x == 0) {
-    const int at = (int)blockIdx.z * A.max_tiles + (int)blockIdx.x;
-    A.shifts[bh * A.jobs * A.max_tiles + at] = (int16_t)(bad ? 0 : sh);
-    A.odd[bh * A.odd_n + at] = bad || some > 1 ? 1 : 0;
+    for (int w = 1; w < SPLIT_WARPS; ++w) norm2 = fmaxf(norm2, norms[w]);
+    TileNote note;
+    note.norm2 = norm2;
+    note.shift = (int16_t)sh;
+    note.odd = (int16_t)(not_finite(m) ? 2 : faint || !in_range ? 1 : 0);
+    A.notes[(bh * A.jobs + (int)blockIdx.z) * A.max_tiles + (int)blockIdx.x] = note;
   }
 }
+
+// How a head is computed: 0 here, 1 by attention_tc.cu, 2 by the FMA kernels.
+struct HeadState {
+  uint32_t odd, q, k;   // over its tiles: the largest note, the largest row norms (bits of the squares)
+  __device__ __forceinline__ void add(int job, uint2 note) {
+    if (note.y >> 16 != 0u) atomicMax(&odd, note.y >> 16);
+    if (job == 0) atomicMax(&k, note.x);
+    if (job == 2) atomicMax(&q, note.x);
+  }
+  __device__ __forceinline__ int state(const AtcDims& D) const {
+    if (odd != 0u) return (int)odd;
+    const float bound = sqrtf(__uint_as_float(q)) * sqrtf(__uint_as_float(k)) * D.scale;
+    return bound <= SCORE_LIMIT ? 0 : 1;   // (also where a square has left the range)
+  }
+};
+// The same for the forward kernel.  All threads; ends with a barrier.
+__device__ __forceinline__ int head_state(HeadState& S, const TileNote* notes, const AtcDims& D) {
+  if (threadIdx.x == 0) S = HeadState{0u, 0u, 0u};
+  __syncthreads();
+  for (int i = threadIdx.x; i < 3 * D.max_tiles; i += (int)blockDim.x) {
+    const int job = i / D.max_tiles;
+    if (i - job * D.max_tiles < (job < 2 ? D.ktiles : D.qtiles)) S.add(job, __ldg((const uint2*)(notes + i)));
+  }
+  __syncthreads();
+  return S.state(D);
+}
+// The images of a picked head: three bf16 planes a tile, in the place of the planes here.  CTA `part` of the `parts` of the head takes its share of the tiles.
+__device__ __noinline__ void images_of_three(const SplitArgs& A, int64_t bh, int part, int parts) {
+  constexpr int U = 4;   // pieces of eight values on their way at once
+  const int64_t b = bh / A.H;
+  const int h = (int)(bh - b * A.H);
+  for (int job = 0; job < A.jobs; ++job) {
+    const SplitJob J = A.job[job];
+    if (J.dst == nullptr) continue;
+    const float* src = (const float*)J.src + b * J.L * J.E + (int64_t)h * J.width;
+    const int own = (J.tiles - part + parts - 1) / parts * (KT * 8);   // pieces of this CTA's tiles part, part + parts, ...
+    for (int i0 = threadIdx.x; i0 < own; i0 += U * (int)blockDim.x) {
+      float x[U][8];
+#pragma unroll
+      for (int u = 0; u < U; ++u) {
+        const int i = i0 + u * (int)blockDim.x, ch = i & 7;
+        const int64_t row = (int64_t)(part + (i >> 9) * parts) * KT + (i >> 3 & (KT - 1));
+        const bool live = i < own && row < J.L;
+        const float* p = src + row * J.E + 8 * ch;
+        if (A.vec) {
+#pragma unroll
+          for (int e = 0; e < 8; e += 4) {
+            float4 t = make_float4(0.f, 0.f, 0.f, 0.f);
+            if (live && 8 * ch + e < J.width) t = __ldg((const float4*)(p + e));
+            x[u][e] = t.x; x[u][e + 1] = t.y; x[u][e + 2] = t.z; x[u][e + 3] = t.w;
+          }
+        } else {
+#pragma unroll
+          for (int e = 0; e < 8; ++e) x[u][e] = (live && 8 * ch + e < J.width) ? __ldg(p + e) : 0.0f;
+        }
+      }
+#pragma unroll
+      for (int u = 0; u < U; ++u) {
+        const int i = i0 + u * (int)blockDim.x, ch = i & 7, r = i >> 3 & (KT - 1);
+        if (i >= own) break;
+        uint8_t* out = J.dst + (bh * J.tiles + part + (i >> 9) * parts) * (int64_t)SLOT + r * 128 + ((ch ^ (r & 7)) << 4);
+        uint32_t q[3][4];
+#pragma unroll
+        for (int e = 0; e < 4; ++e) split3(x[u][2 * e], x[u][2 * e + 1], q[0][e], q[1][e], q[2][e]);
+#pragma unroll
+        for (int n = 0; n < 3; ++n) *(uint4*)(out + n * TILE) = make_uint4(q[n][0], q[n][1], q[n][2], q[n][3]);
+      }
+    }
+  }
+}
+static_assert(KT * 8 == 512, "pieces of a tile");
 
 // ------------------------------------------------------------------------------------------------------ forward ---
 // One CTA owns 128 queries of one (batch, head); warp 0 copies K and V tiles into a ring of slots (K0 V0 K1 V1 ...),
@@ -306,8 +412,8 @@ struct FwdCfg {
 
 __global__ void __launch_bounds__(FWD_THREADS, 2)
 attn_fwd_half_kernel(const float* __restrict__ qmat, const uint8_t* __restrict__ kimg, const uint8_t* __restrict__ vimg,
-                   const int16_t* __restrict__ shifts, float* __restrict__ o, float* __restrict__ lse,
-                   uint8_t* __restrict__ odd_q, int odd_n, AtcDims D, int32_t* __restrict__ dev_err) {
+                   const __grid_constant__ SplitArgs A, float* __restrict__ o, float* __restrict__ lse, uint8_t* __restrict__ pick, uint8_t* __restrict__ fma,
+                   AtcDims D, int32_t* __restrict__ dev_err) {
   fb_after_previous();
   using cfg = FwdCfg;
   constexpr int S = cfg::SLOTS;
@@ -343,8 +449,15 @@ attn_fwd_half_kernel(const float* __restrict__ qmat, const uint8_t* __restrict__
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     fence_proxy_async();
   }
-  __syncthreads();
-  if (*s_skip != 0) return;
+  __shared__ HeadState hs;
+  const TileNote* notes = A.notes + bh * 3 * D.max_tiles;
+  const int state = head_state(hs, notes, D);
+  if (blockIdx.x == 0 && threadIdx.x == 0) {
+    pick[bh] = state == 1 ? 1 : 0;
+    fma[bh] = state == 2 ? 1 : 0;
+  }
+  if (state == 1) images_of_three(A, bh, (int)blockIdx.x, (int)gridDim.x);
+  if (state != 0 || *s_skip != 0) return;
   if (warp == 1) tmem_alloc(s_tmem, 256u);
   tc_fence_before();
   __syncthreads();
@@ -355,12 +468,12 @@ attn_fwd_half_kernel(const float* __restrict__ qmat, const uint8_t* __restrict__
   if (warp == 0) {
     // ---------------------------------------------------------------- producer ---
     if (lane == 0) {
-      const int64_t base = bh * D.ktiles * (int64_t)cfg::SLOT_BYTES;
+      const int64_t base = bh * D.ktiles * (int64_t)SLOT;
       for (int n = 0; n < 2 * nkb; ++n) {
         const int s = n % S;
         if (n >= S && !mbar_wait(bar(B_FREE + s), (uint32_t)(n / S - 1) & 1u, s_abort)) break;
         mbar_arrive_expect_tx(bar(B_FULL + s), (uint32_t)cfg::SLOT_BYTES);
-        bulk_load(sb + (uint32_t)(s * cfg::SLOT_BYTES), ((n & 1) ? vimg : kimg) + base + (int64_t)(n >> 1) * cfg::SLOT_BYTES,
+        bulk_load(sb + (uint32_t)(s * cfg::SLOT_BYTES), ((n & 1) ? vimg : kimg) + base + (int64_t)(n >> 1) * SLOT,
                   (uint32_t)cfg::SLOT_BYTES, bar(B_FULL + s));
       }
     }
@@ -397,16 +510,13 @@ attn_fwd_half_kernel(const float* __restrict__ qmat, const uint8_t* __restrict__
     const bool live = gi < D.Lq;
     const uint32_t t_row = tmem + ((uint32_t)(32 * q) << 16);
     int sq;
-    const bool odd = row_to_tmem(qmat + (b * D.Lq + gi) * D.E + (int64_t)h * D.d, D.d, live, D.vec != 0, t_row, SH_QK, sq);
-    const bool any = __any_sync(0xffffffffu, odd);
-    if (lane == 0) odd_q[bh * odd_n + (int)(i0 / QT) * 4 + q] = any ? 1 : 0;
+    row_to_tmem(qmat + (b * D.Lq + gi) * D.E + (int64_t)h * D.d, D.d, live, D.vec != 0, t_row, SH_QK, sq);
     tc_wait_st();
     tc_fence_before();
     __syncwarp();
     if (lane == 0) mbar_arrive(bar(B_QREADY));
-    const int16_t* sk = shifts + bh * 2 * D.ktiles;   // of the K tiles, then of the V tiles
-    auto shift_at = [&](int i) { const int v = __ldg(sk + i); return v == SH_ZERO ? 0 : v; };
-    int sk_j = shift_at(0), sv_j = shift_at(D.ktiles);
+    auto shift_at = [&](int i) { const int v = __ldg(&notes[i].shift); return v == SH_ZERO ? 0 : v; };   // of the K tiles, then of the V tiles
+    int sk_j = shift_at(0), sv_j = shift_at(D.max_tiles);
     float m = -INFINITY, l = 0.0f, fv = 0.0f;         // fv: the scale of the weights and of the V tile whose product is on its way
     float acc[HD];
 #pragma unroll
@@ -457,7 +567,7 @@ attn_fwd_half_kernel(const float* __restrict__ qmat, const uint8_t* __restrict__
       fv = pow2(-15 - sv_j);
       if (j + 1 < nkb) {
         sk_j = shift_at(j + 1);
-        sv_j = shift_at(D.ktiles + j + 1);
+        sv_j = shift_at(D.max_tiles + j + 1);
       }
       const float m_new = fmaxf(m, fmaxf(mx0, mx1) * sc);
       const float m_use = (m_new == -INFINITY) ? 0.0f : m_new;
@@ -521,41 +631,47 @@ attn_fwd_half_kernel(const float* __restrict__ qmat, const uint8_t* __restrict__
 // Scales.  With s the shifts, scores come times 2^(sq + sk), dP times 2^(sdo + sv).  dS is made in units of 2^-(sdo + svmin): |dP| and
 // |delta| are sums of at most 64 products below 2^30, so |dS| < 2^37 there, and 2^-22 of it fits a half; a K tile's shift above the
 // least one goes into it too, so that all blocks add up in one scale.
-constexpr int SH_SPREAD = 16;   // what the shifts of a head's K, V, Q and dO tiles may differ by, added up: dS then keeps 2^-19 of itself
+constexpr int SH_SPREAD = 8;   // what the shifts of the K, V, Q and dO tiles of a head may differ by, added up (ordinary ones: by 4)
 
-// The shifts of a head's tiles (those of tiles of zeros, whatever is multiplied with them, are the least ones), their least ones, and
-// whether they spread too far.  All threads; ends with a barrier.
+// The shifts of a head's tiles (those of tiles of zeros, whatever is multiplied with them, are the least ones), their least ones; returns how the
+// head is computed.  All threads; ends with a barrier.
 struct HeadShifts {
+  HeadState head;
   int16_t tile[4][BWD_MAX_BLOCKS];   // K, V, Q, dO: as far as there is room (of the operand that a kernel walks there is)
   int least[4], most[4];
 };
-__device__ __forceinline__ bool head_shifts(HeadShifts& S, const int16_t* shifts, int64_t bh, const AtcDims& D) {
+__device__ __forceinline__ int head_shifts(HeadShifts& S, const TileNote* notes, const AtcDims& D) {
   if (threadIdx.x < 4) {
     S.least[threadIdx.x] = SH_ZERO;
     S.most[threadIdx.x] = -SH_ZERO;
   }
+  if (threadIdx.x == 0) S.head = HeadState{0u, 0u, 0u};
   __syncthreads();
   auto each = [&](auto f) {
     for (int i = threadIdx.x; i < 4 * D.max_tiles; i += (int)blockDim.x) {
       const int job = i / D.max_tiles, t = i - job * D.max_tiles;
-      if (t < (job < 2 ? D.ktiles : D.qtiles)) f(job, t, (int)__ldg(shifts + bh * 4 * D.max_tiles + i));
+      if (t < (job < 2 ? D.ktiles : D.qtiles)) f(job, t, __ldg((const uint2*)(notes + i)));
     }
   };
-  each([&](int job, int, int v) {
+  each([&](int job, int, uint2 w) {
+    S.head.add(job, w);
+    const int v = (int16_t)(w.y & 0xffffu);
     if (v == SH_ZERO) return;
     atomicMin(&S.least[job], v);
     atomicMax(&S.most[job], v);
   });
   __syncthreads();
-  each([&](int job, int t, int v) {
+  each([&](int job, int t, uint2 w) {
+    const int v = (int16_t)(w.y & 0xffffu);
     if (t < BWD_MAX_BLOCKS) S.tile[job][t] = (int16_t)(v == SH_ZERO ? (S.least[job] == SH_ZERO ? 0 : S.least[job]) : v);
   });
   int spread = 0;
 #pragma unroll
   for (int j = 0; j < 4; ++j)
     if (S.most[j] >= S.least[j]) spread += S.most[j] - S.least[j];
+  const int state = S.head.state(D);
   __syncthreads();
-  return spread > SH_SPREAD;
+  return state == 0 && spread > SH_SPREAD ? 1 : state;
 }
 // the least shift of a job (0 where all tiles are zeros)
 __device__ __forceinline__ int least_of(const HeadShifts& S, int job) { return S.least[job] == SH_ZERO ? 0 : S.least[job]; }
@@ -568,8 +684,8 @@ struct DqCfg {
 
 __global__ void __launch_bounds__(BWD_THREADS, 1)
 attn_bwd_dq_half_kernel(const float* __restrict__ q, const float* __restrict__ dout, const uint8_t* __restrict__ kimg,
-                      const uint8_t* __restrict__ vimg, const float2* __restrict__ rv, const int16_t* __restrict__ shifts,
-                      uint8_t* __restrict__ odd_spread, int odd_n, float* __restrict__ dq, AtcDims D, int32_t* __restrict__ dev_err) {
+                      const uint8_t* __restrict__ vimg, const float2* __restrict__ rv, const __grid_constant__ SplitArgs A,
+                      uint8_t* __restrict__ pick, uint8_t* __restrict__ fma, int first, float* __restrict__ dq, AtcDims D, int32_t* __restrict__ dev_err) {
   fb_after_previous();
   using cfg = DqCfg;
   constexpr int S = cfg::SLOTS;
@@ -608,9 +724,16 @@ attn_bwd_dq_half_kernel(const float* __restrict__ q, const float* __restrict__ d
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     fence_proxy_async();
   }
-  const bool spread = head_shifts(hs, shifts, bh, D);   // (ends with a barrier)
-  if (blockIdx.x == 0 && threadIdx.x == 0) odd_spread[bh * odd_n] = spread ? 1 : 0;
-  if (*s_skip != 0) return;
+  const TileNote* notes = A.notes + bh * 4 * D.max_tiles;
+  const int state = head_shifts(hs, notes, D);
+  if (first) {   // (the dK / dV kernel has not been launched)
+    if (blockIdx.x == 0 && threadIdx.x == 0) {
+      pick[bh] = state == 1 ? 1 : 0;
+      fma[bh] = state == 2 ? 1 : 0;
+    }
+    if (state == 1) images_of_three(A, bh, (int)blockIdx.x, (int)gridDim.x);
+  }
+  if (state != 0 || *s_skip != 0) return;
   if (warp == 1) tmem_alloc(s_tmem, 512u);
   tc_fence_before();
   __syncthreads();
@@ -621,13 +744,13 @@ attn_bwd_dq_half_kernel(const float* __restrict__ q, const float* __restrict__ d
   if (warp == 0) {
     // ---------------------------------------------------------------- producer ---
     if (lane == 0) {
-      const int64_t base = bh * D.ktiles * (int64_t)(NP * TILE);
+      const int64_t base = bh * D.ktiles * (int64_t)SLOT;
       for (int j = 0; j < nkb; ++j) {
         const int s = j % S;
         if (j >= S && !mbar_wait(bar(B_FREE + s), (uint32_t)(j / S - 1) & 1u, s_abort)) break;
         mbar_arrive_expect_tx(bar(B_FULL + s), (uint32_t)cfg::SLOT_BYTES);
         const uint32_t dst = sb + (uint32_t)(s * cfg::SLOT_BYTES);
-        const int64_t off = base + (int64_t)j * (NP * TILE);
+        const int64_t off = base + (int64_t)j * SLOT;
         bulk_load(dst, kimg + off, NP * TILE, bar(B_FULL + s));
         bulk_load(dst + NP * TILE, vimg + off, NP * TILE, bar(B_FULL + s));
       }
@@ -769,8 +892,8 @@ struct KvCfg {
 
 __global__ void __launch_bounds__(KvCfg::THREADS, 1)
 attn_bwd_dkdv_half_kernel(const uint8_t* __restrict__ qimg, const uint8_t* __restrict__ doimg, const uint8_t* __restrict__ kimg,
-                        const uint8_t* __restrict__ vimg, const float2* __restrict__ rv, const int16_t* __restrict__ shifts,
-                        uint8_t* __restrict__ odd_spread, int odd_n, float* __restrict__ dk, float* __restrict__ dv, AtcDims D,
+                        const uint8_t* __restrict__ vimg, const float2* __restrict__ rv, const __grid_constant__ SplitArgs A,
+                        uint8_t* __restrict__ pick, uint8_t* __restrict__ fma, float* __restrict__ dk, float* __restrict__ dv, AtcDims D,
                         int32_t* __restrict__ dev_err) {
   fb_after_previous();
   using cfg = KvCfg;
@@ -809,9 +932,14 @@ attn_bwd_dkdv_half_kernel(const uint8_t* __restrict__ qimg, const uint8_t* __res
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     fence_proxy_async();
   }
-  const bool spread = head_shifts(hs, shifts, bh, D);   // (ends with a barrier)
-  if (blockIdx.x == 0 && threadIdx.x == 0) odd_spread[bh * odd_n] = spread ? 1 : 0;
-  if (*s_skip != 0) return;
+  const TileNote* notes = A.notes + bh * 4 * D.max_tiles;
+  const int state = head_shifts(hs, notes, D);
+  if (blockIdx.x == 0 && threadIdx.x == 0) {
+    pick[bh] = state == 1 ? 1 : 0;
+    fma[bh] = state == 2 ? 1 : 0;
+  }
+  if (state == 1) images_of_three(A, bh, (int)blockIdx.x, (int)gridDim.x);
+  if (state != 0 || *s_skip != 0) return;
   if (warp == 1) tmem_alloc(s_tmem, 512u);
   tc_fence_before();
   __syncthreads();
@@ -827,7 +955,7 @@ attn_bwd_dkdv_half_kernel(const uint8_t* __restrict__ qimg, const uint8_t* __res
       for (int p = 0; p < NP; ++p)
 #pragma unroll
         for (int t = 0; t < 2; ++t) {   // plane p of the CTA's two 64-key tiles, one after the other
-          const int64_t off = ((bh * D.ktiles + 2 * (int64_t)blockIdx.x + t) * NP + p) * (int64_t)TILE;
+          const int64_t off = (bh * D.ktiles + 2 * (int64_t)blockIdx.x + t) * SLOT + p * TILE;
           bulk_load(sb + (uint32_t)(cfg::K_OFF + (2 * p + t) * TILE), kimg + off, TILE, bar(B_KV));
           bulk_load(sb + (uint32_t)(cfg::V_OFF + (2 * p + t) * TILE), vimg + off, TILE, bar(B_KV));
         }
@@ -838,7 +966,7 @@ attn_bwd_dkdv_half_kernel(const uint8_t* __restrict__ qimg, const uint8_t* __res
         const int64_t tile = bh * D.qtiles + ib0 + (n >> 1);
         const uint32_t dst = sb + (uint32_t)(s * cfg::SLOT_BYTES);
         mbar_arrive_expect_tx(bar(B_FULL + s), (uint32_t)(NP * TILE + (is_do ? 512 : 0)));
-        bulk_load(dst, (is_do ? doimg : qimg) + tile * (int64_t)(NP * TILE), NP * TILE, bar(B_FULL + s));
+        bulk_load(dst, (is_do ? doimg : qimg) + tile * (int64_t)SLOT, NP * TILE, bar(B_FULL + s));
         if (is_do) bulk_load(dst + NP * TILE, rv + tile * KT, 512u, bar(B_FULL + s));
       }
     }
@@ -886,7 +1014,7 @@ attn_bwd_dkdv_half_kernel(const uint8_t* __restrict__ qimg, const uint8_t* __res
     const bool live = kj < D.Lk;
     const uint32_t t_row = tmem + ((uint32_t)(32 * qd) << 16);
     auto own_shift = [&](int job) {   // (of the two key tiles of this CTA; there may be more than BWD_MAX_BLOCKS)
-      const int v = __ldg(shifts + (bh * 4 + job) * D.max_tiles + 2 * (int64_t)blockIdx.x + (qd >> 1));
+      const int v = __ldg(&notes[job * D.max_tiles + 2 * (int64_t)blockIdx.x + (qd >> 1)].shift);
       return v == SH_ZERO ? least_of(hs, job) : v;
     };
     const int skr = own_shift(0), svr = own_shift(1);
@@ -971,17 +1099,16 @@ attn_bwd_dkdv_half_kernel(const uint8_t* __restrict__ qimg, const uint8_t* __res
   if (threadIdx.x == 0 && *s_abort != 0) atomicExch(dev_err, 4004);
 }
 
-// Heads that the planes cannot hold (attn_split_kernel) are computed again by the FMA kernels.  The launch that finds nothing costs 4 - 6
-// us (2048 x 2048, 8 heads of 32, batch 2: 114 -> 119 us; the FMA kernel 853).
+// Behind the kernels here: the picked heads (attention_tc.cu) and those with values that are not finite (attention.cu).  Launches that find none cost
+// 3 - 6 us each.  Batch 8, 16 heads of 64, 2048 x 2048, causal, forward and backward in us: no head picked 420 and 1233, one 505 and 1340, all 630 and
+// 2190 (all heads on three bf16 planes from the start: 560 and 2079; one head on the FMA kernels: 2455 and 9377).
 int32_t fwd_impl(fb_ctx* ctx, cudaStream_t stream, const float* q, const float* k, const float* v, float* o, float* lse, const AtcPlan& P,
                  int64_t batch) {
   const AtcDims& D = P.D;
-  // a byte for every K and V tile and every 32 queries of a (batch, head)
-  const int odd_n = 2 * D.ktiles + 2 * D.qtiles;
-  const int64_t per = 2 * P.kbytes + (int64_t)D.H * (odd_n + 4 * D.ktiles);
+  const int64_t note_bytes = (int64_t)D.H * 3 * D.max_tiles * (int64_t)sizeof(TileNote), per = 2 * P.kbytes + note_bytes + 2 * D.H;
   int64_t chunk = IMAGE_BYTES / per;
   chunk = chunk < 1 ? 1 : (chunk > batch ? batch : chunk);
-  const fb_temp images(ctx, stream, (size_t)(chunk * per + 512));
+  const fb_temp images(ctx, stream, (size_t)(chunk * per));
   uint8_t* img = (uint8_t*)images.p;
   if (!img) return FB_ERR_UNSUPPORTED;
   FB_ONCE(ctx, FB_CUDA(cudaFuncSetAttribute(attn_fwd_half_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, FwdCfg::SMEM)));
@@ -989,18 +1116,20 @@ int32_t fwd_impl(fb_ctx* ctx, cudaStream_t stream, const float* q, const float* 
     const int64_t nb = b0 + chunk > batch ? batch - b0 : chunk;
     const float *qb = q + b0 * D.Lq * D.E, *kb = k + b0 * D.Lk * D.E, *vb = v + b0 * D.Lk * D.Ev;
     float *ob = o + b0 * D.Lq * D.Ev, *lb = lse + b0 * D.H * D.Lq;
-    int16_t* shifts = (int16_t*)(img + nb * 2 * P.kbytes);
-    uint8_t* odd = (uint8_t*)(shifts + nb * D.H * 2 * D.ktiles);
+    TileNote* notes = (TileNote*)(img + nb * 2 * P.kbytes);
+    uint8_t *pick = (uint8_t*)notes + nb * note_bytes, *fma = pick + nb * D.H;   // a byte per head each
     SplitArgs A = {};
-    A.H = D.H; A.vec = D.vec; A.odd = odd; A.odd_n = odd_n; A.shifts = shifts; A.jobs = 2; A.max_tiles = D.ktiles;
+    A.H = D.H; A.vec = D.vec; A.notes = notes; A.jobs = 3; A.max_tiles = D.max_tiles;
     A.job[0] = {kb, img, D.Lk, D.E, D.d, D.ktiles, SH_QK};
     A.job[1] = {vb, img + nb * P.kbytes, D.Lk, D.Ev, D.dv, D.ktiles, SH_V};
-    fb_launch(attn_half_split_kernel, dim3((unsigned)D.ktiles, (unsigned)(nb * D.H), 2), 256, 0, stream, A);
+    A.job[2] = {qb, nullptr, D.Lq, D.E, D.d, D.qtiles, SH_QK};
+    fb_launch(attn_half_split_kernel, dim3((unsigned)D.max_tiles, (unsigned)(nb * D.H), 3), SPLIT_THREADS, 0, stream, A);
     FB_LAUNCH_CHECK();
-    fb_launch(attn_fwd_half_kernel, dim3((unsigned)(D.qtiles / 2), (unsigned)D.H, (unsigned)nb), FWD_THREADS, FwdCfg::SMEM, stream, qb, img, img + nb * P.kbytes, shifts, ob,
-              lb, odd + 2 * D.ktiles, odd_n, D, ctx->dev_error);
+    fb_launch(attn_fwd_half_kernel, dim3((unsigned)(D.qtiles / 2), (unsigned)D.H, (unsigned)nb), FWD_THREADS, FwdCfg::SMEM, stream, qb, img, img + nb * P.kbytes, A, ob, lb,
+              pick, fma, D, ctx->dev_error);
     FB_LAUNCH_CHECK();
-    const int32_t st = fb_attn_fwd_redo(ctx, stream, 0, qb, kb, vb, ob, nullptr, lb, D.E, D.Ev, D.Lq, D.Lk, nb, D.H, D.causal, odd, odd_n);
+    int32_t st = fwd_picked(ctx, stream, qb, img, img + nb * P.kbytes, ob, lb, D, nb, pick);
+    if (st == FB_OK) st = fb_attn_fwd_redo(ctx, stream, 0, qb, kb, vb, ob, nullptr, lb, D.E, D.Ev, D.Lq, D.Lk, nb, D.H, D.causal, fma, 1);
     if (st != FB_OK) return st;
   }
   return FB_OK;
@@ -1009,12 +1138,10 @@ int32_t fwd_impl(fb_ctx* ctx, cudaStream_t stream, const float* q, const float* 
 int32_t bwd_impl(fb_ctx* ctx, cudaStream_t stream, const float* q, const float* k, const float* v, const float* o, const float* lse, const float* dout, float* dq,
                  float* dk, float* dv, const AtcPlan& P, int64_t batch, bool do_kv, bool do_q) {
   const AtcDims& D = P.D;
-  // a byte for every tile of a (batch, head) and one for its shifts
-  const int odd_n = 4 * D.max_tiles + 1;
-  const int64_t per = 2 * P.kbytes + 2 * P.qbytes + P.rvbytes + (int64_t)D.H * (odd_n + 8 * D.max_tiles);
+  const int64_t note_bytes = (int64_t)D.H * 4 * D.max_tiles * (int64_t)sizeof(TileNote), per = 2 * P.kbytes + 2 * P.qbytes + P.rvbytes + note_bytes + 2 * D.H;
   int64_t chunk = IMAGE_BYTES / per;
   chunk = chunk < 1 ? 1 : (chunk > batch ? batch : chunk);
-  const fb_temp images(ctx, stream, (size_t)(chunk * per + 512));
+  const fb_temp images(ctx, stream, (size_t)(chunk * per));
   uint8_t* img = (uint8_t*)images.p;
   if (!img) return FB_ERR_UNSUPPORTED;
   FB_ONCE(ctx, FB_CUDA(cudaFuncSetAttribute(attn_bwd_dkdv_half_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, KvCfg::SMEM)));
@@ -1023,28 +1150,33 @@ int32_t bwd_impl(fb_ctx* ctx, cudaStream_t stream, const float* q, const float* 
     const int64_t nb = b0 + chunk > batch ? batch - b0 : chunk;
     uint8_t *ki = img, *vi = ki + nb * P.kbytes, *qi = vi + nb * P.kbytes, *doi = qi + nb * P.qbytes;
     float2* rv = (float2*)(doi + nb * P.qbytes);
-    int16_t* shifts = (int16_t*)((uint8_t*)rv + nb * P.rvbytes);
-    uint8_t* odd = (uint8_t*)(shifts + nb * D.H * 4 * D.max_tiles);
+    TileNote* notes = (TileNote*)((uint8_t*)rv + nb * P.rvbytes);
+    uint8_t *pick = (uint8_t*)notes + nb * note_bytes, *fma = pick + nb * D.H;
     const int64_t qoff = b0 * D.Lq * D.E, qvoff = b0 * D.Lq * D.Ev, koff = b0 * D.Lk * D.E, kvoff = b0 * D.Lk * D.Ev;
     const float *qb = q + qoff, *kb = k + koff, *vb = v + kvoff, *dob = dout + qvoff, *lb = lse + b0 * D.H * D.Lq;
     float *dqb = do_q ? dq + qoff : nullptr, *dkb = do_kv ? dk + koff : nullptr, *dvb = do_kv ? dv + kvoff : nullptr;
     SplitArgs A = {};
-    A.H = D.H; A.vec = D.vec; A.odd = odd; A.odd_n = odd_n; A.shifts = shifts; A.jobs = 4; A.max_tiles = D.max_tiles;
+    A.H = D.H; A.vec = D.vec; A.notes = notes; A.jobs = 4; A.max_tiles = D.max_tiles;
     A.job[0] = {kb, ki, D.Lk, D.E, D.d, D.ktiles, SH_QK};
     A.job[1] = {vb, vi, D.Lk, D.Ev, D.dv, D.ktiles, SH_V};
     A.job[2] = {qb, qi, D.Lq, D.E, D.d, D.qtiles, SH_QK};
     A.job[3] = {dob, doi, D.Lq, D.Ev, D.dv, D.qtiles, SH_DO};
     A.o = o + qvoff; A.lse = lb; A.rv = rv;
-    // (tiles that one operand has and another has not keep no byte)
-    if (D.qtiles != D.ktiles) FB_CUDA(cudaMemsetAsync(odd, 0, (size_t)(nb * D.H * odd_n), stream));
-    fb_launch(attn_half_split_kernel, dim3((unsigned)D.max_tiles, (unsigned)(nb * D.H), 4), 256, 0, stream, A);
+    fb_launch(attn_half_split_kernel, dim3((unsigned)D.max_tiles, (unsigned)(nb * D.H), 4), SPLIT_THREADS, 0, stream, A);
     FB_LAUNCH_CHECK();
-    if (do_kv) fb_launch(attn_bwd_dkdv_half_kernel, dim3((unsigned)(D.ktiles / 2), (unsigned)D.H, (unsigned)nb), KvCfg::THREADS, KvCfg::SMEM, stream, qi, doi, ki, vi, rv, shifts, odd + 4 * D.max_tiles, odd_n, dkb, dvb, D, ctx->dev_error);
-    FB_LAUNCH_CHECK();
-    if (do_q) fb_launch(attn_bwd_dq_half_kernel, dim3((unsigned)(D.qtiles / 2), (unsigned)D.H, (unsigned)nb), BWD_THREADS, DqCfg::SMEM, stream, qb, dob, ki, vi, rv, shifts, odd + 4 * D.max_tiles, odd_n, dqb, D, ctx->dev_error);
-    FB_LAUNCH_CHECK();
-    const int32_t st = fb_attn_bwd_redo(ctx, stream, 0, qb, kb, vb, lb, (const float*)rv + 1, (int64_t)D.qtiles * KT, dob, dqb, dkb, dvb, D.E, D.Ev, D.Lq, D.Lk, nb,
-                                        D.H, D.causal, odd, odd_n);
+    if (do_kv) {
+      fb_launch(attn_bwd_dkdv_half_kernel, dim3((unsigned)(D.ktiles / 2), (unsigned)D.H, (unsigned)nb), KvCfg::THREADS, KvCfg::SMEM, stream, qi, doi, ki, vi, rv, A, pick, fma,
+                dkb, dvb, D, ctx->dev_error);
+      FB_LAUNCH_CHECK();
+    }
+    if (do_q) {
+      fb_launch(attn_bwd_dq_half_kernel, dim3((unsigned)(D.qtiles / 2), (unsigned)D.H, (unsigned)nb), BWD_THREADS, DqCfg::SMEM, stream, qb, dob, ki, vi, rv, A, pick, fma,
+                do_kv ? 0 : 1, dqb, D, ctx->dev_error);
+      FB_LAUNCH_CHECK();
+    }
+    int32_t st = bwd_picked(ctx, stream, qb, dob, ki, vi, qi, doi, rv, dqb, dkb, dvb, D, nb, pick);
+    if (st == FB_OK)
+      st = fb_attn_bwd_redo(ctx, stream, 0, qb, kb, vb, lb, (const float*)rv + 1, (int64_t)D.qtiles * KT, dob, dqb, dkb, dvb, D.E, D.Ev, D.Lq, D.Lk, nb, D.H, D.causal, fma, 1);
     if (st != FB_OK) return st;
   }
   return FB_OK;
@@ -1057,7 +1189,7 @@ int32_t fb_attn_fwd_tc(fb_ctx* ctx, cudaStream_t stream, const float* q, const f
                        float* o, float* lse, int64_t e_dim, int64_t ev_dim, int64_t lq, int64_t lk, int64_t batch, int nheads,
                        int causal) {
   AtcPlan P;
-  if (!attn_tc_enabled() || mask != nullptr || !make_plan(&P, 2, e_dim, ev_dim, lq, lk, batch, nheads, causal)) return FB_ERR_UNSUPPORTED;
+  if (!attn_tc_enabled() || mask != nullptr || !make_plan(&P, 3, e_dim, ev_dim, lq, lk, batch, nheads, causal)) return FB_ERR_UNSUPPORTED;
   if (!fb_aligned16(q) || !fb_aligned16(k) || !fb_aligned16(v) || !fb_aligned16(o)) P.D.vec = 0;
   return fwd_impl(ctx, stream, q, k, v, o, lse, P, batch);
 }
@@ -1070,7 +1202,7 @@ int32_t fb_attn_bwd_tc(fb_ctx* ctx, cudaStream_t stream, const float* q, const f
                        int64_t lk, int64_t batch, int nheads, int causal, bool* did_kv, bool* did_q) {
   AtcPlan P;
   *did_kv = *did_q = false;
-  if (!attn_tc_enabled() || !attn_bwd_tc_enabled() || mask != nullptr || !make_plan(&P, 2, e_dim, ev_dim, lq, lk, batch, nheads, causal) ||
+  if (!attn_tc_enabled() || !attn_bwd_tc_enabled() || mask != nullptr || !make_plan(&P, 3, e_dim, ev_dim, lq, lk, batch, nheads, causal) ||
       P.D.d != HD || P.D.dv != HD)
     return FB_ERR_UNSUPPORTED;
   // (arrays off the 16-byte boundary have always been the FMA kernels')

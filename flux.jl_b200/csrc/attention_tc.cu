@@ -1,10 +1,11 @@
-// Flash-style attention of bf16 operands on the tensor cores (tcgen05), for head sizes up to 64 forward and of 64 backward.
+// Flash-style attention on bf16 planes on the tensor cores (tcgen05), for head sizes up to 64 forward and of 64 backward: all heads of bf16
+// operands, and those heads of Float32 operands that the half-precision planes of attention_half.cu would hold worse ("picked" ones).
 //
-// An operand is one bf16 plane, exactly; the probabilities and dS are Float32 values, cut into three bf16 planes by truncation (8 + 8 + 8
-// mantissa bits: the split is exact), and a product with them is the sum of three plane products, the smallest ones first, accumulated
-// in Float32 in tensor memory.  A bf16 tile in the 128-byte swizzle serves as K-major and as MN-major operand: a small kernel
-// (`attn_split_kernel`) lays K, V, Q and dO out once per call as the images that the MMAs read from shared memory, and tiles arrive by plain
-// bulk copies.  Head sizes below 64 are padded with zeros in those images; their zero 16-feature steps are skipped.
+// A Float32 value is cut into three bf16 planes by truncation (8 + 8 + 8 mantissa bits, any exponent: the split is exact); a bf16 operand is one
+// plane.  The probabilities and dS have three.  A product is the sum of the plane products that lie above 2^-24 of it (six of three planes by
+// three, three of three by one), the smallest ones first, accumulated in Float32 in tensor memory.  A bf16 tile in the 128-byte swizzle serves as K-major and as MN-major operand: a small kernel
+// (`attn_split_kernel`; for picked heads the kernels that pick them) lays K, V, Q and dO out once per call as the images that the MMAs read from
+// shared memory, and tiles arrive by plain bulk copies.  Head sizes below 64 are padded with zeros in those images; their zero 16-feature steps are skipped.
 //
 // (Two half-precision planes for the probabilities and dS, as attention_half.cu has them, take a third of these MMAs away, but hold 23 bits
 // of them and, where the scales of a head's tiles differ, fewer.)  What bounds the kernels: an MMA with N = 64 takes 44 clocks where its
@@ -20,16 +21,6 @@ using namespace fb_atc;
 
 namespace {
 
-// Two values as three bf16 planes (x in the low half of each word): truncation to the upper 16 bits leaves a remainder of
-// at most 16 significant bits, the same again one of at most 8, which is a bf16 value.
-__device__ __forceinline__ void split3(float x, float y, uint32_t& p0, uint32_t& p1, uint32_t& p2) {
-  const uint32_t xb = __float_as_uint(x), yb = __float_as_uint(y);
-  p0 = __byte_perm(xb, yb, 0x7632);
-  const float rx = x - __uint_as_float(xb & 0xffff0000u), ry = y - __uint_as_float(yb & 0xffff0000u);
-  const uint32_t rxb = __float_as_uint(rx), ryb = __float_as_uint(ry);
-  p1 = __byte_perm(rxb, ryb, 0x7632);
-  p2 = __byte_perm(__float_as_uint(rx - __uint_as_float(rxb & 0xffff0000u)), __float_as_uint(ry - __uint_as_float(ryb & 0xffff0000u)), 0x7632);
-}
 // 32 values of a thread's row into the three planes of an A operand: 16 columns each at t0, t1 and t2
 __device__ __forceinline__ void store_planes32(uint32_t t0, uint32_t t1, uint32_t t2, const uint32_t* v) {
   uint32_t a[16], b[16], c[16];
@@ -128,11 +119,10 @@ __device__ __forceinline__ void mma_planes(uint32_t d, uint32_t t01, uint32_t t2
 }
 
 // -------------------------------------------------------------------------------------------- plane images ---
-// One 64 x 64 tile of one (batch, head): rows of Float32 or bf16 values -> NP bf16 planes, each the shared-memory image of
-// the tile (row r at 128 r, its 16-byte chunks permuted by r & 7); rows past the end and features past the head size are 0.
+// One 64 x 64 tile of one (batch, head): bf16 rows -> the shared-memory image of the tile (row r at 128 r, its 16-byte chunks permuted by r & 7); rows past the end and features past the head size are 0.
 // For dO the same pass forms what the softmax backward needs per query: {log2(e) lse, delta = sum_c dO_c O_c}; queries past
 // the end get {inf, 0}, which makes their weights 0.
-// Bound by memory: 4 bytes in, 6 out per value (Float32).
+// Bound by memory.
 struct SplitJob {
   const void* src;
   uint8_t* dst;
@@ -148,7 +138,6 @@ struct SplitArgs {
   int H, vec, max_tiles, odd_n;
 };
 
-template <int NP>
 __global__ void __launch_bounds__(256) attn_split_kernel(SplitArgs A) {
   fb_after_previous();
   const SplitJob J = A.job[blockIdx.z];
@@ -156,7 +145,7 @@ __global__ void __launch_bounds__(256) attn_split_kernel(SplitArgs A) {
   const int64_t bh = blockIdx.y;
   const int64_t b = bh / A.H;
   const int h = (int)(bh - b * A.H);
-  uint8_t* dst = J.dst + (bh * J.tiles + blockIdx.x) * (int64_t)(NP * TILE);
+  uint8_t* dst = J.dst + (bh * J.tiles + blockIdx.x) * (int64_t)TILE;
   const int ch = threadIdx.x & 7;
   const bool is_do = blockIdx.z == 3;
   int odd = 0;
@@ -168,35 +157,14 @@ __global__ void __launch_bounds__(256) attn_split_kernel(SplitArgs A) {
     const int64_t off = (b * J.L + row) * J.E + (int64_t)h * J.width;
     uint8_t* out = dst + r * 128 + ((ch ^ (r & 7)) << 4);
     float x[8];
-    if (NP == 3) {
-      const float* s = (const float*)J.src + off;
-      if (A.vec) {
+    uint4 t = make_uint4(0u, 0u, 0u, 0u);
+    if (live && 8 * ch < J.width) t = __ldg((const uint4*)((const uint16_t*)J.src + off + 8 * ch));
+    *(uint4*)out = t;
+    const uint32_t w[4] = {t.x, t.y, t.z, t.w};
 #pragma unroll
-        for (int e = 0; e < 8; e += 4) {
-          float4 t = make_float4(0.f, 0.f, 0.f, 0.f);
-          if (live && 8 * ch + e < J.width) t = __ldg((const float4*)(s + 8 * ch + e));
-          x[e] = t.x; x[e + 1] = t.y; x[e + 2] = t.z; x[e + 3] = t.w;
-        }
-      } else {
-#pragma unroll
-        for (int e = 0; e < 8; ++e) x[e] = (live && 8 * ch + e < J.width) ? __ldg(s + 8 * ch + e) : 0.0f;
-      }
-      uint32_t p0[4], p1[4], p2[4];
-#pragma unroll
-      for (int e = 0; e < 4; ++e) split3(x[2 * e], x[2 * e + 1], p0[e], p1[e], p2[e]);
-      *(uint4*)out = make_uint4(p0[0], p0[1], p0[2], p0[3]);
-      *(uint4*)(out + TILE) = make_uint4(p1[0], p1[1], p1[2], p1[3]);
-      *(uint4*)(out + 2 * TILE) = make_uint4(p2[0], p2[1], p2[2], p2[3]);
-    } else {
-      uint4 t = make_uint4(0u, 0u, 0u, 0u);
-      if (live && 8 * ch < J.width) t = __ldg((const uint4*)((const uint16_t*)J.src + off + 8 * ch));
-      *(uint4*)out = t;
-      const uint32_t w[4] = {t.x, t.y, t.z, t.w};
-#pragma unroll
-      for (int e = 0; e < 4; ++e) {
-        x[2 * e] = __uint_as_float(w[e] << 16);
-        x[2 * e + 1] = __uint_as_float(w[e] & 0xffff0000u);
-      }
+    for (int e = 0; e < 4; ++e) {
+      x[2 * e] = __uint_as_float(w[e] << 16);
+      x[2 * e + 1] = __uint_as_float(w[e] & 0xffff0000u);
     }
 #pragma unroll
     for (int e = 0; e < 8; ++e) odd |= not_finite(__float_as_uint(x[e])) ? 1 : 0;
@@ -223,6 +191,70 @@ __global__ void __launch_bounds__(256) attn_split_kernel(SplitArgs A) {
   if (threadIdx.x == 0) A.odd[bh * A.odd_n + (int)blockIdx.z * A.max_tiles + (int)blockIdx.x] = odd ? 1 : 0;
 }
 
+// --------------------------------------------------------------------------------------------- CTAs and items ---
+struct Cta {
+  uint8_t* smem;
+  uint32_t sb, tmem;
+  volatile uint32_t* s_tmem;
+  volatile int* s_abort;
+  int warp, lane;
+};
+// Kernels of picked heads have fewer CTAs than items (a tile of 128 rows of a head each), so that a launch that finds none is soon over: CTA c
+// takes the items c, c + grid, ..., at most this many.  The heads of a tile follow one another, tiles with the most blocks under a causal mask
+// first, so that CTAs with several items have about as much to do.  Each item has barriers of its own: arrivals of the one before may still
+// be on their way.
+constexpr int PICK_ITEMS = 8;
+// a bit for each item of this CTA whose head is picked; the same in all warps
+template <typename F>
+__device__ __forceinline__ uint32_t picked_items(const uint8_t* pick, int64_t items, F head_of) {
+  const int n = (int)(threadIdx.x & 31u);
+  const int64_t item = blockIdx.x + (int64_t)n * gridDim.x;
+  return __ballot_sync(0xffffffffu, n < PICK_ITEMS && item < items && pick[head_of(item)] != 0);
+}
+// Barriers (init, by one thread) and tensor memory; false, for all threads, after an earlier error.
+template <typename F>
+__device__ __forceinline__ bool cta_begin(Cta& c, uint8_t* smem_raw, uint32_t notes, uint32_t cols, const int32_t* dev_err, F init) {
+  const Shared sh = aligned_smem(smem_raw);
+  c.smem = sh.smem;
+  c.sb = sh.sb;
+  c.s_tmem = (volatile uint32_t*)(sh.smem + notes);
+  c.s_abort = (volatile int*)(c.s_tmem + 1);
+  volatile int* s_skip = (volatile int*)(c.s_tmem + 2);
+  c.warp = uniform_warp();
+  c.lane = threadIdx.x & 31;
+  if (threadIdx.x == 0) {
+    init(sh.sb);
+    *c.s_abort = 0;
+    *s_skip = (*(volatile int32_t*)dev_err != 0) ? 1 : 0;
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    fence_proxy_async();
+  }
+  __syncthreads();
+  if (*s_skip != 0) return false;
+  if (c.warp == 1) tmem_alloc(c.s_tmem, cols);
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
+  c.tmem = __reduce_or_sync(0xffffffffu, *c.s_tmem);
+  return true;
+}
+// Between two items: every load has been consumed and every product read.
+__device__ __forceinline__ bool cta_next(const Cta& c) {
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
+  return *c.s_abort == 0;
+}
+__device__ __forceinline__ void cta_end(const Cta& c, uint32_t cols, int32_t* dev_err, int code) {
+  tc_fence_before();
+  __syncthreads();
+  if (c.warp == 1) {
+    __syncwarp();
+    tmem_free(c.tmem, cols);
+  }
+  if (threadIdx.x == 0 && *c.s_abort != 0) atomicExch(dev_err, code);
+}
+
 // ------------------------------------------------------------------------------------------------------ forward ---
 // One CTA owns 128 queries of one (batch, head); warp 0 copies K and V tiles into a ring of slots (K0 V0 K1 V1 ...),
 // warp 1 issues the MMAs, warps 2-5 are the softmax (thread = query).  S = Q K' lands in 64 columns, the weights replace it
@@ -234,58 +266,35 @@ constexpr int FWD_THREADS = 192;
 template <int NP>
 struct FwdCfg {
   static constexpr int SLOTS = NP == 3 ? 4 : 8;
+  enum { B_FULL = 0, B_FREE = SLOTS, B_QREADY = 2 * SLOTS, B_SFULL, B_PREADY, B_OFULL, B_COUNT };
   static constexpr int SLOT_BYTES = NP * TILE;
   static constexpr int BAR = SLOTS * SLOT_BYTES;
-  static constexpr int SMEM = BAR + 256 + 1024;
+  static constexpr int NOTES = BAR + 8 * B_COUNT * (NP == 3 ? PICK_ITEMS : 1);
+  static constexpr int SMEM = NOTES + 64 + 1024;
+  static __device__ __forceinline__ void init(uint32_t bar0) {
+    for (int s = 0; s < 2 * SLOTS; ++s) mbar_init(bar0 + 8u * (uint32_t)s, 1);
+    mbar_init(bar0 + 8u * B_QREADY, 4);
+    mbar_init(bar0 + 8u * B_SFULL, 1);
+    mbar_init(bar0 + 8u * B_PREADY, 4);
+    mbar_init(bar0 + 8u * B_OFULL, 1);
+  }
 };
 
+// Queries i0 .. i0 + 127 of head h, batch entry b.
 template <int NP>
-__global__ void __launch_bounds__(FWD_THREADS, 2)
-attn_fwd_tc_kernel(const void* __restrict__ qmat, const uint8_t* __restrict__ kimg, const uint8_t* __restrict__ vimg,
-                   float* __restrict__ o, uint16_t* __restrict__ o16, float* __restrict__ lse, uint8_t* __restrict__ odd_q, int odd_n,
-                   AtcDims D, int32_t* __restrict__ dev_err) {
-  fb_after_previous();
+__device__ __forceinline__ void fwd_item(const Cta& cta, uint32_t bar0, int64_t i0, int h, int64_t b, const void* __restrict__ qmat, const uint8_t* __restrict__ kimg,
+                                         const uint8_t* __restrict__ vimg, float* __restrict__ o, uint16_t* __restrict__ o16, float* __restrict__ lse,
+                                         uint8_t* __restrict__ odd_q, int odd_n, const AtcDims& D) {
   using cfg = FwdCfg<NP>;
-  constexpr int S = cfg::SLOTS;
-  enum { B_FULL = 0, B_FREE = S, B_QREADY = 2 * S, B_SFULL, B_PREADY, B_OFULL, B_COUNT };
-  extern __shared__ uint8_t smem_raw[];
-  const Shared sh = aligned_smem(smem_raw);
-  const uint32_t sb = sh.sb, bar0 = sb + cfg::BAR;
+  constexpr int S = cfg::SLOTS, B_FULL = cfg::B_FULL, B_FREE = cfg::B_FREE, B_QREADY = cfg::B_QREADY, B_SFULL = cfg::B_SFULL, B_PREADY = cfg::B_PREADY, B_OFULL = cfg::B_OFULL;
+  const uint32_t sb = cta.sb, tmem = cta.tmem;
+  volatile int* s_abort = cta.s_abort;
+  const int warp = cta.warp, lane = cta.lane;
   auto bar = [&](int i) { return bar0 + 8u * (uint32_t)i; };
-  volatile uint32_t* s_tmem = (volatile uint32_t*)(sh.smem + cfg::BAR + 8 * B_COUNT);
-  volatile int* s_abort = (volatile int*)(s_tmem + 1);
-  volatile int* s_skip = (volatile int*)(s_tmem + 2);
-
-  const int warp = uniform_warp(), lane = threadIdx.x & 31;
-  // causal: the last query tiles have the most key blocks, so they are scheduled first
-  const int64_t i0 = (int64_t)(D.causal ? gridDim.x - 1 - blockIdx.x : blockIdx.x) * QT;
-  const int h = blockIdx.y;
-  const int64_t b = blockIdx.z, bh = b * D.H + h;
+  const int64_t bh = b * D.H + h;
   int64_t kv_end = D.Lk;
   if (D.causal && i0 + QT < kv_end) kv_end = i0 + QT;
   const int nkb = (int)((kv_end + KT - 1) / KT);
-
-  if (threadIdx.x == 0) {
-    for (int s = 0; s < S; ++s) {
-      mbar_init(bar(B_FULL + s), 1);
-      mbar_init(bar(B_FREE + s), 1);
-    }
-    mbar_init(bar(B_QREADY), 4);
-    mbar_init(bar(B_SFULL), 1);
-    mbar_init(bar(B_PREADY), 4);
-    mbar_init(bar(B_OFULL), 1);
-    *s_abort = 0;
-    *s_skip = (*(volatile int32_t*)dev_err != 0) ? 1 : 0;
-    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-    fence_proxy_async();
-  }
-  __syncthreads();
-  if (*s_skip != 0) return;
-  if (warp == 1) tmem_alloc(s_tmem, 256u);
-  tc_fence_before();
-  __syncthreads();
-  tc_fence_after();
-  const uint32_t tmem = __reduce_or_sync(0xffffffffu, *s_tmem);
   constexpr uint32_t T_R = 96, T_O = 192;
 
   if (warp == 0) {
@@ -335,7 +344,7 @@ attn_fwd_tc_kernel(const void* __restrict__ qmat, const uint8_t* __restrict__ ki
     const int64_t el = NP == 3 ? 4 : 2;
     const bool odd = row_to_tmem<NP>((const uint8_t*)qmat + el * ((b * D.Lq + gi) * D.E + (int64_t)h * D.d), D.d, live, D.vec != 0, t_row);
     const bool any = __any_sync(0xffffffffu, odd);
-    if (lane == 0) odd_q[bh * odd_n + (int)(i0 / QT) * 4 + q] = any ? 1 : 0;
+    if (NP == 1 && lane == 0) odd_q[bh * odd_n + (int)(i0 / QT) * 4 + q] = any ? 1 : 0;
     tc_wait_st();
     tc_fence_before();
     __syncwarp();
@@ -422,20 +431,53 @@ attn_fwd_tc_kernel(const void* __restrict__ qmat, const uint8_t* __restrict__ ki
       const int64_t off = (b * D.Lq + gi) * D.Ev + (int64_t)h * D.dv;
 #pragma unroll
       for (int hf = 0; hf < 2; ++hf) {
-        if (o != nullptr) store_row32<false>(o + off, 32 * hf, D.dv, D.vec != 0, acc + 32 * hf, inv);
+        if (NP == 3 || o != nullptr) store_row32<false>(o + off, 32 * hf, D.dv, D.vec != 0, acc + 32 * hf, inv);
         if (NP == 1) store_row32<true>(o16 + off, 32 * hf, D.dv, true, acc + 32 * hf, inv);
       }
       lse[bh * D.Lq + gi] = (l > 0.0f) ? m * D.scale + logf(l) : -INFINITY;
     }
   }
+}
 
-  tc_fence_before();
-  __syncthreads();
-  if (warp == 1) {
-    __syncwarp();
-    tmem_free(tmem, 256u);
+__global__ void __launch_bounds__(FWD_THREADS, 2)
+attn_fwd_tc_kernel(const uint16_t* __restrict__ q, const uint8_t* __restrict__ kimg, const uint8_t* __restrict__ vimg, float* __restrict__ o,
+                   uint16_t* __restrict__ o16, float* __restrict__ lse, uint8_t* __restrict__ odd_q, int odd_n, AtcDims D, int32_t* __restrict__ dev_err) {
+  fb_after_previous();
+  extern __shared__ uint8_t smem_raw[];
+  Cta cta;
+  if (!cta_begin(cta, smem_raw, FwdCfg<1>::NOTES, 256u, dev_err, [](uint32_t sb) { FwdCfg<1>::init(sb + FwdCfg<1>::BAR); })) return;
+  // causal: the last query tiles have the most key blocks, so they are scheduled first
+  const int64_t i0 = (int64_t)(D.causal ? gridDim.x - 1 - blockIdx.x : blockIdx.x) * QT;
+  fwd_item<1>(cta, cta.sb + FwdCfg<1>::BAR, i0, (int)blockIdx.y, (int64_t)blockIdx.z, q, kimg, vimg, o, o16, lse, odd_q, odd_n, D);
+  cta_end(cta, 256u, dev_err, 4002);
+}
+
+// Float32 heads, picked ones
+__global__ void __launch_bounds__(FWD_THREADS, 2)
+attn_fwd_picked_kernel(const float* __restrict__ q, const uint8_t* __restrict__ kimg, const uint8_t* __restrict__ vimg, float* __restrict__ o, float* __restrict__ lse,
+                       const uint8_t* __restrict__ pick, int64_t items, AtcDims D, int32_t* __restrict__ dev_err) {
+  fb_after_previous();
+  fb_let_next_start();
+  extern __shared__ uint8_t smem_raw[];
+  const int tiles = D.qtiles / 2;
+  const int64_t heads = items / tiles;
+  auto head_of = [&](int64_t item) { return item % heads; };
+  const uint32_t mine = picked_items(pick, items, head_of);
+  if (mine == 0) return;
+  using cfg = FwdCfg<3>;
+  auto bars = [](uint32_t sb, int n) { return sb + (uint32_t)(cfg::BAR + 8 * cfg::B_COUNT * n); };
+  Cta cta;
+  if (!cta_begin(cta, smem_raw, cfg::NOTES, 256u, dev_err, [&](uint32_t sb) {
+        for (int n = 0; n < PICK_ITEMS; ++n) cfg::init(bars(sb, n));
+      }))
+    return;
+  for (int n = 0; n < PICK_ITEMS; ++n) {
+    if (!(mine >> n & 1)) continue;
+    const int64_t item = blockIdx.x + (int64_t)n * gridDim.x, bh = head_of(item), b = bh / D.H;
+    fwd_item<3>(cta, bars(cta.sb, n), (tiles - 1 - item / heads) * QT, (int)(bh - b * D.H), b, q, kimg, vimg, o, nullptr, lse, nullptr, 0, D);
+    if (!cta_next(cta)) break;
   }
-  if (threadIdx.x == 0 && *s_abort != 0) atomicExch(dev_err, 4002);
+  cta_end(cta, 256u, dev_err, 4002);
 }
 
 // ----------------------------------------------------------------------------------------------------------- dQ ---
@@ -449,59 +491,30 @@ attn_fwd_tc_kernel(const void* __restrict__ qmat, const uint8_t* __restrict__ ki
 template <int NP>
 struct DqCfg {
   static constexpr int SLOTS = NP == 3 ? 4 : 6;
+  enum { B_FULL = 0, B_FREE = SLOTS, B_QREADY = 2 * SLOTS, B_SFULL, B_DSREADY = B_SFULL + 2, B_DONE = B_DSREADY + 2, B_COUNT };
   static constexpr int SLOT_BYTES = 2 * NP * TILE;   // K tile, V tile
   static constexpr int BAR = SLOTS * SLOT_BYTES;
-  static constexpr int SMEM = BAR + 256 + 1024;
+  static constexpr int NOTES = BAR + 8 * B_COUNT * (NP == 3 ? PICK_ITEMS : 1);
+  static constexpr int SMEM = NOTES + 64 + 1024;
+  static __device__ __forceinline__ void init(uint32_t bar0) {
+    for (int s = 0; s < B_COUNT; ++s) mbar_init(bar0 + 8u * (uint32_t)s, s == B_QREADY ? 8 : s == B_DSREADY || s == B_DSREADY + 1 ? 4 : 1);
+  }
 };
 
 template <int NP>
-__global__ void __launch_bounds__(BWD_THREADS, 1)
-attn_bwd_dq_tc_kernel(const void* __restrict__ q, const void* __restrict__ dout, const uint8_t* __restrict__ kimg,
-                      const uint8_t* __restrict__ vimg, const float2* __restrict__ rv, void* __restrict__ dq, AtcDims D,
-                      int32_t* __restrict__ dev_err) {
-  fb_after_previous();
+__device__ __forceinline__ void dq_item(const Cta& cta, uint32_t bar0, int64_t i0, int h, int64_t b, const void* __restrict__ q, const void* __restrict__ dout,
+                                        const uint8_t* __restrict__ kimg, const uint8_t* __restrict__ vimg, const float2* __restrict__ rv, void* __restrict__ dq,
+                                        const AtcDims& D) {
   using cfg = DqCfg<NP>;
-  constexpr int S = cfg::SLOTS;
-  enum { B_FULL = 0, B_FREE = S, B_QREADY = 2 * S, B_SFULL, B_DSREADY = B_SFULL + 2, B_DONE = B_DSREADY + 2, B_COUNT };
-  extern __shared__ uint8_t smem_raw[];
-  const Shared sh = aligned_smem(smem_raw);
-  const uint32_t sb = sh.sb, bar0 = sb + cfg::BAR;
+  constexpr int S = cfg::SLOTS, B_FULL = cfg::B_FULL, B_FREE = cfg::B_FREE, B_QREADY = cfg::B_QREADY, B_SFULL = cfg::B_SFULL, B_DSREADY = cfg::B_DSREADY, B_DONE = cfg::B_DONE;
+  const uint32_t sb = cta.sb, tmem = cta.tmem;
+  volatile int* s_abort = cta.s_abort;
+  const int warp = cta.warp, lane = cta.lane;
   auto bar = [&](int i) { return bar0 + 8u * (uint32_t)i; };
-  volatile uint32_t* s_tmem = (volatile uint32_t*)(sh.smem + cfg::BAR + 8 * B_COUNT);
-  volatile int* s_abort = (volatile int*)(s_tmem + 1);
-  volatile int* s_skip = (volatile int*)(s_tmem + 2);
-
-  const int warp = uniform_warp(), lane = threadIdx.x & 31;
-  const int64_t i0 = (int64_t)(D.causal ? gridDim.x - 1 - blockIdx.x : blockIdx.x) * QT;
-  const int h = blockIdx.y;
-  const int64_t b = blockIdx.z, bh = b * D.H + h;
+  const int64_t bh = b * D.H + h;
   int64_t kv_end = D.Lk;
   if (D.causal && i0 + QT < kv_end) kv_end = i0 + QT;
   const int nkb = (int)((kv_end + KT - 1) / KT);
-
-  if (threadIdx.x == 0) {
-    for (int s = 0; s < S; ++s) {
-      mbar_init(bar(B_FULL + s), 1);
-      mbar_init(bar(B_FREE + s), 1);
-    }
-    mbar_init(bar(B_QREADY), 8);
-    for (int r = 0; r < 2; ++r) {
-      mbar_init(bar(B_SFULL + r), 1);
-      mbar_init(bar(B_DSREADY + r), 4);
-    }
-    mbar_init(bar(B_DONE), 1);
-    *s_abort = 0;
-    *s_skip = (*(volatile int32_t*)dev_err != 0) ? 1 : 0;
-    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-    fence_proxy_async();
-  }
-  __syncthreads();
-  if (*s_skip != 0) return;
-  if (warp == 1) tmem_alloc(s_tmem, 512u);
-  tc_fence_before();
-  __syncthreads();
-  tc_fence_after();
-  const uint32_t tmem = __reduce_or_sync(0xffffffffu, *s_tmem);
   constexpr uint32_t T_DO = 96, T_R = 192, T_DQ = 448;
 
   if (warp == 0) {
@@ -609,14 +622,18 @@ attn_bwd_dq_tc_kernel(const void* __restrict__ q, const void* __restrict__ dout,
         store_row32<NP == 1>((uint8_t*)dq + el * ((b * D.Lq + gi) * D.E + (int64_t)h * D.d), 32 * set, D.d, D.vec != 0, (const float*)v, D.scale);
     }
   }
+}
 
-  tc_fence_before();
-  __syncthreads();
-  if (warp == 1) {
-    __syncwarp();
-    tmem_free(tmem, 512u);
-  }
-  if (threadIdx.x == 0 && *s_abort != 0) atomicExch(dev_err, 4003);
+__global__ void __launch_bounds__(BWD_THREADS, 1)
+attn_bwd_dq_tc_kernel(const uint16_t* __restrict__ q, const uint16_t* __restrict__ dout, const uint8_t* __restrict__ kimg, const uint8_t* __restrict__ vimg,
+                      const float2* __restrict__ rv, uint16_t* __restrict__ dq, AtcDims D, int32_t* __restrict__ dev_err) {
+  fb_after_previous();
+  extern __shared__ uint8_t smem_raw[];
+  Cta cta;
+  if (!cta_begin(cta, smem_raw, DqCfg<1>::NOTES, 512u, dev_err, [](uint32_t sb) { DqCfg<1>::init(sb + DqCfg<1>::BAR); })) return;
+  const int64_t i0 = (int64_t)(D.causal ? gridDim.x - 1 - blockIdx.x : blockIdx.x) * QT;
+  dq_item<1>(cta, cta.sb + DqCfg<1>::BAR, i0, (int)blockIdx.y, (int64_t)blockIdx.z, q, dout, kimg, vimg, rv, dq, D);
+  cta_end(cta, 512u, dev_err, 4003);
 }
 
 // ------------------------------------------------------------------------------------------------------ dK, dV ---
@@ -633,60 +650,32 @@ attn_bwd_dq_tc_kernel(const void* __restrict__ q, const void* __restrict__ dout,
 template <int NP>
 struct KvCfg {
   static constexpr int SLOTS = NP == 3 ? 5 : 8;
+  enum { B_FULL = 0, B_FREE = SLOTS, B_KV = 2 * SLOTS, B_SFULL, B_PREADY = B_SFULL + 2, B_DONE = B_PREADY + 2, B_COUNT };
   static constexpr int SLOT_BYTES = NP * TILE + 1024;   // a tile and, behind dO, {lse, delta} of its 64 queries
   static constexpr int K_OFF = SLOTS * SLOT_BYTES, V_OFF = K_OFF + NP * 2 * TILE;
   static constexpr int BAR = V_OFF + NP * 2 * TILE;
-  static constexpr int SMEM = BAR + 256 + 1024;
+  static constexpr int NOTES = BAR + 8 * B_COUNT * (NP == 3 ? PICK_ITEMS : 1);
+  static constexpr int SMEM = NOTES + 64 + 1024;
+  static __device__ __forceinline__ void init(uint32_t bar0) {
+    for (int s = 0; s < B_COUNT; ++s) mbar_init(bar0 + 8u * (uint32_t)s, s == B_PREADY || s == B_PREADY + 1 ? 4 : 1);
+  }
 };
 
+// Keys j0 .. j0 + 127 of head h, batch entry b.
 template <int NP>
-__global__ void __launch_bounds__(BWD_THREADS, 1)
-attn_bwd_dkdv_tc_kernel(const uint8_t* __restrict__ qimg, const uint8_t* __restrict__ doimg, const uint8_t* __restrict__ kimg,
-                        const uint8_t* __restrict__ vimg, const float2* __restrict__ rv, void* __restrict__ dk, void* __restrict__ dv,
-                        AtcDims D, int32_t* __restrict__ dev_err) {
-  fb_after_previous();
+__device__ __forceinline__ void dkdv_item(const Cta& cta, uint32_t bar0, int64_t j0, int h, int64_t b, const uint8_t* __restrict__ qimg, const uint8_t* __restrict__ doimg,
+                                          const uint8_t* __restrict__ kimg, const uint8_t* __restrict__ vimg, const float2* __restrict__ rv, void* __restrict__ dk,
+                                          void* __restrict__ dv, const AtcDims& D) {
   using cfg = KvCfg<NP>;
-  constexpr int S = cfg::SLOTS;
-  enum { B_FULL = 0, B_FREE = S, B_KV = 2 * S, B_SFULL, B_PREADY = B_SFULL + 2, B_DONE = B_PREADY + 2, B_COUNT };
-  extern __shared__ uint8_t smem_raw[];
-  const Shared sh = aligned_smem(smem_raw);
-  const uint32_t sb = sh.sb, bar0 = sb + cfg::BAR;
+  constexpr int S = cfg::SLOTS, B_FULL = cfg::B_FULL, B_FREE = cfg::B_FREE, B_KV = cfg::B_KV, B_SFULL = cfg::B_SFULL, B_PREADY = cfg::B_PREADY, B_DONE = cfg::B_DONE;
+  const uint32_t sb = cta.sb, tmem = cta.tmem;
+  volatile int* s_abort = cta.s_abort;
+  const int warp = cta.warp, lane = cta.lane;
   auto bar = [&](int i) { return bar0 + 8u * (uint32_t)i; };
-  volatile uint32_t* s_tmem = (volatile uint32_t*)(sh.smem + cfg::BAR + 8 * B_COUNT);
-  volatile int* s_abort = (volatile int*)(s_tmem + 1);
-  volatile int* s_skip = (volatile int*)(s_tmem + 2);
-
-  const int warp = uniform_warp(), lane = threadIdx.x & 31;
-  const int64_t j0 = (int64_t)blockIdx.x * QT;   // first key of this CTA
-  const int h = blockIdx.y;
-  const int64_t b = blockIdx.z, bh = b * D.H + h;
+  const int64_t bh = b * D.H + h;
   // query blocks that see these keys: all of them, or under a causal mask those from the diagonal on
   const int ib0 = D.causal ? (int)(j0 / KT) : 0;
   const int nqb = (int)((D.Lq + KT - 1) / KT) - ib0;   // may be <= 0: nothing attends to these keys
-
-  if (threadIdx.x == 0) {
-    for (int s = 0; s < S; ++s) {
-      mbar_init(bar(B_FULL + s), 1);
-      mbar_init(bar(B_FREE + s), 1);
-    }
-    mbar_init(bar(B_KV), 1);
-    for (int r = 0; r < 2; ++r) {
-      mbar_init(bar(B_SFULL + r), 1);
-      mbar_init(bar(B_PREADY + r), 4);
-    }
-    mbar_init(bar(B_DONE), 1);
-    *s_abort = 0;
-    *s_skip = (*(volatile int32_t*)dev_err != 0) ? 1 : 0;
-    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-    fence_proxy_async();
-  }
-  __syncthreads();
-  if (*s_skip != 0) return;
-  if (warp == 1) tmem_alloc(s_tmem, 512u);
-  tc_fence_before();
-  __syncthreads();
-  tc_fence_after();
-  const uint32_t tmem = __reduce_or_sync(0xffffffffu, *s_tmem);
   constexpr uint32_t T_DV = 384, T_DK = 448;
 
   if (warp == 0) {
@@ -697,7 +686,7 @@ attn_bwd_dkdv_tc_kernel(const uint8_t* __restrict__ qimg, const uint8_t* __restr
       for (int p = 0; p < NP; ++p)
 #pragma unroll
         for (int t = 0; t < 2; ++t) {   // plane p of the CTA's two 64-key tiles, one after the other
-          const int64_t off = ((bh * D.ktiles + 2 * (int64_t)blockIdx.x + t) * NP + p) * (int64_t)TILE;
+          const int64_t off = ((bh * D.ktiles + j0 / KT + t) * NP + p) * (int64_t)TILE;
           bulk_load(sb + (uint32_t)(cfg::K_OFF + (2 * p + t) * TILE), kimg + off, TILE, bar(B_KV));
           bulk_load(sb + (uint32_t)(cfg::V_OFF + (2 * p + t) * TILE), vimg + off, TILE, bar(B_KV));
         }
@@ -761,7 +750,7 @@ attn_bwd_dkdv_tc_kernel(const uint8_t* __restrict__ qimg, const uint8_t* __restr
       ok = mbar_wait(bar(B_FULL + n % S), (uint32_t)(n / S) & 1u, s_abort) && mbar_wait(bar(B_SFULL + set), (uint32_t)(i >> 1) & 1u, s_abort);
       if (!ok) break;
       tc_fence_after();
-      const float4* row = (const float4*)(sh.smem + (n % S) * cfg::SLOT_BYTES + NP * TILE);   // {lse, delta} of two queries
+      const float4* row = (const float4*)(cta.smem + (n % S) * cfg::SLOT_BYTES + NP * TILE);   // {lse, delta} of two queries
       // queries of the block this key is seen by: query < Lq (dead ones carry lse = inf), and query >= key when causal
       const int64_t i0b = (int64_t)(ib0 + i) * KT;
       int clo = 0;
@@ -815,14 +804,61 @@ attn_bwd_dkdv_tc_kernel(const uint8_t* __restrict__ qimg, const uint8_t* __restr
       }
     }
   }
+}
 
-  tc_fence_before();
-  __syncthreads();
-  if (warp == 1) {
-    __syncwarp();
-    tmem_free(tmem, 512u);
+__global__ void __launch_bounds__(BWD_THREADS, 1)
+attn_bwd_dkdv_tc_kernel(const uint8_t* __restrict__ qimg, const uint8_t* __restrict__ doimg, const uint8_t* __restrict__ kimg, const uint8_t* __restrict__ vimg,
+                        const float2* __restrict__ rv, uint16_t* __restrict__ dk, uint16_t* __restrict__ dv, AtcDims D, int32_t* __restrict__ dev_err) {
+  fb_after_previous();
+  extern __shared__ uint8_t smem_raw[];
+  Cta cta;
+  if (!cta_begin(cta, smem_raw, KvCfg<1>::NOTES, 512u, dev_err, [](uint32_t sb) { KvCfg<1>::init(sb + KvCfg<1>::BAR); })) return;
+  dkdv_item<1>(cta, cta.sb + KvCfg<1>::BAR, (int64_t)blockIdx.x * QT, (int)blockIdx.y, (int64_t)blockIdx.z, qimg, doimg, kimg, vimg, rv, dk, dv, D);
+  cta_end(cta, 512u, dev_err, 4004);
+}
+
+// Float32 heads, picked ones: kv_items items of dK and dV, then those of dQ (each may be none)
+__global__ void __launch_bounds__(BWD_THREADS, 1)
+attn_bwd_picked_kernel(const float* __restrict__ q, const float* __restrict__ dout, const uint8_t* __restrict__ kimg, const uint8_t* __restrict__ vimg,
+                       const uint8_t* __restrict__ qimg, const uint8_t* __restrict__ doimg, const float2* __restrict__ rv, float* __restrict__ dq,
+                       float* __restrict__ dk, float* __restrict__ dv, const uint8_t* __restrict__ pick, int64_t kv_items, int64_t items, AtcDims D,
+                       int32_t* __restrict__ dev_err) {
+  fb_after_previous();
+  fb_let_next_start();
+  extern __shared__ uint8_t smem_raw[];
+  const int64_t heads = kv_items > 0 ? kv_items / (D.ktiles / 2) : items / (D.qtiles / 2);
+  auto head_of = [&](int64_t item) { return (item < kv_items ? item : item - kv_items) % heads; };
+  const uint32_t mine = picked_items(pick, items, head_of);
+  if (mine == 0) return;
+  using kv = KvCfg<3>;
+  using qc = DqCfg<3>;
+  static_assert((int)qc::B_COUNT <= (int)kv::B_COUNT && qc::BAR <= kv::BAR, "one layout");
+  auto bars = [](uint32_t sb, int n) { return sb + (uint32_t)(kv::BAR + 8 * kv::B_COUNT * n); };
+  Cta cta;
+  if (!cta_begin(cta, smem_raw, kv::NOTES, 512u, dev_err, [&](uint32_t sb) {
+        for (int n = 0; n < PICK_ITEMS; ++n) {
+          if (blockIdx.x + (int64_t)n * gridDim.x < kv_items) kv::init(bars(sb, n));
+          else qc::init(bars(sb, n));
+        }
+      }))
+    return;
+  for (int n = 0; n < PICK_ITEMS; ++n) {
+    if (!(mine >> n & 1)) continue;
+    const int64_t item = blockIdx.x + (int64_t)n * gridDim.x, bh = head_of(item), b = bh / D.H;
+    const int h = (int)(bh - b * D.H);
+    if (item < kv_items) dkdv_item<3>(cta, bars(cta.sb, n), item / heads * QT, h, b, qimg, doimg, kimg, vimg, rv, dk, dv, D);
+    else dq_item<3>(cta, bars(cta.sb, n), (D.qtiles / 2 - 1 - (item - kv_items) / heads) * QT, h, b, q, dout, kimg, vimg, rv, dq, D);
+    if (!cta_next(cta)) break;
   }
-  if (threadIdx.x == 0 && *s_abort != 0) atomicExch(dev_err, 4004);
+  cta_end(cta, 512u, dev_err, 4004);
+}
+
+// CTAs for so many items: what the GPU holds at once, or more where a CTA would have more than PICK_ITEMS; an odd number beyond one item each, so that the
+// tiles of a single head (items that lie the number of heads apart) are different CTAs'.
+unsigned pick_grid(int64_t items, int64_t resident) {
+  if (items <= resident) return (unsigned)items;
+  const int64_t least = (items + PICK_ITEMS - 1) / PICK_ITEMS;
+  return (unsigned)(least > resident ? least | 1 : (resident - 1) | 1);
 }
 
 // Heads with a value that is not finite are computed again by the FMA kernels.  Planes cannot carry one (the remainder of an infinite value
@@ -840,7 +876,7 @@ int32_t fwd_bf16(fb_ctx* ctx, cudaStream_t stream, const uint16_t* q, const uint
   const fb_temp images(ctx, stream, (size_t)(chunk * per));
   uint8_t* img = (uint8_t*)images.p;
   if (!img) return FB_ERR_UNSUPPORTED;
-  FB_ONCE(ctx, FB_CUDA(cudaFuncSetAttribute(attn_fwd_tc_kernel<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, FwdCfg<1>::SMEM)));
+  FB_ONCE(ctx, FB_CUDA(cudaFuncSetAttribute(attn_fwd_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, FwdCfg<1>::SMEM)));
   for (int64_t b0 = 0; b0 < batch; b0 += chunk) {
     const int64_t nb = b0 + chunk > batch ? batch - b0 : chunk;
     uint8_t* odd = img + nb * 2 * P.kbytes;
@@ -851,9 +887,9 @@ int32_t fwd_bf16(fb_ctx* ctx, cudaStream_t stream, const uint16_t* q, const uint
     A.H = D.H; A.vec = D.vec; A.odd = odd; A.odd_n = odd_n; A.max_tiles = D.ktiles;
     A.job[0] = {kb, img, D.Lk, D.E, D.d, D.ktiles};
     A.job[1] = {vb, img + nb * P.kbytes, D.Lk, D.Ev, D.dv, D.ktiles};
-    fb_launch(attn_split_kernel<1>, dim3((unsigned)D.ktiles, (unsigned)(nb * D.H), 2), 256, 0, stream, A);
+    fb_launch(attn_split_kernel, dim3((unsigned)D.ktiles, (unsigned)(nb * D.H), 2), 256, 0, stream, A);
     FB_LAUNCH_CHECK();
-    fb_launch(attn_fwd_tc_kernel<1>, dim3((unsigned)(D.qtiles / 2), (unsigned)D.H, (unsigned)nb), FWD_THREADS, FwdCfg<1>::SMEM, stream, qb, img, img + nb * P.kbytes, ob, ob16, lb,
+    fb_launch(attn_fwd_tc_kernel, dim3((unsigned)(D.qtiles / 2), (unsigned)D.H, (unsigned)nb), FWD_THREADS, FwdCfg<1>::SMEM, stream, qb, img, img + nb * P.kbytes, ob, ob16, lb,
               odd + 2 * D.ktiles, odd_n, D, ctx->dev_error);
     FB_LAUNCH_CHECK();
     const int32_t st = fb_attn_fwd_redo(ctx, stream, 1, qb, kb, vb, ob, ob16, lb, D.E, D.Ev, D.Lq, D.Lk, nb, D.H, D.causal, odd, odd_n);
@@ -872,8 +908,8 @@ int32_t bwd_bf16(fb_ctx* ctx, cudaStream_t stream, const uint16_t* q, const uint
   const fb_temp images(ctx, stream, (size_t)(chunk * per));
   uint8_t* img = (uint8_t*)images.p;
   if (!img) return FB_ERR_UNSUPPORTED;
-  FB_ONCE(ctx, FB_CUDA(cudaFuncSetAttribute(attn_bwd_dkdv_tc_kernel<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, KvCfg<1>::SMEM)));
-  FB_ONCE(ctx, FB_CUDA(cudaFuncSetAttribute(attn_bwd_dq_tc_kernel<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, DqCfg<1>::SMEM)));
+  FB_ONCE(ctx, FB_CUDA(cudaFuncSetAttribute(attn_bwd_dkdv_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, KvCfg<1>::SMEM)));
+  FB_ONCE(ctx, FB_CUDA(cudaFuncSetAttribute(attn_bwd_dq_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, DqCfg<1>::SMEM)));
   for (int64_t b0 = 0; b0 < batch; b0 += chunk) {
     const int64_t nb = b0 + chunk > batch ? batch - b0 : chunk;
     uint8_t *ki = img, *vi = ki + nb * P.kbytes, *qi = vi + nb * P.kbytes, *doi = qi + nb * P.qbytes;
@@ -891,12 +927,12 @@ int32_t bwd_bf16(fb_ctx* ctx, cudaStream_t stream, const uint16_t* q, const uint
     A.o = o + qvoff; A.lse = lb; A.rv = rv;
     // (tiles that one operand has and another has not keep no byte)
     if (D.qtiles != D.ktiles) FB_CUDA(cudaMemsetAsync(odd, 0, (size_t)(nb * D.H * odd_n), stream));
-    fb_launch(attn_split_kernel<1>, dim3((unsigned)D.max_tiles, (unsigned)(nb * D.H), 4), 256, 0, stream, A);
+    fb_launch(attn_split_kernel, dim3((unsigned)D.max_tiles, (unsigned)(nb * D.H), 4), 256, 0, stream, A);
     FB_LAUNCH_CHECK();
-    fb_launch(attn_bwd_dkdv_tc_kernel<1>, dim3((unsigned)(D.ktiles / 2), (unsigned)D.H, (unsigned)nb), BWD_THREADS, KvCfg<1>::SMEM, stream, qi, doi, ki, vi, rv, dk + koff,
+    fb_launch(attn_bwd_dkdv_tc_kernel, dim3((unsigned)(D.ktiles / 2), (unsigned)D.H, (unsigned)nb), BWD_THREADS, KvCfg<1>::SMEM, stream, qi, doi, ki, vi, rv, dk + koff,
               dv + kvoff, D, ctx->dev_error);
     FB_LAUNCH_CHECK();
-    fb_launch(attn_bwd_dq_tc_kernel<1>, dim3((unsigned)(D.qtiles / 2), (unsigned)D.H, (unsigned)nb), BWD_THREADS, DqCfg<1>::SMEM, stream, qb, dob, ki, vi, rv, dq + qoff, D,
+    fb_launch(attn_bwd_dq_tc_kernel, dim3((unsigned)(D.qtiles / 2), (unsigned)D.H, (unsigned)nb), BWD_THREADS, DqCfg<1>::SMEM, stream, qb, dob, ki, vi, rv, dq + qoff, D,
               ctx->dev_error);
     FB_LAUNCH_CHECK();
     const int32_t st = fb_attn_bwd_redo(ctx, stream, 1, qb, kb, vb, lb, (const float*)rv + 1, (int64_t)D.qtiles * KT, dob, dq + qoff, dk + koff, dv + kvoff, D.E, D.Ev,
@@ -907,6 +943,25 @@ int32_t bwd_bf16(fb_ctx* ctx, cudaStream_t stream, const uint16_t* q, const uint
 }
 
 }  // namespace
+
+int32_t fb_atc::fwd_picked(fb_ctx* ctx, cudaStream_t stream, const float* q, const uint8_t* kimg, const uint8_t* vimg, float* o, float* lse, const AtcDims& D, int64_t batch,
+                           const uint8_t* pick) {
+  FB_ONCE(ctx, FB_CUDA(cudaFuncSetAttribute(attn_fwd_picked_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, FwdCfg<3>::SMEM)));
+  const int64_t items = batch * D.H * (D.qtiles / 2);
+  fb_launch(attn_fwd_picked_kernel, pick_grid(items, 2 * (int64_t)ctx->sm_count), FWD_THREADS, FwdCfg<3>::SMEM, stream, q, kimg, vimg, o, lse, pick, items, D, ctx->dev_error);
+  FB_LAUNCH_CHECK();
+  return FB_OK;
+}
+
+int32_t fb_atc::bwd_picked(fb_ctx* ctx, cudaStream_t stream, const float* q, const float* dout, const uint8_t* kimg, const uint8_t* vimg, const uint8_t* qimg,
+                           const uint8_t* doimg, const float2* rv, float* dq, float* dk, float* dv, const AtcDims& D, int64_t batch, const uint8_t* pick) {
+  FB_ONCE(ctx, FB_CUDA(cudaFuncSetAttribute(attn_bwd_picked_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, KvCfg<3>::SMEM)));
+  const int64_t kv_items = dk != nullptr ? batch * D.H * (D.ktiles / 2) : 0, items = kv_items + (dq != nullptr ? batch * D.H * (D.qtiles / 2) : 0);
+  fb_launch(attn_bwd_picked_kernel, pick_grid(items, ctx->sm_count), BWD_THREADS, KvCfg<3>::SMEM, stream, q, dout, kimg, vimg, qimg, doimg, rv, dq, dk, dv, pick, kv_items,
+            items, D, ctx->dev_error);
+  FB_LAUNCH_CHECK();
+  return FB_OK;
+}
 
 // bf16 q, k, v (and dO): one plane each, outputs rounded to bf16 once.  o32 (optional in the forward call) keeps
 // the Float32 output for the backward pass.  FB_ERR_UNSUPPORTED, without a message, for every call these kernels do not

@@ -86,6 +86,16 @@ __device__ __forceinline__ uint32_t pack2(float lo, float hi) {
   return *reinterpret_cast<const uint32_t*>(&v);
 }
 
+// Two values as three bf16 planes (x in the low half of each word): truncation to the upper 16 bits leaves a remainder of
+// at most 16 significant bits, the same again one of at most 8, which is a bf16 value.
+__device__ __forceinline__ void split3(float x, float y, uint32_t& p0, uint32_t& p1, uint32_t& p2) {
+  const uint32_t xb = __float_as_uint(x), yb = __float_as_uint(y);
+  p0 = __byte_perm(xb, yb, 0x7632);
+  const float rx = x - __uint_as_float(xb & 0xffff0000u), ry = y - __uint_as_float(yb & 0xffff0000u);
+  const uint32_t rxb = __float_as_uint(rx), ryb = __float_as_uint(ry);
+  p1 = __byte_perm(rxb, ryb, 0x7632);
+  p2 = __byte_perm(__float_as_uint(rx - __uint_as_float(rxb & 0xffff0000u)), __float_as_uint(ry - __uint_as_float(ryb & 0xffff0000u)), 0x7632);
+}
 // 32 consecutive features (from c0) of one row as Float32 values; zero beyond the head size or for a dead row
 __device__ __forceinline__ void row_f32(const float* src, int c0, int width, bool live, bool vec, uint32_t* v) {
   if (vec) {
@@ -194,5 +204,12 @@ inline bool make_plan(AtcPlan* P, int np, int64_t e_dim, int64_t ev_dim, int64_t
   P->rvbytes = (int64_t)nheads * D.qtiles * KT * (int64_t)sizeof(float2);
   return true;
 }
+
+// attention_tc.cu: Float32 heads on three bf16 planes, those with a byte of `pick` set (one per (batch, head)).  Images of three planes a tile;
+// dq, or dk and dv, may be NULL.
+int32_t fwd_picked(fb_ctx* ctx, cudaStream_t stream, const float* q, const uint8_t* kimg, const uint8_t* vimg, float* o, float* lse, const AtcDims& D, int64_t batch,
+                   const uint8_t* pick);
+int32_t bwd_picked(fb_ctx* ctx, cudaStream_t stream, const float* q, const float* dout, const uint8_t* kimg, const uint8_t* vimg, const uint8_t* qimg,
+                   const uint8_t* doimg, const float2* rv, float* dq, float* dk, float* dv, const AtcDims& D, int64_t batch, const uint8_t* pick);
 
 }  // namespace fb_atc

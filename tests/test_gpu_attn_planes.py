@@ -391,3 +391,127 @@ def test_bf16_gradients_of_values_with_small_weights(scores, heads, n, batch, ca
     got, want = split(dv)[counts], split(ref[3])[counts]
     err = float(((got - want).norm(dim=1) / want.norm(dim=1)).max())
     assert err < 4e-3, err
+
+
+def _f32_call(q, k, v, do, d, dv, heads, causal):
+    """[o, lse, dq, dk, dv] through the Float32 entry points."""
+    import fluxb200 as F
+    from fluxb200 import lib
+    ctx, (batch, lq, _), lk = F.context(), q.shape, k.shape[1]
+    p, dims = lambda t: t.data_ptr(), (heads * d, heads * dv, lq, lk, batch, heads, causal)
+    o, lse = torch.full_like(do, float("nan")), torch.full((batch * heads * lq,), float("nan"), device="cuda")
+    dq, dk, dvv = (torch.full_like(t, float("nan")) for t in (q, k, v))
+    lib.call("fb_attn_fwd", ctx.handle, ctx.stream, p(q), p(k), p(v), None, p(o), p(lse), *dims)
+    lib.call("fb_attn_bwd", ctx.handle, ctx.stream, p(q), p(k), p(v), None, p(o), p(lse), p(do), p(dq), p(dk), p(dvv), *dims)
+    assert ctx.device_error() == 0
+    return [o, lse, dq, dk, dvv]
+
+
+@pytest.mark.parametrize("d,dv,heads,lq,lk,batch,causal", CASES)
+@pytest.mark.parametrize("shift", [0, 1])
+def test_heads_with_large_scores(d, dv, heads, lq, lk, batch, causal, shift):
+    """Scores eight times the ordinary ones: heads of three bf16 planes.  5e-5 as for the ordinary ones."""
+    g = torch.Generator(device="cuda").manual_seed(lq + 3 * lk + d)
+    mk = lambda n, size, s=1.0: (torch.randn(batch * n * size + 4, device="cuda", generator=g) * s)[shift:shift + batch * n * size].view(batch, n, size)
+    q, k, v, do = mk(lq, heads * d, 8.0), mk(lk, heads * d), mk(lk, heads * dv), mk(lq, heads * dv)
+    o, _, dq, dk, dvv = _f32_call(q, k, v, do, d, dv, heads, causal)
+    for name, got, ref in zip(("o", "dq", "dk", "dv"), (o, dq, dk, dvv), _reference(q, k, v, do, d, dv, heads, causal)):
+        assert _err(got, ref) < 5e-5, (name, _err(got, ref))
+
+
+@pytest.mark.parametrize("heads,n,batch", [(2, 512, 1), (3, 300, 2)])
+def test_a_key_and_a_value_far_above_the_others(heads, n, batch):
+    """One key 1e4 times the others (and read by a feature of Q as much smaller), one value 1e4 times: scores of some thousand, in which 2^-24
+    of the operands is 1e-4 of a weight.  Three bf16 planes: output 6e-7, dQ 1.6e-4, dV 2.5e-4 (23 bits: 3.6e-6, 4.3e-3, 1.7e-3)."""
+    g = torch.Generator(device="cuda").manual_seed(5)
+    q, k, v, do = (torch.randn(batch, n, 64 * heads, device="cuda", generator=g) for _ in range(4))
+    k[:, 5] *= 1e4
+    q[:, :, ::64] *= 1e-4
+    v[:, 7] *= 1e4
+    o, _, dq, dk, dv = _f32_call(q, k, v, do, 64, 64, heads, 1)
+    ref = _reference(q, k, v, do, 64, 64, heads, 1)
+    for name, got, want, tol in zip(("o", "dq", "dk", "dv"), (o, dq, dk, dv), ref, (1.5e-6, 5e-4, 2e-5, 7e-4)):
+        assert _err(got, want) < tol, (name, _err(got, want))
+
+
+@pytest.mark.parametrize("heads,lq,lk,batch,causal", [(2, 300, 300, 2, 1), (3, 130, 450, 1, 0), (1, 64, 64, 1, 0), (2, 1, 9, 3, 0), (1, 700, 65, 1, 1), (2, 2048, 2048, 1, 1)])
+def test_picked_heads_have_the_bits_of_bf16_operands(heads, lq, lk, batch, causal):
+    """Float32 operands that are bf16 values: their lower planes are zeros, which add nothing, so outputs and gradients are those of the bf16
+    entry points before their rounding."""
+    import fluxb200 as F
+    from fluxb200 import lib
+    g = torch.Generator(device="cuda").manual_seed(lq)
+    E, ctx = 64 * heads, F.context()
+    low = [(torch.randn(batch, n, E, device="cuda", generator=g) * s).bfloat16() for n, s in ((lq, 9.0), (lk, 1.0), (lk, 1.0), (lq, 1.0))]
+    o, lse, dq, dk, dv = _f32_call(*[t.float() for t in low], 64, 64, heads, causal)
+    q, k, v, do = low
+    p, dims = lambda t: t.data_ptr(), (E, E, lq, lk, batch, heads, causal)
+    o32, l32, out, rq, rk, rv = torch.empty_like(o), torch.empty_like(lse), *(torch.empty_like(t) for t in (q, q, k, v))
+    lib.call("fb_attn_fwd_bf16", ctx.handle, ctx.stream, p(q), p(k), p(v), p(o32), p(out), p(l32), *dims)
+    lib.call("fb_attn_bwd_bf16", ctx.handle, ctx.stream, p(q), p(k), p(v), p(o32), p(l32), p(do), p(rq), p(rk), p(rv), *dims)
+    assert torch.equal(o, o32) and torch.equal(lse, l32) and torch.equal(o.bfloat16(), out)
+    for got, want in ((dq, rq), (dk, rk), (dv, rv)):
+        assert torch.equal(got.bfloat16(), want)
+
+
+@pytest.mark.parametrize("heads,n,batch,causal,shift", [(16, 2048, 4, 1, 0), (5, 200, 3, 0, 0), (7, 130, 2, 1, 1), (33, 64, 40, 0, 0)])
+@pytest.mark.parametrize("which", ["all", "some", "none of the first"])
+def test_heads_are_picked_one_by_one(heads, n, batch, causal, shift, which):
+    """A head has the bits that it has in a call of its own, whatever the others are: up to eight picked tiles a CTA, none, and a few."""
+    g = torch.Generator(device="cuda").manual_seed(heads)
+    mk = lambda: torch.randn(batch * n * heads * 64 + 4, device="cuda", generator=g)[shift:shift + batch * n * heads * 64].view(batch, n, heads, 64)
+    q, k, v, do = mk(), mk(), mk(), mk()
+    large = torch.zeros(batch, heads, dtype=torch.bool, device="cuda")
+    if which == "all":
+        large[:] = True
+    elif which == "some":
+        large.view(-1)[::7] = True
+        large.view(-1)[3] = True
+    else:
+        large.view(-1)[-1] = True
+    q[:] = torch.where(large[:, None, :, None], q * 12.0, q)
+    flat = lambda t: t.reshape(batch, n, heads * 64) if not shift else t.view(batch, n, heads * 64)
+    got = _f32_call(*map(flat, (q, k, v, do)), 64, 64, heads, causal)
+    lse = got[1].view(batch, heads, n)
+    for b, h in ((0, 0), (0, 3), (batch - 1, heads - 1), (batch // 2, heads // 2)):
+        alone = _f32_call(*(t[b:b + 1, :, h].contiguous() for t in (q, k, v, do)), 64, 64, 1, causal)
+        assert torch.equal(lse[b, h], alone[1])
+        if shift:      # (unaligned arrays have the FMA kernels' gradients)
+            alone = alone[:1]
+        for a, r in zip([got[0]] + got[2:], [alone[0]] + alone[2:]):
+            assert torch.equal(a.view(batch, n, heads, 64)[b, :, h], r[0])
+
+
+@pytest.mark.parametrize("what,picked", [("one faint element", False), ("a faint row", True), ("a faint column", True), ("a row of zeros", False), ("tails", False)])
+@pytest.mark.parametrize("operand", [0, 1, 2, 3])
+def test_which_tiles_the_planes_hold(what, picked, operand):
+    """A position or a feature far below the rest of its tile makes its head one of three bf16 planes; single small elements and zeros do not.
+    Row by row and column by column the results are as exact as ordinary ones (5e-5; forward 2e-6)."""
+    g = torch.Generator(device="cuda").manual_seed(operand)
+    n, heads = 192, 2
+    x = [torch.randn(1, n, 64 * heads, device="cuda", generator=g) for _ in range(4)]
+    t = x[operand]
+    if what == "one faint element":
+        t[0, 70, 3] = 1e-9
+    elif what == "a faint row":
+        t[0, 70, :64] *= 2.0 ** -24
+    elif what == "a faint column":
+        t[0, 64:128, 3] *= 2.0 ** -24
+    elif what == "a row of zeros":
+        t[0, 70] = 0.0
+    else:
+        t[:] = torch.nn.functional.gelu(3.0 * t)
+    got = _f32_call(*x, 64, 64, heads, 0)
+    ref = _reference(*x, 64, 64, heads, 0)
+    for i, (name, a, r) in enumerate(zip(("o", "dq", "dk", "dv"), [got[0]] + got[2:], ref)):
+        a, r = a.double().view(n, heads, 64), r.view(n, heads, 64)
+        for dim in (0, 2):
+            keep = r.abs().amax(dim) > 0
+            err = ((a - r).norm(dim=dim) / r.norm(dim=dim).clamp_min(1e-300))[keep].max()
+            assert float(err) < (2e-6 if i == 0 else 5e-5), (name, dim, float(err))
+    # (three planes hold every exponent: powers of two moved from K to Q change no bit of a picked head)
+    if not picked:
+        return
+    s = 2.0 ** 9
+    same = _f32_call(x[0] * s, x[1] / s, x[2], x[3], 64, 64, heads, 0)
+    assert torch.equal(same[0].view(n, heads, 64)[:, 0], got[0].view(n, heads, 64)[:, 0])
