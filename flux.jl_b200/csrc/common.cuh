@@ -90,8 +90,9 @@ static inline bool fb_aligned16(const void* p) { return (reinterpret_cast<uintpt
 // placed as that one's leave, and wait there for its end and its stores.  What lies between two dependent kernels is then the wait and not a
 // launch.
 __device__ __forceinline__ void fb_after_previous() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
-// Short kernels of at most about one wave let the next one's blocks in at once, where there is room beside their own (a captured step of
-// 21 such kernels: 157 -> 148 us).  Long ones do not: the blocks that wait cost them more (bf16 step 1062 us, with this in all kernels 1094).
+// Short kernels let the next one's blocks in at once, where there is room beside their own (a captured step of 21 such kernels: 157 -> 148
+// us).  It counts when all blocks have said so or left: of a kernel with more blocks than fit, the last ones are placed first.  Long kernels
+// do not: the blocks that wait cost them more (bf16 step 1062 us, with this in all kernels 1094).
 __device__ __forceinline__ void fb_let_next_start() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 static inline cudaLaunchAttribute fb_early_start() {
   cudaLaunchAttribute a;
