@@ -85,6 +85,7 @@ FB_API int32_t fb_ctx_create(int32_t device, fb_ctx** out) {
   int32_t status = fb_side_kernels_prepare_elementwise();
   if (status == FB_OK) status = fb_side_kernels_prepare_peer();
   fb_gemm_query_clusters(c);
+  fb_dense_chain_query_clusters(c);
   if (status != FB_OK) {
     cudaMemPoolDestroy(c->pool);
     cudaFree(c->dev_error);

@@ -29,6 +29,7 @@ struct fb_ctx {
   uint32_t* host_page;   // pinned page that fb_read_scalar's kernel writes
   uint32_t host_seq;
   int clusters[4];       // clusters of 1, 2, 4, 8 CTAs that hold an SM each (GEMM kernels) and are resident at once
+  int chain_clusters;    // the same for the 16 CTAs of the chain of Dense layers
 };
 
 // thread-local last-error message
@@ -345,6 +346,7 @@ static inline float fb_planes_least(int64_t K) { return K < 2048 ? 1.0f / 64.0f 
 int32_t fb_planes_split(cudaStream_t stream, const fb_gemm_args& a, void* mem, fb_planes* out);
 int32_t fb_gemm_dispatch(fb_ctx* ctx, cudaStream_t stream, const fb_gemm_args& a, int precision);
 void fb_gemm_query_clusters(fb_ctx* ctx);
+void fb_dense_chain_query_clusters(fb_ctx* ctx);
 // attention_tc.cu: tensor-core attention; FB_ERR_UNSUPPORTED when the call is not taken
 int32_t fb_attn_fwd_tc(fb_ctx* ctx, cudaStream_t stream, const float* q, const float* k, const float* v, const uint8_t* mask,
                        float* o, float* lse, int64_t e_dim, int64_t ev_dim, int64_t lq, int64_t lk, int64_t batch, int nheads,

@@ -206,32 +206,29 @@ int32_t launch(fb_ctx* ctx, cudaStream_t stream, const DcArgs& A) {
   return FB_OK;
 }
 
-// clusters that are resident at once (7 on a whole B200: the largest GPCs hold one each)
-int resident_clusters() {
-  static const int count = [] {
-    cudaLaunchConfig_t lc = {};
-    cudaLaunchAttribute at[1];
-    at[0].id = cudaLaunchAttributeClusterDimension;
-    at[0].val.clusterDim.x = DC_CTAS;
-    at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
-    lc.gridDim = dim3(DC_CTAS);
-    lc.blockDim = dim3(DC_THREADS);
-    lc.dynamicSmemBytes = DC_SMEM;
-    lc.attrs = at;
-    lc.numAttrs = 1;
-    int n = 0;
-    if (fb_allow_smem(dense_chain_kernel<4>, DC_SMEM) != cudaSuccess ||
-        cudaFuncSetAttribute(dense_chain_kernel<4>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess ||
-        cudaOccupancyMaxActiveClusters(&n, dense_chain_kernel<4>, &lc) != cudaSuccess) {
-      cudaGetLastError();
-      n = 0;
-    }
-    return n;
-  }();
-  return count;
-}
-
 }  // namespace
+
+// How many clusters are resident at once (7 on a whole B200: the largest GPCs hold one each; called by fb_ctx_create).
+void fb_dense_chain_query_clusters(fb_ctx* ctx) {
+  cudaLaunchConfig_t lc = {};
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeClusterDimension;
+  at[0].val.clusterDim.x = DC_CTAS;
+  at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+  lc.gridDim = dim3(DC_CTAS);
+  lc.blockDim = dim3(DC_THREADS);
+  lc.dynamicSmemBytes = DC_SMEM;
+  lc.attrs = at;
+  lc.numAttrs = 1;
+  int n = 0;
+  if (fb_allow_smem(dense_chain_kernel<4>, DC_SMEM) != cudaSuccess ||
+      cudaFuncSetAttribute(dense_chain_kernel<4>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess ||
+      cudaOccupancyMaxActiveClusters(&n, dense_chain_kernel<4>, &lc) != cudaSuccess) {
+    cudaGetLastError();
+    n = 0;
+  }
+  ctx->chain_clusters = n;
+}
 
 FB_API int32_t fb_dense_chain_fwd(fb_ctx* ctx, void* stream, const int64_t* table, int32_t layers, const float* x, float* y, int64_t n) {
   FB_CHECK_CTX(ctx);
@@ -262,7 +259,7 @@ FB_API int32_t fb_dense_chain_fwd(fb_ctx* ctx, void* stream, const int64_t* tabl
     while (nb > 1 && (nb << A.layer[l].log_slice) > DC_WIDTH / DC_CTAS) nb /= 2;
   // Weights through 16 SMs instead of all: from about 2 MB a layer on (1.25 with 3 or 4 columns) the layers alone are faster (1024 -> 1024,
   // 4 MB: 9 us a layer here, 7 alone), and a second wave of clusters would double the time.
-  if (bytes > layers * (nb <= 2 ? (int64_t)2 << 20 : (int64_t)5 << 18) || (n + nb - 1) / nb > resident_clusters()) return FB_ERR_UNSUPPORTED;
+  if (bytes > layers * (nb <= 2 ? (int64_t)2 << 20 : (int64_t)5 << 18) || (n + nb - 1) / nb > ctx->chain_clusters) return FB_ERR_UNSUPPORTED;
   switch (nb) {
     case 4: return launch<4>(ctx, (cudaStream_t)stream, A);
     case 2: return launch<2>(ctx, (cudaStream_t)stream, A);
