@@ -128,12 +128,13 @@ def _dense_chain(layers, x):
     n, d = size[1] if len(size) == 2 else 1, size[0]
     if n > _CHAIN_COLUMNS or x.t.dtype != torch.float32:
         return None
-    table = []
+    table, left = [], len(layers) * _CHAIN_WEIGHTS
     for l in layers:
         if type(l) is not Dense or l.precision != "default":
             return None
         W, b = l.weight, l.bias
-        if W.size[1] != d or W.t.dtype != torch.float32 or (b is not False and b.t.dtype != torch.float32):
+        left -= W.size[0] * d
+        if left < 0 or W.size[1] != d or W.t.dtype != torch.float32 or (b is not False and b.t.dtype != torch.float32):
             return None
         d = W.size[0]
         table += (W.t.data_ptr(), 0 if b is False else b.t.data_ptr(), W.size[1], d, lib.ACT[l.σ])
@@ -145,6 +146,7 @@ def _dense_chain(layers, x):
     return None
 
 
+_CHAIN_WEIGHTS = 1 << 19   # weights of a layer, on average: with more the entry point takes no number of columns (looked at first, as a large model's every call comes here)
 _CHAIN_COLUMNS = 36   # four columns for each sixteen of 148 SMs: no call has more; fewer, where clusters do not fit so tightly, the entry point says itself
 
 

@@ -107,3 +107,18 @@ def test_arrays_of_other_shapes_are_refused_by_the_first_layer(size):
     with pytest.raises(F.DimensionMismatch) as layer:
         m.layers[0](x)
     assert str(chain.value) == str(layer.value)
+
+
+def test_large_weights_are_not_asked_about(monkeypatch):
+    """The entry point refuses them; a call on a few columns of a large model does not get that far.  (The line: its own, for one column.)"""
+    import fluxb200 as F
+    from fluxb200 import layers, lib
+    asked = []
+    real = lib.supported
+    monkeypatch.setattr(lib, "supported", lambda name, *a: asked.append(name) or real(name, *a))
+    g = torch.Generator(device="cuda").manual_seed(0)
+    x = lambda d: F.B200Array(torch.randn(d, device="cuda"), (d, 1))
+    for dims, taken in (([1024, 512, 512], True), ([1024, 512, 1024], True), ([1024, 512, 1025], False), ([2048, 2048, 8], False), ([8, 2048, 2048], False), ([1024, 512, 1024, 513], False)):
+        del asked[:]
+        y = layers._dense_chain(_chain(F, dims, "relu", g).layers, x(dims[0]))
+        assert (y is not None) == taken and asked == (["fb_dense_chain_fwd"] if taken else [])
