@@ -190,15 +190,31 @@ PROFILE = None   # optional {"names": set, "events": list}: CUDA events recorded
 
 def supported(name: str, *args) -> bool:
     """Calls an entry point that may answer FB_ERR_UNSUPPORTED without a message: whether it did what was asked."""
-    f = _fast.get(name)
-    status = f(*args) if f is not None else None
-    if status is None:
-        status = getattr(_lib, name)(*args)
+    prof = PROFILE
+    if prof is not None and name in prof["names"]:
+        status = _timed(prof, name, args)
+    else:
+        f = _fast.get(name)
+        status = f(*args) if f is not None else None
+        if status is None:
+            status = getattr(_lib, name)(*args)
     if status == 0:
         return True
     if status != ERR_UNSUPPORTED:
         check(status)
     return False
+
+
+def _timed(prof, name: str, args) -> int:
+    """The status of a call between two events, which are kept where it was done."""
+    import torch
+    e0, e1 = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+    e0.record()
+    status = getattr(_lib, name)(*args)
+    e1.record()
+    if status == 0:
+        prof["events"].append((name, args, e0, e1))
+    return status
 
 
 def call(name: str, *args):
@@ -213,11 +229,6 @@ def call(name: str, *args):
             if status is not None:
                 check(status)
     elif name in prof["names"]:
-        import torch
-        e0, e1 = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
-        e0.record()
-        check(getattr(_lib, name)(*args))
-        e1.record()
-        prof["events"].append((name, args, e0, e1))
+        check(_timed(prof, name, args))
         return
     check(getattr(_lib, name)(*args))

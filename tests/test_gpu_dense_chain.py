@@ -122,3 +122,20 @@ def test_large_weights_are_not_asked_about(monkeypatch):
         del asked[:]
         y = layers._dense_chain(_chain(F, dims, "relu", g).layers, x(dims[0]))
         assert (y is not None) == taken and asked == (["fb_dense_chain_fwd"] if taken else [])
+
+
+def test_named_entry_points_are_timed(monkeypatch):
+    """A call of several layers in one launch is seen where entry points are timed by name, and a refused one is not."""
+    import fluxb200 as F
+    from fluxb200 import lib
+    g = torch.Generator(device="cuda").manual_seed(0)
+    x = F.B200Array(torch.randn(64, device="cuda"), (64, 1))
+    small, long = _chain(F, [64, 32, 8], "relu", g), _chain(F, [64] * 10, "relu", g)
+    prof = {"names": {"fb_dense_chain_fwd", "fb_dense_fwd"}, "events": []}
+    monkeypatch.setattr(lib, "PROFILE", prof)
+    small(x)
+    assert [e[0] for e in prof["events"]] == ["fb_dense_chain_fwd"]
+    long(x)
+    torch.cuda.synchronize()
+    assert [e[0] for e in prof["events"]] == ["fb_dense_chain_fwd"] + ["fb_dense_fwd"] * 9
+    assert all(e[2].elapsed_time(e[3]) >= 0 for e in prof["events"])
