@@ -45,17 +45,31 @@ def test_layernorm(act, d, n, offset):
 
 
 @pytest.mark.parametrize("kind", ["layer", "batch"])
-def test_which_cotangents_take_it(kind):
-    """A factor times y itself; not a sum of two cotangents, nor a factor times another array."""
+def test_which_cotangents_take_it(kind, monkeypatch):
+    """A factor times y itself; not a sum of two cotangents, a factor times another array, nor a cotangent that somebody has read."""
     import fluxb200 as F
+    from fluxb200 import core, lib
     g = torch.Generator(device="cuda").manual_seed(0)
     m = F.LayerNorm(24) if kind == "layer" else F.BatchNorm(24)
     x = F.B200Array(_new(g, 24 * 10), (24, 10))
     other = F.B200Array(_new(g, 24 * 10), (24, 10))
-    scale = (lambda m: m.diag.scale) if kind == "layer" else (lambda m: m.γ)
-    grad = lambda f: [t for t in _arrays(F.withgradient(f, m)[1])]
-    one = grad(lambda m: F.sum_abs2(m(x)))
-    both = grad(lambda m: F.sum_abs2(F.add(m(x), other)))
+    calls, real = [], lib.call
+    monkeypatch.setattr(lib, "call", lambda name, *a: calls.append(name) or real(name, *a))
+    general, own = f"fb_{kind}norm_bwd_params", f"fb_{kind}norm_bwd_params_own"
+
+    def grad(f, entry):
+        del calls[:]
+        res = _arrays(F.withgradient(f, m)[1])
+        assert [c for c in calls if "norm_bwd" in c] == [entry], calls
+        return res
+    one = grad(lambda m: F.sum_abs2(m(x)), own)
+    both = grad(lambda m: F.sum_abs2(F.add(m(x), other)), general)
+    read = core.is_scaled
+    monkeypatch.setattr(core, "is_scaled", lambda g, y: (g.t, read(g, y))[1])   # (the cotangent's memory has been asked for)
+    import fluxb200.layers as layers
+    monkeypatch.setattr(layers, "is_scaled", core.is_scaled)
+    seen = grad(lambda m: F.sum_abs2(m(x)), general)
+    assert all(torch.equal(a, b) for a, b in zip(seen, one))
     h = x.t.double().view(10, 24)
     h = (h - h.mean(1, keepdim=True)) / (h.var(1, unbiased=False, keepdim=True) + 1e-5).sqrt() if kind == "layer" else \
         (h - h.mean(0)) / (h.var(0, unbiased=False) + 1e-5).sqrt()
@@ -65,7 +79,6 @@ def test_which_cotangents_take_it(kind):
         got = sorted(got, key=lambda t: float(t.double().norm()))
         for a, b in zip(got, want):
             assert float((a.double() - b).abs().max()) < 1e-5 * float(dy.abs().sum(0).max())
-    assert scale(m) is not None
 
 
 def _arrays(v):
