@@ -598,7 +598,8 @@ Dims bn_dims(const fb_ctx* ctx, int64_t s, int64_t c, int64_t n, int W, int nt, 
 template <typename K, typename... A>
 int32_t bn_launch(K kern, cudaStream_t stream, const Dims& g, int64_t clusters, int nt, size_t smem, A... args) {
   FB_REQUIRE(clusters * g.split <= 0x7fffffff, FB_ERR_SHAPE, "batchnorm: too many channels");
-  if (smem > 48 * 1024) FB_CUDA(fb_allow_smem(kern, BN_CACHE_MAX));
+  // (48 KB without asking, the kernels' static shared memory included)
+  if (smem > 48 * 1024 - sizeof(Exchange)) FB_CUDA(fb_allow_smem(kern, BN_CACHE_MAX));
   cudaLaunchConfig_t lc;
   memset(&lc, 0, sizeof(lc));
   lc.gridDim = dim3((unsigned)(clusters * g.split), 1, 1);
