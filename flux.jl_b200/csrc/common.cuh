@@ -66,8 +66,10 @@ struct fb_temp {
 #define FB_CUDA(call)                                                                        \
   do {                                                                                       \
     cudaError_t e__ = (call);                                                                \
-    if (e__ != cudaSuccess)                                                                  \
+    if (e__ != cudaSuccess) {                                                                \
+      cudaGetLastError();   /* (the next call's launch check would find it) */               \
       return fb_fail(FB_ERR_CUDA, "%s: %s failed: %s", __func__, #call, cudaGetErrorString(e__)); \
+    }                                                                                        \
   } while (0)
 
 extern unsigned long long g_fb_kernel_launches;   // kernels launched by this library in this process

@@ -53,3 +53,27 @@ def test_shared_memory_of_two_threads(make, large, small):
     for t in threads:
         t.join()
     assert not errors, errors[0]
+
+
+def test_an_error_is_reported_once():
+    """A runtime call that fails (here: a wait inside a capture) is the error of the entry point that made it, not of the next one."""
+    import fluxb200 as F
+    from fluxb200 import lib
+    ctx = F.context(0)
+    x, y, m, r = torch.randn(64 * 10, device="cuda"), torch.empty(640, device="cuda"), torch.empty(10, device="cuda"), torch.empty(10, device="cuda")
+    out = torch.zeros(1, dtype=torch.int32).pin_memory()
+    side, graph = torch.cuda.Stream(), torch.cuda.CUDAGraph()
+    torch.cuda.synchronize()
+    with torch.cuda.stream(side):
+        graph.capture_begin(capture_error_mode="relaxed")
+        status = lib.raw().fb_device_error(ctx.handle, side.cuda_stream, C.cast(out.data_ptr(), C.POINTER(C.c_int32)))
+    after = lib.raw().fb_layernorm_fwd(ctx.handle, torch.cuda.default_stream().cuda_stream, x.data_ptr(), None, None, y.data_ptr(), m.data_ptr(), r.data_ptr(), 64, 10,
+                                       1e-5, 0)
+    with torch.cuda.stream(side):
+        try:
+            graph.capture_end()
+        except RuntimeError:
+            pass
+    torch.cuda.synchronize()
+    assert status != 0 and after == 0, (status, after)
+    assert torch.isfinite(y).all() and ctx.device_error() == 0
