@@ -564,11 +564,11 @@ def small_config_lines(config, steps, warmup):
         one, zero = np.ones(256, np.float32), np.zeros(256, np.float32)
         cpu = time_cpu(lambda: (O.batchnorm_fwd_train(xs, one, zero, zero.copy(), one.copy(), sigma="relu"),
                                 O.batchnorm_bwd(xs, one, zero, 2 * xs, sigma="relu")))
-        by = 11.0 * E * 4
+        by = 4.0 * E * 4
         add("batchnorm: BatchNorm(256,relu) train, 32x32x256x128 Float32, forward + gradient of sum(abs2,y)", 128, ms, clocks,
             {"bound": "hbm", "achieved": by / ms / 1e6, "peak": hbm, "unit": "GB/s", "frac": by / ms / 1e6 / hbm, "traffic": None,
              "bytes_per_step": by,
-             "note": "11 passes x 134.2 MB: layer (8) + sum(abs2) read (1) + cotangent 2y read+write (2); " + how},
+             "note": "4 passes x 134.2 MB: forward reads x and writes y, sum(abs2) reads y, the parameters' gradients read x; " + how},
             ms_e2e, h2d, 8 / cpu, "8 of 128 samples, best of 2")
         del xg, run, bn
         torch.cuda.empty_cache()
@@ -581,11 +581,11 @@ def small_config_lines(config, steps, warmup):
         xls = xl[:, :1024]
         g1, b1 = np.ones(4096, np.float32), np.zeros(4096, np.float32)
         cpu = time_cpu(lambda: (O.layernorm_fwd(xls, g1, b1), O.layernorm_bwd(xls, g1, b1, 2 * xls)))
-        by = 8.0 * xl.size * 4
+        by = 4.0 * xl.size * 4
         add("layernorm: LayerNorm(4096) on 4096x16384 Float32, forward + gradient of sum(abs2,y)", 16384, ms, clocks,
             {"bound": "hbm", "achieved": by / ms / 1e6, "peak": hbm, "unit": "GB/s", "frac": by / ms / 1e6 / hbm, "traffic": None,
              "bytes_per_step": by,
-             "note": "8 passes x 268.4 MB: layer (5) + sum(abs2) read (1) + cotangent 2y read+write (2); " + how},
+             "note": "4 passes x 268.4 MB: forward reads x and writes y, sum(abs2) reads y, the parameters' gradients read x; " + how},
             ms_e2e, h2d, 1024 / cpu, "1024 of 16384 samples, best of 2")
     elif config == 3:
         Hh, T, B = 512, 256, 64
@@ -631,7 +631,7 @@ def small_config_lines(config, steps, warmup):
                 8, ms, clocks,
                 {"bound": "tensor", "achieved": flops / ms / 1e9, "peak": peak, "unit": "TFLOP/s", "frac": flops / ms / 1e9 / peak, "traffic": None,
                  "flops_per_step": flops,
-                 "note": ("projections on tcgen05 as half-precision planes or 3xTF32, the attention core (forward, dQ, dK/dV) on two half-precision planes per operand; softmax and dS on TMEM read-back; "
+                 "note": ("projections on tcgen05 as half-precision planes or 3xTF32, the attention core (forward, dQ, dK/dV) on two half-precision planes per operand (three bf16 planes where scores are large); softmax and dS on TMEM read-back; "
                           if dtype == "f32" else "the opt-in bf16 path (fluxb200.bf16); ") + how},
                 ms_e2e, h2d, (1 * (512 / 2048) ** 2 * 1.0) / cpu,
                 "1 of 8 samples at seq 512 (1/16 of a sample's attention work, 1/4 of its projections), Float32, 1 run", dtype=dtype)
