@@ -50,10 +50,31 @@ __device__ __forceinline__ float unscale(float v, int e) {
   const int h = e >> 1;
   return v * __int_as_float((h + 127) << 23) * __int_as_float((e - h + 127) << 23);
 }
+// One lane issues, its operands moved to uniform registers one by one (the other GEMM kernels' way takes 88 -> 64 clocks an MMA): here the quicker issue
+// makes the kernel slower, alone as well as at the power limit (8192 x 4096 x 4096: 533 us so, 542 by a converged warp, each within 1 us over
+// several runs in turn; what it then waits for was not found).
 template <bool PAIR>
 __device__ __forceinline__ void tc_mma_h(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc, uint32_t accumulate) {
-  if (PAIR) tc_mma2_f16(d_tmem, a_desc, b_desc, idesc, accumulate);
-  else tc_mma_f16(d_tmem, a_desc, b_desc, idesc, accumulate);
+  if (PAIR)
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "setp.ne.b32 p, %4, 0;\n\t"
+        "tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, {%5, %5, %5, %5, %5, %5, %5, %5}, p;\n\t}"
+        ::"r"(d_tmem), "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate), "r"(0u)
+        : "memory");
+  else
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "setp.ne.b32 p, %4, 0;\n\t"
+        "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, {%5, %5, %5, %5}, p;\n\t}"
+        ::"r"(d_tmem), "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate), "r"(0u)
+        : "memory");
+}
+__device__ __forceinline__ void commit_own(uint32_t bar) {
+  asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar) : "memory");
+}
+__device__ __forceinline__ void commit_pair(uint32_t bar, uint16_t mask) {
+  asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;" ::"r"(bar), "h"(mask) : "memory");
 }
 
 // One operand as its elements are read beside its images: those that the images leave out are listed row by row (planes.cu)
@@ -304,7 +325,7 @@ gemm_planes_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constan
     }
   } else if (warp == 1) {
     // -------------------------------------------------- MMA issuer (the leader CTA of a pair) ---
-    if (leader) {
+    if (lane == 0 && leader) {
       // instruction descriptor: D = F32, A = B = F16 (code 0), operand majors, N >> 3, M >> 4
       const uint32_t idesc = (1u << 4) | ((uint32_t)a_mn << 15) | ((uint32_t)b_mn << 16) | ((uint32_t)(BN >> 3) << 17) |
                              ((uint32_t)((BM * RANKS) >> 4) << 24);
@@ -324,10 +345,10 @@ gemm_planes_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constan
           const int buf = sc & 1, use = sc >> 1;
           if (kb_in_seg == 0 && use > 0) {
             // the epilogue warps must have drained this accumulator buffer's previous segment
-            ok = warp_wait_cluster(tmem_empty_bar(buf), (uint32_t)(use - 1) & 1u, s_abort);
+            ok = mbar_wait_cluster(tmem_empty_bar(buf), (uint32_t)(use - 1) & 1u, s_abort);
             if (!ok) break;
           }
-          ok = warp_wait_cluster(full_bar(s), ph, s_abort);
+          ok = mbar_wait_cluster(full_bar(s), ph, s_abort);
           if (!ok) break;
           tc_fence_after();
           const uint32_t d_tmem = tmem_base + (uint32_t)(buf * BN);
@@ -343,11 +364,11 @@ gemm_planes_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constan
           }
           const bool seg_end = (kb_in_seg == SEG_KB - 1 || kb == p.kb1 - 1);
           if (PAIR) {
-            tc_commit2_mc(empty_bar(s), (uint16_t)(3u << lead_rank));                 // frees the stage in both CTAs
-            if (seg_end) tc_commit2_mc(tmem_full_bar(buf), (uint16_t)(3u << lead_rank));
+            commit_pair(empty_bar(s), (uint16_t)(3u << lead_rank));                 // frees the stage in both CTAs
+            if (seg_end) commit_pair(tmem_full_bar(buf), (uint16_t)(3u << lead_rank));
           } else {
-            tc_commit(empty_bar(s));
-            if (seg_end) tc_commit(tmem_full_bar(buf));
+            commit_own(empty_bar(s));
+            if (seg_end) commit_own(tmem_full_bar(buf));
           }
           kb_in_seg = seg_end ? 0 : kb_in_seg + 1;
           if (seg_end) ++sc;
