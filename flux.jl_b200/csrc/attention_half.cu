@@ -6,8 +6,10 @@
 // a small kernel (`attn_half_split_kernel`) makes the images of K, V, Q and dO once per call, and tiles arrive by plain bulk copies.
 // Head sizes below 64 are padded with zeros in the images; their zero 16-feature steps are skipped.
 //
-// Against three bf16 planes per operand and six products (batch 8, 16 heads of 64, 2048 x 2048, causal; us): images 51 + 114 -> 41
-// + 91, forward 507 -> 350, dK / dV 1113 -> 579, dQ 848 -> 499.  Errors against float64: output 2.3e-7 as before, dQ 4.7e-6 -> 0.9e-6, dK / dV 1.9e-5 -> 3.8e-6 (half as many truncating adds).
+// Against three bf16 planes per operand and six products (batch 8, 16 heads of 64, 2048 x 2048, causal; us): forward 507 -> 349, dK / dV 1113 -> 618,
+// dQ 848 -> 503; images 51 + 114 -> 67 + 104 (with a look at Q ahead of the forward kernel).  Errors against float64: output 2.3e-7
+// as before, dQ 4.7e-6 -> 0.9e-6, dK / dV 1.9e-5 -> 3.8e-6 (half as many truncating adds).  Heads that these planes would hold worse are left to
+// attention_tc.cu, see below.
 // What bounds them: an MMA with N = 64 takes 53 clocks with A in tensor memory and 74 with A in shared memory, where its multiplications
 // need 32, and between the MMAs of a block the weights' arithmetic (one warp of a set per SM partition, 3700 clocks a block).
 //
@@ -879,7 +881,7 @@ attn_bwd_dq_half_kernel(const float* __restrict__ q, const float* __restrict__ d
 // Scales as in the dQ kernel: dS' in units of 2^-(sv of the key's tile + sdomin), P' times 2^15; the shifts of the dO and Q tiles above the
 // least ones go into P' and dS'.
 struct KvCfg {
-  // Compute warps per set: eight with half a row of a block each (four, a thread with a whole row: 659 us, here 579; batch 8, 16 heads, 2048 x
+  // Compute warps per set: eight with half a row of a block each (four, a thread with a whole row: 659 us, here 579 - 618; batch 8, 16 heads, 2048 x
   // 2048, causal).  The dQ kernel gains nothing from it (499 -> 517).
   static constexpr int HALVES = 2;
   static constexpr int THREADS = 64 + 256 * HALVES;

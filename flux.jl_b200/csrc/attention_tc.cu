@@ -7,9 +7,10 @@
 // (`attn_split_kernel`; for picked heads the kernels that pick them) lays K, V, Q and dO out once per call as the images that the MMAs read from
 // shared memory, and tiles arrive by plain bulk copies.  Head sizes below 64 are padded with zeros in those images; their zero 16-feature steps are skipped.
 //
-// (Two half-precision planes for the probabilities and dS, as attention_half.cu has them, take a third of these MMAs away, but hold 23 bits
-// of them and, where the scales of a head's tiles differ, fewer.)  What bounds the kernels: an MMA with N = 64 takes 44 clocks where its
-// multiplications need 32, and between the MMAs of a block the weights' arithmetic.
+// (For bf16 operands two half-precision planes of the probabilities and dS, as attention_half.cu has them, take a third of these MMAs away, but hold
+// 23 bits of a weight above 2^-29 and ever fewer below: forward 299 -> 274 us, dK / dV 471 -> 445, dQ 319 -> 330 for batch 8, 16 heads of 64,
+// 2048 x 2048, causal.)  What bounds the kernels: an MMA with N = 64 takes 44 clocks where its multiplications need 32, and between
+// the MMAs of a block the weights' arithmetic.
 //
 // A block is 64 keys (64 queries in the dK / dV kernel) against the 128 rows of a CTA; a thread of a compute warp owns
 // one row (one TMEM lane).  Every mbarrier wait is bounded; when one runs out the kernel records 4002 (forward), 4003

@@ -543,11 +543,13 @@ const void* seq_bwd_kernel(int ug, int bg) {
 }
 
 // The same for the tensor-core kernels (16 units x 8 or 16 columns a CTA).  Hidden sizes from 48 up to 512 (beyond, the fragments of the
-// weights do not fit the registers), and sequences long enough to pay for the start (fragments, the buffer's fill).  Against the
-// FMA kernels (us, forward and backward with their bulk products): LSTM 512 x 64 columns, 256 steps 1650 + 2390 -> 890 + 1550; 4
-// steps 46 + 78 -> 39 + 75, 2 steps 35 + 67 -> 35 + 68, 1 step 25 + 48 -> 28 + 50; GRU 257 x 128, 50 steps 231 + 463 -> 156 + 360;
-// 200 x 20, 50 steps 105 + 169 -> 97 + 162; 100 x 20, 3 steps 22 + 40 -> 27 + 43; LSTM 48 x 128, 50 steps 103 + 166 -> 97 + 148;
-// 32 x 128, 20 steps 45 + 74 -> 48 + 76; 16 x 1, 100 steps 143 + 167 -> 145 + 160.
+// weights do not fit the registers), and sequences long enough to pay for the start (fragments, the buffer's fill).  The lines and the cost
+// were drawn against the FMA kernels with an earlier backward kernel, which exchanged gate derivatives (us, forward and backward with bulk
+// products): LSTM 512 x 64 columns, 256 steps 1650 + 2390 -> 890 + 1550; 4 steps 46 + 78 -> 39 + 75, 2 steps 35 + 67 -> 35 + 68, 1 step 25 +
+// 48 -> 28 + 50; GRU 100 x 20, 3 steps 22 + 40 -> 27 + 43; LSTM 48 x 128, 50 steps 103 + 166 -> 97 + 148; 32 x 128, 20 steps 45 + 74 -> 48 + 76; 16
+// x 1, 100 steps 143 + 167 -> 145 + 160.  The present backward kernel is no slower at any of 240 sizes tried above the lines (H 48 - 512, 1 - 512
+// columns, 4 - 200 steps: by 1.0 at 48 to 1.46 at 400 units), also where its exchange of (H / 16)^2 blocks a step leaves L2: LSTM 512, 50 steps, 64, 130, 256 and 512
+// columns 369, 885, 1260, 2489 -> 274, 651, 970, 2052; and where the buffer's fill is most of a short sequence: 130 columns, 4 steps 109 -> 81.
 bool plan_mma(const fb_ctx* ctx, int ng, int H, int64_t B, int64_t T, bool bwd, SeqPlan* best) {
   if (!persistent_enabled() || B > (1 << 20) || H < 48 || H > 512 || T * H < 1536) return false;
   const int ugroups = (H + MQ_UG - 1) / MQ_UG;

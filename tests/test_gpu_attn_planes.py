@@ -1,4 +1,4 @@
-"""Tensor-core attention (half-precision planes): head sizes, ragged tiles, unseen keys and slot / region reuse against float64."""
+"""Tensor-core attention (half-precision planes, bf16 planes): head sizes, ragged tiles, unseen keys and slot / region reuse against float64."""
 import numpy as np
 import pytest
 
@@ -314,7 +314,7 @@ def test_attention_captured_without_warm_up():
 
 
 def _skewed(kind, q, k, v, do, heads):
-    """Inputs whose planes lose something: heads that hold such values go to the Float32 kernels."""
+    """Inputs of which half-precision planes would lose something: heads that hold such values are computed on three bf16 planes."""
     if kind == "graded":           # every third feature 2^30 larger in K and V, and as much smaller in Q and dO
         s = torch.ones(q.shape[-1], device=q.device)
         s[::3] = 2.0 ** 30
