@@ -454,10 +454,11 @@ def test_picked_heads_have_the_bits_of_bf16_operands(heads, lq, lk, batch, causa
         assert torch.equal(got.bfloat16(), want)
 
 
-@pytest.mark.parametrize("heads,n,batch,causal,shift", [(16, 2048, 4, 1, 0), (5, 200, 3, 0, 0), (7, 130, 2, 1, 1), (33, 64, 40, 0, 0)])
+@pytest.mark.parametrize("heads,n,batch,causal,shift", [(16, 2048, 4, 1, 0), (5, 200, 3, 0, 0), (7, 130, 2, 1, 1), (33, 64, 40, 0, 0), (16, 1024, 45, 0, 0)])
 @pytest.mark.parametrize("which", ["all", "some", "none of the first"])
 def test_heads_are_picked_one_by_one(heads, n, batch, causal, shift, which):
-    """A head has the bits that it has in a call of its own, whatever the others are: up to eight picked tiles a CTA, none, and a few."""
+    """A head has the bits that it has in a call of its own, whatever the others are: up to eight picked tiles a CTA, none, and a few; images of
+    three chunks of the batch (the last size)."""
     g = torch.Generator(device="cuda").manual_seed(heads)
     mk = lambda: torch.randn(batch * n * heads * 64 + 4, device="cuda", generator=g)[shift:shift + batch * n * heads * 64].view(batch, n, heads, 64)
     q, k, v, do = mk(), mk(), mk(), mk()
@@ -515,3 +516,35 @@ def test_which_tiles_the_planes_hold(what, picked, operand):
     s = 2.0 ** 9
     same = _f32_call(x[0] * s, x[1] / s, x[2], x[3], 64, 64, heads, 0)
     assert torch.equal(same[0].view(n, heads, 64)[:, 0], got[0].view(n, heads, 64)[:, 0])
+
+
+def test_a_replayed_graph_picks_anew():
+    """Which heads are picked is decided on the device: a graph captured with ordinary inputs gives what an eager call gives of others."""
+    import fluxb200 as F
+    from fluxb200 import lib
+    g = torch.Generator(device="cuda").manual_seed(2)
+    heads, n, batch = 4, 300, 2
+    sets = [[torch.randn(batch, n, heads * 64, device="cuda", generator=g) for _ in range(4)] for _ in range(3)]
+    sets[1][0][0, :, :64] *= 12.0
+    sets[2][0] *= 12.0
+    want = [_f32_call(*s, 64, 64, heads, 1) for s in sets]
+    q, k, v, do = (t.clone() for t in sets[0])
+    o, lse = torch.empty_like(q), torch.empty(batch * heads * n, device="cuda")
+    dq, dk, dv = (torch.empty_like(t) for t in (q, k, v))
+    ctx, p, dims = F.context(), lambda t: t.data_ptr(), (heads * 64, heads * 64, n, n, batch, heads, 1)
+
+    def call():
+        lib.call("fb_attn_fwd", ctx.handle, ctx.stream, p(q), p(k), p(v), None, p(o), p(lse), *dims)
+        lib.call("fb_attn_bwd", ctx.handle, ctx.stream, p(q), p(k), p(v), None, p(o), p(lse), p(do), p(dq), p(dk), p(dv), *dims)
+    call()
+    torch.cuda.synchronize()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        call()
+    for s, ref in list(zip(sets, want)) * 2:
+        for t, new in zip((q, k, v, do), s):
+            t.copy_(new)
+        graph.replay()
+        torch.cuda.synchronize()
+        assert all(torch.equal(a, b) for a, b in zip((o, lse, dq, dk, dv), ref))
+    assert ctx.device_error() == 0
