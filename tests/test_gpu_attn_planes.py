@@ -548,3 +548,53 @@ def test_a_replayed_graph_picks_anew():
         torch.cuda.synchronize()
         assert all(torch.equal(a, b) for a, b in zip((o, lse, dq, dk, dv), ref))
     assert ctx.device_error() == 0
+
+
+@pytest.mark.parametrize("lq,lk,causal,low", [(200, 300, 0, False), (130, 130, 1, False), (200, 300, 0, True), (130, 130, 1, True), (2100, 70, 0, False), (70, 2100, 0, False)])
+def test_gradients_of_heads_that_are_not_finite(lq, lk, causal, low):
+    """Heads with an infinite or NaN operand have the gradients of the FMA kernels (reached through an additive bias of zeros): the same values
+    are finite, and those agree as Float32 sums in two orders do (2e-5 of the head; bf16 results 2^-8).  The other heads keep their bits."""
+    import fluxb200 as F
+    from fluxb200 import lib
+    g = torch.Generator(device="cuda").manual_seed(lq)
+    heads, batch, inf = 5, 2, float("inf")
+    E, ctx = 64 * heads, F.context()
+    p, dims = lambda t: t.data_ptr(), (E, E, lq, lk, batch, heads, causal)
+    x = [torch.randn(batch, n, heads, 64, device="cuda", generator=g) for n in (lq, lk, lk, lq)]
+    if low:
+        x = [t.bfloat16().float() for t in x]
+    zero_bias = torch.zeros(lk * lq, device="cuda")
+
+    def gradients(q, k, v, do, general):
+        o, lse = torch.empty(batch, lq, E, device="cuda"), torch.empty(batch * heads * lq, device="cuda")
+        if low and not general:
+            q, k, v, do = (t.bfloat16() for t in (q, k, v, do))
+            out, dq, dk, dv = (torch.empty_like(t) for t in (q, q, k, v))
+            lib.call("fb_attn_fwd_bf16", ctx.handle, ctx.stream, p(q), p(k), p(v), p(o), p(out), p(lse), *dims)
+            lib.call("fb_attn_bwd_bf16", ctx.handle, ctx.stream, p(q), p(k), p(v), p(o), p(lse), p(do), p(dq), p(dk), p(dv), *dims)
+        else:
+            dq, dk, dv = (torch.empty_like(t) for t in (q, k, v))
+            b = p(zero_bias) if general else None
+            lib.call("fb_attn_fwd_ex", ctx.handle, ctx.stream, p(q), p(k), p(v), None, b, 0, 0, 0.0, 0, 0, p(o), p(lse), *dims)
+            lib.call("fb_attn_bwd_ex", ctx.handle, ctx.stream, p(q), p(k), p(v), None, b, 0, 0, 0.0, 0, 0, p(o), p(lse), p(do), None, p(dq), p(dk), p(dv), *dims)
+        assert ctx.device_error() == 0
+        return [t.view(batch, -1, heads, 64).float() for t in (dq, dk, dv)]
+    clean = gradients(*x, False)
+    bad = [t.clone() for t in x]
+    bad[0][0, lq // 2, 0, 1] = inf
+    bad[1][0, lk // 3, 1, 0] = -inf
+    bad[2][1, 3, 2, 5] = inf
+    bad[3][1, lq - 1, 3, 7] = float("nan")
+    got, ref = gradients(*bad, False), gradients(*bad, True)
+    touched = {(0, 0), (0, 1), (1, 2), (1, 3)}
+    for name, a, r, c in zip(("dq", "dk", "dv"), got, ref, clean):
+        for b in range(batch):
+            for h in range(heads):
+                if (b, h) not in touched:
+                    assert torch.equal(a[b, :, h], c[b, :, h]), (name, b, h)
+                    continue
+                fine = torch.isfinite(r[b, :, h])
+                assert torch.equal(torch.isfinite(a[b, :, h]), fine), (name, b, h)
+                if bool(fine.any()):
+                    err = float((a[b, :, h] - r[b, :, h])[fine].abs().max() / r[b, :, h][fine].abs().max().clamp_min(1e-30))
+                    assert err < (2.0 ** -8 if low else 2e-5), (name, b, h, err)
